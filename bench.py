@@ -656,7 +656,7 @@ def run_ours(args):
                "call": "cb200_host_forward (C ABI, pinned host buffers, %d chunk buffers of %d rows; gene indices cross as gap bytes "
                        "while the host rewrites them fast enough)" % (so.chunk_buffers, so.max_chunk_rows),
                "h2d_bytes_per_entry": float(h2d.value) / max(1.0, float(x.nnz)),
-               "schedule": "gene_tiled (codes read at launch)", "stage_device_bytes": int(L.cb200_host_stage_device_bytes(stage)),
+               "schedule": "warp_per_row (codes read at launch)", "stage_device_bytes": int(L.cb200_host_stage_device_bytes(stage)),
                "aggregate_h2d_gbs": world * h2d.value / (e_ms * 1e-3) / 1e9}
         if rank == 0:   # the host result against the device-resident result of the exact schedule, sampled rows vs the oracle
             e2e["parity_check"] = parity_of_what_ran(dict(wl, out=y_host), _NoStatus(), False)

@@ -59,10 +59,10 @@ struct cb200_prepared {
     cb200_spmm_problem problem;
     fwd_schedule schedule;
     const char *schedule_name;
-    std::uint64_t workspace_bytes;
+    std::uint64_t workspace_bytes;    // what the schedule can use
+    std::uint64_t workspace_required; // what a launch has to bring
     std::uint32_t workspace_alignment;
     int sm_count;
-    double mean_row_nnz, max_row_nnz;
     // persistent state built at prepare time (persistent_kernel_state, operation_core.hh:126-129):
     // the rows in descending order of length, on the device; null when no host row_ptr was given
     std::int32_t *row_order;
@@ -372,16 +372,11 @@ schedule_plan plan_schedule(const cb200_spmm_problem &pr) {
         plan.blocked_lo = blocked && plan.split && (limit == 0u || nnz * 8u <= limit);
         return plan;
     }
-    // CSR forward.  Row schedule from the nnz/row distribution: the gene-tiled kernel pays a fixed cost per
-    // (row, gene tile) visit, so it needs enough stored entries per visit and enough row groups to fill the
-    // SMs; short or few rows go to the warp-per-row kernel.
+    // CSR forward.  fp32 products on the CUDA cores: the gather kernel, whose CTAs share their rows' entries evenly, is the
+    // faster one over the whole range (20,000 x 360 entries: 0.09 ms, gene-tiled 0.92; 125,000 x 1,800 at N = 64: 2.5 ms
+    // against 4.4); the gene-tiled one runs where it is asked for by name.
     const std::int64_t row_bytes = pr.n * (pr.dense_dtype == CB200_DTYPE_BF16 ? 2 : 4);
-    const bool shape_ok = (pr.n == 32 || pr.n == 64 || pr.n == 128) && row_bytes <= 256;
-    const double tile_genes = row_bytes > 0 ? 98304.0 / static_cast<double>(row_bytes) : 0.0;
-    const double per_visit = pr.k > 0 ? plan.mean_row_nnz * tile_genes / static_cast<double>(pr.k) : 0.0;
-    bool tiled = shape_ok && pr.m >= 16 * 128 && (per_visit >= 6.0 || tile_genes >= pr.k);
-    if (hint_is(hint, "warp_per_row")) tiled = false;
-    if (hint_is(hint, "gene_tiled")) tiled = shape_ok;
+    bool tiled = hint_is(hint, "gene_tiled") && (pr.n == 32 || pr.n == 64 || pr.n == 128) && row_bytes <= 256;
     // bf16 products allowed: the tensor-core kernel, which treats 512-row x 64-gene windows as dense.  That
     // pays once a window holds enough stored entries (density) and there are row groups for every SM;
     // otherwise the exact kernels above run (they satisfy the policy too).
@@ -411,8 +406,8 @@ schedule_plan plan_schedule(const cb200_spmm_problem &pr) {
     // second array with the next eight mantissa bits when the limit has room for it
     plan.blocked_lo = blocked && split && (limit == 0u || nnz * 8u <= limit);
     if (blocked) {
-        tiled = false; // no length-sorted row order: the copy works in natural row order, and the exact
-        tensor = false; // kernel that serves unaligned row ranges runs in natural order too
+        tiled = false; // no length-sorted row order: the copy works in natural row order, as does the exact
+        tensor = false; // kernel that serves unaligned row ranges
         // Dense enough, bf16 products, and room for rows x genes x 2 bytes: keep the decoded operand tiles
         // instead of the entry words; a launch then streams them and decodes nothing.
         const std::uint64_t tile_bytes = qcsr_dense_tile_bytes(pr.m, pr.k);
@@ -518,8 +513,6 @@ cb200_status cb200_spmm_prepare(const cb200_spmm_problem *problem, cb200_prepare
     p->schedule_name = "warp_per_row";
     p->workspace_alignment = 256u;
     p->workspace_bytes = 0u;
-    p->mean_row_nnz = plan.mean_row_nnz;
-    p->max_row_nnz = p->mean_row_nnz;
     p->bell_cuda_cores = plan.bell_cuda_cores;
     p->arena.borrowed = problem->persistent != nullptr;
     p->arena.base = static_cast<unsigned char *>(problem->persistent);
@@ -537,14 +530,6 @@ cb200_status cb200_spmm_prepare(const cb200_spmm_problem *problem, cb200_prepare
         return abandon(fail(CB200_STATUS_INSUFFICIENT_WORKSPACE, "persistent memory of %llu bytes needed (cb200_spmm_persistent_requirement), %llu given",
                             (unsigned long long)plan_persistent_bytes(*problem, plan), (unsigned long long)p->arena.capacity));
 
-    if (problem->host_row_ptr != nullptr && problem->projection != CB200_PROJECTION_BLOCKED_ELL) {
-        int64_t longest = 0;
-        for (int64_t r = 0; r < problem->m; ++r) {
-            const int64_t c = problem->host_row_ptr[r + 1] - problem->host_row_ptr[r];
-            if (c > longest) longest = c;
-        }
-        p->max_row_nnz = static_cast<double>(longest);
-    }
     device_scope scope(problem->device);
     if (scope.status != cudaSuccess) return abandon(fail(CB200_STATUS_CUDA_ERROR, "%s", cudaGetErrorString(scope.status)));
 
@@ -580,7 +565,8 @@ cb200_status cb200_spmm_prepare(const cb200_spmm_problem *problem, cb200_prepare
             p->schedule = fwd_schedule::gene_tiled;
             p->schedule_name = "gene_tiled";
         }
-        p->workspace_bytes = qcsr_tiled_workspace_bytes(); // status word of the tiled kernel
+        p->workspace_bytes = plan.tiled ? qcsr_tiled_workspace_bytes()
+                                        : qcsr_gather_workspace_bytes(problem->k, problem->nnz, problem->n, problem->dense_dtype);
         if (plan.tensor_windows) {
             p->schedule = fwd_schedule::tensor_windows;
             p->schedule_name = "tensor_windows";
@@ -641,6 +627,9 @@ cb200_status cb200_spmm_prepare(const cb200_spmm_problem *problem, cb200_prepare
             p->persistent_bytes += bytes;
         }
     }
+    // the gather kernel runs with the status block alone: without room for W re-laid it reads W as it is
+    const bool gathers = problem->projection == CB200_PROJECTION_CSR && p->schedule == fwd_schedule::warp_per_row;
+    p->workspace_required = gathers ? std::min<std::uint64_t>(p->workspace_bytes, 256u) : p->workspace_bytes;
     *out = p;
     return CB200_STATUS_SUCCESS;
 }
@@ -693,12 +682,12 @@ cb200_status cb200_spmm_run(const cb200_prepared *prepared, const cb200_launch *
     if (launch->workspace_device != launch->device)
         return fail(CB200_STATUS_INVALID_STREAM, "workspace lives on device %d, stream on device %d",
                     launch->workspace_device, launch->device);
-    if (launch->workspace_bytes < prepared->workspace_bytes ||
-        (prepared->workspace_bytes != 0u &&
+    if (launch->workspace_bytes < prepared->workspace_required ||
+        (prepared->workspace_required != 0u &&
          (launch->workspace == nullptr ||
           (reinterpret_cast<std::uintptr_t>(launch->workspace) & (prepared->workspace_alignment - 1u)) != 0u)))
         return fail(CB200_STATUS_INSUFFICIENT_WORKSPACE, "workspace of %llu bytes needed, %llu given",
-                    (unsigned long long)prepared->workspace_bytes, (unsigned long long)launch->workspace_bytes);
+                    (unsigned long long)prepared->workspace_required, (unsigned long long)launch->workspace_bytes);
     /* lifetimes.hh:160-172: the expected generation of a bound value plane must be the live one; here the
      * "live" values of a prepared copy are those it was built from */
     if ((prepared->blocked.seg_ptr != nullptr || prepared->blocked.dense_tiles != nullptr || prepared->blocked.code_tiles != nullptr ||

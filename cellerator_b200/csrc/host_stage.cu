@@ -346,7 +346,6 @@ struct chunk_buffer {
 struct cb200_host_stage {
     cb200_host_stage_options o{};
     int sm_count = 0;
-    fwd_schedule schedule = fwd_schedule::warp_per_row;
     cudaStream_t h2d = nullptr, compute = nullptr, d2h = nullptr;
     void *w = nullptr;
     float *scales = nullptr, *offsets = nullptr;
@@ -420,14 +419,7 @@ cb200_status cb200_host_stage_create(const cb200_host_stage_options *o, cb200_ho
     s->o = *o;
     cudaError_t err = cudaDeviceGetAttribute(&s->sm_count, cudaDevAttrMultiProcessorCount, o->device);
     const std::uint64_t elem = o->dense_dtype == CB200_DTYPE_BF16 ? 2u : 4u;
-    // the gene-tiled kernel where the shape allows it (its fixed cost per visit needs rows of some length,
-    // which a chunk of a single-cell matrix has); else one warp per row
-    const std::int64_t row_bytes = o->n * static_cast<std::int64_t>(elem);
-    const bool tiled_shape = (o->n == 32 || o->n == 64 || o->n == 128) && row_bytes <= 256;
-    const double mean = static_cast<double>(o->max_chunk_nnz) / static_cast<double>(o->max_chunk_rows);
-    const double per_visit = mean * (98304.0 / static_cast<double>(row_bytes)) / static_cast<double>(o->k);
-    s->schedule = tiled_shape && per_visit >= 6.0 ? fwd_schedule::gene_tiled : fwd_schedule::warp_per_row;
-    s->workspace_bytes = qcsr_tiled_workspace_bytes();
+    s->workspace_bytes = qcsr_gather_workspace_bytes(o->k, o->max_chunk_nnz, o->n, o->dense_dtype);
     for (cudaStream_t *st : {&s->h2d, &s->compute, &s->d2h})
         if (err == cudaSuccess) err = cudaStreamCreateWithFlags(st, cudaStreamNonBlocking);
     if (err == cudaSuccess) err = cudaEventCreateWithFlags(&s->shared_in, cudaEventDisableTiming);
@@ -680,7 +672,7 @@ cb200_status cb200_host_forward(cb200_host_stage *s, const cb200_qcsr *x, const 
         const qcsr_view view{rows, o.k, nnz, o.bits, o.policy, b.row_ptr, o.bits == 4 ? b.packed_row_ptr : nullptr, b.col_idx, b.packed,
                              s->scales, row_policy ? (x->offsets != nullptr ? b.row_offsets : nullptr) : (x->offsets != nullptr ? s->offsets : nullptr)};
         const dense_args d{s->w, o.n, o.dense_dtype, b.y, o.n, o.n, alpha, 0.0f};
-        const cb200_status st = launch_qcsr_forward(view, d, 0, rows, s->schedule, nullptr, nullptr, false, b.workspace, s->workspace_bytes,
+        const cb200_status st = launch_qcsr_forward(view, d, 0, rows, fwd_schedule::warp_per_row, nullptr, nullptr, false, b.workspace, s->workspace_bytes,
                                                     s->sm_count, s->compute);
         if (st != CB200_STATUS_SUCCESS) return st;
         CB200_CUDA_OK(cudaEventRecord(b.computed, s->compute));

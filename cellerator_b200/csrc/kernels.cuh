@@ -89,6 +89,10 @@ cb200_status launch_qcsr_forward_tiled(const qcsr_view &x, const dense_args &d, 
                                        std::int64_t row_end, int *status_word, const std::int32_t *row_order,
                                        int sm_count, cudaStream_t stream, bool *taken);
 
+// What the exact gather kernel can use: the status block and, where N leaves W's rows unaligned, room for W re-laid with rows
+// at a pitch of 16 bytes.  256 bytes are enough to run.
+std::uint64_t qcsr_gather_workspace_bytes(std::int64_t cols, std::int64_t nnz, std::int64_t n, int dense_dtype);
+
 // Tensor-core kernel for bf16 products (decoded values rounded to bf16): entries are scattered
 // into dense operand tiles in shared memory, window by window of 64 genes.  `workspace` holds the
 // status word and W re-laid per window; *taken is false when the shape or workspace rules it out.

@@ -12,6 +12,8 @@
 // the stream into the scratch, ahead of the launch.
 #include "kernels.cuh"
 
+#include <algorithm>
+
 namespace cb200 {
 namespace {
 
@@ -172,7 +174,9 @@ cb200_status route(const cb200_public_layout *l, int32_t projection, const float
     std::uint64_t need = 0;
     std::uint32_t align = 256;
     cb200_prepared_workspace(prepared, &need, &align);
-    // the exact fp32 schedules these calls select need the status block only
+    // the exact fp32 schedules these calls select need the status block only; what a CSR projection could use beyond it is not
+    // in the scratch these calls ask for
+    if (projection == CB200_PROJECTION_CSR) need = std::min<std::uint64_t>(need, 256u);
     void *ws = need == 0u ? nullptr : (need <= 256u ? status_block : cur.take(need));
     if (need != 0u && ws == nullptr) {
         cb200_prepared_destroy(prepared);

@@ -511,7 +511,7 @@ const char *schedule_name(std::uint32_t variant) noexcept {
     // (1M x 33,538 cells x genes at 5.4 % density; 500k x 4,000 at 17 % for the dense and the code tiles; 250k x 8,192 Blocked-ELL).
     double fraction = 0.05;
     switch (variant) {
-    case schedule_warp_per_row: fraction = 0.05; break;
+    case schedule_warp_per_row: fraction = 0.077; break;
     case schedule_gene_tiled: fraction = 0.070; break;
     case schedule_tensor_windows: fraction = 0.062; break;
     case schedule_tensor_blocked:

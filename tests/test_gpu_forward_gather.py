@@ -1,0 +1,65 @@
+"""GPU parity of the exact gather kernels at the edges of how they cut rows into parts, share them out and read W."""
+import numpy as np
+import pytest
+import torch
+
+from cellerator_b200 import capi, ops
+from gpu_util import assert_forward_close, dense, host_pack, row_l1, to_dev
+
+pytestmark = pytest.mark.gpu
+
+# around a segment (64), a part (128), the longest row of 16 parts of 128, and beyond it
+EDGE_LENGTHS = [0, 1, 15, 16, 17, 63, 64, 65, 127, 128, 129, 255, 257, 2047, 2048, 2049, 3500, 0]
+
+
+def matrix(oracle, lengths, cols, bits, policy, seed):
+    rng = np.random.default_rng(seed)
+    row_ptr = np.concatenate([[0], np.cumsum(lengths)]).astype(np.int64)
+    col_idx = np.concatenate([np.sort(rng.choice(cols, size=k, replace=False)) for k in lengths]).astype(np.int32)
+    offsets = rng.uniform(0.0, 1.0, size=cols if policy == 1 else len(lengths)).astype(np.float32)
+    return host_pack(oracle, dict(rows=len(lengths), cols=cols, bits=bits, policy=policy, row_ptr=row_ptr, col_idx=col_idx,
+                                  scales=rng.uniform(0.01, 0.05, size=cols).astype(np.float32), offsets=offsets,
+                                  values=rng.uniform(0.0, 5.0, size=len(col_idx)).astype(np.float32)))
+
+
+def check(oracle, device, c, n, dtype, bias=None):
+    x = to_dev(c, device)
+    w, w_host = dense(np.random.default_rng(n), c["cols"], n, dtype, device)
+    op = ops.PreparedSpmm(capi.PROJECTION_CSR, c["rows"], c["cols"], n, x.nnz, c["bits"], c["policy"], dtype, device)
+    assert op.schedule == "warp_per_row"
+    y = op.run(x, w, torch.full((c["rows"], n), float("nan"), device=device))
+    assert op.status() == 0
+    ref = oracle.qcsr_forward(c["bits"], c["policy"], c["row_ptr"], c["packed_row_ptr"], c["col_idx"], c["packed"], c["scales"],
+                              c["offsets"], w_host, c["cols"])
+    l1, _ = row_l1(oracle, c)
+    assert_forward_close(y.cpu().numpy(), ref, l1, float(np.abs(w_host).max()), bf16=dtype == torch.bfloat16)
+    # a row's sum does not depend on the launch's row range
+    lo, hi = c["rows"] // 5, c["rows"] - 2
+    part = op.run(x, w, torch.full_like(y, -3.0), row_begin=lo, row_end=hi)
+    assert torch.equal(part[lo:hi], y[lo:hi]) and torch.all(part[:lo] == -3.0) and torch.all(part[hi:] == -3.0)
+
+
+@pytest.mark.parametrize("bits,policy", [(8, 1), (4, 2)])
+@pytest.mark.parametrize("n,dtype", [(3, torch.bfloat16), (50, torch.bfloat16), (100, torch.float32), (256, torch.float32),
+                                     (300, torch.bfloat16)])
+def test_row_lengths_around_the_cuts(cuda_device, oracle, bits, policy, n, dtype):
+    check(oracle, cuda_device, matrix(oracle, EDGE_LENGTHS, 4000, bits, policy, 7 * n + bits), n, dtype)
+
+
+@pytest.mark.parametrize("mean,n", [(4, 64), (90, 16), (90, 50)])
+def test_many_rows(cuda_device, oracle, mean, n):
+    """a warp per row (short rows; narrow W) and several rows per CTA, with a last CTA that is not full"""
+    rows = 64 * 160 + 3
+    lengths = np.random.default_rng(mean).integers(0, 2 * mean, size=rows)
+    lengths[77] = 700
+    check(oracle, cuda_device, matrix(oracle, lengths, 900, 8, 1, mean), n, torch.bfloat16)
+
+
+@pytest.mark.parametrize("n,dtype", [(50, torch.bfloat16), (50, torch.float32), (101, torch.bfloat16)])
+def test_w_re_laid_with_aligned_rows(cuda_device, oracle, n, dtype):
+    lengths = np.random.default_rng(1).integers(900, 1300, size=1001)
+    c = matrix(oracle, lengths, 4000, 8, 1, n)
+    assert c["row_ptr"][-1] >= 1 << 20
+    op = ops.PreparedSpmm(capi.PROJECTION_CSR, c["rows"], c["cols"], n, int(c["row_ptr"][-1]), 8, 1, dtype, cuda_device)
+    assert op.workspace_bytes > 256
+    check(oracle, cuda_device, c, n, dtype)
