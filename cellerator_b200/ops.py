@@ -5,6 +5,7 @@ libcellerator_b200.so through `capi`.
 from __future__ import annotations
 
 import ctypes as C
+import struct
 from dataclasses import dataclass, field
 
 import numpy as np
@@ -20,7 +21,23 @@ def _ptr(t):
 
 
 def _stream_handle(device) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+    index = device.index
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index)
+
+
+# One call's cb200_launch as bytes, fields in the order of capi.Launch: packed in one step, a microsecond against the six of
+# setting them one by one.
+_LAUNCH = struct.Struct("@INPPPqPqffQqqPiiPQPiQ")
+assert _LAUNCH.size == C.sizeof(capi.Launch)
+_run_packed = None
+
+
+def _run_entry():
+    """cb200_spmm_run taking the launch as bytes"""
+    global _run_packed
+    if _run_packed is None:
+        _run_packed = C.CFUNCTYPE(C.c_int32, C.c_void_p, C.c_char_p)(("cb200_spmm_run", capi.lib()))
+    return _run_packed
 
 
 # ---- host helpers (no device) ----------------------------------------------------------
@@ -81,6 +98,7 @@ class QuantizedCsr:
     packed_row_ptr: torch.Tensor | None = None   # int64 [rows+1]; None for 8-bit
     host_row_ptr: np.ndarray | None = None
     _desc: capi.QCsr | None = field(default=None, repr=False)
+    _known: tuple | None = field(default=None, repr=False, compare=False)
 
     @property
     def nnz(self) -> int:
@@ -101,6 +119,19 @@ class QuantizedCsr:
         d.offsets = None if self.offsets is None else self.offsets.data_ptr()
         self._desc = d
         return d
+
+    def _bound(self) -> tuple:
+        """(what a descriptor is made from, the descriptor): made anew only when one of the arrays or sizes is another one.
+        A descriptor handed out here is never written again."""
+        prp, scales, offsets = self.packed_row_ptr, self.scales, self.offsets
+        key = (self.rows, self.cols, self.bits, self.policy, self.col_idx.numel(), self.packed.numel(), self.row_ptr.data_ptr(),
+               self.col_idx.data_ptr(), self.packed.data_ptr(), None if prp is None else prp.data_ptr(),
+               None if scales is None else scales.data_ptr(), None if offsets is None else offsets.data_ptr())
+        known = self._known
+        if known is None or known[0] != key:
+            desc = self.desc()
+            known = self._known = (key, desc, C.addressof(desc))
+        return known
 
     @staticmethod
     def from_host(h: dict, device) -> "QuantizedCsr":
@@ -146,6 +177,7 @@ class QuantizedBell:
     scales: torch.Tensor | None
     offsets: torch.Tensor | None
     _desc: capi.QBell | None = field(default=None, repr=False)
+    _known: tuple | None = field(default=None, repr=False, compare=False)
 
     @property
     def device(self):
@@ -161,6 +193,18 @@ class QuantizedBell:
         d.offsets = None if self.offsets is None else self.offsets.data_ptr()
         self._desc = d
         return d
+
+    def _bound(self) -> tuple:
+        """as QuantizedCsr._bound"""
+        scales, offsets = self.scales, self.offsets
+        key = (self.rows, self.cols, self.block_size, self.ell_cols, self.row_stride_bytes, self.bits, self.policy,
+               self.block_col_idx.data_ptr(), self.packed.data_ptr(), None if scales is None else scales.data_ptr(),
+               None if offsets is None else offsets.data_ptr())
+        known = self._known
+        if known is None or known[0] != key:
+            desc = self.desc()
+            known = self._known = (key, desc, C.addressof(desc))
+        return known
 
     @staticmethod
     def from_host(h: dict, device) -> "QuantizedBell":
@@ -240,6 +284,7 @@ class PreparedSpmm:
             pr.persistent, pr.persistent_bytes = persistent.data_ptr(), persistent.numel() * persistent.element_size()
         pr.prepare_stream = prepare_stream
         self.problem = pr
+        self._index = pr.device
         self.handle = C.c_void_p()
         capi.check(capi.lib().cb200_spmm_prepare(C.byref(pr), C.byref(self.handle)))
         nbytes, align = C.c_uint64(), C.c_uint32()
@@ -324,8 +369,25 @@ class PreparedSpmm:
     def run_launch(self, launch: capi.Launch) -> None:
         capi.check(capi.lib().cb200_spmm_run(self.handle, C.byref(launch)))
 
-    def run(self, x, dense, out, **kw) -> torch.Tensor:
-        self.run_launch(self.make_launch(x, dense, out, **kw))
+    def run(self, x, dense: torch.Tensor, out: torch.Tensor, alpha=1.0, beta=0.0, row_begin=0, row_end=capi.ALL_ROWS,
+            stream: int | None = None, epoch: int | None = None, epilogue: str | int = 0, bias: torch.Tensor | None = None,
+            value_generation: int = 0) -> torch.Tensor:
+        """make_launch + run_launch without the descriptor objects in between"""
+        known = x._bound()
+        bell = isinstance(x, QuantizedBell)
+        device, ws, bias_ptr = self._index, self.workspace, None
+        if bias is not None:
+            if bias.dtype != torch.float32 or not bias.is_contiguous() or bias.numel() != self.problem.n:
+                raise ValueError("bias must be a contiguous float32 vector with one value per output column")
+            bias_ptr = bias.data_ptr()
+        launch = _LAUNCH.pack(capi.ABI_VERSION, _LAUNCH.size, 0 if bell else known[2], known[2] if bell else 0, dense.data_ptr(),
+                              dense.stride(0), out.data_ptr(), out.stride(0), alpha, beta, self.epoch if epoch is None else epoch,
+                              row_begin, row_end, (_stream_handle(self.device) if stream is None else stream) or 0, device, device,
+                              0 if ws is None else ws.data_ptr(), self.workspace_bytes, bias_ptr or 0,
+                              capi.EPILOGUE[epilogue] if isinstance(epilogue, str) else int(epilogue), value_generation)
+        status = _run_entry()(self.handle, launch)
+        if status:
+            capi.check(status)
         return out
 
     def close(self):
