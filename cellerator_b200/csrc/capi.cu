@@ -95,6 +95,30 @@ struct cb200_session {
 };
 
 namespace {
+// cudaDeviceGetAttribute answers of a device, asked once (cudaGetDeviceProperties fills dozens of fields
+// and costs milliseconds; the routed public calls prepare on every projection)
+struct device_facts { int major = 0, sm_count = 0; };
+cb200_status facts_of(int device, device_facts *out) {
+    constexpr int kMax = 64;
+    static std::atomic<int> cached_major[kMax], cached_sms[kMax];
+    if (device >= 0 && device < kMax && cached_sms[device].load(std::memory_order_acquire) != 0) {
+        out->major = cached_major[device].load(std::memory_order_relaxed);
+        out->sm_count = cached_sms[device].load(std::memory_order_relaxed);
+        return CB200_STATUS_SUCCESS;
+    }
+    int device_count = 0;
+    CB200_CUDA_OK(cudaGetDeviceCount(&device_count));
+    if (device < 0 || device >= device_count)
+        return fail(CB200_STATUS_INVALID_STREAM, "device %d not present (%d visible)", device, device_count);
+    CB200_CUDA_OK(cudaDeviceGetAttribute(&out->major, cudaDevAttrComputeCapabilityMajor, device));
+    CB200_CUDA_OK(cudaDeviceGetAttribute(&out->sm_count, cudaDevAttrMultiProcessorCount, device));
+    if (device < kMax) {
+        cached_major[device].store(out->major, std::memory_order_relaxed);
+        cached_sms[device].store(out->sm_count, std::memory_order_release);
+    }
+    return CB200_STATUS_SUCCESS;
+}
+
 void account(cb200_allocation_accounting *a, std::uint64_t bytes) {
     a->current_bytes += bytes;
     if (a->current_bytes > a->high_water_bytes) a->high_water_bytes = a->current_bytes;
@@ -190,7 +214,10 @@ cb200_status cb200_quantize_rows(const cb200_qcsr *m, int64_t row_begin, int64_t
     if (!valid_header(m)) return fail(CB200_STATUS_INVALID_ARGUMENT, "bad cb200_qcsr header");
     device_scope scope(device);
     CB200_CUDA_OK(scope.status);
-    return launch_quantize_rows(view_of(*m), row_begin, row_end, values, static_cast<cudaStream_t>(stream));
+    device_facts facts;
+    const cb200_status found = facts_of(device, &facts);
+    if (found != CB200_STATUS_SUCCESS) return found;
+    return launch_quantize_rows(view_of(*m), row_begin, row_end, values, facts.sm_count, static_cast<cudaStream_t>(stream));
 }
 
 cb200_status cb200_dequantize_rows(const cb200_qcsr *m, int64_t row_begin, int64_t row_end, float *values,
@@ -199,7 +226,10 @@ cb200_status cb200_dequantize_rows(const cb200_qcsr *m, int64_t row_begin, int64
     if (!valid_header(m)) return fail(CB200_STATUS_INVALID_ARGUMENT, "bad cb200_qcsr header");
     device_scope scope(device);
     CB200_CUDA_OK(scope.status);
-    return launch_dequantize_rows(view_of(*m), row_begin, row_end, values, static_cast<cudaStream_t>(stream));
+    device_facts facts;
+    const cb200_status found = facts_of(device, &facts);
+    if (found != CB200_STATUS_SUCCESS) return found;
+    return launch_dequantize_rows(view_of(*m), row_begin, row_end, values, facts.sm_count, static_cast<cudaStream_t>(stream));
 }
 
 cb200_status cb200_qbell_quantize_rows(const cb200_qbell *m, int64_t row_begin, int64_t row_end,
@@ -444,30 +474,6 @@ std::uint64_t plan_persistent_bytes(const cb200_spmm_problem &pr, const schedule
     if (plan.codes_wanted) bytes += device_arena::rounded(qcsr_code_tile_bytes(pr.m, pr.k));
     if (plan.row_order) bytes += device_arena::rounded(static_cast<std::uint64_t>(pr.m) * sizeof(std::int32_t));
     return bytes;
-}
-
-// cudaDeviceGetAttribute answers of a device, asked once (cudaGetDeviceProperties fills dozens of fields
-// and costs milliseconds; the routed public calls prepare on every projection)
-struct device_facts { int major = 0, sm_count = 0; };
-cb200_status facts_of(int device, device_facts *out) {
-    constexpr int kMax = 64;
-    static std::atomic<int> cached_major[kMax], cached_sms[kMax];
-    if (device >= 0 && device < kMax && cached_sms[device].load(std::memory_order_acquire) != 0) {
-        out->major = cached_major[device].load(std::memory_order_relaxed);
-        out->sm_count = cached_sms[device].load(std::memory_order_relaxed);
-        return CB200_STATUS_SUCCESS;
-    }
-    int device_count = 0;
-    CB200_CUDA_OK(cudaGetDeviceCount(&device_count));
-    if (device < 0 || device >= device_count)
-        return fail(CB200_STATUS_INVALID_STREAM, "device %d not present (%d visible)", device, device_count);
-    CB200_CUDA_OK(cudaDeviceGetAttribute(&out->major, cudaDevAttrComputeCapabilityMajor, device));
-    CB200_CUDA_OK(cudaDeviceGetAttribute(&out->sm_count, cudaDevAttrMultiProcessorCount, device));
-    if (device < kMax) {
-        cached_major[device].store(out->major, std::memory_order_relaxed);
-        cached_sms[device].store(out->sm_count, std::memory_order_release);
-    }
-    return CB200_STATUS_SUCCESS;
 }
 
 } // namespace

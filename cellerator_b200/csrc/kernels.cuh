@@ -240,9 +240,9 @@ cb200_status launch_qbell_forward(const qbell_view &x, const dense_args &d, std:
 std::uint64_t qbell_tcgen05_workspace_bytes(std::int64_t cols, std::int64_t n);
 
 cb200_status launch_quantize_rows(const qcsr_view &x, std::int64_t row_begin, std::int64_t row_end,
-                                  const float *values, cudaStream_t stream);
+                                  const float *values, int sm_count, cudaStream_t stream);
 cb200_status launch_dequantize_rows(const qcsr_view &x, std::int64_t row_begin, std::int64_t row_end,
-                                    float *values, cudaStream_t stream);
+                                    float *values, int sm_count, cudaStream_t stream);
 
 cb200_status launch_qbell_quantize_rows(const qbell_view &x, std::int64_t row_begin, std::int64_t row_end,
                                         const float *values_by_slot, cudaStream_t stream);

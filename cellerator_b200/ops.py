@@ -155,7 +155,10 @@ class QuantizedCsr:
     def dequantize(self, row_begin=0, row_end=None) -> torch.Tensor:
         row_end = self.rows if row_end is None else row_end
         dev = self.device
-        lo, hi = (int(v) for v in self.row_ptr[[row_begin, row_end]].tolist())
+        if self.host_row_ptr is not None:  # without waiting for the device
+            lo, hi = int(self.host_row_ptr[row_begin]), int(self.host_row_ptr[row_end])
+        else:
+            lo, hi = (int(v) for v in self.row_ptr[[row_begin, row_end]].tolist())
         out = torch.empty(max(hi - lo, 1), dtype=torch.float32, device=dev)
         capi.check(capi.lib().cb200_dequantize_rows(C.byref(self.desc()), row_begin, row_end, out.data_ptr(),
                                                     dev.index, _stream_handle(dev)))

@@ -110,3 +110,33 @@ def test_golden_bell_codec(cuda_device, name):
     ops.quantize_bell_(x, torch.from_numpy(z["values_by_slot"]).to(cuda_device))
     assert np.array_equal(x.packed.cpu().numpy(), z["packed"])          # padding bytes included
     assert np.array_equal(ops.dequantize_bell(x).cpu().numpy(), z["decoded"])
+
+
+@pytest.mark.parametrize("bits", [8, 4])
+@pytest.mark.parametrize("policy,cols", [(1, 3000), (1, 45_000), (2, 21_000)])
+def test_codec_of_a_large_matrix_equals_oracle(cuda_device, oracle, bits, policy, cols):
+    """Sizes at which scales and zero-points go through shared memory, in one and in several ranges of genes; rows of every
+    length from none to many blocks, ties, values and scales out of the ordinary, a row range."""
+    rng = np.random.default_rng(bits + policy + cols)
+    lengths = rng.integers(0, 1900, size=2200)
+    lengths[[5, 6, 900]] = [0, 1, 2999]
+    row_ptr = np.concatenate([[0], np.cumsum(lengths)]).astype(np.int64)
+    col_idx = np.concatenate([np.sort(rng.choice(cols, size=k, replace=False)) for k in lengths]).astype(np.int32)
+    scales = rng.uniform(0.01, 0.5, size=cols).astype(np.float32)
+    scales[::97], scales[1::97], scales[2::97], scales[3::97] = 0.0, 1e-39, 3e38, 0.125
+    offsets = rng.uniform(-1.0, 1.0, size=cols if policy == 1 else len(lengths)).astype(np.float32)
+    offsets[::5] = 0.0
+    values = (rng.integers(-4, 70, size=len(col_idx)) * 0.0625 + rng.choice([0.0, 1e-6, 0.01], size=len(col_idx))).astype(np.float32)
+    values[::1001], values[7::1001], values[11::1001] = 1e9, -1e30, np.nan
+    row_ptr_p, total = oracle.build_packed_row_ptr(bits, row_ptr)
+    expect = oracle.pack_csr(bits, policy, row_ptr, row_ptr_p, col_idx, scales, offsets, values)
+    x = ops.QuantizedCsr.from_host(dict(rows=len(lengths), cols=cols, bits=bits, policy=policy, row_ptr=row_ptr, col_idx=col_idx,
+                                        scales=scales, offsets=offsets, packed_row_ptr=row_ptr_p,
+                                        packed=np.full(total, 0x55, dtype=np.uint8)), cuda_device)
+    assert x.nnz >= 2_000_000
+    x.quantize_(torch.from_numpy(values).to(cuda_device))
+    assert np.array_equal(x.packed.cpu().numpy(), expect)
+    decoded = oracle.unpack_csr(bits, policy, row_ptr, row_ptr_p, col_idx, scales, offsets, expect)
+    assert np.array_equal(x.dequantize().cpu().numpy(), decoded, equal_nan=True)
+    lo, hi = 3, len(lengths) - 2
+    assert np.array_equal(x.dequantize(lo, hi).cpu().numpy(), decoded[row_ptr[lo]:row_ptr[hi]], equal_nan=True)
