@@ -296,6 +296,10 @@ def lib() -> C.CDLL:
         L.cb200_qcsr_gene_major_workspace.argtypes = [C.c_int64, C.c_int64]
         L.cb200_qcsr_gene_major.argtypes = [C.POINTER(QCsr), C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_uint64,
                                             C.c_int32, C.c_void_p]
+        L.cb200_bell_lowering_query.argtypes = [C.POINTER(BellLoweringInput), C.c_uint32, C.POINTER(BellLoweringPolicy), C.c_void_p,
+                                                C.c_uint64, C.c_void_p, C.POINTER(BellGeometry)]
+        L.cb200_bell_lowering_materialize.argtypes = [C.POINTER(BellLoweringInput), C.POINTER(BellGeometry), C.c_int32, C.c_uint64,
+                                                      C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_uint64, C.c_void_p]
         L.cb200_spmm_prepare.argtypes = [C.POINTER(SpmmProblem), C.POINTER(C.c_void_p)]
         L.cb200_prepared_destroy.argtypes = [C.c_void_p]
         L.cb200_prepared_destroy.restype = None

@@ -17,6 +17,12 @@
 // bits is the block row's ELL demand (query); the rank of a bit among the set bits -- a word-level
 // exclusive scan plus a popcount -- is the slot of that block column, ascending as in the reference
 // (materialize), and tells every stored value where it goes.
+//
+// Query and materialize of 249,984 x 8,192 with 76.7 M one-byte codes: 1.04 -> 0.41 ms.  The query checked the CSR with a
+// thread per row (170 us of serial, uncoalesced reads) ahead of the counting pass (298 us of atomics on a few words) and two
+// round trips to the host: now one pass and one round trip (156 us).  The placing pass wrote single bytes over 128 MB of
+// zeroes (488 us and a memset): now a block row is put together in shared memory (254 us).  Both are bound by instruction
+// issue: two look-ups and the arithmetic of a place for every entry, in the placing pass twice.
 #include "kernels.cuh"
 
 #include <algorithm>
@@ -33,14 +39,15 @@ struct lowering_params {
     const unsigned char *values;
     const std::uint32_t *fb_offsets;    // device copy, fb_count + 1
     const std::uint32_t *block_offsets; // physical block column of the first column of every semantic block
-    const std::uint32_t *finv, *rperm;
-    std::uint32_t rows, features, fb_count, value_size, words; // words of the bitmap
+    const std::uint32_t *fperm, *finv, *rperm, *rinv;
+    std::uint32_t rows, features, nnz, fb_count, value_size, words; // words of the bitmap
     std::uint32_t ell_blocks;
     int values_layout;
     unsigned long long row_stride_bytes;
     std::int32_t *column_indices;
     unsigned char *values_out;
-    unsigned int *max_active;
+    std::uint32_t *padded_out;          // fb_count + 1
+    unsigned int *max_active, *flags;
     unsigned long long *occupied;
 };
 
@@ -57,49 +64,167 @@ __device__ __forceinline__ std::uint32_t semantic_block(const lowering_params &p
 // physical block column of an execution feature, and its column within that block
 template<int BS>
 __device__ __forceinline__ std::uint32_t physical_block(const lowering_params &p, std::uint32_t execution, std::uint32_t *local) {
-    const std::uint32_t semantic = p.fb_count == 1u ? 0u : semantic_block(p, execution);
+    if (p.fb_count == 1u) { // no tables
+        *local = execution % BS;
+        return execution / BS;
+    }
+    const std::uint32_t semantic = semantic_block(p, execution);
     const std::uint32_t within = execution - __ldg(p.fb_offsets + semantic);
     *local = within % BS;
     return __ldg(p.block_offsets + semantic) + within / BS;
 }
 
-// Sets, in the shared bitmap, the physical block columns that block row `br` touches.
-template<int BS>
-__device__ __forceinline__ void mark_block_row(const lowering_params &p, std::uint32_t br, unsigned *bitmap) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
-    for (std::uint32_t w = threadIdx.x; w < p.words; w += blockDim.x) bitmap[w] = 0u;
-    __syncthreads();
-    const std::uint32_t begin = br * BS, end = min(p.rows, begin + BS);
-    for (std::uint32_t er = begin + warp; er < end; er += warps) {
-        const std::uint32_t r = __ldg(p.rperm + er);
-        const std::uint32_t lo = __ldg(p.row_offsets + r), hi = __ldg(p.row_offsets + r + 1u);
-        for (std::uint32_t i = lo + lane; i < hi; i += 32u) {
-            std::uint32_t local;
-            const std::uint32_t pb = physical_block<BS>(p, __ldg(p.finv + __ldg(p.feature_ids + i)), &local);
-            atomicOr(bitmap + (pb >> 5), 1u << (pb & 31u));
-        }
+// Shared memory of a block row: which physical block columns it touches, a byte each while the entries are read (plain stores:
+// the lanes of a warp mostly hit the same few columns, which would queue up as atomics), then a bitmap, and, for the placing,
+// the set bits before every word of it.
+struct block_row_marks {
+    unsigned char *seen; // [words * 32]; null: too many block columns, the bitmap is written with atomics
+    unsigned *bitmap;    // [words]
+    // placing only, one of the two:
+    std::uint16_t *slots; // [words * 32] slot of a block column that was seen
+    unsigned *ranks;      // [words] set bits before every word
+};
+constexpr std::uint32_t kMaxSeenWords = 256; // 8 KB of bytes, 16 KB of slots
+
+inline std::size_t marks_bytes(std::uint32_t words, bool placing) {
+    const bool few = words <= kMaxSeenWords;
+    return static_cast<std::size_t>(words) * ((few ? 32u : 0u) + 4u + (placing ? (few ? 64u : 4u) : 0u));
+}
+__device__ __forceinline__ block_row_marks place_marks(unsigned char *at, std::uint32_t words) {
+    const bool few = words <= kMaxSeenWords;
+    block_row_marks m;
+    m.seen = few ? at : nullptr;
+    m.bitmap = reinterpret_cast<unsigned *>(at + (few ? words * 32u : 0u));
+    m.ranks = m.bitmap + words;
+    m.slots = few ? reinterpret_cast<std::uint16_t *>(m.bitmap + words) : nullptr;
+    return m;
+}
+__device__ __forceinline__ std::uint32_t slot_of(const block_row_marks &m, std::uint32_t pb) {
+    if (m.slots != nullptr) return m.slots[pb];
+    return m.ranks[pb >> 5] + __popc(m.bitmap[pb >> 5] & ((1u << (pb & 31u)) - 1u));
+}
+__device__ __forceinline__ void clear_marks(const block_row_marks &m, std::uint32_t words) {
+    if (m.seen != nullptr)
+        for (std::uint32_t w = threadIdx.x; w < words * 8u; w += blockDim.x) reinterpret_cast<unsigned *>(m.seen)[w] = 0u;
+    else
+        for (std::uint32_t w = threadIdx.x; w < words; w += blockDim.x) m.bitmap[w] = 0u;
+}
+__device__ __forceinline__ void mark(const block_row_marks &m, std::uint32_t pb) {
+    if (m.seen != nullptr) m.seen[pb] = 1;
+    else atomicOr(m.bitmap + (pb >> 5), 1u << (pb & 31u));
+}
+__device__ __forceinline__ void gather_marks(const block_row_marks &m, std::uint32_t words) {
+    if (m.seen == nullptr) return;
+    const int lane = threadIdx.x & 31;
+    for (std::uint32_t w = threadIdx.x >> 5; w < words; w += blockDim.x >> 5) {
+        const unsigned bits = __ballot_sync(0xffffffffu, m.seen[w * 32u + lane] != 0);
+        if (lane == 0) m.bitmap[w] = bits;
     }
-    __syncthreads();
 }
 
+constexpr int kLowerSteps = 4; // steps of 32 entries whose loads are in flight together
+
+// The `len` entries from entry `lo` on: a warp walks them in steps of 32 that start at multiples of 32, and hands the feature
+// ids of four steps at a time to `use`, with the place in the row of the first one (lanes outside the row have id 0).
+template<typename F>
+__device__ __forceinline__ void walk_row(const std::uint32_t *feature_ids, std::uint32_t lo, std::uint32_t len, F use) {
+    const std::uint32_t *ids = feature_ids + lo;
+    for (int at = static_cast<int>(threadIdx.x & 31u) - static_cast<int>(lo & 31u), end = static_cast<int>(len) + static_cast<int>(threadIdx.x & 31u); at < end;
+         at += 32 * kLowerSteps) {
+        std::uint32_t id[kLowerSteps];
+#pragma unroll
+        for (int u = 0; u < kLowerSteps; ++u) {
+            id[u] = 0u;
+            if (static_cast<unsigned>(at + u * 32) < len) id[u] = __ldg(ids + at + u * 32);
+        }
+        use(at, id);
+    }
+}
+
+// One pass for the query: checks the input (flags: 1 = feature maps are not inverses, 2 = row maps are not inverses, 4 = CSR
+// invalid; nothing is read out of range whatever the arrays hold) and counts the block columns every block row touches.  The
+// block rows cover every canonical row exactly when the row maps are inverses of each other, so a flag of higher rank is
+// never missed.
 template<int BS>
 __global__ void __launch_bounds__(kLowerThreads) lowering_count_kernel(const lowering_params p) {
-    extern __shared__ unsigned lowering_smem[];
+    extern __shared__ __align__(16) unsigned char lowering_smem[];
     __shared__ unsigned warp_sums[kLowerThreads / 32];
-    mark_block_row<BS>(p, blockIdx.x, lowering_smem);
-    unsigned active = 0u;
-    for (std::uint32_t w = threadIdx.x; w < p.words; w += blockDim.x) active += __popc(lowering_smem[w]);
+    __shared__ std::uint32_t row_lo[BS], row_len[BS];
+    const block_row_marks marks = place_marks(lowering_smem, p.words);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const std::uint32_t begin = blockIdx.x * BS;
+    unsigned bad = 0u;
+    clear_marks(marks, p.words);
+    if (threadIdx.x < BS) {
+        const std::uint32_t er = begin + threadIdx.x;
+        std::uint32_t lo = 0u, hi = 0u;
+        if (er < p.rows && er >= begin) {
+            const std::uint32_t r = __ldg(p.rperm + er);
+            if (r >= p.rows || __ldg(p.rinv + r) != er) bad |= 2u; // in range and rinv o rperm = id: rperm is a bijection
+            if (r < p.rows) {
+                lo = __ldg(p.row_offsets + r);
+                hi = __ldg(p.row_offsets + r + 1u);
+                if (lo > hi || hi > p.nnz) {
+                    bad |= 4u;
+                    lo = hi = 0u;
+                }
+            }
+        }
+        row_lo[threadIdx.x] = lo;
+        row_len[threadIdx.x] = hi - lo;
+    }
+    for (std::uint64_t e = static_cast<std::uint64_t>(blockIdx.x) * kLowerThreads + threadIdx.x; e < p.features; e += static_cast<std::uint64_t>(gridDim.x) * kLowerThreads) {
+        const std::uint32_t c = __ldg(p.fperm + e);
+        if (c >= p.features || __ldg(p.finv + c) != e) bad |= 1u;
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0 && (__ldg(p.row_offsets) != 0u || __ldg(p.row_offsets + p.rows) != p.nnz)) bad |= 4u;
+    __syncthreads();
+    for (int r = warp; r < BS; r += kLowerThreads / 32) {
+        const std::uint32_t len = row_len[r];
+        std::uint32_t before = 0u; // id in front of the step's first entry
+        walk_row(p.feature_ids, row_lo[r], len, [&](int at, const std::uint32_t (&id)[kLowerSteps]) {
+            std::uint32_t execution[kLowerSteps];
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) active += __shfl_xor_sync(0xffffffffu, active, off);
-    if ((threadIdx.x & 31) == 0) warp_sums[threadIdx.x >> 5] = active;
+            for (int u = 0; u < kLowerSteps; ++u) execution[u] = __ldg(p.finv + min(id[u], p.features - 1u));
+#pragma unroll
+            for (int u = 0; u < kLowerSteps; ++u) {
+                std::uint32_t last = __shfl_up_sync(0xffffffffu, id[u], 1);
+                if (lane == 0) last = before;
+                before = __shfl_sync(0xffffffffu, id[u], 31);
+                const bool there = static_cast<unsigned>(at + u * 32) < len, wild = id[u] >= p.features;
+                if (there && (wild || (at + u * 32 > 0 && id[u] <= last))) bad |= 4u;
+                std::uint32_t local;
+                // (an execution feature out of range: the maps are not inverses, flagged above)
+                if (there && !wild && execution[u] < p.features) mark(marks, physical_block<BS>(p, execution[u], &local));
+            }
+        });
+    }
+    __syncthreads();
+    gather_marks(marks, p.words);
+    __syncthreads();
+    unsigned active = 0u;
+    for (std::uint32_t w = threadIdx.x; w < p.words; w += blockDim.x) active += __popc(marks.bitmap[w]);
+    active = __reduce_add_sync(0xffffffffu, active);
+    bad = __reduce_or_sync(0xffffffffu, bad);
+    if (lane == 0) {
+        warp_sums[warp] = active;
+        if (bad != 0u) atomicOr(p.flags, bad);
+    }
     __syncthreads();
     if (threadIdx.x == 0) {
         unsigned total = 0u;
         for (int w = 0; w < kLowerThreads / 32; ++w) total += warp_sums[w];
-        atomicMax(p.max_active, total);
-        atomicAdd(p.occupied, static_cast<unsigned long long>(total));
+        if (total != 0u) {
+            atomicMax(p.max_active, total);
+            atomicAdd(p.occupied, static_cast<unsigned long long>(total));
+        }
     }
 }
+
+template<int VS> struct lowered_value { using type = unsigned char; };
+template<> struct lowered_value<2> { using type = unsigned short; };
+template<> struct lowered_value<4> { using type = unsigned; };
+template<> struct lowered_value<8> { using type = uint2; };
 
 template<int VS>
 __device__ __forceinline__ void copy_value(unsigned char *dst, const unsigned char *src, std::uint32_t value_size) {
@@ -111,89 +236,135 @@ __device__ __forceinline__ void copy_value(unsigned char *dst, const unsigned ch
         for (std::uint32_t b = 0; b < value_size; ++b) dst[b] = src[b];
 }
 
-template<int BS, int VS>
+// Places a block row.  TILE: the block row's values are put together in shared memory, zeros included, and written out as
+// whole 16-byte pieces; else (large tiles, odd value sizes, unaligned outputs) they are scattered over the zeroed output.
+template<int BS, int VS, bool TILE>
 __global__ void __launch_bounds__(kLowerThreads) lowering_fill_kernel(const lowering_params p) {
-    extern __shared__ unsigned lowering_smem[];
-    __shared__ unsigned chunk_sums[kLowerThreads];
-    unsigned *bitmap = lowering_smem, *ranks = lowering_smem + p.words; // ranks[w]: set bits in words before w
-    const std::uint32_t br = blockIdx.x;
-    mark_block_row<BS>(p, br, bitmap);
-    // exclusive scan of the words' popcounts: every thread owns a contiguous run of words
-    const std::uint32_t per = (p.words + blockDim.x - 1u) / blockDim.x;
-    const std::uint32_t w0 = min(p.words, per * threadIdx.x), w1 = min(p.words, w0 + per);
-    unsigned sum = 0u;
-    for (std::uint32_t w = w0; w < w1; ++w) sum += __popc(bitmap[w]);
-    chunk_sums[threadIdx.x] = sum;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        unsigned run = 0u;
-        for (int t = 0; t < kLowerThreads; ++t) {
-            const unsigned v = chunk_sums[t];
-            chunk_sums[t] = run;
-            run += v;
+    extern __shared__ __align__(16) unsigned char lowering_smem[];
+    __shared__ unsigned warp_sums[kLowerThreads / 32];
+    __shared__ std::uint32_t row_lo[BS], row_len[BS];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const std::uint32_t br = blockIdx.x, begin = br * BS;
+    const std::uint32_t value_size = VS != 0 ? VS : p.value_size, row_bytes = p.ell_blocks * BS * value_size; // a row, all slots
+    const std::uint32_t tile_bytes = row_bytes * BS;
+    unsigned char *tile = lowering_smem;
+    const block_row_marks marks = place_marks(lowering_smem + (TILE ? tile_bytes : 0u), p.words);
+    if (br == 0u) // the padded offsets of the semantic blocks
+        for (std::uint32_t b = threadIdx.x; b <= p.fb_count; b += kLowerThreads)
+            p.padded_out[b] = (b == 0u ? 0u : p.fb_count == 1u ? (p.features + BS - 1u) / BS : __ldg(p.block_offsets + b)) * BS;
+    clear_marks(marks, p.words);
+    if constexpr (TILE)
+        for (std::uint32_t i = threadIdx.x; i < tile_bytes / 16u; i += kLowerThreads) reinterpret_cast<uint4 *>(tile)[i] = make_uint4(0u, 0u, 0u, 0u);
+    if (threadIdx.x < BS) {
+        const std::uint32_t er = begin + threadIdx.x;
+        std::uint32_t lo = 0u, hi = 0u;
+        if (er < p.rows) {
+            const std::uint32_t r = __ldg(p.rperm + er);
+            lo = __ldg(p.row_offsets + r);
+            hi = __ldg(p.row_offsets + r + 1u);
         }
+        row_lo[threadIdx.x] = lo;
+        row_len[threadIdx.x] = hi - lo;
     }
     __syncthreads();
-    unsigned at = chunk_sums[threadIdx.x];
+    for (int r = warp; r < BS; r += kLowerThreads / 32)
+        walk_row(p.feature_ids, row_lo[r], row_len[r], [&](int at, const std::uint32_t (&id)[kLowerSteps]) {
+            std::uint32_t execution[kLowerSteps];
+#pragma unroll
+            for (int u = 0; u < kLowerSteps; ++u) execution[u] = __ldg(p.finv + id[u]);
+#pragma unroll
+            for (int u = 0; u < kLowerSteps; ++u) {
+                std::uint32_t local;
+                if (static_cast<unsigned>(at + u * 32) < row_len[r]) mark(marks, physical_block<BS>(p, execution[u], &local));
+            }
+        });
+    __syncthreads();
+    gather_marks(marks, p.words);
+    __syncthreads();
+    // set bits before every word: every thread owns a contiguous run of words
+    const std::uint32_t per = (p.words + kLowerThreads - 1u) / kLowerThreads;
+    const std::uint32_t w0 = min(p.words, per * threadIdx.x), w1 = min(p.words, w0 + per);
+    unsigned own = 0u;
+    for (std::uint32_t w = w0; w < w1; ++w) own += __popc(marks.bitmap[w]);
+    unsigned upto = own;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+        const unsigned below = __shfl_up_sync(0xffffffffu, upto, off);
+        if (lane >= off) upto += below;
+    }
+    if (lane == 31) warp_sums[warp] = upto;
+    __syncthreads();
+    unsigned at = upto - own, all = 0u;
+    for (int w = 0; w < kLowerThreads / 32; ++w) {
+        if (w < warp) at += warp_sums[w];
+        all += warp_sums[w];
+    }
+    std::int32_t *columns = p.column_indices + static_cast<std::size_t>(br) * p.ell_blocks;
     for (std::uint32_t w = w0; w < w1; ++w) {
-        ranks[w] = at;
-        unsigned bits = bitmap[w];
+        if (marks.slots == nullptr) marks.ranks[w] = at;
+        unsigned bits = marks.bitmap[w];
         while (bits != 0u) { // slots in ascending physical block column
             const int b = __ffs(static_cast<int>(bits)) - 1;
             bits &= bits - 1u;
-            if (at < p.ell_blocks) p.column_indices[static_cast<std::size_t>(br) * p.ell_blocks + at] = static_cast<std::int32_t>(w * 32u + b);
+            if (at < p.ell_blocks) columns[at] = static_cast<std::int32_t>(w * 32u + b);
+            if (marks.slots != nullptr) marks.slots[w * 32u + b] = static_cast<std::uint16_t>(min(at, 0xffffu));
             ++at;
         }
     }
+    for (std::uint32_t s = all + threadIdx.x; s < p.ell_blocks; s += kLowerThreads) columns[s] = -1; // empty
     __syncthreads();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
-    const std::uint32_t begin = br * BS, end = min(p.rows, begin + BS);
-    for (std::uint32_t er = begin + warp; er < end; er += warps) {
-        const std::uint32_t r = __ldg(p.rperm + er);
-        const std::uint32_t lo = __ldg(p.row_offsets + r), hi = __ldg(p.row_offsets + r + 1u);
-        for (std::uint32_t i = lo + lane; i < hi; i += 32u) {
-            std::uint32_t local;
-            const std::uint32_t pb = physical_block<BS>(p, __ldg(p.finv + __ldg(p.feature_ids + i)), &local);
-            const unsigned long long slot = ranks[pb >> 5] + __popc(bitmap[pb >> 5] & ((1u << (pb & 31u)) - 1u));
-            if (slot >= p.ell_blocks) continue; // a stale geometry: never write outside the buffers
-            const unsigned long long at_byte =
-                p.values_layout == 1
-                    ? static_cast<unsigned long long>(er) * p.row_stride_bytes + (slot * BS + local) * p.value_size
-                    : ((static_cast<unsigned long long>(br) * p.ell_blocks + slot) * BS * BS +
-                       static_cast<unsigned long long>(er - begin) * BS + local) * p.value_size;
-            copy_value<VS>(p.values_out + at_byte, p.values + static_cast<unsigned long long>(i) * p.value_size, p.value_size);
+    for (int r = warp; r < BS; r += kLowerThreads / 32)
+        walk_row(p.feature_ids, row_lo[r], row_len[r], [&](int at, const std::uint32_t (&id)[kLowerSteps]) {
+            const std::uint32_t len = row_len[r];
+            const unsigned char *src = p.values + (static_cast<long long>(row_lo[r]) + at) * static_cast<int>(value_size);
+            typename lowered_value<TILE ? VS : 0>::type value[kLowerSteps];
+            std::uint32_t execution[kLowerSteps];
+#pragma unroll
+            for (int u = 0; u < kLowerSteps; ++u) {
+                execution[u] = __ldg(p.finv + id[u]);
+                if constexpr (TILE)
+                    if (static_cast<unsigned>(at + u * 32) < len) value[u] = *reinterpret_cast<const typename lowered_value<VS>::type *>(src + u * 32 * VS);
+            }
+#pragma unroll
+            for (int u = 0; u < kLowerSteps; ++u) {
+                if (static_cast<unsigned>(at + u * 32) >= len) continue;
+                std::uint32_t local;
+                const std::uint32_t slot = slot_of(marks, physical_block<BS>(p, execution[u], &local));
+                if (slot >= p.ell_blocks) continue; // a stale geometry: never write outside the buffers
+                if constexpr (TILE) {
+                    const std::uint32_t cell = p.values_layout == 1 ? r * p.ell_blocks * BS + slot * BS + local : (slot * BS + r) * BS + local;
+                    reinterpret_cast<typename lowered_value<VS>::type *>(tile)[cell] = value[u];
+                } else {
+                    const unsigned long long at_byte =
+                        p.values_layout == 1
+                            ? static_cast<unsigned long long>(begin + r) * p.row_stride_bytes + static_cast<unsigned long long>(slot * BS + local) * p.value_size
+                            : ((static_cast<unsigned long long>(br) * p.ell_blocks + slot) * BS * BS + static_cast<unsigned long long>(r) * BS + local) * p.value_size;
+                    copy_value<VS>(p.values_out + at_byte, src + u * 32 * static_cast<int>(value_size), p.value_size);
+                }
+            }
+        });
+    if constexpr (TILE) {
+        __syncthreads();
+        if (p.values_layout == 1) { // rows of the padded stride, the padding written too
+            const std::uint32_t pieces = static_cast<std::uint32_t>(p.row_stride_bytes / 16u), used = row_bytes / 16u;
+            for (std::uint32_t i = threadIdx.x; i < pieces * BS; i += kLowerThreads) {
+                const std::uint32_t r = i / pieces, c = i - r * pieces;
+                uint4 *out = reinterpret_cast<uint4 *>(p.values_out + static_cast<unsigned long long>(begin + r) * p.row_stride_bytes);
+                out[c] = c < used ? reinterpret_cast<const uint4 *>(tile)[r * used + c] : make_uint4(0u, 0u, 0u, 0u);
+            }
+        } else {
+            uint4 *out = reinterpret_cast<uint4 *>(p.values_out + static_cast<unsigned long long>(br) * tile_bytes);
+            for (std::uint32_t i = threadIdx.x; i < tile_bytes / 16u; i += kLowerThreads) out[i] = reinterpret_cast<const uint4 *>(tile)[i];
         }
     }
 }
 
-// flags: 1 = feature maps are not inverses, 2 = row maps are not inverses, 4 = CSR invalid
-__global__ void __launch_bounds__(256) lowering_validate_kernel(const std::uint32_t *row_offsets, const std::uint32_t *feature_ids,
-                                                                const std::uint32_t *fperm, const std::uint32_t *finv,
-                                                                const std::uint32_t *rperm, const std::uint32_t *rinv,
-                                                                std::uint32_t rows, std::uint32_t features, std::uint32_t nnz,
-                                                                unsigned *flags) {
-    const std::uint32_t stride = gridDim.x * blockDim.x, first = blockIdx.x * blockDim.x + threadIdx.x;
-    unsigned bad = 0u;
-    for (std::uint32_t e = first; e < features; e += stride) {
-        const std::uint32_t c = fperm[e];
-        if (c >= features || finv[c] != e) bad |= 1u; // in range and finv o fperm = id: fperm is a bijection
-    }
-    for (std::uint32_t e = first; e < rows; e += stride) {
-        const std::uint32_t c = rperm[e];
-        if (c >= rows || rinv[c] != e) bad |= 2u;
-    }
-    if (first == 0u && (row_offsets[0] != 0u || row_offsets[rows] != nnz)) bad |= 4u;
-    for (std::uint32_t r = first; r < rows; r += stride) {
-        const std::uint32_t lo = row_offsets[r], hi = row_offsets[r + 1u];
-        if (lo > hi || hi > nnz) {
-            bad |= 4u;
-            continue;
-        }
-        for (std::uint32_t i = lo; i < hi; ++i)
-            if (feature_ids[i] >= features || (i != lo && feature_ids[i] <= feature_ids[i - 1u])) bad |= 4u;
-    }
-    if (bad != 0u) atomicOr(flags, bad);
-}
+// The words a query reads back, as stage() lays them out in the workspace.
+struct query_answer {
+    unsigned maximum, unused;
+    unsigned long long occupied;
+    unsigned flags, unused2;
+};
 
 struct host_plan {
     std::vector<std::uint32_t> block_offsets; // fb_count + 1
@@ -253,42 +424,62 @@ cb200_status stage(const cb200_bell_lowering_input &in, std::uint32_t bs, const 
     std::uint32_t *d_fb = reinterpret_cast<std::uint32_t *>(base + 256), *d_bo = reinterpret_cast<std::uint32_t *>(base + 256 + table);
     const std::size_t bytes = (static_cast<std::size_t>(in.feature_block_count) + 1u) * 4u;
     CB200_CUDA_OK(cudaMemsetAsync(base, 0, 256, stream));
-    CB200_CUDA_OK(cudaMemcpyAsync(d_fb, in.feature_block_offsets, bytes, cudaMemcpyHostToDevice, stream));
-    CB200_CUDA_OK(cudaMemcpyAsync(d_bo, plan.block_offsets.data(), bytes, cudaMemcpyHostToDevice, stream));
+    if (in.feature_block_count > 1u) { // a single semantic block needs no tables
+        CB200_CUDA_OK(cudaMemcpyAsync(d_fb, in.feature_block_offsets, bytes, cudaMemcpyHostToDevice, stream));
+        CB200_CUDA_OK(cudaMemcpyAsync(d_bo, plan.block_offsets.data(), bytes, cudaMemcpyHostToDevice, stream));
+    }
     *p = lowering_params{};
     p->row_offsets = in.row_offsets; p->feature_ids = in.feature_ids; p->values = static_cast<const unsigned char *>(in.values);
-    p->fb_offsets = d_fb; p->block_offsets = d_bo; p->finv = in.inverse_feature_permutation; p->rperm = in.row_permutation;
+    p->fb_offsets = d_fb; p->block_offsets = d_bo; p->fperm = in.feature_permutation; p->finv = in.inverse_feature_permutation;
+    p->rperm = in.row_permutation; p->rinv = in.inverse_row_permutation; p->nnz = in.nnz;
     p->rows = in.rows; p->features = in.features; p->fb_count = in.feature_block_count; p->value_size = in.value_size_bytes;
     p->words = static_cast<std::uint32_t>(words);
     p->max_active = reinterpret_cast<unsigned int *>(base);
     p->occupied = reinterpret_cast<unsigned long long *>(base + 8);
+    p->flags = reinterpret_cast<unsigned *>(base + 16);
     (void)bs;
     return CB200_STATUS_SUCCESS;
 }
 
-template<int BS, int VS>
+template<int BS, int VS, bool TILE>
 cb200_status launch_fill(const lowering_params &p, unsigned grid, std::size_t smem, cudaStream_t stream) {
     if (smem > 48u * 1024u)
-        CB200_CUDA_OK(cudaFuncSetAttribute(lowering_fill_kernel<BS, VS>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-    lowering_fill_kernel<BS, VS><<<grid, kLowerThreads, smem, stream>>>(p);
+        CB200_CUDA_OK(cudaFuncSetAttribute(lowering_fill_kernel<BS, VS, TILE>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+    lowering_fill_kernel<BS, VS, TILE><<<grid, kLowerThreads, smem, stream>>>(p);
     count_launch();
     CB200_CUDA_OK(cudaGetLastError());
     return CB200_STATUS_SUCCESS;
 }
 
-// Typed copies need both arrays aligned to the value size; anything else is copied byte by byte.
+// The tile of a block row fits shared memory beside a second CTA's up to 96 KB (configuration 5: 16 KB) and needs outputs that
+// take 16-byte pieces.  Otherwise the values are scattered: typed copies where both arrays are aligned to the value size,
+// anything else byte by byte, over an output that has been cleared.
+constexpr std::uint64_t kMaxTileBytes = 96u * 1024u;
+
 template<int BS>
-cb200_status launch_fill_vs(const lowering_params &p, unsigned grid, std::size_t smem, cudaStream_t stream) {
+cb200_status launch_fill_vs(const lowering_params &p, unsigned grid, std::uint64_t value_bytes, cudaStream_t stream) {
     const std::uintptr_t vs = p.value_size;
-    const bool aligned = reinterpret_cast<std::uintptr_t>(p.values) % vs == 0u && reinterpret_cast<std::uintptr_t>(p.values_out) % vs == 0u &&
-                         (p.values_layout != 1 || p.row_stride_bytes % vs == 0u);
-    if (!aligned) return launch_fill<BS, 0>(p, grid, smem, stream);
-    switch (p.value_size) {
-    case 1: return launch_fill<BS, 1>(p, grid, smem, stream);
-    case 2: return launch_fill<BS, 2>(p, grid, smem, stream);
-    case 4: return launch_fill<BS, 4>(p, grid, smem, stream);
-    case 8: return launch_fill<BS, 8>(p, grid, smem, stream);
-    default: return launch_fill<BS, 0>(p, grid, smem, stream);
+    const std::size_t marks = marks_bytes(p.words, true);
+    const std::uint64_t row_bytes = static_cast<std::uint64_t>(p.ell_blocks) * BS * vs, tile_bytes = row_bytes * BS;
+    const bool typed = reinterpret_cast<std::uintptr_t>(p.values) % vs == 0u && (vs == 1u || vs == 2u || vs == 4u || vs == 8u);
+    if (typed && tile_bytes <= kMaxTileBytes && tile_bytes + marks <= 200u * 1024u && reinterpret_cast<std::uintptr_t>(p.values_out) % 16u == 0u &&
+        (p.values_layout != 1 || (row_bytes % 16u == 0u && p.row_stride_bytes % 16u == 0u && p.row_stride_bytes < (1ull << 28)))) {
+        const std::size_t smem = static_cast<std::size_t>(tile_bytes) + marks;
+        switch (p.value_size) {
+        case 1: return launch_fill<BS, 1, true>(p, grid, smem, stream);
+        case 2: return launch_fill<BS, 2, true>(p, grid, smem, stream);
+        case 4: return launch_fill<BS, 4, true>(p, grid, smem, stream);
+        default: return launch_fill<BS, 8, true>(p, grid, smem, stream);
+        }
+    }
+    CB200_CUDA_OK(cudaMemsetAsync(p.values_out, 0, value_bytes, stream));
+    const bool aligned = typed && reinterpret_cast<std::uintptr_t>(p.values_out) % vs == 0u && (p.values_layout != 1 || p.row_stride_bytes % vs == 0u);
+    switch (aligned ? p.value_size : 0u) {
+    case 1: return launch_fill<BS, 1, false>(p, grid, marks, stream);
+    case 2: return launch_fill<BS, 2, false>(p, grid, marks, stream);
+    case 4: return launch_fill<BS, 4, false>(p, grid, marks, stream);
+    case 8: return launch_fill<BS, 8, false>(p, grid, marks, stream);
+    default: return launch_fill<BS, 0, false>(p, grid, marks, stream);
     }
 }
 
@@ -348,33 +539,19 @@ extern "C" cb200_status cb200_bell_lowering_query(const cb200_bell_lowering_inpu
     lowering_params p;
     st = stage(*in, block_size, plan, workspace, workspace_bytes, stream, &p);
     if (st != CB200_STATUS_SUCCESS) return st;
-    unsigned *flags = reinterpret_cast<unsigned *>(static_cast<unsigned char *>(workspace) + 16);
-    const unsigned vgrid = static_cast<unsigned>(std::min<std::uint64_t>(
-        (std::max<std::uint64_t>(in->rows, in->features) + 255u) / 256u + 1u, 4096u));
-    lowering_validate_kernel<<<vgrid, 256, 0, stream>>>(in->row_offsets, in->feature_ids, in->feature_permutation,
-                                                        in->inverse_feature_permutation, in->row_permutation,
-                                                        in->inverse_row_permutation, in->rows, in->features, in->nnz, flags);
-    count_launch();
-    CB200_CUDA_OK(cudaGetLastError());
-    unsigned host_flags = 0u;
-    CB200_CUDA_OK(cudaMemcpyAsync(&host_flags, flags, sizeof host_flags, cudaMemcpyDeviceToHost, stream));
+    const std::size_t smem = marks_bytes(p.words, false);
+    const unsigned grid = static_cast<unsigned>(std::max<std::uint64_t>(block_rows, 1u)); // an empty matrix's maps are checked too
+    st = block_size == 8u ? launch_count<8>(p, grid, smem, stream)
+                          : (block_size == 16u ? launch_count<16>(p, grid, smem, stream) : launch_count<32>(p, grid, smem, stream));
+    if (st != CB200_STATUS_SUCCESS) return st;
+    query_answer answer{};
+    CB200_CUDA_OK(cudaMemcpyAsync(&answer, workspace, sizeof answer, cudaMemcpyDeviceToHost, stream));
     CB200_CUDA_OK(cudaStreamSynchronize(stream));
-    if (host_flags & 1u) return fail(CB200_STATUS_INVALID_ARGUMENT, "incompatible plan: feature maps are not inverses");
-    if (host_flags & 2u) return fail(CB200_STATUS_INVALID_ARGUMENT, "incompatible order: row maps are not inverses");
-    if (host_flags & 4u) return fail(CB200_STATUS_INVALID_ARGUMENT, "invalid source: CSR offsets or features are not sorted and in range");
-
-    if (block_rows > 0u) {
-        const std::size_t smem = static_cast<std::size_t>(p.words) * 4u;
-        const unsigned grid = static_cast<unsigned>(block_rows);
-        st = block_size == 8u ? launch_count<8>(p, grid, smem, stream)
-                              : (block_size == 16u ? launch_count<16>(p, grid, smem, stream) : launch_count<32>(p, grid, smem, stream));
-        if (st != CB200_STATUS_SUCCESS) return st;
-    }
-    unsigned maximum = 0u;
-    unsigned long long occupied = 0u;
-    CB200_CUDA_OK(cudaMemcpyAsync(&maximum, p.max_active, sizeof maximum, cudaMemcpyDeviceToHost, stream));
-    CB200_CUDA_OK(cudaMemcpyAsync(&occupied, p.occupied, sizeof occupied, cudaMemcpyDeviceToHost, stream));
-    CB200_CUDA_OK(cudaStreamSynchronize(stream));
+    if (answer.flags & 1u) return fail(CB200_STATUS_INVALID_ARGUMENT, "incompatible plan: feature maps are not inverses");
+    if (answer.flags & 2u) return fail(CB200_STATUS_INVALID_ARGUMENT, "incompatible order: row maps are not inverses");
+    if (answer.flags & 4u) return fail(CB200_STATUS_INVALID_ARGUMENT, "invalid source: CSR offsets or features are not sorted and in range");
+    const unsigned maximum = answer.maximum;
+    const unsigned long long occupied = answer.occupied;
 
     // physical_bell_candidates.cc:167-207
     const std::uint64_t stored = block_rows * maximum;
@@ -441,25 +618,25 @@ extern "C" cb200_status cb200_bell_lowering_materialize(const cb200_bell_lowerin
     lowering_params p;
     st = stage(*in, bs, plan, workspace, workspace_bytes, stream, &p);
     if (st != CB200_STATUS_SUCCESS) return st;
-    std::vector<std::uint32_t> padded(plan.block_offsets.size());
-    for (std::size_t b = 0; b < padded.size(); ++b) padded[b] = plan.block_offsets[b] * bs;
-    CB200_CUDA_OK(cudaMemcpyAsync(padded_feature_block_offsets, padded.data(), padded.size() * 4u, cudaMemcpyHostToDevice, stream));
     const std::uint64_t value_bytes = values_layout == CB200_BELL_VALUES_ROW_MAJOR
                                           ? static_cast<std::uint64_t>(geometry->padded_rows) * row_stride_bytes
                                           : geometry->value_bytes;
-    if (geometry->column_index_count != 0u)
-        CB200_CUDA_OK(cudaMemsetAsync(column_indices, 0xff, geometry->column_index_count * sizeof(std::int32_t), stream)); // -1 = empty
-    if (value_bytes != 0u) CB200_CUDA_OK(cudaMemsetAsync(values, 0, value_bytes, stream));
-    if (block_rows == 0u || geometry->ell_blocks_per_row == 0u) return CB200_STATUS_SUCCESS;
+    if (block_rows == 0u || geometry->ell_blocks_per_row == 0u) {
+        std::vector<std::uint32_t> padded(plan.block_offsets.size());
+        for (std::size_t b = 0; b < padded.size(); ++b) padded[b] = plan.block_offsets[b] * bs;
+        CB200_CUDA_OK(cudaMemcpyAsync(padded_feature_block_offsets, padded.data(), padded.size() * 4u, cudaMemcpyHostToDevice, stream));
+        if (value_bytes != 0u) CB200_CUDA_OK(cudaMemsetAsync(values, 0, value_bytes, stream));
+        return CB200_STATUS_SUCCESS;
+    }
     p.ell_blocks = geometry->ell_blocks_per_row;
     p.values_layout = values_layout;
     p.row_stride_bytes = row_stride_bytes;
     p.column_indices = column_indices;
+    p.padded_out = padded_feature_block_offsets;
     p.values_out = static_cast<unsigned char *>(values);
-    const std::size_t smem = static_cast<std::size_t>(p.words) * 8u;
     const unsigned grid = static_cast<unsigned>(block_rows);
-    return bs == 8u ? launch_fill_vs<8>(p, grid, smem, stream)
-                    : (bs == 16u ? launch_fill_vs<16>(p, grid, smem, stream) : launch_fill_vs<32>(p, grid, smem, stream));
+    return bs == 8u ? launch_fill_vs<8>(p, grid, value_bytes, stream)
+                    : (bs == 16u ? launch_fill_vs<16>(p, grid, value_bytes, stream) : launch_fill_vs<32>(p, grid, value_bytes, stream));
 }
 
 // ---------------------------------------------------------------------------------------------

@@ -485,7 +485,7 @@ class BellLowering:
         inp.feature_permutation, inp.inverse_feature_permutation = self.fperm.data_ptr(), self.finv.data_ptr()
         inp.row_permutation, inp.inverse_row_permutation = self.rperm.data_ptr(), self.rinv.data_ptr()
         inp.device = self.device.index if self.device.index is not None else torch.cuda.current_device()
-        self.input = inp
+        self.input, self._input_ref = inp, C.byref(inp)
         need = C.c_uint64()
         capi.check(capi.lib().cb200_bell_lowering_workspace(C.byref(inp), C.byref(need)))
         self.workspace = torch.empty(need.value, dtype=torch.uint8, device=self.device)
@@ -494,23 +494,19 @@ class BellLowering:
               max_persistent=2 ** 63) -> capi.BellGeometry:
         policy = capi.BellLoweringPolicy(max_value_expansion, max_storage_expansion, max_persistent)
         geo = capi.BellGeometry()
-        capi.check(capi.lib().cb200_bell_lowering_query(C.byref(self.input), C.c_uint32(block_size), C.byref(policy),
-                                                        C.c_void_p(self.workspace.data_ptr()),
-                                                        C.c_uint64(self.workspace.numel()),
-                                                        C.c_void_p(_stream_handle(self.device)), C.byref(geo)))
+        capi.check(capi.lib().cb200_bell_lowering_query(self._input_ref, block_size, C.byref(policy), self.workspace.data_ptr(),
+                                                        self.workspace.numel(), _stream_handle(self.device), C.byref(geo)))
         return geo
 
     def materialize(self, geo: capi.BellGeometry, layout=capi.BELL_VALUES_BLOCK_MAJOR, row_stride_bytes=0):
         """-> (padded feature-block offsets int32[blocks + 1], column indices int32, value bytes uint8)"""
+        nbytes = geo.padded_rows * row_stride_bytes if layout == capi.BELL_VALUES_ROW_MAJOR else geo.value_bytes
         pfo = torch.empty(len(self._fb), dtype=torch.int32, device=self.device)
         cols = torch.empty(geo.column_index_count, dtype=torch.int32, device=self.device)
-        nbytes = geo.padded_rows * row_stride_bytes if layout == capi.BELL_VALUES_ROW_MAJOR else geo.value_bytes
         vals = torch.empty(nbytes, dtype=torch.uint8, device=self.device)
         capi.check(capi.lib().cb200_bell_lowering_materialize(
-            C.byref(self.input), C.byref(geo), C.c_int32(layout), C.c_uint64(row_stride_bytes),
-            C.c_void_p(pfo.data_ptr()), C.c_void_p(cols.data_ptr() if cols.numel() else None),
-            C.c_void_p(vals.data_ptr() if vals.numel() else None), C.c_void_p(self.workspace.data_ptr()),
-            C.c_uint64(self.workspace.numel()), C.c_void_p(_stream_handle(self.device))))
+            self._input_ref, C.byref(geo), layout, row_stride_bytes, pfo.data_ptr(), cols.data_ptr(), vals.data_ptr(),
+            self.workspace.data_ptr(), self.workspace.numel(), _stream_handle(self.device)))
         return pfo, cols, vals
 
 

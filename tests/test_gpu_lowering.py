@@ -271,3 +271,33 @@ def test_execution_csr_ids(cuda_device, oracle):
         for a in swapped[1:]:
             a[i], a[i + 1] = a[i + 1], a[i]
         assert ops.build_execution_csr(*[dev(a) for a in swapped], p["features"], p["fb_offsets"], dev(p["fperm"]))[0] == 2
+
+
+@pytest.mark.parametrize("features,mean_nnz,dtype", [(70_000, 40, np.uint8), (70_000, 300, np.float32), (1500, 140, np.uint16)])
+def test_many_block_columns_and_both_layouts(cuda_device, oracle, features, mean_nnz, dtype):
+    """More block columns than the byte marks hold, tiles that do and do not fit shared memory, rows longer than one batch of
+    loads; the row-major layout (stride with padding) holds the same values as the block-major one."""
+    h = synth.make_lowering_host(rows=131, features=features, feature_blocks=3, mean_nnz=mean_nnz, seed=mean_nnz, value_dtype=dtype)
+    args = (h["row_offsets"], h["feature_ids"], h["values"], features, h["fb_offsets"], h["fperm"], h["rperm"])
+    low = ops.BellLowering(*args, cuda_device)
+    vs = np.dtype(dtype).itemsize
+    for bs in (8, 32):
+        geo = assert_same(oracle, low, args, bs, max_value_expansion=1e9, max_storage_expansion=1e9)
+        for pad in (0, 16, 4 * vs):
+            stride = (geo.ell_columns * vs + 15) // 16 * 16 + pad
+            _, _, blocks = low.materialize(geo)
+            _, _, lines = low.materialize(geo, layout=capi.BELL_VALUES_ROW_MAJOR, row_stride_bytes=stride)
+            want = blocks.view(geo.block_rows, geo.ell_blocks_per_row, bs, bs * vs).permute(0, 2, 1, 3).reshape(geo.padded_rows, -1)
+            got = lines.view(geo.padded_rows, stride)
+            assert torch.equal(got[:, :geo.ell_columns * vs], want) and not got[:, geo.ell_columns * vs:].any()
+
+
+@pytest.mark.parametrize("what,match", [("feature", "invalid source"), ("offset", "invalid source"), ("row", "incompatible order"),
+                                        ("inverse", "incompatible plan")])
+def test_values_out_of_range_are_refused(cuda_device, what, match):
+    h = synth.make_lowering_host(rows=70, features=500, feature_blocks=1, mean_nnz=20, seed=5)
+    low = ops.BellLowering(h["row_offsets"], h["feature_ids"], h["values"], 500, h["fb_offsets"], h["fperm"], h["rperm"], cuda_device)
+    array, at = {"feature": (low.feature_ids, 33), "offset": (low.row_offsets, 40), "row": (low.rperm, 69), "inverse": (low.finv, 7)}[what]
+    array[at] = 2 ** 31 - 1
+    with pytest.raises(capi.Cb200Error, match=match):
+        low.query(32)
