@@ -540,7 +540,7 @@ cb200_status cb200_spmm_prepare(const cb200_spmm_problem *problem, cb200_prepare
     if (scope.status != cudaSuccess) return abandon(fail(CB200_STATUS_CUDA_ERROR, "%s", cudaGetErrorString(scope.status)));
 
     if (problem->projection == CB200_PROJECTION_TRANSPOSE) {
-        p->workspace_bytes = qcsr_transpose_workspace_bytes(problem->k, problem->n, p->sm_count);
+        p->workspace_bytes = qcsr_transpose_workspace_bytes(problem->m, problem->k, p->sm_count);
         p->schedule_name = "vector_reductions";
         if (plan.gene_gather) {
             const cb200_status st = build_gene_major_layout(view_of(*problem->device_matrix), p->arena, stream, &p->gene_major);
@@ -636,6 +636,8 @@ cb200_status cb200_spmm_prepare(const cb200_spmm_problem *problem, cb200_prepare
     // the gather kernel runs with the status block alone: without room for W re-laid it reads W as it is
     const bool gathers = problem->projection == CB200_PROJECTION_CSR && p->schedule == fwd_schedule::warp_per_row;
     p->workspace_required = gathers ? std::min<std::uint64_t>(p->workspace_bytes, 256u) : p->workspace_bytes;
+    // the fp32-FMA transpose runs without any: entries are then added one by one instead of sorted first
+    if (problem->projection == CB200_PROJECTION_TRANSPOSE && !plan.gene_gather && !plan.blocked) p->workspace_required = 0u;
     *out = p;
     return CB200_STATUS_SUCCESS;
 }
@@ -763,6 +765,7 @@ cb200_status cb200_prepared_status(const cb200_prepared *prepared, const void *w
     if (prepared == nullptr || host_word == nullptr) return fail(CB200_STATUS_INVALID_ARGUMENT, "status needs a prepared operation and an output");
     *host_word = 0;
     if (prepared->workspace_bytes == 0u) return CB200_STATUS_SUCCESS; // this schedule waits on nothing
+    if (workspace == nullptr && prepared->workspace_required == 0u) return CB200_STATUS_SUCCESS;
     if (workspace == nullptr) return fail(CB200_STATUS_INVALID_ARGUMENT, "status needs the workspace of the launch");
     device_scope scope(prepared->problem.device);
     CB200_CUDA_OK(scope.status);

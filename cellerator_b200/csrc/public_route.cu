@@ -177,6 +177,7 @@ cb200_status route(const cb200_public_layout *l, int32_t projection, const float
     // the exact fp32 schedules these calls select need the status block only; what a CSR projection could use beyond it is not
     // in the scratch these calls ask for
     if (projection == CB200_PROJECTION_CSR) need = std::min<std::uint64_t>(need, 256u);
+    if (projection == CB200_PROJECTION_TRANSPOSE && (need + 255u) / 256u * 256u > cur.left) need = 0u; // runs without
     void *ws = need == 0u ? nullptr : (need <= 256u ? status_block : cur.take(need));
     if (need != 0u && ws == nullptr) {
         cb200_prepared_destroy(prepared);
@@ -187,7 +188,7 @@ cb200_status route(const cb200_public_layout *l, int32_t projection, const float
     ln.alpha = 1.0f; ln.beta = 0.0f; ln.structure_epoch = 1u; ln.stream = stream; ln.device = device;
     ln.row_begin = 0; ln.row_end = CB200_ALL_ROWS;
     ln.workspace_device = device; ln.workspace = ws; ln.workspace_bytes = need;
-    if (need == 0u) { // a schedule without waits: the status block still reads 0 afterwards
+    if (ws != status_block) { // a schedule without waits: the status block still reads 0 afterwards
         device_scope scope(device);
         CB200_CUDA_OK(scope.status);
         CB200_CUDA_OK(cudaMemsetAsync(status_block, 0, sizeof(int), static_cast<cudaStream_t>(stream)));
@@ -209,7 +210,9 @@ extern "C" cb200_status cb200_public_projection_scratch(const cb200_public_layou
     // widened row offsets (CSR) + the status block of the fp32 schedules these calls select
     const std::uint64_t offsets = layout->layout == CB200_PUBLIC_LAYOUT_QUANTIZED_CSR ? (static_cast<std::uint64_t>(layout->rows) + 1u) * 8u : 0u;
     const std::uint64_t arrays = layout->layout == CB200_PUBLIC_LAYOUT_QUANTIZED_CSR && layout->bits == 4u ? 2u : 1u; // + packed row offsets
-    *bytes = arrays * ((offsets + 255u) / 256u * 256u) + 512u;
+    // ... and what the transpose sorts its entries with
+    const std::uint64_t transpose = offsets != 0u ? qcsr_transpose_tiled_workspace_bytes(layout->rows, layout->cols, 160) : 0u;
+    *bytes = arrays * ((offsets + 255u) / 256u * 256u) + 512u + (transpose + 255u) / 256u * 256u;
     return CB200_STATUS_SUCCESS;
 }
 

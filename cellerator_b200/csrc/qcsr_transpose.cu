@@ -43,7 +43,8 @@ __device__ __forceinline__ unsigned tr_load_code(const std::uint8_t *row_bytes, 
 }
 
 // out = beta * out (beta == 0 writes zeros without reading).
-__global__ void __launch_bounds__(256) scale_output_kernel(float *out, std::int64_t rows, int n, std::int64_t ld, float beta) {
+__global__ void __launch_bounds__(256) scale_output_kernel(float *out, std::int64_t rows, int n, std::int64_t ld, float beta, int *status) {
+    if (status != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *status = 0; // nothing here waits
     const std::int64_t total = rows * n;
     for (std::int64_t i = static_cast<std::int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
          i += static_cast<std::int64_t>(gridDim.x) * blockDim.x) {
@@ -157,7 +158,9 @@ cb200_status dispatch(const tr_params &p, bool vector_ok, cudaStream_t stream) {
 
 } // namespace
 
-std::uint64_t qcsr_transpose_workspace_bytes(std::int64_t, std::int64_t, int) { return 0; }
+std::uint64_t qcsr_transpose_workspace_bytes(std::int64_t rows, std::int64_t cols, int sm_count) {
+    return qcsr_transpose_tiled_workspace_bytes(rows, cols, sm_count);
+}
 
 cb200_status launch_qcsr_transpose(const qcsr_view &x, const dense_args &d, std::int64_t row_begin,
                                    std::int64_t row_end, const blocked_layout *blocked, bool split_products,
@@ -170,11 +173,17 @@ cb200_status launch_qcsr_transpose(const qcsr_view &x, const dense_args &d, std:
                                                               split_products, sm_count, stream, &taken);
         if (st != CB200_STATUS_SUCCESS || taken) return st;
     }
+    {
+        bool taken = false;
+        const cb200_status st = launch_qcsr_transpose_tiled(x, d, row_begin, row_end, workspace, workspace_bytes, sm_count, stream, &taken);
+        if (st != CB200_STATUS_SUCCESS || taken) return st;
+    }
     // The output is initialised even for an empty row range: G' = beta * G'.
     {
         const std::int64_t total = x.cols * d.n;
         const unsigned grid = static_cast<unsigned>(std::min<std::int64_t>((total + 255) / 256, static_cast<std::int64_t>(sm_count) * 8));
-        scale_output_kernel<<<grid, 256, 0, stream>>>(d.out, x.cols, static_cast<int>(d.n), d.out_ld, d.beta);
+        int *status = workspace != nullptr && workspace_bytes >= sizeof(int) ? static_cast<int *>(workspace) : nullptr;
+        scale_output_kernel<<<grid, 256, 0, stream>>>(d.out, x.cols, static_cast<int>(d.n), d.out_ld, d.beta, status);
         count_launch();
         CB200_CUDA_OK(cudaGetLastError());
     }
