@@ -127,5 +127,89 @@ __global__ void __launch_bounds__(256) pack_windows_kernel(const WT *w, std::int
     }
 }
 
+// The work of a CTA: whole groups, or parts of a group's windows (window_split_plan).
+struct window_split {
+    int whole;   // groups from this one on are cut
+    int parts;
+    float *sums; // [(group - whole) * parts + part][kRows][N], raw accumulators
+};
+struct window_unit {
+    int group, w0, w1;
+    int slot; // where the sums go; -1: a whole group, written to Y
+};
+__host__ __device__ __forceinline__ int whole_groups_in(const window_split &s, std::int64_t begin, std::int64_t end) {
+    const int last = s.whole < static_cast<int>(end) ? s.whole : static_cast<int>(end);
+    return last > static_cast<int>(begin) ? last - static_cast<int>(begin) : 0;
+}
+// units of the groups [begin, end): whole groups first, then the parts of the others
+__host__ __device__ __forceinline__ int unit_count(const window_split &s, std::int64_t begin, std::int64_t end) {
+    const int whole = whole_groups_in(s, begin, end);
+    return whole + (static_cast<int>(end - begin) - whole) * s.parts;
+}
+__device__ __forceinline__ window_unit unit_at(const window_split &s, std::int64_t begin, std::int64_t end, int windows, int u) {
+    const int whole = whole_groups_in(s, begin, end);
+    if (u < whole) return window_unit{static_cast<int>(begin) + u, 0, windows, -1};
+    const int cut = (u - whole) / s.parts, part = (u - whole) - cut * s.parts;
+    const int group = static_cast<int>(begin) + whole + cut;
+    return window_unit{group, windows * part / s.parts, windows * (part + 1) / s.parts, (group - s.whole) * s.parts + part};
+}
+// units of this CTA: blockIdx.x, + gridDim.x, ...
+__device__ __forceinline__ int units_of_cta(const window_split &s, std::int64_t begin, std::int64_t end) {
+    const int units = unit_count(s, begin, end), first = static_cast<int>(blockIdx.x), step = static_cast<int>(gridDim.x);
+    return units > first ? (units - first + step - 1) / step : 0;
+}
+
+// Y of the groups that were cut: the parts' sums in order, then what the epilogue of a whole group does.
+// result_scale / w_absmax / value_bound: the powers of two the operands were stored times (null: none).
+__global__ void __launch_bounds__(256) add_parts_kernel(const float *sums, int parts, int whole, int first_group, std::int64_t row_end,
+                                                        int n, float *y, std::int64_t y_ld, float alpha, float beta, const float *bias,
+                                                        int epilogue, float result_scale, const unsigned *w_absmax, const unsigned *value_bound) {
+    const std::int64_t group = first_group + static_cast<int>(blockIdx.x);
+    const float *in = sums + (group - whole) * parts * kRows * n;
+    float scale = alpha * result_scale;
+    if (w_absmax != nullptr) scale /= operand_scale(__uint_as_float(__ldg(w_absmax)));
+    if (value_bound != nullptr) scale /= operand_scale(__uint_as_float(__ldg(value_bound)));
+    const int pieces = kRows * n / 4;
+    for (int i = blockIdx.y * 256 + threadIdx.x; i < pieces; i += gridDim.y * 256) {
+        const int r = i / (n / 4), c = (i % (n / 4)) * 4;
+        const std::int64_t row = group * kRows + r;
+        if (row >= row_end) break;
+        float4 v = *reinterpret_cast<const float4 *>(in + 4 * static_cast<std::int64_t>(i));
+        for (int k = 1; k < parts; ++k) {
+            const float4 t = *reinterpret_cast<const float4 *>(in + static_cast<std::int64_t>(k) * kRows * n + 4 * static_cast<std::int64_t>(i));
+            v.x += t.x; v.y += t.y; v.z += t.z; v.w += t.w;
+        }
+        float *out = y + row * y_ld + c;
+        v.x *= scale; v.y *= scale; v.z *= scale; v.w *= scale;
+        if (beta != 0.0f) {
+            const float4 o = *reinterpret_cast<const float4 *>(out);
+            v.x = fmaf(beta, o.x, v.x); v.y = fmaf(beta, o.y, v.y); v.z = fmaf(beta, o.z, v.z); v.w = fmaf(beta, o.w, v.w);
+        }
+        if (epilogue != CB200_EPILOGUE_NONE) {
+            v.x = finish_output(v.x, bias, c, epilogue); v.y = finish_output(v.y, bias, c + 1, epilogue);
+            v.z = finish_output(v.z, bias, c + 2, epilogue); v.w = finish_output(v.w, bias, c + 3, epilogue);
+        }
+        *reinterpret_cast<float4 *>(out) = v;
+    }
+}
+inline cb200_status launch_add_parts(const window_split &s, std::int64_t group_begin, std::int64_t group_end, std::int64_t row_end, int n, float *y,
+                                     std::int64_t y_ld, float alpha, float beta, const float *bias, int epilogue, float result_scale,
+                                     const unsigned *w_absmax, const unsigned *value_bound, cudaStream_t stream) {
+    const int first = static_cast<int>(group_begin) + whole_groups_in(s, group_begin, group_end), cut = static_cast<int>(group_end) - first;
+    if (cut <= 0) return CB200_STATUS_SUCCESS;
+    add_parts_kernel<<<dim3(static_cast<unsigned>(cut), static_cast<unsigned>(n / 16)), 256, 0, stream>>>(
+        s.sums, s.parts, s.whole, first, row_end, n, y, y_ld, alpha, beta, bias, epilogue, result_scale, w_absmax, value_bound);
+    count_launch();
+    CB200_CUDA_OK(cudaGetLastError());
+    return CB200_STATUS_SUCCESS;
+}
+// The split of a launch: cut where the workspace holds the sums behind its `used` bytes.
+inline window_split split_of_launch(const qcsr_view &x, std::int64_t n, void *workspace, std::uint64_t workspace_bytes, std::uint64_t used, int sm_count) {
+    const window_split_plan plan = qcsr_window_split(x.rows, x.cols, sm_count);
+    const std::uint64_t at = device_arena::rounded(used);
+    if (plan.parts == 1 || workspace_bytes < at + qcsr_window_split_bytes(x.rows, x.cols, n, sm_count)) return window_split{0x7fffffff, 1, nullptr};
+    return window_split{static_cast<int>(plan.whole), plan.parts, reinterpret_cast<float *>(static_cast<unsigned char *>(workspace) + at)};
+}
+
 } // namespace
 } // namespace cb200

@@ -615,6 +615,9 @@ cb200_status cb200_spmm_prepare(const cb200_spmm_problem *problem, cb200_prepare
                 if (st != CB200_STATUS_SUCCESS) return abandon(st);
                 if (built) p->schedule_name = "tensor_dense";
             }
+            // behind it, the sums of the groups that are cut between CTAs; a launch whose workspace ends before them cuts none
+            p->workspace_required = p->workspace_bytes;
+            p->workspace_bytes = device_arena::rounded(p->workspace_bytes) + qcsr_window_split_bytes(problem->m, problem->k, problem->n, p->sm_count);
             p->persistent_bytes += p->blocked.bytes;
         }
         if (plan.row_order) {
@@ -635,7 +638,7 @@ cb200_status cb200_spmm_prepare(const cb200_spmm_problem *problem, cb200_prepare
     }
     // the gather kernel runs with the status block alone: without room for W re-laid it reads W as it is
     const bool gathers = problem->projection == CB200_PROJECTION_CSR && p->schedule == fwd_schedule::warp_per_row;
-    p->workspace_required = gathers ? std::min<std::uint64_t>(p->workspace_bytes, 256u) : p->workspace_bytes;
+    if (p->workspace_required == 0u) p->workspace_required = gathers ? std::min<std::uint64_t>(p->workspace_bytes, 256u) : p->workspace_bytes;
     // the fp32-FMA transpose runs without any: entries are then added one by one instead of sorted first
     if (problem->projection == CB200_PROJECTION_TRANSPOSE && !plan.gene_gather && !plan.blocked) p->workspace_required = 0u;
     *out = p;

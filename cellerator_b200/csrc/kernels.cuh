@@ -135,6 +135,15 @@ struct blocked_layout {
     // Scales and offsets are NOT in it: they are applied at launch.
     unsigned char *code_tiles = nullptr;
 };
+// How the tensor kernels over 256-row groups share a matrix out: a CTA takes whole groups, except that the windows of the last
+// groups (those from `whole` on, fewer than two per SM) are cut into `parts` so that every SM has work to the end.  It depends
+// on the matrix alone: a row's sum is cut the same way in every launch.  Sums of parts go through the workspace.
+struct window_split_plan {
+    std::int64_t whole = 0;
+    int parts = 1;
+};
+window_split_plan qcsr_window_split(std::int64_t rows, std::int64_t cols, int sm_count);
+std::uint64_t qcsr_window_split_bytes(std::int64_t rows, std::int64_t cols, std::int64_t n, int sm_count);
 bool qcsr_blocked_shape_ok(std::int64_t rows, std::int64_t cols, std::int64_t n, int bits, int dense_dtype);
 std::uint64_t qcsr_blocked_workspace_bytes(std::int64_t cols, std::int64_t n);
 // Current device; memory from `arena`, kernels on `stream`, which is waited for.

@@ -167,6 +167,7 @@ struct codes_params {
     std::int64_t y_ld;
     std::int64_t row_end; // rows >= row_end are computed but not written
     std::int64_t group_begin, group_end;
+    window_split split;
     int windows;
     float alpha, beta;
     const float *bias;
@@ -249,9 +250,8 @@ __global__ void __launch_bounds__(kCodesThreads, 1) qcsr_fwd_codes_kernel(const 
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const std::uint32_t tmem_base = *tmem_slot;
 
-    const std::int64_t first_group = p.group_begin + blockIdx.x;
-    const int my_groups = first_group < p.group_end ? static_cast<int>((p.group_end - first_group + gridDim.x - 1) / gridDim.x) : 0;
-    const int halves = p.windows * (kWin / 64);
+    const int my_units = units_of_cta(p.split, p.group_begin, p.group_end);
+    const auto unit_of = [&](int i) { return unit_at(p.split, p.group_begin, p.group_end, p.windows, static_cast<int>(blockIdx.x) + i * static_cast<int>(gridDim.x)); };
 
     if (warp < kEpilogueWarps) {
         // ================= a warp reads its 32 rows (TMEM lane = row within the sub-block) 32 columns at a time and turns
@@ -262,9 +262,11 @@ __global__ void __launch_bounds__(kCodesThreads, 1) qcsr_fwd_codes_kernel(const 
         unsigned char *turn = turn0 + warp * kTurnBytes;
         const int chunk = lane & 7, row_of_lane = lane >> 3; // on the way out: this lane's 4 columns, and its row among the 4 of a store
         // both operands were stored times powers of two (fp16 range): the result is divided by them again
-        const float alpha = p.alpha / (operand_scale(__uint_as_float(__ldg(p.w_absmax))) * operand_scale(__uint_as_float(__ldg(p.value_bound))));
-        for (int gi = 0; gi < my_groups; ++gi) {
-            const std::int64_t row0 = (first_group + static_cast<std::int64_t>(gi) * gridDim.x) * kRows + sub * 128 + (warp & 3) * 32;
+        const float full_alpha = p.alpha / (operand_scale(__uint_as_float(__ldg(p.w_absmax))) * operand_scale(__uint_as_float(__ldg(p.value_bound))));
+        for (int gi = 0; gi < my_units; ++gi) {
+            const window_unit unit = unit_of(gi);
+            const std::int64_t row0 = static_cast<std::int64_t>(unit.group) * kRows + sub * 128 + (warp & 3) * 32;
+            const float alpha = unit.slot >= 0 ? 1.0f : full_alpha;
             if (bar_wait_sleeping(smem_addr(acc_full), static_cast<std::uint32_t>(gi & 1), abort_flag, 400u)) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll 1
@@ -290,6 +292,12 @@ __global__ void __launch_bounds__(kCodesThreads, 1) qcsr_fwd_codes_kernel(const 
                     t[i] = *reinterpret_cast<const float4 *>(turn + r * 128 + ((chunk ^ (r & 7)) << 4));
                 }
                 __syncwarp(); // the next 32 columns may overwrite the turn buffer
+                if (unit.slot >= 0) { // a part: raw sums, all rows
+                    float *sums = p.split.sums + (static_cast<std::int64_t>(unit.slot) * kRows + sub * 128 + (warp & 3) * 32 + row_of_lane) * NC + h * 32 + 4 * chunk;
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) *reinterpret_cast<float4 *>(sums + 4 * i * NC) = t[i];
+                    continue;
+                }
                 float *out = p.y + (row0 + row_of_lane) * p.y_ld + h * 32 + 4 * chunk;
                 const std::int64_t rows_left = p.row_end - row0 - row_of_lane; // row 4 * i + row_of_lane is written when 4 * i < rows_left
                 if (p.beta != 0.0f) {
@@ -326,22 +334,23 @@ __global__ void __launch_bounds__(kCodesThreads, 1) qcsr_fwd_codes_kernel(const 
         int sa = 0, s = 0;
         std::uint32_t pa = 0, pb = 0;
         bool dead = false;
-        for (int g = 0; g < my_groups && !dead; ++g) {
+        for (int g = 0; g < my_units && !dead; ++g) {
+            const window_unit unit = unit_of(g);
             if (bar_wait(smem_addr(acc_empty), static_cast<std::uint32_t>((g & 1) ^ 1), abort_flag)) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            for (int w = 0; w < p.windows; ++w) {
+            for (int w = unit.w0; w < unit.w1; ++w) {
                 if (bar_wait(smem_addr(b_full + s), pb, abort_flag) || bar_wait(smem_addr(a_full + sa), pa, abort_flag)) { dead = true; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 if (lane == 0) {
                     const std::uint32_t a_col = tmem_base + kOperandCol0 + sa * kOperandCols;
                     const std::uint32_t b_lo = b_lo0 + static_cast<std::uint32_t>((s * WREC) >> 4);
-                    const std::uint32_t fresh = w != 0 ? 1u : 0u; // the group's first MMAs overwrite the accumulators
+                    const std::uint32_t fresh = w != unit.w0 ? 1u : 0u; // the unit's first MMAs overwrite the accumulators
 #pragma unroll
                     for (int kk = 0; kk < kWin / 16; ++kk)
                         mma_f16_a_in_tmem(tmem_base + sb * NC, a_col + sb * 64 + kk * 8, b_lo + kk * 16, b_hi, IDESC, kk == 0 ? fresh : 1u);
                     mma_commit(smem_addr(a_empty + sa));
                     mma_commit(smem_addr(b_empty + s));
-                    if (w == p.windows - 1) mma_commit(smem_addr(acc_full));
+                    if (w == unit.w1 - 1) mma_commit(smem_addr(acc_full));
                 }
                 __syncwarp();
                 sa ^= 1;
@@ -359,14 +368,16 @@ __global__ void __launch_bounds__(kCodesThreads, 1) qcsr_fwd_codes_kernel(const 
             int s = 0, issued = 0;
             std::uint32_t pb = 1;
             bool dead = false;
-            for (int g = 0; g < my_groups && !dead; ++g)
-                for (int w = 0; w < p.windows; ++w) {
+            for (int g = 0; g < my_units && !dead; ++g) {
+                const window_unit unit = unit_of(g);
+                for (int w = unit.w0; w < unit.w1; ++w) {
                     if (bar_wait_sleeping(smem_addr(b_empty + s), pb, abort_flag, 200u)) { dead = true; break; }
                     bar_arrive_expect_tx(smem_addr(b_full + s), WREC);
                     bulk_copy_g2s(bstage0 + s * WREC, p.records + static_cast<std::size_t>(w) * REC, WREC, smem_addr(b_full + s));
                     ++issued;
                     if (++s == SB) { s = 0; pb ^= 1u; }
                 }
+            }
             if (dead) // the copies still in flight land before the CTA gives up its shared memory
                 for (int i = issued > SB ? issued - SB : 0; i < issued; ++i) bar_wait_drain(smem_addr(b_full + i % SB), static_cast<std::uint32_t>((i / SB) & 1));
         }
@@ -376,9 +387,10 @@ __global__ void __launch_bounds__(kCodesThreads, 1) qcsr_fwd_codes_kernel(const 
             int s = 0, issued = 0;
             std::uint32_t pc = 1;
             bool dead = false;
-            for (int g = 0; g < my_groups && !dead; ++g) {
-                const unsigned char *src = p.stages + static_cast<std::size_t>(first_group + static_cast<std::int64_t>(g) * gridDim.x) * halves * kCodeStageBytes;
-                for (int h = 0; h < halves; ++h, src += kCodeStageBytes) {
+            for (int g = 0; g < my_units && !dead; ++g) {
+                const window_unit unit = unit_of(g);
+                const unsigned char *src = p.stages + (static_cast<std::size_t>(unit.group) * p.windows + unit.w0) * (kWin / 64) * kCodeStageBytes;
+                for (int h = unit.w0 * (kWin / 64); h < unit.w1 * (kWin / 64); ++h, src += kCodeStageBytes) {
                     if (bar_wait_sleeping(smem_addr(c_empty + s), pc, abort_flag, 100u)) { dead = true; break; }
                     bar_arrive_expect_tx(smem_addr(c_full + s), kCodeSlotBytes);
                     bulk_copy_g2s(smem_addr(cstage0 + s * kCodeSlotBytes), src, kCodeStageBytes, smem_addr(c_full + s));
@@ -401,7 +413,11 @@ __global__ void __launch_bounds__(kCodesThreads, 1) qcsr_fwd_codes_kernel(const 
         const __half2 magic = __half2half2(__ushort_as_half(static_cast<unsigned short>(0x6400u))); // 1024: fp16(0x6400 | byte) = 1024 + byte
         const __half2 bias = __float2half2_rn(1024.0f + kPresentBias); // fp16(0x6400 | byte) - bias = the code
         const std::uint32_t lane_base = tmem_base + (static_cast<std::uint32_t>(quarter * 32) << 16) + kOperandCol0 + hf * 32 + pairc * 16;
-        const int windows_total = my_groups * p.windows;
+        int windows_total = 0;
+        for (int g = 0; g < my_units; ++g) {
+            const window_unit unit = unit_of(g);
+            windows_total += unit.w1 - unit.w0;
+        }
         int sa = 0;
         std::uint32_t pa = 1;
         for (int wq = 0; wq < windows_total; ++wq) {
@@ -495,8 +511,7 @@ cb200_status launch_codes(const codes_params &p, int sm_count, cudaStream_t stre
     constexpr std::size_t smem = SB * NC * kWin * 2 + SC * kCodeSlotBytes + kTurnRegionBytes + (2 * SC + 2 * kOperandStages + 2 * SB + 2 + kCodeIssuers) * sizeof(std::uint64_t) + 16;
     static_assert(smem <= 232448, "shared memory budget");
     CB200_CUDA_OK(cudaFuncSetAttribute(qcsr_fwd_codes_kernel<NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-    const std::int64_t groups = p.group_end - p.group_begin;
-    const unsigned grid = static_cast<unsigned>(groups < sm_count ? groups : sm_count);
+    const unsigned grid = static_cast<unsigned>(std::min(unit_count(p.split, p.group_begin, p.group_end), sm_count));
     qcsr_fwd_codes_kernel<NC><<<grid, kCodesThreads, smem, stream>>>(p);
     count_launch();
     CB200_CUDA_OK(cudaGetLastError());
@@ -586,12 +601,17 @@ cb200_status launch_qcsr_forward_codes(const qcsr_view &x, const dense_args &d, 
     p.group_begin = row_begin / kRows; p.group_end = (row_end + kRows - 1) / kRows; p.windows = layout.windows;
     p.alpha = d.alpha; p.beta = d.beta; p.bias = d.bias; p.epilogue = d.epilogue; p.status = status;
     p.w_absmax = w_absmax; p.value_bound = value_bound;
+    p.split = split_of_launch(x, d.n, workspace, workspace_bytes, qcsr_codes_workspace_bytes(x.cols, d.n), sm_count);
     *taken = true;
+    cb200_status st;
     switch (d.n) {
-    case 32: return launch_codes<32>(p, sm_count, stream);
-    case 64: return launch_codes<64>(p, sm_count, stream);
-    default: return launch_codes<128>(p, sm_count, stream);
+    case 32: st = launch_codes<32>(p, sm_count, stream); break;
+    case 64: st = launch_codes<64>(p, sm_count, stream); break;
+    default: st = launch_codes<128>(p, sm_count, stream); break;
     }
+    if (st != CB200_STATUS_SUCCESS) return st;
+    return launch_add_parts(p.split, p.group_begin, p.group_end, row_end, static_cast<int>(d.n), d.out, d.out_ld, p.alpha, p.beta, p.bias, p.epilogue,
+                            1.0f, w_absmax, value_bound, stream);
 }
 
 } // namespace cb200

@@ -87,6 +87,7 @@ struct dense_params {
     std::int64_t y_ld;
     std::int64_t row_end; // rows >= row_end are computed but not written
     std::int64_t group_begin, group_end;
+    window_split split;
     int windows;
     float alpha, beta;
     const float *bias;
@@ -149,22 +150,25 @@ __global__ void __launch_bounds__(kDenseThreads, 1) qcsr_fwd_dense_kernel(const 
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const std::uint32_t tmem_base = *tmem_slot;
 
-    const std::int64_t first_group = p.group_begin + blockIdx.x;
-    const std::int64_t my_groups = first_group < p.group_end ? (p.group_end - first_group + gridDim.x - 1) / gridDim.x : 0;
+    const int my_units = units_of_cta(p.split, p.group_begin, p.group_end);
+    const auto unit_of = [&](int i) { return unit_at(p.split, p.group_begin, p.group_end, p.windows, static_cast<int>(blockIdx.x) + i * static_cast<int>(gridDim.x)); };
 
     if (warp < kEpilogueWarps) {
         // ================= thread t writes row t of the group: TMEM lane = row within the sub-block =================
         const int sub = tid >> 7;
-        for (std::int64_t gi = 0; gi < my_groups; ++gi) {
+        for (int gi = 0; gi < my_units; ++gi) {
+            const window_unit unit = unit_of(gi);
             const std::uint32_t ab = static_cast<std::uint32_t>(gi & 1);
-            const std::int64_t row = (first_group + gi * gridDim.x) * kRows + tid;
+            const std::int64_t row = static_cast<std::int64_t>(unit.group) * kRows + tid;
             bar_wait(smem_addr(acc_full + ab), static_cast<std::uint32_t>((gi >> 1) & 1), abort_flag);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
             for (int h = 0; h < NC / 32; ++h) {
                 float v[32];
                 tmem_ld32(tmem_base + (static_cast<std::uint32_t>((warp & 3) * 32) << 16) + ab * kAccCols + sub * NC + h * 32, v);
-                if (row < p.row_end) {
+                if (unit.slot >= 0) { // raw sums of a part
+                    store_row32(p.split.sums + (static_cast<std::int64_t>(unit.slot) * kRows + tid) * NC + h * 32, v, 1.0f, 0.0f, nullptr, h * 32, CB200_EPILOGUE_NONE);
+                } else if (row < p.row_end) {
                     float *out = p.y + row * p.y_ld + h * 32;
                     store_row32(out, v, p.alpha * p.result_scale / (p.w_absmax != nullptr ? operand_scale(__uint_as_float(__ldg(p.w_absmax))) : 1.0f), p.beta, p.bias, h * 32, p.epilogue);
                 }
@@ -176,11 +180,12 @@ __global__ void __launch_bounds__(kDenseThreads, 1) qcsr_fwd_dense_kernel(const 
     } else if (warp == kEpilogueWarps) {
         // ================= MMA issuer =================
         long long qa = 0, qb = 0;
-        for (std::int64_t g = 0; g < my_groups; ++g) {
+        for (int g = 0; g < my_units; ++g) {
+            const window_unit unit = unit_of(g);
             const std::uint32_t ab = static_cast<std::uint32_t>(g & 1);
             bar_wait(smem_addr(acc_empty + ab), static_cast<std::uint32_t>(((g >> 1) & 1) ^ 1), abort_flag);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            for (int w = 0; w < p.windows; ++w, ++qb) {
+            for (int w = unit.w0; w < unit.w1; ++w, ++qb) {
                 const int s = static_cast<int>(qb % SB);
                 bar_wait(smem_addr(b_full + s), static_cast<std::uint32_t>((qb / SB) & 1), abort_flag);
                 const std::uint32_t b_tile = bstage0 + s * WREC;
@@ -196,12 +201,12 @@ __global__ void __launch_bounds__(kDenseThreads, 1) qcsr_fwd_dense_kernel(const 
 #pragma unroll
                             for (int sb = 0; sb < kSubBlocks; ++sb)
                                 mma_bf16(tmem_base + ab * kAccCols + sb * NC, smem_desc_sw128(a_stage + sb * kHalfBytes + kk * 32), db,
-                                         IDESC, w > 0 || half > 0 || kk > 0);
+                                         IDESC, w > unit.w0 || half > 0 || kk > 0);
                         }
                         mma_commit(smem_addr(a_empty + sa));
                         if (half == kWin / 64 - 1) {
                             mma_commit(smem_addr(b_empty + s));
-                            if (w == p.windows - 1) mma_commit(smem_addr(acc_full + ab));
+                            if (w == unit.w1 - 1) mma_commit(smem_addr(acc_full + ab));
                         }
                     }
                     __syncwarp();
@@ -211,26 +216,31 @@ __global__ void __launch_bounds__(kDenseThreads, 1) qcsr_fwd_dense_kernel(const 
     } else if (warp == kEpilogueWarps + 1) {
         // ================= W loader =================
         if (lane == 0) {
-            const long long total = my_groups * p.windows;
-            for (long long q = 0; q < total; ++q) {
-                const int s = static_cast<int>(q % SB);
-                bar_wait(smem_addr(b_empty + s), static_cast<std::uint32_t>(((q / SB) & 1) ^ 1), abort_flag);
-                bar_arrive_expect_tx(smem_addr(b_full + s), WREC);
-                bulk_copy_g2s(bstage0 + s * WREC, p.records + static_cast<std::size_t>(q % p.windows) * REC, WREC, smem_addr(b_full + s));
+            long long q = 0;
+            for (int g = 0; g < my_units; ++g) {
+                const window_unit unit = unit_of(g);
+                for (int w = unit.w0; w < unit.w1; ++w, ++q) {
+                    const int s = static_cast<int>(q % SB);
+                    bar_wait(smem_addr(b_empty + s), static_cast<std::uint32_t>(((q / SB) & 1) ^ 1), abort_flag);
+                    bar_arrive_expect_tx(smem_addr(b_full + s), WREC);
+                    bulk_copy_g2s(bstage0 + s * WREC, p.records + static_cast<std::size_t>(w) * REC, WREC, smem_addr(b_full + s));
+                }
             }
         }
     } else {
         // ================= A loaders: half-stages in turn =================
         if (lane == 0) {
-            const long long per_group = static_cast<long long>(p.windows) * (kWin / 64);
-            const long long total = my_groups * per_group;
-            for (long long q = warp - kEpilogueWarps - 2; q < total; q += kDenseALoaders) {
-                const int s = static_cast<int>(q % SA);
-                const std::int64_t group = first_group + (q / per_group) * gridDim.x;
-                const unsigned char *src = p.tiles + (static_cast<std::size_t>(group) * per_group + static_cast<std::size_t>(q % per_group)) * kDenseStageBytes;
-                bar_wait(smem_addr(a_empty + s), static_cast<std::uint32_t>(((q / SA) & 1) ^ 1), abort_flag);
-                bar_arrive_expect_tx(smem_addr(a_full + s), kDenseStageBytes);
-                bulk_copy_g2s(smem0 + s * kDenseStageBytes, src, kDenseStageBytes, smem_addr(a_full + s));
+            long long q = 0; // half-stages of this CTA; every loader counts all of them and issues its own
+            for (int g = 0; g < my_units; ++g) {
+                const window_unit unit = unit_of(g);
+                const unsigned char *src = p.tiles + (static_cast<std::size_t>(unit.group) * p.windows + unit.w0) * (kWin / 64) * kDenseStageBytes;
+                for (int h = 0; h < (unit.w1 - unit.w0) * (kWin / 64); ++h, ++q, src += kDenseStageBytes) {
+                    if (q % kDenseALoaders != warp - kEpilogueWarps - 2) continue;
+                    const int s = static_cast<int>(q % SA);
+                    bar_wait(smem_addr(a_empty + s), static_cast<std::uint32_t>(((q / SA) & 1) ^ 1), abort_flag);
+                    bar_arrive_expect_tx(smem_addr(a_full + s), kDenseStageBytes);
+                    bulk_copy_g2s(smem0 + s * kDenseStageBytes, src, kDenseStageBytes, smem_addr(a_full + s));
+                }
             }
         }
     }
@@ -250,8 +260,7 @@ cb200_status launch_dense(const dense_params &p, int sm_count, cudaStream_t stre
                                  (2 * dense_a_stages(NC) + 2 * kDenseBStages + 4) * sizeof(std::uint64_t) + 16;
     static_assert(smem <= 232448, "shared memory budget");
     CB200_CUDA_OK(cudaFuncSetAttribute(qcsr_fwd_dense_kernel<NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-    const std::int64_t groups = p.group_end - p.group_begin;
-    const unsigned grid = static_cast<unsigned>(groups < sm_count ? groups : sm_count);
+    const unsigned grid = static_cast<unsigned>(std::min(unit_count(p.split, p.group_begin, p.group_end), sm_count));
     qcsr_fwd_dense_kernel<NC><<<grid, kDenseThreads, smem, stream>>>(p);
     count_launch();
     CB200_CUDA_OK(cudaGetLastError());
@@ -342,12 +351,17 @@ cb200_status launch_qcsr_forward_dense(const qcsr_view &x, const dense_args &d, 
     p.idesc = instr_desc(static_cast<int>(d.n), half);
     p.result_scale = half ? 1.0f / layout.value_scale : 1.0f;
     p.w_absmax = half ? w_absmax : nullptr;
+    p.split = split_of_launch(x, d.n, workspace, workspace_bytes, qcsr_blocked_workspace_bytes(x.cols, d.n), sm_count);
     *taken = true;
+    cb200_status st;
     switch (d.n) {
-    case 32: return launch_dense<32>(p, sm_count, stream);
-    case 64: return launch_dense<64>(p, sm_count, stream);
-    default: return launch_dense<128>(p, sm_count, stream);
+    case 32: st = launch_dense<32>(p, sm_count, stream); break;
+    case 64: st = launch_dense<64>(p, sm_count, stream); break;
+    default: st = launch_dense<128>(p, sm_count, stream); break;
     }
+    if (st != CB200_STATUS_SUCCESS) return st;
+    return launch_add_parts(p.split, p.group_begin, p.group_end, row_end, static_cast<int>(d.n), d.out, d.out_ld, p.alpha, p.beta, p.bias, p.epilogue,
+                            p.result_scale, p.w_absmax, nullptr, stream);
 }
 
 } // namespace cb200
