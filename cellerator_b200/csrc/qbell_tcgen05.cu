@@ -22,23 +22,22 @@
 // out of the result.  The decode runs on pairs: a byte permute (code -> fp16 1024 + code), a subtraction, a fused
 // multiply-add with the pair's {scale, offset} from a table of fp16 pairs written beside W^T at launch.
 //
-// One CTA (288 threads, two CTAs per SM) streams the present blocks of its block rows, two at a time, through a
-// 2-stage ring (two blocks share a stage's waits, proxy fence and hand-over: 0.273 ms against 0.296 with one
-// block per stage and four stages, on 250k cells x 8,192 genes):
-//   warps 4-7  producers: one thread fetches the block's slice of W^T with a single bulk async copy
-//              (cp.async.bulk, byte-counted on the stage's mbarrier; fetching it as 1,024 separate
-//              16-byte cp.async chunks doubled the L2 sector traffic and ran at half the speed);
-//              all 128 decode the block's 32 x 32 codes to fp16 (per-gene scale / zero-point
-//              applied in registers) straight into the operand layout.  Codes and metadata of a
-//              whole block row are staged in shared memory one block row ahead, so decoding never
-//              waits on DRAM;
-//   warp  8    one elected thread issues the MMAs, commits them to the stage's "empty" barrier
-//              and, after the last block of a block row, to the accumulator's "full" barrier;
-//   warps 0-3  epilogue: tcgen05.ld the accumulators (double buffered in TMEM so the next block
-//              row's MMAs overlap), apply alpha / beta, store Y rows coalesced.
-// Empty blocks (index 0xffffffff) are skipped; genes >= cols and cells past the last row decode
-// to 0.  Every barrier wait is bounded; on a time-out a status word is set, the waits stop
-// blocking, and the kernel still runs to completion and frees its TMEM.
+// What bounds it: every block's slice of W^T comes from L2, N x 64 bytes per 32 x 32 codes (2.05 GB for 250k cells x 8,192 genes,
+// 16 blocks wide, N = 256, against 0.38 GB of codes and Y), and bulk copies reach 14 TB/s of L2 -> shared memory at best.  The
+// tensor pipe needs 40 cycles per 128 x 32 x 16 MMA, half of a block's time.  One CTA per SM walks block rows:
+//   3 warps    one elected thread of each copies every third pair of neighbouring blocks' slices into the stages of a ring (216 KB);
+//   16 warps   decode, in four groups that take the pairs of a block row in turn, into the same stages; their codes and
+//              {scale, offset} pairs are read straight into registers a block row ahead, so nothing waits for DRAM and no
+//              shared memory holds codes;
+//   H warps    issue the MMAs, one per 128 output columns: one wait and one commit per pair of blocks;
+//   warps 0-3  epilogue: tcgen05.ld the accumulators (double buffered, handed back before the last columns' stores), apply
+//              alpha / beta, store Y rows coalesced.
+// A form with two CTAs per SM, each with two stages of two blocks, whose decoding warps also started the copies, ran a stage's
+// copy, MMAs and release one after the other (3,800 cycles per 36 KB): 222 us for that matrix, now 169 (N = 128: 185 -> 126); with
+// a ring of single blocks and a commit per block the issuing threads were the bound (218 us; 331 before they were elected,
+// see elect_one).
+// Empty blocks (index 0xffffffff) are skipped; genes >= cols and cells past the last row decode to 0.  Every barrier wait is
+// bounded; on a time-out a status word is set, every role ends, and the kernel frees its TMEM.
 #include "kernels.cuh"
 #include "operand_scaling.cuh"
 #include "sm100_primitives.cuh"
@@ -54,18 +53,18 @@ std::uint64_t qbell_tcgen05_workspace_bytes(std::int64_t cols, std::int64_t n) {
 
 namespace {
 
-constexpr int kStages = 2;          // ring stages; a stage holds up to kStageBlocks present blocks of one block row
-constexpr int kStageBlocks = 2;     // two blocks share the stage's waits, proxy fence and hand-over
-constexpr int kMaxWidth = 16;                      // blocks per block row the staging area holds
-constexpr int kCodesStageBytes = 32 * 512;         // one block row of codes: 32 cells x up to 512 bytes
-constexpr int kMetaStageBytes = kMaxWidth * 128;   // per block: 16 gene pairs x {scale pair, offset pair} as fp16
-constexpr int kEpilogueThreads = 128; // warps 0-3
-constexpr int kProducerThreads = 128; // warps 4-7
-constexpr int kThreads = 288;         // + MMA warp 8
-constexpr int kATileBytes = 256 * 64; // 256 output columns x 32 genes fp16
+constexpr int kMaxWidth = 16;         // blocks per block row: the pairs whose codes a decode group keeps in registers
+constexpr int kGroups = 4;            // decode groups of four warps
+constexpr int kGroupPairs = kMaxWidth / 2 / kGroups;
+static_assert(kGroupPairs * kGroups * 2 == kMaxWidth, "every pair has its group and place");
+constexpr int kLoaders = 3;           // a copy with its wait and expect-tx holds its thread for hundreds of cycles, whatever its size
 constexpr int kBTileBytes = 32 * 64;  // 32 cells x 32 genes fp16
-constexpr int kBlockBytes = kATileBytes + kBTileBytes; // one block's operands: [A 16 KB | B 2 KB]
-constexpr int kStageBytes = kStageBlocks * kBlockBytes;
+constexpr int kEpilogueWarps = 4;
+constexpr int kDecodeWarps = 4 * kGroups;
+__host__ __device__ constexpr int a_tile_bytes(int h) { return h * 128 * 64; } // 128 h output columns x 32 genes fp16
+__host__ __device__ constexpr int stage_bytes(int h) { return 2 * (a_tile_bytes(h) + kBTileBytes); } // a pair of blocks: [A][A][B][B]
+__host__ __device__ constexpr int stages_of(int h) { return h == 2 ? 6 : 9; } // what shared memory holds; a loader's pairs keep to its stages
+__host__ __device__ constexpr int threads_of(int h) { return 32 * (kEpilogueWarps + kDecodeWarps + h + kLoaders); }
 
 struct tc_params {
     std::int64_t rows, cols;
@@ -93,14 +92,6 @@ struct tc_params {
     int *status;
 };
 
-__device__ __forceinline__ void bar_expect_tx(std::uint32_t bar, std::uint32_t bytes) {
-    asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void cp_async_16(std::uint32_t dst, const void *src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template<int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 // K-major, no swizzle: core matrices of 8 rows x 16 bytes; LBO (between the two core matrices a
 // K = 16 instruction reads) = 128 B, SBO (between groups of 8 rows) = 512 B.
 __device__ __forceinline__ std::uint64_t smem_desc(std::uint32_t addr) {
@@ -114,12 +105,13 @@ __device__ __forceinline__ std::uint64_t smem_desc(std::uint32_t addr) {
 // kind::f16 instruction descriptor: D fp32, A and B fp16 (format 0), both K-major, N = 32, M = 128.
 constexpr std::uint32_t kInstrDesc = (1u << 4) | ((32u >> 3) << 17) | ((128u >> 4) << 24);
 
-__device__ __forceinline__ void mma_f16(std::uint32_t tmem_d, std::uint64_t desc_a, std::uint64_t desc_b, bool accumulate) {
+// descriptors as {low, high} words: the high one is the same for every tile
+__device__ __forceinline__ void mma_f16(std::uint32_t tmem_d, std::uint32_t desc_a, std::uint32_t desc_b, std::uint32_t desc_high, std::uint32_t accumulate) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}"
+        "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\tsetp.ne.b32 p, %4, 0;\n\tmov.b64 da, {%1, %5};\n\tmov.b64 db, {%2, %5};\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, p;\n\t}"
         :
-        : "r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(kInstrDesc), "r"(accumulate ? 1u : 0u), "r"(0u)
+        : "r"(tmem_d), "r"(desc_a), "r"(desc_b), "r"(kInstrDesc), "r"(accumulate), "r"(desc_high)
         : "memory");
 }
 // W [genes][n] (leading dimension ld) -> per gene block of 32, the n x 32 slice of W^T already in
@@ -169,31 +161,57 @@ __global__ void __launch_bounds__(256) pack_w_kernel(const __nv_bfloat16 *w, std
     }
 }
 
-template<int BITS, int H /* N / 128 */>
-__global__ void __launch_bounds__(kThreads, 2) qbell_tcgen05_kernel(const tc_params p) {
-    extern __shared__ __align__(1024) unsigned char smem[];
-    // [kStages][kStageBlocks][A 16 KB | B 2 KB] | staged codes [2] | staged scales/offsets [2] | barriers | tmem base | flags
-    std::uint64_t *bars = reinterpret_cast<std::uint64_t *>(smem + kStages * kStageBytes + 2 * kCodesStageBytes + 2 * kMetaStageBytes);
-    std::uint64_t *full_bar = bars;                  // [kStages]  producers -> MMA      (one arrival per warp)
-    std::uint64_t *empty_bar = bars + kStages;       // [kStages]  MMA commit -> producers (1 arrival)
-    std::uint64_t *acc_full = bars + 2 * kStages;    // [2]        MMA commit -> epilogue  (1 arrival)
-    std::uint64_t *acc_empty = bars + 2 * kStages + 2; // [2]      epilogue -> MMA        (128 arrivals)
-    std::uint32_t *tmem_slot = reinterpret_cast<std::uint32_t *>(bars + 2 * kStages + 4);
-    volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
-    int *row_has_blocks = const_cast<int *>(reinterpret_cast<volatile int *>(tmem_slot + 2)); // [2] per accumulator buffer
+// The present blocks of a block row, and its pairs of neighbouring slots with a present block (bit 2 j of `pairs`: slots
+// 2 j and 2 j + 1).  A block's place in the W ring and a pair's in the decode ring are their numbers in the CTA's walk.
+struct block_row {
+    std::uint32_t column; // of the block in this lane's slot
+    unsigned blocks, pairs;
+};
+__device__ __forceinline__ std::uint32_t load_column(const tc_params &p, std::int64_t br, int lane) {
+    return br < p.block_row_end && lane < p.width ? __ldg(p.block_col_idx + br * p.width + lane) : 0xffffffffu;
+}
+__device__ __forceinline__ block_row make_block_row(std::uint32_t column) {
+    block_row r;
+    r.column = column;
+    r.blocks = __ballot_sync(0xffffffffu, column != 0xffffffffu);
+    r.pairs = (r.blocks | (r.blocks >> 1)) & 0x55555555u;
+    return r;
+}
+// the same answer in every lane: a warp that gives up leaves its loops as one
+__device__ __forceinline__ bool warp_wait(std::uint64_t *bar, int parity, volatile int *abort_flag) {
+    return __any_sync(0xffffffffu, bar_wait(smem_addr(bar), static_cast<std::uint32_t>(parity & 1), abort_flag)) != 0;
+}
+__device__ __forceinline__ bool warp_wait_sleeping(std::uint64_t *bar, int parity, volatile int *abort_flag, unsigned ns) {
+    return __any_sync(0xffffffffu, bar_wait_sleeping(smem_addr(bar), static_cast<std::uint32_t>(parity & 1), abort_flag, ns)) != 0;
+}
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const std::uint32_t smem0 = smem_addr(smem);
+template<int BITS, int H /* N / 128 */>
+__global__ void __launch_bounds__(threads_of(H), 1) qbell_tcgen05_kernel(const tc_params p) {
+    constexpr int kATileBytes = a_tile_bytes(H), kStageBytes = stage_bytes(H), kStages = stages_of(H);
+    static_assert(kStages % kLoaders == 0, "a loader's pairs keep to its stages");
     constexpr int kTmemCols = 2 * H * 32; // two accumulator buffers
+    extern __shared__ __align__(1024) unsigned char smem[];
+    // [kStages][A][A][B][B] | barriers | tmem base | flags
+    std::uint64_t *bars = reinterpret_cast<std::uint64_t *>(smem + kStages * kStageBytes);
+    std::uint64_t *full = bars;                      // [kStages] loader (with the copies' bytes) and the warps of a decode group -> MMA
+    std::uint64_t *empty = full + kStages;           // [kStages] MMA commits -> loader and decode group
+    std::uint64_t *acc_full = empty + kStages;       // [2]       MMA commits -> epilogue
+    std::uint64_t *acc_empty = acc_full + 2;         // [2]       epilogue -> MMA (one arrival per warp)
+    std::uint32_t *tmem_slot = reinterpret_cast<std::uint32_t *>(acc_empty + 2);
+    volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
+    volatile int *row_has_blocks = reinterpret_cast<volatile int *>(tmem_slot + 2); // [2] per accumulator buffer
+
+    const int tid = threadIdx.x, warp = warp_of_block(), lane = tid & 31;
+    const std::uint32_t smem0 = smem_addr(smem);
 
     if (tid == 0) {
         for (int s = 0; s < kStages; ++s) {
-            bar_init(smem_addr(full_bar + s), kProducerThreads / 32); // one arrival per producer warp
-            bar_init(smem_addr(empty_bar + s), 1);
+            bar_init(smem_addr(full + s), 1 + 4);
+            bar_init(smem_addr(empty + s), H);
         }
         for (int b = 0; b < 2; ++b) {
-            bar_init(smem_addr(acc_full + b), 1);
-            bar_init(smem_addr(acc_empty + b), kEpilogueThreads);
+            bar_init(smem_addr(acc_full + b), H);
+            bar_init(smem_addr(acc_empty + b), kEpilogueWarps);
         }
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -208,216 +226,24 @@ __global__ void __launch_bounds__(kThreads, 2) qbell_tcgen05_kernel(const tc_par
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const std::uint32_t tmem_base = *tmem_slot;
 
-    const std::int64_t first = p.block_row_begin + blockIdx.x;
-    const std::int64_t step = gridDim.x;
+    const std::int64_t first = p.block_row_begin + blockIdx.x, step = gridDim.x;
     const bool row_policy = p.policy == CB200_DECODE_COLUMN_SCALE_ROW_OFFSET;
 
-    if (warp >= 4 && warp < 8) {
-        // ================= producers =================
-        const int pt = tid - 128;          // 0..127
-        // B tile: cell within the block row, 8-gene chunk.  A warp takes 16 cells x 2 neighbouring chunks.  The two lanes
-        // of a pair READ the two halves of one 16-byte piece of a cell's staged codes (the pieces of a row are permuted by
-        // cell mod 8 when they are staged, so the eight cells of a half warp read eight different bank groups).  The odd
-        // lanes then swap their codes with the odd lane eight further on, so that a quarter warp DECODES AND STORES cells
-        // c .. c + 3 of one chunk and cells c + 4 .. c + 7 of the next: eight different bank groups of the B tile.
-        const int pair = (pt & 31) >> 1, parity = pt & 1, cell_base = ((pt >> 5) & 1) * 16;
-        const int load_cell = cell_base + pair;
-        const int cell = cell_base + (parity != 0 ? (pair ^ 4) : pair), chunk = (pt >> 6) * 2 + parity;
-        const std::uint32_t codes_stage = smem0 + kStages * kStageBytes;          // [2][32 cells][512 B]
-        const std::uint32_t meta_stage = codes_stage + 2 * kCodesStageBytes;       // [2][16 slots][32 scales | 32 offsets]
-        const int row_bytes = p.width * 32 * BITS / 8;
-        const int chunks_per_row = row_bytes / 16;
-        const float vs = operand_scale(__uint_as_float(__ldg(p.value_bound)) + __uint_as_float(__ldg(p.value_bound + 1)));
-        const __half2 magic = __half2half2(__ushort_as_half(static_cast<unsigned short>(0x6400u))); // 1024: fp16(0x6400 | code) = 1024 + code
-
-        // Codes and per-gene metadata of a whole block row are brought into shared memory one block
-        // row ahead of their use, so that decoding an item never waits on DRAM.
-        auto prefetch_block_row = [&](std::int64_t br, int buf) {
-            for (int i = pt; i < 32 * chunks_per_row; i += kProducerThreads) {
-                const int c_cell = i / chunks_per_row, c = i % chunks_per_row;
-                const std::int64_t row = br * 32 + c_cell;
-                if (row >= p.row_begin && row < p.row_end)
-                    cp_async_16(codes_stage + buf * kCodesStageBytes + c_cell * 512 + ((c ^ (c_cell & 7)) << 4), p.packed + row * p.row_stride + c * 16);
-            }
-            for (int i = pt; i < p.width * 8; i += kProducerThreads) { // a block's 16 pairs: eight 16-byte pieces
-                const int slot = i >> 3, q = i & 7;
-                const std::uint32_t bc = __ldg(p.block_col_idx + br * p.width + slot);
-                if (bc == 0xffffffffu) continue;
-                cp_async_16(meta_stage + buf * kMetaStageBytes + slot * 128 + q * 16, p.pairs + static_cast<std::int64_t>(bc) * 16 + q * 2);
-            }
-        };
-
-        long long item = 0;                // items issued by this thread
-        int iteration = 0;
-        if (first < p.block_row_end) prefetch_block_row(first, 0);
-        cp_async_commit();
-        for (std::int64_t br = first; br < p.block_row_end; br += step, ++iteration) {
-            const int buf = iteration & 1;
-            const std::int64_t row = br * 32 + cell;
-            const bool cell_valid = row >= p.row_begin && row < p.row_end;
-            // row-offset policy: the cell's offset, times the operand's power of two, for both genes of a pair
-            const __half2 row_offset2 = __float2half2_rn((row_policy && p.offsets != nullptr && cell_valid) ? __ldg(p.offsets + row) * vs : 0.0f);
-            // this block row's staged data is complete for every producer thread, and everyone has
-            // finished decoding the previous block row (whose buffer the next prefetch overwrites)
-            cp_async_wait<0>();
-            asm volatile("bar.sync 1, %0;" ::"n"(kProducerThreads) : "memory");
-            if (br + step < p.block_row_end) prefetch_block_row(br + step, buf ^ 1);
-            cp_async_commit();
-            const std::uint32_t my_codes = codes_stage + buf * kCodesStageBytes + load_cell * 512;
-            const std::uint32_t my_meta = meta_stage + buf * kMetaStageBytes + chunk * 32; // the chunk's four gene pairs
-            // the block columns of the block row: one load per lane, handed round by shuffles (a load per block put a
-            // global-memory latency at the head of every item)
-            const std::uint32_t bc_lane = lane < p.width ? __ldg(p.block_col_idx + br * p.width + lane) : 0xffffffffu;
-            // present blocks of the block row, taken two at a time
-            unsigned todo = __ballot_sync(0xffffffffu, bc_lane != 0xffffffffu);
-            while (todo != 0u) {
-                int slots[kStageBlocks];
-                int blocks = 0;
-#pragma unroll
-                for (int j = 0; j < kStageBlocks; ++j) {
-                    slots[j] = todo != 0u ? __ffs(static_cast<int>(todo)) - 1 : -1;
-                    if (todo != 0u) {
-                        todo &= todo - 1u;
-                        ++blocks;
-                    }
-                }
-                const int stage = static_cast<int>(item % kStages);
-                bar_wait(smem_addr(empty_bar + stage), static_cast<std::uint32_t>(((item / kStages) & 1) ^ 1), abort_flag);
-                const std::uint32_t stage_base = smem0 + stage * kStageBytes;
-                // ---- A: the blocks' slices of W^T, already in operand layout: one bulk copy each
-                if (pt == 0) bar_expect_tx(smem_addr(full_bar + stage), static_cast<std::uint32_t>(blocks) * (H * 128 * 64));
-#pragma unroll
-                for (int j = 0; j < kStageBlocks; ++j) {
-                if (slots[j] < 0) break;
-                const int slot = slots[j];
-                const std::uint32_t bc = __shfl_sync(0xffffffffu, bc_lane, slot);
-                const std::uint32_t a_tile = stage_base + j * kBlockBytes;
-                const std::uint32_t b_tile = a_tile + kATileBytes;
-                if (pt == 0)
-                    bulk_copy_g2s(a_tile, p.wt + static_cast<std::int64_t>(bc) * (H * 128 * 32), H * 128 * 64, smem_addr(full_bar + stage));
-                // ---- B: decode 8 codes of (cell, genes chunk) to fp16, from the staged copies: per pair of codes a byte
-                //      permute (code -> fp16 1024 + code), a subtraction (exact), a fused multiply-add with the pair's
-                //      {scale, offset}; genes past the matrix have scale and offset 0
-                std::uint32_t out[4];
-                // every lane reads and swaps (rows outside the launch hold stale bytes that are never decoded)
-                std::uint32_t lo = 0, hi = 0;
-                if constexpr (BITS == 8)
-                    asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=r"(lo), "=r"(hi) : "r"(my_codes + (((slot * 2 + (chunk >> 1)) ^ (load_cell & 7)) << 4) + (chunk & 1) * 8));
-                else
-                    asm volatile("ld.shared.b32 %0, [%1];" : "=r"(lo) : "r"(my_codes + ((slot ^ (load_cell & 7)) << 4) + chunk * 4));
-                {
-                    const std::uint32_t lo_far = __shfl_xor_sync(0xffffffffu, lo, 8), hi_far = __shfl_xor_sync(0xffffffffu, hi, 8);
-                    if (parity != 0) {
-                        lo = lo_far;
-                        hi = hi_far;
-                    }
-                }
-                if (cell_valid) {
-                    std::uint32_t raw[4];
-                    if constexpr (BITS == 8) {
-                        raw[0] = __byte_perm(lo, 0x64646464u, 0x4140u);
-                        raw[1] = __byte_perm(lo, 0x64646464u, 0x4342u);
-                        raw[2] = __byte_perm(hi, 0x64646464u, 0x4140u);
-                        raw[3] = __byte_perm(hi, 0x64646464u, 0x4342u);
-                    } else {
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) {
-                            const std::uint32_t two = lo >> (8 * e); // the byte that holds the pair's two 4-bit codes
-                            raw[e] = 0x64006400u | (two & 0xfu) | ((two & 0xf0u) << 12);
-                        }
-                    }
-                    uint4 m0, m1; // {scale pair, offset pair} of the chunk's pairs 0-1 and 2-3
-                    asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(m0.x), "=r"(m0.y), "=r"(m0.z), "=r"(m0.w) : "r"(my_meta + slot * 128));
-                    asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(m1.x), "=r"(m1.y), "=r"(m1.z), "=r"(m1.w) : "r"(my_meta + slot * 128 + 16));
-                    const std::uint32_t sc[4] = {m0.x, m0.z, m1.x, m1.z}, of[4] = {m0.y, m0.w, m1.y, m1.w};
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        const __half2 code2 = __hsub2(*reinterpret_cast<const __half2 *>(&raw[e]), magic);
-                        __half2 o2 = *reinterpret_cast<const __half2 *>(&of[e]);
-                        if (row_policy) o2 = __hmul2(o2, row_offset2); // the pair's {1 | 0} times the cell's offset
-                        const __half2 v = __hfma2(code2, *reinterpret_cast<const __half2 *>(&sc[e]), o2);
-                        out[e] = *reinterpret_cast<const std::uint32_t *>(&v);
-                    }
-                } else {
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) out[e] = 0u;
-                }
-                {
-                    const std::uint32_t dst = b_tile + (cell >> 3) * 512 + chunk * 128 + (cell & 7) * 16;
-                    const std::uint32_t *w32 = out;
-                    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst), "r"(w32[0]), "r"(w32[1]), "r"(w32[2]), "r"(w32[3])
-                                 : "memory");
-                }
-                } // blocks of the stage
-                fence_async_proxy();                      // the B tiles were written with ordinary stores
-                __syncwarp();
-                if (lane == 0) bar_arrive(smem_addr(full_bar + stage));
-                ++item;
-            }
-        }
-        cp_async_wait<0>();
-    } else if (warp == 8) {
-        // ================= MMA issuer =================
-        long long item = 0;
-        long long use = 0; // block rows handled (accumulator buffer uses)
-        for (std::int64_t br = first; br < p.block_row_end; br += step, ++use) {
-            const int buf = static_cast<int>(use & 1);
-            bar_wait(smem_addr(acc_empty + buf), static_cast<std::uint32_t>(((use >> 1) & 1) ^ 1), abort_flag);
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            bool any = false;
-            const std::uint32_t bc_lane = lane < p.width ? __ldg(p.block_col_idx + br * p.width + lane) : 0xffffffffu;
-            unsigned todo = __ballot_sync(0xffffffffu, bc_lane != 0xffffffffu);
-            while (todo != 0u) {
-                int blocks = 0;
-#pragma unroll
-                for (int j = 0; j < kStageBlocks; ++j)
-                    if (todo != 0u) {
-                        todo &= todo - 1u;
-                        ++blocks;
-                    }
-                const int stage = static_cast<int>(item % kStages);
-                bar_wait(smem_addr(full_bar + stage), static_cast<std::uint32_t>((item / kStages) & 1), abort_flag);
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                if (lane == 0) {
-#pragma unroll
-                    for (int j = 0; j < kStageBlocks; ++j) {
-                        if (j >= blocks) break;
-                        const std::uint32_t a_tile = smem0 + stage * kStageBytes + j * kBlockBytes;
-                        const std::uint32_t b_tile = a_tile + kATileBytes;
-#pragma unroll
-                        for (int h = 0; h < H; ++h) {
-#pragma unroll
-                            for (int kk = 0; kk < 2; ++kk) {
-                                mma_f16(tmem_base + buf * (H * 32) + h * 32, smem_desc(a_tile + h * 8192 + kk * 256),
-                                         smem_desc(b_tile + kk * 256), any || j > 0 || kk > 0);
-                            }
-                        }
-                    }
-                    mma_commit(smem_addr(empty_bar + stage)); // the stage is free once these MMAs have read it
-                }
-                __syncwarp();
-                any = true;
-                ++item;
-            }
-            if (lane == 0) {
-                row_has_blocks[buf] = any ? 1 : 0;
-                mma_commit(smem_addr(acc_full + buf));        // accumulators complete (or nothing was issued)
-            }
-            __syncwarp();
-        }
-    } else if (warp < 4) {
-        // ================= epilogue =================
+    if (warp < kEpilogueWarps) {
+        // ================= epilogue: TMEM lane = output column, TMEM column = cell =================
         // both operands were stored times powers of two (fp16 range): the result is divided by them again
         const float alpha = p.alpha / (operand_scale(__uint_as_float(__ldg(p.w_absmax))) *
                                        operand_scale(__uint_as_float(__ldg(p.value_bound)) + __uint_as_float(__ldg(p.value_bound + 1))));
-        long long use = 0;
+        const bool composed = p.epilogue != CB200_EPILOGUE_NONE;
+        int use = 0; // block rows of this CTA
         for (std::int64_t br = first; br < p.block_row_end; br += step, ++use) {
-            const int buf = static_cast<int>(use & 1);
-            bar_wait(smem_addr(acc_full + buf), static_cast<std::uint32_t>((use >> 1) & 1), abort_flag);
+            const int buf = use & 1;
+            if (warp_wait_sleeping(acc_full + buf, use >> 1, abort_flag, 100u)) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const bool any = *reinterpret_cast<volatile int *>(row_has_blocks + buf) != 0;
+            const bool any = row_has_blocks[buf] != 0;
             const std::int64_t row0 = br * 32;
-#pragma unroll
+            const bool plain = row0 >= p.row_begin && row0 + 32 <= p.row_end && p.beta == 0.0f && !composed;
+#pragma unroll 1
             for (int h = 0; h < H; ++h) {
                 float v[32];
                 if (any) {
@@ -426,25 +252,199 @@ __global__ void __launch_bounds__(kThreads, 2) qbell_tcgen05_kernel(const tc_par
 #pragma unroll
                     for (int i = 0; i < 32; ++i) v[i] = 0.0f;
                 }
+                if (h == H - 1) { // the accumulators are in registers
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0) bar_arrive(smem_addr(acc_empty + buf));
+                }
                 const int col = h * 128 + warp * 32 + lane;
                 // this thread writes one output column of 32 rows: its bias is loaded once
-                const bool composed = p.epilogue != CB200_EPILOGUE_NONE;
                 const float bias = composed && epilogue_has_bias(p.epilogue) ? __ldg(p.bias + col) : 0.0f;
+                float *out = p.y + row0 * p.y_ld + col;
+                if (plain) {
 #pragma unroll
-                for (int c = 0; c < 32; ++c) {
-                    const std::int64_t row = row0 + c;
-                    if (row >= p.row_begin && row < p.row_end) {
-                        float *out = p.y + row * p.y_ld + col;
-                        float r = alpha * v[c];
-                        if (p.beta != 0.0f) r = fmaf(p.beta, *out, r);
-                        if (composed) r = apply_epilogue(r, bias, p.epilogue);
-                        *out = r;
+                    for (int c = 0; c < 32; ++c, out += p.y_ld) *out = alpha * v[c];
+                } else {
+#pragma unroll
+                    for (int c = 0; c < 32; ++c, out += p.y_ld) {
+                        const std::int64_t row = row0 + c;
+                        if (row >= p.row_begin && row < p.row_end) {
+                            float r = alpha * v[c];
+                            if (p.beta != 0.0f) r = fmaf(p.beta, *out, r);
+                            if (composed) r = apply_epilogue(r, bias, p.epilogue);
+                            *out = r;
+                        }
                     }
                 }
             }
-            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            bar_arrive(smem_addr(acc_empty + buf));
         }
+    } else if (warp < kEpilogueWarps + kDecodeWarps) {
+        // ================= decode: group g takes the pairs g, g + kGroups, ... of every block row; a lane decodes eight genes
+        // of one cell of each of the pair's blocks.  The four lanes of a cell read a 32-byte sector; eight lanes of one
+        // chunk store 128 contiguous bytes of the operand tile =================
+        const int group = (warp - kEpilogueWarps) >> 2, cell = ((warp - kEpilogueWarps) & 3) * 8 + (lane & 7), chunk = lane >> 3;
+        const float vs = operand_scale(__uint_as_float(__ldg(p.value_bound)) + __uint_as_float(__ldg(p.value_bound + 1)));
+        const __half2 magic = __half2half2(__ushort_as_half(static_cast<unsigned short>(0x6400u))); // 1024: fp16(0x6400 | code) = 1024 + code
+        uint2 codes[kGroupPairs][2];   // of the block row to come, and its blocks'
+        uint4 meta[kGroupPairs][2][2]; // {scale pair, offset pair} of the chunk's four gene pairs
+        const auto fetch = [&](std::int64_t br, std::uint32_t row_column, int r) {
+            const std::int64_t row = br * 32 + cell;
+            const bool valid = br < p.block_row_end && row >= p.row_begin && row < p.row_end;
+            const std::uint8_t *from = p.packed + (valid ? row * p.row_stride : 0);
+#pragma unroll
+            for (int t = 0; t < 2; ++t) {
+                const int slot = (group + r * kGroups) * 2 + t;
+                const std::uint32_t bc = __shfl_sync(0xffffffffu, row_column, slot);
+                codes[r][t] = make_uint2(0u, 0u);
+                if (bc == 0xffffffffu) continue;
+                if (valid) {
+                    if constexpr (BITS == 8) codes[r][t] = __ldg(reinterpret_cast<const uint2 *>(from + slot * 32 + chunk * 8));
+                    else codes[r][t].x = __ldg(reinterpret_cast<const unsigned *>(from + slot * 16 + chunk * 4));
+                }
+                const uint4 *pairs = reinterpret_cast<const uint4 *>(p.pairs + static_cast<std::int64_t>(bc) * 16 + chunk * 4);
+                meta[r][t][0] = __ldg(pairs);
+                meta[r][t][1] = __ldg(pairs + 1);
+            }
+        };
+        std::uint32_t column = load_column(p, first, lane), next_column = load_column(p, first + step, lane);
+#pragma unroll
+        for (int r = 0; r < kGroupPairs; ++r) fetch(first, column, r);
+        int item0 = 0; // pairs of the CTA before this block row
+        bool dead = false;
+        for (std::int64_t br = first; br < p.block_row_end && !dead; br += step) {
+            const block_row blocks = make_block_row(column);
+            column = next_column;
+            next_column = load_column(p, br + 2 * step, lane);
+            const std::int64_t row = br * 32 + cell;
+            const bool cell_valid = row >= p.row_begin && row < p.row_end;
+            // row-offset policy: the cell's offset, times the operand's power of two, for both genes of a pair
+            const __half2 row_offset2 = __float2half2_rn((row_policy && p.offsets != nullptr && cell_valid) ? __ldg(p.offsets + row) * vs : 0.0f);
+#pragma unroll
+            for (int r = 0; r < kGroupPairs; ++r) {
+                const int j = group + r * kGroups;
+                if (((blocks.pairs >> (2 * j)) & 1u) != 0u) {
+                    const int item = item0 + __popc(blocks.pairs & ((1u << (2 * j)) - 1u)), stage = item % kStages;
+                    if (warp_wait_sleeping(empty + stage, item / kStages + 1, abort_flag, 40u)) { dead = true; break; }
+#pragma unroll
+                    for (int t = 0; t < 2; ++t) {
+                        if (((blocks.blocks >> (2 * j + t)) & 1u) == 0u) continue;
+                        // per pair of codes a byte permute (code -> fp16 1024 + code), a subtraction (exact), a fused
+                        // multiply-add with the pair's {scale, offset}; genes past the matrix have scale and offset 0
+                        std::uint32_t out[4] = {0u, 0u, 0u, 0u};
+                        if (cell_valid) {
+                            const std::uint32_t lo = codes[r][t].x, hi = codes[r][t].y;
+                            std::uint32_t raw[4];
+                            if constexpr (BITS == 8) {
+                                raw[0] = __byte_perm(lo, 0x64646464u, 0x4140u);
+                                raw[1] = __byte_perm(lo, 0x64646464u, 0x4342u);
+                                raw[2] = __byte_perm(hi, 0x64646464u, 0x4140u);
+                                raw[3] = __byte_perm(hi, 0x64646464u, 0x4342u);
+                            } else {
+#pragma unroll
+                                for (int e = 0; e < 4; ++e) {
+                                    const std::uint32_t two = lo >> (8 * e); // the byte that holds the pair's two 4-bit codes
+                                    raw[e] = 0x64006400u | (two & 0xfu) | ((two & 0xf0u) << 12);
+                                }
+                            }
+                            const std::uint32_t sc[4] = {meta[r][t][0].x, meta[r][t][0].z, meta[r][t][1].x, meta[r][t][1].z};
+                            const std::uint32_t of[4] = {meta[r][t][0].y, meta[r][t][0].w, meta[r][t][1].y, meta[r][t][1].w};
+#pragma unroll
+                            for (int e = 0; e < 4; ++e) {
+                                const __half2 code2 = __hsub2(*reinterpret_cast<const __half2 *>(&raw[e]), magic);
+                                __half2 o2 = *reinterpret_cast<const __half2 *>(&of[e]);
+                                if (row_policy) o2 = __hmul2(o2, row_offset2); // the pair's {1 | 0} times the cell's offset
+                                const __half2 v = __hfma2(code2, *reinterpret_cast<const __half2 *>(&sc[e]), o2);
+                                out[e] = *reinterpret_cast<const std::uint32_t *>(&v);
+                            }
+                        }
+                        const std::uint32_t dst = smem0 + stage * kStageBytes + 2 * kATileBytes + t * kBTileBytes + (cell >> 3) * 512 + chunk * 128 + (cell & 7) * 16;
+                        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst), "r"(out[0]), "r"(out[1]), "r"(out[2]), "r"(out[3]) : "memory");
+                    }
+                    fence_async_proxy(); // written with ordinary stores, read by the MMAs
+                    __syncwarp();
+                    if (lane == 0) bar_arrive(smem_addr(full + stage));
+                }
+            }
+#pragma unroll
+            for (int r = 0; r < kGroupPairs; ++r) fetch(br + step, column, r);
+            item0 += __popc(blocks.pairs);
+        }
+    } else if (warp < kEpilogueWarps + kDecodeWarps + H) {
+        // ================= MMA issuers: warp h issues the MMAs of output columns [128 h, 128 h + 128) =================
+        const int h = warp - kEpilogueWarps - kDecodeWarps;
+        const std::uint64_t desc0 = smem_desc(smem0);
+        const std::uint32_t lo0 = static_cast<std::uint32_t>(desc0), hi = static_cast<std::uint32_t>(desc0 >> 32);
+        int use = 0, stage = 0, phase = 0;
+        bool dead = false;
+        std::uint32_t column = load_column(p, first, lane);
+        for (std::int64_t br = first; br < p.block_row_end && !dead; br += step, ++use) {
+            const int buf = use & 1;
+            const block_row blocks = make_block_row(column);
+            column = load_column(p, br + step, lane);
+            if (warp_wait(acc_empty + buf, (use >> 1) + 1, abort_flag)) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const std::uint32_t d = tmem_base + buf * (H * 32) + h * 32;
+            std::uint32_t accumulate = 0; // the block row's first MMA overwrites the accumulators
+            for (unsigned todo = blocks.pairs; todo != 0u; todo &= todo - 1u) {
+                const unsigned present = blocks.blocks >> (__ffs(static_cast<int>(todo)) - 1);
+                dead = warp_wait(full + stage, phase, abort_flag);
+                if (dead) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                if (elect_one()) {
+                    const std::uint32_t a = lo0 + ((stage * kStageBytes + h * 8192) >> 4), b = lo0 + ((stage * kStageBytes + 2 * kATileBytes) >> 4);
+                    if ((present & 1u) != 0u) {
+                        mma_f16(d, a, b, hi, accumulate);
+                        mma_f16(d, a + 16, b + 16, hi, 1u);
+                    }
+                    if ((present & 2u) != 0u) {
+                        mma_f16(d, a + (kATileBytes >> 4), b + (kBTileBytes >> 4), hi, accumulate | (present & 1u));
+                        mma_f16(d, a + (kATileBytes >> 4) + 16, b + (kBTileBytes >> 4) + 16, hi, 1u);
+                    }
+                    mma_commit(smem_addr(empty + stage));
+                }
+                accumulate = 1;
+                if (++stage == kStages) { stage = 0; phase ^= 1; }
+            }
+            if (!dead && elect_one()) {
+                if (h == 0) row_has_blocks[buf] = blocks.blocks != 0u ? 1 : 0;
+                mma_commit(smem_addr(acc_full + buf)); // accumulators complete (or nothing was issued)
+            }
+        }
+    } else {
+        // ================= loaders: a block's slice of W^T is one contiguous copy, already in operand layout; loader l takes the
+        // pairs whose number in the CTA's walk is l modulo kLoaders =================
+        const int loader = warp - kEpilogueWarps - kDecodeWarps - H;
+        int number = 0, stage = loader, phase = 1, issued = 0;
+        bool dead = false; // the elected lane: a wait was given up
+        std::uint32_t column = load_column(p, first, lane);
+        for (std::int64_t br = first; br < p.block_row_end; br += step) {
+            const block_row blocks = make_block_row(column);
+            column = load_column(p, br + step, lane);
+            for (unsigned todo = blocks.pairs; todo != 0u; todo &= todo - 1u, ++number) {
+                if (number % kLoaders != loader) continue;
+                const int even = __ffs(static_cast<int>(todo)) - 1;
+                std::uint32_t bc[2];
+#pragma unroll
+                for (int t = 0; t < 2; ++t) bc[t] = __shfl_sync(0xffffffffu, blocks.column, even + t);
+                if (elect_one() && !dead) {
+                    dead = bar_wait(smem_addr(empty + stage), static_cast<std::uint32_t>(phase), abort_flag);
+                    if (!dead) { // no new copies once a wait of the CTA has run out
+                        bar_arrive_expect_tx(smem_addr(full + stage), ((bc[0] != 0xffffffffu) + (bc[1] != 0xffffffffu)) * kATileBytes);
+#pragma unroll
+                        for (int t = 0; t < 2; ++t)
+                            if (bc[t] != 0xffffffffu)
+                                bulk_copy_g2s(smem0 + stage * kStageBytes + t * kATileBytes, p.wt + static_cast<std::int64_t>(bc[t]) * (H * 128 * 32), kATileBytes,
+                                              smem_addr(full + stage));
+                        ++issued;
+                    }
+                }
+                stage += kLoaders;
+                if (stage >= kStages) { stage = loader; phase ^= 1; }
+            }
+        }
+        // The copies still in flight land before the CTA gives up its shared memory.  Their barriers may lack the decode
+        // group's arrivals, so there is nothing to wait on; a copy takes microseconds, the bound of a wait was milliseconds.
+        if (dead) __nanosleep(1000000u);
     }
 
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -456,15 +456,14 @@ __global__ void __launch_bounds__(kThreads, 2) qbell_tcgen05_kernel(const tc_par
     if (tid == 0 && *abort_flag != 0 && p.status != nullptr) atomicExch(p.status, 1);
 }
 
-constexpr std::size_t kSmemBytes = kStages * kStageBytes + 2 * kCodesStageBytes + 2 * kMetaStageBytes + (2 * kStages + 4) * sizeof(std::uint64_t) + 32;
-
 template<int BITS, int H>
 cb200_status launch(const tc_params &p, int sm_count, cudaStream_t stream) {
-    CB200_CUDA_OK(cudaFuncSetAttribute(qbell_tcgen05_kernel<BITS, H>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       static_cast<int>(kSmemBytes)));
+    constexpr std::size_t smem = stages_of(H) * stage_bytes(H) + (2 * stages_of(H) + 4) * sizeof(std::uint64_t) + 32;
+    static_assert(smem <= 232448, "shared memory budget");
+    CB200_CUDA_OK(cudaFuncSetAttribute(qbell_tcgen05_kernel<BITS, H>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
     const std::int64_t block_rows = p.block_row_end - p.block_row_begin;
-    const unsigned grid = static_cast<unsigned>(block_rows < 2ll * sm_count ? block_rows : 2ll * sm_count);
-    qbell_tcgen05_kernel<BITS, H><<<grid, kThreads, kSmemBytes, stream>>>(p);
+    const unsigned grid = static_cast<unsigned>(std::min<std::int64_t>(block_rows, sm_count));
+    qbell_tcgen05_kernel<BITS, H><<<grid, threads_of(H), smem, stream>>>(p);
     count_launch();
     CB200_CUDA_OK(cudaGetLastError());
     return CB200_STATUS_SUCCESS;
@@ -479,7 +478,7 @@ cb200_status launch_qbell_tcgen05(const qbell_view &x, const dense_args &d, std:
     if (x.block_size != 32 || (d.n != 128 && d.n != 256) || d.dense_dtype != CB200_DTYPE_BF16) return CB200_STATUS_SUCCESS;
     if (x.bits != 8 && x.bits != 4) return CB200_STATUS_SUCCESS;
     if (x.ell_cols <= 0 || x.ell_cols % 32 != 0 || x.ell_cols / 32 > kMaxWidth) return CB200_STATUS_SUCCESS;
-    // staging copies move 16 bytes at a time
+    // the decode warps read up to 8 bytes at a time
     if (x.row_stride_bytes % 16 != 0 || reinterpret_cast<std::uintptr_t>(x.packed) % 16u != 0u) return CB200_STATUS_SUCCESS;
     if (reinterpret_cast<std::uintptr_t>(x.scales) % 16u != 0u || reinterpret_cast<std::uintptr_t>(x.offsets) % 16u != 0u) return CB200_STATUS_SUCCESS;
     if (workspace == nullptr || workspace_bytes < qbell_tcgen05_workspace_bytes(x.cols, d.n)) return CB200_STATUS_SUCCESS;
