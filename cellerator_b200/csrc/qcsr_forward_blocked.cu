@@ -273,7 +273,7 @@ __global__ void __launch_bounds__(kThreads, 1) qcsr_fwd_blocked_kernel(const blo
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
     unsigned char *scratch_slot = reinterpret_cast<unsigned char *>(tmem_slot + 2);
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = warp_of_block(), lane = tid & 31;
     const std::uint32_t smem0 = smem_addr(smem);
     const std::uint32_t wstage0 = smem0 + 2 * kABufBytes;
     const std::uint32_t chunk0 = wstage0 + STAGES * REC;
@@ -416,7 +416,7 @@ __global__ void __launch_bounds__(kThreads, 1) qcsr_fwd_blocked_kernel(const blo
                 bar_wait(smem_addr(w_full + s), static_cast<std::uint32_t>((q / STAGES) & 1), abort_flag);
                 bar_wait(smem_addr(a_full + b), static_cast<std::uint32_t>((q >> 1) & 1), abort_flag);
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                if (lane == 0) {
+                if (elect_one()) {
                     const std::uint32_t a_tile = smem0 + b * kABufBytes;
                     const std::uint32_t b_tile = wstage0 + s * REC;
 #pragma unroll
@@ -443,7 +443,7 @@ __global__ void __launch_bounds__(kThreads, 1) qcsr_fwd_blocked_kernel(const blo
         // kChunkLoaders); each of them walks all segments and issues only its own chunks.
         const int role = warp - kProducerWarps - 1; // 0: W slices, 1..kChunkLoaders: entry chunks
         if (role == 0) {
-            if (lane == 0) {
+            if (elect_one()) {
                 long long q = 0;
                 for (int g = 0; g < my_units; ++g) {
                     const window_unit unit = unit_of(g);
@@ -470,7 +470,7 @@ __global__ void __launch_bounds__(kThreads, 1) qcsr_fwd_blocked_kernel(const blo
                         std::int64_t at = lo;
                         do {
                             const int count = static_cast<int>(min(static_cast<std::int64_t>(kChunkEntries), hi - at));
-                            if (lane == 0 && qc % kChunkLoaders == mine_mod) {
+                            if (qc % kChunkLoaders == mine_mod && elect_one()) {
                                 const int cs = static_cast<int>(qc % CS);
                                 bar_wait(smem_addr(c_empty + cs), static_cast<std::uint32_t>(((qc / CS) & 1) ^ 1), abort_flag);
                                 chunk_meta[cs] = (count << 1) | (at + count >= hi ? 1 : 0);
@@ -583,7 +583,7 @@ __global__ void __launch_bounds__(kThreads2, 1) qcsr_fwd_blocked2_kernel(const b
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
     unsigned char *scratch_slot = reinterpret_cast<unsigned char *>(tmem_slot + 2);
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = warp_of_block(), lane = tid & 31;
     const int limit = TEST_HOOK ? p.poll_limit : kPollLimit;
     const std::uint32_t smem0 = smem_addr(smem);
     const std::uint32_t wstage0 = smem0 + 2 * kABufBytes;
@@ -749,6 +749,8 @@ __global__ void __launch_bounds__(kThreads2, 1) qcsr_fwd_blocked2_kernel(const b
                 const int s = static_cast<int>(q % STAGES);
                 bar_wait(smem_addr(a_full + b), static_cast<std::uint32_t>((q >> 1) & 1), abort_flag, limit); // tile and W stage
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                // (not under elect_one: MMAs issued back to back take the operand reads' bandwidth from the scatter group's stores
+                // in bursts, 575 against 542 us on an eighth of that matrix)
                 if (lane == 0) {
                     const std::uint32_t a_tile = smem0 + b * kABufBytes + sb * kSubBlockBytes;
                     const std::uint32_t b_tile = wstage0 + s * WREC;
@@ -771,7 +773,7 @@ __global__ void __launch_bounds__(kThreads2, 1) qcsr_fwd_blocked2_kernel(const b
         __syncwarp();
     } else if (warp == kProducerWarps + kSubBlocks) {
         // ================= W loader =================
-        if (lane == 0 && !(TEST_HOOK && p.withhold_w != 0)) {
+        if (elect_one() && !(TEST_HOOK && p.withhold_w != 0)) {
             long long q = 0;
             bool dead = false;
             for (int g = 0; g < my_units && !dead; ++g) {
@@ -793,7 +795,7 @@ __global__ void __launch_bounds__(kThreads2, 1) qcsr_fwd_blocked2_kernel(const b
         // ================= entry chunks: window q goes to the ring of scatter group q & 1 =================
         long long q = 0;
         long long qc0 = 0, qc1 = 0; // chunks issued into each ring
-        bool dead = false; // lane 0: a wait was given up, no copy is issued any more (the loops run out empty)
+        bool dead = false; // the elected lane: a wait was given up, no copy is issued any more (the loops run out empty)
         for (int gi = 0; gi < my_units; ++gi) {
             const window_unit unit = unit_of(gi);
             const std::int64_t seg0 = static_cast<std::int64_t>(unit.group) * p.windows;
@@ -807,11 +809,11 @@ __global__ void __launch_bounds__(kThreads2, 1) qcsr_fwd_blocked2_kernel(const b
                     do {
                         const int count = static_cast<int>(min(static_cast<std::int64_t>(kChunk2Entries), hi - at));
                         const long long mine = ring == 0 ? qc0 : qc1;
-                        if (lane == 0 && !dead) {
+                        if (elect_one() && !dead) {
                             const int cs = ring * kRing2 + static_cast<int>(mine % kRing2);
                             dead = bar_wait(smem_addr(c_empty + cs), static_cast<std::uint32_t>(((mine / kRing2) & 1) ^ 1), abort_flag, limit);
                         }
-                        if (lane == 0 && !dead) {
+                        if (elect_one() && !dead) {
                             const int cs = ring * kRing2 + static_cast<int>(mine % kRing2);
                             chunk_meta[cs] = (count << 1) | (at + count >= hi ? 1 : 0);
                             if (count > 0) {
@@ -823,7 +825,7 @@ __global__ void __launch_bounds__(kThreads2, 1) qcsr_fwd_blocked2_kernel(const b
                             }
                         }
                         at += count;
-                        if (!dead) { // lane 0's counters stop with its last issued chunk (the drain below needs them)
+                        if (!dead) { // the elected lane's counters stop with its last issued chunk (the drain below needs them)
                             if (ring == 0) ++qc0;
                             else ++qc1;
                         }
@@ -832,7 +834,7 @@ __global__ void __launch_bounds__(kThreads2, 1) qcsr_fwd_blocked2_kernel(const b
             }
         }
         // after an abort: let the chunk copies still in flight land (the last one issued into each stage of both rings)
-        if (dead && lane == 0) {
+        if (elect_one() && dead) {
             for (int ring = 0; ring < 2; ++ring) {
                 const long long issued = ring == 0 ? qc0 : qc1;
                 for (long long last = issued - 1; last >= 0 && last > issued - 1 - kRing2; --last)

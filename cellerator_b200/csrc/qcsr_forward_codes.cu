@@ -217,7 +217,7 @@ __global__ void __launch_bounds__(kCodesThreads, 1) qcsr_fwd_codes_kernel(const 
     std::uint32_t *tmem_slot = reinterpret_cast<std::uint32_t *>(mma_drain + kCodeIssuers);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = warp_of_block(), lane = tid & 31;
     const std::uint32_t bstage0 = smem_addr(smem);
     unsigned char *cstage0 = smem + SB * WREC;
 
@@ -336,12 +336,14 @@ __global__ void __launch_bounds__(kCodesThreads, 1) qcsr_fwd_codes_kernel(const 
         bool dead = false;
         for (int g = 0; g < my_units && !dead; ++g) {
             const window_unit unit = unit_of(g);
-            if (bar_wait(smem_addr(acc_empty), static_cast<std::uint32_t>((g & 1) ^ 1), abort_flag)) break;
+            if (__any_sync(0xffffffffu, bar_wait(smem_addr(acc_empty), static_cast<std::uint32_t>((g & 1) ^ 1), abort_flag))) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             for (int w = unit.w0; w < unit.w1; ++w) {
-                if (bar_wait(smem_addr(b_full + s), pb, abort_flag) || bar_wait(smem_addr(a_full + sa), pa, abort_flag)) { dead = true; break; }
+                // (the warp leaves as one: the election below needs all its lanes)
+                dead = __any_sync(0xffffffffu, bar_wait(smem_addr(b_full + s), pb, abort_flag) || bar_wait(smem_addr(a_full + sa), pa, abort_flag)) != 0;
+                if (dead) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                if (lane == 0) {
+                if (elect_one()) {
                     const std::uint32_t a_col = tmem_base + kOperandCol0 + sa * kOperandCols;
                     const std::uint32_t b_lo = b_lo0 + static_cast<std::uint32_t>((s * WREC) >> 4);
                     const std::uint32_t fresh = w != unit.w0 ? 1u : 0u; // the unit's first MMAs overwrite the accumulators
@@ -358,13 +360,13 @@ __global__ void __launch_bounds__(kCodesThreads, 1) qcsr_fwd_codes_kernel(const 
                 if (++s == SB) { s = 0; pb ^= 1u; }
             }
         }
-        if (*abort_flag != 0 && lane == 0) { // gave up: let the MMAs in flight finish before tensor memory is freed
+        if (elect_one() && *abort_flag != 0) { // gave up: let the MMAs in flight finish before tensor memory is freed
             mma_commit(smem_addr(mma_drain + sb));
             bar_wait_drain(smem_addr(mma_drain + sb), 0u);
         }
     } else if (warp == kEpilogueWarps + kCodeIssuers) {
         // ================= W loader =================
-        if (lane == 0) {
+        if (elect_one()) {
             int s = 0, issued = 0;
             std::uint32_t pb = 1;
             bool dead = false;
@@ -383,7 +385,7 @@ __global__ void __launch_bounds__(kCodesThreads, 1) qcsr_fwd_codes_kernel(const 
         }
     } else if (warp == kEpilogueWarps + kCodeIssuers + 1) {
         // ================= code stages =================
-        if (lane == 0) {
+        if (elect_one()) {
             int s = 0, issued = 0;
             std::uint32_t pc = 1;
             bool dead = false;

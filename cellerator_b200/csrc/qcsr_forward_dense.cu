@@ -120,7 +120,7 @@ __global__ void __launch_bounds__(kDenseThreads, 1) qcsr_fwd_dense_kernel(const 
     std::uint32_t *tmem_slot = reinterpret_cast<std::uint32_t *>(acc_empty + 2);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = warp_of_block(), lane = tid & 31;
     const std::uint32_t smem0 = smem_addr(smem);
     const std::uint32_t bstage0 = smem0 + SA * kDenseStageBytes;
 
@@ -193,7 +193,7 @@ __global__ void __launch_bounds__(kDenseThreads, 1) qcsr_fwd_dense_kernel(const 
                     const int sa = static_cast<int>(qa % SA);
                     bar_wait(smem_addr(a_full + sa), static_cast<std::uint32_t>((qa / SA) & 1), abort_flag);
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    if (lane == 0) {
+                    if (elect_one()) {
                         const std::uint32_t a_stage = smem0 + sa * kDenseStageBytes;
 #pragma unroll
                         for (int kk = 0; kk < 4; ++kk) {
@@ -215,7 +215,7 @@ __global__ void __launch_bounds__(kDenseThreads, 1) qcsr_fwd_dense_kernel(const 
         }
     } else if (warp == kEpilogueWarps + 1) {
         // ================= W loader =================
-        if (lane == 0) {
+        if (elect_one()) {
             long long q = 0;
             for (int g = 0; g < my_units; ++g) {
                 const window_unit unit = unit_of(g);
@@ -229,7 +229,7 @@ __global__ void __launch_bounds__(kDenseThreads, 1) qcsr_fwd_dense_kernel(const 
         }
     } else {
         // ================= A loaders: half-stages in turn =================
-        if (lane == 0) {
+        if (elect_one()) {
             long long q = 0; // half-stages of this CTA; every loader counts all of them and issues its own
             for (int g = 0; g < my_units; ++g) {
                 const window_unit unit = unit_of(g);

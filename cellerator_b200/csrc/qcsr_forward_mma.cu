@@ -157,7 +157,7 @@ __global__ void __launch_bounds__(kThreads, 1) qcsr_fwd_mma_kernel(const mma_par
     std::uint32_t *tmem_slot = reinterpret_cast<std::uint32_t *>(acc_empty + 1);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = warp_of_block(), lane = tid & 31;
     const std::uint32_t smem0 = smem_addr(smem);
     const std::uint32_t wstage0 = smem0 + 2 * kABufBytes;
     const std::uint32_t ring0 = wstage0 + STAGES * REC;
@@ -355,7 +355,7 @@ __global__ void __launch_bounds__(kThreads, 1) qcsr_fwd_mma_kernel(const mma_par
                 bar_wait(smem_addr(w_full + s), static_cast<std::uint32_t>((q / STAGES) & 1), abort_flag);
                 bar_wait(smem_addr(a_full + b), static_cast<std::uint32_t>((q >> 1) & 1), abort_flag);
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                if (lane == 0) {
+                if (elect_one()) {
                     const std::uint32_t a_tile = smem0 + b * kABufBytes;
                     const std::uint32_t b_tile = wstage0 + s * REC;
 #pragma unroll
@@ -373,7 +373,7 @@ __global__ void __launch_bounds__(kThreads, 1) qcsr_fwd_mma_kernel(const mma_par
                 __syncwarp();
             }
         }
-    } else if (lane == 0) {
+    } else if (elect_one()) {
         // ================= W loader =================
         const long long total = my_groups * p.windows;
         for (long long q = 0; q < total; ++q) {
