@@ -255,8 +255,9 @@ struct gather_params {
     int restrict_rows; // the launch covers a proper sub-range of the rows
     int aligned;       // G rows can be read with one vector load per lane
     float alpha, beta;
-    unsigned *queue;   // next gene to hand out
-    const std::int32_t *gene_order; // position in the queue -> gene (long genes first); null: natural order
+    unsigned *queue;   // [2] next long gene, next short gene to hand out
+    const std::int32_t *gene_order; // genes by descending entry count
+    std::int64_t long_genes;        // the first so many of them are a CTA's work each, the others a warp's
 };
 
 // VEC consecutive floats of a row of G; ALIGNED: one vector load
@@ -293,93 +294,110 @@ __device__ __forceinline__ std::int64_t gather_lower_bound(const std::int32_t *r
     return lo;
 }
 
+// A gene's entries [lo, hi) within the launch's rows, its scale and zero-point.
+struct gather_gene {
+    std::int64_t gene, lo, hi;
+    float scale, offset;
+};
+__device__ __forceinline__ gather_gene gather_gene_at(const gather_params &p, std::int64_t position, bool row_policy) {
+    gather_gene e;
+    e.gene = __ldg(p.gene_order + position);
+    e.lo = __ldg(p.col_ptr + e.gene);
+    e.hi = __ldg(p.col_ptr + e.gene + 1);
+    if (p.restrict_rows) {
+        e.lo = gather_lower_bound(p.row_idx, e.lo, e.hi, p.row_begin);
+        e.hi = gather_lower_bound(p.row_idx, e.lo, e.hi, p.row_end);
+    }
+    e.scale = p.scales != nullptr ? __ldg(p.scales + e.gene) : 1.0f;
+    e.offset = (!row_policy && p.offsets != nullptr) ? __ldg(p.offsets + e.gene) : 0.0f;
+    return e;
+}
+// acc += the entries [begin, end), in order
+template<int VEC, bool ALIGNED, bool PACKED>
+__device__ __forceinline__ void gather_add(const gather_params &p, const gather_gene &e, std::int64_t begin, std::int64_t end, const char *g_lane,
+                                           std::uint32_t g_row_bytes, bool row_policy, int lane, float (&acc)[VEC]) {
+    for (std::int64_t base = begin; base < end; base += 32) {
+        const int count = static_cast<int>(min(static_cast<std::int64_t>(32), end - base));
+        int row = 0;
+        float value = 0.0f;
+        if (lane < count) {
+            row = __ldg(p.row_idx + base + lane);
+            const unsigned code = __ldg(p.codes + base + lane);
+            if constexpr (PACKED) {
+                row = static_cast<int>((static_cast<unsigned>(row) << 8) | code);
+            } else {
+                const float offset = row_policy ? (p.offsets != nullptr ? __ldg(p.offsets + row) : 0.0f) : e.offset;
+                value = fmaf(static_cast<float>(code), e.scale, offset);
+            }
+        }
+        const auto fetch = [&](int j, float (&gv)[VEC], float &v) {
+            unsigned r = static_cast<unsigned>(__shfl_sync(0xffffffffu, row, j));
+            if constexpr (PACKED) {
+                v = fmaf(low_byte_to_float(r), e.scale, e.offset);
+                r >>= 8;
+            } else {
+                v = __shfl_sync(0xffffffffu, value, j);
+            }
+            gather_load<VEC, ALIGNED>(reinterpret_cast<const float *>(g_lane + static_cast<std::uint64_t>(r) * g_row_bytes), gv);
+        };
+        if (count == 32) {
+#pragma unroll
+            for (int j0 = 0; j0 < 32; j0 += 8) { // eight rows of G in flight, then their FMAs in order
+                float gv[8][VEC], vv[8];
+#pragma unroll
+                for (int u = 0; u < 8; ++u) fetch(j0 + u, gv[u], vv[u]);
+#pragma unroll
+                for (int u = 0; u < 8; ++u)
+#pragma unroll
+                    for (int k = 0; k < VEC; ++k) acc[k] = fmaf(vv[u], gv[u][k], acc[k]);
+            }
+        } else {
+            for (int j0 = 0; j0 < count; j0 += 8) { // the places behind the end fetch row 0 and add nothing
+                float gv[8][VEC], vv[8];
+#pragma unroll
+                for (int u = 0; u < 8; ++u) fetch(j0 + u, gv[u], vv[u]);
+#pragma unroll
+                for (int u = 0; u < 8; ++u)
+                    if (j0 + u < count) {
+#pragma unroll
+                        for (int k = 0; k < VEC; ++k) acc[k] = fmaf(vv[u], gv[u][k], acc[k]);
+                    }
+            }
+        }
+    }
+}
+
 // N == 32 * VEC; lane l owns the output columns [l * VEC, l * VEC + VEC).  The inner loop is kept to
 // two shuffles, one 32 x 32 -> 64-bit multiply-add for the address, one load and VEC FMAs per entry:
 // the kernel issues an instruction in most cycles, so every instruction per entry counts.
-// What bounds it then is the load/store unit's data pipe, which also carries the shuffles: 256 B of G
-// and two 128 B shuffles per entry at N = 64.  PACKED (per-gene offsets, cells below 2^24) halves the
-// shuffles: a lane hands out (cell << 8 | code) and every lane decodes the value itself -- the same
+// What bounds it then is the way from L2: a row of G per entry, 256 B at N = 64, 17 TB/s (180 M entries: 3,018 us with the
+// last entries of a chunk fetched one by one, 2,640 with them in groups of eight like the others; with tiles of G in shared
+// memory and running sums per gene and tile 4,081).  PACKED (per-gene offsets, cells
+// below 2^24) halves the shuffles: a lane hands out (cell << 8 | code) and every lane decodes the value itself -- the same
 // fused multiply-add, so the same bits.
+// Summation order of a gene: its entries in chunks of 256, chunk c into partial sum c mod 8, the partial sums in order.  A
+// gene of more than eight chunks is a CTA's work, a warp per partial sum.  A shorter one would leave warps of a CTA without a
+// chunk (and its last chunk is as often a few entries as 256): it is one warp's work, partial sum after partial sum.
+// Launch bounds: three CTAs per SM at N = 128 (647 against 557 us); elsewhere the compiler's own choice of four and five is the best.
 template<int VEC, bool ALIGNED, bool PACKED>
-__global__ void __launch_bounds__(kGatherWarps * 32) qcsr_transpose_gather_kernel(const gather_params p) {
+__global__ void __launch_bounds__(kGatherWarps * 32, VEC == 4 ? 3 : 0) qcsr_transpose_gather_kernel(const gather_params p) {
     __shared__ float part[kGatherWarps][32 * VEC];
     __shared__ unsigned next_gene;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const bool row_policy = p.policy == CB200_DECODE_COLUMN_SCALE_ROW_OFFSET;
     const std::uint32_t g_row_bytes = static_cast<std::uint32_t>(p.g_ld) * 4u; // the launcher checks it fits
+    const char *g_lane = reinterpret_cast<const char *>(p.g + lane * VEC);
     for (;;) {
         if (threadIdx.x == 0) next_gene = atomicAdd(p.queue, 1u);
         __syncthreads();
-        if (next_gene >= p.cols) return;
-        const std::int64_t gene = p.gene_order != nullptr ? __ldg(p.gene_order + next_gene) : static_cast<std::int64_t>(next_gene);
-        std::int64_t lo = __ldg(p.col_ptr + gene), hi = __ldg(p.col_ptr + gene + 1);
-        if (p.restrict_rows) {
-            lo = gather_lower_bound(p.row_idx, lo, hi, p.row_begin);
-            hi = gather_lower_bound(p.row_idx, lo, hi, p.row_end);
-        }
-        const float scale = p.scales != nullptr ? __ldg(p.scales + gene) : 1.0f;
-        const float gene_offset = (!row_policy && p.offsets != nullptr) ? __ldg(p.offsets + gene) : 0.0f;
+        if (next_gene >= p.long_genes) break;
+        const gather_gene e = gather_gene_at(p, next_gene, row_policy);
         float acc[VEC];
 #pragma unroll
         for (int k = 0; k < VEC; ++k) acc[k] = 0.0f;
-        const char *g_lane = reinterpret_cast<const char *>(p.g + lane * VEC);
-        for (std::int64_t chunk = lo + static_cast<std::int64_t>(warp) * kGatherChunk; chunk < hi;
-             chunk += static_cast<std::int64_t>(kGatherWarps) * kGatherChunk) {
-            const std::int64_t chunk_end = min(hi, chunk + kGatherChunk);
-            for (std::int64_t base = chunk; base < chunk_end; base += 32) {
-                const int count = static_cast<int>(min(static_cast<std::int64_t>(32), chunk_end - base));
-                int row = 0;
-                float value = 0.0f;
-                if (lane < count) {
-                    row = __ldg(p.row_idx + base + lane);
-                    const unsigned code = __ldg(p.codes + base + lane);
-                    if constexpr (PACKED) {
-                        row = static_cast<int>((static_cast<unsigned>(row) << 8) | code);
-                    } else {
-                        const float offset = row_policy ? (p.offsets != nullptr ? __ldg(p.offsets + row) : 0.0f) : gene_offset;
-                        value = fmaf(static_cast<float>(code), scale, offset);
-                    }
-                }
-                if (count == 32) {
-#pragma unroll
-                    for (int j0 = 0; j0 < 32; j0 += 8) { // eight rows of G in flight, then their FMAs in order
-                        float gv[8][VEC], vv[8];
-#pragma unroll
-                        for (int u = 0; u < 8; ++u) {
-                            unsigned r = static_cast<unsigned>(__shfl_sync(0xffffffffu, row, j0 + u));
-                            if constexpr (PACKED) {
-                                vv[u] = fmaf(low_byte_to_float(r), scale, gene_offset);
-                                r >>= 8;
-                            } else {
-                                vv[u] = __shfl_sync(0xffffffffu, value, j0 + u);
-                            }
-                            gather_load<VEC, ALIGNED>(
-                                reinterpret_cast<const float *>(g_lane + static_cast<std::uint64_t>(r) * g_row_bytes), gv[u]);
-                        }
-#pragma unroll
-                        for (int u = 0; u < 8; ++u)
-#pragma unroll
-                            for (int k = 0; k < VEC; ++k) acc[k] = fmaf(vv[u], gv[u][k], acc[k]);
-                    }
-                } else {
-                    for (int j = 0; j < count; ++j) {
-                        unsigned r = static_cast<unsigned>(__shfl_sync(0xffffffffu, row, j));
-                        float v;
-                        if constexpr (PACKED) {
-                            v = fmaf(low_byte_to_float(r), scale, gene_offset);
-                            r >>= 8;
-                        } else {
-                            v = __shfl_sync(0xffffffffu, value, j);
-                        }
-                        float gv[VEC];
-                        gather_load<VEC, ALIGNED>(
-                            reinterpret_cast<const float *>(g_lane + static_cast<std::uint64_t>(r) * g_row_bytes), gv);
-#pragma unroll
-                        for (int k = 0; k < VEC; ++k) acc[k] = fmaf(v, gv[k], acc[k]);
-                    }
-                }
-            }
-        }
+        for (std::int64_t chunk = e.lo + static_cast<std::int64_t>(warp) * kGatherChunk; chunk < e.hi;
+             chunk += static_cast<std::int64_t>(kGatherWarps) * kGatherChunk)
+            gather_add<VEC, ALIGNED, PACKED>(p, e, chunk, min(e.hi, chunk + kGatherChunk), g_lane, g_row_bytes, row_policy, lane, acc);
 #pragma unroll
         for (int k = 0; k < VEC; ++k) part[warp][lane * VEC + k] = acc[k];
         __syncthreads();
@@ -387,10 +405,33 @@ __global__ void __launch_bounds__(kGatherWarps * 32) qcsr_transpose_gather_kerne
             float sum = part[0][threadIdx.x];
 #pragma unroll
             for (int w = 1; w < kGatherWarps; ++w) sum = sum + part[w][threadIdx.x];
-            float *dst = p.out + gene * p.out_ld + threadIdx.x;
+            float *dst = p.out + e.gene * p.out_ld + threadIdx.x;
             float result = p.alpha * sum;
             if (p.beta != 0.0f) result = fmaf(p.beta, *dst, result);
             *dst = result;
+        }
+    }
+    for (;;) {
+        unsigned position = 0u;
+        if (lane == 0) position = atomicAdd(p.queue + 1, 1u);
+        position = __shfl_sync(0xffffffffu, position, 0);
+        if (p.long_genes + position >= p.cols) return;
+        const gather_gene e = gather_gene_at(p, p.long_genes + position, row_policy);
+        float sum[VEC], acc[VEC];
+        for (int w = 0; w < kGatherWarps; ++w) { // partial sums without entries are added, too: the bits are those of eight warps
+            const std::int64_t begin = min(e.hi, e.lo + w * kGatherChunk);
+#pragma unroll
+            for (int k = 0; k < VEC; ++k) acc[k] = 0.0f;
+            gather_add<VEC, ALIGNED, PACKED>(p, e, begin, min(e.hi, begin + kGatherChunk), g_lane, g_row_bytes, row_policy, lane, acc);
+#pragma unroll
+            for (int k = 0; k < VEC; ++k) sum[k] = w == 0 ? acc[k] : sum[k] + acc[k];
+        }
+        float *dst = p.out + e.gene * p.out_ld + lane * VEC;
+#pragma unroll
+        for (int k = 0; k < VEC; ++k) {
+            float result = p.alpha * sum[k];
+            if (p.beta != 0.0f) result = fmaf(p.beta, dst[k], result);
+            dst[k] = result;
         }
     }
 }
@@ -498,6 +539,11 @@ cb200_status build_gene_major_layout(const qcsr_view &x, device_arena &arena, cu
         return ptr[static_cast<std::size_t>(a) + 1u] - ptr[static_cast<std::size_t>(a)] >
                ptr[static_cast<std::size_t>(b) + 1u] - ptr[static_cast<std::size_t>(b)];
     });
+    out->long_genes = std::partition_point(order.begin(), order.end(), [&](std::int32_t c) {
+                          return ptr[static_cast<std::size_t>(c) + 1u] - ptr[static_cast<std::size_t>(c)] > kGatherWarps * kGatherChunk;
+                      }) - order.begin();
+    for (std::int64_t i = out->long_genes; i < x.cols; ++i)
+        out->short_entries += ptr[static_cast<std::size_t>(order[static_cast<std::size_t>(i)]) + 1u] - ptr[static_cast<std::size_t>(order[static_cast<std::size_t>(i)])];
     err = cudaMemcpyAsync(out->gene_order, order.data(), order.size() * sizeof(std::int32_t), cudaMemcpyHostToDevice, stream);
     if (err == cudaSuccess) err = cudaStreamSynchronize(stream);
     if (err != cudaSuccess) return give_up(fail(CB200_STATUS_CUDA_ERROR, "gene-major copy: %s", cudaGetErrorString(err)));
@@ -506,6 +552,22 @@ cb200_status build_gene_major_layout(const qcsr_view &x, device_arena &arena, cu
     out->src_row_ptr = x.row_ptr; out->src_col_idx = x.col_idx; out->src_packed = x.packed;
     return CB200_STATUS_SUCCESS;
 }
+
+namespace {
+// Genes of up to eight chunks: a warp each, or a CTA each?  A CTA per gene leaves warps without a chunk, a warp per gene has the
+// whole gene as one chain (eight rows of G in flight, about 0.08 us an entry).  With four genes for every resident warp only
+// the idle warps count, and eight chunks' worth of entries keeps a CTA busy; with fewer, the two chains are compared: the gene's
+// times the rounds of warps, and about ten microseconds per round of CTAs (120 entries of a warp's chain).
+// 33,538 genes x 64: 5,000 cells 551 -> 147 us, 20,000 cells 772 -> 531 us; 4,000 genes of 600 entries 80 -> 54, but of 1,440
+// entries 95 -> 136 and 2,000 genes of 900 52 -> 71, which stay with CTAs.
+bool genes_by_warp(const gene_major_layout &layout, std::int64_t cols, int sm_count) {
+    const std::int64_t genes = cols - layout.long_genes, warps = 32ll * sm_count;
+    if (genes <= 0) return false;
+    const std::int64_t mean = layout.short_entries / genes;
+    if (genes >= 4 * warps) return mean < 1800;
+    return mean * ((genes + warps - 1) / warps) < 120 * ((8 * genes + warps - 1) / warps);
+}
+} // namespace
 
 bool qcsr_transpose_gather_shape_ok(std::int64_t n) { return n == 32 || n == 64 || n == 128; }
 std::uint64_t qcsr_transpose_gather_workspace_bytes() { return 256u; }
@@ -534,6 +596,7 @@ cb200_status launch_qcsr_transpose_gather(const qcsr_view &x, const dense_args &
     // stays 0); the gene queue is the word at byte 64
     p.queue = static_cast<unsigned *>(workspace) + 16;
     p.gene_order = layout.gene_order;
+    p.long_genes = genes_by_warp(layout, x.cols, sm_count) ? layout.long_genes : x.cols;
     CB200_CUDA_OK(cudaMemsetAsync(workspace, 0, 128, stream));
     const unsigned grid = static_cast<unsigned>(std::min<std::int64_t>(x.cols, static_cast<std::int64_t>(sm_count) * 8));
     if (d.dense_ld < 0 || d.dense_ld >= (std::int64_t{1} << 30))

@@ -214,6 +214,8 @@ struct gene_major_layout {
     std::int32_t *row_idx = nullptr;  // nnz
     std::uint8_t *codes = nullptr;    // nnz
     std::int32_t *gene_order = nullptr; // cols: genes by descending entry count (the gather kernel starts the long ones first)
+    std::int64_t long_genes = 0;        // the first so many of them have more entries than eight chunks of the summation order
+    std::int64_t short_entries = 0;     // entries of the others
     std::uint64_t bytes = 0;
     const void *src_row_ptr = nullptr, *src_col_idx = nullptr, *src_packed = nullptr; // arrays it was built from
 };

@@ -191,3 +191,34 @@ def test_deterministic_transpose_skewed_genes(cuda_device, oracle):
     assert rc == 0 and col_ptr[42] - col_ptr[41] == rows
     want = oracle.qcsr_transpose_ordered(1, col_ptr, row_idx, codes, c["scales"], c["offsets"], g_host, 0, rows)
     assert np.array_equal(bits_of(out), bits_of(want))
+
+
+@pytest.mark.parametrize("policy,n,ld", [(1, 32, 32), (1, 64, 64), (2, 64, 67), (1, 128, 128), (2, 128, 131)])
+def test_deterministic_transpose_short_genes_by_warp(cuda_device, oracle, policy, n, ld):
+    """Enough short genes that each is one warp's work, with entry counts around the edges of its batches of eight and 32
+    entries and of the chunks of 256, beside genes of more than eight chunks, which stay a CTA's."""
+    rng = np.random.default_rng(policy + n)
+    rows, cols = 4500, 1300
+    edges = [0, 1, 7, 8, 9, 31, 32, 33, 255, 256, 257, 511, 513, 2047, 2048, 2049, 4096, 4500]
+    counts = np.concatenate([edges, rng.integers(0, 100, size=cols - len(edges))])
+    rng.shuffle(counts)
+    per_gene = [rng.choice(rows, size=int(k), replace=False) for k in counts]
+    order = np.lexsort((np.repeat(np.arange(cols), counts), np.concatenate(per_gene)))
+    row_ptr = np.zeros(rows + 1, dtype=np.int64)
+    np.cumsum(np.bincount(np.concatenate(per_gene), minlength=rows), out=row_ptr[1:])
+    nnz = int(row_ptr[-1])
+    c = host_pack(oracle, dict(rows=rows, cols=cols, bits=8, policy=policy, row_ptr=row_ptr, col_idx=np.repeat(np.arange(cols), counts)[order].astype(np.int32),
+                               scales=rng.uniform(0.01, 0.5, size=cols).astype(np.float32),
+                               offsets=rng.uniform(-1, 1, size=cols if policy == 1 else rows).astype(np.float32),
+                               values=rng.uniform(-2.0, 40.0, size=nnz).astype(np.float32)))
+    x = to_dev(c, cuda_device)
+    g, g_host = dense(rng, rows, n, torch.float32, cuda_device, std=1.0, ld=ld)
+    op = ops.PreparedSpmm(capi.PROJECTION_TRANSPOSE, rows, cols, n, x.nnz, 8, policy, g.dtype, cuda_device, deterministic=True, device_matrix=x)
+    rc, col_ptr, row_idx, codes = oracle.qcsr_gene_major(8, cols, c["row_ptr"], c["packed_row_ptr"], c["col_idx"], c["packed"])
+    assert rc == 0
+    init = rng.normal(size=(cols, n)).astype(np.float32)
+    for lo, hi in [(0, rows), (333, 4097)]:
+        want = oracle.qcsr_transpose_ordered(policy, col_ptr, row_idx, codes, c["scales"], c["offsets"], g_host, lo, hi, alpha=-1.5, beta=0.25, out=init)
+        got = op.run(x, g, torch.from_numpy(init).to(cuda_device), alpha=-1.5, beta=0.25, row_begin=lo, row_end=hi).cpu().numpy()
+        assert np.array_equal(bits_of(got), bits_of(want))
+    op.close()
