@@ -554,7 +554,8 @@ cb200_status cb200_spmm_prepare(const cb200_spmm_problem *problem, cb200_prepare
                                                          true, p->arena, stream, &p->blocked);
             if (st != CB200_STATUS_SUCCESS) return abandon(st);
             p->schedule_name = problem->multiply == CB200_DTYPE_BF16 ? "tensor_blocked" : "tensor_blocked_x3";
-            p->workspace_bytes = qcsr_transpose_blocked_workspace_bytes(problem->m, problem->k, problem->n);
+            p->workspace_required = qcsr_transpose_blocked_workspace_bytes(problem->m, problem->k, problem->n, false);
+            p->workspace_bytes = qcsr_transpose_blocked_workspace_bytes(problem->m, problem->k, problem->n, plan.split && p->blocked.baked);
             p->persistent_bytes += p->blocked.bytes;
         }
     }

@@ -14,12 +14,12 @@
 // as one contiguous segment; they are decoded to bf16 and scattered into a zeroed operand tile in
 // shared memory, laid out gene-major this time (M = gene, K = cell; K-major with the 128-byte
 // swizzle), and sixteen 128 x N x 16 tcgen05 MMAs multiply it with the group's rows of G.  G is
-// converted to bf16 once per launch into one 256 x N record per group, already in the K-major
-// core-matrix operand layout (rows outside the launch's row range are written as zero, which is how a
-// partial row range is honoured).  A CTA keeps the fp32 accumulators of a set of windows (four at N = 64,
-// eight at N = 32; two accumulators per window, one per MMA-issuing warp, 512 TMEM columns in all) while
+// converted to bf16 once per launch into one 256 x N record per group (256 x 2 N, hi and lo parts side by side, for the
+// split products of baked words), already in the K-major core-matrix operand layout (rows outside the launch's row range are written as zero, which is how a
+// partial row range is honoured).  A CTA keeps the fp32 accumulators of a set of windows (four at 64 columns
+// of G, eight at 32, with two accumulators per window, one per MMA-issuing warp; four at 128 with one; 512 TMEM columns in all) while
 // it walks a run of groups, so the group's G record is fetched once per set; at the end of the run the
-// two accumulators of a window are added and the sums are stored to the run's slot of a scratch array.  The
+// accumulators of a window are added and the sums are stored to the run's slot of a scratch array.  The
 // (window set, group) pairs are dealt to the CTAs as equal contiguous runs, so two or three CTAs contribute to
 // the same genes: ordered_sum_kernel adds a set's slots into G' in run order (G' is first scaled by beta by a
 // small kernel), which makes G' the same bits on every launch -- vector reductions straight into G', as this
@@ -37,7 +37,8 @@
 // 1M x 33,538 matrix); baked words are fetched into registers before the tile is released, so that only
 // stores lie between release and hand-over -- and read the accumulators back at the end of a run; warps 16
 // and 17 issue the MMAs, the first and the second eight K steps of every tile (15.7 ms against 17.5 with one
-// issuing warp); warp 18 feeds the G ring (2 stages of 32 KB); warp 19 deals the entry chunks.  Every barrier wait is bounded; on a
+// issuing warp; 780 against 690 us on an eighth of that matrix with one elected issuer; at 128 columns of G one does); warp 18
+// feeds the G ring; warp 19 deals the entry chunks.  Every barrier wait is bounded; on a
 // time-out a status word is raised, waits stop blocking, and the kernel runs to completion and frees
 // its TMEM.  A non-zero status means G' is not valid.
 #include "kernels.cuh"
@@ -51,17 +52,23 @@ namespace {
 
 constexpr int kWin = 128;                     // genes per window (as in the blocked copy)
 constexpr int kRows = 256;                    // cells per group (as in the blocked copy)
-// windows whose accumulators a CTA holds in TMEM: two sets of N columns per window (one per MMA-issuing warp, which
-// take the first and the second half of a tile's K steps), 512 columns in all
-__host__ __device__ constexpr int set_windows(int n) { return 256 / n; }
-constexpr int kIssuers = 2;
+// MMA-issuing warps: two take the first and the second half of a tile's K steps, each into accumulators of its own; at 128
+// columns one keeps the tensor pipe busy and leaves tensor memory to twice the windows
+__host__ __device__ constexpr int issuers(int n) { return n <= 64 ? 2 : 1; }
+// windows whose accumulators a CTA holds in TMEM: N columns per window and issuing warp, 512 columns in all
+__host__ __device__ constexpr int set_windows(int n) { return 512 / (issuers(n) * n); }
+constexpr int kIssuerWarps = 2;
 constexpr int kProducerWarps = 16;
 constexpr int kProducerThreads = kProducerWarps * 32;
 constexpr int kChunkLoaders = 1;
-constexpr int kThreads = kProducerThreads + 32 * (kIssuers + 1 + kChunkLoaders);
+constexpr int kThreads = kProducerThreads + 32 * (kIssuerWarps + 1 + kChunkLoaders);
 constexpr int kTileBytes = kWin * kRows * 2;  // 64 KB: [cell quarter][gene][64 cells]
 constexpr int kQuarterBytes = kWin * 128;     // 16 KB: 128 genes x 64 cells
-constexpr int kGStages = 2;
+constexpr int kPieceRows = 64;                // G comes in pieces of 64 cells, four per group
+constexpr int kGroupPieces = kRows / kPieceRows;
+// pieces in the ring: two groups', or, at 128 columns, the five of 16 KB that shared memory holds: a piece is released as
+// the last window of its group passes over it, and the next group's takes its place while the others are multiplied
+__host__ __device__ constexpr int ring_pieces(int n) { return n <= 64 ? 2 * kGroupPieces : kGroupPieces + 1; }
 constexpr int kChunkEntries = 2048;
 constexpr int kChunkBytes = kChunkEntries * 4;
 constexpr int kChunkStages = 2;               // one per scatter group (two stages each do not fit beside the G ring)
@@ -71,6 +78,7 @@ constexpr int kRing = kChunkStages / 2;       // chunk stages per scatter group
 static_assert(kChunkLoaders == 1 && kRing >= 1, "one loader thread deals the chunks to the two groups' rings");
 
 __host__ __device__ constexpr int g_record_bytes(int n) { return kRows * n * 2; }
+__host__ __device__ constexpr int g_piece_bytes(int n) { return kPieceRows * n * 2; }
 
 struct tb_params {
     const std::uint32_t *entries;
@@ -78,7 +86,8 @@ struct tb_params {
     const float *scales;
     const float *gene_offsets; // per gene, per-gene-affine policy
     const float *row_offsets;  // per cell, row-offset policy
-    const unsigned char *records; // G as bf16, one record per group
+    const unsigned char *records; // G as bf16, one record of kGroupPieces pieces per group
+    int piece_stride;             // bytes from piece to piece
     float *out;
     std::int64_t out_ld;
     std::int64_t cols;
@@ -100,13 +109,13 @@ __host__ __device__ inline std::int64_t runs_of_cta(std::int64_t total, std::int
 }
 
 __device__ __forceinline__ std::int64_t dmin(std::int64_t a, std::int64_t b) { return a < b ? a : b; }
-// K-major operand, no swizzle (the G record): core matrices of 8 columns x 16 bytes (8 cells); the
-// 32 core matrices of 8 output columns sit side by side (LBO = 128 B), groups of 8 columns 4 KB apart.
+// K-major operand, no swizzle (a piece of G): core matrices of 8 columns x 16 bytes (8 cells); the
+// 8 core matrices of 8 output columns sit side by side (LBO = 128 B), groups of 8 columns 1 KB apart.
 __device__ __forceinline__ std::uint64_t smem_desc_g(std::uint32_t addr) {
     std::uint64_t d = 0;
     d |= static_cast<std::uint64_t>((addr & 0x3ffffu) >> 4);
     d |= static_cast<std::uint64_t>(128u >> 4) << 16;
-    d |= static_cast<std::uint64_t>(static_cast<unsigned>(kRows * 16) >> 4) << 32;
+    d |= static_cast<std::uint64_t>(static_cast<unsigned>(kPieceRows * 16) >> 4) << 32;
     d |= static_cast<std::uint64_t>(1) << 46; // descriptor version of this architecture
     return d;
 }
@@ -121,20 +130,23 @@ __global__ void __launch_bounds__(256) scale_output_kernel(float *out, std::int6
     }
 }
 
-// G [cells][n] fp32 (leading dimension ld) -> one bf16 record per group of 256 cells: the n x 256
-// slice of G^T in the no-swizzle K-major operand layout (byte offset of (column c, cell r) =
-// (c/8)*4096 + (r/8)*128 + (c%8)*16 + (r%8)*2).  Cells outside [row_begin, row_end) are zero.
-// part 0 writes hi = bf16(g); part 1 writes lo = bf16(g - hi), the next 8 bits of the mantissa.
+// G [cells][n] fp32 (leading dimension ld) -> one bf16 record per group of 256 cells: four pieces of 64 cells, each the
+// columns x 64 slice of G^T in the no-swizzle K-major operand layout (byte offset of (column c, cell r) in its piece =
+// (c/8)*1024 + (r/8)*128 + (c%8)*16 + (r%8)*2).  Cells outside [row_begin, row_end) are zero.
+// Columns of a record: hi = bf16(g) of the n columns; with both_parts behind them lo = bf16(g - hi), the next 8 bits of the
+// mantissa.  Otherwise part says which of the two the record holds.
 __global__ void __launch_bounds__(256) pack_g_kernel(const float *g, std::int64_t ld, int n, std::int64_t row_begin,
-                                                     std::int64_t row_end, std::int64_t group_begin, int part,
+                                                     std::int64_t row_end, std::int64_t group_begin, int both_parts, int only_part,
                                                      unsigned char *records) {
     const std::int64_t group = group_begin + blockIdx.x;
-    unsigned char *rec = records + static_cast<std::size_t>(blockIdx.x) * g_record_bytes(n);
+    const int columns = both_parts != 0 ? 2 * n : n;
+    unsigned char *rec = records + static_cast<std::size_t>(blockIdx.x) * g_record_bytes(columns);
     // A thread makes one 16-byte piece: a column's values of eight consecutive cells.  Consecutive threads take consecutive
     // columns of the same eight cells: their loads of a cell's row are contiguous, and their pieces are too (8 columns =
     // 128 bytes of the record).
-    for (int item = threadIdx.x; item < n * (kRows / 8); item += blockDim.x) {
-        const int c = item % n, r8 = item / n;
+    for (int item = threadIdx.x; item < columns * (kRows / 8); item += blockDim.x) {
+        const int column = item % columns, r8 = item / columns;
+        const int c = column < n ? column : column - n, part = both_parts != 0 ? (column < n ? 0 : 1) : only_part;
         std::uint32_t packed[4];
 #pragma unroll
         for (int j = 0; j < 8; j += 2) {
@@ -151,29 +163,32 @@ __global__ void __launch_bounds__(256) pack_g_kernel(const float *g, std::int64_
             }
             packed[j >> 1] = static_cast<std::uint32_t>(__bfloat16_as_ushort(b0)) | (static_cast<std::uint32_t>(__bfloat16_as_ushort(b1)) << 16);
         }
-        *reinterpret_cast<uint4 *>(rec + (c >> 3) * (kRows * 16) + r8 * 128 + (c & 7) * 16) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+        *reinterpret_cast<uint4 *>(rec + (r8 >> 3) * g_piece_bytes(columns) + (column >> 3) * (kPieceRows * 16) + (r8 & 7) * 128 + (column & 7) * 16) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
     }
 }
 
 // BAKED: the entry words hold {bf16 value, byte position / 2 in this kernel's tile}, written at prepare
 // (hi and lo arrays for the split passes): the scatter stores them as they are, no table, no arithmetic.
-template<int NC, bool BAKED>
+// NC: columns of G in a piece and of an accumulator; N of G'.  NC == 2 N: the columns are [hi of G | lo of G], and the
+// accumulators' halves are added when they are read back.
+template<int NC, int N, bool BAKED>
 __global__ void __launch_bounds__(kThreads, 1) qcsr_transpose_blocked_kernel(const tb_params p) {
-    constexpr int GREC = g_record_bytes(NC);
+    constexpr int GPIECE = g_piece_bytes(NC), kPieces = ring_pieces(NC), kIssuers = issuers(NC);
+    constexpr int kPerBar = kIssuers; // pieces of a barrier: with two issuing warps, the two that are one warp's work
     constexpr int kSetWindows = set_windows(NC);
     constexpr int kTmemCols = kSetWindows * kIssuers * NC; // 512
     constexpr std::uint32_t IDESC = instr_desc(NC);
     extern __shared__ __align__(1024) unsigned char smem[];
-    // [2][tile] | [kGStages][G record] | [kChunkStages][entry chunk] | tables | row offsets | barriers | ...
-    unsigned char *chunk_base = smem + 2 * kTileBytes + kGStages * GREC;
+    // [2][tile] | [kPieces][piece of G] | [kChunkStages][entry chunk] | tables, row offsets (code words) | barriers | ...
+    unsigned char *chunk_base = smem + 2 * kTileBytes + kPieces * GPIECE;
     float2 *table = reinterpret_cast<float2 *>(chunk_base + kChunkStages * kChunkBytes); // [kSetWindows][kWin] {scale, offset}
     float *row_offset_s = reinterpret_cast<float *>(table + kSetWindows * kWin);         // [kRows]
-    std::uint64_t *bars = reinterpret_cast<std::uint64_t *>(row_offset_s + kRows);
+    std::uint64_t *bars = BAKED ? reinterpret_cast<std::uint64_t *>(chunk_base + kChunkStages * kChunkBytes) : reinterpret_cast<std::uint64_t *>(row_offset_s + kRows);
     std::uint64_t *a_full = bars;                      // [2]            scatter warps -> MMA (one arrival per warp)
     std::uint64_t *a_empty = bars + 2;                 // [2]            MMA commit -> scatter warps
-    std::uint64_t *g_full = bars + 4;                  // [kGStages]     copy engine -> MMA
-    std::uint64_t *g_empty = g_full + kGStages;        // [kGStages]     MMA commit -> loader
-    std::uint64_t *c_full = g_empty + kGStages;        // [kChunkStages] copy engine -> scatter warps
+    std::uint64_t *g_full = bars + 4;                  // [kPieces]      copy engine -> MMA
+    std::uint64_t *g_empty = g_full + kPieces;         // [kPieces]      MMA commit -> loader
+    std::uint64_t *c_full = g_empty + kPieces;         // [kChunkStages] copy engine -> scatter warps
     std::uint64_t *c_empty = c_full + kChunkStages;    // [kChunkStages] scatter warps -> loaders
     std::uint64_t *acc_full = c_empty + kChunkStages;  // MMA commit -> scatter warps
     std::uint64_t *acc_empty = acc_full + 1;           // scatter warps -> MMA
@@ -185,16 +200,16 @@ __global__ void __launch_bounds__(kThreads, 1) qcsr_transpose_blocked_kernel(con
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const std::uint32_t smem0 = smem_addr(smem);
     const std::uint32_t grec0 = smem0 + 2 * kTileBytes;
-    const std::uint32_t chunk0 = grec0 + kGStages * GREC;
+    const std::uint32_t chunk0 = grec0 + kPieces * GPIECE;
 
     if (tid == 0) {
         for (int b = 0; b < 2; ++b) {
             bar_init(smem_addr(a_full + b), kGroupWarps);
             bar_init(smem_addr(a_empty + b), kIssuers); // one commit per MMA warp
         }
-        for (int s = 0; s < kGStages; ++s) {
+        for (int s = 0; s < kPieces; ++s) {
             bar_init(smem_addr(g_full + s), 1);
-            bar_init(smem_addr(g_empty + s), kIssuers);
+            bar_init(smem_addr(g_empty + s), 1); // a piece has one issuing warp
         }
         for (int s = 0; s < kChunkStages; ++s) {
             bar_init(smem_addr(c_full + s), 1);
@@ -366,14 +381,19 @@ __global__ void __launch_bounds__(kThreads, 1) qcsr_transpose_blocked_kernel(con
                 if (wl >= nwin) break; // warp-uniform
                 const std::int64_t gene = (set * kSetWindows + wl) * kWin + quarter * 32 + lane;
 #pragma unroll
-                for (int h = 0; h < NC / 32; ++h) {
-                    float v[32], second[32]; // the two halves of the K steps were accumulated apart
-                    tmem_ld32(tmem_base + (static_cast<std::uint32_t>(quarter * 32) << 16) + wl * kIssuers * NC + h * 32, v);
-                    tmem_ld32(tmem_base + (static_cast<std::uint32_t>(quarter * 32) << 16) + (wl * kIssuers + 1) * NC + h * 32, second);
+                for (int h = 0; h < N / 32; ++h) {
+                    float v[32], other[32];
+                    // the halves of the K steps, and the hi and the lo part of G, were accumulated apart
+                    const std::uint32_t at = tmem_base + (static_cast<std::uint32_t>(quarter * 32) << 16) + wl * kIssuers * NC + h * 32;
+                    tmem_ld32(at, v);
 #pragma unroll
-                    for (int c = 0; c < 32; ++c) v[c] += second[c];
+                    for (int k = 1; k < kIssuers * (NC / N); ++k) {
+                        tmem_ld32(at + k * N, other);
+#pragma unroll
+                        for (int c = 0; c < 32; ++c) v[c] += other[c];
+                    }
                     if (gene < p.cols && *abort_flag == 0) {
-                        float *slot = p.partials + (((first_run + run) * kSetWindows + wl) * kWin + quarter * 32 + lane) * NC + h * 32;
+                        float *slot = p.partials + (((first_run + run) * kSetWindows + wl) * kWin + quarter * 32 + lane) * N + h * 32;
 #pragma unroll
                         for (int c = 0; c < 32; c += 4) *reinterpret_cast<float4 *>(slot + c) = make_float4(v[c], v[c + 1], v[c + 2], v[c + 3]);
                     }
@@ -384,55 +404,87 @@ __global__ void __launch_bounds__(kThreads, 1) qcsr_transpose_blocked_kernel(con
             if (lane == 0) bar_arrive(smem_addr(acc_empty));
             u += count;
         }
-    } else if (warp < kProducerWarps + kIssuers) {
-        // ================= MMA issuers: warp kh issues the K steps [8 kh, 8 kh + 8) of every tile into its own accumulators.
-        // One issuing thread is held to the rate at which the MMAs read their operands and then spends half as long again
-        // on commits, waits and loop overhead while the tensor pipe runs dry; two threads halve the issue time of a tile. ==
+    } else if (warp < kProducerWarps + kIssuerWarps) {
+        // ================= MMA issuers: with two of them, warp kh issues the K steps [8 kh, 8 kh + 8) of every tile into its own
+        // accumulators.  A thread that issues under `lane == 0` is held up by more than the tensor pipe (see elect_one), and two
+        // of them halve that; elected threads issue faster, in bursts that take shared-memory bandwidth from the scatter
+        // groups (neither faster nor slower at N = 64).  At 128 columns, an MMA keeps the pipe busy for 64 cycles and one
+        // elected thread is enough. ==
         const int kh = warp - kProducerWarps;
-        long long q = 0, qg = 0;
+        constexpr int kMyPieces = kGroupPieces / kIssuers;
+        long long q = 0;
+        int qg = 0, slot = kh * kMyPieces, phase = 0; // this warp's first piece of the group, in the ring
         int run = 0;
-        for (std::int64_t u = u0; u < u1; ++run) {
+        for (std::int64_t u = u0; u < u1 && kh < kIssuers; ++run) {
             const std::int64_t set = u / p.group_count, gi0 = u % p.group_count;
             const std::int64_t count = dmin(p.group_count - gi0, u1 - u);
             const int nwin = static_cast<int>(dmin(kSetWindows, p.windows - set * kSetWindows));
             bar_wait(smem_addr(acc_empty), static_cast<std::uint32_t>((run & 1) ^ 1), abort_flag);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             for (std::int64_t gi = 0; gi < count; ++gi, ++qg) {
-                const int gs = static_cast<int>(qg % kGStages);
-                bar_wait(smem_addr(g_full + gs), static_cast<std::uint32_t>((qg / kGStages) & 1), abort_flag);
                 for (int wl = 0; wl < nwin; ++wl, ++q) {
                     const std::uint32_t b = static_cast<std::uint32_t>(q & 1);
                     bar_wait(smem_addr(a_full + b), static_cast<std::uint32_t>((q >> 1) & 1), abort_flag);
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    if (lane == 0) {
-                        const std::uint32_t a_tile = smem0 + b * kTileBytes;
-                        const std::uint32_t g_rec = grec0 + gs * GREC;
+                    const auto multiply = [&](int piece, int s) { // the K steps of a piece
+                        const std::uint32_t a_tile = smem0 + b * kTileBytes + (kh * kMyPieces + piece) * kQuarterBytes;
+                        const std::uint32_t g_piece = grec0 + s * GPIECE;
 #pragma unroll
-                        for (int k8 = 0; k8 < kRows / 16 / kIssuers; ++k8) {
-                            const int kk = kh * (kRows / 16 / kIssuers) + k8;
-                            mma_bf16(tmem_base + (wl * kIssuers + kh) * NC, smem_desc_sw128(a_tile + (kk >> 2) * kQuarterBytes + (kk & 3) * 32),
-                                     smem_desc_g(g_rec + kk * 256), IDESC, gi > 0 || k8 > 0);
+                        for (int kk = 0; kk < kPieceRows / 16; ++kk)
+                            mma_bf16(tmem_base + (wl * kIssuers + kh) * NC, smem_desc_sw128(a_tile + kk * 32), smem_desc_g(g_piece + kk * 256), IDESC,
+                                     gi > 0 || piece > 0 || kk > 0);
+                    };
+                    if constexpr (kIssuers == 2) {
+                        if (wl == 0) bar_wait(smem_addr(g_full + slot / kPerBar), static_cast<std::uint32_t>(phase), abort_flag);
+                        if (lane == 0) {
+#pragma unroll
+                            for (int piece = 0; piece < kMyPieces; ++piece) multiply(piece, slot + piece);
+                            mma_commit(smem_addr(a_empty + b));
+                            if (wl == nwin - 1) {
+                                mma_commit(smem_addr(g_empty + slot / kPerBar));
+                                if (gi == count - 1) mma_commit(smem_addr(acc_full));
+                            }
                         }
-                        mma_commit(smem_addr(a_empty + b));
-                        if (wl == nwin - 1) mma_commit(smem_addr(g_empty + gs));
-                        if (wl == nwin - 1 && gi == count - 1) mma_commit(smem_addr(acc_full));
+                        __syncwarp();
+                    } else {
+                        int s = slot, ph = phase;
+#pragma unroll
+                        for (int piece = 0; piece < kMyPieces; ++piece) {
+                            if (wl == 0) bar_wait(smem_addr(g_full + s), static_cast<std::uint32_t>(ph), abort_flag);
+                            if (elect_one()) {
+                                multiply(piece, s);
+                                if (wl == nwin - 1) mma_commit(smem_addr(g_empty + s));
+                                if (piece == kMyPieces - 1) {
+                                    mma_commit(smem_addr(a_empty + b));
+                                    if (wl == nwin - 1 && gi == count - 1) mma_commit(smem_addr(acc_full));
+                                }
+                            }
+                            if (++s == kPieces) { s = 0; ph ^= 1; }
+                        }
                     }
-                    __syncwarp();
                 }
+                slot += kGroupPieces;
+                if (slot >= kPieces) { slot -= kPieces; phase ^= 1; }
             }
             u += count;
         }
     } else {
-        const int role = warp - kProducerWarps - kIssuers; // 0: G records, 1..kChunkLoaders: entry chunks
+        const int role = warp - kProducerWarps - kIssuerWarps; // 0: pieces of G, 1..kChunkLoaders: entry chunks
         if (role == 0) {
-            if (lane == 0) {
-                long long qg = 0;
-                for (std::int64_t u = u0; u < u1; ++u, ++qg) {
-                    const std::int64_t gi = u % p.group_count;
-                    const int gs = static_cast<int>(qg % kGStages);
-                    bar_wait(smem_addr(g_empty + gs), static_cast<std::uint32_t>(((qg / kGStages) & 1) ^ 1), abort_flag);
-                    bar_arrive_expect_tx(smem_addr(g_full + gs), GREC);
-                    bulk_copy_g2s(grec0 + gs * GREC, p.records + static_cast<std::size_t>(gi) * GREC, GREC, smem_addr(g_full + gs));
+            if (elect_one()) {
+                int s = 0;
+                std::uint32_t ph = 1;
+                for (std::int64_t u = u0; u < u1; ++u) {
+                    const unsigned char *src = p.records + static_cast<std::size_t>(u % p.group_count) * kGroupPieces * p.piece_stride;
+                    for (int piece = 0; piece < kGroupPieces; ++piece, src += p.piece_stride) {
+                        const std::uint32_t full = smem_addr(g_full + s / kPerBar);
+                        if (piece % kPerBar == 0) {
+                            bar_wait(smem_addr(g_empty + s / kPerBar), ph, abort_flag);
+                            bar_arrive_expect_tx(full, kPerBar * GPIECE);
+                        }
+                        bulk_copy_g2s(grec0 + s * GPIECE, src, GPIECE, full);
+                        if (++s == kPieces) { s = 0; ph ^= 1u; }
+                    }
                 }
             }
         } else {
@@ -479,17 +531,16 @@ __global__ void __launch_bounds__(kThreads, 1) qcsr_transpose_blocked_kernel(con
     if (tid == 0 && *abort_flag != 0 && p.status != nullptr) atomicExch(p.status, 1);
 }
 
-template<int NC> constexpr std::size_t tb_smem_bytes() {
-    return 2 * kTileBytes + kGStages * g_record_bytes(NC) + kChunkStages * kChunkBytes + set_windows(NC) * kWin * 8 + kRows * 4 +
-           (6 + 2 * kGStages + 2 * kChunkStages) * sizeof(std::uint64_t) + (kChunkStages + 1) * 4 + 16;
+template<int NC, bool BAKED> constexpr std::size_t tb_smem_bytes() {
+    return 2 * kTileBytes + ring_pieces(NC) * g_piece_bytes(NC) + kChunkStages * kChunkBytes + (BAKED ? 0 : set_windows(NC) * kWin * 8 + kRows * 4) +
+           (6 + 2 * ring_pieces(NC) + 2 * kChunkStages) * sizeof(std::uint64_t) + (kChunkStages + 1) * 4 + 16;
 }
 
 // G'[genes of window wl of set s] += alpha * (the sums of the runs of set s, added in run order).  Block = (set, window of
 // the set); the runs of a set are those of the CTAs whose unit range meets the set, in CTA order.
-template<int NC>
+template<int N, int kSetWindows>
 __global__ void __launch_bounds__(256) ordered_sum_kernel(const float *partials, float *out, std::int64_t out_ld, std::int64_t cols, int windows,
                                                           std::int64_t group_count, std::int64_t grid, float alpha) {
-    constexpr int kSetWindows = set_windows(NC);
     __shared__ std::int64_t slots[512];
     __shared__ int slot_count;
     const std::int64_t set = blockIdx.x / kSetWindows;
@@ -521,13 +572,13 @@ __global__ void __launch_bounds__(256) ordered_sum_kernel(const float *partials,
     if (meets) slots[before_meets] = before_runs + (set - u0 / group_count);
     __syncthreads();
     const int count = slot_count;
-    for (int i = threadIdx.x; i < kWin * (NC / 4); i += blockDim.x) {
-        const int gl = i / (NC / 4), c4 = i % (NC / 4);
+    for (int i = threadIdx.x; i < kWin * (N / 4); i += blockDim.x) {
+        const int gl = i / (N / 4), c4 = i % (N / 4);
         const std::int64_t gene = window * kWin + gl;
         if (gene >= cols) continue;
         float4 sum = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         for (int r = 0; r < count; ++r) {
-            const float4 v = *reinterpret_cast<const float4 *>(partials + ((slots[r] * kSetWindows + wl) * kWin + gl) * NC + 4 * c4);
+            const float4 v = *reinterpret_cast<const float4 *>(partials + ((slots[r] * kSetWindows + wl) * kWin + gl) * N + 4 * c4);
             sum.x += v.x; sum.y += v.y; sum.z += v.z; sum.w += v.w;
         }
         float4 *dst = reinterpret_cast<float4 *>(out + gene * out_ld + 4 * c4);
@@ -537,17 +588,17 @@ __global__ void __launch_bounds__(256) ordered_sum_kernel(const float *partials,
     }
 }
 
-template<int NC, bool BAKED>
+template<int NC, int N, bool BAKED>
 cb200_status launch_one(const tb_params &p, int sm_count, cudaStream_t stream) {
-    constexpr std::size_t smem = tb_smem_bytes<NC>();
+    constexpr std::size_t smem = tb_smem_bytes<NC, BAKED>();
     static_assert(smem <= 232448, "shared memory budget");
-    CB200_CUDA_OK(cudaFuncSetAttribute(qcsr_transpose_blocked_kernel<NC, BAKED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    CB200_CUDA_OK(cudaFuncSetAttribute(qcsr_transpose_blocked_kernel<NC, N, BAKED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        static_cast<int>(smem)));
     const std::int64_t sets = (p.windows + set_windows(NC) - 1) / set_windows(NC);
     const std::int64_t units = sets * p.group_count;
     const unsigned grid = static_cast<unsigned>(units < sm_count ? units : sm_count);
-    qcsr_transpose_blocked_kernel<NC, BAKED><<<grid, kThreads, smem, stream>>>(p);
-    ordered_sum_kernel<NC><<<static_cast<unsigned>(sets * set_windows(NC)), 256, 0, stream>>>(p.partials, p.out, p.out_ld, p.cols, p.windows, p.group_count,
+    qcsr_transpose_blocked_kernel<NC, N, BAKED><<<grid, kThreads, smem, stream>>>(p);
+    ordered_sum_kernel<N, set_windows(NC)><<<static_cast<unsigned>(sets * set_windows(NC)), 256, 0, stream>>>(p.partials, p.out, p.out_ld, p.cols, p.windows, p.group_count,
                                                                                              static_cast<std::int64_t>(grid), p.alpha);
     count_launch(2);
     CB200_CUDA_OK(cudaGetLastError());
@@ -563,10 +614,10 @@ static std::uint64_t record_part_bytes(std::int64_t rows, std::int64_t n) {
     const std::int64_t groups = (rows + kRows - 1) / kRows;
     return (static_cast<std::uint64_t>(256 + groups * g_record_bytes(static_cast<int>(n))) + 255u) & ~static_cast<std::uint64_t>(255u);
 }
-std::uint64_t qcsr_transpose_blocked_workspace_bytes(std::int64_t rows, std::int64_t cols, std::int64_t n) {
-    const std::int64_t per_set = n == 32 ? set_windows(32) : set_windows(64);
+std::uint64_t qcsr_transpose_blocked_workspace_bytes(std::int64_t rows, std::int64_t cols, std::int64_t n, bool both_parts) {
+    const std::int64_t per_set = n == 32 ? set_windows(32) : set_windows(64); // 2 N columns: as many windows or half of them
     const std::int64_t windows = (cols + kWin - 1) / kWin, sets = (windows + per_set - 1) / per_set;
-    return record_part_bytes(rows, n) + static_cast<std::uint64_t>(sets + kMaxTransposeCtas) * per_set * kWin * n * sizeof(float);
+    return record_part_bytes(rows, both_parts ? 2 * n : n) + static_cast<std::uint64_t>(sets + kMaxTransposeCtas) * per_set * kWin * n * sizeof(float);
 }
 
 bool qcsr_transpose_blocked_shape_ok(std::int64_t rows, std::int64_t cols, std::int64_t n, int bits) {
@@ -583,7 +634,7 @@ cb200_status launch_qcsr_transpose_blocked(const qcsr_view &x, const dense_args 
         return CB200_STATUS_SUCCESS; // baked words of the forward tile, or no lo words for the split passes
     if (!qcsr_transpose_blocked_shape_ok(x.rows, x.cols, d.n, x.bits) || d.dense_dtype != CB200_DTYPE_F32) return CB200_STATUS_SUCCESS;
     if (reinterpret_cast<std::uintptr_t>(d.out) % 16u != 0u || (d.out_ld * 4u) % 16u != 0u) return CB200_STATUS_SUCCESS;
-    if (workspace == nullptr || workspace_bytes < qcsr_transpose_blocked_workspace_bytes(x.rows, x.cols, d.n) || sm_count > kMaxTransposeCtas)
+    if (workspace == nullptr || workspace_bytes < qcsr_transpose_blocked_workspace_bytes(x.rows, x.cols, d.n, false) || sm_count > kMaxTransposeCtas)
         return CB200_STATUS_SUCCESS;
     if (reinterpret_cast<std::uintptr_t>(workspace) % 256u != 0u) return CB200_STATUS_SUCCESS;
     const bool row_policy = x.policy == CB200_DECODE_COLUMN_SCALE_ROW_OFFSET;
@@ -615,30 +666,37 @@ cb200_status launch_qcsr_transpose_blocked(const qcsr_view &x, const dense_args 
     p.records = records; p.out = d.out; p.out_ld = d.out_ld; p.cols = x.cols;
     p.group_begin = group_begin; p.group_count = group_end - group_begin; p.windows = layout.windows;
     p.alpha = d.alpha; p.status = status;
-    p.partials = reinterpret_cast<float *>(static_cast<unsigned char *>(workspace) + record_part_bytes(x.rows, d.n));
     // One pass multiplies bf16(value) with bf16(G).  With split products the fp32 product is rebuilt
-    // from three passes, hi*hi + hi*lo + lo*hi (v = hi + lo + O(2^-17 v), likewise G): relative error
-    // per product about 3 * 2^-17, inside the 1e-4 bound of an fp32 dense operand.  The passes run
-    // back to back on the stream, share the record buffer and add into the same G'.
-    const int passes = split_products ? 3 : 1;
-    int packed_part = -1;
-    for (int pass = 0; pass < passes; ++pass) { // (G hi, value hi), (G hi, value lo), (G lo, value hi): G hi is packed once
-        const int g_part = pass == 2 ? 1 : 0;
-        p.value_part = pass == 1 ? 1 : 0;
-        if (layout.baked) p.entries = pass == 1 ? layout.entries_lo : layout.entries; // baked words carry their part
-        if (g_part != packed_part) {
-            pack_g_kernel<<<static_cast<unsigned>(group_end - group_begin), 256, 0, stream>>>(
-                static_cast<const float *>(d.dense), d.dense_ld, static_cast<int>(d.n), row_begin, row_end, group_begin, g_part,
-                records);
-            count_launch();
-            CB200_CUDA_OK(cudaGetLastError());
-            packed_part = g_part;
-        }
-        const cb200_status st = layout.baked ? (d.n == 64 ? launch_one<64, true>(p, sm_count, stream) : launch_one<32, true>(p, sm_count, stream))
-                                             : (d.n == 64 ? launch_one<64, false>(p, sm_count, stream) : launch_one<32, false>(p, sm_count, stream));
-        if (st != CB200_STATUS_SUCCESS) return st;
-    }
-    return CB200_STATUS_SUCCESS;
+    // from hi*hi + hi*lo + lo*hi (v = hi + lo + O(2^-17 v), likewise G): relative error per product
+    // about 3 * 2^-17, inside the 1e-4 bound of an fp32 dense operand.  The passes run back to back on
+    // the stream, share the record buffer and add into the same G'.
+    // The two passes over the hi words build the same tiles, and a tile costs more than its MMAs: they are one pass over
+    // [hi of G | lo of G], with accumulators of 2 N columns (125,000 x 33,538 at N = 64: 670 us a pass, the pair as one 765 us).
+    // That needs entry words as they are scattered, and room for both parts of G in the workspace.
+    const int n = static_cast<int>(d.n);
+    const bool both_parts = split_products && layout.baked && workspace_bytes >= qcsr_transpose_blocked_workspace_bytes(x.rows, x.cols, d.n, true);
+    p.partials = reinterpret_cast<float *>(static_cast<unsigned char *>(workspace) + record_part_bytes(x.rows, both_parts ? 2 * n : n));
+    p.piece_stride = g_piece_bytes(both_parts ? 2 * n : n);
+    const auto pack = [&](int part) {
+        pack_g_kernel<<<static_cast<unsigned>(group_end - group_begin), 256, 0, stream>>>(static_cast<const float *>(d.dense), d.dense_ld, n, row_begin,
+                                                                                         row_end, group_begin, both_parts ? 1 : 0, part, records);
+        count_launch();
+        return cudaGetLastError();
+    };
+    const auto pass = [&](int value_part) {
+        p.value_part = value_part;
+        if (!layout.baked) return n == 64 ? launch_one<64, 64, false>(p, sm_count, stream) : launch_one<32, 32, false>(p, sm_count, stream);
+        p.entries = value_part != 0 ? layout.entries_lo : layout.entries; // baked words carry their part
+        if (both_parts && value_part == 0) return n == 64 ? launch_one<128, 64, true>(p, sm_count, stream) : launch_one<64, 32, true>(p, sm_count, stream);
+        return n == 64 ? launch_one<64, 64, true>(p, sm_count, stream) : launch_one<32, 32, true>(p, sm_count, stream);
+    };
+    CB200_CUDA_OK(pack(0));
+    cb200_status st = pass(0);
+    if (st != CB200_STATUS_SUCCESS || !split_products) return st;
+    st = pass(1); // reads the hi part of G: the first N columns of a piece, with or without the others behind them
+    if (st != CB200_STATUS_SUCCESS || both_parts) return st;
+    CB200_CUDA_OK(pack(1));
+    return pass(0);
 }
 
 } // namespace cb200
