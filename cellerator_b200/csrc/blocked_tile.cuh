@@ -80,42 +80,46 @@ __device__ __forceinline__ std::uint64_t smem_desc(std::uint32_t addr) {
 // W^T in operand layout (byte offset of (column c, gene e) = (c/8)*2048 + (e/8)*128 + (c%8)*16 +
 // (e%8)*2, zero for genes >= cols) followed by 128 x {scale, zero-point}.  part 0 writes
 // hi = bf16(w) (w itself for a bf16 W); part 1 writes lo = bf16(w - hi), the next 8 mantissa bits.
+// both_parts: 2 n columns, hi and then lo.
 // With absmax_bits != null the record holds fp16 instead: hi = fp16(w * s), lo = fp16(w * s - hi), s =
-// operand_scale(largest |w|).  The grid is (windows, column groups): block (w, g) lays out columns [g, g + 1) * n /
+// operand_scale(largest |w|).  The grid is (windows, column groups): block (w, g) lays out the record's columns [g, g + 1) * n /
 // gridDim.y of window w; the blocks of group 0 also write the window's table.
 constexpr int kPackColumns = 16; // columns of W per block of the packing kernel
 template<typename WT>
 __global__ void __launch_bounds__(256) pack_windows_kernel(const WT *w, std::int64_t ld, std::int64_t cols, int n, int part,
                                                            const float *scales, const float *offsets, int per_gene_offsets,
-                                                           unsigned char *records, const unsigned *absmax_bits = nullptr) {
+                                                           unsigned char *records, const unsigned *absmax_bits = nullptr, int both_parts = 0) {
     const std::int64_t window = blockIdx.x;
-    unsigned char *rec = records + window * record_bytes(n);
+    const int columns = both_parts != 0 ? 2 * n : n; // both_parts: the hi part of the n columns, then their lo part
+    unsigned char *rec = records + window * record_bytes(columns);
     __nv_bfloat16 *wt = reinterpret_cast<__nv_bfloat16 *>(rec);
     const bool fp16 = absmax_bits != nullptr;
     const float ws = fp16 ? operand_scale(__uint_as_float(*absmax_bits)) : 1.0f;
-    const int group_cols = n / static_cast<int>(gridDim.y), c_first = static_cast<int>(blockIdx.y) * group_cols;
+    const int group_cols = columns / static_cast<int>(gridDim.y), c_first = static_cast<int>(blockIdx.y) * group_cols;
     for (int i = threadIdx.x; i < group_cols * kWin; i += blockDim.x) {
-        const int e = i / group_cols, c = c_first + i % group_cols; // consecutive threads read consecutive columns of one gene
+        const int e = i / group_cols, column = c_first + i % group_cols; // consecutive threads read consecutive columns of one gene
+        const int c = column < n ? column : column - n;
+        const bool lo = column < n ? part != 0 : true;
         const std::int64_t gene = window * kWin + e;
         float value = 0.0f;
         if (gene < cols) {
             if constexpr (sizeof(WT) == 2) value = __bfloat162float(w[gene * ld + c]);
             else value = w[gene * ld + c];
         }
-        const int at = ((c >> 3) * kRowGroupBytes + (e >> 3) * 128 + (c & 7) * 16 + (e & 7) * 2) >> 1;
+        const int at = ((column >> 3) * kRowGroupBytes + (e >> 3) * 128 + (column & 7) * 16 + (e & 7) * 2) >> 1;
         if (fp16) {
             const float scaled = value * ws;
             __half h = __float2half_rn(scaled);
-            if (part != 0) h = __float2half_rn(scaled - __half2float(h));
+            if (lo) h = __float2half_rn(scaled - __half2float(h));
             reinterpret_cast<__half *>(rec)[at] = h;
             continue;
         }
         __nv_bfloat16 v = __float2bfloat16_rn(value);
-        if (part != 0) v = __float2bfloat16_rn(value - __bfloat162float(v));
+        if (lo) v = __float2bfloat16_rn(value - __bfloat162float(v));
         wt[at] = v;
     }
     if (blockIdx.y != 0) return;
-    float2 *table = reinterpret_cast<float2 *>(rec + n * kWin * 2);
+    float2 *table = reinterpret_cast<float2 *>(rec + columns * kWin * 2);
     for (int e = threadIdx.x; e < kWin; e += blockDim.x) {
         const std::int64_t gene = window * kWin + e;
         float2 so = make_float2(0.0f, 0.0f);

@@ -618,6 +618,8 @@ cb200_status cb200_spmm_prepare(const cb200_spmm_problem *problem, cb200_prepare
             }
             // behind it, the sums of the groups that are cut between CTAs; a launch whose workspace ends before them cuts none
             p->workspace_required = p->workspace_bytes;
+            if (plan.split && p->blocked.baked && qcsr_blocked_takes_both_parts(problem->n, problem->dense_dtype))
+                p->workspace_bytes = std::max<std::uint64_t>(p->workspace_bytes, qcsr_blocked_workspace_bytes(problem->k, 2 * problem->n));
             p->workspace_bytes = device_arena::rounded(p->workspace_bytes) + qcsr_window_split_bytes(problem->m, problem->k, problem->n, p->sm_count);
             p->persistent_bytes += p->blocked.bytes;
         }

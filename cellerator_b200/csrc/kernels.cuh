@@ -146,6 +146,8 @@ window_split_plan qcsr_window_split(std::int64_t rows, std::int64_t cols, int sm
 std::uint64_t qcsr_window_split_bytes(std::int64_t rows, std::int64_t cols, std::int64_t n, int sm_count);
 bool qcsr_blocked_shape_ok(std::int64_t rows, std::int64_t cols, std::int64_t n, int bits, int dense_dtype);
 std::uint64_t qcsr_blocked_workspace_bytes(std::int64_t cols, std::int64_t n);
+// Split products of an fp32 W may use room for 2 N columns: its hi and lo parts side by side.
+bool qcsr_blocked_takes_both_parts(std::int64_t n, int dense_dtype);
 // Current device; memory from `arena`, kernels on `stream`, which is waited for.
 // bake: decoded values in the entry words (forward, bf16 products only)
 // bake_lo (needs bake): also the array of the next eight mantissa bits (split-product schedules)

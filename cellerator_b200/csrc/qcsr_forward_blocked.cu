@@ -233,6 +233,7 @@ struct blocked_params {
     std::int64_t row_end;     // rows >= row_end are computed but not written
     std::int64_t group_begin, group_end;
     window_split split;
+    int record_stride; // bytes from record to record of W
     int windows;
     float alpha, beta;
     const float *bias;   // composed epilogue, applied by the last pass only
@@ -249,7 +250,7 @@ struct blocked_params {
 // Test hook (cb200_test_arm_wait_timeout): read at launch time by the two-group kernel's launcher.
 std::atomic<int> g_test_poll_limit{0}; // 0 = not armed
 
-template<int NC, int CS, bool BAKED>
+template<int NC, int N, int CS, bool BAKED> // NC, N: as in the two-group kernel
 __global__ void __launch_bounds__(kThreads, 1) qcsr_fwd_blocked_kernel(const blocked_params p) {
     constexpr int REC = record_bytes(NC);
     constexpr int STAGES = w_stages(NC, CS);
@@ -389,11 +390,17 @@ __global__ void __launch_bounds__(kThreads, 1) qcsr_fwd_blocked_kernel(const blo
             bar_wait(smem_addr(acc_full), static_cast<std::uint32_t>(gi & 1), abort_flag);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
-            for (int h = 0; h < NC / 32; ++h) {
+            for (int h = 0; h < N / 32; ++h) {
                 float v[32];
                 tmem_ld32(tmem_base + (static_cast<std::uint32_t>((warp & 3) * 32) << 16) + sub * NC + h * 32, v);
+                if constexpr (NC == 2 * N) {
+                    float lo[32];
+                    tmem_ld32(tmem_base + (static_cast<std::uint32_t>((warp & 3) * 32) << 16) + sub * NC + N + h * 32, lo);
+#pragma unroll
+                    for (int c = 0; c < 32; ++c) v[c] += lo[c];
+                }
                 if (unit.slot >= 0) { // raw sums of a part
-                    store_row32(p.split.sums + (static_cast<std::int64_t>(unit.slot) * kRows + tid) * NC + h * 32, v, 1.0f, 0.0f, nullptr, h * 32, CB200_EPILOGUE_NONE);
+                    store_row32(p.split.sums + (static_cast<std::int64_t>(unit.slot) * kRows + tid) * N + h * 32, v, 1.0f, 0.0f, nullptr, h * 32, CB200_EPILOGUE_NONE);
                 } else if (row < p.row_end) {
                     float *out = p.y + row * p.y_ld + h * 32;
                     store_row32(out, v, alpha, p.beta, p.bias, h * 32, p.epilogue);
@@ -451,7 +458,7 @@ __global__ void __launch_bounds__(kThreads, 1) qcsr_fwd_blocked_kernel(const blo
                         const int s = static_cast<int>(q % STAGES);
                         bar_wait(smem_addr(w_empty + s), static_cast<std::uint32_t>(((q / STAGES) & 1) ^ 1), abort_flag);
                         bar_arrive_expect_tx(smem_addr(w_full + s), REC);
-                        bulk_copy_g2s(wstage0 + s * REC, p.records + static_cast<std::size_t>(w) * REC, REC, smem_addr(w_full + s));
+                        bulk_copy_g2s(wstage0 + s * REC, p.records + static_cast<std::size_t>(w) * p.record_stride, REC, smem_addr(w_full + s));
                     }
                 }
             }
@@ -505,15 +512,15 @@ template<int NC, int CS> constexpr std::size_t blocked_smem_bytes() {
            (6 + 2 * w_stages(NC, CS) + 2 * CS) * sizeof(std::uint64_t) + (CS + 1) * 4 + 16;
 }
 
-template<int NC, int CS, bool BAKED>
+template<int NC, int N, int CS, bool BAKED>
 cb200_status launch_cs(const blocked_params &p, int sm_count, cudaStream_t stream) {
     constexpr std::size_t smem = blocked_smem_bytes<NC, CS>();
     static_assert(smem <= 232448, "shared memory budget");
     static_assert(CS % kChunkLoaders == 0, "a loader always refills the same stages");
-    CB200_CUDA_OK(cudaFuncSetAttribute(qcsr_fwd_blocked_kernel<NC, CS, BAKED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    CB200_CUDA_OK(cudaFuncSetAttribute(qcsr_fwd_blocked_kernel<NC, N, CS, BAKED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        static_cast<int>(smem)));
     const unsigned grid = static_cast<unsigned>(std::min(unit_count(p.split, p.group_begin, p.group_end), sm_count));
-    qcsr_fwd_blocked_kernel<NC, CS, BAKED><<<grid, kThreads, smem, stream>>>(p);
+    qcsr_fwd_blocked_kernel<NC, N, CS, BAKED><<<grid, kThreads, smem, stream>>>(p);
     count_launch();
     CB200_CUDA_OK(cudaGetLastError());
     return CB200_STATUS_SUCCESS;
@@ -523,8 +530,8 @@ cb200_status launch_cs(const blocked_params &p, int sm_count, cudaStream_t strea
 // 33,538-gene matrix), three when segments span several chunks (the 17 %-dense 4,000-gene one).
 template<int NC>
 cb200_status launch_one(const blocked_params &p, bool long_segments, bool baked, int sm_count, cudaStream_t stream) {
-    if (baked) return long_segments ? launch_cs<NC, 3, true>(p, sm_count, stream) : launch_cs<NC, 2, true>(p, sm_count, stream);
-    return long_segments ? launch_cs<NC, 3, false>(p, sm_count, stream) : launch_cs<NC, 2, false>(p, sm_count, stream);
+    if (baked) return long_segments ? launch_cs<NC, NC, 3, true>(p, sm_count, stream) : launch_cs<NC, NC, 2, true>(p, sm_count, stream);
+    return long_segments ? launch_cs<NC, NC, 3, false>(p, sm_count, stream) : launch_cs<NC, NC, 2, false>(p, sm_count, stream);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -552,9 +559,10 @@ __host__ __device__ constexpr int w2_stages(int n) {
 // TEST_HOOK: the instantiation cb200_test_arm_wait_timeout selects.  It differs in two places only: the poll limit
 // of the waits comes from the launch (a few thousand instead of 2^22) and the W loader issues no copies, so
 // that the waits for W run out.  Everything that happens after a wait has run out is common code.
-template<int NC, bool TEST_HOOK>
+// NC: columns of W in a record and of the accumulators; N of Y.  NC == 2 N: the columns are [hi of W | lo of W], and the
+// accumulators' halves are added when they are read.
+template<int NC, int N, bool TEST_HOOK>
 __global__ void __launch_bounds__(kThreads2, 1) qcsr_fwd_blocked2_kernel(const blocked_params p) {
-    constexpr int REC = record_bytes(NC);   // distance of the W records in global memory
     constexpr int WREC = NC * kWin * 2;     // the W part of a record (the decode table is not needed)
     constexpr int STAGES = w2_stages(NC);
     constexpr int CHUNKS = 2 * kRing2;
@@ -714,11 +722,17 @@ __global__ void __launch_bounds__(kThreads2, 1) qcsr_fwd_blocked2_kernel(const b
             bar_wait(smem_addr(acc_full), static_cast<std::uint32_t>(gi & 1), abort_flag, limit);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
-            for (int h = 0; h < NC / 32; ++h) {
+            for (int h = 0; h < N / 32; ++h) {
                 float v[32];
                 tmem_ld32(tmem_base + (static_cast<std::uint32_t>((warp & 3) * 32) << 16) + sub * NC + h * 32, v);
+                if constexpr (NC == 2 * N) {
+                    float lo[32];
+                    tmem_ld32(tmem_base + (static_cast<std::uint32_t>((warp & 3) * 32) << 16) + sub * NC + N + h * 32, lo);
+#pragma unroll
+                    for (int c = 0; c < 32; ++c) v[c] += lo[c];
+                }
                 if (unit.slot >= 0) { // raw sums of a part
-                    store_row32(p.split.sums + (static_cast<std::int64_t>(unit.slot) * kRows + tid) * NC + h * 32, v, 1.0f, 0.0f, nullptr, h * 32, CB200_EPILOGUE_NONE);
+                    store_row32(p.split.sums + (static_cast<std::int64_t>(unit.slot) * kRows + tid) * N + h * 32, v, 1.0f, 0.0f, nullptr, h * 32, CB200_EPILOGUE_NONE);
                 } else if (row < p.row_end) {
                     float *out = p.y + row * p.y_ld + h * 32;
                     store_row32(out, v, alpha, p.beta, p.bias, h * 32, p.epilogue);
@@ -783,7 +797,7 @@ __global__ void __launch_bounds__(kThreads2, 1) qcsr_fwd_blocked2_kernel(const b
                     // no new copies once a wait of the CTA has run out
                     if (bar_wait(smem_addr(w_empty + s), static_cast<std::uint32_t>(((q / STAGES) & 1) ^ 1), abort_flag, limit)) { dead = true; break; }
                     bar_arrive_expect_tx(smem_addr(w_full + s), WREC);
-                    bulk_copy_g2s(wstage0 + s * WREC, p.records + static_cast<std::size_t>(w) * REC, WREC, smem_addr(w_full + s));
+                    bulk_copy_g2s(wstage0 + s * WREC, p.records + static_cast<std::size_t>(w) * p.record_stride, WREC, smem_addr(w_full + s));
                 }
             }
             // after an abort: let the copies still in flight land (the last one issued into each stage)
@@ -854,24 +868,25 @@ __global__ void __launch_bounds__(kThreads2, 1) qcsr_fwd_blocked2_kernel(const b
     if (tid == 0 && *abort_flag != 0 && p.status != nullptr) atomicExch(p.status, 1);
 }
 
-template<int NC, bool TEST_HOOK>
+template<int NC, int N, bool TEST_HOOK>
 cb200_status launch_blocked2_as(const blocked_params &p, int sm_count, cudaStream_t stream) {
     constexpr std::size_t smem = 2 * kABufBytes + w2_stages(NC) * NC * kWin * 2 + 2 * kRing2 * kChunk2Bytes +
                                  (8 + 2 * w2_stages(NC) + 4 * kRing2) * sizeof(std::uint64_t) + 2 * kRing2 * 4 + 24;
     static_assert(smem <= 232448, "shared memory budget");
-    CB200_CUDA_OK(cudaFuncSetAttribute(qcsr_fwd_blocked2_kernel<NC, TEST_HOOK>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+    CB200_CUDA_OK(cudaFuncSetAttribute(qcsr_fwd_blocked2_kernel<NC, N, TEST_HOOK>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
     const unsigned grid = static_cast<unsigned>(std::min(unit_count(p.split, p.group_begin, p.group_end), sm_count));
-    qcsr_fwd_blocked2_kernel<NC, TEST_HOOK><<<grid, kThreads2, smem, stream>>>(p);
+    qcsr_fwd_blocked2_kernel<NC, N, TEST_HOOK><<<grid, kThreads2, smem, stream>>>(p);
     count_launch();
     CB200_CUDA_OK(cudaGetLastError());
     return CB200_STATUS_SUCCESS;
 }
-template<int NC>
+template<int NC, int N = NC>
 cb200_status launch_blocked2(const blocked_params &p, int sm_count, cudaStream_t stream) {
-    return p.withhold_w != 0 ? launch_blocked2_as<NC, true>(p, sm_count, stream) : launch_blocked2_as<NC, false>(p, sm_count, stream);
+    return p.withhold_w != 0 ? launch_blocked2_as<NC, N, true>(p, sm_count, stream) : launch_blocked2_as<NC, N, false>(p, sm_count, stream);
 }
 } // namespace
 
+bool qcsr_blocked_takes_both_parts(std::int64_t n, int dense_dtype) { return dense_dtype == CB200_DTYPE_F32 && n <= 64; }
 std::uint64_t qcsr_blocked_workspace_bytes(std::int64_t cols, std::int64_t n) {
     const std::int64_t windows = (cols + kWin - 1) / kWin;
     return static_cast<std::uint64_t>(256 + windows * record_bytes(static_cast<int>(n)));
@@ -1085,9 +1100,15 @@ cb200_status launch_qcsr_forward_blocked(const qcsr_view &x, const dense_args &d
     p.row_offsets = row_policy && !layout.baked ? x.offsets : nullptr; // baked words already hold the row's offset
     p.records = records; p.y = d.out; p.y_ld = d.out_ld; p.row_end = row_end;
     p.group_begin = row_begin / kRows; p.group_end = (row_end + kRows - 1) / kRows; p.windows = layout.windows;
-    p.split = split_of_launch(x, d.n, workspace, workspace_bytes, qcsr_blocked_workspace_bytes(x.cols, d.n), sm_count);
+    const bool long_segments = layout.total_entries > static_cast<std::int64_t>(kChunkEntries) * layout.groups * layout.windows;
+    // two scatter groups pay when a window is a chunk or two; long segments keep one group and deeper chunks
+    const bool two_groups = layout.baked && !long_segments;
+    const int both_parts = split_products && !w_bf16 && layout.baked && qcsr_blocked_takes_both_parts(d.n, d.dense_dtype) &&
+                                   workspace_bytes >= qcsr_blocked_workspace_bytes(x.cols, 2 * d.n) ? 1 : 0;
+    const std::int64_t columns = both_parts != 0 ? 2 * d.n : d.n;
+    p.record_stride = record_bytes(static_cast<int>(columns));
+    p.split = split_of_launch(x, d.n, workspace, workspace_bytes, qcsr_blocked_workspace_bytes(x.cols, columns), sm_count);
     p.alpha = d.alpha; p.status = status;
-    p.idesc = instr_desc(static_cast<int>(d.n), half);
     p.result_scale = half ? 1.0f / layout.value_scale : 1.0f;
     p.w_absmax = half ? w_absmax : nullptr;
     p.poll_limit = kPollLimit;
@@ -1099,18 +1120,21 @@ cb200_status launch_qcsr_forward_blocked(const qcsr_view &x, const dense_args &d
     *taken = true;
     // One pass multiplies bf16(value) with bf16 W.  With split products the fp32 product is rebuilt
     // from bf16 pieces, value = hi + lo and (fp32 W) W = hi + lo:  bf16 W: hi*w + lo*w (two passes, exact
-    // up to the 2^-17 of the value that lo leaves);  fp32 W: hi*hi + hi*lo + lo*hi (three passes,
-    // ~3 * 2^-17 per product).  The passes run back to back on the stream, share the record buffer and
+    // up to the 2^-17 of the value that lo leaves);  fp32 W: hi*hi + hi*lo + lo*hi (~3 * 2^-17 per product).  The passes
+    // run back to back on the stream, share the record buffer and
     // accumulate into Y (beta of the call on the first pass, 1 afterwards); every pass sums a row in
     // the same fixed order, so the result is repeatable.
+    // hi*hi and hi*lo read the same tiles, and a tile costs more than its MMAs: where both parts of W fit an accumulator of
+    // 128 columns they are one pass over [hi of W | lo of W] (30,000 x 12,000 at N = 64: 369 -> 244 us, 75,776 x 2,000 at
+    // N = 32 226 -> 137).
     struct pass_spec { int w_part, value_part; };
     const pass_spec plain[1] = {{0, 0}}, split_bf16[2] = {{0, 0}, {0, 1}}, split_f32[3] = {{0, 0}, {1, 0}, {0, 1}};
-    const pass_spec *passes = !split_products ? plain : (w_bf16 ? split_bf16 : split_f32);
-    const int pass_count = !split_products ? 1 : (w_bf16 ? 2 : 3);
+    const pass_spec *passes = !split_products ? plain : (w_bf16 || both_parts != 0 ? split_bf16 : split_f32);
+    const int pass_count = !split_products ? 1 : (w_bf16 || both_parts != 0 ? 2 : 3);
     int packed_part = -1;
     for (int i = 0; i < pass_count; ++i) {
         if (passes[i].w_part != packed_part) {
-            const dim3 grid(static_cast<unsigned>(layout.windows), static_cast<unsigned>(d.n / kPackColumns));
+            const dim3 grid(static_cast<unsigned>(layout.windows), static_cast<unsigned>(columns / kPackColumns));
             if (w_bf16)
                 pack_windows_kernel<__nv_bfloat16><<<grid, 256, 0, stream>>>(static_cast<const __nv_bfloat16 *>(d.dense), d.dense_ld,
                                                                               x.cols, static_cast<int>(d.n), passes[i].w_part, x.scales,
@@ -1118,7 +1142,7 @@ cb200_status launch_qcsr_forward_blocked(const qcsr_view &x, const dense_args &d
             else
                 pack_windows_kernel<float><<<grid, 256, 0, stream>>>(static_cast<const float *>(d.dense), d.dense_ld, x.cols,
                                                                       static_cast<int>(d.n), passes[i].w_part, x.scales, x.offsets,
-                                                                      row_policy ? 0 : 1, records, half ? w_absmax : nullptr);
+                                                                      row_policy ? 0 : 1, records, half ? w_absmax : nullptr, both_parts);
             count_launch();
             CB200_CUDA_OK(cudaGetLastError());
             packed_part = passes[i].w_part;
@@ -1129,13 +1153,16 @@ cb200_status launch_qcsr_forward_blocked(const qcsr_view &x, const dense_args &d
         p.bias = d.bias;
         p.epilogue = i + 1 == pass_count ? d.epilogue : CB200_EPILOGUE_NONE;
         cb200_status st;
-        const bool long_segments = layout.total_entries > static_cast<std::int64_t>(kChunkEntries) * layout.groups * layout.windows;
-        // two scatter groups pay when a window is a chunk or two; long segments keep one group and deeper chunks
-        const bool two_groups = layout.baked && !long_segments;
-        switch (d.n) {
-        case 32: st = two_groups ? launch_blocked2<32>(p, sm_count, stream) : launch_one<32>(p, long_segments, layout.baked, sm_count, stream); break;
-        case 64: st = two_groups ? launch_blocked2<64>(p, sm_count, stream) : launch_one<64>(p, long_segments, layout.baked, sm_count, stream); break;
-        default: st = two_groups ? launch_blocked2<128>(p, sm_count, stream) : launch_one<128>(p, long_segments, layout.baked, sm_count, stream); break;
+        p.idesc = instr_desc(static_cast<int>(both_parts != 0 && passes[i].value_part == 0 ? columns : d.n), half);
+        if (both_parts != 0 && passes[i].value_part == 0) {
+            if (two_groups) st = d.n == 64 ? launch_blocked2<128, 64>(p, sm_count, stream) : launch_blocked2<64, 32>(p, sm_count, stream);
+            else st = d.n == 64 ? launch_cs<128, 64, 3, true>(p, sm_count, stream) : launch_cs<64, 32, 3, true>(p, sm_count, stream);
+        } else {
+            switch (d.n) {
+            case 32: st = two_groups ? launch_blocked2<32>(p, sm_count, stream) : launch_one<32>(p, long_segments, layout.baked, sm_count, stream); break;
+            case 64: st = two_groups ? launch_blocked2<64>(p, sm_count, stream) : launch_one<64>(p, long_segments, layout.baked, sm_count, stream); break;
+            default: st = two_groups ? launch_blocked2<128>(p, sm_count, stream) : launch_one<128>(p, long_segments, layout.baked, sm_count, stream); break;
+            }
         }
         if (st != CB200_STATUS_SUCCESS) return st;
         st = launch_add_parts(p.split, p.group_begin, p.group_end, row_end, static_cast<int>(d.n), d.out, d.out_ld, p.alpha, p.beta, p.bias, p.epilogue,

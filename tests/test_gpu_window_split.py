@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("schedule,bits,n,dtype,multiply", [
     ("tensor_blocked", 8, 64, torch.bfloat16, capi.DTYPE_BF16), ("tensor_blocked", 8, 128, torch.bfloat16, capi.DTYPE_F32),
-    ("tensor_blocked", 8, 32, torch.float32, capi.DTYPE_F32), ("tensor_dense", 4, 64, torch.bfloat16, capi.DTYPE_BF16),
+    ("tensor_blocked", 8, 32, torch.float32, capi.DTYPE_F32), ("tensor_blocked", 8, 64, torch.float32, capi.DTYPE_F32), ("tensor_dense", 4, 64, torch.bfloat16, capi.DTYPE_BF16),
     ("tensor_codes", 4, 128, torch.bfloat16, capi.DTYPE_BF16), ("tensor_codes", 4, 32, torch.bfloat16, capi.DTYPE_BF16)])
 @pytest.mark.parametrize("rows,windows,density", [(200, 33, 40), (256 * 6 + 1, 12, 40), (256 * 6 + 1, 17, 400), (256 * 150 - 7, 9, 12)])
 def test_cut_groups(cuda_device, oracle, monkeypatch, schedule, bits, n, dtype, multiply, rows, windows, density):
@@ -46,4 +46,8 @@ def test_cut_groups(cuda_device, oracle, monkeypatch, schedule, bits, n, dtype, 
     op.workspace_bytes -= 1                                            # no room for the sums of parts: no group is cut
     uncut = op.run(x, w, torch.empty_like(y)).cpu().numpy()
     assert np.all(np.abs(uncut - y.cpu().numpy()) <= 1e-4 * scale)
+    if schedule == "tensor_blocked":                                   # room for N columns of W: an fp32 W is multiplied in three passes
+        op.workspace_bytes = 256 + windows * 128 * (2 * n + 8)
+        narrow = op.run(x, w, torch.empty_like(y)).cpu().numpy()
+        assert np.all(np.abs(narrow - y.cpu().numpy()) <= 1e-4 * scale)
     op.close()
