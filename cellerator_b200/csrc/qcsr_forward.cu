@@ -33,7 +33,10 @@ struct fwd_params {
     int epilogue;
     int lanes;      // lanes that serve one entry, a power of two
     int group_rows, warps; // rows and warps per CTA
-    int short_rows;  // rows of fewer than 64 entries on average
+    union {
+        unsigned full_groups; // CTAs of that many rows; the others take a quarter of them
+        int short_rows;       // a warp per row: rows of fewer than 64 entries on average
+    };
     int parts;       // sums of parts the shared memory of a CTA holds
     int packed_rows; // W is the re-laid copy: rows at a pitch of 16 bytes
     int out_vector; // rows of Y can be written 16 bytes at a time
@@ -334,15 +337,22 @@ __global__ void __launch_bounds__(128, 8) qcsr_fwd_row_kernel(const fwd_params p
 
 // A CTA owns `group_rows` consecutive rows and deals their parts to its warps, so that a long row does not hold up the
 // others; sums of parts meet in shared memory.
-template<int BITS, typename WT, int V>
+// SHORT_END: the CTAs from p.full_groups on take a quarter of the rows.
+template<int BITS, typename WT, int V, bool SHORT_END>
 __global__ void __launch_bounds__(kGatherMaxWarps * 32, 2) qcsr_fwd_gather_kernel(const fwd_params p) {
     __shared__ std::int64_t row_start[kGatherMaxRows], code_start[kGatherMaxRows];
     __shared__ int row_len[kGatherMaxRows], row_share[kGatherMaxRows], first_part[kGatherMaxRows + 1];
     extern __shared__ __align__(16) int2 staging[];         // [warp][64], then the sums
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
     float *sums = reinterpret_cast<float *>(staging + warps * kSegment); // [p.parts][V][lanes]
-    const std::int64_t row0 = p.row_begin + static_cast<std::int64_t>(blockIdx.x) * p.group_rows;
-    const int rows = static_cast<int>(min(static_cast<std::int64_t>(p.group_rows), p.row_end - row0));
+    std::int64_t row0 = p.row_begin + static_cast<std::int64_t>(blockIdx.x) * p.group_rows;
+    int most_rows = p.group_rows;
+    if constexpr (SHORT_END)
+        if (blockIdx.x >= p.full_groups) {
+            most_rows = p.group_rows >> 2;
+            row0 = p.row_begin + static_cast<std::int64_t>(p.full_groups) * p.group_rows + static_cast<std::int64_t>(blockIdx.x - p.full_groups) * most_rows;
+        }
+    const int rows = static_cast<int>(min(static_cast<std::int64_t>(most_rows), p.row_end - row0));
     if (warp == 0) {
         int len = 0;
         if (lane < rows) {
@@ -436,15 +446,23 @@ __global__ void __launch_bounds__(kGatherMaxWarps * 32, 2) qcsr_fwd_gather_kerne
 //    (125,000 x 1,800 at N = 64: 2.50 ms with 4 rows, 2.57 with 8, 2.64 with 32).
 //  - Where few rows leave the SMs short of CTAs, 16 warps share the longest row (1,024 x 1,800: 0.10 ms, 8 warps 0.14) and
 //    fewer rows per CTA keep at least two CTAs per SM (512 x 1,800: 38 us with one, 67 with 8).
+//  - Of CTAs of eight warps the last third of a resident wave takes a quarter of the rows each: the launch ends when the
+//    longest of them does (20,000 x 2,000 at N = 32: 85 -> 81 us, 10,000 x 4,000 at N = 64: 93 -> 82; a whole wave of them 87
+//    and 87, an eighth of the rows each 98 and 98).  Those of 16 warps share few long rows, and gain nothing.
 //  - Many rows of a few entries, or of W rows of 32 bytes and less, run with a warp per row (200,000 x 24 at N = 32: 108 us,
 //    dealt out by parts 128; 20,000 x 240 at N = 16 bf16: 39 us against 44).
-void gather_shape(const qcsr_view &x, std::int64_t rows, std::int64_t w_row_bytes, int sm_count, int *group_rows, int *warps) {
+void gather_shape(const qcsr_view &x, std::int64_t rows, std::int64_t w_row_bytes, int sm_count, fwd_params *p) {
     const double mean = static_cast<double>(x.nnz) / static_cast<double>(std::max<std::int64_t>(x.rows, 1));
-    *warps = rows <= 8ll * sm_count || (rows <= 64ll * sm_count && mean >= 512.0) ? kGatherMaxWarps : 8;
-    *group_rows = 0;
+    p->warps = rows <= 8ll * sm_count || (rows <= 64ll * sm_count && mean >= 512.0) ? kGatherMaxWarps : 8;
+    p->group_rows = 0;
     if (rows >= 64ll * sm_count && (mean < 64.0 || w_row_bytes <= 32)) return;
-    *group_rows = 1;
-    while (*group_rows < 8 && 2 * *group_rows * mean <= 8192.0 && rows >= 4ll * sm_count * *group_rows) *group_rows *= 2;
+    p->group_rows = 1;
+    while (p->group_rows < 8 && 2 * p->group_rows * mean <= 8192.0 && rows >= 4ll * sm_count * p->group_rows) p->group_rows *= 2;
+    p->full_groups = static_cast<unsigned>((rows + p->group_rows - 1) / p->group_rows);
+    if (p->warps != kGatherMaxWarps && p->group_rows >= 4) { // four CTAs of 64 registers a thread are resident
+        const std::int64_t short_end = std::min<std::int64_t>(rows, 4ll * sm_count * p->group_rows / 3);
+        p->full_groups = static_cast<unsigned>((rows - short_end) / p->group_rows);
+    }
 }
 
 template<int BITS, typename WT, int V>
@@ -460,11 +478,14 @@ cb200_status launch_gather(fwd_params p, cudaStream_t stream) {
         if (p.short_rows) qcsr_fwd_row_kernel<BITS, WT, V, 1><<<grid, 128, 0, stream>>>(p);
         else qcsr_fwd_row_kernel<BITS, WT, V, 2><<<grid, 128, 0, stream>>>(p);
     } else {
-        const unsigned groups = static_cast<unsigned>((rows + p.group_rows - 1) / p.group_rows);
+        const std::int64_t left = rows - static_cast<std::int64_t>(p.full_groups) * p.group_rows;
+        const bool short_end = left > 0;
+        const unsigned groups = p.full_groups + static_cast<unsigned>(short_end ? (left + p.group_rows / 4 - 1) / (p.group_rows / 4) : 0);
         p.parts = std::min(kGatherParts, 32 * 1024 / static_cast<int>(V * p.lanes * sizeof(float)));
         const std::size_t smem = static_cast<std::size_t>(p.warps) * kSegment * sizeof(int2) +
                                  static_cast<std::size_t>(p.parts) * V * p.lanes * sizeof(float);
-        qcsr_fwd_gather_kernel<BITS, WT, V><<<dim3(groups, tiles), p.warps * 32, smem, stream>>>(p);
+        if (short_end) qcsr_fwd_gather_kernel<BITS, WT, V, true><<<dim3(groups, tiles), p.warps * 32, smem, stream>>>(p);
+        else qcsr_fwd_gather_kernel<BITS, WT, V, false><<<dim3(groups, tiles), p.warps * 32, smem, stream>>>(p);
     }
     count_launch();
     CB200_CUDA_OK(cudaGetLastError());
@@ -561,8 +582,8 @@ cb200_status launch_qcsr_forward(const qcsr_view &x, const dense_args &d, std::i
     p.out_vector = reinterpret_cast<std::uintptr_t>(d.out) % 16u == 0u && d.out_ld % 4 == 0 ? 1 : 0;
     p.status = workspace_bytes >= sizeof(int) ? static_cast<int *>(workspace) : nullptr;
     const bool bf16 = d.dense_dtype == CB200_DTYPE_BF16;
-    p.short_rows = x.nnz < 64 * x.rows ? 1 : 0;
-    gather_shape(x, row_end - row_begin, d.n * (bf16 ? 2 : 4), sm_count, &p.group_rows, &p.warps);
+    gather_shape(x, row_end - row_begin, d.n * (bf16 ? 2 : 4), sm_count, &p);
+    if (p.group_rows == 0) p.short_rows = x.nnz < 64 * x.rows ? 1 : 0;
     if (gather_packs(x, d.n, d.dense_dtype) && workspace_bytes >= qcsr_gather_workspace_bytes(x.cols, x.nnz, d.n, d.dense_dtype)) {
         const int per_piece = bf16 ? 8 : 4, pieces = static_cast<int>((d.n + per_piece - 1) / per_piece);
         uint4 *packed = reinterpret_cast<uint4 *>(static_cast<unsigned char *>(workspace) + 256);
