@@ -89,6 +89,8 @@ template<typename WT>
 __global__ void __launch_bounds__(256) pack_windows_kernel(const WT *w, std::int64_t ld, std::int64_t cols, int n, int part,
                                                            const float *scales, const float *offsets, int per_gene_offsets,
                                                            unsigned char *records, const unsigned *absmax_bits = nullptr, int both_parts = 0) {
+    wait_for_previous_launch();
+    let_next_launch_start();
     const std::int64_t window = blockIdx.x;
     const int columns = both_parts != 0 ? 2 * n : n; // both_parts: the hi part of the n columns, then their lo part
     unsigned char *rec = records + window * record_bytes(columns);
@@ -168,6 +170,7 @@ __device__ __forceinline__ int units_of_cta(const window_split &s, std::int64_t 
 __global__ void __launch_bounds__(256) add_parts_kernel(const float *sums, int parts, int whole, int first_group, std::int64_t row_end,
                                                         int n, float *y, std::int64_t y_ld, float alpha, float beta, const float *bias,
                                                         int epilogue, float result_scale, const unsigned *w_absmax, const unsigned *value_bound) {
+    wait_for_previous_launch();
     const std::int64_t group = first_group + static_cast<int>(blockIdx.x);
     const float *in = sums + (group - whole) * parts * kRows * n;
     float scale = alpha * result_scale;
@@ -201,8 +204,8 @@ inline cb200_status launch_add_parts(const window_split &s, std::int64_t group_b
                                      const unsigned *w_absmax, const unsigned *value_bound, cudaStream_t stream) {
     const int first = static_cast<int>(group_begin) + whole_groups_in(s, group_begin, group_end), cut = static_cast<int>(group_end) - first;
     if (cut <= 0) return CB200_STATUS_SUCCESS;
-    add_parts_kernel<<<dim3(static_cast<unsigned>(cut), static_cast<unsigned>(n / 16)), 256, 0, stream>>>(
-        s.sums, s.parts, s.whole, first, row_end, n, y, y_ld, alpha, beta, bias, epilogue, result_scale, w_absmax, value_bound);
+    CB200_CUDA_OK(launch_kernel(true, add_parts_kernel, dim3(static_cast<unsigned>(cut), static_cast<unsigned>(n / 16)), 256, 0, stream, s.sums, s.parts, s.whole,
+                                first, row_end, n, y, y_ld, alpha, beta, bias, epilogue, result_scale, w_absmax, value_bound));
     count_launch();
     CB200_CUDA_OK(cudaGetLastError());
     return CB200_STATUS_SUCCESS;

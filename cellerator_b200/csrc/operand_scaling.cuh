@@ -2,6 +2,7 @@
 // window kernels (blocked_tile.cuh) and the Blocked-ELL kernel.  Everything here has internal linkage.
 #pragma once
 
+#include "dependent_launch.cuh"
 #include <cstdint>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -62,6 +63,7 @@ __device__ __forceinline__ void absmax_body(const WT *w, std::int64_t ld, std::i
 }
 template<typename WT>
 __global__ void __launch_bounds__(256) absmax_kernel(const WT *w, std::int64_t ld, std::int64_t rows, int n, unsigned *out_bits) {
+    let_next_launch_start();
     absmax_body(w, ld, rows, n, out_bits, blockIdx.x, gridDim.x);
 }
 
@@ -95,6 +97,7 @@ __global__ void __launch_bounds__(256) value_bound_kernel(const float *scales, c
 __global__ void __launch_bounds__(256) operand_bounds_kernel(const __nv_bfloat16 *w, std::int64_t ld, std::int64_t genes, int n, unsigned w_blocks,
                                                              const float *scales, const float *gene_offsets, const float *row_offsets,
                                                              std::int64_t rows, float max_code, unsigned *w_absmax, unsigned *value_bound) {
+    let_next_launch_start();
     if (blockIdx.x < w_blocks) absmax_body(w, ld, genes, n, w_absmax, blockIdx.x, w_blocks);
     else value_bound_body(scales, gene_offsets, genes, row_offsets, rows, max_code, value_bound, blockIdx.x - w_blocks);
 }

@@ -124,6 +124,8 @@ __device__ __forceinline__ void mma_f16(std::uint32_t tmem_d, std::uint32_t desc
 __global__ void __launch_bounds__(256) pack_w_kernel(const __nv_bfloat16 *w, std::int64_t ld, std::int64_t cols, int n, __half *packed_wt,
                                                      const float *scales, const float *offsets, int row_policy, const unsigned *w_absmax,
                                                      const unsigned *value_bound, uint2 *pairs) {
+    wait_for_previous_launch();
+    let_next_launch_start();
     const std::int64_t block = blockIdx.x;                     // gene block
     const float ws = operand_scale(__uint_as_float(*w_absmax));
     __half *dst = packed_wt + block * static_cast<std::int64_t>(n) * 32;
@@ -225,6 +227,7 @@ __global__ void __launch_bounds__(threads_of(H), 1) qbell_tcgen05_kernel(const t
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const std::uint32_t tmem_base = *tmem_slot;
+    wait_for_previous_launch();
 
     const std::int64_t first = p.block_row_begin + blockIdx.x, step = gridDim.x;
     const bool row_policy = p.policy == CB200_DECODE_COLUMN_SCALE_ROW_OFFSET;
@@ -463,7 +466,7 @@ cb200_status launch(const tc_params &p, int sm_count, cudaStream_t stream) {
     CB200_CUDA_OK(cudaFuncSetAttribute(qbell_tcgen05_kernel<BITS, H>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
     const std::int64_t block_rows = p.block_row_end - p.block_row_begin;
     const unsigned grid = static_cast<unsigned>(std::min<std::int64_t>(block_rows, sm_count));
-    qbell_tcgen05_kernel<BITS, H><<<grid, threads_of(H), smem, stream>>>(p);
+    CB200_CUDA_OK(launch_kernel(true, qbell_tcgen05_kernel<BITS, H>, grid, threads_of(H), smem, stream, p));
     count_launch();
     CB200_CUDA_OK(cudaGetLastError());
     return CB200_STATUS_SUCCESS;
@@ -499,9 +502,8 @@ cb200_status launch_qbell_tcgen05(const qbell_view &x, const dense_args &d, std:
     operand_bounds_kernel<<<w_blocks + static_cast<unsigned>((span + 255) / 256), 256, 0, stream>>>(
         static_cast<const __nv_bfloat16 *>(d.dense), d.dense_ld, x.cols, static_cast<int>(d.n), w_blocks, x.scales,
         row_policy ? nullptr : x.offsets, row_policy ? x.offsets : nullptr, x.rows, static_cast<float>((1 << x.bits) - 1), w_absmax, value_bound);
-    pack_w_kernel<<<static_cast<unsigned>(kpad / 32), 256, 0, stream>>>(static_cast<const __nv_bfloat16 *>(d.dense), d.dense_ld, x.cols,
-                                                                        static_cast<int>(d.n), wt, x.scales, x.offsets, row_policy ? 1 : 0,
-                                                                        w_absmax, value_bound, pairs);
+    CB200_CUDA_OK(launch_kernel(true, pack_w_kernel, dim3(static_cast<unsigned>(kpad / 32)), 256, 0, stream, static_cast<const __nv_bfloat16 *>(d.dense),
+                                d.dense_ld, x.cols, static_cast<int>(d.n), wt, x.scales, x.offsets, row_policy ? 1 : 0, w_absmax, value_bound, pairs));
     count_launch(2);
     CB200_CUDA_OK(cudaGetLastError());
     tc_params p{};

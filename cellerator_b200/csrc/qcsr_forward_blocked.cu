@@ -306,6 +306,7 @@ __global__ void __launch_bounds__(kThreads, 1) qcsr_fwd_blocked_kernel(const blo
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const std::uint32_t tmem_base = *tmem_slot;
+    wait_for_previous_launch();
 
     const int my_units = units_of_cta(p.split, p.group_begin, p.group_end);
     const auto unit_of = [&](int i) { return unit_at(p.split, p.group_begin, p.group_end, p.windows, static_cast<int>(blockIdx.x) + i * static_cast<int>(gridDim.x)); };
@@ -520,7 +521,7 @@ cb200_status launch_cs(const blocked_params &p, int sm_count, cudaStream_t strea
     CB200_CUDA_OK(cudaFuncSetAttribute(qcsr_fwd_blocked_kernel<NC, N, CS, BAKED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        static_cast<int>(smem)));
     const unsigned grid = static_cast<unsigned>(std::min(unit_count(p.split, p.group_begin, p.group_end), sm_count));
-    qcsr_fwd_blocked_kernel<NC, N, CS, BAKED><<<grid, kThreads, smem, stream>>>(p);
+    CB200_CUDA_OK(launch_kernel(true, qcsr_fwd_blocked_kernel<NC, N, CS, BAKED>, grid, kThreads, smem, stream, p));
     count_launch();
     CB200_CUDA_OK(cudaGetLastError());
     return CB200_STATUS_SUCCESS;
@@ -626,6 +627,7 @@ __global__ void __launch_bounds__(kThreads2, 1) qcsr_fwd_blocked2_kernel(const b
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const std::uint32_t tmem_base = *tmem_slot;
+    wait_for_previous_launch();
 
     const int my_units = units_of_cta(p.split, p.group_begin, p.group_end);
     const auto unit_of = [&](int i) { return unit_at(p.split, p.group_begin, p.group_end, p.windows, static_cast<int>(blockIdx.x) + i * static_cast<int>(gridDim.x)); };
@@ -875,7 +877,7 @@ cb200_status launch_blocked2_as(const blocked_params &p, int sm_count, cudaStrea
     static_assert(smem <= 232448, "shared memory budget");
     CB200_CUDA_OK(cudaFuncSetAttribute(qcsr_fwd_blocked2_kernel<NC, N, TEST_HOOK>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
     const unsigned grid = static_cast<unsigned>(std::min(unit_count(p.split, p.group_begin, p.group_end), sm_count));
-    qcsr_fwd_blocked2_kernel<NC, N, TEST_HOOK><<<grid, kThreads2, smem, stream>>>(p);
+    CB200_CUDA_OK(launch_kernel(true, qcsr_fwd_blocked2_kernel<NC, N, TEST_HOOK>, grid, kThreads2, smem, stream, p));
     count_launch();
     CB200_CUDA_OK(cudaGetLastError());
     return CB200_STATUS_SUCCESS;
@@ -1136,13 +1138,13 @@ cb200_status launch_qcsr_forward_blocked(const qcsr_view &x, const dense_args &d
         if (passes[i].w_part != packed_part) {
             const dim3 grid(static_cast<unsigned>(layout.windows), static_cast<unsigned>(columns / kPackColumns));
             if (w_bf16)
-                pack_windows_kernel<__nv_bfloat16><<<grid, 256, 0, stream>>>(static_cast<const __nv_bfloat16 *>(d.dense), d.dense_ld,
-                                                                              x.cols, static_cast<int>(d.n), passes[i].w_part, x.scales,
-                                                                              x.offsets, row_policy ? 0 : 1, records, half ? w_absmax : nullptr);
+                CB200_CUDA_OK(launch_kernel(half && i == 0, pack_windows_kernel<__nv_bfloat16>, grid, 256, 0, stream, static_cast<const __nv_bfloat16 *>(d.dense),
+                                            d.dense_ld, x.cols, static_cast<int>(d.n), passes[i].w_part, x.scales, x.offsets, row_policy ? 0 : 1, records,
+                                            half ? w_absmax : nullptr, 0));
             else
-                pack_windows_kernel<float><<<grid, 256, 0, stream>>>(static_cast<const float *>(d.dense), d.dense_ld, x.cols,
-                                                                      static_cast<int>(d.n), passes[i].w_part, x.scales, x.offsets,
-                                                                      row_policy ? 0 : 1, records, half ? w_absmax : nullptr, both_parts);
+                CB200_CUDA_OK(launch_kernel(half && i == 0, pack_windows_kernel<float>, grid, 256, 0, stream, static_cast<const float *>(d.dense), d.dense_ld,
+                                            x.cols, static_cast<int>(d.n), passes[i].w_part, x.scales, x.offsets, row_policy ? 0 : 1, records,
+                                            half ? w_absmax : nullptr, both_parts));
             count_launch();
             CB200_CUDA_OK(cudaGetLastError());
             packed_part = passes[i].w_part;

@@ -110,6 +110,8 @@ __global__ void __launch_bounds__(512) bytify_kernel(const std::uint32_t *entrie
 __global__ void __launch_bounds__(256) pack_codes_operands_kernel(const __nv_bfloat16 *w, std::int64_t ld, std::int64_t cols, int n,
                                                                   const float *scales, const float *offsets, unsigned char *records,
                                                                   const unsigned *w_absmax, const unsigned *bound_bits, unsigned char *table) {
+    wait_for_previous_launch();
+    let_next_launch_start();
     const std::int64_t window = blockIdx.x;
     __half *rec = reinterpret_cast<__half *>(records + window * record_bytes(n));
     const float ws = operand_scale(__uint_as_float(*w_absmax));
@@ -249,6 +251,7 @@ __global__ void __launch_bounds__(kCodesThreads, 1) qcsr_fwd_codes_kernel(const 
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const std::uint32_t tmem_base = *tmem_slot;
+    wait_for_previous_launch();
 
     const int my_units = units_of_cta(p.split, p.group_begin, p.group_end);
     const auto unit_of = [&](int i) { return unit_at(p.split, p.group_begin, p.group_end, p.windows, static_cast<int>(blockIdx.x) + i * static_cast<int>(gridDim.x)); };
@@ -514,7 +517,7 @@ cb200_status launch_codes(const codes_params &p, int sm_count, cudaStream_t stre
     static_assert(smem <= 232448, "shared memory budget");
     CB200_CUDA_OK(cudaFuncSetAttribute(qcsr_fwd_codes_kernel<NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
     const unsigned grid = static_cast<unsigned>(std::min(unit_count(p.split, p.group_begin, p.group_end), sm_count));
-    qcsr_fwd_codes_kernel<NC><<<grid, kCodesThreads, smem, stream>>>(p);
+    CB200_CUDA_OK(launch_kernel(true, qcsr_fwd_codes_kernel<NC>, grid, kCodesThreads, smem, stream, p));
     count_launch();
     CB200_CUDA_OK(cudaGetLastError());
     return CB200_STATUS_SUCCESS;
@@ -593,9 +596,9 @@ cb200_status launch_qcsr_forward_codes(const qcsr_view &x, const dense_args &d, 
     operand_bounds_kernel<<<w_blocks + static_cast<unsigned>((x.cols + 255) / 256), 256, 0, stream>>>(
         static_cast<const __nv_bfloat16 *>(d.dense), d.dense_ld, x.cols, static_cast<int>(d.n), w_blocks, x.scales, x.offsets, nullptr, 0,
         static_cast<float>((1 << x.bits) - 1), w_absmax, value_bound);
-    pack_codes_operands_kernel<<<dim3(static_cast<unsigned>(windows), static_cast<unsigned>(d.n / kPackColumns)), 256, 0, stream>>>(
-        static_cast<const __nv_bfloat16 *>(d.dense), d.dense_ld, x.cols, static_cast<int>(d.n), x.scales, x.offsets, records, w_absmax, value_bound,
-        table);
+    CB200_CUDA_OK(launch_kernel(true, pack_codes_operands_kernel, dim3(static_cast<unsigned>(windows), static_cast<unsigned>(d.n / kPackColumns)), 256, 0, stream,
+                                static_cast<const __nv_bfloat16 *>(d.dense), d.dense_ld, x.cols, static_cast<int>(d.n), x.scales, x.offsets, records, w_absmax,
+                                value_bound, table));
     count_launch(2);
     CB200_CUDA_OK(cudaGetLastError());
     codes_params p{};

@@ -149,6 +149,7 @@ __global__ void __launch_bounds__(kDenseThreads, 1) qcsr_fwd_dense_kernel(const 
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const std::uint32_t tmem_base = *tmem_slot;
+    wait_for_previous_launch();
 
     const int my_units = units_of_cta(p.split, p.group_begin, p.group_end);
     const auto unit_of = [&](int i) { return unit_at(p.split, p.group_begin, p.group_end, p.windows, static_cast<int>(blockIdx.x) + i * static_cast<int>(gridDim.x)); };
@@ -261,7 +262,7 @@ cb200_status launch_dense(const dense_params &p, int sm_count, cudaStream_t stre
     static_assert(smem <= 232448, "shared memory budget");
     CB200_CUDA_OK(cudaFuncSetAttribute(qcsr_fwd_dense_kernel<NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
     const unsigned grid = static_cast<unsigned>(std::min(unit_count(p.split, p.group_begin, p.group_end), sm_count));
-    qcsr_fwd_dense_kernel<NC><<<grid, kDenseThreads, smem, stream>>>(p);
+    CB200_CUDA_OK(launch_kernel(true, qcsr_fwd_dense_kernel<NC>, grid, kDenseThreads, smem, stream, p));
     count_launch();
     CB200_CUDA_OK(cudaGetLastError());
     return CB200_STATUS_SUCCESS;
@@ -339,9 +340,9 @@ cb200_status launch_qcsr_forward_dense(const qcsr_view &x, const dense_args &d, 
         count_launch();
         CB200_CUDA_OK(cudaGetLastError());
     }
-    pack_windows_kernel<__nv_bfloat16><<<dim3(static_cast<unsigned>(layout.windows), static_cast<unsigned>(d.n / kPackColumns)), 256, 0, stream>>>(
-        static_cast<const __nv_bfloat16 *>(d.dense), d.dense_ld, x.cols, static_cast<int>(d.n), 0, nullptr, nullptr, 0, records,
-        half ? w_absmax : nullptr);
+    CB200_CUDA_OK(launch_kernel(half, pack_windows_kernel<__nv_bfloat16>, dim3(static_cast<unsigned>(layout.windows), static_cast<unsigned>(d.n / kPackColumns)),
+                                256, 0, stream, static_cast<const __nv_bfloat16 *>(d.dense), d.dense_ld, x.cols, static_cast<int>(d.n), 0, nullptr, nullptr, 0,
+                                records, half ? w_absmax : nullptr, 0));
     count_launch();
     CB200_CUDA_OK(cudaGetLastError());
     dense_params p{};

@@ -21,8 +21,8 @@
 // it walks a run of groups, so the group's G record is fetched once per set; at the end of the run the
 // accumulators of a window are added and the sums are stored to the run's slot of a scratch array.  The
 // (window set, group) pairs are dealt to the CTAs as equal contiguous runs, so two or three CTAs contribute to
-// the same genes: ordered_sum_kernel adds a set's slots into G' in run order (G' is first scaled by beta by a
-// small kernel), which makes G' the same bits on every launch -- vector reductions straight into G', as this
+// the same genes: ordered_sum_kernel adds a set's slots into G' in run order (and, the first time, scales G' by
+// beta), which makes G' the same bits on every launch -- vector reductions straight into G', as this
 // kernel used before, are served in the order the L2 sees them.
 //
 // Entry words.  Prepare normally bakes them for this kernel: {bf16 value, byte position / 2 in the
@@ -41,6 +41,7 @@
 // feeds the G ring; warp 19 deals the entry chunks.  Every barrier wait is bounded; on a
 // time-out a status word is raised, waits stop blocking, and the kernel runs to completion and frees
 // its TMEM.  A non-zero status means G' is not valid.
+#include "dependent_launch.cuh"
 #include "kernels.cuh"
 #include "sm100_primitives.cuh"
 
@@ -94,6 +95,7 @@ struct tb_params {
     std::int64_t group_begin, group_count;
     int windows;
     float alpha;
+    float beta;   // of this pass: the call's, then 1
     int *status;
     int value_part; // 0: tile holds hi = bf16(value); 1: lo = bf16(value - hi)
     // The accumulators of a run (the consecutive units of one window set in one CTA) go to slot `global run index` of
@@ -137,7 +139,9 @@ __global__ void __launch_bounds__(256) scale_output_kernel(float *out, std::int6
 // mantissa.  Otherwise part says which of the two the record holds.
 __global__ void __launch_bounds__(256) pack_g_kernel(const float *g, std::int64_t ld, int n, std::int64_t row_begin,
                                                      std::int64_t row_end, std::int64_t group_begin, int both_parts, int only_part,
-                                                     unsigned char *records) {
+                                                     unsigned char *records, int *status) {
+    let_next_launch_start();
+    if (status != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *status = 0;
     const std::int64_t group = group_begin + blockIdx.x;
     const int columns = both_parts != 0 ? 2 * n : n;
     unsigned char *rec = records + static_cast<std::size_t>(blockIdx.x) * g_record_bytes(columns);
@@ -229,6 +233,7 @@ __global__ void __launch_bounds__(kThreads, 1) qcsr_transpose_blocked_kernel(con
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const std::uint32_t tmem_base = *tmem_slot;
+    wait_for_previous_launch();
 
     // Work: units (window set, group), numbered set * group_count + group; this CTA owns the units
     // [u0, u1).  A run = the consecutive units of one window set; it ends with the accumulators being
@@ -536,11 +541,12 @@ template<int NC, bool BAKED> constexpr std::size_t tb_smem_bytes() {
            (6 + 2 * ring_pieces(NC) + 2 * kChunkStages) * sizeof(std::uint64_t) + (kChunkStages + 1) * 4 + 16;
 }
 
-// G'[genes of window wl of set s] += alpha * (the sums of the runs of set s, added in run order).  Block = (set, window of
+// G'[genes of window wl of set s] = beta * G' + alpha * (the sums of the runs of set s, added in run order).  Block = (set, window of
 // the set); the runs of a set are those of the CTAs whose unit range meets the set, in CTA order.
 template<int N, int kSetWindows>
 __global__ void __launch_bounds__(256) ordered_sum_kernel(const float *partials, float *out, std::int64_t out_ld, std::int64_t cols, int windows,
-                                                          std::int64_t group_count, std::int64_t grid, float alpha) {
+                                                          std::int64_t group_count, std::int64_t grid, float alpha, float beta) {
+    wait_for_previous_launch();
     __shared__ std::int64_t slots[512];
     __shared__ int slot_count;
     const std::int64_t set = blockIdx.x / kSetWindows;
@@ -582,7 +588,11 @@ __global__ void __launch_bounds__(256) ordered_sum_kernel(const float *partials,
             sum.x += v.x; sum.y += v.y; sum.z += v.z; sum.w += v.w;
         }
         float4 *dst = reinterpret_cast<float4 *>(out + gene * out_ld + 4 * c4);
-        float4 o = *dst;
+        float4 o = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (beta != 0.0f) {
+            o = *dst;
+            o.x *= beta; o.y *= beta; o.z *= beta; o.w *= beta;
+        }
         o.x = fmaf(alpha, sum.x, o.x); o.y = fmaf(alpha, sum.y, o.y); o.z = fmaf(alpha, sum.z, o.z); o.w = fmaf(alpha, sum.w, o.w);
         *dst = o;
     }
@@ -597,9 +607,9 @@ cb200_status launch_one(const tb_params &p, int sm_count, cudaStream_t stream) {
     const std::int64_t sets = (p.windows + set_windows(NC) - 1) / set_windows(NC);
     const std::int64_t units = sets * p.group_count;
     const unsigned grid = static_cast<unsigned>(units < sm_count ? units : sm_count);
-    qcsr_transpose_blocked_kernel<NC, N, BAKED><<<grid, kThreads, smem, stream>>>(p);
-    ordered_sum_kernel<N, set_windows(NC)><<<static_cast<unsigned>(sets * set_windows(NC)), 256, 0, stream>>>(p.partials, p.out, p.out_ld, p.cols, p.windows, p.group_count,
-                                                                                             static_cast<std::int64_t>(grid), p.alpha);
+    CB200_CUDA_OK(launch_kernel(true, qcsr_transpose_blocked_kernel<NC, N, BAKED>, grid, kThreads, smem, stream, p));
+    CB200_CUDA_OK(launch_kernel(true, ordered_sum_kernel<N, set_windows(NC)>, dim3(static_cast<unsigned>(sets * set_windows(NC))), 256, 0, stream, p.partials, p.out,
+                                p.out_ld, p.cols, p.windows, p.group_count, static_cast<std::int64_t>(grid), p.alpha, p.beta));
     count_launch(2);
     CB200_CUDA_OK(cudaGetLastError());
     return CB200_STATUS_SUCCESS;
@@ -645,27 +655,25 @@ cb200_status launch_qcsr_transpose_blocked(const qcsr_view &x, const dense_args 
         return fail(CB200_STATUS_STALE_STRUCTURE, "the launch's matrix is not the one the window-blocked copy was built from");
 
     *taken = true;
-    // G' = beta * G', also for an empty row range
-    {
+    if (row_end <= row_begin) { // G' = beta * G'
         const std::int64_t total = x.cols * d.n;
         const unsigned grid = static_cast<unsigned>(std::min<std::int64_t>((total + 255) / 256, static_cast<std::int64_t>(sm_count) * 8));
         scale_output_kernel<<<grid, 256, 0, stream>>>(d.out, x.cols, static_cast<int>(d.n), d.out_ld, d.beta);
         count_launch();
         CB200_CUDA_OK(cudaGetLastError());
+        return CB200_STATUS_SUCCESS;
     }
-    if (row_end <= row_begin) return CB200_STATUS_SUCCESS;
 
     int *status = static_cast<int *>(workspace);
     unsigned char *records = static_cast<unsigned char *>(workspace) + 256;
     const std::int64_t group_begin = row_begin / kRows, group_end = (row_end + kRows - 1) / kRows;
-    CB200_CUDA_OK(cudaMemsetAsync(status, 0, sizeof(int), stream));
 
     tb_params p{};
     p.entries = layout.entries; p.seg_ptr = layout.seg_ptr; p.scales = x.scales;
     p.gene_offsets = row_policy ? nullptr : x.offsets; p.row_offsets = row_policy ? x.offsets : nullptr;
     p.records = records; p.out = d.out; p.out_ld = d.out_ld; p.cols = x.cols;
     p.group_begin = group_begin; p.group_count = group_end - group_begin; p.windows = layout.windows;
-    p.alpha = d.alpha; p.status = status;
+    p.alpha = d.alpha; p.beta = d.beta; p.status = status;
     // One pass multiplies bf16(value) with bf16(G).  With split products the fp32 product is rebuilt
     // from hi*hi + hi*lo + lo*hi (v = hi + lo + O(2^-17 v), likewise G): relative error per product
     // about 3 * 2^-17, inside the 1e-4 bound of an fp32 dense operand.  The passes run back to back on
@@ -679,7 +687,8 @@ cb200_status launch_qcsr_transpose_blocked(const qcsr_view &x, const dense_args 
     p.piece_stride = g_piece_bytes(both_parts ? 2 * n : n);
     const auto pack = [&](int part) {
         pack_g_kernel<<<static_cast<unsigned>(group_end - group_begin), 256, 0, stream>>>(static_cast<const float *>(d.dense), d.dense_ld, n, row_begin,
-                                                                                         row_end, group_begin, both_parts ? 1 : 0, part, records);
+                                                                                         row_end, group_begin, both_parts ? 1 : 0, part, records,
+                                                                                         part == 0 ? status : nullptr);
         count_launch();
         return cudaGetLastError();
     };
@@ -693,6 +702,7 @@ cb200_status launch_qcsr_transpose_blocked(const qcsr_view &x, const dense_args 
     CB200_CUDA_OK(pack(0));
     cb200_status st = pass(0);
     if (st != CB200_STATUS_SUCCESS || !split_products) return st;
+    p.beta = 1.0f;
     st = pass(1); // reads the hi part of G: the first N columns of a piece, with or without the others behind them
     if (st != CB200_STATUS_SUCCESS || both_parts) return st;
     CB200_CUDA_OK(pack(1));
