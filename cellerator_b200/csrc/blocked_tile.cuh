@@ -81,22 +81,27 @@ __device__ __forceinline__ std::uint64_t smem_desc(std::uint32_t addr) {
 // (e%8)*2, zero for genes >= cols) followed by 128 x {scale, zero-point}.  part 0 writes
 // hi = bf16(w) (w itself for a bf16 W); part 1 writes lo = bf16(w - hi), the next 8 mantissa bits.
 // both_parts: 2 n columns, hi and then lo.
-// With absmax_bits != null the record holds fp16 instead: hi = fp16(w * s), lo = fp16(w * s - hi), s =
+// With absmax != null (word 1 of the status block: the largest |w|, written here from absmax_kernel's parts) the record holds fp16: hi = fp16(w * s), lo = fp16(w * s - hi), s =
 // operand_scale(largest |w|).  The grid is (windows, column groups): block (w, g) lays out the record's columns [g, g + 1) * n /
 // gridDim.y of window w; the blocks of group 0 also write the window's table.
 constexpr int kPackColumns = 16; // columns of W per block of the packing kernel
 template<typename WT>
 __global__ void __launch_bounds__(256) pack_windows_kernel(const WT *w, std::int64_t ld, std::int64_t cols, int n, int part,
                                                            const float *scales, const float *offsets, int per_gene_offsets,
-                                                           unsigned char *records, const unsigned *absmax_bits = nullptr, int both_parts = 0) {
+                                                           unsigned char *records, unsigned *absmax = nullptr, int both_parts = 0) {
     wait_for_previous_launch();
     let_next_launch_start();
     const std::int64_t window = blockIdx.x;
     const int columns = both_parts != 0 ? 2 * n : n; // both_parts: the hi part of the n columns, then their lo part
     unsigned char *rec = records + window * record_bytes(columns);
     __nv_bfloat16 *wt = reinterpret_cast<__nv_bfloat16 *>(rec);
-    const bool fp16 = absmax_bits != nullptr;
-    const float ws = fp16 ? operand_scale(__uint_as_float(*absmax_bits)) : 1.0f;
+    const bool fp16 = absmax != nullptr;
+    float ws = 1.0f;
+    if (fp16) {
+        const unsigned most = largest_part(absmax + kAbsmaxWord - 1);
+        if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *absmax = most;
+        ws = operand_scale(__uint_as_float(most));
+    }
     const int group_cols = columns / static_cast<int>(gridDim.y), c_first = static_cast<int>(blockIdx.y) * group_cols;
     for (int i = threadIdx.x; i < group_cols * kWin; i += blockDim.x) {
         const int e = i / group_cols, column = c_first + i % group_cols; // consecutive threads read consecutive columns of one gene

@@ -24,9 +24,9 @@ __host__ __device__ __forceinline__ float operand_scale(float absmax) {
     e = e < -100 ? -100 : (e > 100 ? 100 : e);
     return ldexpf(1.0f, 15 - e);
 }
-// Largest magnitude of a dense operand as the bits of a float in *out_bits (zeroed by the caller before).
+// Largest magnitude among a block's share of a dense operand (the whole of it is dealt to `blocks` blocks), for the thread's warp.
 template<typename WT>
-__device__ __forceinline__ void absmax_body(const WT *w, std::int64_t ld, std::int64_t rows, int n, unsigned *out_bits, unsigned block, unsigned blocks) {
+__device__ __forceinline__ float warp_absmax(const WT *w, std::int64_t ld, std::int64_t rows, int n, unsigned block, unsigned blocks) {
     float m = 0.0f;
     const std::int64_t total = rows * n;
     // a contiguous, 16-byte aligned operand is read 16 bytes at a time (the usual case: a launch of the 8,192 x 256
@@ -59,13 +59,32 @@ __device__ __forceinline__ void absmax_body(const WT *w, std::int64_t ld, std::i
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if ((threadIdx.x & 31) == 0 && m > 0.0f) atomicMax(out_bits, __float_as_uint(m)); // non-negative floats order like their bits
+    return m;
 }
+// Largest |W| in parts, one per block, as the bits of floats; the kernel behind it takes the largest of them (largest_part).  No word
+// has to be zeroed before, so this kernel is the first thing of a call; it clears the status word on the way.
+constexpr int kAbsmaxParts = 48; // 180 KB of the largest W (33,538 x 128 bf16) each
+constexpr int kAbsmaxWord = 16;  // first of their words in the status block
 template<typename WT>
-__global__ void __launch_bounds__(256) absmax_kernel(const WT *w, std::int64_t ld, std::int64_t rows, int n, unsigned *out_bits) {
+__global__ void __launch_bounds__(1024) absmax_kernel(const WT *w, std::int64_t ld, std::int64_t rows, int n, unsigned *status_block) {
+    __shared__ unsigned of_warp[32];
     let_next_launch_start();
-    absmax_body(w, ld, rows, n, out_bits, blockIdx.x, gridDim.x);
+    if (blockIdx.x == 0 && threadIdx.x == 0) status_block[0] = 0u;
+    const float m = warp_absmax(w, ld, rows, n, blockIdx.x, gridDim.x);
+    if ((threadIdx.x & 31) == 0) of_warp[threadIdx.x >> 5] = __float_as_uint(m); // non-negative floats order like their bits
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        const unsigned most = __reduce_max_sync(0xffffffffu, of_warp[threadIdx.x]);
+        if (threadIdx.x == 0) status_block[kAbsmaxWord + blockIdx.x] = most;
+    }
 }
+// all lanes of a warp
+__device__ __forceinline__ unsigned largest_part(const unsigned *parts) {
+    const int lane = threadIdx.x & 31;
+    const unsigned a = __ldcg(parts + lane), b = __ldcg(parts + 32 + (lane & (kAbsmaxParts - 33)));
+    return __reduce_max_sync(0xffffffffu, a > b ? a : b);
+}
+static_assert(kAbsmaxParts == 48, "two words a lane, the second of sixteen lanes");
 
 // Largest magnitude a decoded value can take, from the metadata alone: max over genes of |scale| * max code
 // (+ |offset| of the gene) in bound[0], max over rows of |row offset| in bound[1] (row-offset policy), as the
@@ -98,8 +117,10 @@ __global__ void __launch_bounds__(256) operand_bounds_kernel(const __nv_bfloat16
                                                              const float *scales, const float *gene_offsets, const float *row_offsets,
                                                              std::int64_t rows, float max_code, unsigned *w_absmax, unsigned *value_bound) {
     let_next_launch_start();
-    if (blockIdx.x < w_blocks) absmax_body(w, ld, genes, n, w_absmax, blockIdx.x, w_blocks);
-    else value_bound_body(scales, gene_offsets, genes, row_offsets, rows, max_code, value_bound, blockIdx.x - w_blocks);
+    if (blockIdx.x < w_blocks) {
+        const float m = warp_absmax(w, ld, genes, n, blockIdx.x, w_blocks);
+        if ((threadIdx.x & 31) == 0 && m > 0.0f) atomicMax(w_absmax, __float_as_uint(m)); // non-negative floats order like their bits
+    } else value_bound_body(scales, gene_offsets, genes, row_offsets, rows, max_code, value_bound, blockIdx.x - w_blocks);
 }
 
 } // namespace

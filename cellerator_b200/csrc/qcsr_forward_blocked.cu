@@ -1087,12 +1087,11 @@ cb200_status launch_qcsr_forward_blocked(const qcsr_view &x, const dense_args &d
     unsigned char *records = static_cast<unsigned char *>(workspace) + 256;
     const bool row_policy = x.policy == CB200_DECODE_COLUMN_SCALE_ROW_OFFSET;
     const bool half = layout.baked && layout.half_values;
-    CB200_CUDA_OK(cudaMemsetAsync(status, 0, 2 * sizeof(int), stream));
+    if (!half) CB200_CUDA_OK(cudaMemsetAsync(status, 0, sizeof(int), stream));
     if (half) {
-        const std::int64_t elements = x.cols * d.n;
-        const unsigned blocks = static_cast<unsigned>(std::min<std::int64_t>((elements + 1023) / 1024, 4 * static_cast<std::int64_t>(sm_count)));
-        if (w_bf16) absmax_kernel<__nv_bfloat16><<<blocks, 256, 0, stream>>>(static_cast<const __nv_bfloat16 *>(d.dense), d.dense_ld, x.cols, static_cast<int>(d.n), w_absmax);
-        else absmax_kernel<float><<<blocks, 256, 0, stream>>>(static_cast<const float *>(d.dense), d.dense_ld, x.cols, static_cast<int>(d.n), w_absmax);
+        unsigned *words = static_cast<unsigned *>(workspace);
+        if (w_bf16) absmax_kernel<__nv_bfloat16><<<kAbsmaxParts, 1024, 0, stream>>>(static_cast<const __nv_bfloat16 *>(d.dense), d.dense_ld, x.cols, static_cast<int>(d.n), words);
+        else absmax_kernel<float><<<kAbsmaxParts, 1024, 0, stream>>>(static_cast<const float *>(d.dense), d.dense_ld, x.cols, static_cast<int>(d.n), words);
         count_launch();
         CB200_CUDA_OK(cudaGetLastError());
     }

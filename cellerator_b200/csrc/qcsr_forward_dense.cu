@@ -332,11 +332,10 @@ cb200_status launch_qcsr_forward_dense(const qcsr_view &x, const dense_args &d, 
     unsigned *w_absmax = reinterpret_cast<unsigned *>(workspace) + 1; // fp16 operands: float bits of the largest |W|
     unsigned char *records = static_cast<unsigned char *>(workspace) + 256;
     const bool half = layout.half_values;
-    CB200_CUDA_OK(cudaMemsetAsync(status, 0, 2 * sizeof(int), stream));
+    if (!half) CB200_CUDA_OK(cudaMemsetAsync(status, 0, sizeof(int), stream));
     if (half) {
-        const std::int64_t elements = x.cols * d.n;
-        const unsigned blocks = static_cast<unsigned>(std::min<std::int64_t>((elements + 1023) / 1024, 4 * static_cast<std::int64_t>(sm_count)));
-        absmax_kernel<__nv_bfloat16><<<blocks, 256, 0, stream>>>(static_cast<const __nv_bfloat16 *>(d.dense), d.dense_ld, x.cols, static_cast<int>(d.n), w_absmax);
+        absmax_kernel<__nv_bfloat16><<<kAbsmaxParts, 1024, 0, stream>>>(static_cast<const __nv_bfloat16 *>(d.dense), d.dense_ld, x.cols, static_cast<int>(d.n),
+                                                                      static_cast<unsigned *>(workspace));
         count_launch();
         CB200_CUDA_OK(cudaGetLastError());
     }
