@@ -81,9 +81,10 @@ __device__ __forceinline__ std::uint64_t smem_desc(std::uint32_t addr) {
 // (e%8)*2, zero for genes >= cols) followed by 128 x {scale, zero-point}.  part 0 writes
 // hi = bf16(w) (w itself for a bf16 W); part 1 writes lo = bf16(w - hi), the next 8 mantissa bits.
 // both_parts: 2 n columns, hi and then lo.
-// With absmax != null (word 1 of the status block: the largest |w|, written here from absmax_kernel's parts) the record holds fp16: hi = fp16(w * s), lo = fp16(w * s - hi), s =
-// operand_scale(largest |w|).  The grid is (windows, column groups): block (w, g) lays out the record's columns [g, g + 1) * n /
-// gridDim.y of window w; the blocks of group 0 also write the window's table.
+// With absmax != null the record holds fp16: hi = fp16(w * s), lo = fp16(w * s - hi), s = operand_scale(largest |w|).
+// absmax is word 1 of the status block: the largest |w|, written here from absmax_kernel's parts.
+// The grid is (windows, column groups): block (w, g) lays out the record's columns [g, g + 1) * columns / gridDim.y of window
+// w; the blocks of group 0 also write the window's table.
 constexpr int kPackColumns = 16; // columns of W per block of the packing kernel
 template<typename WT>
 __global__ void __launch_bounds__(256) pack_windows_kernel(const WT *w, std::int64_t ld, std::int64_t cols, int n, int part,
