@@ -203,7 +203,8 @@ cb200_status launch_qcsr_transpose_blocked(const qcsr_view &x, const dense_args 
 cb200_status launch_qcsr_transpose(const qcsr_view &x, const dense_args &d, std::int64_t row_begin,
                                    std::int64_t row_end, const blocked_layout *blocked, bool split_products,
                                    void *workspace, std::uint64_t workspace_bytes, int sm_count, cudaStream_t stream);
-// What the fp32-FMA transpose can use; without it every entry is added in L2 on its own.
+// What the fp32-FMA transpose can use, 32 MB at most; with less it takes the rows in smaller slices, and without it every
+// entry is added in L2 on its own.
 std::uint64_t qcsr_transpose_workspace_bytes(std::int64_t rows, std::int64_t cols, int sm_count);
 // Entries sorted by gene in shared memory, tile by tile of G; *taken is false where the shape or the workspace rules it out.
 std::uint64_t qcsr_transpose_tiled_workspace_bytes(std::int64_t rows, std::int64_t cols, int sm_count);

@@ -59,6 +59,7 @@ struct tiled_transpose_params {
     int start_rows;       // rows per CTA of the pass over the indices
     int pairs;            // column tiles x tiles x ranges
     int out_vector;       // rows of G' take 16-byte reductions
+    int scale_output;     // the pass over the indices also sets G' to beta * G'
 };
 
 // starts[j][row] for every range j, and G' = beta * G'.  An entry whose range lies beyond the one of the entry before it is a
@@ -118,6 +119,7 @@ __global__ void __launch_bounds__(kTileThreads) transpose_starts_kernel(const ti
         for (int j = warp; j <= p.ranges; j += kTileWarps)
             if (lane < rows) p.starts[static_cast<std::int64_t>(j) * p.rows + row0 + lane] = transpose_starts[j * (kStartRows + 1) + lane];
     }
+    if (p.scale_output == 0) return;
     const std::int64_t total = p.cols * p.n;
     for (std::int64_t i = static_cast<std::int64_t>(blockIdx.x) * kTileThreads + threadIdx.x; i < total; i += static_cast<std::int64_t>(gridDim.x) * kTileThreads) {
         float *dst = p.out + (i / p.n) * p.out_ld + i % p.n;
@@ -361,12 +363,27 @@ int ranges_for(std::int64_t cols, int tiles, int sm_count) {
     return static_cast<int>(std::max<std::int64_t>(least, std::min<std::int64_t>({waves * sm_count / tiles, cols, kMaxRanges})));
 }
 
+// The starts of a launch over `rows` rows.  T = column tiles x tiles of 512 rows take at most least + (sm_count - 1) / T ranges
+// (ranges_for), and rows <= 512 T: (ranges + 1) * rows is at most (least + 1) * rows + 512 * sm_count.
+std::uint64_t starts_bytes(std::int64_t rows, int least, int sm_count) {
+    return (static_cast<std::uint64_t>(least + 1) * static_cast<std::uint64_t>(rows) + static_cast<std::uint64_t>(kTileRows) * static_cast<std::uint64_t>(sm_count)) * 4u;
+}
+// A launch over more rows than the workspace holds the starts of takes them slice by slice.  A slice is dear only
+// when it has few tiles: 400,000 x 33,538 at N = 64 take 15.3 ms in four slices (32 MB of starts), 15.1 in 28 (4 MB) and 15.5 in 61.
+constexpr std::uint64_t kMostStartsBytes = 32ull << 20;
+constexpr std::int64_t kLeastSlice = 8 * kTileRows;
+std::int64_t slice_rows(std::int64_t rows, int least, std::uint64_t bytes, int sm_count) {
+    if (bytes >= starts_bytes(rows, least, sm_count)) return rows;
+    const std::uint64_t fixed = starts_bytes(0, least, sm_count);
+    if (bytes < fixed) return 0;
+    return static_cast<std::int64_t>((bytes - fixed) / (4u * static_cast<std::uint64_t>(least + 1))) / kTileRows * kTileRows;
+}
+
 } // namespace
 
 std::uint64_t qcsr_transpose_tiled_workspace_bytes(std::int64_t rows, std::int64_t cols, int sm_count) {
     if (rows == 0 || cols == 0 || fewest_ranges(cols) > kMaxRanges) return 0u;
-    const int least = fewest_ranges(cols); // a launch has at most least + sm_count ranges
-    return 256u + static_cast<std::uint64_t>(std::min(least + sm_count, kMaxRanges) + 1) * static_cast<std::uint64_t>(rows) * 4u;
+    return 256u + std::min(starts_bytes(rows, fewest_ranges(cols), sm_count), kMostStartsBytes);
 }
 
 cb200_status launch_qcsr_transpose_tiled(const qcsr_view &x, const dense_args &d, std::int64_t row_begin, std::int64_t row_end,
@@ -374,41 +391,55 @@ cb200_status launch_qcsr_transpose_tiled(const qcsr_view &x, const dense_args &d
     *taken = false;
     const std::int64_t rows = row_end - row_begin;
     if (rows <= 0 || x.nnz == 0 || workspace == nullptr || (x.bits == 4 && x.packed_row_ptr == nullptr)) return CB200_STATUS_SUCCESS;
-    const std::uint64_t need = qcsr_transpose_tiled_workspace_bytes(rows, x.cols, sm_count);
-    // (32-bit places among the entries of 512 rows)
-    if (need == 0u || workspace_bytes < need || x.cols > (1ll << 21) || rows > 0x3fffffff) return CB200_STATUS_SUCCESS;
-    tiled_transpose_params p{};
-    p.tiles = static_cast<int>((rows + kTileRows - 1) / kTileRows);
-    p.tile_rows = static_cast<int>((rows + p.tiles - 1) / p.tiles);
-    const double entries = static_cast<double>(x.nnz) / static_cast<double>(x.rows) * static_cast<double>(rows);
-    // a gene needs a few entries per tile to be worth its turn, and the sort a few thousand entries to be worth its barriers
-    if (entries < 50000.0 || entries / static_cast<double>(rows) * p.tile_rows < 3.0 * static_cast<double>(x.cols)) return CB200_STATUS_SUCCESS;
+    const int least = fewest_ranges(x.cols);
+    if (least > kMaxRanges || workspace_bytes <= 256u || x.cols > (1ll << 21)) return CB200_STATUS_SUCCESS;
+    const std::int64_t most = slice_rows(rows, least, std::min(workspace_bytes - 256u, kMostStartsBytes), sm_count);
+    if (most < std::min(rows, kLeastSlice)) return CB200_STATUS_SUCCESS;
+    // equal slices, of whole tiles but for the last
+    const std::int64_t slices = (rows + most - 1) / most;
+    const std::int64_t slice = slices == 1 ? rows : std::min(most, ((rows + slices - 1) / slices + kTileRows - 1) / kTileRows * kTileRows);
     const int nc = d.n <= 32 ? 32 : 64;
     const int column_tiles = static_cast<int>((d.n + nc - 1) / nc);
-    p.ranges = ranges_for(x.cols, p.tiles * column_tiles, sm_count);
-    p.width = static_cast<int>((x.cols + p.ranges - 1) / p.ranges);
-    p.ranges = static_cast<int>((x.cols + p.width - 1) / p.width);
-    const std::int64_t pairs = static_cast<std::int64_t>(column_tiles) * p.tiles * p.ranges;
-    if (pairs > 0x7fffffff) return CB200_STATUS_SUCCESS;
-    p.pairs = static_cast<int>(pairs);
+    {
+        const std::int64_t tiles = (slice + kTileRows - 1) / kTileRows;
+        const std::int64_t tile_rows = (slice + tiles - 1) / tiles;
+        const double per_row = static_cast<double>(x.nnz) / static_cast<double>(x.rows);
+        // a gene needs a few entries per tile to be worth its turn, and the sort a few thousand entries to be worth its barriers
+        if (per_row * static_cast<double>(rows) < 50000.0 || per_row * static_cast<double>(tile_rows) < 3.0 * static_cast<double>(x.cols)) return CB200_STATUS_SUCCESS;
+        if (static_cast<std::int64_t>(column_tiles) * tiles * kMaxRanges > 0x7fffffff) return CB200_STATUS_SUCCESS;
+    }
+    tiled_transpose_params p{};
     p.row_ptr = x.row_ptr; p.packed_row_ptr = x.packed_row_ptr; p.col_idx = x.col_idx; p.packed = x.packed; p.scales = x.scales;
     p.offsets = x.offsets; p.g = static_cast<const float *>(d.dense); p.out = d.out; p.g_ld = d.dense_ld; p.out_ld = d.out_ld;
-    p.row_begin = row_begin; p.rows = rows; p.cols = x.cols; p.n = static_cast<int>(d.n); p.policy = x.policy;
-    p.alpha = d.alpha; p.beta = d.beta;
+    p.cols = x.cols; p.n = static_cast<int>(d.n); p.policy = x.policy; p.alpha = d.alpha; p.beta = d.beta;
     p.status = static_cast<int *>(workspace);
     p.starts = reinterpret_cast<std::int32_t *>(static_cast<unsigned char *>(workspace) + 256);
     p.out_vector = reinterpret_cast<std::uintptr_t>(d.out) % 16u == 0u && d.out_ld % 4 == 0 && d.n % 4 == 0 ? 1 : 0;
-    const std::size_t smem = static_cast<std::size_t>(p.ranges + 1) * (kStartRows + 1) * sizeof(int);
-    if (smem > 48u * 1024u)
-        CB200_CUDA_OK(cudaFuncSetAttribute(transpose_starts_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-    p.start_rows = rows >= 32ll * sm_count ? kStartRows : 8;
-    const unsigned grid = static_cast<unsigned>(std::max<std::int64_t>((rows + p.start_rows - 1) / p.start_rows, sm_count));
-    transpose_starts_kernel<<<grid, kTileThreads, smem, stream>>>(p);
-    count_launch();
-    CB200_CUDA_OK(cudaGetLastError());
     *taken = true;
-    if (x.bits == 8) return nc == 32 ? launch_tiles<8, 32>(p, sm_count, stream) : launch_tiles<8, 64>(p, sm_count, stream);
-    return nc == 32 ? launch_tiles<4, 32>(p, sm_count, stream) : launch_tiles<4, 64>(p, sm_count, stream);
+    for (std::int64_t first = row_begin; first < row_end; first += slice) {
+        p.row_begin = first;
+        p.rows = std::min(slice, row_end - first);
+        p.tiles = static_cast<int>((p.rows + kTileRows - 1) / kTileRows);
+        p.tile_rows = static_cast<int>((p.rows + p.tiles - 1) / p.tiles);
+        p.ranges = ranges_for(x.cols, p.tiles * column_tiles, sm_count);
+        p.width = static_cast<int>((x.cols + p.ranges - 1) / p.ranges);
+        p.ranges = static_cast<int>((x.cols + p.width - 1) / p.width);
+        p.pairs = column_tiles * p.tiles * p.ranges;
+        p.scale_output = first == row_begin ? 1 : 0;
+        const std::size_t smem = static_cast<std::size_t>(p.ranges + 1) * (kStartRows + 1) * sizeof(int);
+        if (smem > 48u * 1024u)
+            CB200_CUDA_OK(cudaFuncSetAttribute(transpose_starts_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+        p.start_rows = p.rows >= 32ll * sm_count ? kStartRows : 8;
+        const unsigned grid = static_cast<unsigned>(std::max<std::int64_t>((p.rows + p.start_rows - 1) / p.start_rows, sm_count));
+        transpose_starts_kernel<<<grid, kTileThreads, smem, stream>>>(p);
+        count_launch();
+        CB200_CUDA_OK(cudaGetLastError());
+        cb200_status st;
+        if (x.bits == 8) st = nc == 32 ? launch_tiles<8, 32>(p, sm_count, stream) : launch_tiles<8, 64>(p, sm_count, stream);
+        else st = nc == 32 ? launch_tiles<4, 32>(p, sm_count, stream) : launch_tiles<4, 64>(p, sm_count, stream);
+        if (st != CB200_STATUS_SUCCESS) return st;
+    }
+    return CB200_STATUS_SUCCESS;
 }
 
 } // namespace cb200

@@ -40,3 +40,33 @@ def test_against_oracle(cuda_device, oracle, rows, cols, max_nnz, n, bits, polic
     # without a workspace the entries are added one by one
     op.workspace, op.workspace_bytes = None, 0
     assert_transpose_close(op.run(x, g, torch.empty(cols, n, device=cuda_device)).cpu().numpy(), oracle.qcsr_transpose(*args), cl1, gmax)
+
+
+def test_workspace_does_not_grow_with_the_matrix(cuda_device):
+    """1,000,000 x 33,538, 1.8e9 entries: the rows are taken in slices."""
+    op = ops.PreparedSpmm(capi.PROJECTION_TRANSPOSE, 1_000_000, 33_538, 64, 1_800_000_000, 8, 1, torch.float32, cuda_device)
+    assert op.schedule == "vector_reductions" and 256 < op.workspace_bytes <= 40 << 20
+    op.close()
+
+
+@pytest.mark.parametrize("rows", [4096 * 2, 4096 * 3 + 77])
+def test_slices_against_oracle(cuda_device, oracle, rows):
+    """A workspace for the starts of 4,096 rows at a time; alpha / beta count once; a row range cut into slices of its own."""
+    rng = np.random.default_rng(rows)
+    cols, n, bits, policy = 1025, 36, 8, 1
+    c = host_pack(oracle, random_csr(rng, rows=rows, cols=cols, max_nnz=60, bits=bits, policy=policy))
+    x = to_dev(c, cuda_device)
+    g, g_host = dense(rng, rows, n, torch.float32, cuda_device, std=1.0)
+    op = ops.PreparedSpmm(capi.PROJECTION_TRANSPOSE, rows, cols, n, x.nnz, bits, policy, torch.float32, cuda_device)
+    sms = torch.cuda.get_device_properties(cuda_device).multi_processor_count
+    op.workspace_bytes = 256 + 4 * ((3 + 1) * 4096 + 512 * sms)
+    cl1, gmax = col_l1_of(oracle, c), float(np.abs(g_host).max())
+    args = (bits, policy, c["row_ptr"], c["packed_row_ptr"], c["col_idx"], c["packed"], c["scales"], c["offsets"], g_host, cols)
+    init = torch.from_numpy(rng.normal(size=(cols, n)).astype(np.float32)).to(cuda_device)
+    launches = capi.lib().cb200_kernel_launch_count()
+    out = op.run(x, g, init.clone(), alpha=2.0, beta=0.5).cpu().numpy()
+    assert capi.lib().cb200_kernel_launch_count() - launches == 2 * -(-rows // 4096) and op.status() == 0
+    assert_transpose_close(out, 2.0 * oracle.qcsr_transpose(*args) + 0.5 * init.cpu().numpy(), 2.0 * cl1 + 1.0, gmax)
+    lo, hi = 5, rows - 9
+    part = op.run(x, g, torch.full_like(init, float("nan")), row_begin=lo, row_end=hi).cpu().numpy()
+    assert_transpose_close(part, oracle.qcsr_transpose(*args, lo, hi), cl1, gmax)
