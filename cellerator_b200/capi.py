@@ -241,7 +241,7 @@ EXPORTED_SYMBOLS = [
     "cb200_bell_lowering_workspace", "cb200_bell_lowering_query", "cb200_bell_lowering_materialize",
     "cb200_pack_dense_operand", "cb200_build_execution_csr",
     "cb200_qcsr_gene_major_workspace", "cb200_qcsr_gene_major",
-    "cb200_public_projection_scratch", "cb200_public_projection_forward", "cb200_public_projection_backward_rhs",
+    "cb200_public_projection_scratch", "cb200_public_projection_backward_scratch", "cb200_public_projection_forward", "cb200_public_projection_backward_rhs",
     "cb200_session_create", "cb200_session_reserve_persistent", "cb200_session_reserve_transient",
     "cb200_session_seal", "cb200_session_bind", "cb200_session_synchronize", "cb200_session_destroy",
     "cb200_find_in_row", "cb200_get_code", "cb200_get_value", "cb200_get_values",

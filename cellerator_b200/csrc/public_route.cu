@@ -175,9 +175,9 @@ cb200_status route(const cb200_public_layout *l, int32_t projection, const float
     std::uint32_t align = 256;
     cb200_prepared_workspace(prepared, &need, &align);
     // the exact fp32 schedules these calls select need the status block only; what a CSR projection could use beyond it is not
-    // in the scratch these calls ask for
+    // in the scratch these calls ask for, and the transpose sorts its entries with what the caller's scratch holds beyond it
     if (projection == CB200_PROJECTION_CSR) need = std::min<std::uint64_t>(need, 256u);
-    if (projection == CB200_PROJECTION_TRANSPOSE && (need + 255u) / 256u * 256u > cur.left) need = 0u; // runs without
+    if (projection == CB200_PROJECTION_TRANSPOSE) need = std::min<std::uint64_t>(need, cur.left / 256u * 256u);
     void *ws = need == 0u ? nullptr : (need <= 256u ? status_block : cur.take(need));
     if (need != 0u && ws == nullptr) {
         cb200_prepared_destroy(prepared);
@@ -210,9 +210,17 @@ extern "C" cb200_status cb200_public_projection_scratch(const cb200_public_layou
     // widened row offsets (CSR) + the status block of the fp32 schedules these calls select
     const std::uint64_t offsets = layout->layout == CB200_PUBLIC_LAYOUT_QUANTIZED_CSR ? (static_cast<std::uint64_t>(layout->rows) + 1u) * 8u : 0u;
     const std::uint64_t arrays = layout->layout == CB200_PUBLIC_LAYOUT_QUANTIZED_CSR && layout->bits == 4u ? 2u : 1u; // + packed row offsets
-    // ... and what the transpose sorts its entries with
-    const std::uint64_t transpose = offsets != 0u ? qcsr_transpose_tiled_workspace_bytes(layout->rows, layout->cols, 160) : 0u;
-    *bytes = arrays * ((offsets + 255u) / 256u * 256u) + 512u + (transpose + 255u) / 256u * 256u;
+    *bytes = arrays * ((offsets + 255u) / 256u * 256u) + 512u;
+    return CB200_STATUS_SUCCESS;
+}
+
+extern "C" cb200_status cb200_public_projection_backward_scratch(const cb200_public_layout *layout, int64_t out_cols, uint64_t *bytes) {
+    using namespace cb200;
+    const cb200_status st = cb200_public_projection_scratch(layout, out_cols, bytes);
+    if (st != CB200_STATUS_SUCCESS || layout->layout != CB200_PUBLIC_LAYOUT_QUANTIZED_CSR) return st;
+    // ... and what the transpose sorts its entries with, on the largest device this library is built for
+    constexpr int kMostSms = 160;
+    *bytes += (qcsr_transpose_tiled_workspace_bytes(layout->rows, layout->cols, kMostSms) + 255u) / 256u * 256u;
     return CB200_STATUS_SUCCESS;
 }
 

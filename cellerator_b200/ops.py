@@ -611,7 +611,8 @@ def public_projection(x, dense: torch.Tensor, backward=False) -> torch.Tensor:
     l = public_layout(x)
     n = dense.shape[1]
     need = C.c_uint64()
-    capi.check(capi.lib().cb200_public_projection_scratch(C.byref(l), C.c_int64(n), C.byref(need)))
+    scratch_of = capi.lib().cb200_public_projection_backward_scratch if backward else capi.lib().cb200_public_projection_scratch
+    capi.check(scratch_of(C.byref(l), C.c_int64(n), C.byref(need)))
     scratch = torch.empty(need.value, dtype=torch.uint8, device=dense.device)
     out = torch.empty(x.cols if backward else x.rows, n, dtype=torch.float32, device=dense.device)
     fn = capi.lib().cb200_public_projection_backward_rhs if backward else capi.lib().cb200_public_projection_forward

@@ -687,6 +687,8 @@ typedef struct cb200_public_layout {
 
 /* scratch the calls below need for this layout (device memory, 256-byte aligned); they never allocate */
 cb200_status cb200_public_projection_scratch(const cb200_public_layout *layout, int64_t out_cols, uint64_t *bytes);
+/* the same with room for the sort of cb200_public_projection_backward_rhs (up to 32 MB; that call runs with less, slower) */
+cb200_status cb200_public_projection_backward_scratch(const cb200_public_layout *layout, int64_t out_cols, uint64_t *bytes);
 /* out[rows, out_cols] = deq(X) * rhs[cols, out_cols]; fp32 row-major operands with leading dimensions
  * (matrix_ld_ of abi.cu), exact fp32 products; enqueues on `stream` */
 cb200_status cb200_public_projection_forward(const cb200_public_layout *layout, const float *rhs, int64_t rhs_ld,

@@ -37,6 +37,26 @@ def test_quantized_csr_forward_and_backward(cuda_device, oracle, policy, n, bits
     assert float((gr - direct).abs().max()) <= 1e-5 * float(direct.abs().max())
 
 
+def test_backward_with_the_forwards_scratch(cuda_device, oracle):
+    """A binding that asks for the forward's scratch gets the transpose entry by entry."""
+    rng = np.random.default_rng(5)
+    c = host_pack(oracle, random_csr(rng, rows=2000, cols=700, max_nnz=120, bits=8, policy=1))
+    x = to_dev(c, cuda_device)
+    assert x.nnz >= 50_000
+    g, _ = dense(rng, 2000, 32, torch.float32, cuda_device, std=1.0)
+    lib, l, need, word = capi.lib(), ops.public_layout(x), C.c_uint64(), C.c_int32(-1)
+    assert lib.cb200_public_projection_scratch(C.byref(l), C.c_int64(32), C.byref(need)) == 0
+    scratch = torch.empty(need.value, dtype=torch.uint8, device=cuda_device)
+    out = torch.full((700, 32), float("nan"), device=cuda_device)
+    stream = torch.cuda.current_stream(cuda_device).cuda_stream
+    assert lib.cb200_public_projection_backward_rhs(
+        C.byref(l), C.c_void_p(g.data_ptr()), C.c_int64(32), C.c_int64(32), C.c_void_p(out.data_ptr()), C.c_int64(32), C.c_int32(0),
+        C.c_void_p(stream), C.c_void_p(scratch.data_ptr()), C.c_uint64(need.value)) == 0
+    direct = ops.public_projection(x, g, backward=True)
+    assert float((out - direct).abs().max()) <= 1e-5 * float(direct.abs().max())
+    assert lib.cb200_public_projection_status(C.c_void_p(scratch.data_ptr()), C.c_int32(0), C.c_void_p(stream), C.byref(word)) == 0
+
+
 def test_quantized_blocked_ell_forward(cuda_device, oracle):
     rng = np.random.default_rng(8)
     h = synth.make_qbell_host(32 * 9 + 5, 1000, 32, 4, 0.6, 8, seed=3)

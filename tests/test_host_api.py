@@ -183,3 +183,20 @@ def test_gene_gap_encoding_round_trip(case, threads):
                                              genes.ctypes.data, count - 1, threads) == -1
     assert L.cb200_host_encode_gene_gaps(col.ctypes.data, ptr.ctypes.data, len(ptr) - 1, gaps.ctypes.data, positions.ctypes.data,
                                          genes.ctypes.data, n + 1, 0) == -2
+
+
+@pytest.mark.parametrize("bits", [8, 4])
+def test_routed_scratch_is_what_the_calls_use(bits):
+    """The forward call uses its row offsets and a status block; the transpose's sort is asked for on its own, and bounded."""
+    L = capi.lib()
+    l = capi.header(capi.PublicLayout())
+    l.layout, l.rows, l.cols, l.nnz, l.bits, l.decode_policy = capi.PUBLIC_LAYOUT_QUANTIZED_CSR, 1_000_000, 33_538, 1_800_000_000, bits, 1
+    l.major_ptr = l.minor_idx = l.packed_values = 256                     # addresses that the call does not follow
+    need, back = C.c_uint64(), C.c_uint64()
+    assert L.cb200_public_projection_scratch(C.byref(l), C.c_int64(64), C.byref(need)) == capi.SUCCESS
+    offsets = 8 * (l.rows + 1) * (2 if bits == 4 else 1)
+    assert offsets + 512 <= need.value <= offsets + 1024
+    assert L.cb200_public_projection_backward_scratch(C.byref(l), C.c_int64(64), C.byref(back)) == capi.SUCCESS
+    assert need.value < back.value <= need.value + (40 << 20)
+    l.layout, l.block_size, l.ell_cols, l.block_col_idx = capi.PUBLIC_LAYOUT_QUANTIZED_BLOCKED_ELL, 32, 64, 256
+    assert L.cb200_public_projection_scratch(C.byref(l), C.c_int64(64), C.byref(need)) == capi.SUCCESS and need.value <= 512
