@@ -105,7 +105,7 @@ struct w_slice {
 constexpr int kGatherRuns = 2;      // runs of 32 entries a warp decodes at a time
 constexpr int kSegment = 32 * kGatherRuns;
 constexpr int kGatherMaxWarps = 16; // most warps per CTA
-constexpr int kGatherMaxRows = 32;  // most rows per CTA
+constexpr int kGatherMaxRows = 8;   // most rows per CTA
 constexpr int kGatherParts = 64;    // most sums of parts the shared memory of a CTA holds
 constexpr int kRowParts = 16;       // most parts of a row
 constexpr int kPartEntries = 128;   // entries of a part, for rows of up to 16 of them
@@ -127,20 +127,25 @@ __device__ __forceinline__ std::int32_t load_index_once(const std::int32_t *src)
 // Rows of W gathered straight into registers, for any N and any leading dimension.
 //
 // A row of X is cut into parts by its length alone (about 128 entries each, 16 parts at most), and the row's sum is the sum of
-// its parts in order: the same bits whatever rows stand beside it and whichever of the two kernels below runs.  A warp
-// decodes 64 entries at a time, two per lane with coalesced loads (the raw pairs of the next 64 are in flight meanwhile),
-// into a staging line of {gene, value}; then a group of `lanes` lanes serves one entry, a lane holding V columns (16 bytes
-// where N and the operand's alignment allow), so one load instruction brings 32 / lanes rows of W.
+// its parts in order.  A warp decodes 64 entries at a time, two per lane with coalesced loads (the raw pairs of the next 64 are
+// in flight meanwhile), into a staging line of {gene, value}; then a group of `lanes` lanes serves one entry, a lane holding V
+// columns (16 bytes where N and the operand's alignment allow), so one load instruction brings 32 / lanes rows of W.
+//
+// The order of a part's sum follows from N and W's type alone (summing_lanes): entry e belongs to class e modulo C, a class is
+// summed in order, the classes pairwise.  With 16-byte slices the classes are the C groups of lanes; narrower ones leave
+// 32 / lanes groups, each of which keeps SETS = C * lanes / 32 sums.  So a row's sum has the same bits whatever rows stand
+// beside it, whichever of the two kernels below runs, and whether W was re-laid: in a shard, a chunk, a routed call.
 //
 // What bounds it: rows of W out of L2 (33,538 x 64 bf16: 12.4 TB/s at 125,000 rows of 1,800 entries, 96 Gnnz/s) or, where W
 // fits L1, instruction issue (2,000 x 32 fp32, 20,000 rows of 360: 82 Gnnz/s).  Before, a row was one warp's work from end to
 // end (600 us for 4,099 x 1,800 at N = 64, now 110: the longest row decided) or one lane group's in the gene-tiled kernel (820
 // us for 20,000 x 340 at N = 32, now 84: 40 CTAs for 148 SMs), and a width that is no power of two went column by column
 // through 2-byte loads (2.6 ms for 4,099 x 1,800 at N = 50 bf16, now 118 us).
-template<int BITS, typename WT, int V, int RUNS>
+template<int BITS, typename WT, int V, int SETS, int RUNS>
 struct gather_warp {
     static constexpr int SEG = 32 * RUNS; // entries decoded at a time
     static constexpr int U = V * sizeof(WT) > 4 ? 4 : 8; // rows of W in flight per lane
+    static_assert(U % SETS == 0 && SETS * V * sizeof(WT) <= 16, "a batch holds every class equally often");
     // 32 x 32 -> 64-bit products for the addresses; operands whose rows lie 4 GB or more apart are served with V == 1
     using stride_t = typename std::conditional<V == 1, std::uint64_t, std::uint32_t>::type;
 
@@ -151,7 +156,7 @@ struct gather_warp {
     bool row_policy;
     const unsigned char *wcol;
     stride_t w_row_bytes;
-    float acc[V];
+    float acc[SETS][V];
     int gene[RUNS];
     unsigned code[RUNS];
     float scale[RUNS], offset[RUNS];
@@ -170,7 +175,10 @@ struct gather_warp {
     }
     __device__ __forceinline__ void clear() {
 #pragma unroll
-        for (int i = 0; i < V; ++i) acc[i] = 0.0f;
+        for (int k = 0; k < SETS; ++k) {
+#pragma unroll
+            for (int i = 0; i < V; ++i) acc[k][i] = 0.0f;
+        }
     }
     __device__ __forceinline__ const unsigned char *w_at(int g) const {
         return wcol + static_cast<std::uint64_t>(static_cast<std::uint32_t>(g)) * w_row_bytes;
@@ -232,9 +240,9 @@ struct gather_warp {
                 w[u].load(w_at(e.x));
             }
 #pragma unroll
-            for (int u = 0; u < U; ++u) w[u].fma_into(acc, v[u]);
+            for (int u = 0; u < U; ++u) w[u].fma_into(acc[u % SETS], v[u]);
         }
-        constexpr int T = U / 2;
+        constexpr int T = U / 2 > SETS ? U / 2 : SETS;
         for (; done < count; done += T * per_step) { // entries past the end add nothing
             w_slice<WT, V> w[T];
             float v[T];
@@ -248,15 +256,26 @@ struct gather_warp {
 #pragma unroll
             for (int u = 0; u < T; ++u) {
                 if (done + u * per_step + group >= count) w[u].zero();
-                w[u].fma_into(acc, v[u]);
+                w[u].fma_into(acc[u % SETS], v[u]);
             }
         }
     }
-    // the lane groups' sums together; every group then holds the whole
+    // the classes' sums together, in acc[0] of every lane group
     __device__ __forceinline__ void reduce() {
         for (int off = lanes; off < 32; off <<= 1) {
 #pragma unroll
-            for (int i = 0; i < V; ++i) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], off);
+            for (int k = 0; k < SETS; ++k) {
+#pragma unroll
+                for (int i = 0; i < V; ++i) acc[k][i] += __shfl_xor_sync(0xffffffffu, acc[k][i], off);
+            }
+        }
+#pragma unroll
+        for (int step = 1; step < SETS; step <<= 1) {
+#pragma unroll
+            for (int k = 0; k < SETS; k += 2 * step) {
+#pragma unroll
+                for (int i = 0; i < V; ++i) acc[k][i] += acc[k + step][i];
+            }
         }
     }
     __device__ __forceinline__ void write_row(std::int64_t row, float (&v)[V]) const {
@@ -295,7 +314,7 @@ struct gather_warp {
 
 // A warp per row: no tables, no barriers.  For rows of a few entries (RUNS == 1: 32 at a time) and narrow operands, where the
 // other kernel's start and end cost more than the entries.
-template<int BITS, typename WT, int V, int RUNS>
+template<int BITS, typename WT, int V, int SETS, int RUNS>
 __global__ void __launch_bounds__(128, 8) qcsr_fwd_row_kernel(const fwd_params p) {
     constexpr int SEG = 32 * RUNS;
     __shared__ __align__(16) int2 staging[4][SEG];
@@ -303,7 +322,7 @@ __global__ void __launch_bounds__(128, 8) qcsr_fwd_row_kernel(const fwd_params p
     if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 && p.status != nullptr) *p.status = 0;
     const std::int64_t row = p.row_begin + static_cast<std::int64_t>(blockIdx.x) * 4 + warp;
     if (row >= p.row_end) return;
-    gather_warp<BITS, WT, V, RUNS> g(p, staging[warp]);
+    gather_warp<BITS, WT, V, SETS, RUNS> g(p, staging[warp]);
     const std::int64_t start = __ldg(p.row_ptr + row);
     const int len = static_cast<int>(__ldg(p.row_ptr + row + 1) - start);
     const std::int32_t *cols = p.col_idx + start;
@@ -327,7 +346,7 @@ __global__ void __launch_bounds__(128, 8) qcsr_fwd_row_kernel(const fwd_params p
         if (!part_done) continue;
         g.reduce();
 #pragma unroll
-        for (int i = 0; i < V; ++i) total[i] = first ? g.acc[i] : total[i] + g.acc[i];
+        for (int i = 0; i < V; ++i) total[i] = first ? g.acc[0][i] : total[i] + g.acc[0][i];
         first = false;
         g.clear();
         if (at >= len) break;
@@ -338,7 +357,7 @@ __global__ void __launch_bounds__(128, 8) qcsr_fwd_row_kernel(const fwd_params p
 // A CTA owns `group_rows` consecutive rows and deals their parts to its warps, so that a long row does not hold up the
 // others; sums of parts meet in shared memory.
 // SHORT_END: the CTAs from p.full_groups on take a quarter of the rows.
-template<int BITS, typename WT, int V, bool SHORT_END>
+template<int BITS, typename WT, int V, int SETS, bool SHORT_END>
 __global__ void __launch_bounds__(kGatherMaxWarps * 32, 2) qcsr_fwd_gather_kernel(const fwd_params p) {
     __shared__ std::int64_t row_start[kGatherMaxRows], code_start[kGatherMaxRows];
     __shared__ int row_len[kGatherMaxRows], row_share[kGatherMaxRows], first_part[kGatherMaxRows + 1];
@@ -375,7 +394,7 @@ __global__ void __launch_bounds__(kGatherMaxWarps * 32, 2) qcsr_fwd_gather_kerne
     }
     if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 && p.status != nullptr) *p.status = 0;
     __syncthreads();
-    gather_warp<BITS, WT, V, kGatherRuns> g(p, staging + warp * kSegment);
+    gather_warp<BITS, WT, V, SETS, kGatherRuns> g(p, staging + warp * kSegment);
     const int lanes = g.lanes;
     // rounds of rows whose parts the shared sums hold (one row's always do)
     for (int ra = 0; ra < rows;) {
@@ -413,10 +432,10 @@ __global__ void __launch_bounds__(kGatherMaxWarps * 32, 2) qcsr_fwd_gather_kerne
             if (part_done) {
                 g.reduce();
                 if (first_part[r_now + 1] - first_part[r_now] == 1) {
-                    g.write_row(row0 + r_now, g.acc);
+                    g.write_row(row0 + r_now, g.acc[0]);
                 } else if (lane < lanes) {
 #pragma unroll
-                    for (int i = 0; i < V; ++i) sums[((part_now - base) * V + i) * lanes + lane] = g.acc[i];
+                    for (int i = 0; i < V; ++i) sums[((part_now - base) * V + i) * lanes + lane] = g.acc[0][i];
                 }
                 g.clear();
             }
@@ -465,18 +484,32 @@ void gather_shape(const qcsr_view &x, std::int64_t rows, std::int64_t w_row_byte
     }
 }
 
-template<int BITS, typename WT, int V>
+// Lanes that serve one entry when a lane holds v columns.
+int gather_lanes(int n, int v) {
+    int lanes = 1;
+    while (lanes < 32 && lanes * v < n) lanes *= 2;
+    return lanes;
+}
+// At least four lanes per entry, or the sums of the 32 / lanes groups cost more to bring together than the wider loads save
+// (20,000 x 240, N = 8 bf16: 35 us with 4 lanes of 4 bytes, 40 with one of 16).
+int narrowed(int n, int v) {
+    while (v > 1 && n <= 3 * v) v /= 2;
+    return v;
+}
+// 32 / the classes of a part's entries: the lanes of the widest slices N allows, re-laid W included.
+int summing_lanes(int n, int widest) { return gather_lanes(n, narrowed(n, widest)); }
+
+template<int BITS, typename WT, int V, int SETS>
 cb200_status launch_gather(fwd_params p, cudaStream_t stream) {
     const int tile = 32 * V;
-    p.lanes = 1;
-    while (p.lanes < 32 && p.lanes * V < p.n) p.lanes *= 2;
+    p.lanes = gather_lanes(p.n, V);
     p.out_vector = p.out_vector && p.n % V == 0;
     const std::int64_t rows = p.row_end - p.row_begin;
     const unsigned tiles = static_cast<unsigned>((p.n + tile - 1) / tile);
     if (p.group_rows == 0) {
         const dim3 grid(static_cast<unsigned>((rows + 3) / 4), tiles);
-        if (p.short_rows) qcsr_fwd_row_kernel<BITS, WT, V, 1><<<grid, 128, 0, stream>>>(p);
-        else qcsr_fwd_row_kernel<BITS, WT, V, 2><<<grid, 128, 0, stream>>>(p);
+        if (p.short_rows) qcsr_fwd_row_kernel<BITS, WT, V, SETS, 1><<<grid, 128, 0, stream>>>(p);
+        else qcsr_fwd_row_kernel<BITS, WT, V, SETS, 2><<<grid, 128, 0, stream>>>(p);
     } else {
         const std::int64_t left = rows - static_cast<std::int64_t>(p.full_groups) * p.group_rows;
         const bool short_end = left > 0;
@@ -484,8 +517,8 @@ cb200_status launch_gather(fwd_params p, cudaStream_t stream) {
         p.parts = std::min(kGatherParts, 32 * 1024 / static_cast<int>(V * p.lanes * sizeof(float)));
         const std::size_t smem = static_cast<std::size_t>(p.warps) * kSegment * sizeof(int2) +
                                  static_cast<std::size_t>(p.parts) * V * p.lanes * sizeof(float);
-        if (short_end) qcsr_fwd_gather_kernel<BITS, WT, V, true><<<dim3(groups, tiles), p.warps * 32, smem, stream>>>(p);
-        else qcsr_fwd_gather_kernel<BITS, WT, V, false><<<dim3(groups, tiles), p.warps * 32, smem, stream>>>(p);
+        if (short_end) qcsr_fwd_gather_kernel<BITS, WT, V, SETS, true><<<dim3(groups, tiles), p.warps * 32, smem, stream>>>(p);
+        else qcsr_fwd_gather_kernel<BITS, WT, V, SETS, false><<<dim3(groups, tiles), p.warps * 32, smem, stream>>>(p);
     }
     count_launch();
     CB200_CUDA_OK(cudaGetLastError());
@@ -517,21 +550,30 @@ bool gather_packs(const qcsr_view &x, std::int64_t n, int dense_dtype) {
     return (n * elem) % 16 != 0 && x.nnz >= (1ll << 20) && x.nnz >= 32 * x.cols;
 }
 
+template<int BITS, typename WT, int V>
+cb200_status launch_sets(const fwd_params &p, cudaStream_t stream) {
+    constexpr int widest = 16 / static_cast<int>(sizeof(WT));
+    switch (gather_lanes(p.n, V) / summing_lanes(p.n, widest)) {
+    case 8: if constexpr (8 * V <= widest) return launch_gather<BITS, WT, V, 8>(p, stream); [[fallthrough]];
+    case 4: if constexpr (4 * V <= widest) return launch_gather<BITS, WT, V, 4>(p, stream); [[fallthrough]];
+    case 2: if constexpr (2 * V <= widest) return launch_gather<BITS, WT, V, 2>(p, stream); [[fallthrough]];
+    default: return launch_gather<BITS, WT, V, 1>(p, stream);
+    }
+}
+
 // Columns per lane: the widest slice, up to 16 bytes, that divides N and the rows' alignment.
 template<int BITS, typename WT>
 cb200_status dispatch_gather(const fwd_params &p, cudaStream_t stream) {
     constexpr int widest = 16 / static_cast<int>(sizeof(WT));
     int v = p.w_ld * static_cast<std::int64_t>(sizeof(WT)) <= 0xffffffffll ? widest : 1;
     while (v > 1 && (p.n % v != 0 || reinterpret_cast<std::uintptr_t>(p.w) % (v * sizeof(WT)) != 0u || p.w_ld % v != 0)) v /= 2;
-    // at least four lanes per entry, or the sums of the 32 / lanes groups cost more to bring together than the wider loads
-    // save (20,000 x 240, N = 8 bf16: 35 us with 4 lanes of 4 bytes, 40 with one of 16)
-    while (v > 1 && p.n <= 3 * v) v /= 2;
     if (p.packed_rows) v = widest; // the lane that holds the last columns of a row may hold fewer than v
+    v = narrowed(p.n, v);
     switch (v) {
-    case 8: if constexpr (widest == 8) return launch_gather<BITS, WT, 8>(p, stream); [[fallthrough]];
-    case 4: return launch_gather<BITS, WT, 4>(p, stream);
-    case 2: return launch_gather<BITS, WT, 2>(p, stream);
-    default: return launch_gather<BITS, WT, 1>(p, stream);
+    case 8: if constexpr (widest == 8) return launch_gather<BITS, WT, 8, 1>(p, stream); [[fallthrough]];
+    case 4: return launch_sets<BITS, WT, 4>(p, stream);
+    case 2: return launch_sets<BITS, WT, 2>(p, stream);
+    default: return launch_sets<BITS, WT, 1>(p, stream);
     }
 }
 

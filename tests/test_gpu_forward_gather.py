@@ -63,3 +63,38 @@ def test_w_re_laid_with_aligned_rows(cuda_device, oracle, n, dtype):
     op = ops.PreparedSpmm(capi.PROJECTION_CSR, c["rows"], c["cols"], n, int(c["row_ptr"][-1]), 8, 1, dtype, cuda_device)
     assert op.workspace_bytes > 256
     check(oracle, cuda_device, c, n, dtype)
+
+
+def rows_of(c, lo, hi):
+    """Rows [lo, hi) as a matrix of their own."""
+    s, e, ps, pe = c["row_ptr"][lo], c["row_ptr"][hi], c["packed_row_ptr"][lo], c["packed_row_ptr"][hi]
+    return dict(c, rows=hi - lo, row_ptr=c["row_ptr"][lo:hi + 1] - s, col_idx=c["col_idx"][s:e], values=c["values"][s:e],
+                packed_row_ptr=c["packed_row_ptr"][lo:hi + 1] - ps, packed=c["packed"][ps:pe],
+                offsets=c["offsets"] if c["policy"] == 1 else c["offsets"][lo:hi])
+
+
+@pytest.mark.parametrize("bits,policy", [(8, 1), (4, 2)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_a_rows_bits_follow_from_its_entries(cuda_device, oracle, bits, policy, dtype):
+    """The same bits in the whole matrix, in shards that are matrices of their own, with and without room to re-lay W, from a W
+    whose rows start anywhere, and through the routed call: every width of slices and number of sums per lane."""
+    rng = np.random.default_rng(bits)
+    lengths = np.concatenate([EDGE_LENGTHS, rng.integers(900, 1300, size=1001), rng.integers(0, 40, size=300)])
+    c = matrix(oracle, lengths, 4000, bits, policy, 5)
+    assert c["row_ptr"][-1] >= 1 << 20
+    x = to_dev(c, cuda_device)
+    shards = [(lo, hi, to_dev(rows_of(c, lo, hi), cuda_device)) for lo, hi in ((0, 40), (40, 700), (1019, c["rows"]))]
+    for n in (1, 2, 3, 4, 6, 7, 12, 16, 20, 36, 49, 50, 64, 100, 101, 300):
+        w, _ = dense(rng, 4000, n, dtype, cuda_device)
+        y = ops.spmm_forward(x, w)
+        op = ops.PreparedSpmm(capi.PROJECTION_CSR, c["rows"], 4000, n, x.nnz, bits, policy, dtype, cuda_device)
+        op.workspace_bytes = 256
+        assert torch.equal(op.run(x, w, torch.empty_like(y)), y), n
+        op.close()
+        odd, _ = dense(rng, 4000, n, dtype, cuda_device, ld=n + 3)
+        odd.copy_(w)
+        assert torch.equal(ops.spmm_forward(x, odd), y), n
+        for lo, hi, part in shards:
+            assert torch.equal(ops.spmm_forward(part, w), y[lo:hi]), (n, lo)
+        if dtype == torch.float32:
+            assert torch.equal(ops.public_projection(x, w), y), n
