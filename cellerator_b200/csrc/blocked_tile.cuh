@@ -141,14 +141,18 @@ __global__ void __launch_bounds__(256) pack_windows_kernel(const WT *w, std::int
 
 // The work of a CTA: whole groups, or parts of a group's windows (window_split_plan).
 struct window_split {
-    int whole;   // groups from this one on are cut
+    int whole;    // groups from this one on are cut
     int parts;
-    float *sums; // [(group - whole) * parts + part][kRows][N], raw accumulators
+    int per_unit; // parts of a cut group that a unit takes
+    int slots;    // per cut group: one a part, or one a pair of parts
+    float *sums;  // [(group - whole) * slots + slot][kRows][N], raw accumulators
 };
 struct window_unit {
     int group, w0, w1;
-    int slot; // where the sums go; -1: a whole group, written to Y
+    int slot;        // where its first sums go; -1: a whole group, written to Y
+    int k0, pieces;  // parts of the group's windows that the unit takes: [k0, k0 + pieces)
 };
+__host__ __device__ __forceinline__ int part_begin(int windows, int parts, int part) { return windows * part / parts; }
 __host__ __device__ __forceinline__ int whole_groups_in(const window_split &s, std::int64_t begin, std::int64_t end) {
     const int last = s.whole < static_cast<int>(end) ? s.whole : static_cast<int>(end);
     return last > static_cast<int>(begin) ? last - static_cast<int>(begin) : 0;
@@ -156,14 +160,16 @@ __host__ __device__ __forceinline__ int whole_groups_in(const window_split &s, s
 // units of the groups [begin, end): whole groups first, then the parts of the others
 __host__ __device__ __forceinline__ int unit_count(const window_split &s, std::int64_t begin, std::int64_t end) {
     const int whole = whole_groups_in(s, begin, end);
-    return whole + (static_cast<int>(end - begin) - whole) * s.parts;
+    return whole + (static_cast<int>(end - begin) - whole) * ((s.parts + s.per_unit - 1) / s.per_unit);
 }
 __device__ __forceinline__ window_unit unit_at(const window_split &s, std::int64_t begin, std::int64_t end, int windows, int u) {
     const int whole = whole_groups_in(s, begin, end);
-    if (u < whole) return window_unit{static_cast<int>(begin) + u, 0, windows, -1};
-    const int cut = (u - whole) / s.parts, part = (u - whole) - cut * s.parts;
+    if (u < whole) return window_unit{static_cast<int>(begin) + u, 0, windows, -1, 0, s.parts};
+    const int units = (s.parts + s.per_unit - 1) / s.per_unit;
+    const int cut = (u - whole) / units, part = ((u - whole) - cut * units) * s.per_unit, pieces = min(s.per_unit, s.parts - part);
     const int group = static_cast<int>(begin) + whole + cut;
-    return window_unit{group, windows * part / s.parts, windows * (part + 1) / s.parts, (group - s.whole) * s.parts + part};
+    return window_unit{group, part_begin(windows, s.parts, part), part_begin(windows, s.parts, part + pieces),
+                       (group - s.whole) * s.slots + (s.slots < s.parts ? part / 2 : part), part, pieces};
 }
 // units of this CTA: blockIdx.x, + gridDim.x, ...
 __device__ __forceinline__ int units_of_cta(const window_split &s, std::int64_t begin, std::int64_t end) {
@@ -173,12 +179,13 @@ __device__ __forceinline__ int units_of_cta(const window_split &s, std::int64_t 
 
 // Y of the groups that were cut: the parts' sums in order, then what the epilogue of a whole group does.
 // result_scale / w_absmax / value_bound: the powers of two the operands were stored times (null: none).
-__global__ void __launch_bounds__(256) add_parts_kernel(const float *sums, int parts, int whole, int first_group, std::int64_t row_end,
+// paired: the sums of two neighbouring parts are added first.
+__global__ void __launch_bounds__(256) add_parts_kernel(const float *sums, int slots, int paired, int whole, int first_group, std::int64_t row_end,
                                                         int n, float *y, std::int64_t y_ld, float alpha, float beta, const float *bias,
                                                         int epilogue, float result_scale, const unsigned *w_absmax, const unsigned *value_bound) {
     wait_for_previous_launch();
     const std::int64_t group = first_group + static_cast<int>(blockIdx.x);
-    const float *in = sums + (group - whole) * parts * kRows * n;
+    const float *in = sums + (group - whole) * slots * kRows * n;
     float scale = alpha * result_scale;
     if (w_absmax != nullptr) scale /= operand_scale(__uint_as_float(__ldg(w_absmax)));
     if (value_bound != nullptr) scale /= operand_scale(__uint_as_float(__ldg(value_bound)));
@@ -187,10 +194,25 @@ __global__ void __launch_bounds__(256) add_parts_kernel(const float *sums, int p
         const int r = i / (n / 4), c = (i % (n / 4)) * 4;
         const std::int64_t row = group * kRows + r;
         if (row >= row_end) break;
-        float4 v = *reinterpret_cast<const float4 *>(in + 4 * static_cast<std::int64_t>(i));
-        for (int k = 1; k < parts; ++k) {
-            const float4 t = *reinterpret_cast<const float4 *>(in + static_cast<std::int64_t>(k) * kRows * n + 4 * static_cast<std::int64_t>(i));
-            v.x += t.x; v.y += t.y; v.z += t.z; v.w += t.w;
+        const auto sum_at = [&](int k) {
+            return k < slots ? *reinterpret_cast<const float4 *>(in + static_cast<std::int64_t>(k) * kRows * n + 4 * static_cast<std::int64_t>(i)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        };
+        const auto add = [](float4 a, float4 b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); };
+        float4 v = sum_at(0);
+        const int pair = paired != 0 ? 2 : 1;
+        if (pair == 2 && slots > 1) v = add(v, sum_at(1));
+#pragma unroll 1
+        for (int k = pair; k < slots; k += 4) { // four in flight
+            const float4 t0 = sum_at(k), t1 = sum_at(k + 1), t2 = sum_at(k + 2), t3 = sum_at(k + 3);
+            if (pair == 2) {
+                v = add(v, k + 1 < slots ? add(t0, t1) : t0);
+                if (k + 2 < slots) v = add(v, k + 3 < slots ? add(t2, t3) : t2);
+            } else {
+                v = add(v, t0);
+                if (k + 1 < slots) v = add(v, t1);
+                if (k + 2 < slots) v = add(v, t2);
+                if (k + 3 < slots) v = add(v, t3);
+            }
         }
         float *out = y + row * y_ld + c;
         v.x *= scale; v.y *= scale; v.z *= scale; v.w *= scale;
@@ -205,23 +227,25 @@ __global__ void __launch_bounds__(256) add_parts_kernel(const float *sums, int p
         *reinterpret_cast<float4 *>(out) = v;
     }
 }
-inline cb200_status launch_add_parts(const window_split &s, std::int64_t group_begin, std::int64_t group_end, std::int64_t row_end, int n, float *y,
+inline cb200_status launch_add_parts(const window_split &s, bool pairs, std::int64_t group_begin, std::int64_t group_end, std::int64_t row_end, int n, float *y,
                                      std::int64_t y_ld, float alpha, float beta, const float *bias, int epilogue, float result_scale,
                                      const unsigned *w_absmax, const unsigned *value_bound, cudaStream_t stream) {
     const int first = static_cast<int>(group_begin) + whole_groups_in(s, group_begin, group_end), cut = static_cast<int>(group_end) - first;
     if (cut <= 0) return CB200_STATUS_SUCCESS;
-    CB200_CUDA_OK(launch_kernel(true, add_parts_kernel, dim3(static_cast<unsigned>(cut), static_cast<unsigned>(n / 16)), 256, 0, stream, s.sums, s.parts, s.whole,
+    CB200_CUDA_OK(launch_kernel(true, add_parts_kernel, dim3(static_cast<unsigned>(cut), static_cast<unsigned>(n / 8)), 256, 0, stream, s.sums, s.slots,
+                                pairs && s.slots == s.parts ? 1 : 0, s.whole,
                                 first, row_end, n, y, y_ld, alpha, beta, bias, epilogue, result_scale, w_absmax, value_bound));
     count_launch();
     CB200_CUDA_OK(cudaGetLastError());
     return CB200_STATUS_SUCCESS;
 }
-// The split of a launch: cut where the workspace holds the sums behind its `used` bytes.
-inline window_split split_of_launch(const qcsr_view &x, std::int64_t n, void *workspace, std::uint64_t workspace_bytes, std::uint64_t used, int sm_count) {
-    const window_split_plan plan = qcsr_window_split(x.rows, x.cols, sm_count);
-    const std::uint64_t at = device_arena::rounded(used);
-    if (plan.parts == 1 || workspace_bytes < at + qcsr_window_split_bytes(x.rows, x.cols, n, sm_count)) return window_split{0x7fffffff, 1, nullptr};
-    return window_split{static_cast<int>(plan.whole), plan.parts, reinterpret_cast<float *>(static_cast<unsigned char *>(workspace) + at)};
+// The split of a launch: groups are cut where the workspace holds the sums behind its `used` bytes.
+inline window_split split_of_launch(const qcsr_view &x, std::int64_t n, std::int64_t columns, void *workspace, std::uint64_t workspace_bytes, std::uint64_t used,
+                                    int sm_count) {
+    const window_split_plan plan = qcsr_window_split(x.rows, x.cols, columns, sm_count);
+    const std::uint64_t at = device_arena::rounded(used), sums = qcsr_window_split_bytes(x.rows, x.cols, n, columns, sm_count);
+    if (sums == 0u || workspace_bytes < at + sums) return window_split{0x7fffffff, columns == 0 ? 1 : plan.parts, 1, 1, nullptr};
+    return window_split{static_cast<int>(plan.whole), plan.parts, plan.per_unit, plan.slots, reinterpret_cast<float *>(static_cast<unsigned char *>(workspace) + at)};
 }
 
 } // namespace

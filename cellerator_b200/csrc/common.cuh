@@ -96,26 +96,26 @@ __device__ __forceinline__ float finish_output(float value, const float *bias, i
 // The phases are kept apart -- every load, then the arithmetic, then the optional epilogue calls,
 // then every store -- so that the eight loads of a beta != 0 launch are in flight together; with a
 // call between each load and store they would follow one another.
-__device__ __forceinline__ void store_row32(float *out, float (&v)[32], float alpha, float beta, const float *bias, int col0,
-                                            int kind) {
+template<int C>
+__device__ __forceinline__ void store_row(float *out, float (&v)[C], float alpha, float beta, const float *bias, int col0, int kind) {
 #pragma unroll
-    for (int c = 0; c < 32; ++c) v[c] *= alpha;
+    for (int c = 0; c < C; ++c) v[c] *= alpha;
     if (beta != 0.0f) {
-        float4 o[8];
+        float4 o[C / 4];
 #pragma unroll
-        for (int c = 0; c < 8; ++c) o[c] = *reinterpret_cast<const float4 *>(out + 4 * c);
+        for (int c = 0; c < C / 4; ++c) o[c] = *reinterpret_cast<const float4 *>(out + 4 * c);
 #pragma unroll
-        for (int c = 0; c < 8; ++c) {
+        for (int c = 0; c < C / 4; ++c) {
             v[4 * c + 0] = fmaf(beta, o[c].x, v[4 * c + 0]); v[4 * c + 1] = fmaf(beta, o[c].y, v[4 * c + 1]);
             v[4 * c + 2] = fmaf(beta, o[c].z, v[4 * c + 2]); v[4 * c + 3] = fmaf(beta, o[c].w, v[4 * c + 3]);
         }
     }
     if (kind != CB200_EPILOGUE_NONE) {
 #pragma unroll
-        for (int c = 0; c < 32; ++c) v[c] = finish_output(v[c], bias, col0 + c, kind);
+        for (int c = 0; c < C; ++c) v[c] = finish_output(v[c], bias, col0 + c, kind);
     }
 #pragma unroll
-    for (int c = 0; c < 8; ++c)
+    for (int c = 0; c < C / 4; ++c)
         *reinterpret_cast<float4 *>(out + 4 * c) = make_float4(v[4 * c + 0], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
 }
 

@@ -135,15 +135,19 @@ struct blocked_layout {
     // Scales and offsets are NOT in it: they are applied at launch.
     unsigned char *code_tiles = nullptr;
 };
-// How the tensor kernels over 256-row groups share a matrix out: a CTA takes whole groups, except that the windows of the last
-// groups (those from `whole` on, fewer than two per SM) are cut into `parts` so that every SM has work to the end.  It depends
-// on the matrix alone: a row's sum is cut the same way in every launch.  Sums of parts go through the workspace.
+// How the tensor kernels over 256-row groups share a matrix out: a CTA takes whole groups, except that the last groups (those
+// from `whole` on, fewer than two per SM) are cut along their windows so that every SM has work to the end.  Sums of parts of a
+// cut group go through the workspace.  The kernel over entry words sums the windows of EVERY group in the same parts, so that a
+// row's bits do not depend on which groups are cut.
 struct window_split_plan {
     std::int64_t whole = 0;
     int parts = 1;
+    int per_unit = 1; // of them to a CTA
+    int slots = 1;    // sums that go through the workspace, per group: one a part, or one a pair of parts
 };
-window_split_plan qcsr_window_split(std::int64_t rows, std::int64_t cols, int sm_count);
-std::uint64_t qcsr_window_split_bytes(std::int64_t rows, std::int64_t cols, std::int64_t n, int sm_count);
+// columns: of an accumulator of the kernel over entry words; 0: the kernels over tiles, groups cut into as many parts as pay
+window_split_plan qcsr_window_split(std::int64_t rows, std::int64_t cols, std::int64_t columns, int sm_count);
+std::uint64_t qcsr_window_split_bytes(std::int64_t rows, std::int64_t cols, std::int64_t n, std::int64_t columns, int sm_count);
 bool qcsr_blocked_shape_ok(std::int64_t rows, std::int64_t cols, std::int64_t n, int bits, int dense_dtype);
 std::uint64_t qcsr_blocked_workspace_bytes(std::int64_t cols, std::int64_t n);
 // Split products of an fp32 W may use room for 2 N columns: its hi and lo parts side by side.

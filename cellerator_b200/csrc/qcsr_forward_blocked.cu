@@ -247,6 +247,155 @@ struct blocked_params {
     int withhold_w; // test hook: the W loader issues no copies, so the waits for W run out
 };
 
+// Accumulators.  The windows of a group are summed in parts (window_parts), each in a set of accumulators of its own (one
+// accumulator per row sub-block), and the parts are added in a fixed order, so that a row's sum has the same bits whether a CTA
+// takes the whole group or some of its parts.  Tensor memory (512 columns) holds three sets of up to 64 columns and a running
+// sum: once two parts are done and the next is on its way, the warps that write Y add their sum to the running one (parts two
+// by two, then the pairs in order).  Of 128 columns it holds two sets, for groups of two parts, or one and the running sum,
+// which takes every part before the next may start (the parts in order).
+__host__ __device__ constexpr int most_sets(int columns) { return columns <= 64 ? 3 : 2; }
+template<int NC>
+__device__ __forceinline__ int accumulator_sets(int parts) { return NC <= 64 ? 3 : parts > 2 ? 1 : 2; }
+__host__ __device__ constexpr int accumulator_columns(int columns, int n) {
+    return columns > 64 || 3 * kSubBlocks * columns + kSubBlocks * n > 256 ? 512 : 256;
+}
+// How many parts of a unit are taken into the running sum at a time, and before which window: two windows behind the end of
+// the second of two, so that its MMAs are done or nearly (the third part's need no set of the two, so they and the scatter of
+// the next windows go on); behind the last window of a single one.  The end of the unit takes the rest, as many as there are sets.
+__device__ __forceinline__ int parts_at_a_time(int sets) { return sets == 3 ? 2 : 1; }
+__device__ __forceinline__ int window_of_take(const window_unit &unit, int taken, int windows, int parts, int sets) {
+    if (unit.pieces - taken <= sets) return unit.w1;
+    return sets == 3 ? part_begin(windows, parts, unit.k0 + taken + 2) + 2 : part_begin(windows, parts, unit.k0 + taken + 1);
+}
+// The warps that write Y, thread t < kRows for row t of the group (TMEM lane = row within the sub-block).  Sixteen columns at a
+// time: with 32 the epilogue's registers cost the scatter loop around it more than the longer loads save.
+template<int NC, int N>
+struct part_sums {
+    std::uint32_t first_set, running; // this thread's lane, its sub-block's columns
+    std::uint32_t acc_full, acc_empty;
+    volatile int *abort_flag;
+    int limit, sets, done; // sets used by the CTA before the unit
+
+    __device__ __forceinline__ part_sums(std::uint32_t tmem_base, std::uint64_t *full, std::uint64_t *empty, int parts, volatile int *flag, int polls)
+        : acc_full(smem_addr(full)), acc_empty(smem_addr(empty)), abort_flag(flag), limit(polls), sets(accumulator_sets<NC>(parts)), done(0) {
+        const std::uint32_t row = tmem_base + (static_cast<std::uint32_t>((threadIdx.x >> 5 & 3) * 32) << 16);
+        first_set = row + (threadIdx.x >> 7) * NC;
+        running = row + sets * (kSubBlocks * NC) + (threadIdx.x >> 7) * N;
+    }
+    __device__ __forceinline__ std::uint32_t set_of(int part) const { return first_set + (done + part) % sets * (kSubBlocks * NC); }
+    __device__ __forceinline__ void wait(int part) const {
+        const int use = done + part;
+        bar_wait(acc_full + use % sets * 8, static_cast<std::uint32_t>((use / sets) & 1), abort_flag, limit);
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    }
+    __device__ __forceinline__ void release(int part) const {
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if ((threadIdx.x & 31) == 0) bar_arrive(acc_empty + (done + part) % sets * 8);
+    }
+    // columns [c, c + 16) of a part
+    __device__ __forceinline__ void load(int part, int c, float (&v)[16]) const {
+        const std::uint32_t at = set_of(part) + c;
+        if constexpr (NC == 2 * N) {
+            float lo[16];
+            tmem_ld16(at, at + N, v, lo);
+#pragma unroll
+            for (int i = 0; i < 16; ++i) v[i] += lo[i];
+        } else {
+            tmem_ld16(at, v);
+        }
+    }
+    // raw sums of a part, or of two, of a cut group
+    __device__ __forceinline__ void store_raw(const blocked_params &p, int slot, int part, bool two) const {
+        float *out = p.split.sums + (static_cast<std::int64_t>(slot) * kRows + threadIdx.x) * N;
+#pragma unroll 1
+        for (int c = 0; c < N; c += 16, out += 16) {
+            float v[16], u[16];
+            load(part, c, v);
+            if (two) {
+                load(part + 1, c, u);
+#pragma unroll
+                for (int i = 0; i < 16; ++i) v[i] += u[i];
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) *reinterpret_cast<float4 *>(out + 4 * i) = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+        }
+        release(part);
+        if (two) release(part + 1);
+    }
+    // parts of a unit with more to come, parts_at_a_time of them
+    __device__ __forceinline__ void take(const blocked_params &p, const window_unit &unit, int part) const {
+        constexpr bool two = NC <= 64;
+        wait(part);
+        if (two) wait(part + 1);
+        if (unit.slot >= 0) {
+            store_raw(p, unit.slot + (two ? part / 2 : part), part, two);
+            return;
+        }
+#pragma unroll 1
+        for (int c = 0; c < N; c += 16) {
+            float sum[16], v[16], u[16];
+            if constexpr (NC == 2 * N || !two) {
+                load(part, c, v);
+                if (two) load(part + 1, c, u);
+                if (part > 0) tmem_ld16(running + c, sum);
+            } else if (part > 0) {
+                tmem_ld16(running + c, set_of(part) + c, set_of(part + 1) + c, sum, v, u);
+            } else {
+                tmem_ld16(set_of(part) + c, set_of(part + 1) + c, v, u);
+            }
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+                if (two) v[i] += u[i];
+                sum[i] = part > 0 ? sum[i] + v[i] : v[i];
+            }
+            tmem_st16(running + c, sum);
+        }
+        tmem_wait_stores();
+        release(part);
+        if (two) release(part + 1);
+    }
+    // the rest of a unit, as many parts as there are sets at most
+    __device__ __forceinline__ void finish(const blocked_params &p, const window_unit &unit, int from, float alpha) {
+        for (int k = from; k < unit.pieces; ++k) wait(k);
+        if (unit.slot >= 0) {
+            const int step = p.split.slots < p.split.parts ? 2 : 1;
+            for (int k = from; k < unit.pieces; k += step) store_raw(p, unit.slot + k / step, k, step == 2 && k + 1 < unit.pieces);
+        } else {
+            const std::int64_t row = static_cast<std::int64_t>(unit.group) * kRows + threadIdx.x;
+            const int rest = unit.pieces - from;
+#pragma unroll 1
+            for (int c = 0; c < N; c += 16) {
+                // the first two of the rest (of 128 columns there is one behind a running sum), the running sum, the third
+                float sum[16], v[16];
+                if (NC != 2 * N && rest > 1) {
+                    tmem_ld16(set_of(from) + c, set_of(from + 1) + c, sum, v);
+                } else {
+                    load(from, c, sum);
+                    if (rest > 1) load(from + 1, c, v);
+                }
+                if (rest > 1) {
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) sum[i] += v[i];
+                }
+                if (from > 0) {
+                    tmem_ld16(running + c, v);
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) sum[i] += v[i];
+                }
+                if (rest > 2) {
+                    load(from + 2, c, v);
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) sum[i] += v[i];
+                }
+                if (row < p.row_end) store_row(p.y + row * p.y_ld + c, sum, alpha, p.beta, p.bias, c, p.epilogue);
+            }
+            for (int k = from; k < unit.pieces; ++k) release(k);
+        }
+        done += unit.pieces;
+    }
+};
+
 // Test hook (cb200_test_arm_wait_timeout): read at launch time by the two-group kernel's launcher.
 std::atomic<int> g_test_poll_limit{0}; // 0 = not armed
 
@@ -254,7 +403,7 @@ template<int NC, int N, int CS, bool BAKED> // NC, N: as in the two-group kernel
 __global__ void __launch_bounds__(kThreads, 1) qcsr_fwd_blocked_kernel(const blocked_params p) {
     constexpr int REC = record_bytes(NC);
     constexpr int STAGES = w_stages(NC, CS);
-    constexpr int kTmemCols = kSubBlocks * NC < 32 ? 32 : kSubBlocks * NC; // one accumulator per row sub-block
+    constexpr int SETS = most_sets(NC), kTmemCols = accumulator_columns(NC, N);
     const std::uint32_t IDESC = p.idesc;
     extern __shared__ __align__(1024) unsigned char smem[];
     // [2][A tile] | [STAGES][W record] | [CS][entry chunk] | row offsets | barriers | chunk meta | tmem | abort
@@ -267,9 +416,9 @@ __global__ void __launch_bounds__(kThreads, 1) qcsr_fwd_blocked_kernel(const blo
     std::uint64_t *w_empty = w_full + STAGES;          // [STAGES]       MMA commit -> loader
     std::uint64_t *c_full = w_empty + STAGES;          // [CS] copy engine -> scatter warps
     std::uint64_t *c_empty = c_full + CS;    // [CS] scatter warps -> loader (one arrival per warp)
-    std::uint64_t *acc_full = c_empty + CS;  // MMA commit -> scatter warps
-    std::uint64_t *acc_empty = acc_full + 1;           // scatter warps -> MMA (one arrival per warp)
-    volatile int *chunk_meta = reinterpret_cast<volatile int *>(acc_empty + 1); // [CS] (entries << 1) | last chunk of its window
+    std::uint64_t *acc_full = c_empty + CS;            // [SETS] MMA commit -> scatter warps
+    std::uint64_t *acc_empty = acc_full + SETS;        // [SETS] scatter warps -> MMA (one arrival per warp)
+    volatile int *chunk_meta = reinterpret_cast<volatile int *>(acc_empty + SETS); // [CS] (entries << 1) | last chunk of its window
     std::uint32_t *tmem_slot = reinterpret_cast<std::uint32_t *>(const_cast<int *>(chunk_meta) + CS + 1);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
     unsigned char *scratch_slot = reinterpret_cast<unsigned char *>(tmem_slot + 2);
@@ -292,8 +441,10 @@ __global__ void __launch_bounds__(kThreads, 1) qcsr_fwd_blocked_kernel(const blo
             bar_init(smem_addr(c_full + s), 1);
             bar_init(smem_addr(c_empty + s), kProducerWarps);
         }
-        bar_init(smem_addr(acc_full), 1);
-        bar_init(smem_addr(acc_empty), kEpilogueWarps);
+        for (int k = 0; k < SETS; ++k) {
+            bar_init(smem_addr(acc_full + k), 1);
+            bar_init(smem_addr(acc_empty + k), kEpilogueWarps);
+        }
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -313,12 +464,13 @@ __global__ void __launch_bounds__(kThreads, 1) qcsr_fwd_blocked_kernel(const blo
 
     if (warp < kProducerWarps) {
         // ================= zero, scatter, epilogue =================
-        const int sub = tid >> 7;
         // fp16 operands were stored times powers of two: the result is divided by both again
         const float alpha = p.alpha * p.result_scale / (p.w_absmax != nullptr ? operand_scale(__uint_as_float(__ldg(p.w_absmax))) : 1.0f);
         const bool use_row_offset = p.row_offsets != nullptr;
-        long long q = 0;  // windows done by this CTA
-        long long qc = 0; // chunks done by this CTA
+        unsigned q = 0; // windows done by this CTA
+        int cs = 0, s = 0;                          // the next chunk's stage and, for the decode table, the window's W stage,
+        std::uint32_t chunk_phase = 0, w_phase = 0; // counted along: a 64-bit division per chunk and warp is 10 % of the kernel
+        part_sums<NC, N> parts(tmem_base, acc_full, acc_empty, p.split.parts, abort_flag, kPollLimit);
         for (int gi = 0; gi < my_units; ++gi) {
             const window_unit unit = unit_of(gi);
             const std::int64_t row = static_cast<std::int64_t>(unit.group) * kRows + tid;
@@ -327,145 +479,137 @@ __global__ void __launch_bounds__(kThreads, 1) qcsr_fwd_blocked_kernel(const blo
                 if (tid < kRows) row_offset_s[tid] = row < p.row_end ? __ldg(p.row_offsets + row) : 0.0f;
                 asm volatile("bar.sync 1, %0;" ::"n"(kProducerThreads) : "memory");
             }
-            for (int w = unit.w0; w < unit.w1; ++w, ++q) {
-                const std::uint32_t b = static_cast<std::uint32_t>(q & 1);
-                const int s = static_cast<int>(q % STAGES);
-                bar_wait(smem_addr(a_empty + b), static_cast<std::uint32_t>(((q >> 1) & 1) ^ 1), abort_flag);
-                unsigned char *tile = smem + b * kABufBytes;
+            int taken = 0;
+            for (int w = unit.w0; w < unit.w1;) { // up to the next parts to take
+                const int stop = window_of_take(unit, taken, p.windows, p.split.parts, parts.sets);
+                for (; w < stop; ++w, ++q) {
+                    const std::uint32_t b = q & 1u;
+                    bar_wait(smem_addr(a_empty + b), ((q >> 1) & 1u) ^ 1u, abort_flag);
+                    unsigned char *tile = smem + b * kABufBytes;
 #pragma unroll
-                for (int k = 0; k < kABufBytes / (kProducerThreads * 8); ++k) // 8-byte stores: see the two-group kernel
-                    *reinterpret_cast<uint2 *>(tile + k * (kProducerThreads * 8) + tid * 8) = make_uint2(0u, 0u);
-                asm volatile("bar.sync 1, %0;" ::"n"(kProducerThreads) : "memory"); // the whole tile is zero before anyone scatters
-                // the W stage carries the decode table; baked entries do not need it, only the MMA waits for W
-                if constexpr (!BAKED) bar_wait(smem_addr(w_full + s), static_cast<std::uint32_t>((q / STAGES) & 1), abort_flag);
-                const float2 *table = reinterpret_cast<const float2 *>(smem + 2 * kABufBytes + s * REC + NC * kWin * 2);
-                bool last = false;
-                int guard = 0;
-                while (!last && ++guard < (1 << 20)) {
-                    const int cs = static_cast<int>(qc % CS);
-                    bar_wait(smem_addr(c_full + cs), static_cast<std::uint32_t>((qc / CS) & 1), abort_flag);
-                    const int meta = chunk_meta[cs];
-                    const int count = *abort_flag != 0 ? 0 : (meta >> 1);
-                    last = (meta & 1) != 0 || *abort_flag != 0;
-                    const uint4 *chunk = reinterpret_cast<const uint4 *>(chunk_base + cs * kChunkBytes);
-                    for (int i = tid * 4; i < count; i += kProducerThreads * 4) { // segments are padded to multiples of 4
-                        const uint4 e4 = chunk[i >> 2];
-                        const std::uint32_t e[4] = {e4.x, e4.y, e4.z, e4.w};
-                        if constexpr (BAKED) {
-                            // decoded at prepare time: the word is {bf16 value, byte position / 2}
+                    for (int k = 0; k < kABufBytes / (kProducerThreads * 8); ++k) // 8-byte stores: see the two-group kernel
+                        *reinterpret_cast<uint2 *>(tile + k * (kProducerThreads * 8) + tid * 8) = make_uint2(0u, 0u);
+                    asm volatile("bar.sync 1, %0;" ::"n"(kProducerThreads) : "memory"); // the whole tile is zero before anyone scatters
+                    // the W stage carries the decode table; baked entries do not need it, only the MMA waits for W
+                    if constexpr (!BAKED) bar_wait(smem_addr(w_full + s), w_phase, abort_flag);
+                    const float2 *table = reinterpret_cast<const float2 *>(smem + 2 * kABufBytes + s * REC + NC * kWin * 2);
+                    bool last = false;
+                    int guard = 0;
+                    while (!last && ++guard < (1 << 20)) {
+                        bar_wait(smem_addr(c_full + cs), chunk_phase, abort_flag);
+                        const int meta = chunk_meta[cs];
+                        const int count = *abort_flag != 0 ? 0 : (meta >> 1);
+                        last = (meta & 1) != 0 || *abort_flag != 0;
+                        const uint4 *chunk = reinterpret_cast<const uint4 *>(chunk_base + cs * kChunkBytes);
+                        for (int i = tid * 4; i < count; i += kProducerThreads * 4) { // segments are padded to multiples of 4
+                            const uint4 e4 = chunk[i >> 2];
+                            const std::uint32_t e[4] = {e4.x, e4.y, e4.z, e4.w};
+                            if constexpr (BAKED) {
+                                // decoded at prepare time: the word is {bf16 value, byte position / 2}
+#pragma unroll
+                                for (int k = 0; k < 4; ++k) {
+                                    unsigned char *dst = static_cast<int>(e[k]) >= 0 ? tile + (((e[k] >> 16) & 0x7fffu) << 1) : scratch_slot;
+                                    *reinterpret_cast<unsigned short *>(dst) = static_cast<unsigned short>(e[k] & 0xffffu);
+                                }
+                                continue;
+                            }
+                            float2 t[4];
+#pragma unroll
+                            for (int k = 0; k < 4; ++k) t[k] = table[(e[k] >> 8) & (kWin - 1)];
 #pragma unroll
                             for (int k = 0; k < 4; ++k) {
-                                unsigned char *dst = static_cast<int>(e[k]) >= 0 ? tile + (((e[k] >> 16) & 0x7fffu) << 1) : scratch_slot;
-                                *reinterpret_cast<unsigned short *>(dst) = static_cast<unsigned short>(e[k] & 0xffffu);
+                                const std::uint32_t off = ((e[k] >> 15) & 0x7fffu) << 1;
+                                float add = t[k].y;
+                                if (use_row_offset) // row within the group, back from the byte position in the tile
+                                    add = row_offset_s[((off / kSubBlockBytes) << 7) | (((off >> 10) & 15u) << 3) | ((off >> 7) & 7u)];
+                                const float value = fmaf(static_cast<float>(e[k] & 0xffu), t[k].x, add);
+                                // padding words (top bit set) are stored to a scratch slot instead of branching
+                                unsigned char *dst = static_cast<int>(e[k]) >= 0 ? tile + off : scratch_slot;
+                                __nv_bfloat16 bv = __float2bfloat16_rn(value);
+                                if (p.value_part != 0) bv = __float2bfloat16_rn(value - __bfloat162float(bv)); // the next 8 mantissa bits
+                                *reinterpret_cast<__nv_bfloat16 *>(dst) = bv;
                             }
-                            continue;
                         }
-                        float2 t[4];
-#pragma unroll
-                        for (int k = 0; k < 4; ++k) t[k] = table[(e[k] >> 8) & (kWin - 1)];
-#pragma unroll
-                        for (int k = 0; k < 4; ++k) {
-                            const std::uint32_t off = ((e[k] >> 15) & 0x7fffu) << 1;
-                            float add = t[k].y;
-                            if (use_row_offset) // row within the group, back from the byte position in the tile
-                                add = row_offset_s[((off / kSubBlockBytes) << 7) | (((off >> 10) & 15u) << 3) | ((off >> 7) & 7u)];
-                            const float value = fmaf(static_cast<float>(e[k] & 0xffu), t[k].x, add);
-                            // padding words (top bit set) are stored to a scratch slot instead of branching
-                            unsigned char *dst = static_cast<int>(e[k]) >= 0 ? tile + off : scratch_slot;
-                            __nv_bfloat16 bv = __float2bfloat16_rn(value);
-                            if (p.value_part != 0) bv = __float2bfloat16_rn(value - __bfloat162float(bv)); // the next 8 mantissa bits
-                            *reinterpret_cast<__nv_bfloat16 *>(dst) = bv;
-                        }
+                        __syncwarp();
+                        if (lane == 0) bar_arrive(smem_addr(c_empty + cs));
+                        if (++cs == CS) { cs = 0; chunk_phase ^= 1u; }
                     }
+                    if (!BAKED && ++s == STAGES) { s = 0; w_phase ^= 1u; }
+                    fence_async_proxy(); // the tile was written with ordinary stores, the MMA reads it through the async proxy
                     __syncwarp();
-                    if (lane == 0) bar_arrive(smem_addr(c_empty + cs));
-                    ++qc;
+                    if (lane == 0) bar_arrive(smem_addr(a_full + b));
                 }
-                fence_async_proxy(); // the tile was written with ordinary stores, the MMA reads it through the async proxy
-                __syncwarp();
-                if (lane == 0) bar_arrive(smem_addr(a_full + b));
-            }
-
-            // ---- thread t < 256 writes row t of the group: TMEM lane = row within the sub-block
-            if (warp >= kEpilogueWarps) continue;
-            bar_wait(smem_addr(acc_full), static_cast<std::uint32_t>(gi & 1), abort_flag);
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-#pragma unroll
-            for (int h = 0; h < N / 32; ++h) {
-                float v[32];
-                tmem_ld32(tmem_base + (static_cast<std::uint32_t>((warp & 3) * 32) << 16) + sub * NC + h * 32, v);
-                if constexpr (NC == 2 * N) {
-                    float lo[32];
-                    tmem_ld32(tmem_base + (static_cast<std::uint32_t>((warp & 3) * 32) << 16) + sub * NC + N + h * 32, lo);
-#pragma unroll
-                    for (int c = 0; c < 32; ++c) v[c] += lo[c];
-                }
-                if (unit.slot >= 0) { // raw sums of a part
-                    store_row32(p.split.sums + (static_cast<std::int64_t>(unit.slot) * kRows + tid) * N + h * 32, v, 1.0f, 0.0f, nullptr, h * 32, CB200_EPILOGUE_NONE);
-                } else if (row < p.row_end) {
-                    float *out = p.y + row * p.y_ld + h * 32;
-                    store_row32(out, v, alpha, p.beta, p.bias, h * 32, p.epilogue);
+                if (w < unit.w1) {
+                    __syncwarp();
+                    if (warp < kEpilogueWarps) parts.take(p, unit, taken);
+                    taken += parts_at_a_time(parts.sets);
                 }
             }
-            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            __syncwarp();
-            if (lane == 0) bar_arrive(smem_addr(acc_empty));
+            if (warp < kEpilogueWarps) parts.finish(p, unit, taken, alpha);
         }
     } else if (warp == kProducerWarps) {
         // ================= MMA issuer =================
-        long long q = 0;
+        const int sets = accumulator_sets<NC>(p.split.parts);
+        unsigned q = 0;
+        int use = 0, s = 0;
+        std::uint32_t w_phase = 0;
         for (int g = 0; g < my_units; ++g) {
             const window_unit unit = unit_of(g);
-            bar_wait(smem_addr(acc_empty), static_cast<std::uint32_t>((g & 1) ^ 1), abort_flag);
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            for (int w = unit.w0; w < unit.w1; ++w, ++q) {
-                const std::uint32_t b = static_cast<std::uint32_t>(q & 1);
-                const int s = static_cast<int>(q % STAGES);
-                bar_wait(smem_addr(w_full + s), static_cast<std::uint32_t>((q / STAGES) & 1), abort_flag);
-                bar_wait(smem_addr(a_full + b), static_cast<std::uint32_t>((q >> 1) & 1), abort_flag);
+            for (int k = unit.k0, w = unit.w0; k < unit.k0 + unit.pieces; ++k, ++use) {
+                const int set = use % sets, first = w, end = part_begin(p.windows, p.split.parts, k + 1);
+                bar_wait(smem_addr(acc_empty + set), static_cast<std::uint32_t>(((use / sets) & 1) ^ 1), abort_flag);
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                if (elect_one()) {
-                    const std::uint32_t a_tile = smem0 + b * kABufBytes;
-                    const std::uint32_t b_tile = wstage0 + s * REC;
+                const std::uint32_t acc = tmem_base + set * (kSubBlocks * NC);
+                for (; w < end; ++w, ++q) {
+                    const std::uint32_t b = q & 1u;
+                    bar_wait(smem_addr(w_full + s), w_phase, abort_flag);
+                    bar_wait(smem_addr(a_full + b), (q >> 1) & 1u, abort_flag);
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    if (elect_one()) {
+                        const std::uint32_t a_tile = smem0 + b * kABufBytes;
+                        const std::uint32_t b_tile = wstage0 + s * REC;
 #pragma unroll
-                    for (int kk = 0; kk < kWin / 16; ++kk) {
-                        const std::uint64_t db = smem_desc(b_tile + kk * 256);
+                        for (int kk = 0; kk < kWin / 16; ++kk) {
+                            const std::uint64_t db = smem_desc(b_tile + kk * 256);
 #pragma unroll
-                        for (int sb = 0; sb < kSubBlocks; ++sb)
-                            mma_bf16(tmem_base + sb * NC,
-                                     smem_desc_sw128(a_tile + sb * kSubBlockBytes + (kk >> 2) * kHalfBytes + (kk & 3) * 32), db, IDESC,
-                                     w > unit.w0 || kk > 0);
+                            for (int sb = 0; sb < kSubBlocks; ++sb)
+                                mma_bf16(acc + sb * NC,
+                                         smem_desc_sw128(a_tile + sb * kSubBlockBytes + (kk >> 2) * kHalfBytes + (kk & 3) * 32), db, IDESC,
+                                         w > first || kk > 0);
+                        }
+                        mma_commit(smem_addr(a_empty + b));
+                        mma_commit(smem_addr(w_empty + s));
+                        if (w == end - 1) mma_commit(smem_addr(acc_full + set));
                     }
-                    mma_commit(smem_addr(a_empty + b));
-                    mma_commit(smem_addr(w_empty + s));
-                    if (w == unit.w1 - 1) mma_commit(smem_addr(acc_full));
+                    __syncwarp();
+                    if (++s == STAGES) { s = 0; w_phase ^= 1u; }
                 }
-                __syncwarp();
             }
         }
     } else {
         // ================= loaders =================
         // Issuing a bulk copy costs its thread several hundred cycles (barrier wait, expect-tx, the
         // copy itself), so the copies of a window are spread over threads: one warp's elected lane
-        // feeds the W ring, kChunkLoaders warps take the entry chunks in turn (chunk number modulo
-        // kChunkLoaders); each of them walks all segments and issues only its own chunks.
-        const int role = warp - kProducerWarps - 1; // 0: W slices, 1..kChunkLoaders: entry chunks
+        // feeds the W ring, another's the ring of entry chunks.
+        static_assert(kChunkLoaders == 1, "one warp takes all chunks");
+        const int role = warp - kProducerWarps - 1; // 0: W slices, 1: entry chunks
         if (role == 0) {
             if (elect_one()) {
-                long long q = 0;
+                int s = 0;
+                std::uint32_t phase = 1;
                 for (int g = 0; g < my_units; ++g) {
                     const window_unit unit = unit_of(g);
-                    for (int w = unit.w0; w < unit.w1; ++w, ++q) {
-                        const int s = static_cast<int>(q % STAGES);
-                        bar_wait(smem_addr(w_empty + s), static_cast<std::uint32_t>(((q / STAGES) & 1) ^ 1), abort_flag);
+                    for (int w = unit.w0; w < unit.w1; ++w) {
+                        bar_wait(smem_addr(w_empty + s), phase, abort_flag);
                         bar_arrive_expect_tx(smem_addr(w_full + s), REC);
                         bulk_copy_g2s(wstage0 + s * REC, p.records + static_cast<std::size_t>(w) * p.record_stride, REC, smem_addr(w_full + s));
+                        if (++s == STAGES) { s = 0; phase ^= 1u; }
                     }
                 }
             }
         } else {
-            const int mine_mod = role - 1;
-            long long qc = 0;
+            int cs = 0;
+            std::uint32_t phase = 1;
             for (int gi = 0; gi < my_units; ++gi) {
                 const window_unit unit = unit_of(gi);
                 const std::int64_t seg0 = static_cast<std::int64_t>(unit.group) * p.windows;
@@ -478,9 +622,8 @@ __global__ void __launch_bounds__(kThreads, 1) qcsr_fwd_blocked_kernel(const blo
                         std::int64_t at = lo;
                         do {
                             const int count = static_cast<int>(min(static_cast<std::int64_t>(kChunkEntries), hi - at));
-                            if (qc % kChunkLoaders == mine_mod && elect_one()) {
-                                const int cs = static_cast<int>(qc % CS);
-                                bar_wait(smem_addr(c_empty + cs), static_cast<std::uint32_t>(((qc / CS) & 1) ^ 1), abort_flag);
+                            if (elect_one()) {
+                                bar_wait(smem_addr(c_empty + cs), phase, abort_flag);
                                 chunk_meta[cs] = (count << 1) | (at + count >= hi ? 1 : 0);
                                 if (count > 0) {
                                     bar_arrive_expect_tx(smem_addr(c_full + cs), static_cast<std::uint32_t>(count) * 4u);
@@ -491,7 +634,7 @@ __global__ void __launch_bounds__(kThreads, 1) qcsr_fwd_blocked_kernel(const blo
                                 }
                             }
                             at += count;
-                            ++qc;
+                            if (++cs == CS) { cs = 0; phase ^= 1u; }
                         } while (at < hi);
                     }
                 }
@@ -510,7 +653,7 @@ __global__ void __launch_bounds__(kThreads, 1) qcsr_fwd_blocked_kernel(const blo
 
 template<int NC, int CS> constexpr std::size_t blocked_smem_bytes() {
     return 2 * kABufBytes + w_stages(NC, CS) * record_bytes(NC) + CS * kChunkBytes + kRows * 4 +
-           (6 + 2 * w_stages(NC, CS) + 2 * CS) * sizeof(std::uint64_t) + (CS + 1) * 4 + 16;
+           (4 + 2 * w_stages(NC, CS) + 2 * CS + 2 * most_sets(NC)) * sizeof(std::uint64_t) + (CS + 1) * 4 + 16;
 }
 
 template<int NC, int N, int CS, bool BAKED>
@@ -572,7 +715,7 @@ __global__ void __launch_bounds__(kThreads2, 1) qcsr_fwd_blocked2_kernel(const b
     // stages as buffers (N = 128) that would be a cycle -- the group waits for its next window's W, whose copy waits for
     // the release the group has not passed on yet -- so there the MMA warps commit to the stage's barrier themselves.
     constexpr bool FORWARD_W_RELEASE = STAGES > 2;
-    constexpr int kTmemCols = kSubBlocks * NC < 32 ? 32 : kSubBlocks * NC;
+    constexpr int SETS = most_sets(NC), kTmemCols = accumulator_columns(NC, N);
     const std::uint32_t IDESC = p.idesc;
     extern __shared__ __align__(1024) unsigned char smem[];
     // [2][A tile] | [STAGES][W window] | [2][kRing2][entry chunk] | barriers | chunk meta | tmem | abort | scratch
@@ -584,9 +727,9 @@ __global__ void __launch_bounds__(kThreads2, 1) qcsr_fwd_blocked2_kernel(const b
     std::uint64_t *w_empty = w_full + STAGES;     // [STAGES] MMA commit -> W loader
     std::uint64_t *c_full = w_empty + STAGES;     // [CHUNKS] copy engine -> scatter group
     std::uint64_t *c_empty = c_full + CHUNKS;     // [CHUNKS] scatter group -> chunk loader (one arrival per warp)
-    std::uint64_t *acc_full = c_empty + CHUNKS;   // MMA commit -> epilogue warps
-    std::uint64_t *acc_empty = acc_full + 1;      // epilogue warps -> MMA
-    std::uint64_t *mma_drain = acc_empty + 1;     // [2] MMA commit -> the MMA warp itself, used once, after an abort
+    std::uint64_t *acc_full = c_empty + CHUNKS;   // [SETS] MMA commit -> epilogue warps
+    std::uint64_t *acc_empty = acc_full + SETS;   // [SETS] epilogue warps -> MMA
+    std::uint64_t *mma_drain = acc_empty + SETS;  // [2] MMA commit -> the MMA warp itself, used once, after an abort
     volatile int *chunk_meta = reinterpret_cast<volatile int *>(mma_drain + 2); // [CHUNKS] (entries << 1) | last chunk of its window
     std::uint32_t *tmem_slot = reinterpret_cast<std::uint32_t *>(const_cast<int *>(chunk_meta) + CHUNKS);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
@@ -611,8 +754,10 @@ __global__ void __launch_bounds__(kThreads2, 1) qcsr_fwd_blocked2_kernel(const b
             bar_init(smem_addr(c_full + s), 1);
             bar_init(smem_addr(c_empty + s), kGroupWarps);
         }
-        bar_init(smem_addr(acc_full), kSubBlocks);
-        bar_init(smem_addr(acc_empty), kEpilogueWarps);
+        for (int k = 0; k < SETS; ++k) {
+            bar_init(smem_addr(acc_full + k), kSubBlocks);
+            bar_init(smem_addr(acc_empty + k), kEpilogueWarps);
+        }
         bar_init(smem_addr(mma_drain), 1);
         bar_init(smem_addr(mma_drain + 1), 1);
         *abort_flag = 0;
@@ -635,114 +780,100 @@ __global__ void __launch_bounds__(kThreads2, 1) qcsr_fwd_blocked2_kernel(const b
     if (warp < kProducerWarps) {
         // ================= two scatter groups; group 0 also writes Y =================
         const int grp = warp / kGroupWarps, gtid = tid - grp * kGroupThreads;
-        const int sub = tid >> 7;
         // fp16 operands were stored times powers of two: the result is divided by both again
         const float alpha = p.alpha * p.result_scale / (p.w_absmax != nullptr ? operand_scale(__uint_as_float(__ldg(p.w_absmax))) : 1.0f);
         unsigned char *tile = smem + grp * kABufBytes;
-        long long q = 0;  // windows of this CTA, both groups count all of them
-        long long qc = 0; // chunks this group has consumed
+        unsigned q = 0;  // windows of this CTA, both groups count all of them
+        unsigned qc = 0; // chunks this group has consumed
+        int s = 0;       // W stage of the window, and its phase
+        std::uint32_t w_phase = 0;
+        part_sums<NC, N> parts(tmem_base, acc_full, acc_empty, p.split.parts, abort_flag, limit);
         for (int gi = 0; gi < my_units; ++gi) {
             const window_unit unit = unit_of(gi);
-            const std::int64_t row = static_cast<std::int64_t>(unit.group) * kRows + tid;
-            for (int w = unit.w0; w < unit.w1; ++w, ++q) {
-                if (static_cast<int>(q & 1) != grp) continue;
-                // The window's first chunk (all of it for all but the densest matrices) goes into registers while the tile
-                // is still being read by the previous window's MMAs: between the tile's release and its hand-over there
-                // are then only stores.
-                bool last;
-                uint4 held[kChunk2Entries / (kGroupThreads * 4)];
-                {
-                    const int cs = grp * kRing2 + static_cast<int>(qc % kRing2);
-                    bar_wait(smem_addr(c_full + cs), static_cast<std::uint32_t>((qc / kRing2) & 1), abort_flag, limit);
-                    const int meta = chunk_meta[cs];
-                    const int count = *abort_flag != 0 ? 0 : (meta >> 1);
-                    last = (meta & 1) != 0 || *abort_flag != 0;
-                    const uint4 *chunk = reinterpret_cast<const uint4 *>(chunk_base + cs * kChunk2Bytes);
-#pragma unroll
-                    for (int k = 0; k < kChunk2Entries / (kGroupThreads * 4); ++k) { // segments are padded to multiples of 4
-                        const int i = (k * kGroupThreads + gtid) * 4;
-                        held[k] = i < count ? chunk[i >> 2] : make_uint4(kInvalidEntry, kInvalidEntry, kInvalidEntry, kInvalidEntry);
-                    }
-                    // the words are used much later, but they must be in the registers before the stage goes back to the copy engine
+            int taken = 0;
+            for (int w = unit.w0; w < unit.w1;) { // up to the next parts to take (the take inside the loop over windows cost 1.7 %)
+                const int stop = grp == 0 ? window_of_take(unit, taken, p.windows, p.split.parts, parts.sets) : unit.w1;
+                for (; w < stop; ++w, ++q, s = s + 1 == STAGES ? 0 : s + 1, w_phase ^= s == 0 ? 1u : 0u) {
+                    if (static_cast<int>(q & 1u) != grp) continue;
+                    // The window's first chunk (all of it for all but the densest matrices) goes into registers while the tile
+                    // is still being read by the previous window's MMAs: between the tile's release and its hand-over there
+                    // are then only stores.
+                    bool last;
+                    uint4 held[kChunk2Entries / (kGroupThreads * 4)];
                     {
-                        std::uint32_t all = 0;
+                        const int cs = grp * kRing2 + static_cast<int>(qc % kRing2);
+                        bar_wait(smem_addr(c_full + cs), (qc / kRing2) & 1u, abort_flag, limit);
+                        const int meta = chunk_meta[cs];
+                        const int count = *abort_flag != 0 ? 0 : (meta >> 1);
+                        last = (meta & 1) != 0 || *abort_flag != 0;
+                        const uint4 *chunk = reinterpret_cast<const uint4 *>(chunk_base + cs * kChunk2Bytes);
 #pragma unroll
-                        for (int k = 0; k < kChunk2Entries / (kGroupThreads * 4); ++k) all |= held[k].x | held[k].y | held[k].z | held[k].w;
-                        arrive_when_loaded(smem_addr(c_empty + cs), all, lane, static_cast<std::uint32_t>(p.windows) >> 31);
-                    }
-                    ++qc;
-                }
-                // The hand-over of the tile also vouches for the window's W stage: one warp of the group waits for it here,
-                // where the group has slack, and the MMA warps then wait for a single barrier per window.
-                if (gtid < 32) bar_wait(smem_addr(w_full + static_cast<int>(q % STAGES)), static_cast<std::uint32_t>((q / STAGES) & 1), abort_flag, limit);
-                bar_wait(smem_addr(a_empty + grp), static_cast<std::uint32_t>(((q >> 1) & 1) ^ 1), abort_flag, limit);
-                // the MMAs of the group's previous window are done with the tile, hence with that window's W stage too: the
-                // MMA warps commit to the tile's barrier only, and the release of the W stage is passed on from here
-                if (FORWARD_W_RELEASE && gtid == 0 && q >= 2) bar_arrive(smem_addr(w_empty + static_cast<int>((q - 2) % STAGES)));
-#pragma unroll
-                for (int k = 0; k < kABufBytes / (kGroupThreads * 8); ++k) // 8-byte stores: a warp's 16-byte store costs 7 wavefronts of
-                    *reinterpret_cast<uint2 *>(tile + k * (kGroupThreads * 8) + gtid * 8) = make_uint2(0u, 0u); // the LSU data pipe for 512 bytes, two 8-byte stores 4 (4.79 -> 4.60 ms)
-                // the whole tile is zero before anyone of the group scatters (named barrier 1 or 2)
-                if (grp == 0) asm volatile("bar.sync 1, %0;" ::"n"(kGroupThreads) : "memory");
-                else asm volatile("bar.sync 2, %0;" ::"n"(kGroupThreads) : "memory");
-#pragma unroll
-                for (int k = 0; k < kChunk2Entries / (kGroupThreads * 4); ++k) {
-                    const std::uint32_t e[4] = {held[k].x, held[k].y, held[k].z, held[k].w};
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) // padding words (top bit set) are not stored
-                        if (static_cast<int>(e[j]) >= 0)
-                            *reinterpret_cast<unsigned short *>(tile + (((e[j] >> 16) & 0x7fffu) << 1)) = static_cast<unsigned short>(e[j] & 0xffffu);
-                }
-                int guard = 0;
-                while (!last && ++guard < (1 << 20)) { // further chunks of a long segment: scattered from shared memory
-                    const int cs = grp * kRing2 + static_cast<int>(qc % kRing2);
-                    bar_wait(smem_addr(c_full + cs), static_cast<std::uint32_t>((qc / kRing2) & 1), abort_flag, limit);
-                    const int meta = chunk_meta[cs];
-                    const int count = *abort_flag != 0 ? 0 : (meta >> 1);
-                    last = (meta & 1) != 0 || *abort_flag != 0;
-                    const uint4 *chunk = reinterpret_cast<const uint4 *>(chunk_base + cs * kChunk2Bytes);
-                    for (int i = gtid * 4; i < count; i += kGroupThreads * 4) {
-                        const uint4 e4 = chunk[i >> 2];
-                        const std::uint32_t e[4] = {e4.x, e4.y, e4.z, e4.w};
-#pragma unroll
-                        for (int k = 0; k < 4; ++k) {
-                            unsigned char *dst = static_cast<int>(e[k]) >= 0 ? tile + (((e[k] >> 16) & 0x7fffu) << 1) : scratch_slot;
-                            *reinterpret_cast<unsigned short *>(dst) = static_cast<unsigned short>(e[k] & 0xffffu);
+                        for (int k = 0; k < kChunk2Entries / (kGroupThreads * 4); ++k) { // segments are padded to multiples of 4
+                            const int i = (k * kGroupThreads + gtid) * 4;
+                            held[k] = i < count ? chunk[i >> 2] : make_uint4(kInvalidEntry, kInvalidEntry, kInvalidEntry, kInvalidEntry);
                         }
+                        // the words are used much later, but they must be in the registers before the stage goes back to the copy engine
+                        {
+                            std::uint32_t all = 0;
+#pragma unroll
+                            for (int k = 0; k < kChunk2Entries / (kGroupThreads * 4); ++k) all |= held[k].x | held[k].y | held[k].z | held[k].w;
+                            arrive_when_loaded(smem_addr(c_empty + cs), all, lane, static_cast<std::uint32_t>(p.windows) >> 31);
+                        }
+                        ++qc;
                     }
+                    // The hand-over of the tile also vouches for the window's W stage: one warp of the group waits for it here,
+                    // where the group has slack, and the MMA warps then wait for a single barrier per window.
+                    if (gtid < 32) bar_wait(smem_addr(w_full + s), w_phase, abort_flag, limit);
+                    bar_wait(smem_addr(a_empty + grp), ((q >> 1) & 1u) ^ 1u, abort_flag, limit);
+                    // the MMAs of the group's previous window are done with the tile, hence with that window's W stage too: the
+                    // MMA warps commit to the tile's barrier only, and the release of the W stage is passed on from here
+                    if (FORWARD_W_RELEASE && gtid == 0 && q >= 2) bar_arrive(smem_addr(w_empty + (s >= 2 ? s - 2 : s + STAGES - 2)));
+#pragma unroll
+                    for (int k = 0; k < kABufBytes / (kGroupThreads * 8); ++k) // 8-byte stores: a warp's 16-byte store costs 7 wavefronts of
+                        *reinterpret_cast<uint2 *>(tile + k * (kGroupThreads * 8) + gtid * 8) = make_uint2(0u, 0u); // the LSU data pipe for 512 bytes, two 8-byte stores 4 (4.79 -> 4.60 ms)
+                    // the whole tile is zero before anyone of the group scatters (named barrier 1 or 2)
+                    if (grp == 0) asm volatile("bar.sync 1, %0;" ::"n"(kGroupThreads) : "memory");
+                    else asm volatile("bar.sync 2, %0;" ::"n"(kGroupThreads) : "memory");
+#pragma unroll
+                    for (int k = 0; k < kChunk2Entries / (kGroupThreads * 4); ++k) {
+                        const std::uint32_t e[4] = {held[k].x, held[k].y, held[k].z, held[k].w};
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) // padding words (top bit set) are not stored
+                            if (static_cast<int>(e[j]) >= 0)
+                                *reinterpret_cast<unsigned short *>(tile + (((e[j] >> 16) & 0x7fffu) << 1)) = static_cast<unsigned short>(e[j] & 0xffffu);
+                    }
+                    int guard = 0;
+                    while (!last && ++guard < (1 << 20)) { // further chunks of a long segment: scattered from shared memory
+                        const int cs = grp * kRing2 + static_cast<int>(qc % kRing2);
+                        bar_wait(smem_addr(c_full + cs), (qc / kRing2) & 1u, abort_flag, limit);
+                        const int meta = chunk_meta[cs];
+                        const int count = *abort_flag != 0 ? 0 : (meta >> 1);
+                        last = (meta & 1) != 0 || *abort_flag != 0;
+                        const uint4 *chunk = reinterpret_cast<const uint4 *>(chunk_base + cs * kChunk2Bytes);
+                        for (int i = gtid * 4; i < count; i += kGroupThreads * 4) {
+                            const uint4 e4 = chunk[i >> 2];
+                            const std::uint32_t e[4] = {e4.x, e4.y, e4.z, e4.w};
+#pragma unroll
+                            for (int k = 0; k < 4; ++k) {
+                                unsigned char *dst = static_cast<int>(e[k]) >= 0 ? tile + (((e[k] >> 16) & 0x7fffu) << 1) : scratch_slot;
+                                *reinterpret_cast<unsigned short *>(dst) = static_cast<unsigned short>(e[k] & 0xffffu);
+                            }
+                        }
+                        __syncwarp();
+                        if (lane == 0) bar_arrive(smem_addr(c_empty + cs));
+                        ++qc;
+                    }
+                    fence_async_proxy(); // the tile was written with ordinary stores, the MMA reads it through the async proxy
                     __syncwarp();
-                    if (lane == 0) bar_arrive(smem_addr(c_empty + cs));
-                    ++qc;
+                    if (lane == 0) bar_arrive(smem_addr(a_full + grp));
                 }
-                fence_async_proxy(); // the tile was written with ordinary stores, the MMA reads it through the async proxy
-                __syncwarp();
-                if (lane == 0) bar_arrive(smem_addr(a_full + grp));
-            }
-
-            // ---- thread t < 256 (group 0) writes row t of the row group: TMEM lane = row within the sub-block
-            if (grp != 0) continue;
-            bar_wait(smem_addr(acc_full), static_cast<std::uint32_t>(gi & 1), abort_flag, limit);
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-#pragma unroll
-            for (int h = 0; h < N / 32; ++h) {
-                float v[32];
-                tmem_ld32(tmem_base + (static_cast<std::uint32_t>((warp & 3) * 32) << 16) + sub * NC + h * 32, v);
-                if constexpr (NC == 2 * N) {
-                    float lo[32];
-                    tmem_ld32(tmem_base + (static_cast<std::uint32_t>((warp & 3) * 32) << 16) + sub * NC + N + h * 32, lo);
-#pragma unroll
-                    for (int c = 0; c < 32; ++c) v[c] += lo[c];
-                }
-                if (unit.slot >= 0) { // raw sums of a part
-                    store_row32(p.split.sums + (static_cast<std::int64_t>(unit.slot) * kRows + tid) * N + h * 32, v, 1.0f, 0.0f, nullptr, h * 32, CB200_EPILOGUE_NONE);
-                } else if (row < p.row_end) {
-                    float *out = p.y + row * p.y_ld + h * 32;
-                    store_row32(out, v, alpha, p.beta, p.bias, h * 32, p.epilogue);
+                if (w < unit.w1) {
+                    __syncwarp();
+                    parts.take(p, unit, taken);
+                    taken += parts_at_a_time(parts.sets);
                 }
             }
-            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            __syncwarp();
-            if (lane == 0) bar_arrive(smem_addr(acc_empty));
+            if (grp == 0) parts.finish(p, unit, taken, alpha);
         }
     } else if (warp < kProducerWarps + kSubBlocks) {
         // ================= MMA issuers: one warp per 128-row sub-block of the tile =================
@@ -755,30 +886,36 @@ __global__ void __launch_bounds__(kThreads2, 1) qcsr_fwd_blocked2_kernel(const b
         // therefore still issued (on stale tiles, into this CTA's own TMEM; the waits return at once) and only
         // the end of the role looks at the flag.
         const int sb = warp - kProducerWarps;
-        long long q = 0;
+        const int sets = accumulator_sets<NC>(p.split.parts);
+        unsigned q = 0;
+        int use = 0, s = 0;
         for (int g = 0; g < my_units; ++g) {
             const window_unit unit = unit_of(g);
-            bar_wait(smem_addr(acc_empty), static_cast<std::uint32_t>((g & 1) ^ 1), abort_flag, limit);
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            for (int w = unit.w0; w < unit.w1; ++w, ++q) {
-                const std::uint32_t b = static_cast<std::uint32_t>(q & 1);
-                const int s = static_cast<int>(q % STAGES);
-                bar_wait(smem_addr(a_full + b), static_cast<std::uint32_t>((q >> 1) & 1), abort_flag, limit); // tile and W stage
+            for (int k = unit.k0, w = unit.w0; k < unit.k0 + unit.pieces; ++k, ++use) {
+                const int set = use % sets, first = w, end = part_begin(p.windows, p.split.parts, k + 1);
+                bar_wait(smem_addr(acc_empty + set), static_cast<std::uint32_t>(((use / sets) & 1) ^ 1), abort_flag, limit);
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                // (not under elect_one: MMAs issued back to back take the operand reads' bandwidth from the scatter group's stores
-                // in bursts, 575 against 542 us on an eighth of that matrix)
-                if (lane == 0) {
-                    const std::uint32_t a_tile = smem0 + b * kABufBytes + sb * kSubBlockBytes;
-                    const std::uint32_t b_tile = wstage0 + s * WREC;
+                const std::uint32_t acc = tmem_base + set * (kSubBlocks * NC) + sb * NC;
+                for (; w < end; ++w, ++q) {
+                    const std::uint32_t b = q & 1u;
+                    bar_wait(smem_addr(a_full + b), (q >> 1) & 1u, abort_flag, limit); // tile and W stage
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    // (not under elect_one: MMAs issued back to back take the operand reads' bandwidth from the scatter group's
+                    // stores in bursts, 575 against 542 us on an eighth of that matrix)
+                    if (lane == 0) {
+                        const std::uint32_t a_tile = smem0 + b * kABufBytes + sb * kSubBlockBytes;
+                        const std::uint32_t b_tile = wstage0 + s * WREC;
 #pragma unroll
-                    for (int kk = 0; kk < kWin / 16; ++kk)
-                        mma_bf16(tmem_base + sb * NC, smem_desc_sw128(a_tile + (kk >> 2) * kHalfBytes + (kk & 3) * 32), smem_desc(b_tile + kk * 256),
-                                 IDESC, w > unit.w0 || kk > 0);
-                    mma_commit(smem_addr(a_empty + b));
-                    if constexpr (!FORWARD_W_RELEASE) mma_commit(smem_addr(w_empty + s));
-                    if (w == unit.w1 - 1) mma_commit(smem_addr(acc_full));
+                        for (int kk = 0; kk < kWin / 16; ++kk)
+                            mma_bf16(acc, smem_desc_sw128(a_tile + (kk >> 2) * kHalfBytes + (kk & 3) * 32), smem_desc(b_tile + kk * 256), IDESC,
+                                     w > first || kk > 0);
+                        mma_commit(smem_addr(a_empty + b));
+                        if constexpr (!FORWARD_W_RELEASE) mma_commit(smem_addr(w_empty + s));
+                        if (w == end - 1) mma_commit(smem_addr(acc_full + set));
+                    }
+                    __syncwarp();
+                    s = s + 1 == STAGES ? 0 : s + 1;
                 }
-                __syncwarp();
             }
         }
         // after an abort: the MMAs already issued finish before the CTA frees its TMEM and shared memory
@@ -873,7 +1010,7 @@ __global__ void __launch_bounds__(kThreads2, 1) qcsr_fwd_blocked2_kernel(const b
 template<int NC, int N, bool TEST_HOOK>
 cb200_status launch_blocked2_as(const blocked_params &p, int sm_count, cudaStream_t stream) {
     constexpr std::size_t smem = 2 * kABufBytes + w2_stages(NC) * NC * kWin * 2 + 2 * kRing2 * kChunk2Bytes +
-                                 (8 + 2 * w2_stages(NC) + 4 * kRing2) * sizeof(std::uint64_t) + 2 * kRing2 * 4 + 24;
+                                 (6 + 2 * w2_stages(NC) + 4 * kRing2 + 2 * most_sets(NC)) * sizeof(std::uint64_t) + 2 * kRing2 * 4 + 24;
     static_assert(smem <= 232448, "shared memory budget");
     CB200_CUDA_OK(cudaFuncSetAttribute(qcsr_fwd_blocked2_kernel<NC, N, TEST_HOOK>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
     const unsigned grid = static_cast<unsigned>(std::min(unit_count(p.split, p.group_begin, p.group_end), sm_count));
@@ -894,37 +1031,56 @@ std::uint64_t qcsr_blocked_workspace_bytes(std::int64_t cols, std::int64_t n) {
     return static_cast<std::uint64_t>(256 + windows * record_bytes(static_cast<int>(n)));
 }
 
+// Parts of a group's windows, `columns` to an accumulator: a function of the genes and N alone, so that every shard of a matrix
+// sums a row the same way.  More parts share a small launch out better (over all group counts below the SMs', 262 windows: three
+// parts take 183 window times on average, six 169, twelve 166) and cost every whole group their turns through the running sum
+// (six parts: two turns, 0.8 % of 303,104 x 33,538 at N = 64).
+static int window_parts(int windows, std::int64_t columns) {
+    if (columns > 64) return windows < 8 ? 1 : windows < 64 ? 2 : 3;
+    return windows < 8 ? 1 : windows < 16 ? 2 : windows < 128 ? 3 : 6;
+}
 // A launch over G groups on S SMs takes ceil(G / S) rounds of a group's windows, the last of them nearly empty as often as
 // not (125,000 rows: 489 groups, 3.3 rounds of 148 in the time of 4), and fewer groups than SMs leave the rest idle
-// altogether.  The groups of the last round, or of the last two, are cut into the number of parts that takes the fewest
-// window times, with four of them charged for the start and the epilogue of a part and five for the pass that adds the parts.
-// 125,000 x 33,538 at N = 64 with split products (two passes): 1,429 -> 1,310 us, the 45 groups behind 3 x 148 in three parts each.
-window_split_plan qcsr_window_split(std::int64_t rows, std::int64_t cols, int sm_count) {
+// altogether.  So the parts of the last round's groups, or of the last two's, are given to CTAs of their own where that takes
+// fewer window times, with four of them charged for the start and the epilogue of a unit, three for the pass that adds the
+// sums and one for 60 of the sums.  5,000 x 33,538 at N = 64: 189 -> 56 us; 125,000 rows, split products (two passes): 1,428 ->
+// 1,181 us, the 45 groups behind 3 x 148 in three units each.
+window_split_plan qcsr_window_split(std::int64_t rows, std::int64_t cols, std::int64_t columns, int sm_count) {
+    constexpr int kMostSums = 6; // of cut groups, per SM: what bounds the workspace
     const std::int64_t groups = (rows + kRows - 1) / kRows;
     const int windows = static_cast<int>((cols + kWin - 1) / kWin);
     window_split_plan best;
     best.whole = groups;
-    if (groups == 0 || windows < 2) return best;
-    constexpr double kPerPart = 4.0, kAdding = 5.0;
-    double best_cost = static_cast<double>((groups + sm_count - 1) / sm_count) * (windows + kPerPart);
+    if (columns != 0) best.parts = window_parts(windows, columns);
+    if (groups == 0 || windows < 2 || (columns != 0 && best.parts == 1)) return best;
+    constexpr double kPerUnit = 4.0, kAdding = 3.0, kPerSum = 1.0 / 60.0;
+    double best_cost = static_cast<double>((groups + sm_count - 1) / sm_count) * (windows + kPerUnit);
+    const int parts = best.parts;
     for (std::int64_t whole = groups / sm_count * sm_count; whole >= 0 && groups - whole < 2 * sm_count; whole -= sm_count) {
         const std::int64_t cut = groups - whole;
-        for (int parts = 2; cut > 0 && parts <= windows / 2 && cut * parts <= 3 * sm_count; ++parts) {
-            const double rounds = static_cast<double>((cut * parts + sm_count - 1) / sm_count);
-            const double cost = static_cast<double>(whole / sm_count) * (windows + kPerPart) + rounds * ((windows + parts - 1) / parts + kPerPart) + kAdding;
+        for (int units = 2; cut > 0 && units <= (columns == 0 ? windows / 2 : parts); ++units) {
+            const int into = columns == 0 ? units : parts, per_unit = (into + units - 1) / units;
+            const bool pairs = columns != 0 && columns <= 64 && per_unit > 1;
+            if ((into + per_unit - 1) / per_unit != units || (pairs && per_unit % 2 != 0)) continue;
+            const int slots = pairs ? (into + 1) / 2 : into;
+            if (cut * slots > (columns == 0 ? 3 : kMostSums) * sm_count) continue;
+            const double rounds = static_cast<double>((cut * units + sm_count - 1) / sm_count);
+            const double cost = static_cast<double>(whole / sm_count) * (windows + kPerUnit) + rounds * ((windows * per_unit + into - 1) / into + kPerUnit) + kAdding +
+                                kPerSum * static_cast<double>(cut * slots);
             if (cost < 0.99 * best_cost) {
                 best_cost = cost;
                 best.whole = whole;
-                best.parts = parts;
+                best.parts = into;
+                best.per_unit = per_unit;
+                best.slots = slots;
             }
         }
     }
     return best;
 }
-std::uint64_t qcsr_window_split_bytes(std::int64_t rows, std::int64_t cols, std::int64_t n, int sm_count) {
-    const window_split_plan plan = qcsr_window_split(rows, cols, sm_count);
-    if (plan.parts == 1) return 0u;
-    return static_cast<std::uint64_t>((rows + kRows - 1) / kRows - plan.whole) * static_cast<std::uint64_t>(plan.parts) * kRows * static_cast<std::uint64_t>(n) * 4u;
+std::uint64_t qcsr_window_split_bytes(std::int64_t rows, std::int64_t cols, std::int64_t n, std::int64_t columns, int sm_count) {
+    const window_split_plan plan = qcsr_window_split(rows, cols, columns, sm_count);
+    return static_cast<std::uint64_t>((rows + kRows - 1) / kRows - plan.whole) * static_cast<std::uint64_t>(plan.slots) * kRows * static_cast<std::uint64_t>(n) * 4u;
 }
 
 bool qcsr_blocked_shape_ok(std::int64_t rows, std::int64_t cols, std::int64_t n, int bits, int dense_dtype) {
@@ -1108,7 +1264,6 @@ cb200_status launch_qcsr_forward_blocked(const qcsr_view &x, const dense_args &d
                                    workspace_bytes >= qcsr_blocked_workspace_bytes(x.cols, 2 * d.n) ? 1 : 0;
     const std::int64_t columns = both_parts != 0 ? 2 * d.n : d.n;
     p.record_stride = record_bytes(static_cast<int>(columns));
-    p.split = split_of_launch(x, d.n, workspace, workspace_bytes, qcsr_blocked_workspace_bytes(x.cols, columns), sm_count);
     p.alpha = d.alpha; p.status = status;
     p.result_scale = half ? 1.0f / layout.value_scale : 1.0f;
     p.w_absmax = half ? w_absmax : nullptr;
@@ -1154,7 +1309,9 @@ cb200_status launch_qcsr_forward_blocked(const qcsr_view &x, const dense_args &d
         p.bias = d.bias;
         p.epilogue = i + 1 == pass_count ? d.epilogue : CB200_EPILOGUE_NONE;
         cb200_status st;
-        p.idesc = instr_desc(static_cast<int>(both_parts != 0 && passes[i].value_part == 0 ? columns : d.n), half);
+        const std::int64_t pass_columns = both_parts != 0 && passes[i].value_part == 0 ? columns : d.n;
+        p.idesc = instr_desc(static_cast<int>(pass_columns), half);
+        p.split = split_of_launch(x, d.n, pass_columns, workspace, workspace_bytes, qcsr_blocked_workspace_bytes(x.cols, columns), sm_count);
         if (both_parts != 0 && passes[i].value_part == 0) {
             if (two_groups) st = d.n == 64 ? launch_blocked2<128, 64>(p, sm_count, stream) : launch_blocked2<64, 32>(p, sm_count, stream);
             else st = d.n == 64 ? launch_cs<128, 64, 3, true>(p, sm_count, stream) : launch_cs<64, 32, 3, true>(p, sm_count, stream);
@@ -1166,7 +1323,7 @@ cb200_status launch_qcsr_forward_blocked(const qcsr_view &x, const dense_args &d
             }
         }
         if (st != CB200_STATUS_SUCCESS) return st;
-        st = launch_add_parts(p.split, p.group_begin, p.group_end, row_end, static_cast<int>(d.n), d.out, d.out_ld, p.alpha, p.beta, p.bias, p.epilogue,
+        st = launch_add_parts(p.split, pass_columns <= 64, p.group_begin, p.group_end, row_end, static_cast<int>(d.n), d.out, d.out_ld, p.alpha, p.beta, p.bias, p.epilogue,
                               p.result_scale, p.w_absmax, nullptr, stream);
         if (st != CB200_STATUS_SUCCESS) return st;
     }

@@ -606,7 +606,7 @@ cb200_status launch_qcsr_forward_codes(const qcsr_view &x, const dense_args &d, 
     p.group_begin = row_begin / kRows; p.group_end = (row_end + kRows - 1) / kRows; p.windows = layout.windows;
     p.alpha = d.alpha; p.beta = d.beta; p.bias = d.bias; p.epilogue = d.epilogue; p.status = status;
     p.w_absmax = w_absmax; p.value_bound = value_bound;
-    p.split = split_of_launch(x, d.n, workspace, workspace_bytes, qcsr_codes_workspace_bytes(x.cols, d.n), sm_count);
+    p.split = split_of_launch(x, d.n, 0, workspace, workspace_bytes, qcsr_codes_workspace_bytes(x.cols, d.n), sm_count);
     *taken = true;
     cb200_status st;
     switch (d.n) {
@@ -615,7 +615,7 @@ cb200_status launch_qcsr_forward_codes(const qcsr_view &x, const dense_args &d, 
     default: st = launch_codes<128>(p, sm_count, stream); break;
     }
     if (st != CB200_STATUS_SUCCESS) return st;
-    return launch_add_parts(p.split, p.group_begin, p.group_end, row_end, static_cast<int>(d.n), d.out, d.out_ld, p.alpha, p.beta, p.bias, p.epilogue,
+    return launch_add_parts(p.split, false, p.group_begin, p.group_end, row_end, static_cast<int>(d.n), d.out, d.out_ld, p.alpha, p.beta, p.bias, p.epilogue,
                             1.0f, w_absmax, value_bound, stream);
 }
 

@@ -168,10 +168,10 @@ __global__ void __launch_bounds__(kDenseThreads, 1) qcsr_fwd_dense_kernel(const 
                 float v[32];
                 tmem_ld32(tmem_base + (static_cast<std::uint32_t>((warp & 3) * 32) << 16) + ab * kAccCols + sub * NC + h * 32, v);
                 if (unit.slot >= 0) { // raw sums of a part
-                    store_row32(p.split.sums + (static_cast<std::int64_t>(unit.slot) * kRows + tid) * NC + h * 32, v, 1.0f, 0.0f, nullptr, h * 32, CB200_EPILOGUE_NONE);
+                    store_row(p.split.sums + (static_cast<std::int64_t>(unit.slot) * kRows + tid) * NC + h * 32, v, 1.0f, 0.0f, nullptr, h * 32, CB200_EPILOGUE_NONE);
                 } else if (row < p.row_end) {
                     float *out = p.y + row * p.y_ld + h * 32;
-                    store_row32(out, v, p.alpha * p.result_scale / (p.w_absmax != nullptr ? operand_scale(__uint_as_float(__ldg(p.w_absmax))) : 1.0f), p.beta, p.bias, h * 32, p.epilogue);
+                    store_row(out, v, p.alpha * p.result_scale / (p.w_absmax != nullptr ? operand_scale(__uint_as_float(__ldg(p.w_absmax))) : 1.0f), p.beta, p.bias, h * 32, p.epilogue);
                 }
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -351,7 +351,7 @@ cb200_status launch_qcsr_forward_dense(const qcsr_view &x, const dense_args &d, 
     p.idesc = instr_desc(static_cast<int>(d.n), half);
     p.result_scale = half ? 1.0f / layout.value_scale : 1.0f;
     p.w_absmax = half ? w_absmax : nullptr;
-    p.split = split_of_launch(x, d.n, workspace, workspace_bytes, qcsr_blocked_workspace_bytes(x.cols, d.n), sm_count);
+    p.split = split_of_launch(x, d.n, 0, workspace, workspace_bytes, qcsr_blocked_workspace_bytes(x.cols, d.n), sm_count);
     *taken = true;
     cb200_status st;
     switch (d.n) {
@@ -360,7 +360,7 @@ cb200_status launch_qcsr_forward_dense(const qcsr_view &x, const dense_args &d, 
     default: st = launch_dense<128>(p, sm_count, stream); break;
     }
     if (st != CB200_STATUS_SUCCESS) return st;
-    return launch_add_parts(p.split, p.group_begin, p.group_end, row_end, static_cast<int>(d.n), d.out, d.out_ld, p.alpha, p.beta, p.bias, p.epilogue,
+    return launch_add_parts(p.split, false, p.group_begin, p.group_end, row_end, static_cast<int>(d.n), d.out, d.out_ld, p.alpha, p.beta, p.bias, p.epilogue,
                             p.result_scale, p.w_absmax, nullptr, stream);
 }
 

@@ -335,7 +335,7 @@ __global__ void __launch_bounds__(kThreads, 1) qcsr_fwd_mma_kernel(const mma_par
                 tmem_ld32(tmem_base + (static_cast<std::uint32_t>((warp & 3) * 32) << 16) + sub * NC + h * 32, v);
                 if (row >= 0) {
                     float *out = p.y + row * p.y_ld + h * 32;
-                    store_row32(out, v, p.alpha, p.beta, p.bias, h * 32, p.epilogue);
+                    store_row(out, v, p.alpha, p.beta, p.bias, h * 32, p.epilogue);
                 }
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");

@@ -138,4 +138,50 @@ __device__ __forceinline__ void tmem_ld32(std::uint32_t taddr, float (&v)[32]) {
     for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
 }
 
+// Sixteen columns of this thread's lane of tensor memory, of one, two or three places with one wait.
+__device__ __forceinline__ void tmem_ld16(std::uint32_t at_v, float (&v)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n\t"
+        "tcgen05.wait::ld.sync.aligned;"
+        : "=&f"(v[0]), "=&f"(v[1]), "=&f"(v[2]), "=&f"(v[3]), "=&f"(v[4]), "=&f"(v[5]), "=&f"(v[6]), "=&f"(v[7]), "=&f"(v[8]), "=&f"(v[9]),
+          "=&f"(v[10]), "=&f"(v[11]), "=&f"(v[12]), "=&f"(v[13]), "=&f"(v[14]), "=&f"(v[15])
+        : "r"(at_v)
+        : "memory");
+}
+__device__ __forceinline__ void tmem_ld16(std::uint32_t at_v, std::uint32_t at_u, float (&v)[16], float (&u)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%32];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%33];\n\t"
+        "tcgen05.wait::ld.sync.aligned;"
+        : "=&f"(v[0]), "=&f"(v[1]), "=&f"(v[2]), "=&f"(v[3]), "=&f"(v[4]), "=&f"(v[5]), "=&f"(v[6]), "=&f"(v[7]), "=&f"(v[8]), "=&f"(v[9]),
+          "=&f"(v[10]), "=&f"(v[11]), "=&f"(v[12]), "=&f"(v[13]), "=&f"(v[14]), "=&f"(v[15]), "=&f"(u[0]), "=&f"(u[1]), "=&f"(u[2]),
+          "=&f"(u[3]), "=&f"(u[4]), "=&f"(u[5]), "=&f"(u[6]), "=&f"(u[7]), "=&f"(u[8]), "=&f"(u[9]), "=&f"(u[10]), "=&f"(u[11]),
+          "=&f"(u[12]), "=&f"(u[13]), "=&f"(u[14]), "=&f"(u[15])
+        : "r"(at_v), "r"(at_u)
+        : "memory");
+}
+__device__ __forceinline__ void tmem_ld16(std::uint32_t at_v, std::uint32_t at_u, std::uint32_t at_t, float (&v)[16], float (&u)[16], float (&t)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%48];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%49];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%32, %33, %34, %35, %36, %37, %38, %39, %40, %41, %42, %43, %44, %45, %46, %47}, [%50];\n\t"
+        "tcgen05.wait::ld.sync.aligned;"
+        : "=&f"(v[0]), "=&f"(v[1]), "=&f"(v[2]), "=&f"(v[3]), "=&f"(v[4]), "=&f"(v[5]), "=&f"(v[6]), "=&f"(v[7]), "=&f"(v[8]), "=&f"(v[9]),
+          "=&f"(v[10]), "=&f"(v[11]), "=&f"(v[12]), "=&f"(v[13]), "=&f"(v[14]), "=&f"(v[15]), "=&f"(u[0]), "=&f"(u[1]), "=&f"(u[2]),
+          "=&f"(u[3]), "=&f"(u[4]), "=&f"(u[5]), "=&f"(u[6]), "=&f"(u[7]), "=&f"(u[8]), "=&f"(u[9]), "=&f"(u[10]), "=&f"(u[11]),
+          "=&f"(u[12]), "=&f"(u[13]), "=&f"(u[14]), "=&f"(u[15]), "=&f"(t[0]), "=&f"(t[1]), "=&f"(t[2]), "=&f"(t[3]), "=&f"(t[4]),
+          "=&f"(t[5]), "=&f"(t[6]), "=&f"(t[7]), "=&f"(t[8]), "=&f"(t[9]), "=&f"(t[10]), "=&f"(t[11]), "=&f"(t[12]), "=&f"(t[13]),
+          "=&f"(t[14]), "=&f"(t[15])
+        : "r"(at_v), "r"(at_u), "r"(at_t)
+        : "memory");
+}
+// ... and the way back; tmem_wait_stores before they are read
+__device__ __forceinline__ void tmem_st16(std::uint32_t at, const float (&v)[16]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15};" ::
+                 "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]), "f"(v[8]), "f"(v[9]), "f"(v[10]),
+                 "f"(v[11]), "f"(v[12]), "f"(v[13]), "f"(v[14]), "f"(v[15]), "r"(at)
+                 : "memory");
+}
+__device__ __forceinline__ void tmem_wait_stores() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
 } // namespace cb200

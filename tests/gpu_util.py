@@ -49,3 +49,11 @@ def dense(rng, rows, n, dtype, device, std=0.02, ld=None):
     full = torch.from_numpy(rng.normal(0.0, std, size=(rows, ld)).astype(np.float32)).to(device).to(dtype)
     view = full[:, :n]
     return view, view.float().cpu().numpy()
+
+
+def rows_of(c, lo, hi):
+    """Rows [lo, hi) as a matrix of their own."""
+    s, e, ps, pe = c["row_ptr"][lo], c["row_ptr"][hi], c["packed_row_ptr"][lo], c["packed_row_ptr"][hi]
+    return dict(c, rows=hi - lo, row_ptr=c["row_ptr"][lo:hi + 1] - s, col_idx=c["col_idx"][s:e], values=c["values"][s:e],
+                packed_row_ptr=c["packed_row_ptr"][lo:hi + 1] - ps, packed=c["packed"][ps:pe],
+                offsets=c["offsets"] if c["policy"] == 1 else c["offsets"][lo:hi])

@@ -4,7 +4,7 @@ import pytest
 import torch
 
 from cellerator_b200 import capi, ops
-from gpu_util import assert_forward_close, dense, host_pack, row_l1, to_dev
+from gpu_util import assert_forward_close, dense, host_pack, row_l1, rows_of, to_dev
 
 pytestmark = pytest.mark.gpu
 
@@ -63,14 +63,6 @@ def test_w_re_laid_with_aligned_rows(cuda_device, oracle, n, dtype):
     op = ops.PreparedSpmm(capi.PROJECTION_CSR, c["rows"], c["cols"], n, int(c["row_ptr"][-1]), 8, 1, dtype, cuda_device)
     assert op.workspace_bytes > 256
     check(oracle, cuda_device, c, n, dtype)
-
-
-def rows_of(c, lo, hi):
-    """Rows [lo, hi) as a matrix of their own."""
-    s, e, ps, pe = c["row_ptr"][lo], c["row_ptr"][hi], c["packed_row_ptr"][lo], c["packed_row_ptr"][hi]
-    return dict(c, rows=hi - lo, row_ptr=c["row_ptr"][lo:hi + 1] - s, col_idx=c["col_idx"][s:e], values=c["values"][s:e],
-                packed_row_ptr=c["packed_row_ptr"][lo:hi + 1] - ps, packed=c["packed"][ps:pe],
-                offsets=c["offsets"] if c["policy"] == 1 else c["offsets"][lo:hi])
 
 
 @pytest.mark.parametrize("bits,policy", [(8, 1), (4, 2)])

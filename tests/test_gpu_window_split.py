@@ -5,7 +5,7 @@ import torch
 
 from cellerator_b200 import capi, ops
 from conftest import random_csr
-from gpu_util import dense, host_pack, row_l1, to_dev
+from gpu_util import dense, host_pack, row_l1, rows_of, to_dev
 
 pytestmark = pytest.mark.gpu
 
@@ -51,3 +51,40 @@ def test_cut_groups(cuda_device, oracle, monkeypatch, schedule, bits, n, dtype, 
         narrow = op.run(x, w, torch.empty_like(y)).cpu().numpy()
         assert np.all(np.abs(narrow - y.cpu().numpy()) <= 1e-4 * scale)
     op.close()
+
+
+@pytest.mark.parametrize("schedule,bits,n,dtype,multiply", [
+    ("tensor_blocked", 8, 32, torch.bfloat16, capi.DTYPE_BF16), ("tensor_blocked", 8, 64, torch.bfloat16, capi.DTYPE_BF16),
+    ("tensor_blocked", 4, 128, torch.bfloat16, capi.DTYPE_BF16), ("tensor_blocked", 8, 64, torch.bfloat16, capi.DTYPE_F32),
+    ("tensor_blocked", 8, 32, torch.float32, capi.DTYPE_F32), ("tensor_blocked", 8, 64, torch.float32, capi.DTYPE_F32),
+    ("tensor_blocked", 8, 128, torch.float32, capi.DTYPE_F32)])
+@pytest.mark.parametrize("rows,windows,density", [(256 * 6 + 1, 7, 40), (256 * 6 + 1, 9, 300), (700, 17, 40), (256 * 150 - 7, 9, 12), (1800, 33, 1200),
+                                                  (256 * 13, 64, 60), (256 * 47 + 3, 129, 15), (300, 200, 4000)])
+def test_a_rows_bits_follow_from_its_entries(cuda_device, oracle, monkeypatch, schedule, bits, n, dtype, multiply, rows, windows, density):
+    """The same bits in the whole matrix, in shards that are matrices of their own, and without room for the sums of parts: every
+    number of parts and of parts to a CTA, whole groups beside cut ones, short and long segments."""
+    monkeypatch.setitem(ops.SCHEDULE_REQUEST, capi.PROJECTION_CSR, schedule)
+    rng = np.random.default_rng(rows + windows + n)
+    cols = 128 * windows - 50
+    c = host_pack(oracle, random_csr(rng, rows=rows, cols=cols, max_nnz=min(density, cols), bits=bits, policy=1))
+    w, _ = dense(rng, cols, n, dtype, cuda_device)
+
+    def project(c, uncut=False):
+        x = to_dev(c, cuda_device)
+        op = ops.PreparedSpmm(capi.PROJECTION_CSR, c["rows"], cols, n, x.nnz, bits, 1, dtype, cuda_device, host_row_ptr=x.host_row_ptr,
+                              multiply=multiply, device_matrix=x)
+        assert op.schedule.startswith(schedule)
+        # the status block and the records of W, hi and lo of an fp32 W side by side
+        records = 256 + windows * 128 * (2 * n * (2 if dtype == torch.float32 and n <= 64 else 1) + 8)
+        if uncut and op.workspace_bytes > records:
+            op.workspace_bytes = records
+        y = op.run(x, w, torch.empty(c["rows"], n, device=cuda_device))
+        assert op.status() == 0
+        op.close()
+        return y
+
+    y = project(c)
+    assert torch.equal(project(c, uncut=True), y)
+    cuts = sorted({0, 1, 290, 556, rows // 2 + 100, rows} & set(range(rows + 1)))
+    for lo, hi in zip(cuts[:-1], cuts[1:]):
+        assert torch.equal(project(rows_of(c, lo, hi)), y[lo:hi])
