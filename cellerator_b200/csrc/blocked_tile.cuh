@@ -178,17 +178,16 @@ __device__ __forceinline__ int units_of_cta(const window_split &s, std::int64_t 
 }
 
 // Y of the groups that were cut: the parts' sums in order, then what the epilogue of a whole group does.
-// result_scale / w_absmax / value_bound: the powers of two the operands were stored times (null: none).
+// result_scale / w_absmax: the powers of two the operands were stored times (null: none).
 // paired: the sums of two neighbouring parts are added first.
 __global__ void __launch_bounds__(256) add_parts_kernel(const float *sums, int slots, int paired, int whole, int first_group, std::int64_t row_end,
                                                         int n, float *y, std::int64_t y_ld, float alpha, float beta, const float *bias,
-                                                        int epilogue, float result_scale, const unsigned *w_absmax, const unsigned *value_bound) {
+                                                        int epilogue, float result_scale, const unsigned *w_absmax) {
     wait_for_previous_launch();
     const std::int64_t group = first_group + static_cast<int>(blockIdx.x);
     const float *in = sums + (group - whole) * slots * kRows * n;
     float scale = alpha * result_scale;
     if (w_absmax != nullptr) scale /= operand_scale(__uint_as_float(__ldg(w_absmax)));
-    if (value_bound != nullptr) scale /= operand_scale(__uint_as_float(__ldg(value_bound)));
     const int pieces = kRows * n / 4;
     for (int i = blockIdx.y * 256 + threadIdx.x; i < pieces; i += gridDim.y * 256) {
         const int r = i / (n / 4), c = (i % (n / 4)) * 4;
@@ -229,12 +228,12 @@ __global__ void __launch_bounds__(256) add_parts_kernel(const float *sums, int s
 }
 inline cb200_status launch_add_parts(const window_split &s, bool pairs, std::int64_t group_begin, std::int64_t group_end, std::int64_t row_end, int n, float *y,
                                      std::int64_t y_ld, float alpha, float beta, const float *bias, int epilogue, float result_scale,
-                                     const unsigned *w_absmax, const unsigned *value_bound, cudaStream_t stream) {
+                                     const unsigned *w_absmax, cudaStream_t stream) {
     const int first = static_cast<int>(group_begin) + whole_groups_in(s, group_begin, group_end), cut = static_cast<int>(group_end) - first;
     if (cut <= 0) return CB200_STATUS_SUCCESS;
     CB200_CUDA_OK(launch_kernel(true, add_parts_kernel, dim3(static_cast<unsigned>(cut), static_cast<unsigned>(n / 8)), 256, 0, stream, s.sums, s.slots,
                                 pairs && s.slots == s.parts ? 1 : 0, s.whole,
-                                first, row_end, n, y, y_ld, alpha, beta, bias, epilogue, result_scale, w_absmax, value_bound));
+                                first, row_end, n, y, y_ld, alpha, beta, bias, epilogue, result_scale, w_absmax));
     count_launch();
     CB200_CUDA_OK(cudaGetLastError());
     return CB200_STATUS_SUCCESS;
@@ -244,7 +243,7 @@ inline window_split split_of_launch(const qcsr_view &x, std::int64_t n, std::int
                                     int sm_count) {
     const window_split_plan plan = qcsr_window_split(x.rows, x.cols, columns, sm_count);
     const std::uint64_t at = device_arena::rounded(used), sums = qcsr_window_split_bytes(x.rows, x.cols, n, columns, sm_count);
-    if (sums == 0u || workspace_bytes < at + sums) return window_split{0x7fffffff, columns == 0 ? 1 : plan.parts, 1, 1, nullptr};
+    if (sums == 0u || workspace_bytes < at + sums) return window_split{0x7fffffff, plan.parts, 1, 1, nullptr};
     return window_split{static_cast<int>(plan.whole), plan.parts, plan.per_unit, plan.slots, reinterpret_cast<float *>(static_cast<unsigned char *>(workspace) + at)};
 }
 

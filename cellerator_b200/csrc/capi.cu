@@ -620,9 +620,9 @@ cb200_status cb200_spmm_prepare(const cb200_spmm_problem *problem, cb200_prepare
             p->workspace_required = p->workspace_bytes;
             const bool both_parts = plan.split && p->blocked.baked && qcsr_blocked_takes_both_parts(problem->n, problem->dense_dtype);
             if (both_parts) p->workspace_bytes = std::max<std::uint64_t>(p->workspace_bytes, qcsr_blocked_workspace_bytes(problem->k, 2 * problem->n));
-            const auto sums_of = [&](std::int64_t columns) {
-                const bool tiles = p->blocked.code_tiles != nullptr || p->blocked.dense_tiles != nullptr;
-                return qcsr_window_split_bytes(problem->m, problem->k, problem->n, tiles ? 0 : columns, p->sm_count);
+            const auto sums_of = [&](std::int64_t columns) -> std::uint64_t {
+                if (p->blocked.code_tiles != nullptr) return 0u; // halves groups by rows
+                return qcsr_window_split_bytes(problem->m, problem->k, problem->n, p->blocked.dense_tiles != nullptr ? -columns : columns, p->sm_count);
             };
             p->workspace_bytes = device_arena::rounded(p->workspace_bytes) + std::max(sums_of(problem->n), both_parts ? sums_of(2 * problem->n) : 0u);
             p->persistent_bytes += p->blocked.bytes;

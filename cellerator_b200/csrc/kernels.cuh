@@ -135,17 +135,17 @@ struct blocked_layout {
     // Scales and offsets are NOT in it: they are applied at launch.
     unsigned char *code_tiles = nullptr;
 };
-// How the tensor kernels over 256-row groups share a matrix out: a CTA takes whole groups, except that the last groups (those
-// from `whole` on, fewer than two per SM) are cut along their windows so that every SM has work to the end.  Sums of parts of a
-// cut group go through the workspace.  The kernel over entry words sums the windows of EVERY group in the same parts, so that a
-// row's bits do not depend on which groups are cut.
+// How the tensor kernels over entry words and over decoded tiles share a matrix out: a CTA takes whole 256-row groups, except
+// that the last groups (those from `whole` on, fewer than two per SM) are cut along their windows so that every SM has work to
+// the end.  Sums of parts of a cut group go through the workspace.  The windows of EVERY group are summed in the same parts, so
+// that a row's bits do not depend on which groups are cut.
 struct window_split_plan {
     std::int64_t whole = 0;
     int parts = 1;
     int per_unit = 1; // of them to a CTA
     int slots = 1;    // sums that go through the workspace, per group: one a part, or one a pair of parts
 };
-// columns: of an accumulator of the kernel over entry words; 0: the kernels over tiles, groups cut into as many parts as pay
+// columns: of an accumulator of the kernel over entry words; negative: the kernel over decoded tiles
 window_split_plan qcsr_window_split(std::int64_t rows, std::int64_t cols, std::int64_t columns, int sm_count);
 std::uint64_t qcsr_window_split_bytes(std::int64_t rows, std::int64_t cols, std::int64_t n, std::int64_t columns, int sm_count);
 bool qcsr_blocked_shape_ok(std::int64_t rows, std::int64_t cols, std::int64_t n, int bits, int dense_dtype);

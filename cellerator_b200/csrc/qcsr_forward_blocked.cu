@@ -1031,11 +1031,14 @@ std::uint64_t qcsr_blocked_workspace_bytes(std::int64_t cols, std::int64_t n) {
     return static_cast<std::uint64_t>(256 + windows * record_bytes(static_cast<int>(n)));
 }
 
-// Parts of a group's windows, `columns` to an accumulator: a function of the genes and N alone, so that every shard of a matrix
+// Parts of a group's windows, `columns` to an accumulator (negative: the kernel over decoded tiles): a function of the genes and N alone, so that every shard of a matrix
 // sums a row the same way.  More parts share a small launch out better (over all group counts below the SMs', 262 windows: three
 // parts take 183 window times on average, six 169, twelve 166) and cost every whole group their turns through the running sum
 // (six parts: two turns, 0.8 % of 303,104 x 33,538 at N = 64).
 static int window_parts(int windows, std::int64_t columns) {
+    // decoded tiles: the running sum is in registers, which hold no 128 columns beside the epilogue (two threads to a row spill, and
+    // 400,000 x 2,000 took 355 instead of 294 us)
+    if (columns < 0) return columns < -64 || windows < 8 ? 1 : windows < 16 ? 2 : windows < 64 ? 4 : 6;
     if (columns > 64) return windows < 8 ? 1 : windows < 64 ? 2 : 3;
     return windows < 8 ? 1 : windows < 16 ? 2 : windows < 128 ? 3 : 6;
 }
@@ -1051,26 +1054,25 @@ window_split_plan qcsr_window_split(std::int64_t rows, std::int64_t cols, std::i
     const int windows = static_cast<int>((cols + kWin - 1) / kWin);
     window_split_plan best;
     best.whole = groups;
-    if (columns != 0) best.parts = window_parts(windows, columns);
-    if (groups == 0 || windows < 2 || (columns != 0 && best.parts == 1)) return best;
+    best.parts = window_parts(windows, columns);
+    if (groups == 0 || best.parts == 1) return best;
     constexpr double kPerUnit = 4.0, kAdding = 3.0, kPerSum = 1.0 / 60.0;
     double best_cost = static_cast<double>((groups + sm_count - 1) / sm_count) * (windows + kPerUnit);
     const int parts = best.parts;
     for (std::int64_t whole = groups / sm_count * sm_count; whole >= 0 && groups - whole < 2 * sm_count; whole -= sm_count) {
         const std::int64_t cut = groups - whole;
-        for (int units = 2; cut > 0 && units <= (columns == 0 ? windows / 2 : parts); ++units) {
-            const int into = columns == 0 ? units : parts, per_unit = (into + units - 1) / units;
-            const bool pairs = columns != 0 && columns <= 64 && per_unit > 1;
-            if ((into + per_unit - 1) / per_unit != units || (pairs && per_unit % 2 != 0)) continue;
-            const int slots = pairs ? (into + 1) / 2 : into;
-            if (cut * slots > (columns == 0 ? 3 : kMostSums) * sm_count) continue;
+        for (int units = 2; cut > 0 && units <= parts; ++units) {
+            const int per_unit = (parts + units - 1) / units;
+            const bool pairs = columns > 0 && columns <= 64 && per_unit > 1;
+            if ((parts + per_unit - 1) / per_unit != units || (pairs && per_unit % 2 != 0)) continue;
+            const int slots = pairs ? (parts + 1) / 2 : parts;
+            if (cut * slots > kMostSums * sm_count) continue;
             const double rounds = static_cast<double>((cut * units + sm_count - 1) / sm_count);
-            const double cost = static_cast<double>(whole / sm_count) * (windows + kPerUnit) + rounds * ((windows * per_unit + into - 1) / into + kPerUnit) + kAdding +
+            const double cost = static_cast<double>(whole / sm_count) * (windows + kPerUnit) + rounds * ((windows * per_unit + parts - 1) / parts + kPerUnit) + kAdding +
                                 kPerSum * static_cast<double>(cut * slots);
             if (cost < 0.99 * best_cost) {
                 best_cost = cost;
                 best.whole = whole;
-                best.parts = into;
                 best.per_unit = per_unit;
                 best.slots = slots;
             }
@@ -1324,7 +1326,7 @@ cb200_status launch_qcsr_forward_blocked(const qcsr_view &x, const dense_args &d
         }
         if (st != CB200_STATUS_SUCCESS) return st;
         st = launch_add_parts(p.split, pass_columns <= 64, p.group_begin, p.group_end, row_end, static_cast<int>(d.n), d.out, d.out_ld, p.alpha, p.beta, p.bias, p.epilogue,
-                              p.result_scale, p.w_absmax, nullptr, stream);
+                              p.result_scale, p.w_absmax, stream);
         if (st != CB200_STATUS_SUCCESS) return st;
     }
     return CB200_STATUS_SUCCESS;

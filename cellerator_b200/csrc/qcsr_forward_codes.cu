@@ -45,6 +45,7 @@
 #include "blocked_tile.cuh"
 
 #include <algorithm>
+#include <type_traits>
 
 namespace cb200 {
 namespace {
@@ -161,6 +162,28 @@ __global__ void __launch_bounds__(256) pack_codes_operands_kernel(const __nv_bfl
     if ((threadIdx.x & 31) == 0) *reinterpret_cast<std::uint32_t *>(half_table + kPairTableBytes) = all_plain ? 1u : 0u;
 }
 
+// How the groups [begin, end) of a launch are shared out: a CTA takes whole groups, or one row sub-block of a group.  A row's sum
+// does not know which (cut along the windows it would; tensor memory has no room for a second set of accumulators beside the
+// operand stages).  Groups of the last round are halved where that leaves no SM with two halves: 1,954 groups on 148 SMs are 13
+// rounds and one of 60 halves (500,000 x 4,000 at N = 128: 448 us, and 442 cut along the windows).
+struct row_units {
+    int begin, whole, count; // the first `whole` units are whole groups, the others halves
+};
+struct row_unit {
+    int group;
+    unsigned subs; // bit s: row sub-block s
+};
+row_units units_of_launch(std::int64_t begin, std::int64_t end, int sm_count) {
+    const int groups = static_cast<int>(end - begin), rest = groups % sm_count;
+    const int cut = 2 * rest <= sm_count ? rest : 0;
+    return row_units{static_cast<int>(begin), groups - cut, groups + cut};
+}
+__device__ __forceinline__ row_unit row_unit_at(const row_units &s, int u) {
+    if (u < s.whole) return row_unit{s.begin + u, 3u};
+    return row_unit{s.begin + s.whole + (u - s.whole) / 2, 1u << ((u - s.whole) & 1)};
+}
+static_assert(kSubBlocks == 2, "a group has two halves");
+
 struct codes_params {
     const unsigned char *stages;  // [group][window][half][16 KB]
     const unsigned char *records; // W windows in operand layout (fp16), record_bytes(N) apart
@@ -168,8 +191,7 @@ struct codes_params {
     float *y;
     std::int64_t y_ld;
     std::int64_t row_end; // rows >= row_end are computed but not written
-    std::int64_t group_begin, group_end;
-    window_split split;
+    row_units units;
     int windows;
     float alpha, beta;
     const float *bias;
@@ -253,8 +275,8 @@ __global__ void __launch_bounds__(kCodesThreads, 1) qcsr_fwd_codes_kernel(const 
     const std::uint32_t tmem_base = *tmem_slot;
     wait_for_previous_launch();
 
-    const int my_units = units_of_cta(p.split, p.group_begin, p.group_end);
-    const auto unit_of = [&](int i) { return unit_at(p.split, p.group_begin, p.group_end, p.windows, static_cast<int>(blockIdx.x) + i * static_cast<int>(gridDim.x)); };
+    const int my_units = (p.units.count - static_cast<int>(blockIdx.x) + static_cast<int>(gridDim.x) - 1) / static_cast<int>(gridDim.x);
+    const auto unit_of = [&](int i) { return row_unit_at(p.units, static_cast<int>(blockIdx.x) + i * static_cast<int>(gridDim.x)); };
 
     if (warp < kEpilogueWarps) {
         // ================= a warp reads its 32 rows (TMEM lane = row within the sub-block) 32 columns at a time and turns
@@ -265,13 +287,16 @@ __global__ void __launch_bounds__(kCodesThreads, 1) qcsr_fwd_codes_kernel(const 
         unsigned char *turn = turn0 + warp * kTurnBytes;
         const int chunk = lane & 7, row_of_lane = lane >> 3; // on the way out: this lane's 4 columns, and its row among the 4 of a store
         // both operands were stored times powers of two (fp16 range): the result is divided by them again
-        const float full_alpha = p.alpha / (operand_scale(__uint_as_float(__ldg(p.w_absmax))) * operand_scale(__uint_as_float(__ldg(p.value_bound))));
+        const float alpha = p.alpha / (operand_scale(__uint_as_float(__ldg(p.w_absmax))) * operand_scale(__uint_as_float(__ldg(p.value_bound))));
         for (int gi = 0; gi < my_units; ++gi) {
-            const window_unit unit = unit_of(gi);
+            const row_unit unit = unit_of(gi);
             const std::int64_t row0 = static_cast<std::int64_t>(unit.group) * kRows + sub * 128 + (warp & 3) * 32;
-            const float alpha = unit.slot >= 0 ? 1.0f : full_alpha;
             if (bar_wait_sleeping(smem_addr(acc_full), static_cast<std::uint32_t>(gi & 1), abort_flag, 400u)) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            if ((unit.subs >> sub & 1u) == 0u) { // the other half's CTA writes these rows
+                if (lane == 0) bar_arrive(smem_addr(acc_empty));
+                continue;
+            }
 #pragma unroll 1
             for (int h = 0; h < NC / 32; ++h) {
                 {
@@ -295,12 +320,6 @@ __global__ void __launch_bounds__(kCodesThreads, 1) qcsr_fwd_codes_kernel(const 
                     t[i] = *reinterpret_cast<const float4 *>(turn + r * 128 + ((chunk ^ (r & 7)) << 4));
                 }
                 __syncwarp(); // the next 32 columns may overwrite the turn buffer
-                if (unit.slot >= 0) { // a part: raw sums, all rows
-                    float *sums = p.split.sums + (static_cast<std::int64_t>(unit.slot) * kRows + sub * 128 + (warp & 3) * 32 + row_of_lane) * NC + h * 32 + 4 * chunk;
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) *reinterpret_cast<float4 *>(sums + 4 * i * NC) = t[i];
-                    continue;
-                }
                 float *out = p.y + (row0 + row_of_lane) * p.y_ld + h * 32 + 4 * chunk;
                 const std::int64_t rows_left = p.row_end - row0 - row_of_lane; // row 4 * i + row_of_lane is written when 4 * i < rows_left
                 if (p.beta != 0.0f) {
@@ -338,10 +357,11 @@ __global__ void __launch_bounds__(kCodesThreads, 1) qcsr_fwd_codes_kernel(const 
         std::uint32_t pa = 0, pb = 0;
         bool dead = false;
         for (int g = 0; g < my_units && !dead; ++g) {
-            const window_unit unit = unit_of(g);
+            const row_unit unit = unit_of(g);
             if (__any_sync(0xffffffffu, bar_wait(smem_addr(acc_empty), static_cast<std::uint32_t>((g & 1) ^ 1), abort_flag))) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            for (int w = unit.w0; w < unit.w1; ++w) {
+            const bool mine = (unit.subs >> sb & 1u) != 0u; // the commits hand over as ever
+            for (int w = 0; w < p.windows; ++w) {
                 // (the warp leaves as one: the election below needs all its lanes)
                 dead = __any_sync(0xffffffffu, bar_wait(smem_addr(b_full + s), pb, abort_flag) || bar_wait(smem_addr(a_full + sa), pa, abort_flag)) != 0;
                 if (dead) break;
@@ -349,13 +369,15 @@ __global__ void __launch_bounds__(kCodesThreads, 1) qcsr_fwd_codes_kernel(const 
                 if (elect_one()) {
                     const std::uint32_t a_col = tmem_base + kOperandCol0 + sa * kOperandCols;
                     const std::uint32_t b_lo = b_lo0 + static_cast<std::uint32_t>((s * WREC) >> 4);
-                    const std::uint32_t fresh = w != unit.w0 ? 1u : 0u; // the unit's first MMAs overwrite the accumulators
+                    const std::uint32_t fresh = w != 0 ? 1u : 0u; // the unit's first MMAs overwrite the accumulators
+                    if (mine) {
 #pragma unroll
-                    for (int kk = 0; kk < kWin / 16; ++kk)
-                        mma_f16_a_in_tmem(tmem_base + sb * NC, a_col + sb * 64 + kk * 8, b_lo + kk * 16, b_hi, IDESC, kk == 0 ? fresh : 1u);
+                        for (int kk = 0; kk < kWin / 16; ++kk)
+                            mma_f16_a_in_tmem(tmem_base + sb * NC, a_col + sb * 64 + kk * 8, b_lo + kk * 16, b_hi, IDESC, kk == 0 ? fresh : 1u);
+                    }
                     mma_commit(smem_addr(a_empty + sa));
                     mma_commit(smem_addr(b_empty + s));
-                    if (w == unit.w1 - 1) mma_commit(smem_addr(acc_full));
+                    if (w == p.windows - 1) mma_commit(smem_addr(acc_full));
                 }
                 __syncwarp();
                 sa ^= 1;
@@ -374,8 +396,7 @@ __global__ void __launch_bounds__(kCodesThreads, 1) qcsr_fwd_codes_kernel(const 
             std::uint32_t pb = 1;
             bool dead = false;
             for (int g = 0; g < my_units && !dead; ++g) {
-                const window_unit unit = unit_of(g);
-                for (int w = unit.w0; w < unit.w1; ++w) {
+                for (int w = 0; w < p.windows; ++w) {
                     if (bar_wait_sleeping(smem_addr(b_empty + s), pb, abort_flag, 200u)) { dead = true; break; }
                     bar_arrive_expect_tx(smem_addr(b_full + s), WREC);
                     bulk_copy_g2s(bstage0 + s * WREC, p.records + static_cast<std::size_t>(w) * REC, WREC, smem_addr(b_full + s));
@@ -393,9 +414,10 @@ __global__ void __launch_bounds__(kCodesThreads, 1) qcsr_fwd_codes_kernel(const 
             std::uint32_t pc = 1;
             bool dead = false;
             for (int g = 0; g < my_units && !dead; ++g) {
-                const window_unit unit = unit_of(g);
-                const unsigned char *src = p.stages + (static_cast<std::size_t>(unit.group) * p.windows + unit.w0) * (kWin / 64) * kCodeStageBytes;
-                for (int h = unit.w0 * (kWin / 64); h < unit.w1 * (kWin / 64); ++h, src += kCodeStageBytes) {
+                const row_unit unit = unit_of(g);
+                // (a half of a group reads whole stages: its rows are four pieces of 2 KB, and a copy costs this thread more than bytes)
+                const unsigned char *src = p.stages + static_cast<std::size_t>(unit.group) * p.windows * (kWin / 64) * kCodeStageBytes;
+                for (int h = 0; h < p.windows * (kWin / 64); ++h, src += kCodeStageBytes) {
                     if (bar_wait_sleeping(smem_addr(c_empty + s), pc, abort_flag, 100u)) { dead = true; break; }
                     bar_arrive_expect_tx(smem_addr(c_full + s), kCodeSlotBytes);
                     bulk_copy_g2s(smem_addr(cstage0 + s * kCodeSlotBytes), src, kCodeStageBytes, smem_addr(c_full + s));
@@ -418,17 +440,14 @@ __global__ void __launch_bounds__(kCodesThreads, 1) qcsr_fwd_codes_kernel(const 
         const __half2 magic = __half2half2(__ushort_as_half(static_cast<unsigned short>(0x6400u))); // 1024: fp16(0x6400 | byte) = 1024 + byte
         const __half2 bias = __float2half2_rn(1024.0f + kPresentBias); // fp16(0x6400 | byte) - bias = the code
         const std::uint32_t lane_base = tmem_base + (static_cast<std::uint32_t>(quarter * 32) << 16) + kOperandCol0 + hf * 32 + pairc * 16;
-        int windows_total = 0;
-        for (int g = 0; g < my_units; ++g) {
-            const window_unit unit = unit_of(g);
-            windows_total += unit.w1 - unit.w0;
-        }
-        int sa = 0;
+        int sa = 0, wq = 0;
         std::uint32_t pa = 1;
-        for (int wq = 0; wq < windows_total; ++wq) {
+        // one window; SUBS: the row sub-blocks of the unit, known to the compiler
+        const auto decode = [&](auto subs) {
+            constexpr unsigned SUBS = decltype(subs)::value;
             const int q = 2 * wq + hf; // this warp's half window in the sequence of code stages
             const int sc = q % SC;
-            if (bar_wait(smem_addr(c_full + sc), static_cast<std::uint32_t>((q / SC) & 1), abort_flag)) break;
+            if (bar_wait(smem_addr(c_full + sc), static_cast<std::uint32_t>((q / SC) & 1), abort_flag)) return false;
             const unsigned char *in = cstage0 + sc * kCodeSlotBytes;
             const bool plain = *reinterpret_cast<const std::uint32_t *>(in + kCodeStageBytes + kPairTableBytes) != 0u; // no masks needed
             uint4 x[2][kSubBlocks];
@@ -436,9 +455,9 @@ __global__ void __launch_bounds__(kCodesThreads, 1) qcsr_fwd_codes_kernel(const 
             for (int c = 0; c < 2; ++c)
 #pragma unroll
                 for (int k = 0; k < kSubBlocks; ++k)
-                    x[c][k] = *reinterpret_cast<const uint4 *>(in + (pairc * 2 + c) * kChunkPlaneBytes + (k * 128 + quarter * 32 + lane) * 16);
+                    if (SUBS >> k & 1u) x[c][k] = *reinterpret_cast<const uint4 *>(in + (pairc * 2 + c) * kChunkPlaneBytes + (k * 128 + quarter * 32 + lane) * 16);
             // a new window: its operand stage must have been read by the MMAs that used it last
-            if (bar_wait(smem_addr(a_empty + sa), pa, abort_flag)) break;
+            if (bar_wait(smem_addr(a_empty + sa), pa, abort_flag)) return false;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
             for (int c = 0; c < 2; ++c) {
@@ -452,6 +471,7 @@ __global__ void __launch_bounds__(kCodesThreads, 1) qcsr_fwd_codes_kernel(const 
                 }
 #pragma unroll
                 for (int k = 0; k < kSubBlocks; ++k) {
+                    if (!(SUBS >> k & 1u)) continue;
                     const std::uint32_t w[4] = {x[c][k].x, x[c][k].y, x[c][k].z, x[c][k].w};
                     std::uint32_t r[8];
                     if (plain) { // two bytes -> fp16 pair 1024 + byte; minus 1264 = the code, or -240 for an empty slot; max(0, code * scale + offset)
@@ -494,6 +514,15 @@ __global__ void __launch_bounds__(kCodesThreads, 1) qcsr_fwd_codes_kernel(const 
             if (lane == 0) bar_arrive(smem_addr(a_full + sa));
             sa ^= 1;
             if (sa == 0) pa ^= 1u;
+            ++wq;
+            return true;
+        };
+        bool alive = true;
+        for (int g = 0; g < my_units && alive; ++g) {
+            const row_unit unit = unit_of(g);
+            for (int w = 0; w < p.windows && alive; ++w)
+                alive = unit.subs == 3u ? decode(std::integral_constant<unsigned, 3u>()) : unit.subs == 1u ? decode(std::integral_constant<unsigned, 1u>())
+                                                                                                          : decode(std::integral_constant<unsigned, 2u>());
         }
         // a wait that ran out can end the loop between a store and its wait: nothing of this warp is in flight when the
         // CTA frees tensor memory
@@ -516,7 +545,7 @@ cb200_status launch_codes(const codes_params &p, int sm_count, cudaStream_t stre
     constexpr std::size_t smem = SB * NC * kWin * 2 + SC * kCodeSlotBytes + kTurnRegionBytes + (2 * SC + 2 * kOperandStages + 2 * SB + 2 + kCodeIssuers) * sizeof(std::uint64_t) + 16;
     static_assert(smem <= 232448, "shared memory budget");
     CB200_CUDA_OK(cudaFuncSetAttribute(qcsr_fwd_codes_kernel<NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-    const unsigned grid = static_cast<unsigned>(std::min(unit_count(p.split, p.group_begin, p.group_end), sm_count));
+    const unsigned grid = static_cast<unsigned>(std::min(p.units.count, sm_count));
     CB200_CUDA_OK(launch_kernel(true, qcsr_fwd_codes_kernel<NC>, grid, kCodesThreads, smem, stream, p));
     count_launch();
     CB200_CUDA_OK(cudaGetLastError());
@@ -603,20 +632,15 @@ cb200_status launch_qcsr_forward_codes(const qcsr_view &x, const dense_args &d, 
     CB200_CUDA_OK(cudaGetLastError());
     codes_params p{};
     p.stages = layout.code_tiles; p.records = records; p.table = table; p.y = d.out; p.y_ld = d.out_ld; p.row_end = row_end;
-    p.group_begin = row_begin / kRows; p.group_end = (row_end + kRows - 1) / kRows; p.windows = layout.windows;
+    p.units = units_of_launch(row_begin / kRows, (row_end + kRows - 1) / kRows, sm_count); p.windows = layout.windows;
     p.alpha = d.alpha; p.beta = d.beta; p.bias = d.bias; p.epilogue = d.epilogue; p.status = status;
     p.w_absmax = w_absmax; p.value_bound = value_bound;
-    p.split = split_of_launch(x, d.n, 0, workspace, workspace_bytes, qcsr_codes_workspace_bytes(x.cols, d.n), sm_count);
     *taken = true;
-    cb200_status st;
     switch (d.n) {
-    case 32: st = launch_codes<32>(p, sm_count, stream); break;
-    case 64: st = launch_codes<64>(p, sm_count, stream); break;
-    default: st = launch_codes<128>(p, sm_count, stream); break;
+    case 32: return launch_codes<32>(p, sm_count, stream);
+    case 64: return launch_codes<64>(p, sm_count, stream);
+    default: return launch_codes<128>(p, sm_count, stream);
     }
-    if (st != CB200_STATUS_SUCCESS) return st;
-    return launch_add_parts(p.split, false, p.group_begin, p.group_end, row_end, static_cast<int>(d.n), d.out, d.out_ld, p.alpha, p.beta, p.bias, p.epilogue,
-                            1.0f, w_absmax, value_bound, stream);
 }
 
 } // namespace cb200

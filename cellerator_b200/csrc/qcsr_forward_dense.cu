@@ -157,60 +157,105 @@ __global__ void __launch_bounds__(kDenseThreads, 1) qcsr_fwd_dense_kernel(const 
     if (warp < kEpilogueWarps) {
         // ================= thread t writes row t of the group: TMEM lane = row within the sub-block =================
         const int sub = tid >> 7;
+        int use = 0; // accumulators used by the CTA
         for (int gi = 0; gi < my_units; ++gi) {
             const window_unit unit = unit_of(gi);
-            const std::uint32_t ab = static_cast<std::uint32_t>(gi & 1);
             const std::int64_t row = static_cast<std::int64_t>(unit.group) * kRows + tid;
-            bar_wait(smem_addr(acc_full + ab), static_cast<std::uint32_t>((gi >> 1) & 1), abort_flag);
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const float alpha = p.alpha * p.result_scale / (p.w_absmax != nullptr ? operand_scale(__uint_as_float(__ldg(p.w_absmax))) : 1.0f);
+            const auto load = [&](std::uint32_t ab, int c, float (&v)[32]) {
+                tmem_ld32(tmem_base + (static_cast<std::uint32_t>((warp & 3) * 32) << 16) + ab * kAccCols + sub * NC + c, v);
+            };
+            const auto wait = [&]() {
+                const std::uint32_t ab = static_cast<std::uint32_t>(use & 1);
+                bar_wait(smem_addr(acc_full + ab), static_cast<std::uint32_t>((use >> 1) & 1), abort_flag);
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                return ab;
+            };
+            const auto release = [&](std::uint32_t ab) {
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) bar_arrive(smem_addr(acc_empty + ab));
+                ++use;
+            };
+            if (unit.slot >= 0) { // parts of a cut group
+                for (int k = 0; k < unit.pieces; ++k) {
+                    const std::uint32_t ab = wait();
+                    float *out = p.split.sums + (static_cast<std::int64_t>(unit.slot + k) * kRows + tid) * NC;
+#pragma unroll 1
+                    for (int c = 0; c < NC; c += 32) {
+                        float v[32];
+                        load(ab, c, v);
 #pragma unroll
-            for (int h = 0; h < NC / 32; ++h) {
-                float v[32];
-                tmem_ld32(tmem_base + (static_cast<std::uint32_t>((warp & 3) * 32) << 16) + ab * kAccCols + sub * NC + h * 32, v);
-                if (unit.slot >= 0) { // raw sums of a part
-                    store_row(p.split.sums + (static_cast<std::int64_t>(unit.slot) * kRows + tid) * NC + h * 32, v, 1.0f, 0.0f, nullptr, h * 32, CB200_EPILOGUE_NONE);
-                } else if (row < p.row_end) {
-                    float *out = p.y + row * p.y_ld + h * 32;
-                    store_row(out, v, p.alpha * p.result_scale / (p.w_absmax != nullptr ? operand_scale(__uint_as_float(__ldg(p.w_absmax))) : 1.0f), p.beta, p.bias, h * 32, p.epilogue);
+                        for (int i = 0; i < 32; i += 4) *reinterpret_cast<float4 *>(out + c + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+                    }
+                    release(ab);
+                }
+            } else if (NC > 64) { // one part
+                const std::uint32_t ab = wait();
+#pragma unroll
+                for (int c = 0; c < NC; c += 32) {
+                    float v[32];
+                    load(ab, c, v);
+                    if (row < p.row_end) store_row(p.y + row * p.y_ld + c, v, alpha, p.beta, p.bias, c, p.epilogue);
+                }
+                release(ab);
+            } else { // the parts of a whole group, added in order in registers
+                constexpr int COLS = NC > 64 ? 32 : NC;
+                float sum[COLS / 32][32];
+                for (int k = 0; k < unit.pieces; ++k) {
+                    const std::uint32_t ab = wait();
+#pragma unroll
+                    for (int h = 0; h < COLS / 32; ++h) {
+                        float v[32];
+                        load(ab, h * 32, v);
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) sum[h][i] = k == 0 ? v[i] : sum[h][i] + v[i];
+                    }
+                    release(ab);
+                }
+                if (row < p.row_end) {
+#pragma unroll
+                    for (int h = 0; h < COLS / 32; ++h) store_row(p.y + row * p.y_ld + h * 32, sum[h], alpha, p.beta, p.bias, h * 32, p.epilogue);
                 }
             }
-            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            __syncwarp();
-            if (lane == 0) bar_arrive(smem_addr(acc_empty + ab));
         }
     } else if (warp == kEpilogueWarps) {
         // ================= MMA issuer =================
         long long qa = 0, qb = 0;
+        int use = 0;
         for (int g = 0; g < my_units; ++g) {
             const window_unit unit = unit_of(g);
-            const std::uint32_t ab = static_cast<std::uint32_t>(g & 1);
-            bar_wait(smem_addr(acc_empty + ab), static_cast<std::uint32_t>(((g >> 1) & 1) ^ 1), abort_flag);
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            for (int w = unit.w0; w < unit.w1; ++w, ++qb) {
-                const int s = static_cast<int>(qb % SB);
-                bar_wait(smem_addr(b_full + s), static_cast<std::uint32_t>((qb / SB) & 1), abort_flag);
-                const std::uint32_t b_tile = bstage0 + s * WREC;
-                for (int half = 0; half < kWin / 64; ++half, ++qa) {
-                    const int sa = static_cast<int>(qa % SA);
-                    bar_wait(smem_addr(a_full + sa), static_cast<std::uint32_t>((qa / SA) & 1), abort_flag);
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    if (elect_one()) {
-                        const std::uint32_t a_stage = smem0 + sa * kDenseStageBytes;
+            for (int k = unit.k0, w = unit.w0; k < unit.k0 + unit.pieces; ++k, ++use) {
+                const std::uint32_t ab = static_cast<std::uint32_t>(use & 1);
+                const int first = w, end = part_begin(p.windows, p.split.parts, k + 1);
+                bar_wait(smem_addr(acc_empty + ab), static_cast<std::uint32_t>(((use >> 1) & 1) ^ 1), abort_flag);
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                for (; w < end; ++w, ++qb) {
+                    const int s = static_cast<int>(qb % SB);
+                    bar_wait(smem_addr(b_full + s), static_cast<std::uint32_t>((qb / SB) & 1), abort_flag);
+                    const std::uint32_t b_tile = bstage0 + s * WREC;
+                    for (int half = 0; half < kWin / 64; ++half, ++qa) {
+                        const int sa = static_cast<int>(qa % SA);
+                        bar_wait(smem_addr(a_full + sa), static_cast<std::uint32_t>((qa / SA) & 1), abort_flag);
+                        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                        if (elect_one()) {
+                            const std::uint32_t a_stage = smem0 + sa * kDenseStageBytes;
 #pragma unroll
-                        for (int kk = 0; kk < 4; ++kk) {
-                            const std::uint64_t db = smem_desc(b_tile + (half * 4 + kk) * 256);
+                            for (int kk = 0; kk < 4; ++kk) {
+                                const std::uint64_t db = smem_desc(b_tile + (half * 4 + kk) * 256);
 #pragma unroll
-                            for (int sb = 0; sb < kSubBlocks; ++sb)
-                                mma_bf16(tmem_base + ab * kAccCols + sb * NC, smem_desc_sw128(a_stage + sb * kHalfBytes + kk * 32), db,
-                                         IDESC, w > unit.w0 || half > 0 || kk > 0);
+                                for (int sb = 0; sb < kSubBlocks; ++sb)
+                                    mma_bf16(tmem_base + ab * kAccCols + sb * NC, smem_desc_sw128(a_stage + sb * kHalfBytes + kk * 32), db,
+                                             IDESC, w > first || half > 0 || kk > 0);
+                            }
+                            mma_commit(smem_addr(a_empty + sa));
+                            if (half == kWin / 64 - 1) {
+                                mma_commit(smem_addr(b_empty + s));
+                                if (w == end - 1) mma_commit(smem_addr(acc_full + ab));
+                            }
                         }
-                        mma_commit(smem_addr(a_empty + sa));
-                        if (half == kWin / 64 - 1) {
-                            mma_commit(smem_addr(b_empty + s));
-                            if (w == unit.w1 - 1) mma_commit(smem_addr(acc_full + ab));
-                        }
+                        __syncwarp();
                     }
-                    __syncwarp();
                 }
             }
         }
@@ -351,7 +396,7 @@ cb200_status launch_qcsr_forward_dense(const qcsr_view &x, const dense_args &d, 
     p.idesc = instr_desc(static_cast<int>(d.n), half);
     p.result_scale = half ? 1.0f / layout.value_scale : 1.0f;
     p.w_absmax = half ? w_absmax : nullptr;
-    p.split = split_of_launch(x, d.n, 0, workspace, workspace_bytes, qcsr_blocked_workspace_bytes(x.cols, d.n), sm_count);
+    p.split = split_of_launch(x, d.n, -d.n, workspace, workspace_bytes, qcsr_blocked_workspace_bytes(x.cols, d.n), sm_count);
     *taken = true;
     cb200_status st;
     switch (d.n) {
@@ -361,7 +406,7 @@ cb200_status launch_qcsr_forward_dense(const qcsr_view &x, const dense_args &d, 
     }
     if (st != CB200_STATUS_SUCCESS) return st;
     return launch_add_parts(p.split, false, p.group_begin, p.group_end, row_end, static_cast<int>(d.n), d.out, d.out_ld, p.alpha, p.beta, p.bias, p.epilogue,
-                            p.result_scale, p.w_absmax, nullptr, stream);
+                            p.result_scale, p.w_absmax, stream);
 }
 
 } // namespace cb200

@@ -57,7 +57,10 @@ def test_cut_groups(cuda_device, oracle, monkeypatch, schedule, bits, n, dtype, 
     ("tensor_blocked", 8, 32, torch.bfloat16, capi.DTYPE_BF16), ("tensor_blocked", 8, 64, torch.bfloat16, capi.DTYPE_BF16),
     ("tensor_blocked", 4, 128, torch.bfloat16, capi.DTYPE_BF16), ("tensor_blocked", 8, 64, torch.bfloat16, capi.DTYPE_F32),
     ("tensor_blocked", 8, 32, torch.float32, capi.DTYPE_F32), ("tensor_blocked", 8, 64, torch.float32, capi.DTYPE_F32),
-    ("tensor_blocked", 8, 128, torch.float32, capi.DTYPE_F32)])
+    ("tensor_blocked", 8, 128, torch.float32, capi.DTYPE_F32), ("tensor_dense", 8, 32, torch.bfloat16, capi.DTYPE_BF16),
+    ("tensor_dense", 4, 64, torch.bfloat16, capi.DTYPE_BF16), ("tensor_dense", 8, 128, torch.bfloat16, capi.DTYPE_BF16),
+    ("tensor_codes", 4, 32, torch.bfloat16, capi.DTYPE_BF16), ("tensor_codes", 4, 64, torch.bfloat16, capi.DTYPE_BF16),
+    ("tensor_codes", 4, 128, torch.bfloat16, capi.DTYPE_BF16)])
 @pytest.mark.parametrize("rows,windows,density", [(256 * 6 + 1, 7, 40), (256 * 6 + 1, 9, 300), (700, 17, 40), (256 * 150 - 7, 9, 12), (1800, 33, 1200),
                                                   (256 * 13, 64, 60), (256 * 47 + 3, 129, 15), (300, 200, 4000)])
 def test_a_rows_bits_follow_from_its_entries(cuda_device, oracle, monkeypatch, schedule, bits, n, dtype, multiply, rows, windows, density):
@@ -74,8 +77,8 @@ def test_a_rows_bits_follow_from_its_entries(cuda_device, oracle, monkeypatch, s
         op = ops.PreparedSpmm(capi.PROJECTION_CSR, c["rows"], cols, n, x.nnz, bits, 1, dtype, cuda_device, host_row_ptr=x.host_row_ptr,
                               multiply=multiply, device_matrix=x)
         assert op.schedule.startswith(schedule)
-        # the status block and the records of W, hi and lo of an fp32 W side by side
-        records = 256 + windows * 128 * (2 * n * (2 if dtype == torch.float32 and n <= 64 else 1) + 8)
+        # the status block and the records of W, hi and lo of an fp32 W side by side; behind them the tables of the code tiles
+        records = 256 + windows * 128 * (2 * n * (2 if dtype == torch.float32 and n <= 64 else 1) + 8) + (windows * 544 if schedule == "tensor_codes" else 0)
         if uncut and op.workspace_bytes > records:
             op.workspace_bytes = records
         y = op.run(x, w, torch.empty(c["rows"], n, device=cuda_device))
