@@ -244,6 +244,9 @@ cb200_status launch_qcsr_transpose_gather(const qcsr_view &x, const dense_args &
                                           std::int64_t row_end, const gene_major_layout &layout, void *workspace,
                                           std::uint64_t workspace_bytes, int sm_count, cudaStream_t stream);
 
+// Polls a bounded wait makes under the test hook (cb200_test_arm_wait_timeout); 0: not armed.
+int test_poll_limit();
+
 struct qbell_view {
     std::int64_t rows, cols;
     int block_size, ell_cols;

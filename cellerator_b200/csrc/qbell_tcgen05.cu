@@ -37,7 +37,8 @@
 // a ring of single blocks and a commit per block the issuing threads were the bound (218 us; 331 before they were elected,
 // see elect_one).
 // Empty blocks (index 0xffffffff) are skipped; genes >= cols and cells past the last row decode to 0.  Every barrier wait is
-// bounded; on a time-out a status word is set, every role ends, and the kernel frees its TMEM.
+// bounded; on a time-out a status word is set, every role ends, the copies and MMAs in flight are waited for, and the kernel
+// frees its TMEM.
 #include "kernels.cuh"
 #include "operand_scaling.cuh"
 #include "sm100_primitives.cuh"
@@ -90,6 +91,7 @@ struct tc_params {
     const float *bias;
     int epilogue;
     int *status;
+    int poll_limit; // test hook: polls the MMA warps' waits for operands make
 };
 
 // K-major, no swizzle: core matrices of 8 rows x 16 bytes; LBO (between the two core matrices a
@@ -180,28 +182,33 @@ __device__ __forceinline__ block_row make_block_row(std::uint32_t column) {
     return r;
 }
 // the same answer in every lane: a warp that gives up leaves its loops as one
-__device__ __forceinline__ bool warp_wait(std::uint64_t *bar, int parity, volatile int *abort_flag) {
-    return __any_sync(0xffffffffu, bar_wait(smem_addr(bar), static_cast<std::uint32_t>(parity & 1), abort_flag)) != 0;
+__device__ __forceinline__ bool warp_wait(std::uint64_t *bar, int parity, volatile int *abort_flag, int limit = kPollLimit) {
+    return __any_sync(0xffffffffu, bar_wait(smem_addr(bar), static_cast<std::uint32_t>(parity & 1), abort_flag, limit)) != 0;
 }
 __device__ __forceinline__ bool warp_wait_sleeping(std::uint64_t *bar, int parity, volatile int *abort_flag, unsigned ns) {
     return __any_sync(0xffffffffu, bar_wait_sleeping(smem_addr(bar), static_cast<std::uint32_t>(parity & 1), abort_flag, ns)) != 0;
 }
 
-template<int BITS, int H /* N / 128 */>
+// TEST_HOOK: what cb200_test_arm_wait_timeout selects.  Decode group 0 hands nothing over, so that the MMA warps' waits run out
+// (after p.poll_limit polls) with copies in flight whose barriers lack arrivals; the rest is common code.
+template<int BITS, int H /* N / 128 */, bool TEST_HOOK>
 __global__ void __launch_bounds__(threads_of(H), 1) qbell_tcgen05_kernel(const tc_params p) {
     constexpr int kATileBytes = a_tile_bytes(H), kStageBytes = stage_bytes(H), kStages = stages_of(H);
     static_assert(kStages % kLoaders == 0, "a loader's pairs keep to its stages");
     constexpr int kTmemCols = 2 * H * 32; // two accumulator buffers
     extern __shared__ __align__(1024) unsigned char smem[];
-    // [kStages][A][A][B][B] | barriers | tmem base | flags
+    // [kStages][A][A][B][B] | barriers | tmem base | flags | what an abort drains
     std::uint64_t *bars = reinterpret_cast<std::uint64_t *>(smem + kStages * kStageBytes);
     std::uint64_t *full = bars;                      // [kStages] loader (with the copies' bytes) and the warps of a decode group -> MMA
     std::uint64_t *empty = full + kStages;           // [kStages] MMA commits -> loader and decode group
     std::uint64_t *acc_full = empty + kStages;       // [2]       MMA commits -> epilogue
     std::uint64_t *acc_empty = acc_full + 2;         // [2]       epilogue -> MMA (one arrival per warp)
-    std::uint32_t *tmem_slot = reinterpret_cast<std::uint32_t *>(acc_empty + 2);
+    std::uint64_t *mma_drain = acc_empty + 2;        // [H]       an MMA warp's own, used once, after an abort
+    std::uint32_t *tmem_slot = reinterpret_cast<std::uint32_t *>(mma_drain + H);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
     volatile int *row_has_blocks = reinterpret_cast<volatile int *>(tmem_slot + 2); // [2] per accumulator buffer
+    volatile int *issued = reinterpret_cast<volatile int *>(tmem_slot + 4); // [kStages] pair last copied into the stage, x kGroups + its decode group; -1
+    volatile int *handed_over = issued + kStages;                          // [kDecodeWarps] last pair the warp handed over, once it has ended
 
     const int tid = threadIdx.x, warp = warp_of_block(), lane = tid & 31;
     const std::uint32_t smem0 = smem_addr(smem);
@@ -210,7 +217,9 @@ __global__ void __launch_bounds__(threads_of(H), 1) qbell_tcgen05_kernel(const t
         for (int s = 0; s < kStages; ++s) {
             bar_init(smem_addr(full + s), 1 + 4);
             bar_init(smem_addr(empty + s), H);
+            issued[s] = -1;
         }
+        for (int h = 0; h < H; ++h) bar_init(smem_addr(mma_drain + h), 1);
         for (int b = 0; b < 2; ++b) {
             bar_init(smem_addr(acc_full + b), H);
             bar_init(smem_addr(acc_empty + b), kEpilogueWarps);
@@ -313,6 +322,7 @@ __global__ void __launch_bounds__(threads_of(H), 1) qbell_tcgen05_kernel(const t
 #pragma unroll
         for (int r = 0; r < kGroupPairs; ++r) fetch(first, column, r);
         int item0 = 0; // pairs of the CTA before this block row
+        int last = -1; // pair last handed over
         bool dead = false;
         for (std::int64_t br = first; br < p.block_row_end && !dead; br += step) {
             const block_row blocks = make_block_row(column);
@@ -365,13 +375,16 @@ __global__ void __launch_bounds__(threads_of(H), 1) qbell_tcgen05_kernel(const t
                     }
                     fence_async_proxy(); // written with ordinary stores, read by the MMAs
                     __syncwarp();
+                    if (TEST_HOOK && group == 0) continue;
                     if (lane == 0) bar_arrive(smem_addr(full + stage));
+                    last = item;
                 }
             }
 #pragma unroll
             for (int r = 0; r < kGroupPairs; ++r) fetch(br + step, column, r);
             item0 += __popc(blocks.pairs);
         }
+        if (lane == 0) handed_over[warp - kEpilogueWarps] = last;
     } else if (warp < kEpilogueWarps + kDecodeWarps + H) {
         // ================= MMA issuers: warp h issues the MMAs of output columns [128 h, 128 h + 128) =================
         const int h = warp - kEpilogueWarps - kDecodeWarps;
@@ -390,7 +403,7 @@ __global__ void __launch_bounds__(threads_of(H), 1) qbell_tcgen05_kernel(const t
             std::uint32_t accumulate = 0; // the block row's first MMA overwrites the accumulators
             for (unsigned todo = blocks.pairs; todo != 0u; todo &= todo - 1u) {
                 const unsigned present = blocks.blocks >> (__ffs(static_cast<int>(todo)) - 1);
-                dead = warp_wait(full + stage, phase, abort_flag);
+                dead = warp_wait(full + stage, phase, abort_flag, TEST_HOOK ? p.poll_limit : kPollLimit);
                 if (dead) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 if (elect_one()) {
@@ -417,7 +430,7 @@ __global__ void __launch_bounds__(threads_of(H), 1) qbell_tcgen05_kernel(const t
         // ================= loaders: a block's slice of W^T is one contiguous copy, already in operand layout; loader l takes the
         // pairs whose number in the CTA's walk is l modulo kLoaders =================
         const int loader = warp - kEpilogueWarps - kDecodeWarps - H;
-        int number = 0, stage = loader, phase = 1, issued = 0;
+        int number = 0, stage = loader, phase = 1;
         bool dead = false; // the elected lane: a wait was given up
         std::uint32_t column = load_column(p, first, lane);
         for (std::int64_t br = first; br < p.block_row_end; br += step) {
@@ -432,26 +445,44 @@ __global__ void __launch_bounds__(threads_of(H), 1) qbell_tcgen05_kernel(const t
                 if (elect_one() && !dead) {
                     dead = bar_wait(smem_addr(empty + stage), static_cast<std::uint32_t>(phase), abort_flag);
                     if (!dead) { // no new copies once a wait of the CTA has run out
+                        issued[stage] = number * kGroups + (even >> 1) % kGroups;
                         bar_arrive_expect_tx(smem_addr(full + stage), ((bc[0] != 0xffffffffu) + (bc[1] != 0xffffffffu)) * kATileBytes);
 #pragma unroll
                         for (int t = 0; t < 2; ++t)
                             if (bc[t] != 0xffffffffu)
                                 bulk_copy_g2s(smem0 + stage * kStageBytes + t * kATileBytes, p.wt + static_cast<std::int64_t>(bc[t]) * (H * 128 * 32), kATileBytes,
                                               smem_addr(full + stage));
-                        ++issued;
                     }
                 }
                 stage += kLoaders;
                 if (stage >= kStages) { stage = loader; phase ^= 1; }
             }
         }
-        // The copies still in flight land before the CTA gives up its shared memory.  Their barriers may lack the decode
-        // group's arrivals, so there is nothing to wait on; a copy takes microseconds, the bound of a wait was milliseconds.
-        if (dead) __nanosleep(1000000u);
     }
 
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    if (*abort_flag != 0) {
+        // Every role has ended.  The copies and MMAs still in flight finish before the CTA gives up its shared and tensor memory.
+        // A stage's barrier may lack arrivals of the decode group that owns its pair: the loader makes up for them.
+        if (warp >= kEpilogueWarps + kDecodeWarps + H) {
+            if (elect_one()) {
+                for (int stage = warp - kEpilogueWarps - kDecodeWarps - H; stage < kStages; stage += kLoaders) {
+                    if (issued[stage] < 0) continue;
+                    const int item = issued[stage] / kGroups, group = issued[stage] % kGroups;
+                    for (int w = 0; w < 4; ++w)
+                        if (handed_over[group * 4 + w] < item) bar_arrive(smem_addr(full + stage));
+                    bar_wait_drain(smem_addr(full + stage), static_cast<std::uint32_t>((item / kStages) & 1));
+                }
+            }
+        } else if (warp >= kEpilogueWarps + kDecodeWarps) {
+            if (elect_one()) {
+                mma_commit(smem_addr(mma_drain + (warp - kEpilogueWarps - kDecodeWarps)));
+                bar_wait_drain(smem_addr(mma_drain + (warp - kEpilogueWarps - kDecodeWarps)), 0u);
+            }
+        }
+        __syncthreads();
+    }
     if (warp == 0) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemCols) : "memory");
@@ -459,14 +490,14 @@ __global__ void __launch_bounds__(threads_of(H), 1) qbell_tcgen05_kernel(const t
     if (tid == 0 && *abort_flag != 0 && p.status != nullptr) atomicExch(p.status, 1);
 }
 
-template<int BITS, int H>
+template<int BITS, int H, bool TEST_HOOK = false>
 cb200_status launch(const tc_params &p, int sm_count, cudaStream_t stream) {
-    constexpr std::size_t smem = stages_of(H) * stage_bytes(H) + (2 * stages_of(H) + 4) * sizeof(std::uint64_t) + 32;
+    constexpr std::size_t smem = stages_of(H) * stage_bytes(H) + (2 * stages_of(H) + 4 + H) * sizeof(std::uint64_t) + (4 + stages_of(H) + kDecodeWarps) * sizeof(int);
     static_assert(smem <= 232448, "shared memory budget");
-    CB200_CUDA_OK(cudaFuncSetAttribute(qbell_tcgen05_kernel<BITS, H>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+    CB200_CUDA_OK(cudaFuncSetAttribute(qbell_tcgen05_kernel<BITS, H, TEST_HOOK>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
     const std::int64_t block_rows = p.block_row_end - p.block_row_begin;
     const unsigned grid = static_cast<unsigned>(std::min<std::int64_t>(block_rows, sm_count));
-    CB200_CUDA_OK(launch_kernel(true, qbell_tcgen05_kernel<BITS, H>, grid, threads_of(H), smem, stream, p));
+    CB200_CUDA_OK(launch_kernel(true, qbell_tcgen05_kernel<BITS, H, TEST_HOOK>, grid, threads_of(H), smem, stream, p));
     count_launch();
     CB200_CUDA_OK(cudaGetLastError());
     return CB200_STATUS_SUCCESS;
@@ -514,6 +545,10 @@ cb200_status launch_qbell_tcgen05(const qbell_view &x, const dense_args &d, std:
     p.row_begin = row_begin; p.row_end = row_end;
     p.n = static_cast<int>(d.n); p.policy = x.policy; p.alpha = d.alpha; p.beta = d.beta; p.bias = d.bias; p.epilogue = d.epilogue; p.status = status;
     *taken = true;
+    if (x.bits == 8 && d.n == 256 && test_poll_limit() != 0) {
+        p.poll_limit = test_poll_limit();
+        return launch<8, 2, true>(p, sm_count, stream);
+    }
     if (x.bits == 8) return d.n == 256 ? launch<8, 2>(p, sm_count, stream) : launch<8, 1>(p, sm_count, stream);
     return d.n == 256 ? launch<4, 2>(p, sm_count, stream) : launch<4, 1>(p, sm_count, stream);
 }

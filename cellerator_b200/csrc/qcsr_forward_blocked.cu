@@ -1025,6 +1025,7 @@ cb200_status launch_blocked2(const blocked_params &p, int sm_count, cudaStream_t
 }
 } // namespace
 
+int test_poll_limit() { return g_test_poll_limit.load(std::memory_order_relaxed); }
 bool qcsr_blocked_takes_both_parts(std::int64_t n, int dense_dtype) { return dense_dtype == CB200_DTYPE_F32 && n <= 64; }
 std::uint64_t qcsr_blocked_workspace_bytes(std::int64_t cols, std::int64_t n) {
     const std::int64_t windows = (cols + kWin - 1) / kWin;
@@ -1271,7 +1272,7 @@ cb200_status launch_qcsr_forward_blocked(const qcsr_view &x, const dense_args &d
     p.w_absmax = half ? w_absmax : nullptr;
     p.poll_limit = kPollLimit;
     p.withhold_w = 0;
-    if (const int armed = g_test_poll_limit.load(std::memory_order_relaxed)) { // test hook: see cb200_test_arm_wait_timeout
+    if (const int armed = test_poll_limit()) { // test hook: see cb200_test_arm_wait_timeout
         p.poll_limit = armed;
         p.withhold_w = 1;
     }

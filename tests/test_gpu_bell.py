@@ -168,3 +168,27 @@ def test_bell_tensor_kernel_keeps_its_accuracy_over_magnitudes(cuda_device, orac
         assert torch.all(y == 0.0)
     else:
         assert_bell_close(y.cpu().numpy(), ref, l1, float(np.abs(w_host).max()), bf16_multiply=True)
+
+
+@pytest.mark.parametrize("rows,ell_blocks", [(32, 16), (32 * 300, 16), (32 * 600 + 5, 7), (32 * 4, 1)])
+def test_bounded_wait_path(cuda_device, rows, ell_blocks):
+    """Operands that are never handed over, with copies in flight whose barriers lack arrivals: the launch ends with its status
+    word set, the copies and MMAs drained, and the next launch on the stream has the right bits."""
+    L = capi.lib()
+    x = synth.make_qbell_device(rows, 2048, 32, ell_blocks, 0.6, 8, cuda_device, seed=3)
+    w = (torch.randn(2048, 256, device=cuda_device) * 0.02).to(torch.bfloat16)
+    op = ops.PreparedSpmm(capi.PROJECTION_BLOCKED_ELL, rows, 2048, 256, rows * x.ell_cols, x.bits, x.policy, torch.bfloat16, cuda_device)
+    assert op.schedule == "tcgen05_block_rows"
+    good = op.run(x, w, torch.empty(rows, 256, device=cuda_device)).clone()
+    assert op.status() == 0
+    for _ in range(3):
+        L.cb200_test_arm_wait_timeout(4096)
+        try:
+            op.run(x, w, torch.empty(rows, 256, device=cuda_device))
+        finally:
+            L.cb200_test_disarm_wait_timeout()
+        with pytest.raises(capi.Cb200Error) as e:
+            op.status()
+        assert e.value.status == capi.DEVICE_WAIT_TIMEOUT
+        assert torch.equal(op.run(x, w, torch.full((rows, 256), float("nan"), device=cuda_device)), good) and op.status() == 0
+    op.close()
