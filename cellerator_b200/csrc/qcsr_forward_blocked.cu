@@ -418,10 +418,12 @@ __global__ void __launch_bounds__(kThreads, 1) qcsr_fwd_blocked_kernel(const blo
     std::uint64_t *c_empty = c_full + CS;    // [CS] scatter warps -> loader (one arrival per warp)
     std::uint64_t *acc_full = c_empty + CS;            // [SETS] MMA commit -> scatter warps
     std::uint64_t *acc_empty = acc_full + SETS;        // [SETS] scatter warps -> MMA (one arrival per warp)
-    volatile int *chunk_meta = reinterpret_cast<volatile int *>(acc_empty + SETS); // [CS] (entries << 1) | last chunk of its window
+    std::uint64_t *mma_drain = acc_empty + SETS;       // the MMA warp's own, used once, after an abort
+    volatile int *chunk_meta = reinterpret_cast<volatile int *>(mma_drain + 1); // [CS] (entries << 1) | last chunk of its window
     std::uint32_t *tmem_slot = reinterpret_cast<std::uint32_t *>(const_cast<int *>(chunk_meta) + CS + 1);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
     unsigned char *scratch_slot = reinterpret_cast<unsigned char *>(tmem_slot + 2);
+    volatile int *fills = reinterpret_cast<volatile int *>(tmem_slot + 3); // [2] of the W ring and of the chunk ring, once their loaders have ended
 
     const int tid = threadIdx.x, warp = warp_of_block(), lane = tid & 31;
     const std::uint32_t smem0 = smem_addr(smem);
@@ -445,6 +447,7 @@ __global__ void __launch_bounds__(kThreads, 1) qcsr_fwd_blocked_kernel(const blo
             bar_init(smem_addr(acc_full + k), 1);
             bar_init(smem_addr(acc_empty + k), kEpilogueWarps);
         }
+        bar_init(smem_addr(mma_drain), 1);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -595,20 +598,26 @@ __global__ void __launch_bounds__(kThreads, 1) qcsr_fwd_blocked_kernel(const blo
         const int role = warp - kProducerWarps - 1; // 0: W slices, 1: entry chunks
         if (role == 0) {
             if (elect_one()) {
-                int s = 0;
+                int s = 0, issued = 0;
                 std::uint32_t phase = 1;
-                for (int g = 0; g < my_units; ++g) {
+                // the test hook: no copies, and the wait for the first of them runs out
+                bool dead = p.withhold_w != 0 && bar_wait(smem_addr(w_full), 0u, abort_flag, p.poll_limit);
+                for (int g = 0; g < my_units && !dead; ++g) {
                     const window_unit unit = unit_of(g);
                     for (int w = unit.w0; w < unit.w1; ++w) {
-                        bar_wait(smem_addr(w_empty + s), phase, abort_flag);
+                        dead = bar_wait(smem_addr(w_empty + s), phase, abort_flag);
+                        if (dead) break; // no new copies once a wait of the CTA has run out
+                        ++issued;
                         bar_arrive_expect_tx(smem_addr(w_full + s), REC);
                         bulk_copy_g2s(wstage0 + s * REC, p.records + static_cast<std::size_t>(w) * p.record_stride, REC, smem_addr(w_full + s));
                         if (++s == STAGES) { s = 0; phase ^= 1u; }
                     }
                 }
+                fills[0] = issued;
             }
         } else {
-            int cs = 0;
+            int cs = 0, issued = 0;
+            bool dead = false; // the elected lane: a wait was given up, no copy is issued any more (the loops run out empty)
             std::uint32_t phase = 1;
             for (int gi = 0; gi < my_units; ++gi) {
                 const window_unit unit = unit_of(gi);
@@ -622,8 +631,9 @@ __global__ void __launch_bounds__(kThreads, 1) qcsr_fwd_blocked_kernel(const blo
                         std::int64_t at = lo;
                         do {
                             const int count = static_cast<int>(min(static_cast<std::int64_t>(kChunkEntries), hi - at));
-                            if (elect_one()) {
-                                bar_wait(smem_addr(c_empty + cs), phase, abort_flag);
+                            if (elect_one() && !dead) dead = bar_wait(smem_addr(c_empty + cs), phase, abort_flag);
+                            if (elect_one() && !dead) {
+                                ++issued;
                                 chunk_meta[cs] = (count << 1) | (at + count >= hi ? 1 : 0);
                                 if (count > 0) {
                                     bar_arrive_expect_tx(smem_addr(c_full + cs), static_cast<std::uint32_t>(count) * 4u);
@@ -639,11 +649,20 @@ __global__ void __launch_bounds__(kThreads, 1) qcsr_fwd_blocked_kernel(const blo
                     }
                 }
             }
+            if (elect_one()) fills[1] = issued;
         }
     }
 
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    if (*abort_flag != 0) { // every role has ended: what is in flight finishes before the CTA gives up its shared and tensor memory
+        if (warp == kProducerWarps) {
+            if (elect_one()) drain_mmas(smem_addr(mma_drain));
+        } else if (warp > kProducerWarps) {
+            if (elect_one()) drain_fills(smem_addr(warp == kProducerWarps + 1 ? w_full : c_full), warp == kProducerWarps + 1 ? STAGES : CS, fills[warp - kProducerWarps - 1]);
+        }
+        __syncthreads();
+    }
     if (warp == 0) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemCols) : "memory");
@@ -653,7 +672,7 @@ __global__ void __launch_bounds__(kThreads, 1) qcsr_fwd_blocked_kernel(const blo
 
 template<int NC, int CS> constexpr std::size_t blocked_smem_bytes() {
     return 2 * kABufBytes + w_stages(NC, CS) * record_bytes(NC) + CS * kChunkBytes + kRows * 4 +
-           (4 + 2 * w_stages(NC, CS) + 2 * CS + 2 * most_sets(NC)) * sizeof(std::uint64_t) + (CS + 1) * 4 + 16;
+           (5 + 2 * w_stages(NC, CS) + 2 * CS + 2 * most_sets(NC)) * sizeof(std::uint64_t) + (CS + 1) * 4 + 24;
 }
 
 template<int NC, int N, int CS, bool BAKED>

@@ -93,6 +93,7 @@ struct dense_params {
     const float *bias;
     int epilogue;
     int *status;
+    int poll_limit; // test hook (cb200_test_arm_wait_timeout): the W loader issues no copies and gives up after so many polls; 0: none
     std::uint32_t idesc;       // bf16 or fp16 operands
     float result_scale;        // fp16 tiles: 1 / (the power of two the values were stored times)
     const unsigned *w_absmax;  // fp16 operands: largest |W| of this launch as float bits; else null
@@ -117,8 +118,10 @@ __global__ void __launch_bounds__(kDenseThreads, 1) qcsr_fwd_dense_kernel(const 
     std::uint64_t *b_empty = b_full + SB;      // [SB] MMA commit -> W loader
     std::uint64_t *acc_full = b_empty + SB;    // [2]  MMA commit -> epilogue warps
     std::uint64_t *acc_empty = acc_full + 2;   // [2]  epilogue warps -> MMA (one arrival per warp)
-    std::uint32_t *tmem_slot = reinterpret_cast<std::uint32_t *>(acc_empty + 2);
+    std::uint64_t *mma_drain = acc_empty + 2;  // the MMA warp's own, used once, after an abort
+    std::uint32_t *tmem_slot = reinterpret_cast<std::uint32_t *>(mma_drain + 1);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
+    volatile int *fills = reinterpret_cast<volatile int *>(tmem_slot + 2); // [1 + kDenseALoaders] of the W ring, and behind each A loader's last, once they have ended
 
     const int tid = threadIdx.x, warp = warp_of_block(), lane = tid & 31;
     const std::uint32_t smem0 = smem_addr(smem);
@@ -137,6 +140,7 @@ __global__ void __launch_bounds__(kDenseThreads, 1) qcsr_fwd_dense_kernel(const 
             bar_init(smem_addr(acc_full + b), 1);
             bar_init(smem_addr(acc_empty + b), kEpilogueWarps);
         }
+        bar_init(smem_addr(mma_drain), 1);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -262,37 +266,54 @@ __global__ void __launch_bounds__(kDenseThreads, 1) qcsr_fwd_dense_kernel(const 
     } else if (warp == kEpilogueWarps + 1) {
         // ================= W loader =================
         if (elect_one()) {
-            long long q = 0;
-            for (int g = 0; g < my_units; ++g) {
+            int q = 0;
+            bool dead = p.poll_limit != 0 && bar_wait(smem_addr(b_full), 0u, abort_flag, p.poll_limit);
+            for (int g = 0; g < my_units && !dead; ++g) {
                 const window_unit unit = unit_of(g);
                 for (int w = unit.w0; w < unit.w1; ++w, ++q) {
-                    const int s = static_cast<int>(q % SB);
-                    bar_wait(smem_addr(b_empty + s), static_cast<std::uint32_t>(((q / SB) & 1) ^ 1), abort_flag);
+                    const int s = q % SB;
+                    dead = bar_wait(smem_addr(b_empty + s), static_cast<std::uint32_t>(((q / SB) & 1) ^ 1), abort_flag);
+                    if (dead) break; // no new copies once a wait of the CTA has run out
                     bar_arrive_expect_tx(smem_addr(b_full + s), WREC);
                     bulk_copy_g2s(bstage0 + s * WREC, p.records + static_cast<std::size_t>(w) * REC, WREC, smem_addr(b_full + s));
                 }
             }
+            fills[0] = q;
         }
     } else {
         // ================= A loaders: half-stages in turn =================
         if (elect_one()) {
-            long long q = 0; // half-stages of this CTA; every loader counts all of them and issues its own
-            for (int g = 0; g < my_units; ++g) {
+            int q = 0, issued = 0; // half-stages of this CTA: every loader counts all of them and issues its own; one behind its last
+            bool dead = false;
+            for (int g = 0; g < my_units && !dead; ++g) {
                 const window_unit unit = unit_of(g);
                 const unsigned char *src = p.tiles + (static_cast<std::size_t>(unit.group) * p.windows + unit.w0) * (kWin / 64) * kDenseStageBytes;
                 for (int h = 0; h < (unit.w1 - unit.w0) * (kWin / 64); ++h, ++q, src += kDenseStageBytes) {
                     if (q % kDenseALoaders != warp - kEpilogueWarps - 2) continue;
-                    const int s = static_cast<int>(q % SA);
-                    bar_wait(smem_addr(a_empty + s), static_cast<std::uint32_t>(((q / SA) & 1) ^ 1), abort_flag);
+                    const int s = q % SA;
+                    dead = bar_wait(smem_addr(a_empty + s), static_cast<std::uint32_t>(((q / SA) & 1) ^ 1), abort_flag);
+                    if (dead) break;
+                    issued = q + 1;
                     bar_arrive_expect_tx(smem_addr(a_full + s), kDenseStageBytes);
                     bulk_copy_g2s(smem0 + s * kDenseStageBytes, src, kDenseStageBytes, smem_addr(a_full + s));
                 }
             }
+            fills[warp - kEpilogueWarps - 1] = issued;
         }
     }
 
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    if (*abort_flag != 0) { // every role has ended: what is in flight finishes before the CTA gives up its shared and tensor memory
+        if (warp == kEpilogueWarps) {
+            if (elect_one()) drain_mmas(smem_addr(mma_drain));
+        } else if (warp == kEpilogueWarps + 1) {
+            if (elect_one()) drain_fills(smem_addr(b_full), SB, fills[0]);
+        } else if (warp > kEpilogueWarps) {
+            if (elect_one()) drain_fills(smem_addr(a_full), SA, fills[warp - kEpilogueWarps - 1], kDenseALoaders);
+        }
+        __syncthreads();
+    }
     if (warp == 0) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemCols) : "memory");
@@ -303,7 +324,7 @@ __global__ void __launch_bounds__(kDenseThreads, 1) qcsr_fwd_dense_kernel(const 
 template<int NC>
 cb200_status launch_dense(const dense_params &p, int sm_count, cudaStream_t stream) {
     constexpr std::size_t smem = dense_a_stages(NC) * kDenseStageBytes + kDenseBStages * NC * kWin * 2 +
-                                 (2 * dense_a_stages(NC) + 2 * kDenseBStages + 4) * sizeof(std::uint64_t) + 16;
+                                 (2 * dense_a_stages(NC) + 2 * kDenseBStages + 5) * sizeof(std::uint64_t) + (3 + kDenseALoaders) * sizeof(int);
     static_assert(smem <= 232448, "shared memory budget");
     CB200_CUDA_OK(cudaFuncSetAttribute(qcsr_fwd_dense_kernel<NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
     const unsigned grid = static_cast<unsigned>(std::min(unit_count(p.split, p.group_begin, p.group_end), sm_count));
@@ -392,7 +413,7 @@ cb200_status launch_qcsr_forward_dense(const qcsr_view &x, const dense_args &d, 
     dense_params p{};
     p.tiles = layout.dense_tiles; p.records = records; p.y = d.out; p.y_ld = d.out_ld; p.row_end = row_end;
     p.group_begin = row_begin / kRows; p.group_end = (row_end + kRows - 1) / kRows; p.windows = layout.windows;
-    p.alpha = d.alpha; p.beta = d.beta; p.bias = d.bias; p.epilogue = d.epilogue; p.status = status;
+    p.alpha = d.alpha; p.beta = d.beta; p.bias = d.bias; p.epilogue = d.epilogue; p.status = status; p.poll_limit = test_poll_limit();
     p.idesc = instr_desc(static_cast<int>(d.n), half);
     p.result_scale = half ? 1.0f / layout.value_scale : 1.0f;
     p.w_absmax = half ? w_absmax : nullptr;

@@ -89,6 +89,7 @@ struct mma_params {
     const float *bias;
     int epilogue;
     int *status;
+    int poll_limit; // test hook (cb200_test_arm_wait_timeout): the W loader issues no copies and gives up after so many polls; 0: none
     const std::int32_t *row_order;
 };
 
@@ -154,8 +155,10 @@ __global__ void __launch_bounds__(kThreads, 1) qcsr_fwd_mma_kernel(const mma_par
     std::uint64_t *w_empty = bars + 4 + STAGES;      // [STAGES] MMA commit -> loader
     std::uint64_t *acc_full = bars + 4 + 2 * STAGES; // MMA commit -> row threads
     std::uint64_t *acc_empty = acc_full + 1;         // row threads -> MMA   (one arrival per warp)
-    std::uint32_t *tmem_slot = reinterpret_cast<std::uint32_t *>(acc_empty + 1);
+    std::uint64_t *mma_drain = acc_empty + 1;        // the MMA warp's own, used once, after an abort
+    std::uint32_t *tmem_slot = reinterpret_cast<std::uint32_t *>(mma_drain + 1);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
+    volatile int *fills = reinterpret_cast<volatile int *>(tmem_slot + 2); // of the W ring, once its loader has ended
 
     const int tid = threadIdx.x, warp = warp_of_block(), lane = tid & 31;
     const std::uint32_t smem0 = smem_addr(smem);
@@ -173,6 +176,7 @@ __global__ void __launch_bounds__(kThreads, 1) qcsr_fwd_mma_kernel(const mma_par
         }
         bar_init(smem_addr(acc_full), 1);
         bar_init(smem_addr(acc_empty), kProducerWarps);
+        bar_init(smem_addr(mma_drain), 1);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -376,16 +380,28 @@ __global__ void __launch_bounds__(kThreads, 1) qcsr_fwd_mma_kernel(const mma_par
     } else if (elect_one()) {
         // ================= W loader =================
         const long long total = my_groups * p.windows;
-        for (long long q = 0; q < total; ++q) {
+        long long q = 0;
+        bool dead = p.poll_limit != 0 && bar_wait(smem_addr(w_full), 0u, abort_flag, p.poll_limit);
+        for (; q < total && !dead; ++q) {
             const int s = static_cast<int>(q % STAGES);
-            bar_wait(smem_addr(w_empty + s), static_cast<std::uint32_t>(((q / STAGES) & 1) ^ 1), abort_flag);
+            dead = bar_wait(smem_addr(w_empty + s), static_cast<std::uint32_t>(((q / STAGES) & 1) ^ 1), abort_flag);
+            if (dead) break; // no new copies once a wait of the CTA has run out
             bar_arrive_expect_tx(smem_addr(w_full + s), REC);
             bulk_copy_g2s(wstage0 + s * REC, p.records + static_cast<std::size_t>(q % p.windows) * REC, REC, smem_addr(w_full + s));
         }
+        *fills = static_cast<int>(q);
     }
 
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    if (*abort_flag != 0) { // every role has ended: what is in flight finishes before the CTA gives up its shared and tensor memory
+        if (warp == kProducerWarps) {
+            if (elect_one()) drain_mmas(smem_addr(mma_drain));
+        } else if (warp > kProducerWarps) {
+            if (elect_one()) drain_fills(smem_addr(w_full), STAGES, *fills);
+        }
+        __syncthreads();
+    }
     if (warp == 0) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemCols) : "memory");
@@ -394,7 +410,7 @@ __global__ void __launch_bounds__(kThreads, 1) qcsr_fwd_mma_kernel(const mma_par
 }
 
 template<int NC> constexpr std::size_t mma_smem_bytes() {
-    return 2 * kABufBytes + w_stages(NC) * record_bytes(NC) + kRingBytes + (6 + 2 * w_stages(NC)) * sizeof(std::uint64_t) + 16;
+    return 2 * kABufBytes + w_stages(NC) * record_bytes(NC) + kRingBytes + (7 + 2 * w_stages(NC)) * sizeof(std::uint64_t) + 16;
 }
 
 template<int BITS, int NC>
@@ -460,7 +476,7 @@ cb200_status launch_qcsr_forward_mma(const qcsr_view &x, const dense_args &d, st
     p.row_ptr = x.row_ptr; p.packed_row_ptr = x.packed_row_ptr; p.col_idx = x.col_idx; p.packed = x.packed;
     p.row_offsets = row_policy ? x.offsets : nullptr; p.records = records; p.y = d.out; p.y_ld = d.out_ld;
     p.row_begin = row_begin; p.row_end = row_end; p.groups = (row_end - row_begin + kRows - 1) / kRows;
-    p.windows = windows; p.alpha = d.alpha; p.beta = d.beta; p.bias = d.bias; p.epilogue = d.epilogue; p.status = status;
+    p.windows = windows; p.alpha = d.alpha; p.beta = d.beta; p.bias = d.bias; p.epilogue = d.epilogue; p.status = status; p.poll_limit = test_poll_limit();
     // a row order describes the whole matrix; a partial row range runs in natural order
     p.row_order = (row_begin == 0 && row_end == x.rows) ? row_order : nullptr;
     *taken = true;

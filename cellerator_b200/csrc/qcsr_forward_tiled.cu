@@ -237,6 +237,7 @@ __global__ void __launch_bounds__(kThreads, 1) qcsr_fwd_tiled_kernel(const tiled
         bulk_copy_g2s(wbuf0 + b * WBUF, static_cast<const unsigned char *>(p.w) + static_cast<std::size_t>(g0) * RB, bytes,
                       bar0 + 8 * b);
     };
+    std::int64_t issued = total_tiles < 2 ? total_tiles : 2; // thread 0: tiles copied
     if (tid == 0) {
         if (total_tiles > 0) issue_tile(0);
         if (total_tiles > 1) issue_tile(1);
@@ -424,9 +425,10 @@ __global__ void __launch_bounds__(kThreads, 1) qcsr_fwd_tiled_kernel(const tiled
                 }
             }
             __syncthreads();
-            if (tid == 0 && q + 2 < total_tiles) {
+            if (tid == 0 && q + 2 < total_tiles && *static_cast<volatile int *>(abort_flag) == 0) { // no new copies once a wait has run out
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 issue_tile(q + 2);
+                issued = q + 3;
             }
         }
 
@@ -461,7 +463,13 @@ __global__ void __launch_bounds__(kThreads, 1) qcsr_fwd_tiled_kernel(const tiled
         }
         __syncthreads(); // meta / lens are rewritten by the next group
     }
-    if (tid == 0 && *abort_flag != 0 && p.status != nullptr) atomicExch(p.status, 1);
+    if (tid == 0 && *abort_flag != 0) {
+        // the copies in flight land before the CTA gives up its shared memory
+        for (std::int64_t i = issued - 1; i >= 0 && i >= issued - 2; --i)
+            for (int spins = 0; spins <= (1 << 22) && !mbar_try_wait(bar0 + 8 * static_cast<std::uint32_t>(i & 1), static_cast<std::uint32_t>((i >> 1) & 1)); ++spins) {
+            }
+        if (p.status != nullptr) atomicExch(p.status, 1);
+    }
 }
 
 template<typename WT, int LPN>

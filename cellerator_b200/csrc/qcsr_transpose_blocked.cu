@@ -97,6 +97,7 @@ struct tb_params {
     float alpha;
     float beta;   // of this pass: the call's, then 1
     int *status;
+    int poll_limit; // test hook (cb200_test_arm_wait_timeout): the loader of G issues no copies and gives up after so many polls; 0: none
     int value_part; // 0: tile holds hi = bf16(value); 1: lo = bf16(value - hi)
     // The accumulators of a run (the consecutive units of one window set in one CTA) go to slot `global run index` of
     // this array, [run][window of the set][gene][N]; ordered_sum_kernel adds the slots of a set into G' in run order,
@@ -196,10 +197,12 @@ __global__ void __launch_bounds__(kThreads, 1) qcsr_transpose_blocked_kernel(con
     std::uint64_t *c_empty = c_full + kChunkStages;    // [kChunkStages] scatter warps -> loaders
     std::uint64_t *acc_full = c_empty + kChunkStages;  // MMA commit -> scatter warps
     std::uint64_t *acc_empty = acc_full + 1;           // scatter warps -> MMA
-    volatile int *chunk_meta = reinterpret_cast<volatile int *>(acc_empty + 1); // [kChunkStages]
+    std::uint64_t *mma_drain = acc_empty + 1;          // [kIssuers] an MMA warp's own, used once, after an abort
+    volatile int *chunk_meta = reinterpret_cast<volatile int *>(mma_drain + kIssuers); // [kChunkStages]
     std::uint32_t *tmem_slot = reinterpret_cast<std::uint32_t *>(const_cast<int *>(chunk_meta) + kChunkStages + 1);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
     unsigned char *scratch_slot = reinterpret_cast<unsigned char *>(tmem_slot + 2);
+    volatile int *fills = reinterpret_cast<volatile int *>(tmem_slot + 3); // [3] of the ring of G and of the groups' chunk rings, once the loaders have ended
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const std::uint32_t smem0 = smem_addr(smem);
@@ -221,6 +224,7 @@ __global__ void __launch_bounds__(kThreads, 1) qcsr_transpose_blocked_kernel(con
         }
         bar_init(smem_addr(acc_full), kIssuers);
         bar_init(smem_addr(acc_empty), kProducerWarps);
+        for (int i = 0; i < kIssuers; ++i) bar_init(smem_addr(mma_drain + i), 1);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -477,23 +481,28 @@ __global__ void __launch_bounds__(kThreads, 1) qcsr_transpose_blocked_kernel(con
         const int role = warp - kProducerWarps - kIssuerWarps; // 0: pieces of G, 1..kChunkLoaders: entry chunks
         if (role == 0) {
             if (elect_one()) {
-                int s = 0;
+                int s = 0, issued = 0;
                 std::uint32_t ph = 1;
-                for (std::int64_t u = u0; u < u1; ++u) {
+                bool dead = p.poll_limit != 0 && bar_wait(smem_addr(g_full), 0u, abort_flag, p.poll_limit);
+                for (std::int64_t u = u0; u < u1 && !dead; ++u) {
                     const unsigned char *src = p.records + static_cast<std::size_t>(u % p.group_count) * kGroupPieces * p.piece_stride;
                     for (int piece = 0; piece < kGroupPieces; ++piece, src += p.piece_stride) {
                         const std::uint32_t full = smem_addr(g_full + s / kPerBar);
                         if (piece % kPerBar == 0) {
-                            bar_wait(smem_addr(g_empty + s / kPerBar), ph, abort_flag);
+                            dead = bar_wait(smem_addr(g_empty + s / kPerBar), ph, abort_flag);
+                            if (dead) break; // no new copies once a wait of the CTA has run out
+                            ++issued;
                             bar_arrive_expect_tx(full, kPerBar * GPIECE);
                         }
                         bulk_copy_g2s(grec0 + s * GPIECE, src, GPIECE, full);
                         if (++s == kPieces) { s = 0; ph ^= 1u; }
                     }
                 }
+                fills[0] = issued;
             }
         } else {
             long long q = 0, qc0 = 0, qc1 = 0; // tiles; chunks issued into each group's ring
+            bool dead = false; // lane 0: a wait was given up, no copy is issued any more (the loops run out empty)
             for (std::int64_t u = u0; u < u1; ++u) {
                 const std::int64_t set = u / p.group_count, group = p.group_begin + u % p.group_count;
                 const int nwin = static_cast<int>(dmin(kSetWindows, p.windows - set * kSetWindows));
@@ -506,9 +515,9 @@ __global__ void __launch_bounds__(kThreads, 1) qcsr_transpose_blocked_kernel(con
                     do {
                         const int n_entries = static_cast<int>(dmin(kChunkEntries, hi - at));
                         const long long mine = ring == 0 ? qc0 : qc1;
-                        if (lane == 0) {
-                            const int cs = ring * kRing + static_cast<int>(mine % kRing);
-                            bar_wait(smem_addr(c_empty + cs), static_cast<std::uint32_t>(((mine / kRing) & 1) ^ 1), abort_flag);
+                        const int cs = ring * kRing + static_cast<int>(mine % kRing);
+                        if (lane == 0 && !dead) dead = bar_wait(smem_addr(c_empty + cs), static_cast<std::uint32_t>(((mine / kRing) & 1) ^ 1), abort_flag);
+                        if (lane == 0 && !dead) {
                             chunk_meta[cs] = (n_entries << 1) | (at + n_entries >= hi ? 1 : 0);
                             if (n_entries > 0) {
                                 bar_arrive_expect_tx(smem_addr(c_full + cs), static_cast<std::uint32_t>(n_entries) * 4u);
@@ -519,16 +528,38 @@ __global__ void __launch_bounds__(kThreads, 1) qcsr_transpose_blocked_kernel(con
                             }
                         }
                         at += n_entries;
-                        if (ring == 0) ++qc0;
-                        else ++qc1;
+                        if (!dead) { // lane 0's counters stop with its last issued chunk
+                            if (ring == 0) ++qc0;
+                            else ++qc1;
+                        }
                     } while (at < hi);
                 }
+            }
+            if (lane == 0) {
+                fills[1] = static_cast<int>(qc0);
+                fills[2] = static_cast<int>(qc1);
             }
         }
     }
 
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    if (*abort_flag != 0) { // every role has ended: what is in flight finishes before the CTA gives up its shared and tensor memory
+        const int role = warp - kProducerWarps - kIssuerWarps;
+        if (warp >= kProducerWarps && warp < kProducerWarps + kIssuers) {
+            // by the thread that issued
+            if constexpr (kIssuers == 2) {
+                if (lane == 0) drain_mmas(smem_addr(mma_drain + (warp - kProducerWarps)));
+            } else {
+                if (elect_one()) drain_mmas(smem_addr(mma_drain));
+            }
+        } else if (role == 0) {
+            if (elect_one()) drain_fills(smem_addr(g_full), kPieces / kPerBar, fills[0]);
+        } else if (role == 1 && lane == 0) {
+            for (int ring = 0; ring < 2; ++ring) drain_fills(smem_addr(c_full + ring * kRing), kRing, fills[1 + ring]);
+        }
+        __syncthreads();
+    }
     if (warp == 0) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemCols) : "memory");
@@ -538,7 +569,7 @@ __global__ void __launch_bounds__(kThreads, 1) qcsr_transpose_blocked_kernel(con
 
 template<int NC, bool BAKED> constexpr std::size_t tb_smem_bytes() {
     return 2 * kTileBytes + ring_pieces(NC) * g_piece_bytes(NC) + kChunkStages * kChunkBytes + (BAKED ? 0 : set_windows(NC) * kWin * 8 + kRows * 4) +
-           (6 + 2 * ring_pieces(NC) + 2 * kChunkStages) * sizeof(std::uint64_t) + (kChunkStages + 1) * 4 + 16;
+           (6 + issuers(NC) + 2 * ring_pieces(NC) + 2 * kChunkStages) * sizeof(std::uint64_t) + (kChunkStages + 1) * 4 + 24;
 }
 
 // G'[genes of window wl of set s] = beta * G' + alpha * (the sums of the runs of set s, added in run order).  Block = (set, window of
@@ -673,7 +704,7 @@ cb200_status launch_qcsr_transpose_blocked(const qcsr_view &x, const dense_args 
     p.gene_offsets = row_policy ? nullptr : x.offsets; p.row_offsets = row_policy ? x.offsets : nullptr;
     p.records = records; p.out = d.out; p.out_ld = d.out_ld; p.cols = x.cols;
     p.group_begin = group_begin; p.group_count = group_end - group_begin; p.windows = layout.windows;
-    p.alpha = d.alpha; p.beta = d.beta; p.status = status;
+    p.alpha = d.alpha; p.beta = d.beta; p.status = status; p.poll_limit = test_poll_limit();
     // One pass multiplies bf16(value) with bf16(G).  With split products the fp32 product is rebuilt
     // from hi*hi + hi*lo + lo*hi (v = hi + lo + O(2^-17 v), likewise G): relative error per product
     // about 3 * 2^-17, inside the 1e-4 bound of an fp32 dense operand.  The passes run back to back on

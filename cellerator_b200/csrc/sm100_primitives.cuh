@@ -63,6 +63,11 @@ __device__ __forceinline__ bool bar_wait_drain(std::uint32_t bar, std::uint32_t 
         if (bar_try_wait(bar, parity)) return true;
     return false;
 }
+// The same for a loader's copies, behind the barrier that ends the roles: `issued` fills of the stages in turn (every `step`-th of
+// them this loader's), whose barriers receive nothing but the fills.
+__device__ __forceinline__ void drain_fills(std::uint32_t bars, int stages, int issued, int step = 1) {
+    for (int i = issued - 1; i >= 0 && i >= issued - stages; i -= step) bar_wait_drain(bars + i % stages * 8, static_cast<std::uint32_t>((i / stages) & 1));
+}
 // One contiguous global -> shared copy by the copy engine (this GPU's own memory, no multicast).
 __device__ __forceinline__ void bulk_copy_g2s(std::uint32_t dst, const void *src, std::uint32_t bytes, std::uint32_t bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
@@ -122,6 +127,11 @@ __device__ __forceinline__ void mma_bf16(std::uint32_t tmem_d, std::uint64_t des
 }
 __device__ __forceinline__ void mma_commit(std::uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+// After an abort, behind the barrier that ends the roles: the MMAs this thread has issued finish.  `bar` is its own, used once.
+__device__ __forceinline__ void drain_mmas(std::uint32_t bar) {
+    mma_commit(bar);
+    bar_wait_drain(bar, 0u);
 }
 __device__ __forceinline__ void tmem_ld32(std::uint32_t taddr, float (&v)[32]) {
     std::uint32_t r[32];

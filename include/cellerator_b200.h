@@ -931,12 +931,12 @@ cb200_status cb200_host_forward(cb200_host_stage *stage, const cb200_qcsr *x, co
                                 int64_t y_ld, float alpha, uint64_t *h2d_bytes, uint64_t *d2h_bytes);
 
 /* ------------------------------------------------------------------------------------------
- * Test hook (no counterpart in the reference).  Makes the bounded waits of the tensor-core forward
- * kernel over the window-blocked copy observable: while armed, that kernel's W loader issues no
- * copies and every wait of the launch gives up after `poll_limit` polls, so the launch ends within
- * microseconds with the status word set, its TMEM freed and its output invalid.  The 8-bit, N = 256
- * Blocked-ELL kernel does the same: a quarter of its decoded operands is not handed over, and the MMA
- * warps' waits give up with copies in flight.  The next launch after
+ * Test hook (no counterpart in the reference).  Makes the bounded waits of the tensor-core kernels
+ * observable: while armed, the loader of the dense operand (forward over entry words, decoded tiles and
+ * CSR windows; transpose) issues no copies and a wait of the launch gives up after `poll_limit` polls,
+ * so the launch ends within microseconds with the status word set, its TMEM freed and its output
+ * invalid.  The 8-bit, N = 256 Blocked-ELL kernel does the same: a quarter of its decoded operands is
+ * not handed over, and the MMA warps' waits give up with copies in flight.  The next launch after
  * cb200_test_disarm_wait_timeout is a normal one.  poll_limit is clamped to [64, 2^22]. */
 void cb200_test_arm_wait_timeout(uint32_t poll_limit);
 void cb200_test_disarm_wait_timeout(void);

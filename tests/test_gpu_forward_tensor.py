@@ -390,3 +390,36 @@ def test_fp16_schedules_keep_their_accuracy_over_magnitudes(cuda_device, oracle,
         scale = l1[:, None] * float(np.abs(w_host).max()) + 1e-300
         assert np.all(err <= 2e-3 * scale), f"max err/scale {np.max(err / scale):.3e}"
     op.close()
+
+
+@pytest.mark.parametrize("schedule,n,multiply", [("tensor_blocked", 32, capi.DTYPE_BF16), ("tensor_blocked", 64, capi.DTYPE_F32), ("tensor_blocked", 128, capi.DTYPE_BF16),
+                                                 ("tensor_dense", 64, capi.DTYPE_BF16), ("tensor_dense", 128, capi.DTYPE_BF16),
+                                                 ("tensor_windows", 64, capi.DTYPE_BF16), ("transpose", 32, capi.DTYPE_F32), ("transpose", 64, capi.DTYPE_F32),
+                                                 ("transpose", 64, capi.DTYPE_BF16)])
+def test_bounded_wait_path(cuda_device, oracle, schedule, n, multiply):
+    """The dense operand is withheld while entries and tiles are copied: the launch ends with its status word set, what is in
+    flight drained, and the next launch on the stream has the right bits."""
+    L = capi.lib()
+    rng = np.random.default_rng(n)
+    rows, cols = 256 * 40 + 5, 128 * 9                     # long segments: the kernel with one scatter group
+    c = host_pack(oracle, random_csr(rng, rows=rows, cols=cols, max_nnz=400, bits=8, policy=1))
+    x = to_dev(c, cuda_device)
+    back = schedule == "transpose"
+    d, _ = dense(rng, rows if back else cols, n, torch.float32 if back else torch.bfloat16, cuda_device)
+    op = ops.PreparedSpmm(capi.PROJECTION_TRANSPOSE if back else capi.PROJECTION_CSR, rows, cols, n, x.nnz, 8, 1, d.dtype, cuda_device,
+                          host_row_ptr=x.host_row_ptr, multiply=multiply, device_matrix=x, schedule="tensor_blocked" if back else schedule)
+    assert op.schedule.startswith("tensor_blocked" if back else schedule)
+    shape = (cols if back else rows, n)
+    good = op.run(x, d, torch.empty(shape, device=cuda_device)).clone()
+    assert op.status() == 0
+    for _ in range(3):
+        L.cb200_test_arm_wait_timeout(4096)
+        try:
+            op.run(x, d, torch.empty(shape, device=cuda_device))
+        finally:
+            L.cb200_test_disarm_wait_timeout()
+        with pytest.raises(capi.Cb200Error) as e:
+            op.status()
+        assert e.value.status == capi.DEVICE_WAIT_TIMEOUT
+        assert torch.equal(op.run(x, d, torch.full(shape, float("nan"), device=cuda_device)), good) and op.status() == 0
+    op.close()
