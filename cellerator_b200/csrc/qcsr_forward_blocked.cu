@@ -1282,10 +1282,8 @@ cb200_status launch_qcsr_forward_blocked(const qcsr_view &x, const dense_args &d
     const bool long_segments = layout.total_entries > static_cast<std::int64_t>(kChunkEntries) * layout.groups * layout.windows;
     // two scatter groups pay when a window is a chunk or two; long segments keep one group and deeper chunks
     const bool two_groups = layout.baked && !long_segments;
-    const int both_parts = split_products && !w_bf16 && layout.baked && qcsr_blocked_takes_both_parts(d.n, d.dense_dtype) &&
-                                   workspace_bytes >= qcsr_blocked_workspace_bytes(x.cols, 2 * d.n) ? 1 : 0;
-    const std::int64_t columns = both_parts != 0 ? 2 * d.n : d.n;
-    p.record_stride = record_bytes(static_cast<int>(columns));
+    const bool both_parts = split_products && !w_bf16 && layout.baked && qcsr_blocked_takes_both_parts(d.n, d.dense_dtype);
+    const bool halves = both_parts && workspace_bytes < qcsr_blocked_workspace_bytes(x.cols, 2 * d.n);
     p.alpha = d.alpha; p.status = status;
     p.result_scale = half ? 1.0f / layout.value_scale : 1.0f;
     p.w_absmax = half ? w_absmax : nullptr;
@@ -1304,39 +1302,59 @@ cb200_status launch_qcsr_forward_blocked(const qcsr_view &x, const dense_args &d
     // the same fixed order, so the result is repeatable.
     // hi*hi and hi*lo read the same tiles, and a tile costs more than its MMAs: where both parts of W fit an accumulator of
     // 128 columns they are one pass over [hi of W | lo of W] (30,000 x 12,000 at N = 64: 369 -> 244 us, 75,776 x 2,000 at
-    // N = 32 226 -> 137).
-    struct pass_spec { int w_part, value_part; };
-    const pass_spec plain[1] = {{0, 0}}, split_bf16[2] = {{0, 0}, {0, 1}}, split_f32[3] = {{0, 0}, {1, 0}, {0, 1}};
-    const pass_spec *passes = !split_products ? plain : (w_bf16 || both_parts != 0 ? split_bf16 : split_f32);
-    const int pass_count = !split_products ? 1 : (w_bf16 || both_parts != 0 ? 2 : 3);
-    int packed_part = -1;
+    // N = 32 226 -> 137).  A workspace with room for N columns of W holds both parts of half of them: two passes, the same bits.
+    struct pass_spec {
+        int w_part, value_part;
+        bool both;             // [hi of W | lo of W]
+        std::int64_t col0, n;  // columns of W and Y
+        bool packs;            // the records hold something else
+    };
+    pass_spec passes[3];
+    int pass_count = 0;
+    const auto add_pass = [&](int w_part, int value_part, bool both, std::int64_t col0, std::int64_t n, bool packs) {
+        passes[pass_count++] = pass_spec{w_part, value_part, both, col0, n, packs};
+    };
+    if (halves) {
+        add_pass(0, 0, true, 0, d.n / 2, true);
+        add_pass(0, 0, true, d.n / 2, d.n / 2, true);
+    } else {
+        add_pass(0, 0, both_parts, 0, d.n, true);
+        if (split_products && !w_bf16 && !both_parts) add_pass(1, 0, false, 0, d.n, true);
+    }
+    if (split_products) add_pass(0, 1, false, 0, d.n, !w_bf16 && (halves || !both_parts));
     for (int i = 0; i < pass_count; ++i) {
-        if (passes[i].w_part != packed_part) {
+        const pass_spec &pass = passes[i];
+        if (pass.packs) {
+            const std::int64_t columns = pass.both ? 2 * pass.n : pass.n;
+            p.record_stride = record_bytes(static_cast<int>(columns));
             const dim3 grid(static_cast<unsigned>(layout.windows), static_cast<unsigned>(columns / kPackColumns));
             if (w_bf16)
                 CB200_CUDA_OK(launch_kernel(half && i == 0, pack_windows_kernel<__nv_bfloat16>, grid, 256, 0, stream, static_cast<const __nv_bfloat16 *>(d.dense),
-                                            d.dense_ld, x.cols, static_cast<int>(d.n), passes[i].w_part, x.scales, x.offsets, row_policy ? 0 : 1, records,
+                                            d.dense_ld, x.cols, static_cast<int>(pass.n), pass.w_part, x.scales, x.offsets, row_policy ? 0 : 1, records,
                                             half ? w_absmax : nullptr, 0));
             else
-                CB200_CUDA_OK(launch_kernel(half && i == 0, pack_windows_kernel<float>, grid, 256, 0, stream, static_cast<const float *>(d.dense), d.dense_ld,
-                                            x.cols, static_cast<int>(d.n), passes[i].w_part, x.scales, x.offsets, row_policy ? 0 : 1, records,
-                                            half ? w_absmax : nullptr, both_parts));
+                CB200_CUDA_OK(launch_kernel(half && i == 0, pack_windows_kernel<float>, grid, 256, 0, stream, static_cast<const float *>(d.dense) + pass.col0, d.dense_ld,
+                                            x.cols, static_cast<int>(pass.n), pass.w_part, x.scales, x.offsets, row_policy ? 0 : 1, records,
+                                            half ? w_absmax : nullptr, pass.both ? 1 : 0));
             count_launch();
             CB200_CUDA_OK(cudaGetLastError());
-            packed_part = passes[i].w_part;
         }
-        p.value_part = passes[i].value_part;
-        if (layout.baked) p.entries = passes[i].value_part != 0 ? layout.entries_lo : layout.entries; // baked words carry their part
-        p.beta = i == 0 ? d.beta : 1.0f;
+        p.value_part = pass.value_part;
+        if (layout.baked) p.entries = pass.value_part != 0 ? layout.entries_lo : layout.entries; // baked words carry their part
+        p.y = d.out + pass.col0;
+        p.beta = i == 0 || pass.col0 != 0 ? d.beta : 1.0f;
         p.bias = d.bias;
         p.epilogue = i + 1 == pass_count ? d.epilogue : CB200_EPILOGUE_NONE;
         cb200_status st;
-        const std::int64_t pass_columns = both_parts != 0 && passes[i].value_part == 0 ? columns : d.n;
-        p.idesc = instr_desc(static_cast<int>(pass_columns), half);
-        p.split = split_of_launch(x, d.n, pass_columns, workspace, workspace_bytes, qcsr_blocked_workspace_bytes(x.cols, columns), sm_count);
-        if (both_parts != 0 && passes[i].value_part == 0) {
-            if (two_groups) st = d.n == 64 ? launch_blocked2<128, 64>(p, sm_count, stream) : launch_blocked2<64, 32>(p, sm_count, stream);
-            else st = d.n == 64 ? launch_cs<128, 64, 3, true>(p, sm_count, stream) : launch_cs<64, 32, 3, true>(p, sm_count, stream);
+        p.idesc = instr_desc(static_cast<int>(pass.both ? 2 * pass.n : pass.n), half);
+        const std::int64_t columns = pass.both ? 2 * d.n : d.n; // halves are summed as the whole is
+        p.split = split_of_launch(x, pass.n, columns, workspace, workspace_bytes, qcsr_blocked_workspace_bytes(x.cols, both_parts && !halves ? 2 * d.n : d.n), sm_count);
+        if (pass.both) {
+            switch (pass.n) {
+            case 16: st = two_groups ? launch_blocked2<32, 16>(p, sm_count, stream) : launch_cs<32, 16, 3, true>(p, sm_count, stream); break;
+            case 32: st = two_groups ? launch_blocked2<64, 32>(p, sm_count, stream) : launch_cs<64, 32, 3, true>(p, sm_count, stream); break;
+            default: st = two_groups ? launch_blocked2<128, 64>(p, sm_count, stream) : launch_cs<128, 64, 3, true>(p, sm_count, stream); break;
+            }
         } else {
             switch (d.n) {
             case 32: st = two_groups ? launch_blocked2<32>(p, sm_count, stream) : launch_one<32>(p, long_segments, layout.baked, sm_count, stream); break;
@@ -1345,7 +1363,7 @@ cb200_status launch_qcsr_forward_blocked(const qcsr_view &x, const dense_args &d
             }
         }
         if (st != CB200_STATUS_SUCCESS) return st;
-        st = launch_add_parts(p.split, pass_columns <= 64, p.group_begin, p.group_end, row_end, static_cast<int>(d.n), d.out, d.out_ld, p.alpha, p.beta, p.bias, p.epilogue,
+        st = launch_add_parts(p.split, columns <= 64, p.group_begin, p.group_end, row_end, static_cast<int>(pass.n), p.y, d.out_ld, p.alpha, p.beta, p.bias, p.epilogue,
                               p.result_scale, p.w_absmax, stream);
         if (st != CB200_STATUS_SUCCESS) return st;
     }
