@@ -64,7 +64,8 @@ struct cb200_prepared {
     std::uint32_t workspace_alignment;
     int sm_count;
     // persistent state built at prepare time (persistent_kernel_state, operation_core.hh:126-129):
-    // the rows in descending order of length, on the device; null when no host row_ptr was given
+    // the rows in descending order of length, on the device, for the two kernels that give a row to one lane group or thread
+    // ("gene_tiled", "tensor_windows"); null when no host row_ptr was given
     std::int32_t *row_order;
     // ... and, when prepare was given the device-resident matrix and bf16 products are allowed, the
     // window-blocked copy the tensor-core kernel streams
@@ -315,7 +316,7 @@ struct schedule_plan {
     bool dense_forced = false;   // ... asked for by name: the free-memory rule does not apply
     bool codes_wanted = false;   // forward, 4-bit codes: tiles of codes (a byte per slot) instead of decoded tiles
     bool gene_gather = false;    // transpose with a fixed order of the sums
-    bool row_order = false;      // length-sorted row order for the tiled kernels
+    bool row_order = false;      // length-sorted row order ("gene_tiled", "tensor_windows")
     bool bell_cuda_cores = false;
     double mean_row_nnz = 0.0;
 };

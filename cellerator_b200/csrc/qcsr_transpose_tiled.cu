@@ -11,8 +11,9 @@
 // per gene walks the gene's entries, reads their rows of G from the tile and keeps the sum in registers: one vector reduction
 // per (gene, tile) instead of one per entry.
 //
-// What bounds it: shared memory, 80 % of its bandwidth.  Rows of G are two 128-byte wavefronts per entry at N = 64 (110 of the
-// 255 us), the sort and its look-ups the other half.  A tile of 512 rows is what leaves room for the entries of 512 genes;
+// What bounds it: the LSU data pipe, 80 % busy: 56.7 M wavefronts of shared memory for 14.6 M entries, 40 M of them loads (rows
+// of G are two wavefronts per entry at N = 64) and 14 M the sort's atomics; 281 us, and 48 us of the pass over the indices, whose
+// 256 CTAs of 1,024 threads are dealt unevenly to 148 SMs.  A tile of 512 rows is what leaves room for the entries of 512 genes;
 // smaller tiles would make the runs per gene too short to pay for their start and the reduction (27 entries at 5 % density),
 // more rows do not fit.  8,191 x 33,538, 14.7 M entries: N = 64 1.37 -> 0.31 ms, N = 50 2.54 -> 0.32 ms; 16,384 rows at N = 128
 // (two column tiles, sorted twice) 4.33 -> 1.12 ms.

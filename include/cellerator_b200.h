@@ -322,7 +322,10 @@ cb200_status cb200_spmm_prepare(const cb200_spmm_problem *problem, cb200_prepare
 cb200_status cb200_spmm_persistent_requirement(const cb200_spmm_problem *problem, uint64_t *bytes);
 void cb200_prepared_destroy(cb200_prepared *prepared);
 /* workspace_requirement, launch_bindings.hh:67-71: what the schedule can use.  "vector_reductions" reports up to 32 MB (it
- * sorts the entries with it, slice of rows by slice) and also runs with less or with none, slower. */
+ * sorts the entries with it, slice of rows by slice) and also runs with less or with none, slower.  "warp_per_row" (unaligned
+ * N) and the tensor_blocked and tensor_dense forward schedules also run with less, down to the status block and the records of
+ * W, slower and with the same bits: a row's sum follows from its entries, N and W's type, not from the room, the launch's row
+ * range or the rows beside it. */
 cb200_status cb200_prepared_workspace(const cb200_prepared *prepared, uint64_t *minimum_bytes, uint32_t *alignment);
 /* kernel choice made at prepare time, as text: "warp_per_row", "gene_tiled" (exact fp32 products);
  * "tensor_windows", "tensor_blocked", "tensor_dense", "tensor_codes" (CSR, 16-bit products on tcgen05);

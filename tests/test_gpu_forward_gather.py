@@ -90,3 +90,14 @@ def test_a_rows_bits_follow_from_its_entries(cuda_device, oracle, bits, policy, 
             assert torch.equal(ops.spmm_forward(part, w), y[lo:hi]), (n, lo)
         if dtype == torch.float32:
             assert torch.equal(ops.public_projection(x, w), y), n
+
+
+def test_chunks_of_a_host_call_have_the_matrixs_bits(cuda_device, oracle):
+    """W is re-laid for the whole matrix, not for a chunk of it, nor for a chunk of 1,000 rows but for one of 1,300."""
+    from test_gpu_fleet_host import _host_forward_all_forms
+    c = matrix(oracle, np.random.default_rng(3).integers(900, 1300, size=1301), 4000, 8, 1, 9)
+    w, _ = dense(np.random.default_rng(4), 4000, 50, torch.bfloat16, cuda_device)
+    y = ops.spmm_forward(to_dev(c, cuda_device), w).cpu().numpy()
+    for rows in (300, 1000, 1301):
+        got = _host_forward_all_forms(cuda_device, c, w.cpu().pin_memory(), 50, (0,), chunk_rows=rows, chunk_nnz=1_700_000)
+        assert np.array_equal(got[0][0].numpy(), y)
