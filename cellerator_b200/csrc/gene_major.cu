@@ -371,7 +371,7 @@ __device__ __forceinline__ void gather_add(const gather_params &p, const gather_
 // two shuffles, one 32 x 32 -> 64-bit multiply-add for the address, one load and VEC FMAs per entry:
 // the kernel issues an instruction in most cycles, so every instruction per entry counts.
 // What bounds it then is the way from L2: a row of G per entry, 256 B at N = 64, 17 TB/s (180 M entries: 3,018 us with the
-// last entries of a chunk fetched one by one, 2,640 with them in groups of eight like the others; with tiles of G in shared
+// last entries of a chunk fetched one by one, 2,640 to 2,870 on different GPUs with them in groups of eight like the others; with tiles of G in shared
 // memory and running sums per gene and tile 4,081).  PACKED (per-gene offsets, cells
 // below 2^24) halves the shuffles: a lane hands out (cell << 8 | code) and every lane decodes the value itself -- the same
 // fused multiply-add, so the same bits.

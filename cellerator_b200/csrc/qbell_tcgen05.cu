@@ -33,7 +33,7 @@
 //   warps 0-3  epilogue: tcgen05.ld the accumulators (double buffered, handed back before the last columns' stores), apply
 //              alpha / beta, store Y rows coalesced.
 // A form with two CTAs per SM, each with two stages of two blocks, whose decoding warps also started the copies, ran a stage's
-// copy, MMAs and release one after the other (3,800 cycles per 36 KB): 222 us for that matrix, now 169 (N = 128: 185 -> 126); with
+// copy, MMAs and release one after the other (3,800 cycles per 36 KB): 222 us for that matrix, now 160 (N = 128: 185 -> 126); with
 // a ring of single blocks and a commit per block the issuing threads were the bound (218 us; 331 before they were elected,
 // see elect_one).
 // Empty blocks (index 0xffffffff) are skipped; genes >= cols and cells past the last row decode to 0.  Every barrier wait is
