@@ -1069,7 +1069,7 @@ static int window_parts(int windows, std::int64_t columns) {
 // sums and one for 60 of the sums.  5,000 x 33,538 at N = 64: 189 -> 56 us; 125,000 rows, split products (two passes): 1,428 ->
 // 1,181 us, the 45 groups behind 3 x 148 in three units each.
 window_split_plan qcsr_window_split(std::int64_t rows, std::int64_t cols, std::int64_t columns, int sm_count) {
-    constexpr int kMostSums = 6; // of cut groups, per SM: what bounds the workspace
+    constexpr int kMostSums = 4; // of cut groups, per SM: what bounds the workspace (39 MB at N = 64)
     const std::int64_t groups = (rows + kRows - 1) / kRows;
     const int windows = static_cast<int>((cols + kWin - 1) / kWin);
     window_split_plan best;

@@ -101,3 +101,14 @@ def test_chunks_of_a_host_call_have_the_matrixs_bits(cuda_device, oracle):
     for rows in (300, 1000, 1301):
         got = _host_forward_all_forms(cuda_device, c, w.cpu().pin_memory(), 50, (0,), chunk_rows=rows, chunk_nnz=1_700_000)
         assert np.array_equal(got[0][0].numpy(), y)
+
+
+@pytest.mark.parametrize("mean", [40, 100])
+def test_both_kernels_give_a_row_the_same_bits(cuda_device, oracle, mean):
+    """Many short rows, or narrow operands, run with a warp per row (32 or 64 entries at a time); a shard of them by parts."""
+    rng = np.random.default_rng(mean)
+    c = matrix(oracle, np.concatenate([EDGE_LENGTHS, rng.integers(0, 2 * mean, size=64 * 160)]), 4000, 8, 1, mean)
+    x, part = to_dev(c, cuda_device), to_dev(rows_of(c, 0, 600), cuda_device)
+    for n, dtype in ((1, torch.float32), (5, torch.bfloat16), (8, torch.float32), (16, torch.bfloat16), (50, torch.bfloat16), (64, torch.float32)):
+        w, _ = dense(rng, 4000, n, dtype, cuda_device)
+        assert torch.equal(ops.spmm_forward(part, w), ops.spmm_forward(x, w)[:600]), n
