@@ -72,6 +72,9 @@ struct cb200_prepared {
     blocked_layout blocked;
     // ... or, for a transpose that has to be deterministic, the gene-major copy the gather kernel reads
     gene_major_layout gene_major;
+    // ... or the words of the transpose with integer sums, and how many digits of G it takes
+    digit_layout digits;
+    int digit_slices;
     std::uint64_t persistent_bytes;
     // the device memory all of the above lives in: the caller's block or this operation's own allocations
     device_arena arena;
@@ -316,6 +319,7 @@ struct schedule_plan {
     bool dense_forced = false;   // ... asked for by name: the free-memory rule does not apply
     bool codes_wanted = false;   // forward, 4-bit codes: tiles of codes (a byte per slot) instead of decoded tiles
     bool gene_gather = false;    // transpose with a fixed order of the sums
+    int digits = 0;              // transpose with integer sums: digits of G (0: another kernel)
     bool row_order = false;      // length-sorted row order ("gene_tiled", "tensor_windows")
     bool bell_cuda_cores = false;
     double mean_row_nnz = 0.0;
@@ -375,17 +379,25 @@ schedule_plan plan_schedule(const cb200_spmm_problem &pr) {
         return plan;
     }
     if (pr.projection == CB200_PROJECTION_TRANSPOSE) {
-        // With the matrix at hand: the tensor-core kernel over the window-blocked copy.  bf16 products
-        // allowed: one pass (decoded values and G rounded to bf16).  fp32 products: three bf16 passes
-        // (hi*hi + hi*lo + lo*hi) rebuild each product to ~3 * 2^-17 relative, inside the 1e-4 bound of
-        // an fp32 G; that is not bit-equal to an fp32 multiply, and callers that need the fp32-FMA kernel
-        // do not hand the matrix to prepare.  The cost follows the dense area, so it needs density.
-        // Same bits on every run: the tensor-core kernel over the window-blocked copy gives that too (every CTA's sums go to
-        // a slot of their own and are added in a fixed order), and a deterministic request that names it gets it; the
-        // default stays the gather gene by gene from a gene-major copy, whose fp32 sums the oracle restates entry by entry.
+        // With the matrix at hand: a tensor-core kernel over a window-blocked copy.  bf16 products allowed: one pass (decoded
+        // values and G rounded to bf16).  fp32 products: exact integer sums of the codes times three digits of G, or, with
+        // zero-points per row, three bf16 passes (hi*hi + hi*lo + lo*hi) that rebuild each product to ~3 * 2^-17 relative; both
+        // inside the 1e-4 bound of an fp32 G.  The cost follows the dense area, so it needs density.
+        // Same bits on every run: both give that (integer sums have no order, and every CTA's sums go to a slot of their own and
+        // are added in a fixed order), and a deterministic request that names them gets them.  Otherwise such a request is served
+        // under the name "gene_gather": with four digits of G, which are more exact than fp32 sums, where a tile of 256 x 128
+        // holds 600 entries or more (every one of them pays for its tile; 2 %) and there are tiles for every SM (256 of them; 5,000
+        // x 2,000, 320 tiles: 37 us against 42 gathered at N = 32, 38 against 49 at 64); by the gather gene by gene from a gene-major copy, whose fp32
+        // sums the oracle restates entry by entry, below that, with zero-points per row, and where it is asked for by name.
+        const bool digits_ok = pr.device_matrix != nullptr && qcsr_transpose_digits_shape_ok(pr.m, pr.k, pr.n, pr.bits, pr.policy) &&
+                               (limit == 0u || qcsr_digit_words_bytes_bound(pr.m, pr.k, pr.nnz) <= limit);
         const bool named_blocked = hint != nullptr && hint_starts(hint, "tensor_blocked") && pr.device_matrix != nullptr &&
                                    qcsr_transpose_blocked_shape_ok(pr.m, pr.k, pr.n, pr.bits) && (limit == 0u || nnz * 4u <= limit);
         if (pr.deterministic && !named_blocked) {
+            if (hint == nullptr && digits_ok && plan.mean_row_nnz >= 0.02 * static_cast<double>(pr.k) && pr.m * pr.k >= (1ll << 23)) {
+                plan.digits = 4;
+                return plan;
+            }
             plan.gene_gather = true;
             if (limit != 0u && nnz * 5u + static_cast<std::uint64_t>(pr.k + 1) * 12u > limit) {
                 plan.status = fail(CB200_STATUS_UNSUPPORTED, "the gene-major copy of a deterministic transpose exceeds the persistent memory limit");
@@ -396,6 +408,10 @@ schedule_plan plan_schedule(const cb200_spmm_problem &pr) {
         if (hint == nullptr) blocked = blocked && pr.m >= 16 * 256 && plan.mean_row_nnz >= 0.004 * static_cast<double>(pr.k);
         else blocked = blocked && hint_starts(hint, "tensor_blocked");
         if (blocked && limit != 0u && nnz * 4u > limit) blocked = false; // a word per entry has to fit under the caller's limit
+        if (blocked && digits_ok && pr.multiply != CB200_DTYPE_BF16) {
+            plan.digits = 3;
+            return plan;
+        }
         plan.blocked = blocked;
         plan.split = pr.multiply != CB200_DTYPE_BF16;
         // decoded values in the entry words, positions of this kernel's gene-major tile; a second array with the
@@ -469,6 +485,7 @@ schedule_plan plan_schedule(const cb200_spmm_problem &pr) {
 
 std::uint64_t plan_persistent_bytes(const cb200_spmm_problem &pr, const schedule_plan &plan) {
     std::uint64_t bytes = 0;
+    if (plan.digits != 0) bytes += qcsr_digit_words_bytes_bound(pr.m, pr.k, pr.nnz);
     if (plan.gene_gather) bytes += qcsr_gene_major_layout_bytes_bound(pr.m, pr.k, pr.nnz);
     if (plan.blocked) bytes += qcsr_blocked_layout_bytes_bound(pr.m, pr.k, pr.nnz, plan.blocked_lo);
     if (plan.dense_wanted) bytes += device_arena::rounded(qcsr_dense_tile_bytes(pr.m, pr.k));
@@ -543,6 +560,17 @@ cb200_status cb200_spmm_prepare(const cb200_spmm_problem *problem, cb200_prepare
     if (problem->projection == CB200_PROJECTION_TRANSPOSE) {
         p->workspace_bytes = qcsr_transpose_workspace_bytes(problem->m, problem->k, p->sm_count);
         p->schedule_name = "vector_reductions";
+        if (problem->device_matrix == nullptr)
+            p->workspace_bytes = std::max(p->workspace_bytes, qcsr_transpose_digits_once_bytes(problem->m, problem->k, problem->n, problem->nnz, problem->bits, problem->policy));
+        if (plan.digits != 0) {
+            const cb200_status st = build_digit_words(view_of(*problem->device_matrix), p->arena, stream, &p->digits);
+            if (st != CB200_STATUS_SUCCESS) return abandon(st);
+            p->digit_slices = plan.digits;
+            p->schedule_name = plan.digits == 4 ? "gene_gather" : "tensor_blocked_x3";
+            p->workspace_bytes = qcsr_transpose_digits_workspace_bytes(problem->m, problem->k, problem->n, plan.digits);
+            p->workspace_required = qcsr_transpose_digits_least_workspace(problem->m, problem->k, problem->n, plan.digits, p->sm_count);
+            p->persistent_bytes += p->digits.bytes;
+        }
         if (plan.gene_gather) {
             const cb200_status st = build_gene_major_layout(view_of(*problem->device_matrix), p->arena, stream, &p->gene_major);
             if (st != CB200_STATUS_SUCCESS) return abandon(st);
@@ -648,7 +676,7 @@ cb200_status cb200_spmm_prepare(const cb200_spmm_problem *problem, cb200_prepare
     const bool gathers = problem->projection == CB200_PROJECTION_CSR && p->schedule == fwd_schedule::warp_per_row;
     if (p->workspace_required == 0u) p->workspace_required = gathers ? std::min<std::uint64_t>(p->workspace_bytes, 256u) : p->workspace_bytes;
     // the fp32-FMA transpose runs without any: entries are then added one by one instead of sorted first
-    if (problem->projection == CB200_PROJECTION_TRANSPOSE && !plan.gene_gather && !plan.blocked) p->workspace_required = 0u;
+    if (problem->projection == CB200_PROJECTION_TRANSPOSE && !plan.gene_gather && !plan.blocked && plan.digits == 0) p->workspace_required = 0u;
     *out = p;
     return CB200_STATUS_SUCCESS;
 }
@@ -710,7 +738,7 @@ cb200_status cb200_spmm_run(const cb200_prepared *prepared, const cb200_launch *
     /* lifetimes.hh:160-172: the expected generation of a bound value plane must be the live one; here the
      * "live" values of a prepared copy are those it was built from */
     if ((prepared->blocked.seg_ptr != nullptr || prepared->blocked.dense_tiles != nullptr || prepared->blocked.code_tiles != nullptr ||
-         prepared->gene_major.col_ptr != nullptr) &&
+         prepared->gene_major.col_ptr != nullptr || prepared->digits.words != nullptr) &&
         pr.value_generation != 0u &&
         launch->value_generation != 0u && launch->value_generation != pr.value_generation)
         return fail(CB200_STATUS_STALE_VALUE, "the prepared operation keeps a copy of value generation %llu, the launch binds %llu",
@@ -764,7 +792,7 @@ cb200_status cb200_spmm_run(const cb200_prepared *prepared, const cb200_launch *
         return launch_qcsr_transpose_gather(view_of(x), d, row_begin, row_end, prepared->gene_major, launch->workspace,
                                             launch->workspace_bytes, prepared->sm_count, stream);
     if (pr.projection == CB200_PROJECTION_TRANSPOSE)
-        return launch_qcsr_transpose(view_of(x), d, row_begin, row_end, &prepared->blocked, pr.multiply != CB200_DTYPE_BF16,
+        return launch_qcsr_transpose(view_of(x), d, row_begin, row_end, &prepared->blocked, &prepared->digits, prepared->digit_slices, pr.multiply != CB200_DTYPE_BF16,
                                      launch->workspace, launch->workspace_bytes, prepared->sm_count, stream);
     return launch_qcsr_forward(view_of(x), d, row_begin, row_end, prepared->schedule, prepared->row_order, &prepared->blocked,
                                pr.multiply != CB200_DTYPE_BF16, launch->workspace, launch->workspace_bytes, prepared->sm_count,

@@ -202,10 +202,33 @@ cb200_status launch_qcsr_transpose_blocked(const qcsr_view &x, const dense_args 
                                            const blocked_layout &layout, bool split_products, int sm_count,
                                            cudaStream_t stream, bool *taken);
 
+// Transpose with exact integer sums on the tensor cores (zero-points per gene): codes times the digits of G in fixed point.
+// slices: digits of G, 3 (products as exact as three bf16 ones) or 4 (as fp32 ones).
+// The entries in pieces of 32 cells, by window of 128 genes; scales and zero-points are read at launch.
+struct digit_layout {
+    std::uint32_t *words = nullptr;
+    std::uint32_t *bounds = nullptr; // [pieces][windows + 1]
+    std::int64_t *bases = nullptr;   // [pieces]
+    std::uint64_t bytes = 0;
+    const void *src_row_ptr = nullptr, *src_col_idx = nullptr, *src_packed = nullptr; // arrays it was built from
+};
+bool qcsr_transpose_digits_shape_ok(std::int64_t rows, std::int64_t cols, std::int64_t n, int bits, int policy);
+std::uint64_t qcsr_digit_words_bytes_bound(std::int64_t rows, std::int64_t cols, std::int64_t nnz);
+// current device; memory from `arena`, kernels on `stream`, which is waited for
+cb200_status build_digit_words(const qcsr_view &x, device_arena &arena, cudaStream_t stream, digit_layout *out);
+std::uint64_t qcsr_transpose_digits_workspace_bytes(std::int64_t rows, std::int64_t cols, std::int64_t n, int slices);
+std::uint64_t qcsr_transpose_digits_least_workspace(std::int64_t rows, std::int64_t cols, std::int64_t n, int slices, int sm_count); // slower
+// Whether a call that sees its matrix once should make the words in its workspace (0: no), and what it then needs
+std::uint64_t qcsr_transpose_digits_once_bytes(std::int64_t rows, std::int64_t cols, std::int64_t n, std::int64_t nnz, int bits, int policy);
+// layout null: the words are made in the workspace.  *taken is false where the shape or the workspace rules it out.
+cb200_status launch_qcsr_transpose_digits(const qcsr_view &x, const dense_args &d, std::int64_t row_begin, std::int64_t row_end, void *workspace,
+                                          std::uint64_t workspace_bytes, const digit_layout *layout, int slices, int sm_count, cudaStream_t stream, bool *taken);
+
 // G'[g,:] = alpha * sum_{r in range, col_i == g} deq(code_i) * G[r,:] + beta * G'[g,:]
-// `blocked` (optional): the window-blocked copy of a prepared bf16-product operation.
+// `blocked` (optional): the window-blocked copy of a prepared bf16-product operation.  `digits` (optional): the words of a prepared
+// operation with fp32 products, and how many digits of G it takes.
 cb200_status launch_qcsr_transpose(const qcsr_view &x, const dense_args &d, std::int64_t row_begin,
-                                   std::int64_t row_end, const blocked_layout *blocked, bool split_products,
+                                   std::int64_t row_end, const blocked_layout *blocked, const digit_layout *digits, int slices, bool split_products,
                                    void *workspace, std::uint64_t workspace_bytes, int sm_count, cudaStream_t stream);
 // What the fp32-FMA transpose can use, 32 MB at most; with less it takes the rows in smaller slices, and without it every
 // entry is added in L2 on its own.

@@ -163,10 +163,19 @@ std::uint64_t qcsr_transpose_workspace_bytes(std::int64_t rows, std::int64_t col
 }
 
 cb200_status launch_qcsr_transpose(const qcsr_view &x, const dense_args &d, std::int64_t row_begin,
-                                   std::int64_t row_end, const blocked_layout *blocked, bool split_products,
+                                   std::int64_t row_end, const blocked_layout *blocked, const digit_layout *digits, int slices, bool split_products,
                                    void *workspace, std::uint64_t workspace_bytes, int sm_count, cudaStream_t stream) {
     if (d.n == 0 || x.cols == 0) return CB200_STATUS_SUCCESS;
     if (d.dense_dtype != CB200_DTYPE_F32) return fail(CB200_STATUS_UNSUPPORTED, "transpose takes an fp32 dense operand");
+    const bool prepared_words = digits != nullptr && digits->words != nullptr;
+    const std::int64_t part_nnz = x.rows > 0 ? static_cast<std::int64_t>(static_cast<double>(x.nnz) * static_cast<double>(row_end - row_begin) / static_cast<double>(x.rows)) : 0;
+    const bool copied = prepared_words || (blocked != nullptr && blocked->seg_ptr != nullptr);
+    if (prepared_words || (!copied && qcsr_transpose_digits_once_bytes(row_end - row_begin, x.cols, d.n, part_nnz, x.bits, x.policy) != 0u)) {
+        bool taken = false;
+        const cb200_status st = launch_qcsr_transpose_digits(x, d, row_begin, row_end, workspace, workspace_bytes, prepared_words ? digits : nullptr,
+                                                             prepared_words ? slices : 4, sm_count, stream, &taken);
+        if (st != CB200_STATUS_SUCCESS || taken) return st;
+    }
     if (blocked != nullptr && blocked->seg_ptr != nullptr) {
         bool taken = false;
         const cb200_status st = launch_qcsr_transpose_blocked(x, d, row_begin, row_end, workspace, workspace_bytes, *blocked,

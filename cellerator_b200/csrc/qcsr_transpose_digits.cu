@@ -1,0 +1,1176 @@
+// Gene-side transpose with exact integer sums on the tensor cores:
+//     G'[genes, N] = alpha * deq(X)^T[genes, cells] * G[cells, N] + beta * G',   zero-points per gene.
+//
+// Reference counterpart: csr_spmm_bwd_rhs_kernel_ (src/compute/sparse/ops/kernels/base_sparse/csr_spmm_bwd_rhs_kernel_.cuh:1-22),
+// one atomicAdd per (stored entry, output column).
+//
+// Formulation.  The stored value of (cell, gene) is scale * code + offset with scale and offset of the gene, so
+//     G'[gene] = scale * (sum over cells of code * G[cell]) + offset * (sum over the gene's cells of G[cell]).
+// Both sums have whole numbers on the matrix's side: the codes, and ones.  A column of G is written in fixed point, to 8 S - 1 bits below
+// its largest magnitude, as S signed digits of base 256 (S = 4: rounded at 2^-31 of the largest; S = 3: at 2^-23).  Codes
+// (less 128, to be signed) and digits are what the tensor cores' 8-bit integer MMAs multiply, and these add in 32 bits without
+// rounding: every product and every sum up to the end of a run is exact, whatever their order.  The only errors are the rounding
+// of G to its fixed point and a handful of fp32 roundings at the end.  Against 64 bits (2-norm, genes of the 33,538-gene
+// matrices): S = 4 4e-8, where fp32 FMAs leave 1.2e-7 (8,191 cells) to 4.8e-7 (100,003 cells, in a fixed order); S = 3 2e-7, where
+// products put together from three bf16 products and summed by the fp32 MMAs leave 6.2e-6.
+//
+// A column whose largest magnitude is more than 64 times its root mean square, or that holds an infinity or a NaN, would lose
+// bits (or everything) in fixed point: the launch then takes the entries one by one, in double precision and in a fixed order
+// (finish_kernel).  So does a matrix in which a cell holds a gene twice.  The device decides; nothing is read back.
+//
+// Data.  The entries lie in pieces of 32 cells; inside a piece they are ordered by window of 128 genes, one word per entry
+// {code, place in the operand tile}, cell after cell (digit_words_kernel: a CTA per piece counts the entries of each cell and window in
+// shared memory, adds them up, and places the words; no atomics between CTAs, the same words on every run).
+// A prepared operation keeps the words; a call that sees its matrix once makes them in its workspace.
+//
+// Structure of the main kernel (640 threads, one CTA per SM): warps 0-15 in two groups of eight on alternate tiles zero a tile
+// of 256 cells x 128 genes (32 KB of codes, 32 KB of ones, K-major with the 128-byte swizzle) and scatter its words; warp 16
+// issues the MMAs (M = genes, K = cells, N = S digits x the columns of G); warp 18 feeds the ring of G; warps 17 and 19 the
+// words, each to one of the groups.  The two sums of a window take 2 S N columns of tensor memory, all 512 at S = 4, N = 64, and stay there while
+// the CTA walks the groups of its run.  Every wait is bounded (sm100_primitives.cuh).
+//
+// What bounds it: at S = 4, N = 64 the tensor pipe, sixteen 128 x 256 x 32 MMAs of 128 cycles in the 2,410 cycles of a tile; at S = 3
+// the scatter groups' chain (release, zeroes, two one-byte stores a word, fence, hand-over), 2,125 cycles against 1,536 of MMAs; over a
+// second of launches the power cap (1.6 GHz).  One B200, start of this kernel's life -> now: 125,000 x 33,538, N = 64, S = 3 1,645 (bf16
+// products) -> 1,186 us; 100,003 cells, S = 4 2,879 (rows of G gathered gene by gene) -> 1,087; 8,191 cells, S = 4 with the words made in
+// the call 313 (sorted in shared memory) -> 171.
+#include "dependent_launch.cuh"
+#include "kernels.cuh"
+#include "sm100_primitives.cuh"
+
+#include <algorithm>
+
+namespace cb200 {
+namespace {
+
+constexpr int kWin = 128;                       // genes per window
+constexpr int kRows = 256;                      // cells per group
+constexpr int kPieceRows = 32;                  // cells whose words one CTA lays out
+constexpr int kGroupPieces = kRows / kPieceRows;
+constexpr int kBuildThreads = 768;
+constexpr int kBuildWarps = kBuildThreads / 32;
+constexpr int kBuildSteps = 8;                  // reads of 32 entries in flight per warp
+constexpr std::uint32_t kPadding = 0x80000000u; // a word that holds no entry
+
+constexpr int kProducerWarps = 16;
+constexpr int kProducerThreads = kProducerWarps * 32;
+constexpr int kGroupThreads = kProducerThreads / 2;
+constexpr int kThreads = kProducerThreads + 4 * 32;
+constexpr int kPlaneBytes = kWin * kRows;       // 32 KB: [cell half][gene][128 cells], a byte each
+constexpr int kTileBytes = 2 * kPlaneBytes;     // codes, then ones
+constexpr int kGPieceRows = 64;                 // G comes in pieces of 64 cells, four per group
+constexpr int kGPieces = kRows / kGPieceRows;
+constexpr int kChunkEntries = 2048;
+constexpr int kChunkBytes = kChunkEntries * 4;
+constexpr int kMaxCtas = 256;
+// |code - 128| <= 128 and |digit| <= 128: 2^31 / 2^14 cells until a sum could leave 32 bits
+constexpr std::int64_t kRunGroups = (1 << 17) / kRows - 1;
+
+// digits x columns of one MMA, windows whose sums fit in tensor memory, pieces in the ring of G
+__host__ __device__ constexpr int mma_columns(int nb, int slices) { return nb * slices; }
+__host__ __device__ constexpr int set_windows(int nb, int slices) { return 512 / (2 * mma_columns(nb, slices)); }
+__host__ __device__ constexpr int g_piece_bytes(int nb, int slices) { return kGPieceRows * mma_columns(nb, slices); }
+__host__ __device__ constexpr int ring_pieces(int nb, int slices) { return mma_columns(nb, slices) >= 256 ? 5 : mma_columns(nb, slices) >= 192 ? 6 : 8; }
+
+// workspace: status block {status, wide, ...}, largest magnitudes and sums of squares of the columns in parts, steps of the
+// columns, G in digits, sums of the runs, and for a call that sees its matrix once the words
+constexpr int kParts = 48;
+constexpr int kMaxColumns = 256;
+constexpr std::uint64_t kStepsAt = 256, kPartMaxAt = kStepsAt + kMaxColumns * 8, kPartSquareAt = kPartMaxAt + kParts * kMaxColumns * 4,
+                        kRecordsAt = kPartSquareAt + kParts * kMaxColumns * 8;
+static_assert(kParts % 48 == 0, "six at a time on up to eight lanes");
+static_assert(kRecordsAt % 256 == 0, "G's records are copied 16 bytes at a time");
+
+// A call that sees its matrix once and holds more entries adds them in shared memory (qcsr_transpose_tiled.cu), in 32 MB of workspace:
+// the words of this many take 200 MB.
+constexpr std::int64_t kMostOnceEntries = 50'000'000, kLeastOnceEntries = 2'000'000;
+
+// ---- the words -----------------------------------------------------------------------------------------------------------
+
+struct words_params {
+    const std::int64_t *row_ptr;
+    const std::int64_t *packed_row_ptr;
+    const std::int32_t *col_idx;
+    const std::uint8_t *packed;
+    std::int64_t row_begin, row_end, cols;
+    int windows, code_bias;
+    std::uint32_t *words;
+    std::uint32_t *bounds; // [pieces][windows + 1], from the piece's base
+    std::int64_t *bases;   // [pieces]; kTwice: a cell of the piece holds a gene more than once
+    int *status;           // cleared, where given
+};
+constexpr std::int64_t kTwice = 1ll << 62;
+
+// A CTA's cells are one stretch of the CSR arrays, which its warps take 256 entries at a time whatever cells they belong to (rows
+// are of very different lengths: a warp per row took 240 us for 8,191 x 33,538 with 14.7 M entries, this takes 59).  Where genes ascend,
+// an entry starts a window if the one before it lies in another; from those starts follow the sizes, the places of the windows and
+// so the place of every entry, without an atomic, which the second pass computes from a look-up per entry.  A CTA that finds a gene
+// outside the matrix or not above the one before it counts and places entry by entry with atomics instead, and looks for genes that a cell
+// holds twice: a tile has one place for them.
+//
+// What bounds it: the latency of the genes' loads (eight in flight per warp, 48 warps per SM) and issue, half of the slots.
+template<int BITS>
+__global__ void __launch_bounds__(kBuildThreads) digit_words_kernel(const words_params p) {
+    extern __shared__ std::uint32_t place_of[]; // [kPieceRows][pitch]; see below
+    __shared__ std::int64_t codes_of[kPieceRows]; // where the codes of a cell begin
+    __shared__ int cell_start[kPieceRows + 1];    // from the CTA's first entry
+    __shared__ std::uint32_t cell_bits[kPieceRows]; // of the words of a cell
+    __shared__ std::uint32_t warp_sums[kBuildWarps];
+    __shared__ std::uint32_t carry;
+    __shared__ int irregular;
+    constexpr std::uint32_t kNone = 0xffffffffu;
+    const int tid = threadIdx.x, lane = tid & 31, warp = warp_of_block(), pitch = p.windows;
+    const std::int64_t row0 = p.row_begin + static_cast<std::int64_t>(blockIdx.x) * kPieceRows;
+    const int cells = static_cast<int>(min(static_cast<std::int64_t>(kPieceRows), p.row_end - row0));
+    let_next_launch_start();
+    if (p.status != nullptr && blockIdx.x == 0 && tid == 0) *p.status = 0;
+    const std::int64_t first = __ldg(p.row_ptr + row0);
+    if (tid <= cells) {
+        const std::int64_t at = __ldg(p.row_ptr + row0 + tid);
+        cell_start[tid] = static_cast<int>(at - first);
+        if (tid < cells) {
+            const std::uint32_t cell = (blockIdx.x * kPieceRows + tid) & (kRows - 1);
+            codes_of[tid] = p.packed_row_ptr != nullptr ? __ldg(p.packed_row_ptr + row0 + tid) : at;
+            cell_bits[tid] = ((cell >> 7) * (kPlaneBytes / 2) + ((cell & 127u) >> 4 << 4) + (cell & 15u)) << 8 | static_cast<std::uint32_t>(p.code_bias);
+        }
+    }
+    for (int i = tid; i < kPieceRows * pitch; i += kBuildThreads) place_of[i] = kNone;
+    if (tid == 0) {
+        carry = 0u;
+        irregular = 0;
+    }
+    __syncthreads();
+    const std::int32_t *genes = p.col_idx + first;
+    const std::int64_t base = ((first - __ldg(p.row_ptr + p.row_begin) + 3) & ~static_cast<std::int64_t>(3)) + static_cast<std::int64_t>(blockIdx.x) * (4 * p.windows + 4);
+    std::uint32_t *out = p.words + base;
+
+    // Work is dealt to the warps in pieces of up to 256 entries of one cell.  A lane holds what its cell needs: the number of the
+    // cell's first piece, where its entries begin, how many they are.
+    const int my_begin = cell_start[min(lane, cells)], my_length = lane < cells ? cell_start[lane + 1] - my_begin : 0;
+    const int my_pieces = (my_length + 32 * kBuildSteps - 1) / (32 * kBuildSteps);
+    int my_first = my_pieces;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const int below = __shfl_up_sync(0xffffffffu, my_first, d);
+        if (lane >= d) my_first += below;
+    }
+    const int items = __shfl_sync(0xffffffffu, my_first, 31);
+    my_first -= my_pieces;
+    struct piece { int cell, begin, at, length; }; // begin: the cell's first entry, at: the piece's, in the cell
+    const auto piece_at = [&](int item) {
+        const int r = 31 - __clz(__ballot_sync(0xffffffffu, my_first <= item));
+        return piece{r, __shfl_sync(0xffffffffu, my_begin, r), (item - __shfl_sync(0xffffffffu, my_first, r)) * (32 * kBuildSteps), __shfl_sync(0xffffffffu, my_length, r)};
+    };
+
+    // ---- the first entry of each (cell, window): place_of[cell][window] = its place among the cell's ----
+    {
+        bool odd = false;
+        for (int item = warp; item < items; item += kBuildWarps) {
+            const piece w = piece_at(item);
+            const std::int32_t *from = genes + w.begin + w.at + lane;
+            const int left = w.length - w.at; // of the cell, from the piece on
+            std::uint32_t *mine = place_of + w.cell * pitch;
+            int gene[kBuildSteps];
+#pragma unroll
+            for (int u = 0; u < kBuildSteps; ++u) gene[u] = u * 32 + lane < left ? __ldg(from + u * 32) : 0;
+            int before = w.at > 0 ? __ldg(genes + w.begin + w.at - 1) : -1;
+#pragma unroll
+            for (int u = 0; u < kBuildSteps; ++u) {
+                if (u * 32 >= left) break;
+                int last = __shfl_up_sync(0xffffffffu, gene[u], 1);
+                if (lane == 0) last = before;
+                before = __shfl_sync(0xffffffffu, gene[u], 31);
+                const bool valid = u * 32 + lane < left, inside = static_cast<unsigned>(gene[u]) < static_cast<unsigned>(p.cols) && last < gene[u];
+                odd = odd || (valid && !inside);
+                if (valid && inside && static_cast<unsigned>(last ^ gene[u]) >= kWin) mine[gene[u] >> 7] = static_cast<std::uint32_t>(w.at + u * 32 + lane);
+            }
+        }
+        if (odd) irregular = 1;
+    }
+    __syncthreads();
+    const bool ordered = irregular == 0;
+    const auto each_entry = [&](auto &&f) { // f(cell, gene, place among the cell's)
+        for (int r = warp; r < cells; r += kBuildWarps)
+            for (int e = cell_start[r] + lane; e < cell_start[r + 1]; e += 32) {
+                const int gene = __ldg(genes + e);
+                if (static_cast<unsigned>(gene) < static_cast<unsigned>(p.cols)) f(r, gene, e - cell_start[r]);
+            }
+    };
+    const auto word_of = [&](std::uint32_t bits, int gene, std::uint32_t code) {
+        // {code less the bias, place in the tile << 8}: plane half, gene, 16-byte piece of the gene's line ^ gene % 8, byte
+        return bits ^ (static_cast<std::uint32_t>(gene & (kWin - 1)) << 15 | static_cast<std::uint32_t>(gene & 7) << 12) ^ code;
+    };
+    const auto code_at = [&](int r, int i) -> std::uint32_t {
+        if constexpr (BITS == 8) return __ldg(p.packed + codes_of[r] + i);
+        const std::uint32_t byte = __ldg(p.packed + codes_of[r] + (i >> 1));
+        return (i & 1) != 0 ? byte >> 4 : byte & 0xfu;
+    };
+    if (ordered) {
+        // windows a cell has no entry in start where the next one does; then {entries << 24 | place of the first}
+        for (int r = warp; r < cells; r += kBuildWarps) {
+            std::uint32_t follow = static_cast<std::uint32_t>(cell_start[r + 1] - cell_start[r]);
+            for (int w0 = (p.windows - 1) & ~31; w0 >= 0; w0 -= 32) {
+                std::uint32_t v = w0 + lane < p.windows ? place_of[r * pitch + w0 + lane] : kNone;
+#pragma unroll
+                for (int d = 1; d < 32; d <<= 1) v = min(v, __shfl_down_sync(0xffffffffu, v, d)); // the lanes past the end give their own
+                v = min(v, follow);
+                std::uint32_t up = __shfl_down_sync(0xffffffffu, v, 1);
+                if (lane == 31) up = follow;
+                if (w0 + lane < p.windows) place_of[r * pitch + w0 + lane] = (up - v) << 24 | v;
+                follow = __shfl_sync(0xffffffffu, v, 0);
+            }
+        }
+    } else {
+        for (int i = tid; i < kPieceRows * pitch; i += kBuildThreads) place_of[i] = 0u;
+        __syncthreads();
+        each_entry([&](int r, int gene, int) { atomicAdd(place_of + r * pitch + (gene >> 7), 1u); });
+    }
+    __syncthreads();
+    // the places: window after window, inside a window cell after cell; a window's words are padded to a multiple of four
+    for (int w0 = 0; w0 < p.windows; w0 += kBuildThreads) {
+        const int w = w0 + tid;
+        std::uint32_t total = 0u;
+        if (w < p.windows) {
+#pragma unroll 8
+            for (int r = 0; r < cells; ++r) total += ordered ? place_of[r * pitch + w] >> 24 : place_of[r * pitch + w];
+        }
+        const std::uint32_t padded = (total + 3u) & ~3u;
+        std::uint32_t upto = padded;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const std::uint32_t below = __shfl_up_sync(0xffffffffu, upto, d);
+            if (lane >= d) upto += below;
+        }
+        if (lane == 31) warp_sums[warp] = upto;
+        __syncthreads();
+        std::uint32_t start = carry + upto - padded;
+        for (int k = 0; k < warp; ++k) start += warp_sums[k];
+        __syncthreads();
+        if (tid == kBuildThreads - 1) carry = start + padded;
+        if (w < p.windows) {
+            p.bounds[static_cast<std::int64_t>(blockIdx.x) * (p.windows + 1) + w] = start;
+            std::uint32_t place = start;
+#pragma unroll 8
+            for (int r = 0; r < cells; ++r) { // ordered: what to add to an entry's place in its cell; otherwise the next free place
+                const std::uint32_t v = place_of[r * pitch + w];
+                place_of[r * pitch + w] = ordered ? place - (v & 0xffffffu) : place;
+                place += ordered ? v >> 24 : v;
+            }
+            for (; place < start + padded; ++place) out[place] = kPadding;
+        }
+        __syncthreads();
+    }
+    if (tid == 0) {
+        p.bounds[static_cast<std::int64_t>(blockIdx.x) * (p.windows + 1) + p.windows] = carry;
+        p.bases[blockIdx.x] = base;
+    }
+    if (!ordered) {
+        __shared__ std::uint32_t seen_of[kBuildWarps][kWin]; // a window's (gene, cell)
+        each_entry([&](int r, int gene, int i) { out[atomicAdd(place_of + r * pitch + (gene >> 7), 1u)] = word_of(cell_bits[r], gene, code_at(r, i)); });
+        __syncthreads();
+        std::uint32_t *seen = seen_of[warp];
+        bool twice = false;
+        const std::uint32_t *bounds = p.bounds + static_cast<std::int64_t>(blockIdx.x) * (p.windows + 1);
+        for (int w = warp; w < p.windows; w += kBuildWarps) {
+            for (int i = lane; i < kWin; i += 32) seen[i] = 0u;
+            __syncwarp();
+            for (std::uint32_t i = bounds[w] + lane; i < bounds[w + 1]; i += 32) {
+                const std::uint32_t e = out[i];
+                if (static_cast<int>(e) < 0) continue;
+                const std::uint32_t gl = (e >> 15) & (kWin - 1), cell = ((((e >> 12) ^ gl) & 7u) << 4 | ((e >> 8) & 15u)) & (kPieceRows - 1);
+                twice = twice || (atomicOr(seen + gl, 1u << cell) >> cell & 1u) != 0u;
+            }
+            __syncwarp();
+        }
+        if (__syncthreads_or(twice ? 1 : 0) != 0 && tid == 0) p.bases[blockIdx.x] = base | kTwice;
+        return;
+    }
+    for (int item = warp; item < items; item += kBuildWarps) {
+        const piece w = piece_at(item);
+        const std::int32_t *from = genes + w.begin + w.at + lane;
+        const std::uint8_t *codes = p.packed + codes_of[w.cell] + (BITS == 8 ? w.at + lane : (w.at + lane) >> 1); // (pieces begin at even entries)
+        const int left = w.length - w.at;
+        const std::uint32_t *mine = place_of + w.cell * pitch;
+        const std::uint32_t bits = cell_bits[w.cell];
+        std::uint32_t *dst = out + w.at + lane; // place_of is what to add to an entry's place in its cell: it can be negative
+        int gene[kBuildSteps];
+        std::uint32_t code[kBuildSteps];
+#pragma unroll
+        for (int u = 0; u < kBuildSteps; ++u) {
+            const bool valid = u * 32 + lane < left;
+            gene[u] = valid ? __ldg(from + u * 32) : 0;
+            code[u] = valid ? __ldg(codes + (BITS == 8 ? u * 32 : u * 16)) : 0u;
+        }
+#pragma unroll
+        for (int u = 0; u < kBuildSteps; ++u) {
+            if (u * 32 + lane >= left) break;
+            std::uint32_t c = code[u];
+            if constexpr (BITS == 4) c = (lane & 1) != 0 ? c >> 4 : c & 0xfu;
+            dst[static_cast<std::int32_t>(mine[gene[u] >> 7]) + u * 32] = word_of(bits, gene[u], c);
+        }
+    }
+}
+
+// ---- G in digits -----------------------------------------------------------------------------------------------------------
+
+// Largest magnitude (as bits; an infinity or a NaN is the largest) and sum of squares of each column, in kParts parts.  HBM or L2.
+__global__ void __launch_bounds__(1024) column_range_kernel(const float *g, std::int64_t ld, int n, int padded, std::int64_t row_begin, std::int64_t row_end,
+                                                            unsigned *part_max, double *part_square, int *status) {
+    __shared__ unsigned most_of[1024];
+    __shared__ double square_of[1024];
+    let_next_launch_start();
+    if (status != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *status = 0;
+    const int c = threadIdx.x % padded, lanes = 1024 / padded;
+    unsigned most = 0u;
+    double square = 0.0;
+    if (c < n) {
+        const std::int64_t step = static_cast<std::int64_t>(gridDim.x) * lanes;
+        std::int64_t r = row_begin + static_cast<std::int64_t>(blockIdx.x) * lanes + threadIdx.x / padded;
+        const float *at = g + r * ld + c;
+        const auto take = [&](float v) {
+            most = max(most, __float_as_uint(v) & 0x7fffffffu);
+            square = fma(static_cast<double>(v), static_cast<double>(v), square);
+        };
+        for (; r + 7 * step < row_end; r += 8 * step, at += 8 * step * ld) {
+            float v[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) v[k] = __ldg(at + k * step * ld);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) take(v[k]);
+        }
+        for (; r < row_end; r += step, at += step * ld) take(__ldg(at));
+    }
+    most_of[threadIdx.x] = most;
+    square_of[threadIdx.x] = square;
+    __syncthreads();
+    if (threadIdx.x < static_cast<unsigned>(padded)) {
+        for (int k = 1; k < lanes; ++k) {
+            most = max(most, most_of[threadIdx.x + k * padded]);
+            square += square_of[threadIdx.x + k * padded];
+        }
+        part_max[blockIdx.x * kMaxColumns + threadIdx.x] = most;
+        part_square[blockIdx.x * kMaxColumns + threadIdx.x] = square;
+    }
+    // beside digit_words_kernel in a call that makes its words: what waits for this kernel waits for that one too
+    wait_for_previous_launch();
+}
+
+// G -> per (block of NB columns, group of 256 cells) a record of four pieces of 64 cells, each the S NB x 64 digits in the no-swizzle
+// K-major operand layout (byte of (column k NB + c: digit k of column c, the highest first; cell r) = column / 8 * 512 + r / 16 *
+// 128 + column % 8 * 16 + r % 16).  Cells outside [row_begin, row_end) and columns from n on are zero.
+// Every block adds the parts up for itself; the first one writes the columns' steps and whether the entries have to be taken one by one.
+template<int NB, int SLICES>
+__global__ void __launch_bounds__(256) pack_digits_kernel(const float *g, std::int64_t ld, int n, int padded, std::int64_t first_row, std::int64_t row_begin,
+                                                          std::int64_t row_end, std::int64_t groups, const unsigned *part_max, const double *part_square,
+                                                          double *steps, unsigned char *records, const std::int64_t *bases, std::int64_t word_pieces, int *wide) {
+    __shared__ unsigned most_of[256];
+    __shared__ double square_of[256];
+    __shared__ double factor[kMaxColumns]; // 2^k: what a column is multiplied by
+    wait_for_previous_launch();
+    let_next_launch_start();
+    const int tid = threadIdx.x;
+    {
+        const int c = tid % padded, lanes = 256 / padded;
+        unsigned most = 0u;
+        double square = 0.0;
+        for (int k0 = tid / padded; k0 < kParts; k0 += 6 * lanes) { // lanes 1, 2, 4, 8: six loads of each kind in flight
+            unsigned m[6];
+            double q[6];
+#pragma unroll
+            for (int k = 0; k < 6; ++k) {
+                m[k] = __ldcg(part_max + (k0 + k * lanes) * kMaxColumns + c);
+                q[k] = __ldcg(part_square + (k0 + k * lanes) * kMaxColumns + c);
+            }
+#pragma unroll
+            for (int k = 0; k < 6; ++k) {
+                most = max(most, m[k]);
+                square += q[k];
+            }
+        }
+        most_of[tid] = most;
+        square_of[tid] = square;
+        __syncthreads();
+        int too_wide = 0;
+        if (tid < padded) {
+            for (int k = 1; k < lanes; ++k) {
+                most = max(most, most_of[tid + k * padded]);
+                square += square_of[tid + k * padded];
+            }
+            double f = 0.0, step = 0.0;
+            if (most >= 0x7f800000u) {
+                too_wide = 1;
+            } else if (most != 0u) {
+                const double largest = static_cast<double>(__uint_as_float(most));
+                // largest = m 2^e, m in [0.5, 1); the largest number of S balanced digits is 0.996 * 2^(8 S - 1)
+                const int e = most >= 0x800000u ? static_cast<int>(most >> 23) - 126 : 32 - __clz(most) - 149;
+                const int k = 8 * SLICES - 1 - e - ((most & 0x7fffffu) > 8220000u || most < 0x800000u ? 1 : 0);
+                f = __longlong_as_double(static_cast<long long>(1023 + k) << 52);
+                step = __longlong_as_double(static_cast<long long>(1023 - k) << 52);
+                too_wide = largest * largest * static_cast<double>(row_end - row_begin) > 4096.0 * square ? 1 : 0;
+            }
+            factor[tid] = f;
+            if (blockIdx.x == 0) steps[tid] = step;
+        }
+        if (blockIdx.x == 0) {
+#pragma unroll 8
+            for (std::int64_t k = tid; k < word_pieces; k += 256) too_wide |= (__ldcg(bases + k) & kTwice) != 0 ? 1 : 0;
+        }
+        too_wide = __syncthreads_or(too_wide);
+        if (blockIdx.x == 0 && tid == 0) *wide = too_wide;
+    }
+    constexpr int NC = mma_columns(NB, SLICES);
+    const std::int64_t pieces = static_cast<std::int64_t>((n + NB - 1) / NB) * groups * kGPieces;
+    for (std::int64_t b = blockIdx.x; b < pieces; b += gridDim.x) {
+        const int c0 = static_cast<int>(b / (groups * kGPieces)) * NB;
+        const std::int64_t row0 = first_row + b % (groups * kGPieces) * kGPieceRows;
+        unsigned char *rec = records + b * (kGPieceRows * NC);
+        for (int item = tid; item < NB * (kGPieceRows / 16); item += 256) {
+            const int c = item % NB, r16 = item / NB;
+            const double f = c0 + c < n ? factor[c0 + c] : 0.0;
+            float v[16];
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+                const std::int64_t row = row0 + r16 * 16 + j;
+                v[j] = row >= row_begin && row < row_end && c0 + c < n ? __ldg(g + row * ld + c0 + c) : 0.0f;
+            }
+            std::uint32_t digit[SLICES][4];
+#pragma unroll
+            for (int k = 0; k < SLICES; ++k)
+#pragma unroll
+                for (int w = 0; w < 4; ++w) digit[k][w] = 0u;
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+                int q = __double2int_rn(static_cast<double>(v[j]) * f);
+#pragma unroll
+                for (int k = SLICES - 1; k >= 0; --k) {
+                    digit[k][j >> 2] |= (static_cast<std::uint32_t>(q) & 0xffu) << ((j & 3) * 8);
+                    q = (q - static_cast<int>(static_cast<signed char>(q & 0xff))) >> 8;
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < SLICES; ++k) {
+                const int column = k * NB + c;
+                *reinterpret_cast<uint4 *>(rec + (column >> 3) * 512 + r16 * 128 + (column & 7) * 16) =
+                    make_uint4(digit[k][0], digit[k][1], digit[k][2], digit[k][3]);
+            }
+        }
+    }
+}
+
+// ---- the sums --------------------------------------------------------------------------------------------------------------
+
+struct digit_params {
+    const std::uint32_t *words;
+    const std::uint32_t *bounds;
+    const std::int64_t *bases;
+    std::int64_t pieces;
+    const float *scales, *offsets;
+    const unsigned char *records;
+    const double *steps;
+    const int *wide;
+    float *partials;         // [run_of + CTA][window of the set][gene][NB]
+    std::int64_t cols;
+    std::int64_t group_begin, group_count;
+    std::int64_t run_groups; // groups after which a run ends at the latest
+    int windows, column_blocks, code_bias;
+    int *status;
+    int poll_limit;          // test hook (cb200_test_arm_wait_timeout): the loader of G issues no copies and gives up after so many polls; 0: none
+};
+
+// Units (column block, window set, group), numbered in this order, are dealt to the CTAs in equal contiguous shares; a run is a CTA's
+// consecutive units of one set, cut every run_groups groups.  run_of numbers the runs of an undivided walk; the shares' borders cut them
+// further, and run_of + CTA is a number no two runs have.
+__host__ __device__ inline std::int64_t run_of(std::int64_t unit, std::int64_t groups, std::int64_t run_groups) {
+    return unit / groups * ((groups + run_groups - 1) / run_groups) + unit % groups / run_groups;
+}
+__device__ __forceinline__ std::int64_t run_end(std::int64_t u, std::int64_t u1, std::int64_t groups, std::int64_t run_groups) {
+    const std::int64_t gi = u % groups, last = min((gi / run_groups + 1) * run_groups, groups);
+    return min(u + (last - gi), u1);
+}
+// the CTA whose share [total b / grid, total (b + 1) / grid) holds a unit
+__device__ __forceinline__ std::int64_t cta_of(std::int64_t unit, std::int64_t total, std::int64_t grid) { return ((unit + 1) * grid - 1) / total; }
+// A walk over the units' tiles, without a division a tile.
+struct tile_cursor {
+    std::int64_t unit;
+    int group, set, wl, windows_of_set; // group: of the launch; set: of the column block
+    const int groups, sets, windows, per_set;
+    __device__ __forceinline__ int windows_in(int s) const { return min(per_set, windows - s * per_set); }
+    __device__ __forceinline__ tile_cursor(const digit_params &p, std::int64_t sets_, std::int64_t first, int per_set_)
+        : unit(first), group(static_cast<int>(first % p.group_count)), set(static_cast<int>(first / p.group_count % sets_)), wl(0), windows_of_set(0),
+          groups(static_cast<int>(p.group_count)), sets(static_cast<int>(sets_)), windows(p.windows), per_set(per_set_) {
+        windows_of_set = windows_in(set);
+    }
+    __device__ __forceinline__ void next() {
+        if (++wl < windows_of_set) return;
+        wl = 0;
+        ++unit;
+        if (++group < groups) return;
+        group = 0;
+        if (++set == sets) set = 0;
+        windows_of_set = windows_in(set);
+    }
+};
+// K-major operand, no swizzle (a piece of G): core matrices of 8 columns x 16 cells; the next 16 cells 128 bytes on, the next 8
+// columns 512.
+__device__ __forceinline__ std::uint64_t smem_desc_digits(std::uint32_t addr) {
+    std::uint64_t d = 0;
+    d |= static_cast<std::uint64_t>((addr & 0x3ffffu) >> 4);
+    d |= static_cast<std::uint64_t>(128u >> 4) << 16;
+    d |= static_cast<std::uint64_t>(static_cast<unsigned>(kGPieceRows * 8) >> 4) << 32;
+    d |= static_cast<std::uint64_t>(1) << 46; // descriptor version of this architecture
+    return d;
+}
+
+template<int NB, int SLICES>
+__global__ void __launch_bounds__(kThreads, 1) qcsr_transpose_digits_kernel(const digit_params p) {
+    constexpr int NC = mma_columns(NB, SLICES), kSet = set_windows(NB, SLICES), GPIECE = g_piece_bytes(NB, SLICES), kPieces = ring_pieces(NB, SLICES);
+    constexpr std::uint32_t IDESC = instr_desc_i8(NC);
+    extern __shared__ __align__(1024) unsigned char smem[];
+    unsigned char *chunk_base = smem + 2 * kTileBytes + kPieces * GPIECE;
+    std::uint64_t *a_full = reinterpret_cast<std::uint64_t *>(chunk_base + 2 * kChunkBytes); // [2] scatter warps -> MMA
+    std::uint64_t *a_empty = a_full + 2;           // [2] MMA commit -> scatter warps
+    std::uint64_t *c_full = a_empty + 2;           // [2] copy engine -> scatter warps (a chunk stage per scatter group)
+    std::uint64_t *c_empty = c_full + 2;           // [2] scatter warps -> loader
+    std::uint64_t *acc_full = c_empty + 2;         // MMA commit -> scatter warps
+    std::uint64_t *acc_empty = acc_full + 1;       // scatter warps -> MMA
+    std::uint64_t *mma_drain = acc_empty + 1;      // the MMA warp's own, used once, after an abort
+    std::uint64_t *g_full = mma_drain + 1;         // [kPieces]
+    std::uint64_t *g_empty = g_full + kPieces;     // [kPieces]
+    volatile int *chunk_meta = reinterpret_cast<volatile int *>(g_empty + kPieces); // [2]
+    std::uint32_t *tmem_slot = reinterpret_cast<std::uint32_t *>(const_cast<int *>(chunk_meta) + 2);
+    volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
+    volatile int *fills = reinterpret_cast<volatile int *>(tmem_slot + 2); // [3] of the ring of G and of the groups' chunk stages, once the loaders have ended
+    unsigned char *scratch_slot = reinterpret_cast<unsigned char *>(tmem_slot + 5); // where padding words go
+
+    const int tid = threadIdx.x, warp = warp_of_block(), lane = tid & 31;
+    const std::uint32_t smem0 = smem_addr(smem), grec0 = smem0 + 2 * kTileBytes, chunk0 = grec0 + kPieces * GPIECE;
+    if (tid == 0) {
+        for (int b = 0; b < 2; ++b) {
+            bar_init(smem_addr(a_full + b), kProducerWarps / 2);
+            bar_init(smem_addr(a_empty + b), 1);
+            bar_init(smem_addr(c_full + b), 1);
+            bar_init(smem_addr(c_empty + b), kProducerWarps / 2);
+        }
+        for (int s = 0; s < kPieces; ++s) {
+            bar_init(smem_addr(g_full + s), 1);
+            bar_init(smem_addr(g_empty + s), 1);
+        }
+        bar_init(smem_addr(acc_full), 1);
+        bar_init(smem_addr(acc_empty), kProducerWarps);
+        bar_init(smem_addr(mma_drain), 1);
+        *abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(tmem_slot)), "r"(512) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const std::uint32_t tmem_base = *tmem_slot;
+    wait_for_previous_launch();
+
+    const std::int64_t sets = (p.windows + kSet - 1) / kSet;
+    const std::int64_t total_units = sets * p.column_blocks * p.group_count;
+    const std::int64_t u0 = total_units * blockIdx.x / gridDim.x;
+    // a column that does not fit fixed point: nothing to do here, finish_kernel takes the entries one by one
+    const std::int64_t u1 = __ldcg(p.wide) != 0 ? u0 : total_units * (blockIdx.x + 1) / gridDim.x;
+
+    if (warp < kProducerWarps) {
+        // ================= zero, scatter, read back =================
+        const int grp = warp / (kProducerWarps / 2), gtid = tid - grp * kGroupThreads;
+        unsigned char *tile = smem + grp * kTileBytes;
+        const std::uint32_t chunk_full = smem_addr(c_full + grp), chunk_empty = smem_addr(c_empty + grp);
+        const uint4 *chunk = reinterpret_cast<const uint4 *>(chunk_base + grp * kChunkBytes);
+        std::uint32_t q = 0, qc = 0; // this group's tiles and chunks
+        int run = 0; // runs read back
+        const auto scatter = [&](std::uint32_t e) {
+            unsigned char *dst = static_cast<int>(e) >= 0 ? tile + ((e >> 8) & 0x7fffu) : scratch_slot;
+            dst[0] = static_cast<unsigned char>(e);
+            (static_cast<int>(e) >= 0 ? dst + kPlaneBytes : dst + 1)[0] = 1;
+        };
+        // End of a run: the digits' sums are put together.  TMEM lane = gene within the window; a warp reads the lane quarter its
+        // number allows, sixteen columns of one window.  `from` is the run's first unit, `to` the one behind its last.
+        const auto put_together = [&](std::int64_t from, std::int64_t to) {
+            const std::int64_t set_of_all = from / p.group_count, set = set_of_all % sets;
+            const int nwin = static_cast<int>(min(static_cast<std::int64_t>(kSet), p.windows - set * kSet));
+            bar_wait(smem_addr(acc_full), static_cast<std::uint32_t>(run & 1), abort_flag);
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const int quarter = warp & 3, wl = NB == 64 ? 0 : warp >> 3, c0 = (NB == 64 ? warp >> 2 : (warp >> 2) & 1) * 16;
+            const std::int64_t gene = (set * kSet + wl) * kWin + quarter * 32 + lane;
+            if (wl < nwin) { // warp-uniform
+                double scale = 0.0, offset = 0.0;
+                if (gene < p.cols) {
+                    scale = p.scales != nullptr ? static_cast<double>(__ldg(p.scales + gene)) : 1.0;
+                    offset = p.offsets != nullptr ? static_cast<double>(__ldg(p.offsets + gene)) : 0.0;
+                }
+                const std::uint32_t at = tmem_base + (static_cast<std::uint32_t>(quarter * 32) << 16) + wl * 2 * NC + c0;
+                float *slot = p.partials + (((run_of(to - 1, p.group_count, p.run_groups) + blockIdx.x) * kSet + wl) * kWin + quarter * 32 + lane) * NB + c0;
+                const double *steps = p.steps + set_of_all / sets * NB + c0;
+#pragma unroll
+                for (int h = 0; h < 16; h += 8) {
+                    long long coded[8], present[8];
+#pragma unroll
+                    for (int k = 0; k < SLICES; ++k) {
+                        int a[8], b[8];
+                        tmem_ld8(at + k * NB + h, a);
+                        tmem_ld8(at + NC + k * NB + h, b);
+#pragma unroll
+                        for (int c = 0; c < 8; ++c) {
+                            coded[c] = k == 0 ? a[c] : coded[c] * 256 + a[c];
+                            present[c] = k == 0 ? b[c] : present[c] * 256 + b[c];
+                        }
+                    }
+                    float v[8];
+#pragma unroll
+                    for (int c = 0; c < 8; ++c) // below 2^56: in double precision scale and offset may cancel to the last bits of fp32
+                        v[c] = static_cast<float>((scale * static_cast<double>(coded[c] + p.code_bias * present[c]) + offset * static_cast<double>(present[c])) * __ldg(steps + h + c));
+                    if (gene < p.cols && *abort_flag == 0) {
+                        *reinterpret_cast<float4 *>(slot + h) = make_float4(v[0], v[1], v[2], v[3]);
+                        *reinterpret_cast<float4 *>(slot + h + 4) = make_float4(v[4], v[5], v[6], v[7]);
+                    }
+                }
+            }
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) bar_arrive(smem_addr(acc_empty));
+            ++run;
+        };
+        // A run's sums are read once the group has scattered a tile of a later run, so that the MMAs of that have a tile to start with.
+        std::int64_t drained = u0, drained_end = u0 < u1 ? run_end(u0, u1, p.group_count, p.run_groups) : u1;
+        tile_cursor at(p, sets, u0, kSet);
+        if (grp != 0) at.next();
+        while (at.unit < u1) {
+            // the tile's first chunk goes into registers while the MMAs still read the group's previous tile
+            bar_wait(chunk_full, qc & 1u, abort_flag);
+            const int meta = chunk_meta[grp];
+            const int n_entries = *abort_flag != 0 ? 0 : meta >> 1;
+            bool last = (meta & 1) != 0 || *abort_flag != 0;
+            uint4 held[kChunkEntries / (kGroupThreads * 4)];
+            std::uint32_t all = 0;
+#pragma unroll
+            for (int k = 0; k < kChunkEntries / (kGroupThreads * 4); ++k) {
+                const int i = (k * kGroupThreads + gtid) * 4;
+                held[k] = i < n_entries ? chunk[i >> 2] : make_uint4(kPadding, kPadding, kPadding, kPadding);
+                all |= held[k].x | held[k].y | held[k].z | held[k].w;
+            }
+            arrive_when_loaded(chunk_empty, all, lane, static_cast<std::uint32_t>(p.windows) >> 31);
+            ++qc;
+            bar_wait(smem_addr(a_empty + grp), (q & 1u) ^ 1u, abort_flag);
+#pragma unroll
+            for (int k = 0; k < kTileBytes / (kGroupThreads * 8); ++k) // 8-byte stores: fewer wavefronts of the LSU data pipe per byte than 16-byte ones
+                *reinterpret_cast<uint2 *>(tile + k * (kGroupThreads * 8) + gtid * 8) = make_uint2(0u, 0u);
+            if (grp == 0) asm volatile("bar.sync 2, %0;" ::"n"(kGroupThreads) : "memory");
+            else asm volatile("bar.sync 3, %0;" ::"n"(kGroupThreads) : "memory");
+#pragma unroll
+            for (int k = 0; k < kChunkEntries / (kGroupThreads * 4); ++k) {
+                scatter(held[k].x); scatter(held[k].y); scatter(held[k].z); scatter(held[k].w);
+            }
+            int guard = 0;
+            while (!last && ++guard < (1 << 20)) {
+                bar_wait(chunk_full, qc & 1u, abort_flag);
+                const int more = chunk_meta[grp];
+                const int n_more = *abort_flag != 0 ? 0 : more >> 1;
+                last = (more & 1) != 0 || *abort_flag != 0;
+                for (int i = gtid * 4; i < n_more; i += kGroupThreads * 4) {
+                    const uint4 e = chunk[i >> 2];
+                    scatter(e.x); scatter(e.y); scatter(e.z); scatter(e.w);
+                }
+                __syncwarp();
+                if (lane == 0) bar_arrive(chunk_empty);
+                ++qc;
+            }
+            fence_async_proxy(); // ordinary stores, read by the MMA through the async proxy
+            __syncwarp();
+            if (lane == 0) bar_arrive(smem_addr(a_full + grp));
+            ++q;
+            while (drained_end <= at.unit) {
+                put_together(drained, drained_end);
+                drained = drained_end;
+                drained_end = run_end(drained, u1, p.group_count, p.run_groups);
+            }
+            at.next();
+            at.next();
+        }
+        while (drained < u1) {
+            put_together(drained, drained_end);
+            drained = drained_end;
+            if (drained < u1) drained_end = run_end(drained, u1, p.group_count, p.run_groups);
+        }
+    } else if (warp == kProducerWarps) {
+        // ================= MMA issuer: one thread, which does the waiting too =================
+        if (elect_one()) {
+            std::uint32_t q = 0, phase = 0;
+            int slot = 0, run = 0;
+            for (std::int64_t u = u0; u < u1; ++run) {
+                const std::int64_t ub = u, ue = run_end(u, u1, p.group_count, p.run_groups);
+                const std::int64_t set = u / p.group_count % sets;
+                const int nwin = static_cast<int>(min(static_cast<std::int64_t>(kSet), p.windows - set * kSet));
+                bar_wait(smem_addr(acc_empty), static_cast<std::uint32_t>((run & 1) ^ 1), abort_flag);
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                for (; u < ue; ++u) {
+                    int s = slot;
+                    std::uint32_t ph = phase;
+                    for (int wl = 0; wl < nwin; ++wl, ++q) {
+                        const std::uint32_t b = q & 1u;
+                        bar_wait(smem_addr(a_full + b), (q >> 1) & 1u, abort_flag);
+                        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                        s = slot;
+                        ph = phase;
+#pragma unroll
+                        for (int piece = 0; piece < kGPieces; ++piece) {
+                            if (wl == 0) bar_wait(smem_addr(g_full + s), ph, abort_flag);
+                            const std::uint32_t a = smem0 + b * kTileBytes + (piece >> 1) * (kPlaneBytes / 2) + (piece & 1) * 64, g_piece = grec0 + s * GPIECE;
+                            const std::uint32_t d = tmem_base + wl * 2 * NC;
+#pragma unroll
+                            for (int kk = 0; kk < kGPieceRows / 32; ++kk) {
+                                mma_i8(d, smem_desc_sw128(a + kk * 32), smem_desc_digits(g_piece + kk * 256), IDESC, u > ub || piece > 0 || kk > 0);
+                                mma_i8(d + NC, smem_desc_sw128(a + kPlaneBytes + kk * 32), smem_desc_digits(g_piece + kk * 256), IDESC, u > ub || piece > 0 || kk > 0);
+                            }
+                            if (wl == nwin - 1) mma_commit(smem_addr(g_empty + s));
+                            if (++s == kPieces) { s = 0; ph ^= 1u; }
+                        }
+                        mma_commit(smem_addr(a_empty + b));
+                    }
+                    slot = s;
+                    phase = ph;
+                }
+                mma_commit(smem_addr(acc_full));
+            }
+        }
+    } else if (warp == kProducerWarps + 2) {
+        // ================= the ring of G =================
+        if (elect_one()) {
+            int s = 0, issued = 0;
+            std::uint32_t ph = 1;
+            bool dead = p.poll_limit != 0 && bar_wait(smem_addr(g_full), 0u, abort_flag, p.poll_limit);
+            std::int64_t group = u0 % p.group_count, set_of_all = u0 / p.group_count;
+            const unsigned char *block = p.records + set_of_all / sets * p.group_count * (kGPieces * GPIECE); // of the column block
+            for (std::int64_t u = u0; u < u1 && !dead; ++u) {
+                const unsigned char *src = block + group * (kGPieces * GPIECE);
+                if (++group == p.group_count) {
+                    group = 0;
+                    block = p.records + ++set_of_all / sets * p.group_count * (kGPieces * GPIECE);
+                }
+                for (int piece = 0; piece < kGPieces; ++piece, src += GPIECE) {
+                    dead = bar_wait(smem_addr(g_empty + s), ph, abort_flag);
+                    if (dead) break; // no new copies once a wait of the CTA has run out
+                    ++issued;
+                    bar_arrive_expect_tx(smem_addr(g_full + s), GPIECE);
+                    bulk_copy_g2s(grec0 + s * GPIECE, src, GPIECE, smem_addr(g_full + s));
+                    if (++s == kPieces) { s = 0; ph ^= 1u; }
+                }
+            }
+            fills[0] = issued;
+        }
+    } else {
+        // ================= the words: a warp per scatter group; a tile's lie in the group's eight pieces, a lane each =================
+        const int ring = warp == kProducerWarps + 1 ? 0 : 1;
+        const std::uint32_t full = smem_addr(c_full + ring), empty = smem_addr(c_empty + ring), dst = chunk0 + ring * kChunkBytes;
+        tile_cursor at(p, sets, u0, kSet);
+        if (ring != 0) at.next();
+        // the bounds of the next tile's words are on their way while this one's are copied: 64-bit divisions and loads that were waited
+        // for held this warp up for 2,450 cycles a tile, more than its MMAs take
+        std::uint32_t lo = 0, hi = 0;
+        std::int64_t base = 0;
+        const auto fetch = [&]() {
+            lo = hi = 0u;
+            const std::int64_t piece = (p.group_begin + at.group) * kGroupPieces + lane;
+            if (at.unit < u1 && lane < kGroupPieces && piece < p.pieces) {
+                const std::uint32_t *bound = p.bounds + piece * (p.windows + 1) + at.set * kSet + at.wl;
+                lo = __ldcg(bound);
+                hi = __ldcg(bound + 1);
+                base = __ldcg(p.bases + piece) & (kTwice - 1);
+            }
+        };
+        fetch();
+        int done = 0; // chunks issued
+        bool dead = false;
+        while (at.unit < u1 && !dead) {
+            const int words = static_cast<int>(hi - lo);
+            const std::uint32_t *src = p.words + base + lo;
+            at.next();
+            at.next();
+            fetch();
+            int upto = words;
+#pragma unroll
+            for (int d = 1; d < kGroupPieces; d <<= 1) {
+                const int below = __shfl_up_sync(0xffffffffu, upto, d);
+                if (lane >= d) upto += below;
+            }
+            const int begin = upto - words, total = __shfl_sync(0xffffffffu, upto, kGroupPieces - 1);
+            int c0 = 0;
+            do {
+                const int n = min(kChunkEntries, total - c0);
+                dead = __any_sync(0xffffffffu, bar_wait(empty, static_cast<std::uint32_t>((done & 1) ^ 1), abort_flag));
+                if (dead) break; // no new copies once a wait of the CTA has run out
+                if (lane == 0) {
+                    chunk_meta[ring] = (n << 1) | (c0 + n >= total ? 1 : 0);
+                    if (n > 0) bar_arrive_expect_tx(full, static_cast<std::uint32_t>(n) * 4u);
+                    else bar_arrive(full); // a tile without entries still hands over one (empty) chunk
+                }
+                __syncwarp();
+                const int first = max(begin, c0), last = min(begin + words, c0 + n);
+                if (lane < kGroupPieces && first < last)
+                    bulk_copy_g2s(dst + (first - c0) * 4, src + (first - begin), static_cast<std::uint32_t>(last - first) * 4u, full);
+                __syncwarp();
+                ++done;
+                c0 += n;
+            } while (c0 < total);
+        }
+        if (lane == 0) fills[1 + ring] = done;
+    }
+
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (*abort_flag != 0) { // every role has ended: what is in flight finishes before the CTA gives up its shared and tensor memory
+        if (warp == kProducerWarps) {
+            if (elect_one()) drain_mmas(smem_addr(mma_drain)); // by the thread that issued
+        } else if (warp == kProducerWarps + 2) {
+            if (elect_one()) drain_fills(smem_addr(g_full), kPieces, fills[0]);
+        } else if (warp > kProducerWarps && lane == 0) {
+            const int ring = warp == kProducerWarps + 1 ? 0 : 1;
+            drain_fills(smem_addr(c_full + ring), 1, fills[1 + ring]);
+        }
+        __syncthreads();
+    }
+    if (warp == 0) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512) : "memory");
+    }
+    if (tid == 0 && *abort_flag != 0) atomicExch(p.status, 1);
+}
+
+template<int NB, int SLICES> constexpr std::size_t digits_smem_bytes() {
+    return 2 * kTileBytes + ring_pieces(NB, SLICES) * g_piece_bytes(NB, SLICES) + 2 * kChunkBytes + (11 + 2 * ring_pieces(NB, SLICES)) * sizeof(std::uint64_t) + 32;
+}
+
+struct finish_params {
+    digit_params d;
+    const float *g;
+    std::int64_t g_ld, first_row, row_begin, row_end; // row_begin, row_end: of the launch; first_row: of the words
+    float *out;
+    std::int64_t out_ld;
+    std::int64_t grid; // CTAs of the main kernel
+    int n, out_vector;
+    float alpha, beta;
+};
+
+// G'[genes of one window, columns of one block] = beta * G' + alpha * (the sums of the set's runs, added in run order).
+// Where a column's range is too wide for fixed point, or a scale or a zero-point of the window is not finite (0 * infinity, in a
+// product of sums, would reach cells that hold no entry): from the entries, in double precision.  A warp has every eighth gene
+// of the window to itself and walks the words in order, so this too has the same bits on every run.
+template<int NB, int SLICES>
+__global__ void __launch_bounds__(256) finish_kernel(const finish_params p) {
+    extern __shared__ double slow_sums[]; // [kWin][NB]
+    constexpr int kSet = set_windows(NB, SLICES);
+    __shared__ float2 meta[kWin];
+    wait_for_previous_launch();
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const std::int64_t sets = (p.d.windows + kSet - 1) / kSet;
+    const int wl = static_cast<int>(blockIdx.x % kSet);
+    const std::int64_t set = blockIdx.x / kSet, window = set * kSet + wl; // the set among the block's, and among all of them:
+    const int c0 = static_cast<int>(blockIdx.y) * NB;
+    const std::int64_t set_of_all = blockIdx.y * sets + set;
+    if (window >= p.d.windows) return;
+    int odd = 0;
+    if (tid < kWin) {
+        const std::int64_t gene = window * kWin + tid;
+        float2 so = make_float2(0.0f, 0.0f);
+        if (gene < p.d.cols) so = make_float2(p.d.scales != nullptr ? __ldg(p.d.scales + gene) : 1.0f, p.d.offsets != nullptr ? __ldg(p.d.offsets + gene) : 0.0f);
+        meta[tid] = so;
+        odd = isfinite(so.x) && isfinite(so.y) ? 0 : 1;
+    }
+    const bool slow = __syncthreads_or(odd) != 0 || *p.d.wide != 0;
+    if (slow) {
+        for (int i = tid; i < kWin * NB; i += 256) slow_sums[i] = 0.0;
+        __syncthreads();
+        const std::int64_t piece0 = (p.row_begin - p.first_row) / kPieceRows, piece1 = (p.row_end - p.first_row + kPieceRows - 1) / kPieceRows;
+        for (std::int64_t piece = piece0; piece < piece1; ++piece) {
+            const std::uint32_t *at = p.d.bounds + piece * (p.d.windows + 1) + window;
+            const int words = static_cast<int>(__ldcg(at + 1) - __ldcg(at));
+            const std::uint32_t *w = p.d.words + (__ldcg(p.d.bases + piece) & (kTwice - 1)) + __ldcg(at);
+            const std::int64_t group_row = p.first_row + piece / kGroupPieces * kRows;
+            for (int i0 = 0; i0 < words; i0 += 32) {
+                const std::uint32_t e = i0 + lane < words ? __ldcg(w + i0 + lane) : kPadding;
+                const int place = static_cast<int>((e >> 8) & 0x7fffu), gl = (place >> 7) & (kWin - 1);
+                const int cell = (place >> 14) * 128 + ((((place >> 4) & 7) ^ (gl & 7)) << 4) + (place & 15);
+                const std::int64_t row = group_row + cell;
+                std::uint32_t todo = __ballot_sync(0xffffffffu, static_cast<int>(e) >= 0 && (gl & 7) == warp && row >= p.row_begin && row < p.row_end);
+                while (todo != 0u) {
+                    const int j = __ffs(todo) - 1;
+                    todo &= todo - 1u;
+                    const std::uint32_t ej = __shfl_sync(0xffffffffu, e, j);
+                    const int gj = __shfl_sync(0xffffffffu, gl, j);
+                    const std::int64_t rj = group_row + __shfl_sync(0xffffffffu, cell, j);
+                    const int code = static_cast<int>(static_cast<signed char>(ej & 0xffu)) + p.d.code_bias;
+                    const double value = static_cast<double>(fmaf(static_cast<float>(code), meta[gj].x, meta[gj].y));
+                    for (int c = lane; c < NB; c += 32)
+                        if (c0 + c < p.n) slow_sums[gj * NB + c] += value * static_cast<double>(__ldg(p.g + rj * p.g_ld + c0 + c));
+                }
+            }
+        }
+        __syncthreads();
+    }
+    // the set's slots: the CTAs whose shares meet its runs, run after run
+    const std::int64_t total = sets * p.d.column_blocks * p.d.group_count, L = p.d.group_count, cuts = (L + p.d.run_groups - 1) / p.d.run_groups;
+    const auto from_of = [&](std::int64_t cut) { return set_of_all * L + cut * p.d.run_groups; };
+    const auto to_of = [&](std::int64_t cut) { return min(from_of(cut) + p.d.run_groups, (set_of_all + 1) * L); };
+    const std::int64_t first0 = cta_of(from_of(0), total, p.grid), last0 = cta_of(to_of(0) - 1, total, p.grid);
+    constexpr int kItems = kWin * (NB / 4) / 256; // of a thread
+    float4 sums[kItems];
+#pragma unroll
+    for (int k = 0; k < kItems; ++k) sums[k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    for (std::int64_t cut = 0; cut < cuts && !slow; ++cut) {
+        const std::int64_t last = cut == 0 ? last0 : cta_of(to_of(cut) - 1, total, p.grid);
+        for (std::int64_t b = cut == 0 ? first0 : cta_of(from_of(cut), total, p.grid); b <= last; ++b) {
+            const float4 *slot = reinterpret_cast<const float4 *>(p.d.partials + ((set_of_all * cuts + cut + b) * kSet + wl) * kWin * NB) + tid;
+            float4 v[kItems];
+#pragma unroll
+            for (int k = 0; k < kItems; ++k) v[k] = __ldcg(slot + k * 256);
+#pragma unroll
+            for (int k = 0; k < kItems; ++k) { sums[k].x += v[k].x; sums[k].y += v[k].y; sums[k].z += v[k].z; sums[k].w += v[k].w; }
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < kItems; ++k) {
+        const int i = tid + k * 256, gl = i / (NB / 4), c = i % (NB / 4) * 4;
+        const std::int64_t gene = window * kWin + gl;
+        if (gene >= p.d.cols || c0 + c >= p.n) continue;
+        float4 sum = sums[k];
+        if (slow) {
+            const double *s = slow_sums + gl * NB + c;
+            sum = make_float4(static_cast<float>(s[0]), static_cast<float>(s[1]), static_cast<float>(s[2]), static_cast<float>(s[3]));
+        }
+        float *dst = p.out + gene * p.out_ld + c0 + c;
+        const float v[4] = {sum.x, sum.y, sum.z, sum.w};
+        if (p.out_vector != 0) {
+            float4 o = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (p.beta != 0.0f) {
+                o = *reinterpret_cast<const float4 *>(dst);
+                o.x *= p.beta; o.y *= p.beta; o.z *= p.beta; o.w *= p.beta;
+            }
+            *reinterpret_cast<float4 *>(dst) = make_float4(fmaf(p.alpha, v[0], o.x), fmaf(p.alpha, v[1], o.y), fmaf(p.alpha, v[2], o.z), fmaf(p.alpha, v[3], o.w));
+        } else {
+            for (int j = 0; j < 4 && c0 + c + j < p.n; ++j) dst[j] = fmaf(p.alpha, v[j], p.beta == 0.0f ? 0.0f : p.beta * dst[j]);
+        }
+    }
+}
+
+int column_block(std::int64_t n) { return n <= 32 ? 32 : 64; }
+int padded_columns(std::int64_t n) { return n <= 32 ? 32 : n <= 64 ? 64 : n <= 128 ? 128 : 256; }
+
+std::uint64_t record_bytes(std::int64_t groups, std::int64_t n, int slices) {
+    const int nb = column_block(n);
+    return device_arena::rounded(static_cast<std::uint64_t>(groups) * static_cast<std::uint64_t>((n + nb - 1) / nb) * kRows * static_cast<std::uint64_t>(mma_columns(nb, slices)));
+}
+// a run ends with its set, after kRunGroups groups, or with its CTA's share of the units
+std::uint64_t partial_bytes(std::int64_t groups, std::int64_t cols, std::int64_t n, int slices, int ctas) {
+    const std::int64_t nb = column_block(n), per_set = set_windows(static_cast<int>(nb), slices), windows = (cols + kWin - 1) / kWin;
+    const std::int64_t sets = (windows + per_set - 1) / per_set * ((n + nb - 1) / nb), cuts = (groups + kRunGroups - 1) / kRunGroups;
+    return device_arena::rounded(static_cast<std::uint64_t>(sets * cuts + ctas) * static_cast<std::uint64_t>(per_set * kWin * nb) * sizeof(float));
+}
+// what a launch over `groups` groups at a time needs, without the words
+std::uint64_t launch_bytes(std::int64_t groups, std::int64_t cols, std::int64_t n, int slices, int ctas) {
+    return kRecordsAt + record_bytes(groups, n, slices) + partial_bytes(groups, cols, n, slices, ctas);
+}
+std::int64_t group_count_of(std::int64_t rows) { return (rows + kRows - 1) / kRows; }
+std::int64_t piece_count(std::int64_t rows) { return (rows + kPieceRows - 1) / kPieceRows; }
+std::uint64_t word_bytes(std::int64_t rows, std::int64_t cols, std::int64_t nnz) {
+    const std::int64_t windows = (cols + kWin - 1) / kWin;
+    return static_cast<std::uint64_t>(nnz + 4 + piece_count(rows) * (4 * windows + 4)) * 4u;
+}
+std::uint64_t bound_bytes(std::int64_t rows, std::int64_t cols) { return static_cast<std::uint64_t>(piece_count(rows) * ((cols + kWin - 1) / kWin + 1)) * 4u; }
+int build_smem_bytes(std::int64_t cols) { return static_cast<int>(kPieceRows * ((cols + kWin - 1) / kWin) * 4); }
+
+cb200_status launch_words(const qcsr_view &x, std::int64_t row_begin, std::int64_t row_end, std::uint32_t *words, std::uint32_t *bounds,
+                          std::int64_t *bases, int *status, cudaStream_t stream) {
+    words_params p{};
+    p.row_ptr = x.row_ptr; p.packed_row_ptr = x.packed_row_ptr; p.col_idx = x.col_idx; p.packed = x.packed;
+    p.row_begin = row_begin; p.row_end = row_end; p.cols = x.cols; p.windows = static_cast<int>((x.cols + kWin - 1) / kWin);
+    p.code_bias = x.bits == 8 ? 128 : 0;
+    p.words = words; p.bounds = bounds; p.bases = bases; p.status = status;
+    const int smem = build_smem_bytes(x.cols);
+    const unsigned grid = static_cast<unsigned>(piece_count(row_end - row_begin));
+    if (x.bits == 8) {
+        CB200_CUDA_OK(cudaFuncSetAttribute(digit_words_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        digit_words_kernel<8><<<grid, kBuildThreads, smem, stream>>>(p);
+    } else {
+        CB200_CUDA_OK(cudaFuncSetAttribute(digit_words_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        digit_words_kernel<4><<<grid, kBuildThreads, smem, stream>>>(p);
+    }
+    count_launch();
+    CB200_CUDA_OK(cudaGetLastError());
+    return CB200_STATUS_SUCCESS;
+}
+
+struct digit_launch {
+    digit_params main;       // group_begin, group_count: of the whole row range
+    finish_params finish;
+    std::int64_t slice;      // groups at a time
+    unsigned *part_max;
+    double *part_square, *steps;
+    unsigned char *records;
+    int *wide;
+    bool early; // the launch in front is a kernel of this call
+};
+
+template<int NB, int SLICES>
+cb200_status launch_digits(const digit_launch &l, int sm_count, cudaStream_t stream) {
+    constexpr std::size_t smem = digits_smem_bytes<NB, SLICES>();
+    static_assert(smem <= 232448, "shared memory budget");
+    constexpr int slow_smem = kWin * NB * 8;
+    CB200_CUDA_OK(cudaFuncSetAttribute(qcsr_transpose_digits_kernel<NB, SLICES>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+    CB200_CUDA_OK(cudaFuncSetAttribute(finish_kernel<NB, SLICES>, cudaFuncAttributeMaxDynamicSharedMemorySize, slow_smem));
+    const int n = l.finish.n, padded = padded_columns(n);
+    CB200_CUDA_OK(launch_kernel(l.early, column_range_kernel, dim3(kParts), 1024, 0, stream, l.finish.g, l.finish.g_ld, n, padded, l.finish.row_begin, l.finish.row_end,
+                                l.part_max, l.part_square, l.early ? nullptr : l.main.status));
+    const std::int64_t group_end = l.main.group_begin + l.main.group_count;
+    for (std::int64_t begin = l.main.group_begin; begin < group_end; begin += l.slice) {
+        digit_params m = l.main;
+        finish_params f = l.finish;
+        m.group_begin = begin;
+        m.group_count = std::min(l.slice, group_end - begin);
+        m.partials = reinterpret_cast<float *>(l.records + record_bytes(m.group_count, n, SLICES));
+        const std::int64_t row0 = f.first_row + begin * kRows, blocks = m.group_count * m.column_blocks;
+        CB200_CUDA_OK(launch_kernel(true, pack_digits_kernel<NB, SLICES>, dim3(static_cast<unsigned>(std::min<std::int64_t>(blocks * kGPieces, 4 * sm_count))), 256, 0, stream, f.g,
+                                    f.g_ld, n, padded, row0, f.row_begin, f.row_end, m.group_count, l.part_max, l.part_square, l.steps, l.records, m.bases, m.pieces,
+                                    l.wide));
+        const std::int64_t sets = (m.windows + set_windows(NB, SLICES) - 1) / set_windows(NB, SLICES);
+        const unsigned grid = static_cast<unsigned>(std::min<std::int64_t>(sets * blocks, sm_count));
+        CB200_CUDA_OK(launch_kernel(true, qcsr_transpose_digits_kernel<NB, SLICES>, dim3(grid), kThreads, smem, stream, m));
+        f.d = m;
+        f.grid = grid;
+        f.row_begin = std::max(f.row_begin, row0);
+        f.row_end = std::min(f.row_end, row0 + m.group_count * kRows);
+        if (begin != l.main.group_begin) f.beta = 1.0f;
+        CB200_CUDA_OK(launch_kernel(true, finish_kernel<NB, SLICES>, dim3(static_cast<unsigned>(sets * set_windows(NB, SLICES)), static_cast<unsigned>(m.column_blocks)), 256,
+                                    slow_smem, stream, f));
+        count_launch(3);
+    }
+    count_launch();
+    CB200_CUDA_OK(cudaGetLastError());
+    return CB200_STATUS_SUCCESS;
+}
+
+} // namespace
+
+bool qcsr_transpose_digits_shape_ok(std::int64_t rows, std::int64_t cols, std::int64_t n, int bits, int policy) {
+    // the counters of a piece have to fit in shared memory: 224,000 genes
+    return (bits == 8 || bits == 4) && policy == CB200_DECODE_PER_GENE_AFFINE && n > 0 && n <= kMaxColumns && rows > 0 && cols > 0 &&
+           (cols + kWin - 1) / kWin * kPieceRows * 4 <= 224 * 1024;
+}
+std::uint64_t qcsr_digit_words_bytes_bound(std::int64_t rows, std::int64_t cols, std::int64_t nnz) {
+    return device_arena::rounded(word_bytes(rows, cols, nnz)) + device_arena::rounded(bound_bytes(rows, cols)) +
+           device_arena::rounded(static_cast<std::uint64_t>(piece_count(rows)) * 8u);
+}
+std::uint64_t qcsr_transpose_digits_workspace_bytes(std::int64_t rows, std::int64_t cols, std::int64_t n, int slices) {
+    return launch_bytes(group_count_of(rows), cols, n, slices, kMaxCtas);
+}
+std::uint64_t qcsr_transpose_digits_least_workspace(std::int64_t rows, std::int64_t cols, std::int64_t n, int slices, int sm_count) {
+    return launch_bytes(std::min<std::int64_t>(group_count_of(rows), 16), cols, n, slices, std::min(sm_count, kMaxCtas));
+}
+std::uint64_t qcsr_transpose_digits_once_bytes(std::int64_t rows, std::int64_t cols, std::int64_t n, std::int64_t nnz, int bits, int policy) {
+    if (!qcsr_transpose_digits_shape_ok(rows, cols, n, bits, policy)) return 0u;
+    // Sparser, a tile is mostly zeroes; fewer entries, and the five launches take longer than the two of the other kernel.  One call, N =
+    // 64: 2,000 x 8,000 (1.6 M entries) 48 us against 45, 1,500 x 33,538 (2.7 M) 75 against 75, 4,000 x 4,000 (2.1 M) 49 against 57,
+    // 8,191 x 33,538 (14.7 M) 171 against 318; at N = 32 8,000 x 2,000 (2.9 M) 51 against 53, 16,384 x 2,000 (5.9 M) 74 against 108.
+    if (static_cast<double>(nnz) < 0.02 * static_cast<double>(rows) * static_cast<double>(cols) || nnz < kLeastOnceEntries || nnz > kMostOnceEntries) return 0u;
+    return qcsr_transpose_digits_workspace_bytes(rows, cols, n, 4) + qcsr_digit_words_bytes_bound(rows, cols, nnz);
+}
+
+cb200_status build_digit_words(const qcsr_view &x, device_arena &arena, cudaStream_t stream, digit_layout *out) {
+    *out = digit_layout{};
+    if (x.row_ptr == nullptr || (x.nnz != 0 && (x.col_idx == nullptr || x.packed == nullptr)))
+        return fail(CB200_STATUS_INVALID_ARGUMENT, "the matrix handed to prepare has null arrays");
+    if (x.bits == 4 && x.packed_row_ptr == nullptr) return fail(CB200_STATUS_INVALID_ARGUMENT, "4-bit codes need packed_row_ptr");
+    const std::uint64_t words = word_bytes(x.rows, x.cols, x.nnz), bounds = bound_bytes(x.rows, x.cols), bases = static_cast<std::uint64_t>(piece_count(x.rows)) * 8u;
+    out->words = static_cast<std::uint32_t *>(arena.take(words));
+    out->bounds = static_cast<std::uint32_t *>(arena.take(bounds));
+    out->bases = static_cast<std::int64_t *>(arena.take(bases));
+    cb200_status st = CB200_STATUS_SUCCESS;
+    if (out->words == nullptr || out->bounds == nullptr || out->bases == nullptr)
+        st = fail(CB200_STATUS_INSUFFICIENT_WORKSPACE, "no device memory for the entry words of the transpose");
+    if (st == CB200_STATUS_SUCCESS) st = launch_words(x, 0, x.rows, out->words, out->bounds, out->bases, nullptr, stream);
+    if (st == CB200_STATUS_SUCCESS) {
+        const cudaError_t err = cudaStreamSynchronize(stream);
+        if (err != cudaSuccess) st = fail(CB200_STATUS_CUDA_ERROR, "building the entry words of the transpose: %s", cudaGetErrorString(err));
+    }
+    if (st != CB200_STATUS_SUCCESS) {
+        arena.give_back(out->bases, bases);
+        arena.give_back(out->bounds, bounds);
+        arena.give_back(out->words, words);
+        *out = digit_layout{};
+        return st;
+    }
+    out->bytes = words + bounds + bases;
+    out->src_row_ptr = x.row_ptr; out->src_col_idx = x.col_idx; out->src_packed = x.packed;
+    return st;
+}
+
+cb200_status launch_qcsr_transpose_digits(const qcsr_view &x, const dense_args &d, std::int64_t row_begin, std::int64_t row_end, void *workspace,
+                                          std::uint64_t workspace_bytes, const digit_layout *layout, int slices, int sm_count, cudaStream_t stream, bool *taken) {
+    *taken = false;
+    if (row_end <= row_begin || d.dense_dtype != CB200_DTYPE_F32 || !qcsr_transpose_digits_shape_ok(x.rows, x.cols, d.n, x.bits, x.policy)) return CB200_STATUS_SUCCESS;
+    if (workspace == nullptr || reinterpret_cast<std::uintptr_t>(workspace) % 256u != 0u || sm_count > kMaxCtas) return CB200_STATUS_SUCCESS;
+    if (x.bits == 4 && x.packed_row_ptr == nullptr) return CB200_STATUS_SUCCESS;
+    // With less workspace than for the whole range the groups are taken in slices.  A call that has to make its words has room for
+    // everything or is another kernel's.
+    const std::uint64_t own = qcsr_transpose_digits_workspace_bytes(x.rows, x.cols, d.n, slices);
+    if (layout == nullptr && workspace_bytes < own + qcsr_digit_words_bytes_bound(x.rows, x.cols, x.nnz)) return CB200_STATUS_SUCCESS;
+    const std::int64_t first_row = layout != nullptr ? 0 : row_begin, rows_of_words = layout != nullptr ? x.rows : row_end - row_begin;
+    const std::int64_t group_begin = (row_begin - first_row) / kRows, group_count = (row_end - first_row + kRows - 1) / kRows - group_begin;
+    std::int64_t slice = group_count;
+    while (slice > 1 && launch_bytes(slice, x.cols, d.n, slices, sm_count) > workspace_bytes) slice = (slice + 1) / 2;
+    if (launch_bytes(slice, x.cols, d.n, slices, sm_count) > workspace_bytes) return CB200_STATUS_SUCCESS;
+    if (layout != nullptr && (x.row_ptr != layout->src_row_ptr || x.col_idx != layout->src_col_idx || x.packed != layout->src_packed))
+        return fail(CB200_STATUS_STALE_STRUCTURE, "the launch's matrix is not the one the entry words were built from");
+    *taken = true;
+    unsigned char *ws = static_cast<unsigned char *>(workspace);
+    digit_launch l{};
+    l.early = layout == nullptr;
+    l.part_max = reinterpret_cast<unsigned *>(ws + kPartMaxAt);
+    l.part_square = reinterpret_cast<double *>(ws + kPartSquareAt);
+    l.steps = reinterpret_cast<double *>(ws + kStepsAt);
+    l.records = ws + kRecordsAt;
+    l.wide = reinterpret_cast<int *>(ws) + 1;
+    digit_params &p = l.main;
+    p.status = reinterpret_cast<int *>(ws);
+    l.slice = slice;
+    if (layout != nullptr) {
+        p.words = layout->words; p.bounds = layout->bounds; p.bases = layout->bases;
+    } else {
+        unsigned char *at = ws + own;
+        std::uint32_t *words = reinterpret_cast<std::uint32_t *>(at);
+        at += device_arena::rounded(word_bytes(x.rows, x.cols, x.nnz));
+        std::uint32_t *bounds = reinterpret_cast<std::uint32_t *>(at);
+        at += device_arena::rounded(bound_bytes(x.rows, x.cols));
+        std::int64_t *bases = reinterpret_cast<std::int64_t *>(at);
+        const cb200_status st = launch_words(x, row_begin, row_end, words, bounds, bases, p.status, stream);
+        if (st != CB200_STATUS_SUCCESS) return st;
+        p.words = words; p.bounds = bounds; p.bases = bases;
+    }
+    const int nb = column_block(d.n);
+    p.pieces = piece_count(rows_of_words);
+    p.scales = x.scales; p.offsets = x.offsets;
+    p.records = l.records; p.steps = l.steps; p.wide = l.wide;
+    p.cols = x.cols;
+    p.group_begin = group_begin;
+    p.group_count = group_count;
+    p.run_groups = kRunGroups;
+    p.windows = static_cast<int>((x.cols + kWin - 1) / kWin);
+    p.column_blocks = static_cast<int>((d.n + nb - 1) / nb);
+    p.code_bias = x.bits == 8 ? 128 : 0;
+    p.poll_limit = test_poll_limit();
+    finish_params &f = l.finish;
+    f.g = static_cast<const float *>(d.dense); f.g_ld = d.dense_ld;
+    f.first_row = first_row; f.row_begin = row_begin; f.row_end = row_end;
+    f.out = d.out; f.out_ld = d.out_ld; f.n = static_cast<int>(d.n);
+    f.out_vector = reinterpret_cast<std::uintptr_t>(d.out) % 16u == 0u && d.out_ld % 4 == 0 && d.n % 4 == 0 ? 1 : 0;
+    f.alpha = d.alpha; f.beta = d.beta;
+    if (slices == 4) return nb == 64 ? launch_digits<64, 4>(l, sm_count, stream) : launch_digits<32, 4>(l, sm_count, stream);
+    return nb == 64 ? launch_digits<64, 3>(l, sm_count, stream) : launch_digits<32, 3>(l, sm_count, stream);
+}
+
+} // namespace cb200

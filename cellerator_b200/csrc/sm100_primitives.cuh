@@ -125,6 +125,19 @@ __device__ __forceinline__ void mma_bf16(std::uint32_t tmem_d, std::uint64_t des
         : "r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate ? 1u : 0u), "r"(0u)
         : "memory");
 }
+// kind::i8: D int32, A and B both signed 8-bit, both K-major, M = 128, K = 32.  Measured, A and B from shared memory, elected issuer:
+// 48, 56, 64, 96, 128 cycles at n = 64, 96, 128, 192, 256; the sums are exact.
+__host__ __device__ constexpr std::uint32_t instr_desc_i8(int n) {
+    return (2u << 4) | (1u << 7) | (1u << 10) | ((static_cast<std::uint32_t>(n) >> 3) << 17) | ((128u >> 4) << 24);
+}
+__device__ __forceinline__ void mma_i8(std::uint32_t tmem_d, std::uint64_t desc_a, std::uint64_t desc_b, std::uint32_t idesc, bool accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}"
+        :
+        : "r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate ? 1u : 0u)
+        : "memory");
+}
 __device__ __forceinline__ void mma_commit(std::uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
@@ -148,6 +161,15 @@ __device__ __forceinline__ void tmem_ld32(std::uint32_t taddr, float (&v)[32]) {
     for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
 }
 
+// Eight columns of this thread's lane, as integers.
+__device__ __forceinline__ void tmem_ld8(std::uint32_t at, int (&v)[8]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n\t"
+        "tcgen05.wait::ld.sync.aligned;"
+        : "=&r"(v[0]), "=&r"(v[1]), "=&r"(v[2]), "=&r"(v[3]), "=&r"(v[4]), "=&r"(v[5]), "=&r"(v[6]), "=&r"(v[7])
+        : "r"(at)
+        : "memory");
+}
 // Sixteen columns of this thread's lane of tensor memory, of one, two or three places with one wait.
 __device__ __forceinline__ void tmem_ld16(std::uint32_t at_v, float (&v)[16]) {
     asm volatile(

@@ -427,7 +427,7 @@ def spmm_transpose(x: QuantizedCsr, g: torch.Tensor, out: torch.Tensor | None = 
     """G' = alpha * deq(X)^T G + beta * G'.
 
     multiply=capi.DTYPE_BF16 asks for tensor-core products (decoded values and G rounded to bf16);
-    deterministic=True for the gather schedule whose fp32 sums have a fixed order."""
+    deterministic=True for sums that are the same bits on every call."""
     n = g.shape[1]
     if out is None:
         out = torch.empty(x.cols, n, dtype=torch.float32, device=x.device)

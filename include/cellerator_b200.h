@@ -248,9 +248,12 @@ typedef struct cb200_spmm_problem {
     /* Optional host copy of row_ptr (m+1) used to choose the row schedule; NULL = default. */
     const int64_t *host_row_ptr;
     int32_t deterministic; /* prepare_policy.deterministic, operation_core.hh:116-124; a transpose needs
-                            * device_matrix for it, else prepare is refused: schedule "gene_gather" (fp32 FMAs
-                            * entry by entry), or, with schedule_hint "tensor_blocked", the tensor-core schedules
-                            * over the window-blocked copy, whose CTAs' sums are added in a fixed order too */
+                            * device_matrix for it, else prepare is refused: schedule "gene_gather" (exact
+                            * integer sums of codes times four digits of G where the matrix is large and dense
+                            * enough and its zero-points are per gene, else fp32 FMAs entry by entry; the latter
+                            * always with schedule_hint "gene_gather"), or, with schedule_hint "tensor_blocked", the
+                            * tensor-core schedules over the window-blocked copy, whose CTAs' sums are added in a
+                            * fixed order too */
     /* numeric_policy.multiply of the request: 0 or CB200_DTYPE_F32 = exact fp32 products;
      * CB200_DTYPE_BF16 = decoded values may be rounded to bf16 and multiplied on the tensor cores
      * (CSR forward with bf16 W: schedules "tensor_windows" / "tensor_blocked"; transpose with the
@@ -260,8 +263,10 @@ typedef struct cb200_spmm_problem {
      * "tensor_blocked_x2" (forward, bf16 W) / "tensor_blocked_x3" (forward with fp32 W; transpose)
      * rebuild each fp32 product from bf16 tensor-core passes (value = hi + lo, fp32 dense operand =
      * hi + lo; hi*hi + hi*lo + lo*hi), relative error about 3 * 2^-17 per product: inside the 1e-4
-     * bound of an fp32 operand, not bit-equal to an fp32 multiply.  Without device_matrix the fp32-FMA
-     * kernels ("gene_tiled" / "warp_per_row", "vector_reductions") run. */
+     * bound of an fp32 operand, not bit-equal to an fp32 multiply.  The transpose with zero-points per gene
+     * multiplies the codes with three digits of G in fixed point instead (2^-23 of a column's largest
+     * magnitude) and adds without rounding.  Without device_matrix "gene_tiled" / "warp_per_row" (fp32 FMAs)
+     * and "vector_reductions" (fp32 FMAs, or four digits of G and integer sums) run. */
     int32_t multiply;
     /* Optional: the device-resident matrix itself (arrays on `device`, final contents).  With bf16
      * products allowed, prepare then builds a persistent window-blocked copy of it (one 32-bit
@@ -322,7 +327,8 @@ cb200_status cb200_spmm_prepare(const cb200_spmm_problem *problem, cb200_prepare
 cb200_status cb200_spmm_persistent_requirement(const cb200_spmm_problem *problem, uint64_t *bytes);
 void cb200_prepared_destroy(cb200_prepared *prepared);
 /* workspace_requirement, launch_bindings.hh:67-71: what the schedule can use.  "vector_reductions" reports up to 32 MB (it
- * sorts the entries with it, slice of rows by slice) and also runs with less or with none, slower.  "warp_per_row" (unaligned
+ * sorts the entries with it, slice of rows by slice), or for 2 to 50 million entries about 4 bytes an entry (words for integer
+ * sums), and also runs with less or with none, slower.  "warp_per_row" (unaligned
  * N) and the tensor_blocked and tensor_dense forward schedules also run with less, down to the status block and the records of
  * W, slower and with the same bits: a row's sum follows from its entries, N and W's type, not from the room, the launch's row
  * range or the rows beside it. */
@@ -652,7 +658,7 @@ cb200_status cb200_build_execution_csr(const cb200_execution_csr *view, void *st
  * (0 = shape outside the limits), and its first 32-bit word is 0 afterwards unless a column index lay
  * outside the matrix (bit 0).
  * cb200_spmm_prepare builds this copy itself for a transpose problem with deterministic = 1 and the
- * device matrix at hand (schedule "gene_gather"): the sums then have a fixed order -- per gene, eight
+ * device matrix at hand where it gathers entry by entry (schedule "gene_gather", see there): the sums then have a fixed order -- per gene, eight
  * interleaved runs of 256-entry chunks added entry by entry with fp32 FMAs, the eight partial sums
  * added in order -- and the output is the same bits on every run. */
 uint64_t cb200_qcsr_gene_major_workspace(int64_t rows, int64_t cols);

@@ -1,0 +1,177 @@
+"""GPU parity of the transpose with exact integer sums, at the edges of its tiles, pieces, chunks and runs."""
+import numpy as np
+import pytest
+import torch
+
+from cellerator_b200 import capi, ops
+from conftest import random_csr
+from gpu_util import dense, host_pack, to_dev
+
+pytestmark = pytest.mark.gpu
+
+
+def reference(oracle, c, g, lo=0, hi=None):
+    """The sums over stored entries in 64 bits, and over their magnitudes; these with the zero-point's added, because the oracle decodes with
+    two roundings, the product's and the sum's."""
+    hi = c["rows"] if hi is None else hi
+    dec = oracle.unpack_csr(c["bits"], c["policy"], c["row_ptr"], c["packed_row_ptr"], c["col_idx"], c["scales"], c["offsets"], c["packed"]).astype(np.float64)
+    s, e = c["row_ptr"][lo], c["row_ptr"][hi]
+    rows = np.repeat(np.arange(lo, hi), np.diff(c["row_ptr"][lo:hi + 1]))
+    x = np.zeros((hi - lo, c["cols"]))
+    x[rows - lo, c["col_idx"][s:e]] = dec[s:e]
+    return x.T @ g[lo:hi].astype(np.float64), np.abs(x).sum(0) + np.bincount(c["col_idx"][s:e], minlength=c["cols"]) * np.abs(c["offsets"])
+
+
+def assert_within(got, want, l1, g, slices):
+    """G is rounded at 2 max|G| / 2^(8 S - 1) at most (max|G| of the column; 0.99 of the digits' range is used), the oracle's decoded value
+    at 2^-24 of its terms; the sums are exact.  The end of a run, the sums of up to six runs, alpha and beta round at 2^-24 each."""
+    most = np.abs(g).max(0, initial=0.0)
+    bound = (1.02 * 2.0 ** (1 - 8 * slices) + 10 * 2.0 ** -24) * l1[:, None] * most[None, :] + 1e-30
+    worst = np.max(np.abs(got.astype(np.float64) - want) / bound)
+    assert worst <= 1.0, worst
+
+
+def prepared(x, n, slices, device, **kw):
+    """3 digits: fp32 products with the matrix in hand; 4: a request that has to be repeatable."""
+    op = ops.PreparedSpmm(capi.PROJECTION_TRANSPOSE, x.rows, x.cols, n, x.nnz, x.bits, x.policy, torch.float32, device, device_matrix=x,
+                          deterministic=slices == 4, schedule="tensor_blocked" if slices == 3 else None, **kw)
+    assert op.schedule == ("tensor_blocked_x3" if slices == 3 else "gene_gather")
+    return op
+
+
+# fewer cells than a piece, a group and one cell, windows of one gene and of all but one, pieces without entries, tiles of several
+# chunks (dense), and sizes from which on a repeatable request takes integer sums
+@pytest.mark.parametrize("rows,cols,max_nnz,slices", [(31, 129, 60, 3), (257, 128, 90, 3), (256 * 3 + 33, 383, 20, 3), (700, 640, 640, 3),
+                                                      (256 * 20 + 1, 1664, 120, 4), (256 * 17 - 1, 2047, 900, 4)])
+@pytest.mark.parametrize("n,bits", [(64, 8), (32, 4), (32, 8)])
+def test_prepared_against_64_bits(cuda_device, oracle, rows, cols, max_nnz, slices, n, bits):
+    rng = np.random.default_rng(rows + n + bits)
+    c = host_pack(oracle, random_csr(rng, rows=rows, cols=cols, max_nnz=max_nnz, bits=bits))
+    x = to_dev(c, cuda_device)
+    g, g_host = dense(rng, rows, n, torch.float32, cuda_device, std=1.0, ld=n + 3)
+    op = prepared(x, n, slices, cuda_device)
+    want, l1 = reference(oracle, c, g_host)
+    first = op.run(x, g, torch.full((cols, n), float("nan"), device=cuda_device))
+    assert op.status() == 0
+    assert_within(first.cpu().numpy(), want, l1, g_host, slices)
+    assert torch.equal(first, op.run(x, g, torch.full((cols, n), float("nan"), device=cuda_device)))
+    lo, hi = rows // 7, rows - rows // 9                              # borders inside groups and pieces
+    init = rng.normal(size=(cols, n)).astype(np.float32)
+    want, l1 = reference(oracle, c, g_host, lo, hi)
+    room = op.workspace_bytes
+    for op.workspace_bytes in (room, room - 1 if rows < 4096 else room * 3 // 4):  # groups in slices
+        part = op.run(x, g, torch.from_numpy(init).to(cuda_device), alpha=2.0, beta=0.5, row_begin=lo, row_end=hi).cpu().numpy()
+        assert op.status() == 0
+        assert_within(part, 2.0 * want + 0.5 * init, 2.0 * l1 + 1.0, np.maximum(np.abs(g_host[lo:hi]), 1.0), slices)
+    op.close()
+
+
+@pytest.mark.parametrize("n", [1, 33, 64, 100, 130])
+@pytest.mark.parametrize("bits,ordered", [(8, True), (4, True), (8, False)])
+def test_words_made_in_the_call(cuda_device, oracle, n, bits, ordered):
+    """A matrix that is seen once, with enough entries; column blocks with a remainder; rows in any order, a row range."""
+    rng = np.random.default_rng(n + bits)
+    rows, cols = 2111, 1500
+    c = random_csr(rng, rows=rows, cols=cols, max_nnz=3000, bits=bits)
+    if not ordered:
+        for r in range(3, rows, 41):
+            lo, hi = c["row_ptr"][r], c["row_ptr"][r + 1]
+            c["col_idx"][lo:hi] = rng.permutation(c["col_idx"][lo:hi])
+    c = host_pack(oracle, c)
+    x = to_dev(c, cuda_device)
+    assert x.nnz >= 2_200_000
+    g, g_host = dense(rng, rows, n, torch.float32, cuda_device, std=1.0, ld=n + 3)
+    op = ops.PreparedSpmm(capi.PROJECTION_TRANSPOSE, rows, cols, n, x.nnz, bits, 1, torch.float32, cuda_device)
+    assert op.schedule == "vector_reductions" and op.workspace_bytes > 4 * x.nnz
+    for lo, hi in [(0, rows), (5, rows - 40)]:
+        launches = capi.lib().cb200_kernel_launch_count()
+        out = op.run(x, g, torch.full((cols, n), float("nan"), device=cuda_device), row_begin=lo, row_end=hi)
+        assert capi.lib().cb200_kernel_launch_count() - launches == 5 and op.status() == 0
+        want, l1 = reference(oracle, c, g_host, lo, hi)
+        assert_within(out.cpu().numpy(), want, l1, g_host[lo:hi], 4)
+    op.close()
+
+
+def test_long_runs_stay_inside_32_bits(cuda_device):
+    """140,000 cells: more than a run holds.  Every code is 0 (-128 as an operand) and G is the same everywhere: the largest sums there are."""
+    rows, cols, n = 140_000, 40, 32
+    row_ptr = np.arange(rows + 1, dtype=np.int64) * 20
+    col_idx = (2 * np.tile(np.arange(20), rows) + np.repeat(np.arange(rows) & 1, 20)).astype(np.int32)
+    c = dict(rows=rows, cols=cols, bits=8, policy=1, row_ptr=row_ptr, packed_row_ptr=row_ptr, col_idx=col_idx, packed=np.zeros(rows * 20, dtype=np.uint8),
+             scales=np.full(cols, 0.25, dtype=np.float32), offsets=np.full(cols, 0.5, dtype=np.float32))
+    x = to_dev(c, cuda_device)
+    op = prepared(x, n, 3, cuda_device)
+    for value in (0.99, -0.99):
+        out = op.run(x, torch.full((rows, n), value, device=cuda_device), torch.empty(cols, n, device=cuda_device))
+        assert op.status() == 0
+        assert float((out / (np.float32(value).item() * 0.5 * rows / 2) - 1).abs().max()) <= 2.0 ** -22 + 8 * 2.0 ** -24
+    op.close()
+
+
+@pytest.mark.parametrize("slices", [3, 4])
+def test_what_integer_sums_do_not_cover(cuda_device, oracle, slices):
+    """Genes that a cell holds twice count twice; a column with an outlier keeps the others' bits; infinities and NaNs reach the genes of
+    their cells and no others; so do scales that are not finite, of genes with and without entries."""
+    rng = np.random.default_rng(slices)
+    rows, cols, n = 256 * 20, 1664, 64
+    c = host_pack(oracle, random_csr(rng, rows=rows, cols=cols, max_nnz=100, bits=8))
+    c["col_idx"][c["col_idx"] == 300] = 303                           # gene 300 has no entries, rows may not ascend, cells may hold a gene twice
+    assert any(np.any(np.diff(np.sort(c["col_idx"][a:b])) == 0) for a, b in zip(c["row_ptr"][:-1], c["row_ptr"][1:]))
+    x = to_dev(c, cuda_device)
+    g, g_host = dense(rng, rows, n, torch.float32, cuda_device, std=1.0)
+    g_host = g_host.copy()
+    op = prepared(x, n, slices, cuda_device)
+
+    def entry_by_entry():
+        dec = oracle.unpack_csr(8, 1, c["row_ptr"], c["packed_row_ptr"], c["col_idx"], c["scales"], c["offsets"], c["packed"]).astype(np.float64)
+        r = np.repeat(np.arange(rows), np.diff(c["row_ptr"]))
+        want, scale = np.zeros((cols, n)), np.zeros((cols, n))
+        with np.errstate(invalid="ignore"):
+            for j in range(n):
+                np.add.at(want[:, j], c["col_idx"], dec * g_host[r, j])
+                np.add.at(scale[:, j], c["col_idx"], (np.abs(dec) + np.abs(c["offsets"][c["col_idx"]])) * np.abs(g_host[r, j]))
+        return want, scale
+
+    def check():
+        out = op.run(x, torch.from_numpy(g_host).to(cuda_device), torch.empty(cols, n, device=cuda_device))
+        assert op.status() == 0 and torch.equal(out.view(torch.int32), op.run(x, torch.from_numpy(g_host).to(cuda_device), torch.empty(cols, n, device=cuda_device)).view(torch.int32))
+        got, (want, scale) = out.cpu().numpy(), entry_by_entry()
+        finite = np.isfinite(want)
+        assert np.array_equal(np.isnan(got), np.isnan(want)) and np.array_equal(got[np.isinf(want)], want[np.isinf(want)])
+        # an entry's value v = s c + o: rounded once here, at 2^-24 |v|, twice by the oracle, at 2^-24 |s c| <= 2^-24 (|v| + |o|) and 2^-24 |v|;
+        # the sum once at the end, at 2^-24 of itself: four times 2^-24 (|v| + |o|) |g| in all
+        assert np.all(np.abs(got[finite] - want[finite]) <= 2.0 ** -22 * scale[finite] + 1e-30)
+
+    check()
+    g_host[77, 5] = 1e6                                               # in double precision, one rounding at the end
+    check()
+    g_host[123, 9], g_host[4000, 9], g_host[4001, 11] = np.inf, -np.inf, np.nan
+    check()
+    g_host[:] = rng.normal(size=g_host.shape)
+    c["scales"][300], c["offsets"][7] = np.nan, np.inf
+    x.scales.copy_(torch.from_numpy(c["scales"])), x.offsets.copy_(torch.from_numpy(c["offsets"]))
+    out = op.run(x, torch.from_numpy(g_host).to(cuda_device), torch.empty(cols, n, device=cuda_device)).cpu().numpy()
+    assert np.all(out[300] == 0.0) and not np.any(np.isfinite(out[7])) and np.all(np.isfinite(np.delete(out, 7, axis=0)))
+    op.close()
+
+
+def test_bounded_wait_path(cuda_device, oracle):
+    """The loader of G withholds its copies and every wait gives up: the status says so, and the next launch is correct."""
+    rng = np.random.default_rng(4)
+    rows, cols, n = 256 * 6, 1000, 64
+    c = host_pack(oracle, random_csr(rng, rows=rows, cols=cols, max_nnz=100, bits=8, empty_rows=False))
+    x = to_dev(c, cuda_device)
+    g, _ = dense(rng, rows, n, torch.float32, cuda_device, std=1.0)
+    op = prepared(x, n, 3, cuda_device)
+    good = op.run(x, g, torch.empty(cols, n, device=cuda_device)).clone()
+    assert op.status() == 0
+    capi.lib().cb200_test_arm_wait_timeout(4096)
+    try:
+        op.run(x, g, torch.empty(cols, n, device=cuda_device))
+    finally:
+        capi.lib().cb200_test_disarm_wait_timeout()
+    with pytest.raises(capi.Cb200Error) as e:
+        op.status()
+    assert e.value.status == capi.DEVICE_WAIT_TIMEOUT
+    assert torch.equal(op.run(x, g, torch.full((cols, n), float("nan"), device=cuda_device)), good) and op.status() == 0
+    op.close()
