@@ -29,7 +29,7 @@ struct dense_args {
     int epilogue = CB200_EPILOGUE_NONE;   // out = act(alpha * product + beta * out + bias[column])
 };
 
-enum class fwd_schedule : int { warp_per_row = 0, gene_tiled = 1, tensor_windows = 2, tensor_blocked = 3 };
+enum class fwd_schedule : int { warp_per_row = 0, gene_tiled = 1, tensor_windows = 2, tensor_blocked = 3, integer_windows = 4 };
 
 // Device memory a prepared operation keeps.  Two modes: pieces carved out of a block the caller owns (a
 // session's persistent reservation: nothing is allocated or freed here), or pieces allocated one by one
@@ -189,7 +189,7 @@ cb200_status launch_qcsr_forward_blocked(const qcsr_view &x, const dense_args &d
 // Y[r,:] = alpha * sum_i deq(code_i) * W[col_i,:] + beta * Y[r,:]  for r in [row_begin,row_end)
 cb200_status launch_qcsr_forward(const qcsr_view &x, const dense_args &d, std::int64_t row_begin,
                                  std::int64_t row_end, fwd_schedule schedule, const void *persistent,
-                                 const blocked_layout *blocked, bool split_products, void *workspace,
+                                 const blocked_layout *blocked, const struct digit_layout *digits, bool split_products, void *workspace,
                                  std::uint64_t workspace_bytes, int sm_count, cudaStream_t stream);
 
 // Transpose on the tensor cores from the window-blocked copy (N in {32, 64}).  split_products == false:
@@ -204,18 +204,26 @@ cb200_status launch_qcsr_transpose_blocked(const qcsr_view &x, const dense_args 
 
 // Transpose with exact integer sums on the tensor cores (zero-points per gene): codes times the digits of G in fixed point.
 // slices: digits of G, 3 (products as exact as three bf16 ones) or 4 (as fp32 ones).
-// The entries in pieces of 32 cells, by window of 128 genes; scales and zero-points are read at launch.
+// The entries in pieces of 16 or 32 cells (by the number of the matrix's rows), by window of 128 genes, a word each: {code, less 128 if it has 8 bits, place in the operand
+// tile << 8}; scales and zero-points are read at launch.
 struct digit_layout {
     std::uint32_t *words = nullptr;
-    std::uint32_t *bounds = nullptr; // [pieces][windows + 1]
-    std::int64_t *bases = nullptr;   // [pieces]
+    std::uint32_t *bounds = nullptr; // [pieces][windows + 1], from the piece's base
+    std::int64_t *bases = nullptr;   // [pieces]; kDigitWordsTwice: a cell of the piece holds a gene more than once
     std::uint64_t bytes = 0;
     const void *src_row_ptr = nullptr, *src_col_idx = nullptr, *src_packed = nullptr; // arrays it was built from
 };
+constexpr std::int64_t kDigitWordsTwice = 1ll << 62;
+int qcsr_digit_piece_rows(std::int64_t rows);
 bool qcsr_transpose_digits_shape_ok(std::int64_t rows, std::int64_t cols, std::int64_t n, int bits, int policy);
 std::uint64_t qcsr_digit_words_bytes_bound(std::int64_t rows, std::int64_t cols, std::int64_t nnz);
 // current device; memory from `arena`, kernels on `stream`, which is waited for
-cb200_status build_digit_words(const qcsr_view &x, device_arena &arena, cudaStream_t stream, digit_layout *out);
+// forward: the places of the forward kernel's tile, else of the transpose's
+cb200_status build_digit_words(const qcsr_view &x, bool forward, device_arena &arena, cudaStream_t stream, digit_layout *out);
+// ... and without the wait, into memory of that size
+digit_layout digit_words_at(void *memory, const qcsr_view &x);
+cb200_status launch_digit_words(const qcsr_view &x, std::int64_t row_begin, std::int64_t row_end, bool forward, std::uint32_t *words, std::uint32_t *bounds,
+                                std::int64_t *bases, int *status, cudaStream_t stream);
 std::uint64_t qcsr_transpose_digits_workspace_bytes(std::int64_t rows, std::int64_t cols, std::int64_t n, int slices);
 std::uint64_t qcsr_transpose_digits_least_workspace(std::int64_t rows, std::int64_t cols, std::int64_t n, int slices, int sm_count); // slower
 // Whether a call that sees its matrix once should make the words in its workspace (0: no), and what it then needs
@@ -223,6 +231,13 @@ std::uint64_t qcsr_transpose_digits_once_bytes(std::int64_t rows, std::int64_t c
 // layout null: the words are made in the workspace.  *taken is false where the shape or the workspace rules it out.
 cb200_status launch_qcsr_transpose_digits(const qcsr_view &x, const dense_args &d, std::int64_t row_begin, std::int64_t row_end, void *workspace,
                                           std::uint64_t workspace_bytes, const digit_layout *layout, int slices, int sm_count, cudaStream_t stream, bool *taken);
+
+// Forward with exact integer sums of codes times digits of W (zero-points per gene).  layout null: the words are made in the workspace.
+// *taken is false where the shape or the workspace rules it out.
+bool qcsr_forward_digits_shape_ok(std::int64_t rows, std::int64_t cols, std::int64_t n, int bits, int policy);
+std::uint64_t qcsr_forward_digits_workspace_bytes(std::int64_t cols, std::int64_t n);
+cb200_status launch_qcsr_forward_digits(const qcsr_view &x, const dense_args &d, std::int64_t row_begin, std::int64_t row_end, void *workspace,
+                                        std::uint64_t workspace_bytes, const digit_layout *layout, int sm_count, cudaStream_t stream, bool *taken);
 
 // G'[g,:] = alpha * sum_{r in range, col_i == g} deq(code_i) * G[r,:] + beta * G'[g,:]
 // `blocked` (optional): the window-blocked copy of a prepared bf16-product operation.  `digits` (optional): the words of a prepared

@@ -168,6 +168,7 @@ cb200_status route(const cb200_public_layout *l, int32_t projection, const float
         csr.packed_values = l->packed_values; csr.scales = l->column_scales; csr.offsets = offsets_of(*l);
         ln.csr = &csr;
     }
+    if (projection == CB200_PROJECTION_CSR) pr.schedule_hint = "warp_per_row"; // what the scratch has room for
     cb200_prepared *prepared = nullptr;
     st = cb200_spmm_prepare(&pr, &prepared);
     if (st != CB200_STATUS_SUCCESS) return st;
@@ -175,9 +176,13 @@ cb200_status route(const cb200_public_layout *l, int32_t projection, const float
     std::uint32_t align = 256;
     cb200_prepared_workspace(prepared, &need, &align);
     // the exact fp32 schedules these calls select need the status block only; what a CSR projection could use beyond it is not
-    // in the scratch these calls ask for, and the transpose sorts its entries with what the caller's scratch holds beyond it
+    // in the scratch these calls ask for, and the transpose sorts its entries with what the caller's scratch holds beyond it (not
+    // more: with room for it, it would wait on barriers, and these calls' status is that of a schedule that does not)
     if (projection == CB200_PROJECTION_CSR) need = std::min<std::uint64_t>(need, 256u);
-    if (projection == CB200_PROJECTION_TRANSPOSE) need = std::min<std::uint64_t>(need, cur.left / 256u * 256u);
+    if (projection == CB200_PROJECTION_TRANSPOSE) {
+        constexpr int kMostSms = 160;
+        need = std::min<std::uint64_t>({need, cur.left / 256u * 256u, qcsr_transpose_tiled_workspace_bytes(l->rows, l->cols, kMostSms) / 256u * 256u});
+    }
     void *ws = need == 0u ? nullptr : (need <= 256u ? status_block : cur.take(need));
     if (need != 0u && ws == nullptr) {
         cb200_prepared_destroy(prepared);

@@ -590,7 +590,7 @@ std::uint64_t qcsr_gather_workspace_bytes(std::int64_t cols, std::int64_t nnz, s
 
 cb200_status launch_qcsr_forward(const qcsr_view &x, const dense_args &d, std::int64_t row_begin,
                                  std::int64_t row_end, fwd_schedule schedule, const void *persistent,
-                                 const blocked_layout *blocked, bool split_products, void *workspace,
+                                 const blocked_layout *blocked, const digit_layout *digits, bool split_products, void *workspace,
                                  std::uint64_t workspace_bytes, int sm_count, cudaStream_t stream) {
     if (row_end <= row_begin || d.n == 0) return CB200_STATUS_SUCCESS;
     if (row_end - row_begin > 0x7fffffffll) return fail(CB200_STATUS_INVALID_SHAPE, "row range too large for one launch");
@@ -613,6 +613,12 @@ cb200_status launch_qcsr_forward(const qcsr_view &x, const dense_args &d, std::i
         const cb200_status st = launch_qcsr_forward_tiled(x, d, row_begin, row_end, static_cast<int *>(workspace),
                                                           static_cast<const std::int32_t *>(persistent), sm_count,
                                                           stream, &taken);
+        if (st != CB200_STATUS_SUCCESS || taken) return st;
+    }
+    if (schedule == fwd_schedule::integer_windows) {
+        bool taken = false;
+        const cb200_status st = launch_qcsr_forward_digits(x, d, row_begin, row_end, workspace, workspace_bytes,
+                                                           digits != nullptr && digits->words != nullptr ? digits : nullptr, sm_count, stream, &taken);
         if (st != CB200_STATUS_SUCCESS || taken) return st;
     }
     fwd_params p{};

@@ -14,8 +14,8 @@
 // matrices): S = 4 4e-8, where fp32 FMAs leave 1.2e-7 (8,191 cells) to 4.8e-7 (100,003 cells, in a fixed order); S = 3 2e-7, where
 // products put together from three bf16 products and summed by the fp32 MMAs leave 6.2e-6.
 //
-// A column whose largest magnitude is more than 64 times its root mean square, or that holds an infinity or a NaN, would lose
-// bits (or everything) in fixed point: the launch then takes the entries one by one, in double precision and in a fixed order
+// A column whose numbers are small beside its largest (kMostSpread), or that holds an infinity or a NaN, would lose bits (or
+// everything) in fixed point: the launch then takes the entries one by one, in double precision and in a fixed order
 // (finish_kernel).  So does a matrix in which a cell holds a gene twice.  The device decides; nothing is read back.
 //
 // Data.  The entries lie in pieces of 32 cells; inside a piece they are ordered by window of 128 genes, one word per entry
@@ -41,17 +41,21 @@
 #include <algorithm>
 
 namespace cb200 {
+
+// Thirty-two cells to a piece, or sixteen where those would leave SMs without a CTA to lay them out (4,099 x 33,538: 49 us and 38; 8,191
+// rows, two CTAs to most SMs: 65 and 70).
+int qcsr_digit_piece_rows(std::int64_t rows) { return rows >= 32 * 148 ? 32 : 16; }
+
 namespace {
 
 constexpr int kWin = 128;                       // genes per window
 constexpr int kRows = 256;                      // cells per group
-constexpr int kPieceRows = 32;                  // cells whose words one CTA lays out
-constexpr int kGroupPieces = kRows / kPieceRows;
+constexpr int kPieceRows = 32;                  // most cells whose words one CTA lays out
 constexpr int kBuildThreads = 768;
 constexpr int kBuildWarps = kBuildThreads / 32;
-constexpr int kBuildSteps = 8;                  // reads of 32 entries in flight per warp
 constexpr std::uint32_t kPadding = 0x80000000u; // a word that holds no entry
 
+constexpr int kMostGroupPieces = kRows / 16;
 constexpr int kProducerWarps = 16;
 constexpr int kProducerThreads = kProducerWarps * 32;
 constexpr int kGroupThreads = kProducerThreads / 2;
@@ -72,12 +76,16 @@ __host__ __device__ constexpr int set_windows(int nb, int slices) { return 512 /
 __host__ __device__ constexpr int g_piece_bytes(int nb, int slices) { return kGPieceRows * mma_columns(nb, slices); }
 __host__ __device__ constexpr int ring_pieces(int nb, int slices) { return mma_columns(nb, slices) >= 256 ? 5 : mma_columns(nb, slices) >= 192 ? 6 : 8; }
 
-// workspace: status block {status, wide, ...}, largest magnitudes and sums of squares of the columns in parts, steps of the
+// workspace: status block {status, wide, ...}, largest magnitudes and sums of the exponents of the columns in parts, steps of the
 // columns, G in digits, sums of the runs, and for a call that sees its matrix once the words
 constexpr int kParts = 48;
 constexpr int kMaxColumns = 256;
-constexpr std::uint64_t kStepsAt = 256, kPartMaxAt = kStepsAt + kMaxColumns * 8, kPartSquareAt = kPartMaxAt + kParts * kMaxColumns * 4,
-                        kRecordsAt = kPartSquareAt + kParts * kMaxColumns * 8;
+// A column is written in fixed point if its numbers are on average (of the binary exponents of those that are not zero, which a few
+// large ones do not move) not more than 2^6 below the largest: half a step is then at most 2^-24 of the average number, what fp32
+// rounds a product at, while a normal distribution leaves 2^-27 (S = 4; S = 3: 2^-16 and 2^-19).
+constexpr unsigned kMostSpread = 6;
+constexpr std::uint64_t kStepsAt = 256, kPartMaxAt = kStepsAt + kMaxColumns * 8, kPartSumAt = kPartMaxAt + kParts * kMaxColumns * 4,
+                        kRecordsAt = kPartSumAt + kParts * kMaxColumns * 16;
 static_assert(kParts % 48 == 0, "six at a time on up to eight lanes");
 static_assert(kRecordsAt % 256 == 0, "G's records are copied 16 bytes at a time");
 
@@ -93,13 +101,13 @@ struct words_params {
     const std::int32_t *col_idx;
     const std::uint8_t *packed;
     std::int64_t row_begin, row_end, cols;
-    int windows, code_bias;
+    int windows, code_bias, piece_rows;
     std::uint32_t *words;
     std::uint32_t *bounds; // [pieces][windows + 1], from the piece's base
     std::int64_t *bases;   // [pieces]; kTwice: a cell of the piece holds a gene more than once
     int *status;           // cleared, where given
 };
-constexpr std::int64_t kTwice = 1ll << 62;
+constexpr std::int64_t kTwice = kDigitWordsTwice;
 
 // A CTA's cells are one stretch of the CSR arrays, which its warps take 256 entries at a time whatever cells they belong to (rows
 // are of very different lengths: a warp per row took 240 us for 8,191 x 33,538 with 14.7 M entries, this takes 59).  Where genes ascend,
@@ -109,9 +117,10 @@ constexpr std::int64_t kTwice = 1ll << 62;
 // holds twice: a tile has one place for them.
 //
 // What bounds it: the latency of the genes' loads (eight in flight per warp, 48 warps per SM) and issue, half of the slots.
-template<int BITS>
-__global__ void __launch_bounds__(kBuildThreads) digit_words_kernel(const words_params p) {
-    extern __shared__ std::uint32_t place_of[]; // [kPieceRows][pitch]; see below
+// FORWARD: the places are those of the forward kernel's tile (qcsr_forward_digits.cu), in units of two bytes.
+template<int BITS, bool FORWARD>
+__global__ void __launch_bounds__(kBuildThreads, 2) digit_words_kernel(const words_params p) {
+    extern __shared__ std::uint32_t place_of[]; // [kPieceRows][pitch]; see below.  Behind it [chunks][kPieceRows + 1] and [windows]
     __shared__ std::int64_t codes_of[kPieceRows]; // where the codes of a cell begin
     __shared__ int cell_start[kPieceRows + 1];    // from the CTA's first entry
     __shared__ std::uint32_t cell_bits[kPieceRows]; // of the words of a cell
@@ -119,9 +128,9 @@ __global__ void __launch_bounds__(kBuildThreads) digit_words_kernel(const words_
     __shared__ std::uint32_t carry;
     __shared__ int irregular;
     constexpr std::uint32_t kNone = 0xffffffffu;
-    const int tid = threadIdx.x, lane = tid & 31, warp = warp_of_block(), pitch = p.windows;
-    const std::int64_t row0 = p.row_begin + static_cast<std::int64_t>(blockIdx.x) * kPieceRows;
-    const int cells = static_cast<int>(min(static_cast<std::int64_t>(kPieceRows), p.row_end - row0));
+    const int tid = threadIdx.x, lane = tid & 31, warp = warp_of_block(), pitch = p.windows | 1; // an odd pitch: a lane per cell reads without conflicts
+    const std::int64_t row0 = p.row_begin + static_cast<std::int64_t>(blockIdx.x) * p.piece_rows;
+    const int cells = static_cast<int>(min(static_cast<std::int64_t>(p.piece_rows), p.row_end - row0));
     let_next_launch_start();
     if (p.status != nullptr && blockIdx.x == 0 && tid == 0) *p.status = 0;
     const std::int64_t first = __ldg(p.row_ptr + row0);
@@ -129,9 +138,11 @@ __global__ void __launch_bounds__(kBuildThreads) digit_words_kernel(const words_
         const std::int64_t at = __ldg(p.row_ptr + row0 + tid);
         cell_start[tid] = static_cast<int>(at - first);
         if (tid < cells) {
-            const std::uint32_t cell = (blockIdx.x * kPieceRows + tid) & (kRows - 1);
+            const std::uint32_t cell = (blockIdx.x * p.piece_rows + tid) & (kRows - 1);
             codes_of[tid] = p.packed_row_ptr != nullptr ? __ldg(p.packed_row_ptr + row0 + tid) : at;
-            cell_bits[tid] = ((cell >> 7) * (kPlaneBytes / 2) + ((cell & 127u) >> 4 << 4) + (cell & 15u)) << 8 | static_cast<std::uint32_t>(p.code_bias);
+            // transpose: plane half, 16-byte piece, byte; forward (two bytes): cell, 16-byte piece
+            const std::uint32_t place = FORWARD ? cell * 64u + ((cell & 7u) << 3) : (cell >> 7) * (kPlaneBytes / 2) + ((cell & 127u) >> 4 << 4) + (cell & 15u);
+            cell_bits[tid] = place << 8 | static_cast<std::uint32_t>(p.code_bias);
         }
     }
     for (int i = tid; i < kPieceRows * pitch; i += kBuildThreads) place_of[i] = kNone;
@@ -144,45 +155,56 @@ __global__ void __launch_bounds__(kBuildThreads) digit_words_kernel(const words_
     const std::int64_t base = ((first - __ldg(p.row_ptr + p.row_begin) + 3) & ~static_cast<std::int64_t>(3)) + static_cast<std::int64_t>(blockIdx.x) * (4 * p.windows + 4);
     std::uint32_t *out = p.words + base;
 
-    // Work is dealt to the warps in pieces of up to 256 entries of one cell.  A lane holds what its cell needs: the number of the
-    // cell's first piece, where its entries begin, how many they are.
-    const int my_begin = cell_start[min(lane, cells)], my_length = lane < cells ? cell_start[lane + 1] - my_begin : 0;
-    const int my_pieces = (my_length + 32 * kBuildSteps - 1) / (32 * kBuildSteps);
-    int my_first = my_pieces;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        const int below = __shfl_up_sync(0xffffffffu, my_first, d);
-        if (lane >= d) my_first += below;
-    }
-    const int items = __shfl_sync(0xffffffffu, my_first, 31);
-    my_first -= my_pieces;
-    struct piece { int cell, begin, at, length; }; // begin: the cell's first entry, at: the piece's, in the cell
-    const auto piece_at = [&](int item) {
-        const int r = 31 - __clz(__ballot_sync(0xffffffffu, my_first <= item));
-        return piece{r, __shfl_sync(0xffffffffu, my_begin, r), (item - __shfl_sync(0xffffffffu, my_first, r)) * (32 * kBuildSteps), __shfl_sync(0xffffffffu, my_length, r)};
+    // A lane takes four neighbouring entries at a time, at places of the whole matrix that are multiples of four, so that they are one
+    // load; a warp 128 kSteps of them.  e: the first of the four, from the CTA's first entry.
+    const int end = cell_start[cells], skew = static_cast<int>(first & 3);
+    const bool wide_loads = (reinterpret_cast<std::uintptr_t>(p.col_idx) & 15u) == 0u;
+    const auto four_genes = [&](int e) {
+        if (wide_loads && e + 3 < end) return __ldg(reinterpret_cast<const int4 *>(genes + e)); // (entries before the first are the cell's before)
+        const auto at = [&](int k) { return e + k >= 0 && e + k < end ? __ldg(genes + e + k) : 0; };
+        return make_int4(at(0), at(1), at(2), at(3));
+    };
+    struct { int r, begin, next; } in; // the cell of the lane's entry, and where it begins and ends
+    const auto find = [&](int e) { // last cell that begins at or before e and is not empty
+        int lo = 0, hi = cells - 1;
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (cell_start[mid] <= e) lo = mid;
+            else hi = mid - 1;
+        }
+        in = {lo, cell_start[lo], cell_start[lo + 1]};
+    };
+    const auto advance = [&](int e) {
+        while (e >= in.next) in = {in.r + 1, in.next, cell_start[in.r + 2]};
     };
 
     // ---- the first entry of each (cell, window): place_of[cell][window] = its place among the cell's ----
     {
+        constexpr int kSteps = 4;
         bool odd = false;
-        for (int item = warp; item < items; item += kBuildWarps) {
-            const piece w = piece_at(item);
-            const std::int32_t *from = genes + w.begin + w.at + lane;
-            const int left = w.length - w.at; // of the cell, from the piece on
-            std::uint32_t *mine = place_of + w.cell * pitch;
-            int gene[kBuildSteps];
+        for (int e0 = warp * (128 * kSteps) - skew; e0 < end; e0 += kBuildThreads * 4 * kSteps) {
+            int4 four[kSteps];
 #pragma unroll
-            for (int u = 0; u < kBuildSteps; ++u) gene[u] = u * 32 + lane < left ? __ldg(from + u * 32) : 0;
-            int before = w.at > 0 ? __ldg(genes + w.begin + w.at - 1) : -1;
+            for (int u = 0; u < kSteps; ++u) four[u] = four_genes(min(e0 + u * 128 + lane * 4, end));
+            int before = e0 > 0 ? __ldg(genes + e0 - 1) : 0; // of the warp's first entry
+            find(max(e0 + lane * 4, 0));
 #pragma unroll
-            for (int u = 0; u < kBuildSteps; ++u) {
-                if (u * 32 >= left) break;
-                int last = __shfl_up_sync(0xffffffffu, gene[u], 1);
+            for (int u = 0; u < kSteps; ++u) {
+                const int e = e0 + u * 128 + lane * 4;
+                int last = __shfl_up_sync(0xffffffffu, four[u].w, 1);
                 if (lane == 0) last = before;
-                before = __shfl_sync(0xffffffffu, gene[u], 31);
-                const bool valid = u * 32 + lane < left, inside = static_cast<unsigned>(gene[u]) < static_cast<unsigned>(p.cols) && last < gene[u];
-                odd = odd || (valid && !inside);
-                if (valid && inside && static_cast<unsigned>(last ^ gene[u]) >= kWin) mine[gene[u] >> 7] = static_cast<std::uint32_t>(w.at + u * 32 + lane);
+                before = __shfl_sync(0xffffffffu, four[u].w, 31);
+                const int gene[4] = {four[u].x, four[u].y, four[u].z, four[u].w};
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    if (e + j >= 0 && e + j < end) {
+                        advance(e + j);
+                        if (e + j == in.begin) last = -1;
+                        if (static_cast<unsigned>(gene[j]) >= static_cast<unsigned>(p.cols) || last >= gene[j]) odd = true;
+                        else if (static_cast<unsigned>(last ^ gene[j]) >= kWin) place_of[in.r * pitch + (gene[j] >> 7)] = static_cast<std::uint32_t>(e + j - in.begin);
+                    }
+                    last = gene[j];
+                }
             }
         }
         if (odd) irregular = 1;
@@ -197,7 +219,9 @@ __global__ void __launch_bounds__(kBuildThreads) digit_words_kernel(const words_
             }
     };
     const auto word_of = [&](std::uint32_t bits, int gene, std::uint32_t code) {
-        // {code less the bias, place in the tile << 8}: plane half, gene, 16-byte piece of the gene's line ^ gene % 8, byte
+        // {code less the bias, place in the tile << 8}.  Transpose: [plane half][gene][piece ^ gene % 8][byte]; forward: [gene half][cell]
+        // [piece ^ cell % 8][gene % 8]
+        if constexpr (FORWARD) return bits ^ (static_cast<std::uint32_t>(gene & 64) << 16 | static_cast<std::uint32_t>(gene & 63) << 8) ^ code;
         return bits ^ (static_cast<std::uint32_t>(gene & (kWin - 1)) << 15 | static_cast<std::uint32_t>(gene & 7) << 12) ^ code;
     };
     const auto code_at = [&](int r, int i) -> std::uint32_t {
@@ -205,20 +229,20 @@ __global__ void __launch_bounds__(kBuildThreads) digit_words_kernel(const words_
         const std::uint32_t byte = __ldg(p.packed + codes_of[r] + (i >> 1));
         return (i & 1) != 0 ? byte >> 4 : byte & 0xfu;
     };
+    const int chunks = (p.windows + 31) / 32;
+    std::uint32_t *first_in = place_of + kPieceRows * pitch; // [chunk][cell]: the first entry of 32 windows
+    std::uint32_t *start_of = first_in + chunks * (kPieceRows + 1);
     if (ordered) {
-        // windows a cell has no entry in start where the next one does; then {entries << 24 | place of the first}
-        for (int r = warp; r < cells; r += kBuildWarps) {
-            std::uint32_t follow = static_cast<std::uint32_t>(cell_start[r + 1] - cell_start[r]);
-            for (int w0 = (p.windows - 1) & ~31; w0 >= 0; w0 -= 32) {
-                std::uint32_t v = w0 + lane < p.windows ? place_of[r * pitch + w0 + lane] : kNone;
+        // windows a cell has no entry in start where the next one does: inside 32 windows here, beyond them below
+        const int shift = p.piece_rows == 32 ? 5 : 4;
+#pragma unroll 2
+        for (int item = warp; item < chunks << shift; item += kBuildWarps) {
+            const int r = item & (p.piece_rows - 1), chunk = item >> shift, w = chunk * 32 + lane; // (rows past the last hold kNone)
+            std::uint32_t v = w < p.windows ? place_of[r * pitch + w] : kNone;
 #pragma unroll
-                for (int d = 1; d < 32; d <<= 1) v = min(v, __shfl_down_sync(0xffffffffu, v, d)); // the lanes past the end give their own
-                v = min(v, follow);
-                std::uint32_t up = __shfl_down_sync(0xffffffffu, v, 1);
-                if (lane == 31) up = follow;
-                if (w0 + lane < p.windows) place_of[r * pitch + w0 + lane] = (up - v) << 24 | v;
-                follow = __shfl_sync(0xffffffffu, v, 0);
-            }
+            for (int d = 1; d < 32; d <<= 1) v = min(v, __shfl_down_sync(0xffffffffu, v, d)); // the lanes past the end give their own
+            if (w < p.windows) place_of[r * pitch + w] = v;
+            if (lane == 0) first_in[chunk * (kPieceRows + 1) + r] = v;
         }
     } else {
         for (int i = tid; i < kPieceRows * pitch; i += kBuildThreads) place_of[i] = 0u;
@@ -226,15 +250,47 @@ __global__ void __launch_bounds__(kBuildThreads) digit_words_kernel(const words_
         each_entry([&](int r, int gene, int) { atomicAdd(place_of + r * pitch + (gene >> 7), 1u); });
     }
     __syncthreads();
-    // the places: window after window, inside a window cell after cell; a window's words are padded to a multiple of four
+    // The places: window after window, inside a window cell after cell; a window's words are padded to a multiple of four.  A lane per
+    // cell and a run of windows per warp, from the last to the first: place_of[cell][window] becomes, where genes ascend, what to add to
+    // an entry's place in its cell, and otherwise the next free place, both from the window's first.
+    const int share = (p.windows + kBuildWarps - 1) / kBuildWarps, w_first = warp * share, w_last = min(p.windows, w_first + share) - 1;
+    {
+        const bool mine = lane < cells;
+        const std::uint32_t length = mine ? static_cast<std::uint32_t>(cell_start[lane + 1] - cell_start[lane]) : 0u;
+        const auto beyond = [&](int chunk) { // the first entry behind the 32 windows of a chunk
+            std::uint32_t v = length;
+            for (int k = chunk + 1; k < chunks; ++k) v = min(v, first_in[k * (kPieceRows + 1) + lane]);
+            return v;
+        };
+        std::uint32_t follow = length, up = length;
+        if (ordered && w_first <= w_last && mine) {
+            follow = beyond(w_last >> 5);
+            if (w_last + 1 < p.windows) up = min(place_of[lane * pitch + w_last + 1], (w_last + 1) % 32 == 0 ? beyond((w_last + 1) >> 5) : follow);
+        }
+        __syncthreads(); // the window above the warp's has been read
+#pragma unroll 4
+        for (int w = w_last; w >= w_first; --w) {
+            std::uint32_t v = mine ? place_of[lane * pitch + w] : 0u, entries = v;
+            if (ordered) {
+                if (w % 32 == 31 && mine) follow = w + 1 < p.windows ? up : length; // into the chunk before: what follows it is the window above
+                v = mine ? min(v, follow) : 0u;
+                entries = mine ? up - v : 0u;
+                up = v;
+            }
+            std::uint32_t upto = entries;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const std::uint32_t below = __shfl_up_sync(0xffffffffu, upto, d);
+                if (lane >= d) upto += below;
+            }
+            if (mine) place_of[lane * pitch + w] = upto - entries - (ordered ? v : 0u);
+            if (lane == 31) start_of[w] = upto;
+        }
+    }
+    __syncthreads();
     for (int w0 = 0; w0 < p.windows; w0 += kBuildThreads) {
         const int w = w0 + tid;
-        std::uint32_t total = 0u;
-        if (w < p.windows) {
-#pragma unroll 8
-            for (int r = 0; r < cells; ++r) total += ordered ? place_of[r * pitch + w] >> 24 : place_of[r * pitch + w];
-        }
-        const std::uint32_t padded = (total + 3u) & ~3u;
+        const std::uint32_t total = w < p.windows ? start_of[w] : 0u, padded = (total + 3u) & ~3u;
         std::uint32_t upto = padded;
 #pragma unroll
         for (int d = 1; d < 32; d <<= 1) {
@@ -243,23 +299,21 @@ __global__ void __launch_bounds__(kBuildThreads) digit_words_kernel(const words_
         }
         if (lane == 31) warp_sums[warp] = upto;
         __syncthreads();
-        std::uint32_t start = carry + upto - padded;
-        for (int k = 0; k < warp; ++k) start += warp_sums[k];
+        std::uint32_t before = lane < warp ? warp_sums[lane] : 0u;
+        before = __reduce_add_sync(0xffffffffu, before);
+        const std::uint32_t start = carry + before + upto - padded;
         __syncthreads();
         if (tid == kBuildThreads - 1) carry = start + padded;
         if (w < p.windows) {
             p.bounds[static_cast<std::int64_t>(blockIdx.x) * (p.windows + 1) + w] = start;
-            std::uint32_t place = start;
-#pragma unroll 8
-            for (int r = 0; r < cells; ++r) { // ordered: what to add to an entry's place in its cell; otherwise the next free place
-                const std::uint32_t v = place_of[r * pitch + w];
-                place_of[r * pitch + w] = ordered ? place - (v & 0xffffffu) : place;
-                place += ordered ? v >> 24 : v;
-            }
-            for (; place < start + padded; ++place) out[place] = kPadding;
+            start_of[w] = start;
+            for (std::uint32_t k = total; k < padded; ++k) out[start + k] = kPadding;
         }
         __syncthreads();
     }
+    for (int w = w_first; w <= w_last; ++w)
+        if (lane < cells) place_of[lane * pitch + w] += start_of[w];
+    __syncthreads();
     if (tid == 0) {
         p.bounds[static_cast<std::int64_t>(blockIdx.x) * (p.windows + 1) + p.windows] = carry;
         p.bases[blockIdx.x] = base;
@@ -277,7 +331,9 @@ __global__ void __launch_bounds__(kBuildThreads) digit_words_kernel(const words_
             for (std::uint32_t i = bounds[w] + lane; i < bounds[w + 1]; i += 32) {
                 const std::uint32_t e = out[i];
                 if (static_cast<int>(e) < 0) continue;
-                const std::uint32_t gl = (e >> 15) & (kWin - 1), cell = ((((e >> 12) ^ gl) & 7u) << 4 | ((e >> 8) & 15u)) & (kPieceRows - 1);
+                const std::uint32_t place = e >> 8;
+                const std::uint32_t gl = FORWARD ? (place >> 14 & 1u) << 6 | ((place ^ (place >> 3)) & 0x38u) | (place & 7u) : (place >> 7) & (kWin - 1);
+                const std::uint32_t cell = (FORWARD ? place >> 6 : ((place >> 4 ^ gl) & 7u) << 4 | (place & 15u)) & (kPieceRows - 1);
                 twice = twice || (atomicOr(seen + gl, 1u << cell) >> cell & 1u) != 0u;
             }
             __syncwarp();
@@ -285,24 +341,38 @@ __global__ void __launch_bounds__(kBuildThreads) digit_words_kernel(const words_
         if (__syncthreads_or(twice ? 1 : 0) != 0 && tid == 0) p.bases[blockIdx.x] = base | kTwice;
         return;
     }
-    for (int item = warp; item < items; item += kBuildWarps) {
-        const piece w = piece_at(item);
-        const std::int32_t *from = genes + w.begin + w.at + lane;
-        const std::uint8_t *codes = p.packed + codes_of[w.cell] + (BITS == 8 ? w.at + lane : (w.at + lane) >> 1); // (pieces begin at even entries)
-        const int left = w.length - w.at;
-        const std::uint32_t *mine = place_of + w.cell * pitch;
-        const std::uint32_t bits = cell_bits[w.cell];
-        std::uint32_t *dst = out + w.at + lane; // place_of is what to add to an entry's place in its cell: it can be negative
-        int gene[kBuildSteps];
-        std::uint32_t code[kBuildSteps];
+    // Here a warp takes 256 entries of one cell: neighbouring entries of a window go to neighbouring words, so a store of 32 of them touches
+    // six or seven places (four entries to a lane, as above, spread a store over four times as many: 54 us against 38).
+    constexpr int kSteps = 8;
+    const int my_begin = cell_start[min(lane, cells)], my_length = lane < cells ? cell_start[lane + 1] - my_begin : 0;
+    const int my_pieces = (my_length + 32 * kSteps - 1) / (32 * kSteps);
+    int my_first = my_pieces;
 #pragma unroll
-        for (int u = 0; u < kBuildSteps; ++u) {
+    for (int d = 1; d < 32; d <<= 1) {
+        const int below = __shfl_up_sync(0xffffffffu, my_first, d);
+        if (lane >= d) my_first += below;
+    }
+    const int items = __shfl_sync(0xffffffffu, my_first, 31);
+    my_first -= my_pieces;
+    for (int item = warp; item < items; item += kBuildWarps) {
+        const int r = 31 - __clz(__ballot_sync(0xffffffffu, my_first <= item));
+        const int begin = __shfl_sync(0xffffffffu, my_begin, r), at = (item - __shfl_sync(0xffffffffu, my_first, r)) * (32 * kSteps);
+        const int left = __shfl_sync(0xffffffffu, my_length, r) - at; // of the cell, from here on
+        const std::int32_t *from = genes + begin + at + lane;
+        const std::uint8_t *codes = p.packed + codes_of[r] + (BITS == 8 ? at + lane : (at + lane) >> 1); // (`at` is even)
+        const std::uint32_t *mine = place_of + r * pitch;
+        const std::uint32_t bits = cell_bits[r];
+        std::uint32_t *dst = out + at + lane; // place_of is what to add to an entry's place in its cell: it can be negative
+        int gene[kSteps];
+        std::uint32_t code[kSteps];
+#pragma unroll
+        for (int u = 0; u < kSteps; ++u) {
             const bool valid = u * 32 + lane < left;
             gene[u] = valid ? __ldg(from + u * 32) : 0;
             code[u] = valid ? __ldg(codes + (BITS == 8 ? u * 32 : u * 16)) : 0u;
         }
 #pragma unroll
-        for (int u = 0; u < kBuildSteps; ++u) {
+        for (int u = 0; u < kSteps; ++u) {
             if (u * 32 + lane >= left) break;
             std::uint32_t c = code[u];
             if constexpr (BITS == 4) c = (lane & 1) != 0 ? c >> 4 : c & 0xfu;
@@ -313,23 +383,25 @@ __global__ void __launch_bounds__(kBuildThreads) digit_words_kernel(const words_
 
 // ---- G in digits -----------------------------------------------------------------------------------------------------------
 
-// Largest magnitude (as bits; an infinity or a NaN is the largest) and sum of squares of each column, in kParts parts.  HBM or L2.
+// Largest magnitude (as bits; an infinity or a NaN is the largest) of each column, and the binary exponents' sum and number where
+// a number is not zero, in kParts parts.  HBM or L2.
 __global__ void __launch_bounds__(1024) column_range_kernel(const float *g, std::int64_t ld, int n, int padded, std::int64_t row_begin, std::int64_t row_end,
-                                                            unsigned *part_max, double *part_square, int *status) {
+                                                            unsigned *part_max, ulonglong2 *part_sum, int *status) {
     __shared__ unsigned most_of[1024];
-    __shared__ double square_of[1024];
+    __shared__ unsigned exponents_of[1024], count_of[1024];
     let_next_launch_start();
     if (status != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *status = 0;
     const int c = threadIdx.x % padded, lanes = 1024 / padded;
-    unsigned most = 0u;
-    double square = 0.0;
+    unsigned most = 0u, exponents = 0u, count = 0u;
     if (c < n) {
         const std::int64_t step = static_cast<std::int64_t>(gridDim.x) * lanes;
         std::int64_t r = row_begin + static_cast<std::int64_t>(blockIdx.x) * lanes + threadIdx.x / padded;
         const float *at = g + r * ld + c;
         const auto take = [&](float v) {
-            most = max(most, __float_as_uint(v) & 0x7fffffffu);
-            square = fma(static_cast<double>(v), static_cast<double>(v), square);
+            const unsigned bits = __float_as_uint(v) & 0x7fffffffu;
+            most = max(most, bits);
+            exponents += bits >> 23;
+            count += bits != 0u ? 1u : 0u;
         };
         for (; r + 7 * step < row_end; r += 8 * step, at += 8 * step * ld) {
             float v[8];
@@ -341,15 +413,18 @@ __global__ void __launch_bounds__(1024) column_range_kernel(const float *g, std:
         for (; r < row_end; r += step, at += step * ld) take(__ldg(at));
     }
     most_of[threadIdx.x] = most;
-    square_of[threadIdx.x] = square;
+    exponents_of[threadIdx.x] = exponents;
+    count_of[threadIdx.x] = count;
     __syncthreads();
     if (threadIdx.x < static_cast<unsigned>(padded)) {
+        unsigned long long sum = exponents, number = count;
         for (int k = 1; k < lanes; ++k) {
             most = max(most, most_of[threadIdx.x + k * padded]);
-            square += square_of[threadIdx.x + k * padded];
+            sum += exponents_of[threadIdx.x + k * padded];
+            number += count_of[threadIdx.x + k * padded];
         }
         part_max[blockIdx.x * kMaxColumns + threadIdx.x] = most;
-        part_square[blockIdx.x * kMaxColumns + threadIdx.x] = square;
+        part_sum[blockIdx.x * kMaxColumns + threadIdx.x] = make_ulonglong2(sum, number);
     }
     // beside digit_words_kernel in a call that makes its words: what waits for this kernel waits for that one too
     wait_for_previous_launch();
@@ -361,10 +436,10 @@ __global__ void __launch_bounds__(1024) column_range_kernel(const float *g, std:
 // Every block adds the parts up for itself; the first one writes the columns' steps and whether the entries have to be taken one by one.
 template<int NB, int SLICES>
 __global__ void __launch_bounds__(256) pack_digits_kernel(const float *g, std::int64_t ld, int n, int padded, std::int64_t first_row, std::int64_t row_begin,
-                                                          std::int64_t row_end, std::int64_t groups, const unsigned *part_max, const double *part_square,
+                                                          std::int64_t row_end, std::int64_t groups, const unsigned *part_max, const ulonglong2 *part_sum,
                                                           double *steps, unsigned char *records, const std::int64_t *bases, std::int64_t word_pieces, int *wide) {
     __shared__ unsigned most_of[256];
-    __shared__ double square_of[256];
+    __shared__ ulonglong2 sum_of[256];
     __shared__ double factor[kMaxColumns]; // 2^k: what a column is multiplied by
     wait_for_previous_launch();
     let_next_launch_start();
@@ -372,41 +447,42 @@ __global__ void __launch_bounds__(256) pack_digits_kernel(const float *g, std::i
     {
         const int c = tid % padded, lanes = 256 / padded;
         unsigned most = 0u;
-        double square = 0.0;
+        ulonglong2 sum = make_ulonglong2(0u, 0u);
         for (int k0 = tid / padded; k0 < kParts; k0 += 6 * lanes) { // lanes 1, 2, 4, 8: six loads of each kind in flight
             unsigned m[6];
-            double q[6];
+            ulonglong2 q[6];
 #pragma unroll
             for (int k = 0; k < 6; ++k) {
                 m[k] = __ldcg(part_max + (k0 + k * lanes) * kMaxColumns + c);
-                q[k] = __ldcg(part_square + (k0 + k * lanes) * kMaxColumns + c);
+                q[k] = __ldcg(part_sum + (k0 + k * lanes) * kMaxColumns + c);
             }
 #pragma unroll
             for (int k = 0; k < 6; ++k) {
                 most = max(most, m[k]);
-                square += q[k];
+                sum.x += q[k].x;
+                sum.y += q[k].y;
             }
         }
         most_of[tid] = most;
-        square_of[tid] = square;
+        sum_of[tid] = sum;
         __syncthreads();
         int too_wide = 0;
         if (tid < padded) {
             for (int k = 1; k < lanes; ++k) {
                 most = max(most, most_of[tid + k * padded]);
-                square += square_of[tid + k * padded];
+                sum.x += sum_of[tid + k * padded].x;
+                sum.y += sum_of[tid + k * padded].y;
             }
             double f = 0.0, step = 0.0;
             if (most >= 0x7f800000u) {
                 too_wide = 1;
             } else if (most != 0u) {
-                const double largest = static_cast<double>(__uint_as_float(most));
                 // largest = m 2^e, m in [0.5, 1); the largest number of S balanced digits is 0.996 * 2^(8 S - 1)
                 const int e = most >= 0x800000u ? static_cast<int>(most >> 23) - 126 : 32 - __clz(most) - 149;
                 const int k = 8 * SLICES - 1 - e - ((most & 0x7fffffu) > 8220000u || most < 0x800000u ? 1 : 0);
                 f = __longlong_as_double(static_cast<long long>(1023 + k) << 52);
                 step = __longlong_as_double(static_cast<long long>(1023 - k) << 52);
-                too_wide = largest * largest * static_cast<double>(row_end - row_begin) > 4096.0 * square ? 1 : 0;
+                too_wide = (most >> 23) * sum.y > sum.x + kMostSpread * sum.y ? 1 : 0;
             }
             factor[tid] = f;
             if (blockIdx.x == 0) steps[tid] = step;
@@ -464,10 +540,11 @@ struct digit_params {
     const std::uint32_t *bounds;
     const std::int64_t *bases;
     std::int64_t pieces;
+    int group_pieces, piece_rows;
     const float *scales, *offsets;
     const unsigned char *records;
     const double *steps;
-    const int *wide;
+    const int *wide;         // a column of G does not fit, or a cell holds a gene twice
     float *partials;         // [run_of + CTA][window of the set][gene][NB]
     std::int64_t cols;
     std::int64_t group_begin, group_count;
@@ -765,7 +842,7 @@ __global__ void __launch_bounds__(kThreads, 1) qcsr_transpose_digits_kernel(cons
             fills[0] = issued;
         }
     } else {
-        // ================= the words: a warp per scatter group; a tile's lie in the group's eight pieces, a lane each =================
+        // ================= the words: a warp per scatter group; a tile's lie in the group's eight or sixteen pieces, a lane each =================
         const int ring = warp == kProducerWarps + 1 ? 0 : 1;
         const std::uint32_t full = smem_addr(c_full + ring), empty = smem_addr(c_empty + ring), dst = chunk0 + ring * kChunkBytes;
         tile_cursor at(p, sets, u0, kSet);
@@ -776,8 +853,8 @@ __global__ void __launch_bounds__(kThreads, 1) qcsr_transpose_digits_kernel(cons
         std::int64_t base = 0;
         const auto fetch = [&]() {
             lo = hi = 0u;
-            const std::int64_t piece = (p.group_begin + at.group) * kGroupPieces + lane;
-            if (at.unit < u1 && lane < kGroupPieces && piece < p.pieces) {
+            const std::int64_t piece = (p.group_begin + at.group) * p.group_pieces + lane;
+            if (at.unit < u1 && lane < p.group_pieces && piece < p.pieces) {
                 const std::uint32_t *bound = p.bounds + piece * (p.windows + 1) + at.set * kSet + at.wl;
                 lo = __ldcg(bound);
                 hi = __ldcg(bound + 1);
@@ -795,11 +872,11 @@ __global__ void __launch_bounds__(kThreads, 1) qcsr_transpose_digits_kernel(cons
             fetch();
             int upto = words;
 #pragma unroll
-            for (int d = 1; d < kGroupPieces; d <<= 1) {
+            for (int d = 1; d < kMostGroupPieces; d <<= 1) {
                 const int below = __shfl_up_sync(0xffffffffu, upto, d);
                 if (lane >= d) upto += below;
             }
-            const int begin = upto - words, total = __shfl_sync(0xffffffffu, upto, kGroupPieces - 1);
+            const int begin = upto - words, total = __shfl_sync(0xffffffffu, upto, kMostGroupPieces - 1);
             int c0 = 0;
             do {
                 const int n = min(kChunkEntries, total - c0);
@@ -812,7 +889,7 @@ __global__ void __launch_bounds__(kThreads, 1) qcsr_transpose_digits_kernel(cons
                 }
                 __syncwarp();
                 const int first = max(begin, c0), last = min(begin + words, c0 + n);
-                if (lane < kGroupPieces && first < last)
+                if (first < last)
                     bulk_copy_g2s(dst + (first - c0) * 4, src + (first - begin), static_cast<std::uint32_t>(last - first) * 4u, full);
                 __syncwarp();
                 ++done;
@@ -882,16 +959,16 @@ __global__ void __launch_bounds__(256) finish_kernel(const finish_params p) {
         meta[tid] = so;
         odd = isfinite(so.x) && isfinite(so.y) ? 0 : 1;
     }
-    const bool slow = __syncthreads_or(odd) != 0 || *p.d.wide != 0;
+    const bool slow = __syncthreads_or(odd) != 0 || __ldcg(p.d.wide) != 0;
     if (slow) {
         for (int i = tid; i < kWin * NB; i += 256) slow_sums[i] = 0.0;
         __syncthreads();
-        const std::int64_t piece0 = (p.row_begin - p.first_row) / kPieceRows, piece1 = (p.row_end - p.first_row + kPieceRows - 1) / kPieceRows;
+        const std::int64_t piece0 = (p.row_begin - p.first_row) / p.d.piece_rows, piece1 = (p.row_end - p.first_row + p.d.piece_rows - 1) / p.d.piece_rows;
         for (std::int64_t piece = piece0; piece < piece1; ++piece) {
             const std::uint32_t *at = p.d.bounds + piece * (p.d.windows + 1) + window;
             const int words = static_cast<int>(__ldcg(at + 1) - __ldcg(at));
             const std::uint32_t *w = p.d.words + (__ldcg(p.d.bases + piece) & (kTwice - 1)) + __ldcg(at);
-            const std::int64_t group_row = p.first_row + piece / kGroupPieces * kRows;
+            const std::int64_t group_row = p.first_row + piece / p.d.group_pieces * kRows;
             for (int i0 = 0; i0 < words; i0 += 32) {
                 const std::uint32_t e = i0 + lane < words ? __ldcg(w + i0 + lane) : kPadding;
                 const int place = static_cast<int>((e >> 8) & 0x7fffu), gl = (place >> 7) & (kWin - 1);
@@ -976,33 +1053,15 @@ std::uint64_t launch_bytes(std::int64_t groups, std::int64_t cols, std::int64_t 
     return kRecordsAt + record_bytes(groups, n, slices) + partial_bytes(groups, cols, n, slices, ctas);
 }
 std::int64_t group_count_of(std::int64_t rows) { return (rows + kRows - 1) / kRows; }
-std::int64_t piece_count(std::int64_t rows) { return (rows + kPieceRows - 1) / kPieceRows; }
+std::int64_t piece_count(std::int64_t rows) { return (rows + qcsr_digit_piece_rows(rows) - 1) / qcsr_digit_piece_rows(rows); }
 std::uint64_t word_bytes(std::int64_t rows, std::int64_t cols, std::int64_t nnz) {
     const std::int64_t windows = (cols + kWin - 1) / kWin;
     return static_cast<std::uint64_t>(nnz + 4 + piece_count(rows) * (4 * windows + 4)) * 4u;
 }
 std::uint64_t bound_bytes(std::int64_t rows, std::int64_t cols) { return static_cast<std::uint64_t>(piece_count(rows) * ((cols + kWin - 1) / kWin + 1)) * 4u; }
-int build_smem_bytes(std::int64_t cols) { return static_cast<int>(kPieceRows * ((cols + kWin - 1) / kWin) * 4); }
-
-cb200_status launch_words(const qcsr_view &x, std::int64_t row_begin, std::int64_t row_end, std::uint32_t *words, std::uint32_t *bounds,
-                          std::int64_t *bases, int *status, cudaStream_t stream) {
-    words_params p{};
-    p.row_ptr = x.row_ptr; p.packed_row_ptr = x.packed_row_ptr; p.col_idx = x.col_idx; p.packed = x.packed;
-    p.row_begin = row_begin; p.row_end = row_end; p.cols = x.cols; p.windows = static_cast<int>((x.cols + kWin - 1) / kWin);
-    p.code_bias = x.bits == 8 ? 128 : 0;
-    p.words = words; p.bounds = bounds; p.bases = bases; p.status = status;
-    const int smem = build_smem_bytes(x.cols);
-    const unsigned grid = static_cast<unsigned>(piece_count(row_end - row_begin));
-    if (x.bits == 8) {
-        CB200_CUDA_OK(cudaFuncSetAttribute(digit_words_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        digit_words_kernel<8><<<grid, kBuildThreads, smem, stream>>>(p);
-    } else {
-        CB200_CUDA_OK(cudaFuncSetAttribute(digit_words_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        digit_words_kernel<4><<<grid, kBuildThreads, smem, stream>>>(p);
-    }
-    count_launch();
-    CB200_CUDA_OK(cudaGetLastError());
-    return CB200_STATUS_SUCCESS;
+int build_smem_bytes(std::int64_t cols) {
+    const std::int64_t windows = (cols + kWin - 1) / kWin;
+    return static_cast<int>((kPieceRows * (windows | 1) + (windows + 31) / 32 * (kPieceRows + 1) + windows) * 4);
 }
 
 struct digit_launch {
@@ -1010,7 +1069,8 @@ struct digit_launch {
     finish_params finish;
     std::int64_t slice;      // groups at a time
     unsigned *part_max;
-    double *part_square, *steps;
+    ulonglong2 *part_sum;
+    double *steps;
     unsigned char *records;
     int *wide;
     bool early; // the launch in front is a kernel of this call
@@ -1025,7 +1085,7 @@ cb200_status launch_digits(const digit_launch &l, int sm_count, cudaStream_t str
     CB200_CUDA_OK(cudaFuncSetAttribute(finish_kernel<NB, SLICES>, cudaFuncAttributeMaxDynamicSharedMemorySize, slow_smem));
     const int n = l.finish.n, padded = padded_columns(n);
     CB200_CUDA_OK(launch_kernel(l.early, column_range_kernel, dim3(kParts), 1024, 0, stream, l.finish.g, l.finish.g_ld, n, padded, l.finish.row_begin, l.finish.row_end,
-                                l.part_max, l.part_square, l.early ? nullptr : l.main.status));
+                                l.part_max, l.part_sum, l.early ? nullptr : l.main.status));
     const std::int64_t group_end = l.main.group_begin + l.main.group_count;
     for (std::int64_t begin = l.main.group_begin; begin < group_end; begin += l.slice) {
         digit_params m = l.main;
@@ -1035,7 +1095,7 @@ cb200_status launch_digits(const digit_launch &l, int sm_count, cudaStream_t str
         m.partials = reinterpret_cast<float *>(l.records + record_bytes(m.group_count, n, SLICES));
         const std::int64_t row0 = f.first_row + begin * kRows, blocks = m.group_count * m.column_blocks;
         CB200_CUDA_OK(launch_kernel(true, pack_digits_kernel<NB, SLICES>, dim3(static_cast<unsigned>(std::min<std::int64_t>(blocks * kGPieces, 4 * sm_count))), 256, 0, stream, f.g,
-                                    f.g_ld, n, padded, row0, f.row_begin, f.row_end, m.group_count, l.part_max, l.part_square, l.steps, l.records, m.bases, m.pieces,
+                                    f.g_ld, n, padded, row0, f.row_begin, f.row_end, m.group_count, l.part_max, l.part_sum, l.steps, l.records, m.bases, m.pieces,
                                     l.wide));
         const std::int64_t sets = (m.windows + set_windows(NB, SLICES) - 1) / set_windows(NB, SLICES);
         const unsigned grid = static_cast<unsigned>(std::min<std::int64_t>(sets * blocks, sm_count));
@@ -1056,14 +1116,46 @@ cb200_status launch_digits(const digit_launch &l, int sm_count, cudaStream_t str
 
 } // namespace
 
+cb200_status launch_digit_words(const qcsr_view &x, std::int64_t row_begin, std::int64_t row_end, bool forward, std::uint32_t *words, std::uint32_t *bounds,
+                                std::int64_t *bases, int *status, cudaStream_t stream) {
+    words_params p{};
+    p.row_ptr = x.row_ptr; p.packed_row_ptr = x.packed_row_ptr; p.col_idx = x.col_idx; p.packed = x.packed;
+    p.row_begin = row_begin; p.row_end = row_end; p.cols = x.cols; p.windows = static_cast<int>((x.cols + kWin - 1) / kWin);
+    p.code_bias = x.bits == 8 ? 128 : 0;
+    p.piece_rows = qcsr_digit_piece_rows(x.rows);
+    p.words = words; p.bounds = bounds; p.bases = bases; p.status = status;
+    const int smem = build_smem_bytes(x.cols);
+    const unsigned grid = static_cast<unsigned>((row_end - row_begin + p.piece_rows - 1) / p.piece_rows);
+    const auto run = [&](auto kernel) {
+        const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (err == cudaSuccess) kernel<<<grid, kBuildThreads, smem, stream>>>(p);
+        return err;
+    };
+    if (x.bits == 8) CB200_CUDA_OK(forward ? run(digit_words_kernel<8, true>) : run(digit_words_kernel<8, false>));
+    else CB200_CUDA_OK(forward ? run(digit_words_kernel<4, true>) : run(digit_words_kernel<4, false>));
+    count_launch();
+    CB200_CUDA_OK(cudaGetLastError());
+    return CB200_STATUS_SUCCESS;
+}
+
 bool qcsr_transpose_digits_shape_ok(std::int64_t rows, std::int64_t cols, std::int64_t n, int bits, int policy) {
-    // the counters of a piece have to fit in shared memory: 224,000 genes
+    // the counters of a piece have to fit in shared memory: 190,000 genes
     return (bits == 8 || bits == 4) && policy == CB200_DECODE_PER_GENE_AFFINE && n > 0 && n <= kMaxColumns && rows > 0 && cols > 0 &&
-           (cols + kWin - 1) / kWin * kPieceRows * 4 <= 224 * 1024;
+           cols <= 190'000 && build_smem_bytes(cols) <= 210 * 1024;
 }
 std::uint64_t qcsr_digit_words_bytes_bound(std::int64_t rows, std::int64_t cols, std::int64_t nnz) {
     return device_arena::rounded(word_bytes(rows, cols, nnz)) + device_arena::rounded(bound_bytes(rows, cols)) +
            device_arena::rounded(static_cast<std::uint64_t>(piece_count(rows)) * 8u);
+}
+digit_layout digit_words_at(void *memory, const qcsr_view &x) {
+    unsigned char *at = static_cast<unsigned char *>(memory);
+    digit_layout l;
+    l.words = reinterpret_cast<std::uint32_t *>(at);
+    at += device_arena::rounded(word_bytes(x.rows, x.cols, x.nnz));
+    l.bounds = reinterpret_cast<std::uint32_t *>(at);
+    at += device_arena::rounded(bound_bytes(x.rows, x.cols));
+    l.bases = reinterpret_cast<std::int64_t *>(at);
+    return l;
 }
 std::uint64_t qcsr_transpose_digits_workspace_bytes(std::int64_t rows, std::int64_t cols, std::int64_t n, int slices) {
     return launch_bytes(group_count_of(rows), cols, n, slices, kMaxCtas);
@@ -1080,7 +1172,7 @@ std::uint64_t qcsr_transpose_digits_once_bytes(std::int64_t rows, std::int64_t c
     return qcsr_transpose_digits_workspace_bytes(rows, cols, n, 4) + qcsr_digit_words_bytes_bound(rows, cols, nnz);
 }
 
-cb200_status build_digit_words(const qcsr_view &x, device_arena &arena, cudaStream_t stream, digit_layout *out) {
+cb200_status build_digit_words(const qcsr_view &x, bool forward, device_arena &arena, cudaStream_t stream, digit_layout *out) {
     *out = digit_layout{};
     if (x.row_ptr == nullptr || (x.nnz != 0 && (x.col_idx == nullptr || x.packed == nullptr)))
         return fail(CB200_STATUS_INVALID_ARGUMENT, "the matrix handed to prepare has null arrays");
@@ -1091,11 +1183,11 @@ cb200_status build_digit_words(const qcsr_view &x, device_arena &arena, cudaStre
     out->bases = static_cast<std::int64_t *>(arena.take(bases));
     cb200_status st = CB200_STATUS_SUCCESS;
     if (out->words == nullptr || out->bounds == nullptr || out->bases == nullptr)
-        st = fail(CB200_STATUS_INSUFFICIENT_WORKSPACE, "no device memory for the entry words of the transpose");
-    if (st == CB200_STATUS_SUCCESS) st = launch_words(x, 0, x.rows, out->words, out->bounds, out->bases, nullptr, stream);
+        st = fail(CB200_STATUS_INSUFFICIENT_WORKSPACE, "no device memory for the entry words");
+    if (st == CB200_STATUS_SUCCESS) st = launch_digit_words(x, 0, x.rows, forward, out->words, out->bounds, out->bases, nullptr, stream);
     if (st == CB200_STATUS_SUCCESS) {
         const cudaError_t err = cudaStreamSynchronize(stream);
-        if (err != cudaSuccess) st = fail(CB200_STATUS_CUDA_ERROR, "building the entry words of the transpose: %s", cudaGetErrorString(err));
+        if (err != cudaSuccess) st = fail(CB200_STATUS_CUDA_ERROR, "building the entry words: %s", cudaGetErrorString(err));
     }
     if (st != CB200_STATUS_SUCCESS) {
         arena.give_back(out->bases, bases);
@@ -1131,7 +1223,7 @@ cb200_status launch_qcsr_transpose_digits(const qcsr_view &x, const dense_args &
     digit_launch l{};
     l.early = layout == nullptr;
     l.part_max = reinterpret_cast<unsigned *>(ws + kPartMaxAt);
-    l.part_square = reinterpret_cast<double *>(ws + kPartSquareAt);
+    l.part_sum = reinterpret_cast<ulonglong2 *>(ws + kPartSumAt);
     l.steps = reinterpret_cast<double *>(ws + kStepsAt);
     l.records = ws + kRecordsAt;
     l.wide = reinterpret_cast<int *>(ws) + 1;
@@ -1141,18 +1233,15 @@ cb200_status launch_qcsr_transpose_digits(const qcsr_view &x, const dense_args &
     if (layout != nullptr) {
         p.words = layout->words; p.bounds = layout->bounds; p.bases = layout->bases;
     } else {
-        unsigned char *at = ws + own;
-        std::uint32_t *words = reinterpret_cast<std::uint32_t *>(at);
-        at += device_arena::rounded(word_bytes(x.rows, x.cols, x.nnz));
-        std::uint32_t *bounds = reinterpret_cast<std::uint32_t *>(at);
-        at += device_arena::rounded(bound_bytes(x.rows, x.cols));
-        std::int64_t *bases = reinterpret_cast<std::int64_t *>(at);
-        const cb200_status st = launch_words(x, row_begin, row_end, words, bounds, bases, p.status, stream);
+        const digit_layout made = digit_words_at(ws + own, x);
+        const cb200_status st = launch_digit_words(x, row_begin, row_end, false, made.words, made.bounds, made.bases, p.status, stream);
         if (st != CB200_STATUS_SUCCESS) return st;
-        p.words = words; p.bounds = bounds; p.bases = bases;
+        p.words = made.words; p.bounds = made.bounds; p.bases = made.bases;
     }
     const int nb = column_block(d.n);
-    p.pieces = piece_count(rows_of_words);
+    p.piece_rows = qcsr_digit_piece_rows(x.rows);
+    p.group_pieces = kRows / p.piece_rows;
+    p.pieces = (rows_of_words + p.piece_rows - 1) / p.piece_rows;
     p.scales = x.scales; p.offsets = x.offsets;
     p.records = l.records; p.steps = l.steps; p.wide = l.wide;
     p.cols = x.cols;
