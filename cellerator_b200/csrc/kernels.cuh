@@ -233,11 +233,12 @@ cb200_status launch_qcsr_transpose_digits(const qcsr_view &x, const dense_args &
                                           std::uint64_t workspace_bytes, const digit_layout *layout, int slices, int sm_count, cudaStream_t stream, bool *taken);
 
 // Forward with exact integer sums of codes times digits of W (zero-points per gene).  layout null: the words are made in the workspace.
-// *taken is false where the shape or the workspace rules it out.
+// *wide is null where the shape or the workspace rules it out, else the device's word that says whether W fits fixed point: where it is
+// not 0, the launches have left Y alone and the caller's next one takes the rows.
 bool qcsr_forward_digits_shape_ok(std::int64_t rows, std::int64_t cols, std::int64_t n, int bits, int policy);
 std::uint64_t qcsr_forward_digits_workspace_bytes(std::int64_t cols, std::int64_t n);
 cb200_status launch_qcsr_forward_digits(const qcsr_view &x, const dense_args &d, std::int64_t row_begin, std::int64_t row_end, void *workspace,
-                                        std::uint64_t workspace_bytes, const digit_layout *layout, int sm_count, cudaStream_t stream, bool *taken);
+                                        std::uint64_t workspace_bytes, const digit_layout *layout, int sm_count, cudaStream_t stream, const int **wide);
 
 // G'[g,:] = alpha * sum_{r in range, col_i == g} deq(code_i) * G[r,:] + beta * G'[g,:]
 // `blocked` (optional): the window-blocked copy of a prepared bf16-product operation.  `digits` (optional): the words of a prepared

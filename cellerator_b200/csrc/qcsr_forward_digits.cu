@@ -13,8 +13,8 @@
 // Against 64 bits (2-norm, 20,000 x 2,000 and 4,099 x 33,538): 4.3e-8 and 4.6e-8, where fp32 FMAs leave 1.1e-7 and 1.3e-7.
 //
 // A column whose operands are small beside the largest (kMostSpread), or an operand that is not finite, does not fit: the
-// device notices while it lays W out, this kernel then does nothing, and the one behind it takes all rows entry by entry, in double
-// precision.  So are the rows of pieces in which a cell holds a gene twice.
+// device notices while it lays W out, this kernel then does nothing, and the gather kernel behind it takes all rows.  The rows of pieces
+// in which a cell holds a gene twice are summed here, entry by entry.
 //
 // Data.  The entries come as words {code, place in the tile}, in pieces of 16 or 32 cells and inside them by window of 128 genes
 // (digit_words_kernel); a prepared operation keeps them, a call that sees its matrix once makes them in its workspace.  (Reading the
@@ -316,56 +316,43 @@ __device__ __forceinline__ bool cell_is_odd(const fwd_digit_params &p, int group
     const std::int64_t at = static_cast<std::int64_t>(p.first_group + group) * p.group_pieces + r / p.piece_rows;
     return at < p.pieces && (__ldcg(p.bases + at) & kDigitWordsTwice) != 0;
 }
-// Columns [c0, c0 + nb) of a row by one warp, in double precision: 32 entries are decoded at a time, then their rows of W are
-// read one after another, two columns of 64 to a lane.
+__device__ __forceinline__ void put_sum(const fwd_digit_params &p, std::int64_t row, int c, double sum) {
+    float v = p.alpha * static_cast<float>(sum);
+    float *dst = p.out + row * p.out_ld + c;
+    if (p.beta != 0.0f) v = fmaf(p.beta, *dst, v);
+    *dst = finish_output(v, p.bias, c, p.epilogue);
+}
+// A warp's columns [c0, c0 + nb) of a row, entry by entry: 32 of them decoded at a time, two columns of 64 to a lane; fp32 FMAs over
+// 32 entries, whose sums are added in double precision.
 __device__ __noinline__ void row_by_entries(const fwd_digit_params &p, std::int64_t row, int c0, int nb, int lane) {
-    const std::int64_t begin = __ldg(p.row_ptr + row), end = __ldg(p.row_ptr + row + 1);
+    const std::int64_t begin = __ldg(p.row_ptr + row), length = __ldg(p.row_ptr + row + 1) - begin;
     const std::uint8_t *codes = p.packed + (p.packed_row_ptr != nullptr ? __ldg(p.packed_row_ptr + row) : begin);
-    const int most = min(c0 + nb, p.n), ca = c0 + lane, cb = c0 + 32 + lane;
-    const auto w_at = [&](std::int64_t gene, int c) -> float {
-        if (c >= most) return 0.0f;
-        return p.w_bf16 != 0 ? load1(static_cast<const __nv_bfloat16 *>(p.w) + gene * p.w_ld + c) : load1(static_cast<const float *>(p.w) + gene * p.w_ld + c);
-    };
-    double a = 0.0, b = 0.0;
-    for (std::int64_t e0 = begin; e0 < end; e0 += 32) {
-        const std::int64_t i = e0 - begin + lane;
-        int gene = -1;
+    const int end = min(c0 + nb, p.n), ca = min(c0 + lane, end - 1), cb = min(c0 + 32 + lane, end - 1); // (lanes past the last column read it again)
+    double sum_a = 0.0, sum_b = 0.0;
+    for (std::int64_t e0 = 0; e0 < length; e0 += 32) {
+        const std::int64_t i = e0 + lane;
+        int gene = i < length ? __ldg(p.col_idx + begin + i) : -1;
+        const std::uint32_t valid_of = __ballot_sync(0xffffffffu, gene >= 0 && gene < p.cols); // others, and those past the end, add nothing
         float value = 0.0f;
-        if (e0 + lane < end) gene = __ldg(p.col_idx + e0 + lane);
-        if (gene >= 0 && gene < p.cols) {
+        if ((valid_of >> lane & 1u) != 0u) {
             unsigned code = __ldg(codes + (p.bits == 8 ? i : i >> 1));
             if (p.bits == 4) code = (i & 1) != 0 ? code >> 4 : code & 0xfu;
             const float2 so = p.meta.of(gene);
             value = fmaf(static_cast<float>(code), so.x, so.y);
         }
-        const std::uint32_t valid = __ballot_sync(0xffffffffu, gene >= 0 && gene < p.cols);
-#pragma unroll 8
-        for (int j = 0; j < 32; ++j) {
-            const int g = __shfl_sync(0xffffffffu, gene, j);
-            const double v = static_cast<double>(__shfl_sync(0xffffffffu, value, j));
-            if ((valid >> j & 1u) == 0u) continue; // warp-uniform
-            a = fma(v, static_cast<double>(w_at(g, ca)), a);
-            b = fma(v, static_cast<double>(w_at(g, cb)), b);
+        float a = 0.0f, b = 0.0f;
+        for (std::uint32_t left = valid_of; left != 0u; left &= left - 1u) {
+            const int j = __ffs(left) - 1;
+            const std::int64_t at = __shfl_sync(0xffffffffu, gene, j) * p.w_ld;
+            const float v = __shfl_sync(0xffffffffu, value, j);
+            a = fmaf(v, p.w_bf16 != 0 ? load1(static_cast<const __nv_bfloat16 *>(p.w) + at + ca) : load1(static_cast<const float *>(p.w) + at + ca), a);
+            b = fmaf(v, p.w_bf16 != 0 ? load1(static_cast<const __nv_bfloat16 *>(p.w) + at + cb) : load1(static_cast<const float *>(p.w) + at + cb), b);
         }
+        sum_a += static_cast<double>(a);
+        sum_b += static_cast<double>(b);
     }
-    const auto put = [&](int c, double sum) {
-        if (c >= most) return;
-        float v = p.alpha * static_cast<float>(sum);
-        float *dst = p.out + row * p.out_ld + c;
-        if (p.beta != 0.0f) v = fmaf(p.beta, *dst, v);
-        *dst = finish_output(v, p.bias, c, p.epilogue);
-    };
-    put(ca, a);
-    put(cb, b);
-}
-
-// All rows, where W does not fit fixed point; a warp per row and column block.
-__global__ void __launch_bounds__(256) rows_by_entries_kernel(const __grid_constant__ fwd_digit_params p, int nb) {
-    wait_for_previous_launch();
-    if (__ldcg(p.wide) == 0) return;
-    const std::int64_t rows = p.row_end - p.row_begin, warps = static_cast<std::int64_t>(gridDim.x) * 8;
-    for (std::int64_t i = static_cast<std::int64_t>(blockIdx.x) * 8 + (threadIdx.x >> 5); i < rows * p.column_blocks; i += warps)
-        row_by_entries(p, p.row_begin + i % rows, static_cast<int>(i / rows) * nb, nb, threadIdx.x & 31);
+    if (c0 + lane < end) put_sum(p, row, c0 + lane, sum_a);
+    if (c0 + 32 + lane < end) put_sum(p, row, c0 + 32 + lane, sum_b);
 }
 
 template<int NB>
@@ -422,7 +409,7 @@ __global__ void __launch_bounds__(kThreads, 1) qcsr_fwd_digits_kernel(const __gr
     const int ctas = static_cast<int>(gridDim.x);
     const std::int64_t total = static_cast<std::int64_t>(p.column_blocks) * p.groups * p.windows;
     const std::int64_t t0 = share_begin(total, blockIdx.x, ctas);
-    const std::int64_t t1 = __ldcg(p.wide) != 0 ? t0 : share_begin(total, blockIdx.x + 1, ctas); // too wide: rows_by_entries_kernel's work
+    const std::int64_t t1 = __ldcg(p.wide) != 0 ? t0 : share_begin(total, blockIdx.x + 1, ctas); // too wide: the gather kernel's work
 
     if (warp < kScatterWarps) {
         // ================= zero, scatter, read back =================
@@ -760,9 +747,7 @@ cb200_status launch_all(const fwd_digit_params &p, unsigned *part_max, ulonglong
         CB200_CUDA_OK(launch_kernel(true, sum_parts_kernel<NB>, dim3(static_cast<unsigned>(cuts.count), kRows / 32, NB / 8), 256, 0, stream, p, cuts));
         count_launch();
     }
-    const std::int64_t by_warp = (p.row_end - p.row_begin) * p.column_blocks;
-    CB200_CUDA_OK(launch_kernel(true, rows_by_entries_kernel, dim3(static_cast<unsigned>(std::min<std::int64_t>((by_warp + 7) / 8, 8 * sm_count))), 256, 0, stream, p, NB));
-    count_launch(4);
+    count_launch(3);
     CB200_CUDA_OK(cudaGetLastError());
     return CB200_STATUS_SUCCESS;
 }
@@ -775,8 +760,8 @@ bool qcsr_forward_digits_shape_ok(std::int64_t rows, std::int64_t cols, std::int
 std::uint64_t qcsr_forward_digits_workspace_bytes(std::int64_t cols, std::int64_t n) { return kRecordsAt + record_bytes(cols, n) + slot_bytes(n); }
 
 cb200_status launch_qcsr_forward_digits(const qcsr_view &x, const dense_args &d, std::int64_t row_begin, std::int64_t row_end, void *workspace,
-                                        std::uint64_t workspace_bytes, const digit_layout *layout, int sm_count, cudaStream_t stream, bool *taken) {
-    *taken = false;
+                                        std::uint64_t workspace_bytes, const digit_layout *layout, int sm_count, cudaStream_t stream, const int **wide_word) {
+    *wide_word = nullptr;
     const std::uint64_t own = qcsr_forward_digits_workspace_bytes(x.cols, d.n);
     if (!qcsr_forward_digits_shape_ok(x.rows, x.cols, d.n, x.bits, x.policy) || workspace == nullptr || reinterpret_cast<std::uintptr_t>(workspace) % 256u != 0u ||
         workspace_bytes < own + (layout == nullptr ? qcsr_digit_words_bytes_bound(x.rows, x.cols, x.nnz) : 0u) || sm_count > kMaxCtas ||
@@ -824,7 +809,7 @@ cb200_status launch_qcsr_forward_digits(const qcsr_view &x, const dense_args &d,
     p.poll_limit = test_poll_limit();
     unsigned *part_max = reinterpret_cast<unsigned *>(ws + kPartMaxAt);
     ulonglong2 *part_sum = reinterpret_cast<ulonglong2 *>(ws + kPartSumAt);
-    *taken = true;
+    *wide_word = wide;
     if (d.dense_dtype == CB200_DTYPE_BF16)
         return nb == 64 ? launch_all<__nv_bfloat16, 64>(p, part_max, part_sum, steps, records, wide, layout == nullptr, sm_count, stream)
                         : launch_all<__nv_bfloat16, 32>(p, part_max, part_sum, steps, records, wide, layout == nullptr, sm_count, stream);

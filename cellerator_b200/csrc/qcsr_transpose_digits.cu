@@ -14,9 +14,10 @@
 // matrices): S = 4 4e-8, where fp32 FMAs leave 1.2e-7 (8,191 cells) to 4.8e-7 (100,003 cells, in a fixed order); S = 3 2e-7, where
 // products put together from three bf16 products and summed by the fp32 MMAs leave 6.2e-6.
 //
-// A column whose numbers are small beside its largest (kMostSpread), or that holds an infinity or a NaN, would lose bits (or
-// everything) in fixed point: the launch then takes the entries one by one, in double precision and in a fixed order
-// (finish_kernel).  So does a matrix in which a cell holds a gene twice.  The device decides; nothing is read back.
+// Where the numbers of a column are small beside its largest (kMostSpread), the launch takes as many digits again, those behind the
+// first ones, in a second pass over the tiles: 62 bits (S = 4) or 46.  A column that spreads further, or holds an infinity or a NaN,
+// and a matrix in which a cell holds a gene twice, are taken entry by entry, in double precision and in a fixed order
+// (finish_kernel).  The device decides; nothing is read back.
 //
 // Data.  The entries lie in pieces of 32 cells; inside a piece they are ordered by window of 128 genes, one word per entry
 // {code, place in the operand tile}, cell after cell (digit_words_kernel: a CTA per piece counts the entries of each cell and window in
@@ -76,15 +77,15 @@ __host__ __device__ constexpr int set_windows(int nb, int slices) { return 512 /
 __host__ __device__ constexpr int g_piece_bytes(int nb, int slices) { return kGPieceRows * mma_columns(nb, slices); }
 __host__ __device__ constexpr int ring_pieces(int nb, int slices) { return mma_columns(nb, slices) >= 256 ? 5 : mma_columns(nb, slices) >= 192 ? 6 : 8; }
 
-// workspace: status block {status, wide, ...}, largest magnitudes and sums of the exponents of the columns in parts, steps of the
+// workspace: status block {status, passes, ...}, largest magnitudes and sums of the exponents of the columns in parts, steps of the
 // columns, G in digits, sums of the runs, and for a call that sees its matrix once the words
 constexpr int kParts = 48;
 constexpr int kMaxColumns = 256;
-// A column is written in fixed point if its numbers are on average (of the binary exponents of those that are not zero, which a few
+// One pass serves a column if its numbers are on average (of the binary exponents of those that are not zero, which a few
 // large ones do not move) not more than 2^6 below the largest: half a step is then at most 2^-24 of the average number, what fp32
 // rounds a product at, while a normal distribution leaves 2^-27 (S = 4; S = 3: 2^-16 and 2^-19).
 constexpr unsigned kMostSpread = 6;
-constexpr std::uint64_t kStepsAt = 256, kPartMaxAt = kStepsAt + kMaxColumns * 8, kPartSumAt = kPartMaxAt + kParts * kMaxColumns * 4,
+constexpr std::uint64_t kStepsAt = 256, kPartMaxAt = kStepsAt + 2 * kMaxColumns * 8, kPartSumAt = kPartMaxAt + kParts * kMaxColumns * 4,
                         kRecordsAt = kPartSumAt + kParts * kMaxColumns * 16;
 static_assert(kParts % 48 == 0, "six at a time on up to eight lanes");
 static_assert(kRecordsAt % 256 == 0, "G's records are copied 16 bytes at a time");
@@ -430,10 +431,10 @@ __global__ void __launch_bounds__(1024) column_range_kernel(const float *g, std:
     wait_for_previous_launch();
 }
 
-// G -> per (block of NB columns, group of 256 cells) a record of four pieces of 64 cells, each the S NB x 64 digits in the no-swizzle
+// G -> per (pass, block of NB columns, group of 256 cells) a record of four pieces of 64 cells, each the S NB x 64 digits in the no-swizzle
 // K-major operand layout (byte of (column k NB + c: digit k of column c, the highest first; cell r) = column / 8 * 512 + r / 16 *
 // 128 + column % 8 * 16 + r % 16).  Cells outside [row_begin, row_end) and columns from n on are zero.
-// Every block adds the parts up for itself; the first one writes the columns' steps and whether the entries have to be taken one by one.
+// Every block adds the parts up for itself; the first one writes the columns' steps and how the launch goes on (digit_params::wide).
 template<int NB, int SLICES>
 __global__ void __launch_bounds__(256) pack_digits_kernel(const float *g, std::int64_t ld, int n, int padded, std::int64_t first_row, std::int64_t row_begin,
                                                           std::int64_t row_end, std::int64_t groups, const unsigned *part_max, const ulonglong2 *part_sum,
@@ -441,6 +442,9 @@ __global__ void __launch_bounds__(256) pack_digits_kernel(const float *g, std::i
     __shared__ unsigned most_of[256];
     __shared__ ulonglong2 sum_of[256];
     __shared__ double factor[kMaxColumns]; // 2^k: what a column is multiplied by
+    // the second pass takes up what the first rounds off, at most half a step
+    constexpr double kSecond = 1.0 / static_cast<double>(1ull << (8 * SLICES - 1));
+    int passes;
     wait_for_previous_launch();
     let_next_launch_start();
     const int tid = threadIdx.x;
@@ -475,29 +479,36 @@ __global__ void __launch_bounds__(256) pack_digits_kernel(const float *g, std::i
             }
             double f = 0.0, step = 0.0;
             if (most >= 0x7f800000u) {
-                too_wide = 1;
+                too_wide = 2;
             } else if (most != 0u) {
                 // largest = m 2^e, m in [0.5, 1); the largest number of S balanced digits is 0.996 * 2^(8 S - 1)
                 const int e = most >= 0x800000u ? static_cast<int>(most >> 23) - 126 : 32 - __clz(most) - 149;
                 const int k = 8 * SLICES - 1 - e - ((most & 0x7fffffu) > 8220000u || most < 0x800000u ? 1 : 0);
                 f = __longlong_as_double(static_cast<long long>(1023 + k) << 52);
                 step = __longlong_as_double(static_cast<long long>(1023 - k) << 52);
-                too_wide = (most >> 23) * sum.y > sum.x + kMostSpread * sum.y ? 1 : 0;
+                const unsigned long long spread = (most >> 23) * sum.y - sum.x; // times the number of numbers
+                too_wide = spread <= kMostSpread * sum.y ? 0 : spread <= (kMostSpread + 8 * SLICES - 1) * sum.y ? 1 : 2;
             }
             factor[tid] = f;
-            if (blockIdx.x == 0) steps[tid] = step;
+            if (blockIdx.x == 0) {
+                const int columns = (n + NB - 1) / NB * NB;
+                if (tid < columns) steps[tid] = step;
+                if (tid < columns) steps[columns + tid] = step * kSecond; // of the second pass
+            }
         }
         if (blockIdx.x == 0) {
 #pragma unroll 8
-            for (std::int64_t k = tid; k < word_pieces; k += 256) too_wide |= (__ldcg(bases + k) & kTwice) != 0 ? 1 : 0;
+            for (std::int64_t k = tid; k < word_pieces; k += 256) too_wide |= (__ldcg(bases + k) & kTwice) != 0 ? 2 : 0;
         }
-        too_wide = __syncthreads_or(too_wide);
-        if (blockIdx.x == 0 && tid == 0) *wide = too_wide;
+        const bool second = __syncthreads_or(too_wide & 1) != 0, by_entry = __syncthreads_or(too_wide & 2) != 0;
+        if (blockIdx.x == 0 && tid == 0) *wide = by_entry ? 2 : second ? 1 : 0;
+        passes = second ? 2 : 1;
     }
     constexpr int NC = mma_columns(NB, SLICES);
     const std::int64_t pieces = static_cast<std::int64_t>((n + NB - 1) / NB) * groups * kGPieces;
-    for (std::int64_t b = blockIdx.x; b < pieces; b += gridDim.x) {
-        const int c0 = static_cast<int>(b / (groups * kGPieces)) * NB;
+    for (std::int64_t b = blockIdx.x; b < passes * pieces; b += gridDim.x) {
+        const bool second = b >= pieces;
+        const int c0 = static_cast<int>((second ? b - pieces : b) / (groups * kGPieces)) * NB;
         const std::int64_t row0 = first_row + b % (groups * kGPieces) * kGPieceRows;
         unsigned char *rec = records + b * (kGPieceRows * NC);
         for (int item = tid; item < NB * (kGPieceRows / 16); item += 256) {
@@ -516,7 +527,9 @@ __global__ void __launch_bounds__(256) pack_digits_kernel(const float *g, std::i
                 for (int w = 0; w < 4; ++w) digit[k][w] = 0u;
 #pragma unroll
             for (int j = 0; j < 16; ++j) {
-                int q = __double2int_rn(static_cast<double>(v[j]) * f);
+                const double scaled = static_cast<double>(v[j]) * f;
+                int q = __double2int_rn(scaled);
+                if (second) q = __double2int_rn((scaled - static_cast<double>(q)) * (1.0 / kSecond));
 #pragma unroll
                 for (int k = SLICES - 1; k >= 0; --k) {
                     digit[k][j >> 2] |= (static_cast<std::uint32_t>(q) & 0xffu) << ((j & 3) * 8);
@@ -544,7 +557,7 @@ struct digit_params {
     const float *scales, *offsets;
     const unsigned char *records;
     const double *steps;
-    const int *wide;         // a column of G does not fit, or a cell holds a gene twice
+    const int *wide;         // 0: one pass, 1: two, 2: entry by entry
     float *partials;         // [run_of + CTA][window of the set][gene][NB]
     std::int64_t cols;
     std::int64_t group_begin, group_count;
@@ -649,10 +662,12 @@ __global__ void __launch_bounds__(kThreads, 1) qcsr_transpose_digits_kernel(cons
     wait_for_previous_launch();
 
     const std::int64_t sets = (p.windows + kSet - 1) / kSet;
-    const std::int64_t total_units = sets * p.column_blocks * p.group_count;
+    const int wide = __ldcg(p.wide);
+    // the second pass: as many column blocks again
+    const std::int64_t total_units = sets * p.column_blocks * p.group_count * (wide == 1 ? 2 : 1);
     const std::int64_t u0 = total_units * blockIdx.x / gridDim.x;
-    // a column that does not fit fixed point: nothing to do here, finish_kernel takes the entries one by one
-    const std::int64_t u1 = __ldcg(p.wide) != 0 ? u0 : total_units * (blockIdx.x + 1) / gridDim.x;
+    // entry by entry: nothing to do here, it is finish_kernel's work
+    const std::int64_t u1 = wide == 2 ? u0 : total_units * (blockIdx.x + 1) / gridDim.x;
 
     if (warp < kProducerWarps) {
         // ================= zero, scatter, read back =================
@@ -947,9 +962,8 @@ __global__ void __launch_bounds__(256) finish_kernel(const finish_params p) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const std::int64_t sets = (p.d.windows + kSet - 1) / kSet;
     const int wl = static_cast<int>(blockIdx.x % kSet);
-    const std::int64_t set = blockIdx.x / kSet, window = set * kSet + wl; // the set among the block's, and among all of them:
+    const std::int64_t set = blockIdx.x / kSet, window = set * kSet + wl;
     const int c0 = static_cast<int>(blockIdx.y) * NB;
-    const std::int64_t set_of_all = blockIdx.y * sets + set;
     if (window >= p.d.windows) return;
     int odd = 0;
     if (tid < kWin) {
@@ -959,7 +973,8 @@ __global__ void __launch_bounds__(256) finish_kernel(const finish_params p) {
         meta[tid] = so;
         odd = isfinite(so.x) && isfinite(so.y) ? 0 : 1;
     }
-    const bool slow = __syncthreads_or(odd) != 0 || __ldcg(p.d.wide) != 0;
+    const int wide = __ldcg(p.d.wide);
+    const bool slow = __syncthreads_or(odd) != 0 || wide == 2;
     if (slow) {
         for (int i = tid; i < kWin * NB; i += 256) slow_sums[i] = 0.0;
         __syncthreads();
@@ -990,24 +1005,26 @@ __global__ void __launch_bounds__(256) finish_kernel(const finish_params p) {
         }
         __syncthreads();
     }
-    // the set's slots: the CTAs whose shares meet its runs, run after run
-    const std::int64_t total = sets * p.d.column_blocks * p.d.group_count, L = p.d.group_count, cuts = (L + p.d.run_groups - 1) / p.d.run_groups;
-    const auto from_of = [&](std::int64_t cut) { return set_of_all * L + cut * p.d.run_groups; };
-    const auto to_of = [&](std::int64_t cut) { return min(from_of(cut) + p.d.run_groups, (set_of_all + 1) * L); };
-    const std::int64_t first0 = cta_of(from_of(0), total, p.grid), last0 = cta_of(to_of(0) - 1, total, p.grid);
+    // the set's slots: the CTAs whose shares meet its runs, run after run, pass after pass
+    const int passes = wide == 1 ? 2 : 1;
+    const std::int64_t total = sets * p.d.column_blocks * p.d.group_count * passes, L = p.d.group_count, cuts = (L + p.d.run_groups - 1) / p.d.run_groups;
     constexpr int kItems = kWin * (NB / 4) / 256; // of a thread
     float4 sums[kItems];
 #pragma unroll
     for (int k = 0; k < kItems; ++k) sums[k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    for (std::int64_t cut = 0; cut < cuts && !slow; ++cut) {
-        const std::int64_t last = cut == 0 ? last0 : cta_of(to_of(cut) - 1, total, p.grid);
-        for (std::int64_t b = cut == 0 ? first0 : cta_of(from_of(cut), total, p.grid); b <= last; ++b) {
-            const float4 *slot = reinterpret_cast<const float4 *>(p.d.partials + ((set_of_all * cuts + cut + b) * kSet + wl) * kWin * NB) + tid;
-            float4 v[kItems];
+    for (int pass = 0; pass < passes && !slow; ++pass) {
+        const std::int64_t set_of_all = (static_cast<std::int64_t>(pass) * p.d.column_blocks + blockIdx.y) * sets + set;
+        for (std::int64_t cut = 0; cut < cuts; ++cut) {
+            const std::int64_t from = set_of_all * L + cut * p.d.run_groups, to = min(from + p.d.run_groups, (set_of_all + 1) * L);
+            const std::int64_t last = cta_of(to - 1, total, p.grid);
+            for (std::int64_t b = cta_of(from, total, p.grid); b <= last; ++b) {
+                const float4 *slot = reinterpret_cast<const float4 *>(p.d.partials + ((set_of_all * cuts + cut + b) * kSet + wl) * kWin * NB) + tid;
+                float4 v[kItems];
 #pragma unroll
-            for (int k = 0; k < kItems; ++k) v[k] = __ldcg(slot + k * 256);
+                for (int k = 0; k < kItems; ++k) v[k] = __ldcg(slot + k * 256);
 #pragma unroll
-            for (int k = 0; k < kItems; ++k) { sums[k].x += v[k].x; sums[k].y += v[k].y; sums[k].z += v[k].z; sums[k].w += v[k].w; }
+                for (int k = 0; k < kItems; ++k) { sums[k].x += v[k].x; sums[k].y += v[k].y; sums[k].z += v[k].z; sums[k].w += v[k].w; }
+            }
         }
     }
 #pragma unroll
@@ -1038,15 +1055,16 @@ __global__ void __launch_bounds__(256) finish_kernel(const finish_params p) {
 int column_block(std::int64_t n) { return n <= 32 ? 32 : 64; }
 int padded_columns(std::int64_t n) { return n <= 32 ? 32 : n <= 64 ? 64 : n <= 128 ? 128 : 256; }
 
+// (both with room for the second pass)
 std::uint64_t record_bytes(std::int64_t groups, std::int64_t n, int slices) {
     const int nb = column_block(n);
-    return device_arena::rounded(static_cast<std::uint64_t>(groups) * static_cast<std::uint64_t>((n + nb - 1) / nb) * kRows * static_cast<std::uint64_t>(mma_columns(nb, slices)));
+    return device_arena::rounded(2u * static_cast<std::uint64_t>(groups) * static_cast<std::uint64_t>((n + nb - 1) / nb) * kRows * static_cast<std::uint64_t>(mma_columns(nb, slices)));
 }
 // a run ends with its set, after kRunGroups groups, or with its CTA's share of the units
 std::uint64_t partial_bytes(std::int64_t groups, std::int64_t cols, std::int64_t n, int slices, int ctas) {
     const std::int64_t nb = column_block(n), per_set = set_windows(static_cast<int>(nb), slices), windows = (cols + kWin - 1) / kWin;
     const std::int64_t sets = (windows + per_set - 1) / per_set * ((n + nb - 1) / nb), cuts = (groups + kRunGroups - 1) / kRunGroups;
-    return device_arena::rounded(static_cast<std::uint64_t>(sets * cuts + ctas) * static_cast<std::uint64_t>(per_set * kWin * nb) * sizeof(float));
+    return device_arena::rounded(static_cast<std::uint64_t>(2 * sets * cuts + ctas) * static_cast<std::uint64_t>(per_set * kWin * nb) * sizeof(float));
 }
 // what a launch over `groups` groups at a time needs, without the words
 std::uint64_t launch_bytes(std::int64_t groups, std::int64_t cols, std::int64_t n, int slices, int ctas) {

@@ -106,7 +106,8 @@ def test_what_integer_sums_do_not_cover(cuda_device, oracle):
             finite = np.isfinite(want)
             assert np.array_equal(np.isnan(got), np.isnan(want)) and np.array_equal(got[np.isinf(want)], want[np.isinf(want)])
             # fixed point: half a step, 2^-30.9 of the largest operand, counts up to 382 times an entry, and the average operand is not more than 2^6
-            # below the largest: 2^-15 of it at worst, 2^-19 where, as here, only uniform scales and normal W spread them; else double precision
+            # below the largest: 2^-15 of it at worst, 2^-19 where, as here, only uniform scales and normal W spread them; else fp32 products,
+            # in sums of up to 100: 100 * 2^-24 of them at worst
             assert np.all(np.abs(got[finite] - want[finite]) <= 2.0 ** -19 * scale[finite] + 1e-30)
 
     check()
@@ -117,6 +118,22 @@ def test_what_integer_sums_do_not_cover(cuda_device, oracle):
     w_host[:] = rng.normal(size=w_host.shape)
     c["scales"][500], c["offsets"][7] = np.nan, np.inf
     check()
+
+
+@pytest.mark.parametrize("bits,n,dtype", [(8, 64, torch.float32), (4, 50, torch.bfloat16), (8, 33, torch.bfloat16), (4, 100, torch.float32), (8, 3, torch.float32)])
+def test_a_wide_operand_gets_the_gather_kernels_bits(cuda_device, oracle, bits, n, dtype):
+    """More groups of rows than are resident at a time, a last one that is not full, and a row range."""
+    rng = np.random.default_rng(n)
+    rows, cols = 8 * 2 * 148 * 2 + 5, 700
+    x = to_dev(host_pack(oracle, random_csr(rng, rows=rows, cols=cols, max_nnz=300, bits=bits)), cuda_device)
+    w, _ = dense(rng, cols, n, dtype, cuda_device)
+    w[5] = 1e6
+    gather = ops.PreparedSpmm(capi.PROJECTION_CSR, rows, cols, n, x.nnz, bits, 1, dtype, cuda_device, schedule="warp_per_row")
+    op = prepare(x, n, dtype, cuda_device)
+    y = gather.run(x, w, torch.empty(rows, n, device=cuda_device))
+    assert torch.equal(op.run(x, w, torch.full_like(y, float("nan"))), y) and op.status() == 0
+    part = op.run(x, w, torch.full_like(y, -3.0), row_begin=130, row_end=rows - 9)
+    assert torch.equal(part[130:-9], y[130:-9]) and torch.all(part[:130] == -3.0) and torch.all(part[-9:] == -3.0)
 
 
 def test_bounded_wait_path(cuda_device, oracle):
