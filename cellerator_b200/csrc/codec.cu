@@ -133,14 +133,18 @@ __global__ void __launch_bounds__(256) dequantize_rows_kernel(const codec_params
 // take six or seven cycles, and goes through its rows once per range: genes ascend in a row, so a range is a contiguous piece
 // of it, found by bisection.  Pieces are cut at multiples of 32 entries (bytes, for 4-bit codes); the few entries on the wrong
 // side of a cut, and any that a row which does not ascend has out of place, are looked up in global memory.  CTAs get equal
-// shares of the entries, and a CTA's warps draw blocks of at most 1,024 of them, so that a long row holds up nobody.
+// shares of the entries, and a CTA's warps draw blocks of at most 1,152 of them, so that a long row holds up nobody.
 //
-// 100,000 x 33,538, 180 M entries of 8 bits: coding 1.74 -> 0.42 ms, decoding 0.76 -> 0.37 ms (9 bytes per entry: 3.9 and
-// 4.4 TB/s); bound by the latency of the one step of loads a warp has in flight at 32 warps per SM.
+// 100,000 x 33,538, 180 M entries of 8 bits: coding 1.74 -> 0.42 ms, decoding 0.76 -> 0.37 ms with an entry to a lane; with four
+// neighbouring ones (16-byte loads and stores, a step of 384 entries) 0.785 -> 0.68-0.69 ms together, 4.7 TB/s.  Bound by issue (57 % of the
+// slots when coding) and by the latency of the one step of loads a warp has in flight at 32 warps per SM.  Measured on the way there: two
+// groups a step 0.73 ms, four 0.83 (registers), one 0.86; groups that hold a neighbour row's entries too, masked entry by entry, 0.76; the row's
+// start looked up in global memory for each block 0.70; a rest of a row in steps of its own length 0.82 (three copies of the step for the
+// instruction cache); more than 196 KB of shared memory, which leaves L1 28 KB, 0.82.
 constexpr int kTableThreads = 1024;
 constexpr int kTableGenes = 20 * 1024; // genes of a range: 160 KB
-constexpr int kTableRows = 4 * 1024;   // rows of a CTA between two loads of the table: 48 KB of places
-constexpr int kTableBlock = 1024;      // units (entries, bytes) a warp draws
+constexpr int kTableRows = 2 * 1024;   // rows of a CTA between two loads of the table: 40 KB of places
+constexpr int kTableBlock = 1152;      // units (entries, bytes) a warp draws: three steps of 384
 
 // first row in [lo, hi] whose start is at least `target` (one warp; the rows' starts ascend)
 __device__ __forceinline__ std::int64_t first_row_from(const std::int64_t *row_ptr, std::int64_t lo, std::int64_t hi, std::int64_t target) {
@@ -157,10 +161,11 @@ __device__ __forceinline__ std::int64_t first_row_from(const std::int64_t *row_p
 }
 
 template<int BITS, bool CODE>
-__global__ void __launch_bounds__(kTableThreads, 1) codec_table_kernel(const codec_params p, int range_genes, int ranges) {
-    constexpr int CPB = 8 / BITS, U = BITS == 8 ? 6 : 4; // steps of loads in flight, what 64 registers hold
+__global__ void __launch_bounds__(kTableThreads, 1) codec_table_kernel(const codec_params p, int range_genes, int ranges, bool quads) {
+    constexpr int CPB = 8 / BITS, kQuads = 3, U = BITS == 8 ? 6 : 4; // steps of loads in flight, what 64 registers hold
     extern __shared__ __align__(16) float2 codec_table[];
-    int *from = reinterpret_cast<int *>(codec_table + range_genes); // [kTableRows] first unit of the row in this range
+    std::int64_t *begins = reinterpret_cast<std::int64_t *>(codec_table + range_genes); // [kTableRows] first entry of the row
+    int *from = reinterpret_cast<int *>(begins + kTableRows);       // [kTableRows] first unit of the row in this range
     int *upto = from + kTableRows;                                  // [kTableRows] ... and past its last
     int *blocks = upto + kTableRows;                                // [kTableRows] blocks of this range up to and with the row
     __shared__ std::int64_t share[2];
@@ -207,6 +212,7 @@ __global__ void __launch_bounds__(kTableThreads, 1) codec_table_kernel(const cod
                         }
                         last = max(first, min(units, ((lo / CPB + lead) / 32) * 32));
                     }
+                    if (range == 0) begins[r] = begin;
                     from[r] = first;
                     upto[r] = last;
                     count = (last - first + kTableBlock - 1) / kTableBlock;
@@ -235,11 +241,12 @@ __global__ void __launch_bounds__(kTableThreads, 1) codec_table_kernel(const cod
                 __syncthreads();
             }
             const int all_blocks = carry;
-            for (;;) {
-                int block = 0;
-                if (lane == 0) block = atomicAdd(&next_block, 1);
-                block = __shfl_sync(0xffffffffu, block, 0);
+            const auto draw = [&] { return lane == 0 ? atomicAdd(&next_block, 1) : 0; };
+            for (int drawn = BITS == 8 ? draw() : 0;;) { // the next one early (4-bit: 0.6 % slower so)
+                if constexpr (BITS == 4) drawn = draw();
+                const int block = __shfl_sync(0xffffffffu, drawn, 0);
                 if (block >= all_blocks) break;
+                if constexpr (BITS == 8) drawn = draw();
                 int lo = 0, hi = rows - 1; // first row with blocks[row] > block
                 while (lo < hi) {
                     const int mid = (lo + hi) >> 1;
@@ -248,8 +255,9 @@ __global__ void __launch_bounds__(kTableThreads, 1) codec_table_kernel(const cod
                 }
                 const int r = lo, start = from[r] + (block - (r == 0 ? 0 : blocks[r - 1])) * kTableBlock;
                 const int stop = min(upto[r], start + kTableBlock);
-                const std::int64_t begin = __ldg(p.row_ptr + r0 + r);
-                const int len = static_cast<int>(__ldg(p.row_ptr + r0 + r + 1) - begin), lead = lead_of(begin);
+                const std::int64_t begin = begins[r];
+                const int lead = lead_of(begin); // 8-bit: a row's units end with it
+                const int len = BITS == 8 ? stop - lead : static_cast<int>(__ldg(p.row_ptr + r0 + r + 1) - begin);
                 const float row_offset = (row_policy && p.offsets != nullptr) ? __ldg(p.offsets + r0 + r) : 0.0f;
                 std::uint8_t *codes = p.packed + (p.packed_row_ptr != nullptr ? __ldg(p.packed_row_ptr + r0 + r) : begin) - lead;
                 const std::int32_t *cols = p.col_idx + begin - lead;
@@ -338,6 +346,98 @@ __global__ void __launch_bounds__(kTableThreads, 1) codec_table_kernel(const cod
                         }
                     }
                 };
+                // 8-bit, arrays on 16 bytes: groups of four entries, a lane kQuads of them per step; the entries before the first group and behind
+                // the last, three at most of each, are a lane's each, loaded before the steps and finished after them
+                if constexpr (BITS == 8) {
+                    if (quads && ((reinterpret_cast<std::uintptr_t>(cols) | reinterpret_cast<std::uintptr_t>(values)) & 15u) == 0u && (reinterpret_cast<std::uintptr_t>(codes) & 3u) == 0u) {
+                        const int first = max(lead, start), last = stop, first4 = (first + 3) & ~3, last4 = last & ~3;
+                        const auto meta_of = [&](int gene) {
+                            const unsigned local = static_cast<unsigned>(gene - g0);
+                            float2 m = local < static_cast<unsigned>(genes) ? codec_table[local] : make_float2(scale_of(gene), offset_of(gene));
+                            if (row_policy) m.y = row_offset;
+                            return m;
+                        };
+                        int edge = lane < 3 ? first + lane : max(last4, first4) + lane - 3;
+                        if (lane < 3 ? edge >= min(first4, last) : lane >= 6 || edge >= last) edge = -1;
+                        int edge_gene = g0;
+                        float edge_value = 0.0f;
+                        unsigned edge_code = 0u;
+                        if (edge >= 0) {
+                            edge_gene = __ldg(cols + edge);
+                            if constexpr (CODE) edge_value = __ldg(values + edge);
+                            else edge_code = __ldg(codes + edge);
+                        }
+                        const auto quad_step = [&](auto whole, int at) {
+                                                        const int e0 = at + lane * 4;
+                            const auto there = [&](int q) { return decltype(whole)::value || (e0 + q * 128 >= first4 && e0 + q * 128 < last4); };
+                            const std::int32_t *step_cols = cols + e0;
+                            float *step_values = values + e0;
+                            std::uint8_t *step_codes = codes + e0;
+                            int4 gene[kQuads];
+                            float4 value[kQuads];
+                            std::uint32_t code[kQuads];
+#pragma unroll
+                            for (int q = 0; q < kQuads; ++q) {
+                                gene[q] = make_int4(g0, g0, g0, g0);
+                                value[q] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                                code[q] = 0u;
+                                if (!there(q)) continue;
+                                gene[q] = __ldg(reinterpret_cast<const int4 *>(step_cols + q * 128));
+                                if constexpr (CODE) value[q] = __ldg(reinterpret_cast<const float4 *>(step_values + q * 128));
+                                else code[q] = __ldg(reinterpret_cast<const std::uint32_t *>(step_codes + q * 128));
+                            }
+#pragma unroll
+                            for (int q = 0; q < kQuads; ++q) {
+                                const int g[4] = {gene[q].x, gene[q].y, gene[q].z, gene[q].w};
+                                const float v[4] = {value[q].x, value[q].y, value[q].z, value[q].w};
+                                float2 meta[4];
+                                bool elsewhere = false;
+#pragma unroll
+                                for (int k = 0; k < 4; ++k) {
+                                    const unsigned local = static_cast<unsigned>(g[k] - g0);
+                                    elsewhere |= local >= static_cast<unsigned>(genes);
+                                    meta[k] = codec_table[min(local, static_cast<unsigned>(genes - 1))];
+                                    if (row_policy) meta[k].y = row_offset;
+                                }
+                                if (elsewhere) {
+#pragma unroll
+                                    for (int k = 0; k < 4; ++k) meta[k] = meta_of(g[k]);
+                                }
+                                if constexpr (CODE) {
+                                    std::uint32_t packed = 0u;
+                                    bool sure = true;
+#pragma unroll
+                                    for (int k = 0; k < 4; ++k) {
+                                        unsigned c;
+                                        sure &= quantize_fast<8>(v[k], meta[k].x, meta[k].y, &c);
+                                        packed |= c << (8 * k);
+                                    }
+                                    if (!sure && there(q)) { // a thousandth of the values
+                                        packed = 0u;
+#pragma unroll
+                                        for (int k = 0; k < 4; ++k) packed |= quantize_one<8>(v[k], meta[k].x, meta[k].y) << (8 * k);
+                                    }
+                                    if (there(q)) *reinterpret_cast<std::uint32_t *>(step_codes + q * 128) = packed;
+                                } else {
+                                    float w[4];
+#pragma unroll
+                                    for (int k = 0; k < 4; ++k) w[k] = __fadd_rn(__fmul_rn(static_cast<float>(code[q] >> (8 * k) & 0xffu), meta[k].x), meta[k].y);
+                                    if (there(q)) *reinterpret_cast<float4 *>(step_values + q * 128) = make_float4(w[0], w[1], w[2], w[3]);
+                                }
+                            }
+                        };
+                        for (int at = first4; at < last4; at += kQuads * 128) {
+                            if (at + kQuads * 128 <= last4) quad_step(std::true_type{}, at);
+                            else quad_step(std::false_type{}, at);
+                        }
+                        if (edge >= 0) {
+                            const float2 m = meta_of(edge_gene);
+                            if constexpr (CODE) codes[edge] = static_cast<std::uint8_t>(quantize_one<8>(edge_value, m.x, m.y));
+                            else values[edge] = __fadd_rn(__fmul_rn(static_cast<float>(edge_code), m.x), m.y);
+                        }
+                        continue;
+                    }
+                }
                 for (int at = start; at < stop; at += U * 32) {
                     if (at >= lead && at + U * 32 <= stop && (at + U * 32) * CPB <= lead + len) step(std::true_type{}, at);
                     else step(std::false_type{}, at);
@@ -357,10 +457,13 @@ cb200_status launch_codec_table(const qcsr_view &x, const codec_params &p, int s
     if (entries < 2.0e6 || x.nnz < 64 * x.rows || x.cols > 16ll * kTableGenes) return CB200_STATUS_SUCCESS;
     const int ranges = static_cast<int>((x.cols + kTableGenes - 1) / kTableGenes);
     const int range_genes = (static_cast<int>(x.cols) + ranges - 1) / ranges;
-    const std::size_t smem = static_cast<std::size_t>(range_genes) * sizeof(float2) + 3u * kTableRows * sizeof(int);
+    // Groups of four where a row's piece of a range fills at least half a step of them (1,000,000 rows of 80 entries: 1.00 ms one by one,
+    // 1.20 in groups; 300,000 x 30,000, 180 entries in two ranges, 0.71 one by one; 60,000 rows of 800: 0.39 and 0.33).
+    const bool quads = x.nnz >= 192ll * ranges * x.rows;
+    const std::size_t smem = static_cast<std::size_t>(range_genes) * sizeof(float2) + 5u * kTableRows * sizeof(int);
     const auto kernel = x.bits == 8 ? codec_table_kernel<8, CODE> : codec_table_kernel<4, CODE>;
     CB200_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-    kernel<<<static_cast<unsigned>(sm_count), kTableThreads, smem, stream>>>(p, range_genes, ranges);
+    kernel<<<static_cast<unsigned>(sm_count), kTableThreads, smem, stream>>>(p, range_genes, ranges, quads);
     count_launch();
     CB200_CUDA_OK(cudaGetLastError());
     *taken = true;

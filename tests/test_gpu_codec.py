@@ -140,3 +140,30 @@ def test_codec_of_a_large_matrix_equals_oracle(cuda_device, oracle, bits, policy
     assert np.array_equal(x.dequantize().cpu().numpy(), decoded, equal_nan=True)
     lo, hi = 3, len(lengths) - 2
     assert np.array_equal(x.dequantize(lo, hi).cpu().numpy(), decoded[row_ptr[lo]:row_ptr[hi]], equal_nan=True)
+
+
+@pytest.mark.parametrize("policy,cols,shift", [(1, 2500, 0), (1, 41_000, 0), (2, 2500, 0), (1, 2500, 1)])
+def test_groups_of_four_entries(cuda_device, oracle, policy, cols, shift):
+    """8-bit rows of long matrices in groups of four, three to a step, blocks of 1,152: rows around each of them, genes that do not ascend,
+    a row range whose first entry lies on 16 bytes, and codes that lie a byte off their entries, which go one by one."""
+    rng = np.random.default_rng(policy + cols)
+    lengths = np.concatenate([np.arange(14), np.repeat([127, 128, 129, 383, 384, 385, 387, 1151, 1152, 1153, 1155, 2303, 2305], 3), rng.integers(900, 1500, size=1800)])
+    row_ptr = np.concatenate([[0], np.cumsum(lengths)]).astype(np.int64)
+    col_idx = np.concatenate([np.sort(rng.choice(cols, size=k, replace=False)) for k in lengths]).astype(np.int32)
+    for r in range(20, len(lengths), 90):
+        col_idx[row_ptr[r]:row_ptr[r + 1]] = rng.permutation(col_idx[row_ptr[r]:row_ptr[r + 1]])
+    scales = rng.uniform(0.01, 0.5, size=cols).astype(np.float32)
+    offsets = rng.uniform(-1.0, 1.0, size=cols if policy == 1 else len(lengths)).astype(np.float32)
+    values = rng.uniform(-1.0, 9.0, size=len(col_idx)).astype(np.float32)
+    values[:: 997] = np.nan
+    row_ptr_p = row_ptr + shift
+    expect = np.concatenate([np.full(shift, 0x55, dtype=np.uint8), oracle.pack_csr(8, policy, row_ptr, row_ptr, col_idx, scales, offsets, values)])
+    x = ops.QuantizedCsr.from_host(dict(rows=len(lengths), cols=cols, bits=8, policy=policy, row_ptr=row_ptr, col_idx=col_idx, scales=scales,
+                                        offsets=offsets, packed_row_ptr=row_ptr_p, packed=np.full(len(expect), 0x55, dtype=np.uint8)), cuda_device)
+    assert x.nnz >= 2_000_000
+    x.quantize_(torch.from_numpy(values).to(cuda_device))
+    assert np.array_equal(x.packed.cpu().numpy(), expect)
+    decoded = oracle.unpack_csr(8, policy, row_ptr, row_ptr, col_idx, scales, offsets, expect[shift:])
+    assert np.array_equal(x.dequantize().cpu().numpy(), decoded, equal_nan=True)
+    lo = next(r for r in range(15, 100) if row_ptr[r] % 4 == 0)
+    assert np.array_equal(x.dequantize(lo, len(lengths) - 1).cpu().numpy(), decoded[row_ptr[lo]:row_ptr[-2]], equal_nan=True)
