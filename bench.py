@@ -165,11 +165,11 @@ def build_workload(name, device, rank, world, seed=0, rows_override=None, multip
         dense = torch.randn(rows, n, generator=g).to(device)
         out = torch.empty(cfg["cols"], n, dtype=torch.float32, device=device)
         # G is fp32, for which the contract's bound is 1e-4 * ||.||_1 * max|G|: the default arm asks for
-        # fp32 products and hands the matrix to prepare, which selects the tensor-core schedule with
-        # split products (three bf16 passes rebuild each product to ~3 * 2^-17; "tensor_blocked_x3").
+        # fp32 products and hands the matrix to prepare, which selects the tensor-core schedule "tensor_blocked_x3":
+        # exact sums of the codes times three base-256 digits of G (2^-23 of a column's largest magnitude).
         # --multiply bf16: one pass, values and G rounded to bf16 (1e-2 bound).  --no-prepare-matrix:
-        # the fp32-FMA kernel with L2 vector reductions.  --deterministic: fp32 FMAs in a fixed order, gathered
-        # gene by gene from a gene-major copy that prepare builds ("gene_gather").
+        # the fp32-FMA kernel with L2 vector reductions.  --deterministic ("gene_gather"): four digits of G, or, for small
+        # shards, fp32 FMAs in a fixed order, gathered gene by gene from a gene-major copy that prepare builds.
         torch.cuda.synchronize(device)
         t_prepare = time.perf_counter()           # prepare is outside the timed region; its cost is reported
         def make_op():
@@ -722,14 +722,19 @@ def run_ours(args):
 
     kind_bell = args.workload == "c5_bell"
     schedule = main["schedule"]
-    baked = schedule in ("tensor_blocked", "tensor_blocked_x2", "tensor_blocked_x3", "tensor_dense", "gene_gather")
+    # transpose by exact integer sums: zero-points are per gene here, the density is 5 %; fixed order below 2^23 places
+    digits = 0
+    if args.workload == "c3_transpose":
+        digits = {"tensor_blocked_x3": 3, "gene_gather": 4 if main["rows"] * main["cols"] >= 1 << 23 else 0}.get(schedule, 0)
+    baked = digits == 0 and schedule in ("tensor_blocked", "tensor_blocked_x2", "tensor_blocked_x3", "tensor_dense", "gene_gather")
     result = {
         "metric": ("quantized Blocked-ELL projection throughput" if kind_bell else
                    "quantized CSR SpMM throughput (dequant fused into the multiply, fp32 accumulate)"),
         "value": main["value"], "unit": "Gslot/s" if kind_bell else "Gnnz/s",
         "n_gpus": world, "steps": args.steps, "warmup": max(args.warmup, 3), "ms_per_step": main["ms_per_step"],
         "higher_is_better": True, "scaling": args.scaling, "vs_baseline": None,
-        "dtype": f"u{main['bits']} codes -> " + ("bf16 products (tcgen05), f32 accumulate"
+        "dtype": f"u{main['bits']} codes -> " + (f"int8 products with {digits} digits of f32 G (tcgen05), exact int32 sums, f32 result"
+                                                 if digits else "bf16 products (tcgen05), f32 accumulate"
                                                  if schedule == "tensor_windows"
                                                  else "fp16 products (tcgen05), f32 accumulate"
                                                  if schedule in ("tensor_blocked", "tensor_dense", "tensor_codes", "tcgen05_block_rows")
@@ -745,6 +750,9 @@ def run_ours(args):
                    "dequantisation": ("at prepare: the timed kernel streams {fp16 decoded value, tile position} words that prepare "
                                       "wrote from the codes, scales and offsets; a change of any of them needs a new prepare"
                                       if baked else
+                                      "at launch: the timed kernel streams {code, tile position} words that prepare laid out; scales and "
+                                      "offsets are read at every launch"
+                                      if digits else
                                       "at launch, in registers: the timed kernel streams dense tiles of codes (a byte per slot) that "
                                       "prepare laid out; scales and offsets are read at every launch"
                                       if schedule == "tensor_codes" else "at launch: codes, scales and offsets are read by the timed kernel"),

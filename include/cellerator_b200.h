@@ -333,7 +333,7 @@ void cb200_prepared_destroy(cb200_prepared *prepared);
  * bytes a gene.  "warp_per_row" (unaligned
  * N) and the tensor_blocked and tensor_dense forward schedules also run with less, down to the status block and the records of
  * W, slower and with the same bits: a row's sum follows from its entries, N and W's type, not from the room, the launch's row
- * range or the rows beside it. */
+ * range or the rows beside it ("integer_windows" with less than it reports runs "warp_per_row", whose sums differ by rounding). */
 cb200_status cb200_prepared_workspace(const cb200_prepared *prepared, uint64_t *minimum_bytes, uint32_t *alignment);
 /* kernel choice made at prepare time, as text: "warp_per_row", "gene_tiled" (exact fp32 products), "integer_windows" (codes
  * times digits of W, exact integer sums; zero-points per gene, 2 to 50 million entries, N times entries from 200 million on);
