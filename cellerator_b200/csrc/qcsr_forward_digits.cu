@@ -663,40 +663,58 @@ template<int NB> constexpr std::size_t fwd_digits_smem_bytes() {
 
 // The lines (column block, group) that lie in the shares of several CTAs, counted on the host: 64-bit divisions in every block of
 // sum_parts_kernel cost it 1.9 M instructions.
+constexpr int kSumColumns = 16; // of a block of sum_parts_kernel
 struct cut_lines {
     int count;
     struct { int line; unsigned char first, last; bool second_slot; } at[kMaxCtas]; // the first and the last CTA; the first's slot for it
 };
 
-// Y of those lines.  Block (j, y, z): rows [32 y, 32 y + 32) and columns [8 z, 8 z + 8) of the j-th; a warp per column and a lane per
-// row, whose sums change places in shared memory to be written a row's eight columns at a time.
+// Y of those lines.  Block (j, y, z): rows [32 y, 32 y + 32) and kSumColumns columns of the j-th; a warp for each eighth of the columns and a
+// lane per row, whose sums change places in shared memory to be written a row's columns side by side.  Bound by the latency of the slots'
+// loads, wave after wave of blocks: sixteen columns instead of eight take the whole call of 8,000 x 4,000, N = 64 from 66.2 to 63.6 us, of
+// 8,192 x 33,538 from 172.5 to 169.9, of 20,000 x 2,000, N = 32 from 75.1 to 74.9 and of 4,099 x 33,538, N = 50 from 107.5 to 107.7; 32
+// columns 64.7, 171.1, 77.6 and 109.0.
 template<int NB>
 __global__ void __launch_bounds__(256) sum_parts_kernel(const __grid_constant__ fwd_digit_params p, const __grid_constant__ cut_lines cuts) {
-    __shared__ float turned[32][9];
+    constexpr int kColumns = kSumColumns;
+    __shared__ float turned[32][kColumns + 1];
     const int line = cuts.at[blockIdx.x].line, b0 = cuts.at[blockIdx.x].first, b1 = cuts.at[blockIdx.x].last;
-    const int group = line % p.groups, c0 = line / p.groups * NB, r0 = blockIdx.y * 32, column = blockIdx.z * 8;
+    const int group = line % p.groups, c0 = line / p.groups * NB, r0 = blockIdx.y * 32, column = blockIdx.z * kColumns;
     const std::int64_t first_row = p.first_row + static_cast<std::int64_t>(group) * kRows + r0;
     if (first_row >= p.row_end || first_row + 32 <= p.row_begin || c0 + column >= p.n) return;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     wait_for_previous_launch();
     const int wide = __ldcg(p.wide);
-    const double step = __ldcg(p.steps + c0 + column + warp);
-    const bool odd = cell_is_odd(p, group, r0 + lane), odd_row = cell_is_odd(p, group, r0 + (tid >> 3));
+    const bool odd = cell_is_odd(p, group, r0 + lane);
+    bool odd_row[kColumns / 8];
+#pragma unroll
+    for (int k = 0; k < kColumns / 8; ++k) odd_row[k] = cell_is_odd(p, group, r0 + tid / kColumns + k * (256 / kColumns));
     // only the group's first CTA can have another group before it: its slot may be the second of its two, the others' is the first
     const long long *src = p.slots + static_cast<std::int64_t>(column + warp) * kRows + r0 + lane;
     constexpr std::int64_t kSlot = static_cast<std::int64_t>(NB) * kRows;
-    long long sum = __ldcg(src + (2 * b0 + (cuts.at[blockIdx.x].second_slot ? 1 : 0)) * kSlot);
-#pragma unroll 8
-    for (int b = b0 + 1; b <= b1; ++b) sum += __ldcg(src + 2 * b * kSlot);
+    const std::int64_t first_slot = (2 * b0 + (cuts.at[blockIdx.x].second_slot ? 1 : 0)) * kSlot;
+    double step[kColumns / 8];
+    long long sum[kColumns / 8];
+#pragma unroll
+    for (int k = 0; k < kColumns / 8; ++k) {
+        step[k] = __ldcg(p.steps + c0 + column + warp + 8 * k);
+        sum[k] = __ldcg(src + first_slot + 8 * k * kRows);
+    }
+#pragma unroll 4
+    for (int b = b0 + 1; b <= b1; ++b)
+#pragma unroll
+        for (int k = 0; k < kColumns / 8; ++k) sum[k] += __ldcg(src + 2 * b * kSlot + 8 * k * kRows);
     if (wide != 0) return;
-    turned[lane][warp] = sum_to_output(sum, step, p);
+#pragma unroll
+    for (int k = 0; k < kColumns / 8; ++k) turned[lane][warp + 8 * k] = sum_to_output(sum[k], step[k], p);
     __syncthreads();
-    {
-        const std::int64_t row = first_row + (tid >> 3);
-        const int c = c0 + column + (tid & 7);
-        if (row >= p.row_begin && row < p.row_end && c < p.n && !odd_row) {
+#pragma unroll
+    for (int k = 0; k < kColumns / 8; ++k) {
+        const int r = tid / kColumns + k * (256 / kColumns), c = c0 + column + tid % kColumns;
+        const std::int64_t row = first_row + r;
+        if (row >= p.row_begin && row < p.row_end && c < p.n && !odd_row[k]) {
             float *dst = p.out + row * p.out_ld + c;
-            float v = turned[tid >> 3][tid & 7];
+            float v = turned[r][tid % kColumns];
             if (p.beta != 0.0f) v = fmaf(p.beta, *dst, v);
             *dst = finish_output(v, p.bias, c, p.epilogue);
         }
@@ -744,7 +762,7 @@ cb200_status launch_all(const fwd_digit_params &p, unsigned *part_max, ulonglong
         cut.second_slot = share_begin(total, b, ctas) / p.windows != line;
     }
     if (cuts.count > 0) {
-        CB200_CUDA_OK(launch_kernel(true, sum_parts_kernel<NB>, dim3(static_cast<unsigned>(cuts.count), kRows / 32, NB / 8), 256, 0, stream, p, cuts));
+        CB200_CUDA_OK(launch_kernel(true, sum_parts_kernel<NB>, dim3(static_cast<unsigned>(cuts.count), kRows / 32, NB / kSumColumns), 256, 0, stream, p, cuts));
         count_launch();
     }
     count_launch(3);
