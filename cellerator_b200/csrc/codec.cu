@@ -133,18 +133,17 @@ __global__ void __launch_bounds__(256) dequantize_rows_kernel(const codec_params
 // take six or seven cycles, and goes through its rows once per range: genes ascend in a row, so a range is a contiguous piece
 // of it, found by bisection.  Pieces are cut at multiples of 32 entries (bytes, for 4-bit codes); the few entries on the wrong
 // side of a cut, and any that a row which does not ascend has out of place, are looked up in global memory.  CTAs get equal
-// shares of the entries, and a CTA's warps draw blocks of at most 1,152 of them, so that a long row holds up nobody.
+// shares of the entries, and a CTA's warps draw blocks of at most 1,536 of them, so that a long row holds up nobody.
 //
 // 100,000 x 33,538, 180 M entries of 8 bits: coding 1.74 -> 0.42 ms, decoding 0.76 -> 0.37 ms with an entry to a lane; with four
-// neighbouring ones (16-byte loads and stores, a step of 384 entries) 0.785 -> 0.68-0.69 ms together, 4.7 TB/s.  Bound by issue (57 % of the
+// neighbouring ones (16-byte loads and stores, a step of 384 entries, decoding of 512) 0.785 -> 0.66-0.68 ms together, 4.8 TB/s.  Bound by issue (57 % of the
 // slots when coding) and by the latency of the one step of loads a warp has in flight at 32 warps per SM.  Measured on the way there: two
-// groups a step 0.73 ms, four 0.83 (registers), one 0.86; groups that hold a neighbour row's entries too, masked entry by entry, 0.76; the row's
+// groups a step 0.73 ms, four 0.83 (coding: registers; for decoding alone 0.663, three 0.674), one 0.86; groups that hold a neighbour row's entries too, masked entry by entry, 0.76; the row's
 // start looked up in global memory for each block 0.70; a rest of a row in steps of its own length 0.82 (three copies of the step for the
 // instruction cache); more than 196 KB of shared memory, which leaves L1 28 KB, 0.82.
 constexpr int kTableThreads = 1024;
 constexpr int kTableGenes = 20 * 1024; // genes of a range: 160 KB
 constexpr int kTableRows = 2 * 1024;   // rows of a CTA between two loads of the table: 40 KB of places
-constexpr int kTableBlock = 1152;      // units (entries, bytes) a warp draws: three steps of 384
 
 // first row in [lo, hi] whose start is at least `target` (one warp; the rows' starts ascend)
 __device__ __forceinline__ std::int64_t first_row_from(const std::int64_t *row_ptr, std::int64_t lo, std::int64_t hi, std::int64_t target) {
@@ -162,7 +161,8 @@ __device__ __forceinline__ std::int64_t first_row_from(const std::int64_t *row_p
 
 template<int BITS, bool CODE>
 __global__ void __launch_bounds__(kTableThreads, 1) codec_table_kernel(const codec_params p, int range_genes, int ranges, bool quads) {
-    constexpr int CPB = 8 / BITS, kQuads = 3, U = BITS == 8 ? 6 : 4; // steps of loads in flight, what 64 registers hold
+    constexpr int CPB = 8 / BITS, kQuads = CODE ? 3 : 4, U = BITS == 8 ? 6 : 4; // steps of loads in flight, what 64 registers hold
+    constexpr int kTableBlock = BITS == 8 ? 1536 : 1024; // units (entries, bytes) a warp draws: four steps of 384, three of 512
     extern __shared__ __align__(16) float2 codec_table[];
     std::int64_t *begins = reinterpret_cast<std::int64_t *>(codec_table + range_genes); // [kTableRows] first entry of the row
     int *from = reinterpret_cast<int *>(begins + kTableRows);       // [kTableRows] first unit of the row in this range

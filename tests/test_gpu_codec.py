@@ -144,10 +144,10 @@ def test_codec_of_a_large_matrix_equals_oracle(cuda_device, oracle, bits, policy
 
 @pytest.mark.parametrize("policy,cols,shift", [(1, 2500, 0), (1, 41_000, 0), (2, 2500, 0), (1, 2500, 1)])
 def test_groups_of_four_entries(cuda_device, oracle, policy, cols, shift):
-    """8-bit rows of long matrices in groups of four, three to a step, blocks of 1,152: rows around each of them, genes that do not ascend,
+    """8-bit rows of long matrices in groups of four, three or four to a step, blocks of 1,536: rows around each of them, genes that do not ascend,
     a row range whose first entry lies on 16 bytes, and codes that lie a byte off their entries, which go one by one."""
     rng = np.random.default_rng(policy + cols)
-    lengths = np.concatenate([np.arange(14), np.repeat([127, 128, 129, 383, 384, 385, 387, 1151, 1152, 1153, 1155, 2303, 2305], 3), rng.integers(900, 1500, size=1800)])
+    lengths = np.concatenate([np.arange(14), np.repeat([127, 128, 129, 383, 384, 385, 387, 511, 512, 513, 515, 1535, 1536, 1537, 1539, 2305], 3), rng.integers(900, 1500, size=1800)])
     row_ptr = np.concatenate([[0], np.cumsum(lengths)]).astype(np.int64)
     col_idx = np.concatenate([np.sort(rng.choice(cols, size=k, replace=False)) for k in lengths]).astype(np.int32)
     for r in range(20, len(lengths), 90):
