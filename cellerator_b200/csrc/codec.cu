@@ -136,11 +136,13 @@ __global__ void __launch_bounds__(256) dequantize_rows_kernel(const codec_params
 // shares of the entries, and a CTA's warps draw blocks of at most 1,536 of them, so that a long row holds up nobody.
 //
 // 100,000 x 33,538, 180 M entries of 8 bits: coding 1.74 -> 0.42 ms, decoding 0.76 -> 0.37 ms with an entry to a lane; with four
-// neighbouring ones (16-byte loads and stores, a step of 384 entries, decoding of 512) 0.785 -> 0.66-0.68 ms together, 4.8 TB/s.  Bound by issue (57 % of the
-// slots when coding) and by the latency of the one step of loads a warp has in flight at 32 warps per SM.  Measured on the way there: two
-// groups a step 0.73 ms, four 0.83 (coding: registers; for decoding alone 0.663, three 0.674), one 0.86; groups that hold a neighbour row's entries too, masked entry by entry, 0.76; the row's
-// start looked up in global memory for each block 0.70; a rest of a row in steps of its own length 0.82 (three copies of the step for the
-// instruction cache); more than 196 KB of shared memory, which leaves L1 28 KB, 0.82.
+// neighbouring ones (16-byte loads and stores, a step of 384 entries, decoding of 512) 0.785 -> 0.66-0.70 ms together, 4.7 TB/s.
+// Bound by issue (65 % of the slots when coding) and by the latency of the one step of loads a warp has in flight at 32 warps per SM.
+// Measured on the way there: two groups a step 0.73 ms, four 0.83 (coding: registers; for decoding alone 0.663, three 0.674), one
+// 0.86; groups that hold a neighbour row's entries too, masked entry by entry, 0.76; the row's start looked up in global memory for each
+// block 0.70; a rest of a row in steps of its own length 0.82 (three copies of the step for the instruction cache); more than 196 KB of
+// shared memory, which leaves L1 28 KB, 0.82; reciprocals in the table, so that an entry that goes the exact way looks its scale
+// up in global memory, 0.70.
 constexpr int kTableThreads = 1024;
 constexpr int kTableGenes = 20 * 1024; // genes of a range: 160 KB
 constexpr int kTableRows = 2 * 1024;   // rows of a CTA between two loads of the table: 40 KB of places
