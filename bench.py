@@ -577,7 +577,7 @@ def run_ours(args):
     exact_arm = None
     if default_arm and not args.no_extras:
         ex = ops.PreparedSpmm(capi.PROJECTION_CSR, wl["rows"], wl["cfg"]["cols"], wl["n"], x.nnz, x.bits, x.policy, dense.dtype, device,
-                              host_row_ptr=x.host_row_ptr, multiply=capi.DTYPE_F32, schedule="warp_per_row")
+                              host_row_ptr=x.host_row_ptr, multiply=capi.DTYPE_F32)
         ex_out = torch.empty_like(out)
         ex_launch = ex.make_launch(x, dense, ex_out)
         _, ex_ms = timed_loop(lambda: ex.run_launch(ex_launch), 5, 2, device)

@@ -319,7 +319,6 @@ struct schedule_plan {
     bool dense_forced = false;   // ... asked for by name: the free-memory rule does not apply
     bool codes_wanted = false;   // forward, 4-bit codes: tiles of codes (a byte per slot) instead of decoded tiles
     bool gene_gather = false;    // transpose with a fixed order of the sums
-    bool integer = false;        // CSR forward: integer sums from the CSR arrays
     int digits = 0;              // transpose with integer sums: digits of G (0: another kernel)
     bool row_order = false;      // length-sorted row order ("gene_tiled", "tensor_windows")
     bool bell_cuda_cores = false;
@@ -478,15 +477,6 @@ schedule_plan plan_schedule(const cb200_spmm_problem &pr) {
     }
     plan.tiled = tiled;
     plan.tensor_windows = tensor;
-    // Integer sums on the tensor cores instead of gathered rows of W: more exact, and faster where an entry's row of W is long and a tile
-    // of 256 x 128 holds some 1,300 entries, but the words take room and time of their own.  One B200, gathered -> this: 20,000 x 2,000
-    // (6.8 M entries) N = 16 62 -> 77 us, N = 32 85 -> 78, N = 64 bf16 105 -> 91; 8,000 x 2,000 (2.7 M) N = 32 41 -> 49; 8,000 x 4,000 (4.2 M)
-    // N = 64 82 -> 65, N = 128 140 -> 79; 4,099 x 33,538 (7.4 M) N = 50 bf16 117 -> 106; 8,192 rows of it N = 32 150 -> 142, N = 128 455 -> 248.
-    // Words of more than 50 M entries (200 MB) are more than a call should ask for.
-    const bool integer_ok = !blocked && !tensor && !tiled && qcsr_forward_digits_shape_ok(pr.m, pr.k, pr.n, pr.bits, pr.policy);
-    plan.integer = integer_ok && (hint_is(hint, "integer_windows") ||
-                                  (hint == nullptr && pr.nnz >= 2'000'000 && pr.nnz <= 50'000'000 && pr.n * pr.nnz >= 200'000'000 &&
-                                   plan.mean_row_nnz >= (pr.n <= 64 ? 0.04 : 0.03) * static_cast<double>(pr.k)));
     // The tiled kernel gives each row to one lane group, so a CTA is as slow as its longest row.  With the
     // row lengths at hand, order the rows by length once: every CTA then works on rows of nearly equal length.
     plan.row_order = tiled && pr.host_row_ptr != nullptr && pr.m > 0 && pr.m <= 0x7fffffff;
@@ -573,7 +563,7 @@ cb200_status cb200_spmm_prepare(const cb200_spmm_problem *problem, cb200_prepare
         if (problem->device_matrix == nullptr)
             p->workspace_bytes = std::max(p->workspace_bytes, qcsr_transpose_digits_once_bytes(problem->m, problem->k, problem->n, problem->nnz, problem->bits, problem->policy));
         if (plan.digits != 0) {
-            const cb200_status st = build_digit_words(view_of(*problem->device_matrix), false, p->arena, stream, &p->digits);
+            const cb200_status st = build_digit_words(view_of(*problem->device_matrix), p->arena, stream, &p->digits);
             if (st != CB200_STATUS_SUCCESS) return abandon(st);
             p->digit_slices = plan.digits;
             p->schedule_name = plan.digits == 4 ? "gene_gather" : "tensor_blocked_x3";
@@ -613,11 +603,6 @@ cb200_status cb200_spmm_prepare(const cb200_spmm_problem *problem, cb200_prepare
         }
         p->workspace_bytes = plan.tiled ? qcsr_tiled_workspace_bytes()
                                         : qcsr_gather_workspace_bytes(problem->k, problem->nnz, problem->n, problem->dense_dtype);
-        if (plan.integer) {
-            p->schedule = fwd_schedule::integer_windows;
-            p->schedule_name = "integer_windows";
-            p->workspace_bytes = qcsr_forward_digits_workspace_bytes(problem->k, problem->n) + qcsr_digit_words_bytes_bound(problem->m, problem->k, problem->nnz);
-        }
         if (plan.tensor_windows) {
             p->schedule = fwd_schedule::tensor_windows;
             p->schedule_name = "tensor_windows";
@@ -809,7 +794,7 @@ cb200_status cb200_spmm_run(const cb200_prepared *prepared, const cb200_launch *
     if (pr.projection == CB200_PROJECTION_TRANSPOSE)
         return launch_qcsr_transpose(view_of(x), d, row_begin, row_end, &prepared->blocked, &prepared->digits, prepared->digit_slices, pr.multiply != CB200_DTYPE_BF16,
                                      launch->workspace, launch->workspace_bytes, prepared->sm_count, stream);
-    return launch_qcsr_forward(view_of(x), d, row_begin, row_end, prepared->schedule, prepared->row_order, &prepared->blocked, &prepared->digits,
+    return launch_qcsr_forward(view_of(x), d, row_begin, row_end, prepared->schedule, prepared->row_order, &prepared->blocked,
                                pr.multiply != CB200_DTYPE_BF16, launch->workspace, launch->workspace_bytes, prepared->sm_count,
                                stream);
 }

@@ -672,7 +672,7 @@ cb200_status cb200_host_forward(cb200_host_stage *s, const cb200_qcsr *x, const 
         const qcsr_view view{rows, o.k, nnz, o.bits, o.policy, b.row_ptr, o.bits == 4 ? b.packed_row_ptr : nullptr, b.col_idx, b.packed,
                              s->scales, row_policy ? (x->offsets != nullptr ? b.row_offsets : nullptr) : (x->offsets != nullptr ? s->offsets : nullptr)};
         const dense_args d{s->w, o.n, o.dense_dtype, b.y, o.n, o.n, alpha, 0.0f};
-        const cb200_status st = launch_qcsr_forward(view, d, 0, rows, fwd_schedule::warp_per_row, nullptr, nullptr, nullptr, false, b.workspace, s->workspace_bytes,
+        const cb200_status st = launch_qcsr_forward(view, d, 0, rows, fwd_schedule::warp_per_row, nullptr, nullptr, false, b.workspace, s->workspace_bytes,
                                                     s->sm_count, s->compute);
         if (st != CB200_STATUS_SUCCESS) return st;
         CB200_CUDA_OK(cudaEventRecord(b.computed, s->compute));

@@ -29,7 +29,7 @@ struct dense_args {
     int epilogue = CB200_EPILOGUE_NONE;   // out = act(alpha * product + beta * out + bias[column])
 };
 
-enum class fwd_schedule : int { warp_per_row = 0, gene_tiled = 1, tensor_windows = 2, tensor_blocked = 3, integer_windows = 4 };
+enum class fwd_schedule : int { warp_per_row = 0, gene_tiled = 1, tensor_windows = 2, tensor_blocked = 3 };
 
 // Device memory a prepared operation keeps.  Two modes: pieces carved out of a block the caller owns (a
 // session's persistent reservation: nothing is allocated or freed here), or pieces allocated one by one
@@ -189,7 +189,7 @@ cb200_status launch_qcsr_forward_blocked(const qcsr_view &x, const dense_args &d
 // Y[r,:] = alpha * sum_i deq(code_i) * W[col_i,:] + beta * Y[r,:]  for r in [row_begin,row_end)
 cb200_status launch_qcsr_forward(const qcsr_view &x, const dense_args &d, std::int64_t row_begin,
                                  std::int64_t row_end, fwd_schedule schedule, const void *persistent,
-                                 const blocked_layout *blocked, const struct digit_layout *digits, bool split_products, void *workspace,
+                                 const blocked_layout *blocked, bool split_products, void *workspace,
                                  std::uint64_t workspace_bytes, int sm_count, cudaStream_t stream);
 
 // Transpose on the tensor cores from the window-blocked copy (N in {32, 64}).  split_products == false:
@@ -214,15 +214,13 @@ struct digit_layout {
     const void *src_row_ptr = nullptr, *src_col_idx = nullptr, *src_packed = nullptr; // arrays it was built from
 };
 constexpr std::int64_t kDigitWordsTwice = 1ll << 62;
-int qcsr_digit_piece_rows(std::int64_t rows);
 bool qcsr_transpose_digits_shape_ok(std::int64_t rows, std::int64_t cols, std::int64_t n, int bits, int policy);
 std::uint64_t qcsr_digit_words_bytes_bound(std::int64_t rows, std::int64_t cols, std::int64_t nnz);
 // current device; memory from `arena`, kernels on `stream`, which is waited for
-// forward: the places of the forward kernel's tile, else of the transpose's
-cb200_status build_digit_words(const qcsr_view &x, bool forward, device_arena &arena, cudaStream_t stream, digit_layout *out);
+cb200_status build_digit_words(const qcsr_view &x, device_arena &arena, cudaStream_t stream, digit_layout *out);
 // ... and without the wait, into memory of that size
 digit_layout digit_words_at(void *memory, const qcsr_view &x);
-cb200_status launch_digit_words(const qcsr_view &x, std::int64_t row_begin, std::int64_t row_end, bool forward, std::uint32_t *words, std::uint32_t *bounds,
+cb200_status launch_digit_words(const qcsr_view &x, std::int64_t row_begin, std::int64_t row_end, std::uint32_t *words, std::uint32_t *bounds,
                                 std::int64_t *bases, int *status, cudaStream_t stream);
 std::uint64_t qcsr_transpose_digits_workspace_bytes(std::int64_t rows, std::int64_t cols, std::int64_t n, int slices);
 std::uint64_t qcsr_transpose_digits_least_workspace(std::int64_t rows, std::int64_t cols, std::int64_t n, int slices, int sm_count); // slower
@@ -231,14 +229,6 @@ std::uint64_t qcsr_transpose_digits_once_bytes(std::int64_t rows, std::int64_t c
 // layout null: the words are made in the workspace.  *taken is false where the shape or the workspace rules it out.
 cb200_status launch_qcsr_transpose_digits(const qcsr_view &x, const dense_args &d, std::int64_t row_begin, std::int64_t row_end, void *workspace,
                                           std::uint64_t workspace_bytes, const digit_layout *layout, int slices, int sm_count, cudaStream_t stream, bool *taken);
-
-// Forward with exact integer sums of codes times digits of W (zero-points per gene).  layout null: the words are made in the workspace.
-// *wide is null where the shape or the workspace rules it out, else the device's word that says whether W fits fixed point: where it is
-// not 0, the launches have left Y alone and the caller's next one takes the rows.
-bool qcsr_forward_digits_shape_ok(std::int64_t rows, std::int64_t cols, std::int64_t n, int bits, int policy);
-std::uint64_t qcsr_forward_digits_workspace_bytes(std::int64_t cols, std::int64_t n);
-cb200_status launch_qcsr_forward_digits(const qcsr_view &x, const dense_args &d, std::int64_t row_begin, std::int64_t row_end, void *workspace,
-                                        std::uint64_t workspace_bytes, const digit_layout *layout, int sm_count, cudaStream_t stream, const int **wide);
 
 // G'[g,:] = alpha * sum_{r in range, col_i == g} deq(code_i) * G[r,:] + beta * G'[g,:]
 // `blocked` (optional): the window-blocked copy of a prepared bf16-product operation.  `digits` (optional): the words of a prepared

@@ -168,7 +168,6 @@ cb200_status route(const cb200_public_layout *l, int32_t projection, const float
         csr.packed_values = l->packed_values; csr.scales = l->column_scales; csr.offsets = offsets_of(*l);
         ln.csr = &csr;
     }
-    if (projection == CB200_PROJECTION_CSR) pr.schedule_hint = "warp_per_row"; // what the scratch has room for
     cb200_prepared *prepared = nullptr;
     st = cb200_spmm_prepare(&pr, &prepared);
     if (st != CB200_STATUS_SUCCESS) return st;

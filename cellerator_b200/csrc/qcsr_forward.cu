@@ -5,7 +5,6 @@
 // (include/Cellerator/quantized/portable_dequantize_kernel.cuh:7-19) and then runs
 // csr_spmm_fwd_kernel_ (src/compute/sparse/project/kernels/csr_spmm_fwd_kernel_.cuh:1-22), one
 // thread per (row, output column), every thread re-reading the row.
-#include "dependent_launch.cuh"
 #include "kernels.cuh"
 
 #include <algorithm>
@@ -42,7 +41,6 @@ struct fwd_params {
     int packed_rows; // W is the re-laid copy: rows at a pitch of 16 bytes
     int out_vector; // rows of Y can be written 16 bytes at a time
     int *status;    // status word of the launch (this kernel waits on nothing: it clears it)
-    const int *wide; // the launch behind the integer kernel: works only where this word of the device's is not 0
 };
 
 // Code of entry `local` (index within its row) for a row whose packed bytes start at `row_bytes`.
@@ -360,18 +358,18 @@ __global__ void __launch_bounds__(128, 8) qcsr_fwd_row_kernel(const fwd_params p
 // others; sums of parts meet in shared memory.
 // SHORT_END: the CTAs from p.full_groups on take a quarter of the rows.
 template<int BITS, typename WT, int V, int SETS, bool SHORT_END>
-__device__ __forceinline__ void gather_group(const fwd_params &p, unsigned block) {
+__global__ void __launch_bounds__(kGatherMaxWarps * 32, 2) qcsr_fwd_gather_kernel(const fwd_params p) {
     __shared__ std::int64_t row_start[kGatherMaxRows], code_start[kGatherMaxRows];
     __shared__ int row_len[kGatherMaxRows], row_share[kGatherMaxRows], first_part[kGatherMaxRows + 1];
     extern __shared__ __align__(16) int2 staging[];         // [warp][64], then the sums
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
     float *sums = reinterpret_cast<float *>(staging + warps * kSegment); // [p.parts][V][lanes]
-    std::int64_t row0 = p.row_begin + static_cast<std::int64_t>(block) * p.group_rows;
+    std::int64_t row0 = p.row_begin + static_cast<std::int64_t>(blockIdx.x) * p.group_rows;
     int most_rows = p.group_rows;
     if constexpr (SHORT_END)
-        if (block >= p.full_groups) {
+        if (blockIdx.x >= p.full_groups) {
             most_rows = p.group_rows >> 2;
-            row0 = p.row_begin + static_cast<std::int64_t>(p.full_groups) * p.group_rows + static_cast<std::int64_t>(block - p.full_groups) * most_rows;
+            row0 = p.row_begin + static_cast<std::int64_t>(p.full_groups) * p.group_rows + static_cast<std::int64_t>(blockIdx.x - p.full_groups) * most_rows;
         }
     const int rows = static_cast<int>(min(static_cast<std::int64_t>(most_rows), p.row_end - row0));
     if (warp == 0) {
@@ -394,7 +392,7 @@ __device__ __forceinline__ void gather_group(const fwd_params &p, unsigned block
         if (lane == 0) first_part[0] = 0;
         if (lane < rows) first_part[lane + 1] = upto;
     }
-    if (block == 0 && blockIdx.y == 0 && threadIdx.x == 0 && p.status != nullptr) *p.status = 0;
+    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 && p.status != nullptr) *p.status = 0;
     __syncthreads();
     gather_warp<BITS, WT, V, SETS, kGatherRuns> g(p, staging + warp * kSegment);
     const int lanes = g.lanes;
@@ -460,24 +458,6 @@ __device__ __forceinline__ void gather_group(const fwd_params &p, unsigned block
         if (ra < rows) __syncthreads();
     }
 }
-template<int BITS, typename WT, int V, int SETS, bool SHORT_END>
-__global__ void __launch_bounds__(kGatherMaxWarps * 32, 2) qcsr_fwd_gather_kernel(const fwd_params p) {
-    gather_group<BITS, WT, V, SETS, SHORT_END>(p, blockIdx.x);
-}
-// The same, for a W that the integer kernel before it found too wide for fixed point.  The CTAs that are resident take the groups of
-// rows in turn: where W fits, which is the usual case, a CTA per group would have thousands start for nothing (20,000 x 2,000 at
-// N = 32: 79.8 us, the resident ones 75.2, as without this launch).  A wide W costs what the integer kernel's preparation did besides (145 us,
-// the gather kernel alone 84; one row of W in 2,000 of 1e6).
-template<int BITS, typename WT, int V, int SETS>
-__global__ void __launch_bounds__(kGatherMaxWarps * 32, 2) qcsr_fwd_gather_if_wide_kernel(const fwd_params p) {
-    wait_for_previous_launch();
-    if (__ldcg(p.wide) == 0) return;
-    const std::int64_t rows = p.row_end - p.row_begin;
-    for (std::int64_t first = static_cast<std::int64_t>(blockIdx.x) * p.group_rows; first < rows; first += static_cast<std::int64_t>(gridDim.x) * p.group_rows) {
-        gather_group<BITS, WT, V, SETS, false>(p, static_cast<unsigned>(first / p.group_rows));
-        __syncthreads();
-    }
-}
 
 // Rows and warps per CTA for a launch over `rows` rows; *group_rows == 0: a warp per row (none of it touches the order of a
 // row's sum).  Measured from 64 to 1,000,000 rows of 24 to 1,800 entries.
@@ -520,7 +500,7 @@ int narrowed(int n, int v) {
 int summing_lanes(int n, int widest) { return gather_lanes(n, narrowed(n, widest)); }
 
 template<int BITS, typename WT, int V, int SETS>
-cb200_status launch_gather(fwd_params p, int sm_count, cudaStream_t stream) {
+cb200_status launch_gather(fwd_params p, cudaStream_t stream) {
     const int tile = 32 * V;
     p.lanes = gather_lanes(p.n, V);
     p.out_vector = p.out_vector && p.n % V == 0;
@@ -532,16 +512,12 @@ cb200_status launch_gather(fwd_params p, int sm_count, cudaStream_t stream) {
         else qcsr_fwd_row_kernel<BITS, WT, V, SETS, 2><<<grid, 128, 0, stream>>>(p);
     } else {
         const std::int64_t left = rows - static_cast<std::int64_t>(p.full_groups) * p.group_rows;
-        const bool short_end = left > 0 && p.wide == nullptr;
+        const bool short_end = left > 0;
         const unsigned groups = p.full_groups + static_cast<unsigned>(short_end ? (left + p.group_rows / 4 - 1) / (p.group_rows / 4) : 0);
         p.parts = std::min(kGatherParts, 32 * 1024 / static_cast<int>(V * p.lanes * sizeof(float)));
         const std::size_t smem = static_cast<std::size_t>(p.warps) * kSegment * sizeof(int2) +
                                  static_cast<std::size_t>(p.parts) * V * p.lanes * sizeof(float);
-        if (p.wide != nullptr) {
-            const std::int64_t resident = 2ll * sm_count * kGatherMaxWarps / p.warps;
-            const unsigned ctas = static_cast<unsigned>(std::min((rows + p.group_rows - 1) / p.group_rows, resident));
-            CB200_CUDA_OK(launch_kernel(true, qcsr_fwd_gather_if_wide_kernel<BITS, WT, V, SETS>, dim3(ctas, tiles), p.warps * 32, smem, stream, p));
-        } else if (short_end) qcsr_fwd_gather_kernel<BITS, WT, V, SETS, true><<<dim3(groups, tiles), p.warps * 32, smem, stream>>>(p);
+        if (short_end) qcsr_fwd_gather_kernel<BITS, WT, V, SETS, true><<<dim3(groups, tiles), p.warps * 32, smem, stream>>>(p);
         else qcsr_fwd_gather_kernel<BITS, WT, V, SETS, false><<<dim3(groups, tiles), p.warps * 32, smem, stream>>>(p);
     }
     count_launch();
@@ -575,29 +551,29 @@ bool gather_packs(const qcsr_view &x, std::int64_t n, int dense_dtype) {
 }
 
 template<int BITS, typename WT, int V>
-cb200_status launch_sets(const fwd_params &p, int sm_count, cudaStream_t stream) {
+cb200_status launch_sets(const fwd_params &p, cudaStream_t stream) {
     constexpr int widest = 16 / static_cast<int>(sizeof(WT));
     switch (gather_lanes(p.n, V) / summing_lanes(p.n, widest)) {
-    case 8: if constexpr (8 * V <= widest) return launch_gather<BITS, WT, V, 8>(p, sm_count, stream); [[fallthrough]];
-    case 4: if constexpr (4 * V <= widest) return launch_gather<BITS, WT, V, 4>(p, sm_count, stream); [[fallthrough]];
-    case 2: if constexpr (2 * V <= widest) return launch_gather<BITS, WT, V, 2>(p, sm_count, stream); [[fallthrough]];
-    default: return launch_gather<BITS, WT, V, 1>(p, sm_count, stream);
+    case 8: if constexpr (8 * V <= widest) return launch_gather<BITS, WT, V, 8>(p, stream); [[fallthrough]];
+    case 4: if constexpr (4 * V <= widest) return launch_gather<BITS, WT, V, 4>(p, stream); [[fallthrough]];
+    case 2: if constexpr (2 * V <= widest) return launch_gather<BITS, WT, V, 2>(p, stream); [[fallthrough]];
+    default: return launch_gather<BITS, WT, V, 1>(p, stream);
     }
 }
 
 // Columns per lane: the widest slice, up to 16 bytes, that divides N and the rows' alignment.
 template<int BITS, typename WT>
-cb200_status dispatch_gather(const fwd_params &p, int sm_count, cudaStream_t stream) {
+cb200_status dispatch_gather(const fwd_params &p, cudaStream_t stream) {
     constexpr int widest = 16 / static_cast<int>(sizeof(WT));
     int v = p.w_ld * static_cast<std::int64_t>(sizeof(WT)) <= 0xffffffffll ? widest : 1;
     while (v > 1 && (p.n % v != 0 || reinterpret_cast<std::uintptr_t>(p.w) % (v * sizeof(WT)) != 0u || p.w_ld % v != 0)) v /= 2;
     if (p.packed_rows) v = widest; // the lane that holds the last columns of a row may hold fewer than v
     v = narrowed(p.n, v);
     switch (v) {
-    case 8: if constexpr (widest == 8) return launch_gather<BITS, WT, 8, 1>(p, sm_count, stream); [[fallthrough]];
-    case 4: return launch_sets<BITS, WT, 4>(p, sm_count, stream);
-    case 2: return launch_sets<BITS, WT, 2>(p, sm_count, stream);
-    default: return launch_sets<BITS, WT, 1>(p, sm_count, stream);
+    case 8: if constexpr (widest == 8) return launch_gather<BITS, WT, 8, 1>(p, stream); [[fallthrough]];
+    case 4: return launch_sets<BITS, WT, 4>(p, stream);
+    case 2: return launch_sets<BITS, WT, 2>(p, stream);
+    default: return launch_sets<BITS, WT, 1>(p, stream);
     }
 }
 
@@ -614,7 +590,7 @@ std::uint64_t qcsr_gather_workspace_bytes(std::int64_t cols, std::int64_t nnz, s
 
 cb200_status launch_qcsr_forward(const qcsr_view &x, const dense_args &d, std::int64_t row_begin,
                                  std::int64_t row_end, fwd_schedule schedule, const void *persistent,
-                                 const blocked_layout *blocked, const digit_layout *digits, bool split_products, void *workspace,
+                                 const blocked_layout *blocked, bool split_products, void *workspace,
                                  std::uint64_t workspace_bytes, int sm_count, cudaStream_t stream) {
     if (row_end <= row_begin || d.n == 0) return CB200_STATUS_SUCCESS;
     if (row_end - row_begin > 0x7fffffffll) return fail(CB200_STATUS_INVALID_SHAPE, "row range too large for one launch");
@@ -640,23 +616,17 @@ cb200_status launch_qcsr_forward(const qcsr_view &x, const dense_args &d, std::i
         if (st != CB200_STATUS_SUCCESS || taken) return st;
     }
     fwd_params p{};
-    if (schedule == fwd_schedule::integer_windows) {
-        const cb200_status st = launch_qcsr_forward_digits(x, d, row_begin, row_end, workspace, workspace_bytes,
-                                                           digits != nullptr && digits->words != nullptr ? digits : nullptr, sm_count, stream, &p.wide);
-        if (st != CB200_STATUS_SUCCESS) return st;
-    }
     p.row_ptr = x.row_ptr; p.packed_row_ptr = x.packed_row_ptr; p.col_idx = x.col_idx; p.packed = x.packed;
     p.scales = x.scales; p.offsets = x.offsets; p.w = d.dense; p.y = d.out; p.w_ld = d.dense_ld; p.y_ld = d.out_ld;
     p.row_begin = row_begin; p.row_end = row_end; p.n = static_cast<int>(d.n); p.policy = x.policy;
     p.alpha = d.alpha; p.beta = d.beta; p.bias = d.bias; p.epilogue = d.epilogue;
 
     p.out_vector = reinterpret_cast<std::uintptr_t>(d.out) % 16u == 0u && d.out_ld % 4 == 0 ? 1 : 0;
-    p.status = workspace_bytes >= sizeof(int) && p.wide == nullptr ? static_cast<int *>(workspace) : nullptr;
+    p.status = workspace_bytes >= sizeof(int) ? static_cast<int *>(workspace) : nullptr;
     const bool bf16 = d.dense_dtype == CB200_DTYPE_BF16;
     gather_shape(x, row_end - row_begin, d.n * (bf16 ? 2 : 4), sm_count, &p);
-    if (p.group_rows == 0 && p.wide != nullptr) p.group_rows = kGatherMaxRows;
     if (p.group_rows == 0) p.short_rows = x.nnz < 64 * x.rows ? 1 : 0;
-    if (p.wide == nullptr && gather_packs(x, d.n, d.dense_dtype) && workspace_bytes >= qcsr_gather_workspace_bytes(x.cols, x.nnz, d.n, d.dense_dtype)) {
+    if (gather_packs(x, d.n, d.dense_dtype) && workspace_bytes >= qcsr_gather_workspace_bytes(x.cols, x.nnz, d.n, d.dense_dtype)) {
         const int per_piece = bf16 ? 8 : 4, pieces = static_cast<int>((d.n + per_piece - 1) / per_piece);
         uint4 *packed = reinterpret_cast<uint4 *>(static_cast<unsigned char *>(workspace) + 256);
         const unsigned grid = static_cast<unsigned>((x.cols * pieces + 255) / 256);
@@ -668,13 +638,13 @@ cb200_status launch_qcsr_forward(const qcsr_view &x, const dense_args &d, std::i
         p.packed_rows = 1;
     }
     if (x.bits == 8) {
-        if (bf16) return dispatch_gather<8, __nv_bfloat16>(p, sm_count, stream);
-        return dispatch_gather<8, float>(p, sm_count, stream);
+        if (bf16) return dispatch_gather<8, __nv_bfloat16>(p, stream);
+        return dispatch_gather<8, float>(p, stream);
     }
     if (x.bits == 4) {
         if (x.packed_row_ptr == nullptr) return fail(CB200_STATUS_INVALID_ARGUMENT, "4-bit codes need packed_row_ptr");
-        if (bf16) return dispatch_gather<4, __nv_bfloat16>(p, sm_count, stream);
-        return dispatch_gather<4, float>(p, sm_count, stream);
+        if (bf16) return dispatch_gather<4, __nv_bfloat16>(p, stream);
+        return dispatch_gather<4, float>(p, stream);
     }
     return fail(CB200_STATUS_UNSUPPORTED, "forward SpMM supports 8-bit and 4-bit codes, got %d", x.bits);
 }

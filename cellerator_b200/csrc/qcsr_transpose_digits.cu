@@ -43,11 +43,11 @@
 
 namespace cb200 {
 
+namespace {
+
 // Thirty-two cells to a piece, or sixteen where those would leave SMs without a CTA to lay them out (4,099 x 33,538: 49 us and 38; 8,191
 // rows, two CTAs to most SMs: 65 and 70).
-int qcsr_digit_piece_rows(std::int64_t rows) { return rows >= 32 * 148 ? 32 : 16; }
-
-namespace {
+int piece_rows_of(std::int64_t rows) { return rows >= 32 * 148 ? 32 : 16; }
 
 constexpr int kWin = 128;                       // genes per window
 constexpr int kRows = 256;                      // cells per group
@@ -118,8 +118,7 @@ constexpr std::int64_t kTwice = kDigitWordsTwice;
 // holds twice: a tile has one place for them.
 //
 // What bounds it: the latency of the genes' loads (eight in flight per warp, 48 warps per SM) and issue, half of the slots.
-// FORWARD: the places are those of the forward kernel's tile (qcsr_forward_digits.cu), in units of two bytes.
-template<int BITS, bool FORWARD>
+template<int BITS>
 __global__ void __launch_bounds__(kBuildThreads, 2) digit_words_kernel(const words_params p) {
     extern __shared__ std::uint32_t place_of[]; // [kPieceRows][pitch]; see below.  Behind it [chunks][kPieceRows + 1] and [windows]
     __shared__ std::int64_t codes_of[kPieceRows]; // where the codes of a cell begin
@@ -141,8 +140,7 @@ __global__ void __launch_bounds__(kBuildThreads, 2) digit_words_kernel(const wor
         if (tid < cells) {
             const std::uint32_t cell = (blockIdx.x * p.piece_rows + tid) & (kRows - 1);
             codes_of[tid] = p.packed_row_ptr != nullptr ? __ldg(p.packed_row_ptr + row0 + tid) : at;
-            // transpose: plane half, 16-byte piece, byte; forward (two bytes): cell, 16-byte piece
-            const std::uint32_t place = FORWARD ? cell * 64u + ((cell & 7u) << 3) : (cell >> 7) * (kPlaneBytes / 2) + ((cell & 127u) >> 4 << 4) + (cell & 15u);
+            const std::uint32_t place = (cell >> 7) * (kPlaneBytes / 2) + ((cell & 127u) >> 4 << 4) + (cell & 15u); // plane half, 16-byte piece, byte
             cell_bits[tid] = place << 8 | static_cast<std::uint32_t>(p.code_bias);
         }
     }
@@ -220,9 +218,7 @@ __global__ void __launch_bounds__(kBuildThreads, 2) digit_words_kernel(const wor
             }
     };
     const auto word_of = [&](std::uint32_t bits, int gene, std::uint32_t code) {
-        // {code less the bias, place in the tile << 8}.  Transpose: [plane half][gene][piece ^ gene % 8][byte]; forward: [gene half][cell]
-        // [piece ^ cell % 8][gene % 8]
-        if constexpr (FORWARD) return bits ^ (static_cast<std::uint32_t>(gene & 64) << 16 | static_cast<std::uint32_t>(gene & 63) << 8) ^ code;
+        // {code less the bias, place in the tile << 8}; the place: [plane half][gene][piece ^ gene % 8][byte]
         return bits ^ (static_cast<std::uint32_t>(gene & (kWin - 1)) << 15 | static_cast<std::uint32_t>(gene & 7) << 12) ^ code;
     };
     const auto code_at = [&](int r, int i) -> std::uint32_t {
@@ -333,8 +329,7 @@ __global__ void __launch_bounds__(kBuildThreads, 2) digit_words_kernel(const wor
                 const std::uint32_t e = out[i];
                 if (static_cast<int>(e) < 0) continue;
                 const std::uint32_t place = e >> 8;
-                const std::uint32_t gl = FORWARD ? (place >> 14 & 1u) << 6 | ((place ^ (place >> 3)) & 0x38u) | (place & 7u) : (place >> 7) & (kWin - 1);
-                const std::uint32_t cell = (FORWARD ? place >> 6 : ((place >> 4 ^ gl) & 7u) << 4 | (place & 15u)) & (kPieceRows - 1);
+                const std::uint32_t gl = (place >> 7) & (kWin - 1), cell = (((place >> 4 ^ gl) & 7u) << 4 | (place & 15u)) & (kPieceRows - 1);
                 twice = twice || (atomicOr(seen + gl, 1u << cell) >> cell & 1u) != 0u;
             }
             __syncwarp();
@@ -1071,7 +1066,7 @@ std::uint64_t launch_bytes(std::int64_t groups, std::int64_t cols, std::int64_t 
     return kRecordsAt + record_bytes(groups, n, slices) + partial_bytes(groups, cols, n, slices, ctas);
 }
 std::int64_t group_count_of(std::int64_t rows) { return (rows + kRows - 1) / kRows; }
-std::int64_t piece_count(std::int64_t rows) { return (rows + qcsr_digit_piece_rows(rows) - 1) / qcsr_digit_piece_rows(rows); }
+std::int64_t piece_count(std::int64_t rows) { return (rows + piece_rows_of(rows) - 1) / piece_rows_of(rows); }
 std::uint64_t word_bytes(std::int64_t rows, std::int64_t cols, std::int64_t nnz) {
     const std::int64_t windows = (cols + kWin - 1) / kWin;
     return static_cast<std::uint64_t>(nnz + 4 + piece_count(rows) * (4 * windows + 4)) * 4u;
@@ -1134,13 +1129,13 @@ cb200_status launch_digits(const digit_launch &l, int sm_count, cudaStream_t str
 
 } // namespace
 
-cb200_status launch_digit_words(const qcsr_view &x, std::int64_t row_begin, std::int64_t row_end, bool forward, std::uint32_t *words, std::uint32_t *bounds,
+cb200_status launch_digit_words(const qcsr_view &x, std::int64_t row_begin, std::int64_t row_end, std::uint32_t *words, std::uint32_t *bounds,
                                 std::int64_t *bases, int *status, cudaStream_t stream) {
     words_params p{};
     p.row_ptr = x.row_ptr; p.packed_row_ptr = x.packed_row_ptr; p.col_idx = x.col_idx; p.packed = x.packed;
     p.row_begin = row_begin; p.row_end = row_end; p.cols = x.cols; p.windows = static_cast<int>((x.cols + kWin - 1) / kWin);
     p.code_bias = x.bits == 8 ? 128 : 0;
-    p.piece_rows = qcsr_digit_piece_rows(x.rows);
+    p.piece_rows = piece_rows_of(x.rows);
     p.words = words; p.bounds = bounds; p.bases = bases; p.status = status;
     const int smem = build_smem_bytes(x.cols);
     const unsigned grid = static_cast<unsigned>((row_end - row_begin + p.piece_rows - 1) / p.piece_rows);
@@ -1149,8 +1144,7 @@ cb200_status launch_digit_words(const qcsr_view &x, std::int64_t row_begin, std:
         if (err == cudaSuccess) kernel<<<grid, kBuildThreads, smem, stream>>>(p);
         return err;
     };
-    if (x.bits == 8) CB200_CUDA_OK(forward ? run(digit_words_kernel<8, true>) : run(digit_words_kernel<8, false>));
-    else CB200_CUDA_OK(forward ? run(digit_words_kernel<4, true>) : run(digit_words_kernel<4, false>));
+    CB200_CUDA_OK(x.bits == 8 ? run(digit_words_kernel<8>) : run(digit_words_kernel<4>));
     count_launch();
     CB200_CUDA_OK(cudaGetLastError());
     return CB200_STATUS_SUCCESS;
@@ -1190,7 +1184,7 @@ std::uint64_t qcsr_transpose_digits_once_bytes(std::int64_t rows, std::int64_t c
     return qcsr_transpose_digits_workspace_bytes(rows, cols, n, 4) + qcsr_digit_words_bytes_bound(rows, cols, nnz);
 }
 
-cb200_status build_digit_words(const qcsr_view &x, bool forward, device_arena &arena, cudaStream_t stream, digit_layout *out) {
+cb200_status build_digit_words(const qcsr_view &x, device_arena &arena, cudaStream_t stream, digit_layout *out) {
     *out = digit_layout{};
     if (x.row_ptr == nullptr || (x.nnz != 0 && (x.col_idx == nullptr || x.packed == nullptr)))
         return fail(CB200_STATUS_INVALID_ARGUMENT, "the matrix handed to prepare has null arrays");
@@ -1202,7 +1196,7 @@ cb200_status build_digit_words(const qcsr_view &x, bool forward, device_arena &a
     cb200_status st = CB200_STATUS_SUCCESS;
     if (out->words == nullptr || out->bounds == nullptr || out->bases == nullptr)
         st = fail(CB200_STATUS_INSUFFICIENT_WORKSPACE, "no device memory for the entry words");
-    if (st == CB200_STATUS_SUCCESS) st = launch_digit_words(x, 0, x.rows, forward, out->words, out->bounds, out->bases, nullptr, stream);
+    if (st == CB200_STATUS_SUCCESS) st = launch_digit_words(x, 0, x.rows, out->words, out->bounds, out->bases, nullptr, stream);
     if (st == CB200_STATUS_SUCCESS) {
         const cudaError_t err = cudaStreamSynchronize(stream);
         if (err != cudaSuccess) st = fail(CB200_STATUS_CUDA_ERROR, "building the entry words: %s", cudaGetErrorString(err));
@@ -1252,12 +1246,12 @@ cb200_status launch_qcsr_transpose_digits(const qcsr_view &x, const dense_args &
         p.words = layout->words; p.bounds = layout->bounds; p.bases = layout->bases;
     } else {
         const digit_layout made = digit_words_at(ws + own, x);
-        const cb200_status st = launch_digit_words(x, row_begin, row_end, false, made.words, made.bounds, made.bases, p.status, stream);
+        const cb200_status st = launch_digit_words(x, row_begin, row_end, made.words, made.bounds, made.bases, p.status, stream);
         if (st != CB200_STATUS_SUCCESS) return st;
         p.words = made.words; p.bounds = made.bounds; p.bases = made.bases;
     }
     const int nb = column_block(d.n);
-    p.piece_rows = qcsr_digit_piece_rows(x.rows);
+    p.piece_rows = piece_rows_of(x.rows);
     p.group_pieces = kRows / p.piece_rows;
     p.pieces = (rows_of_words + p.piece_rows - 1) / p.piece_rows;
     p.scales = x.scales; p.offsets = x.offsets;

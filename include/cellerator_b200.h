@@ -265,9 +265,8 @@ typedef struct cb200_spmm_problem {
      * hi + lo; hi*hi + hi*lo + lo*hi), relative error about 3 * 2^-17 per product: inside the 1e-4
      * bound of an fp32 operand, not bit-equal to an fp32 multiply.  The transpose with zero-points per gene
      * multiplies the codes with three digits of G in fixed point instead (2^-23 of a column's largest
-     * magnitude) and adds without rounding.  Without device_matrix "gene_tiled" / "warp_per_row" (fp32 FMAs),
-     * "integer_windows" (four digits of W and integer sums: more exact than fp32) and "vector_reductions" (fp32
-     * FMAs, or four digits of G and integer sums) run. */
+     * magnitude) and adds without rounding.  Without device_matrix "gene_tiled" / "warp_per_row" (fp32 FMAs)
+     * and "vector_reductions" (fp32 FMAs, or four digits of G and integer sums) run. */
     int32_t multiply;
     /* Optional: the device-resident matrix itself (arrays on `device`, final contents).  With bf16
      * products allowed, prepare then builds a persistent window-blocked copy of it (one 32-bit
@@ -299,7 +298,7 @@ typedef struct cb200_spmm_problem {
      * CB200_STATUS_STALE_VALUE instead of multiplying stale values. */
     uint64_t value_generation;
     /* Optional request for one schedule by the name cb200_prepared_schedule reports ("gene_tiled",
-     * "warp_per_row", "integer_windows", "tensor_windows", "tensor_blocked", "tensor_dense", "tensor_codes"; transpose:
+     * "warp_per_row", "tensor_windows", "tensor_blocked", "tensor_dense", "tensor_codes"; transpose:
      * "tensor_blocked", "vector_reductions", "gene_gather"; Blocked-ELL: "cuda_cores"); NULL or "" lets prepare choose from the shape and
      * the row statistics.  A request the shape or the policy cannot serve is not an error: prepare
      * keeps its own choice, and cb200_prepared_schedule tells which schedule runs.  This is the
@@ -329,14 +328,12 @@ cb200_status cb200_spmm_persistent_requirement(const cb200_spmm_problem *problem
 void cb200_prepared_destroy(cb200_prepared *prepared);
 /* workspace_requirement, launch_bindings.hh:67-71: what the schedule can use.  "vector_reductions" reports up to 32 MB (it
  * sorts the entries with it, slice of rows by slice), or for 2 to 50 million entries about 4 bytes an entry (words for integer
- * sums), and also runs with less or with none, slower.  "integer_windows" needs what it reports, some 4 bytes an entry and 8 N
- * bytes a gene.  "warp_per_row" (unaligned
+ * sums), and also runs with less or with none, slower.  "warp_per_row" (unaligned
  * N) and the tensor_blocked and tensor_dense forward schedules also run with less, down to the status block and the records of
  * W, slower and with the same bits: a row's sum follows from its entries, N and W's type, not from the room, the launch's row
- * range or the rows beside it ("integer_windows" with less than it reports runs "warp_per_row", whose sums differ by rounding). */
+ * range or the rows beside it. */
 cb200_status cb200_prepared_workspace(const cb200_prepared *prepared, uint64_t *minimum_bytes, uint32_t *alignment);
-/* kernel choice made at prepare time, as text: "warp_per_row", "gene_tiled" (exact fp32 products), "integer_windows" (codes
- * times digits of W, exact integer sums; zero-points per gene, 2 to 50 million entries, N times entries from 200 million on);
+/* kernel choice made at prepare time, as text: "warp_per_row", "gene_tiled" (exact fp32 products);
  * "tensor_windows", "tensor_blocked", "tensor_dense", "tensor_codes" (CSR, 16-bit products on tcgen05);
  * "tensor_blocked_x2" / "_x3" (fp32 products from bf16 passes); "tcgen05_block_rows" (Blocked-ELL);
  * transpose: "vector_reductions" (exact) or "tensor_blocked" */

@@ -112,3 +112,58 @@ def test_both_kernels_give_a_row_the_same_bits(cuda_device, oracle, mean):
     for n, dtype in ((1, torch.float32), (5, torch.bfloat16), (8, torch.float32), (16, torch.bfloat16), (50, torch.bfloat16), (64, torch.float32)):
         w, _ = dense(rng, 4000, n, dtype, cuda_device)
         assert torch.equal(ops.spmm_forward(part, w), ops.spmm_forward(x, w)[:600]), n
+
+
+@pytest.mark.parametrize("n,dtype", [(64, torch.bfloat16), (130, torch.float32)])
+def test_a_rows_bits_in_matrices_of_any_size(cuda_device, oracle, n, dtype):
+    """Millions of entries or thousands of them, dense rows, wide W: the whole matrix, shards of a few and of most of its rows, row ranges and a
+    launch with the least workspace give a row the same bits."""
+    rng = np.random.default_rng(n)
+    c = matrix(oracle, rng.integers(300, 700, size=6500), 4000, 8, 1, n)
+    x = to_dev(c, cuda_device)
+    assert x.nnz >= 3_000_000
+    w, _ = dense(rng, 4000, n, dtype, cuda_device)
+    y = ops.spmm_forward(x, w)
+    op = ops.PreparedSpmm(capi.PROJECTION_CSR, c["rows"], 4000, n, x.nnz, 8, 1, dtype, cuda_device)
+    op.workspace_bytes = 256
+    assert torch.equal(op.run(x, w, torch.empty_like(y)), y)
+    assert torch.equal(op.run(x, w, torch.empty_like(y), row_begin=5, row_end=41)[5:41], y[5:41])
+    op.close()
+    for lo, hi in ((0, 7), (30, 1500), (1, 6499)):
+        assert torch.equal(ops.spmm_forward(to_dev(rows_of(c, lo, hi), cuda_device), w), y[lo:hi]), (lo, hi)
+
+
+def test_what_reaches_a_row(cuda_device, oracle):
+    """Genes that a row holds twice count twice, rows may be in any order; outliers, infinities and NaNs reach the rows that hold their genes and
+    no others; so do scales that are not finite."""
+    rng = np.random.default_rng(8)
+    rows, cols, n = 256 * 5 + 40, 1100, 64
+    c = matrix(oracle, rng.integers(0, 101, size=rows), cols, 8, 1, 8)
+    for r in range(200, rows, 41):
+        lo, hi = c["row_ptr"][r], c["row_ptr"][r + 1]
+        c["col_idx"][lo:hi] = rng.permutation(c["col_idx"][lo:hi])
+    c["col_idx"][(c["col_idx"] == 300) & (np.arange(len(c["col_idx"])) > len(c["col_idx"]) // 2)] = 303
+    w_host = dense(rng, cols, n, torch.float32, cuda_device)[1].copy()
+
+    def compare():
+        got = ops.spmm_forward(to_dev(c, cuda_device), torch.from_numpy(w_host).to(cuda_device)).cpu().numpy()
+        with np.errstate(invalid="ignore", over="ignore"):
+            dec = oracle.unpack_csr(8, 1, c["row_ptr"], c["packed_row_ptr"], c["col_idx"], c["scales"], c["offsets"], c["packed"]).astype(np.float64)
+            r = np.repeat(np.arange(rows), np.diff(c["row_ptr"]))
+            want, scale = np.zeros((rows, n)), np.zeros((rows, n))
+            for j in range(n):
+                np.add.at(want[:, j], r, dec * w_host[c["col_idx"], j])
+                np.add.at(scale[:, j], r, (2 * np.abs(dec) + np.abs(c["offsets"][c["col_idx"]])) * np.abs(w_host[c["col_idx"], j]))
+            finite = np.isfinite(want)
+            assert np.array_equal(np.isnan(got), np.isnan(want)) and np.array_equal(got[np.isinf(want)], want[np.isinf(want)])
+            # fp32 sums of up to 100 products, 2^-24 of the terms' magnitudes each; the oracle decodes with two roundings
+            assert np.all(np.abs(got[finite] - want[finite]) <= 102 * 2.0 ** -24 * scale[finite] + 1e-30)
+
+    compare()
+    w_host[77, 5] = 1e6
+    compare()
+    w_host[123, 9], w_host[400, 9], w_host[401, 11] = np.inf, -np.inf, np.nan
+    compare()
+    w_host[:] = rng.normal(size=w_host.shape)
+    c["scales"][500], c["offsets"][7] = np.nan, np.inf
+    compare()
