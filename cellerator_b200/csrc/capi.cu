@@ -567,8 +567,8 @@ cb200_status cb200_spmm_prepare(const cb200_spmm_problem *problem, cb200_prepare
             if (st != CB200_STATUS_SUCCESS) return abandon(st);
             p->digit_slices = plan.digits;
             p->schedule_name = plan.digits == 4 ? "gene_gather" : "tensor_blocked_x3";
-            p->workspace_bytes = qcsr_transpose_digits_workspace_bytes(problem->m, problem->k, problem->n, plan.digits);
-            p->workspace_required = qcsr_transpose_digits_least_workspace(problem->m, problem->k, problem->n, plan.digits, p->sm_count);
+            p->workspace_bytes = qcsr_transpose_digits_workspace_bytes(problem->m, problem->k, problem->n, plan.digits, plan.digits == 4);
+            p->workspace_required = qcsr_transpose_digits_least_workspace(problem->m, problem->k, problem->n, plan.digits, plan.digits == 4, p->sm_count);
             p->persistent_bytes += p->digits.bytes;
         }
         if (plan.gene_gather) {

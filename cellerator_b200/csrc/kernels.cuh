@@ -203,7 +203,8 @@ cb200_status launch_qcsr_transpose_blocked(const qcsr_view &x, const dense_args 
                                            cudaStream_t stream, bool *taken);
 
 // Transpose with exact integer sums on the tensor cores (zero-points per gene): codes times the digits of G in fixed point.
-// slices: digits of G, 3 (products as exact as three bf16 ones) or 4 (as fp32 ones).
+// slices: digits of G, 3 (products as exact as three bf16 ones) or 4 (as fp32 ones).  repeatable (prepared words and 4 digits only): the bits
+// follow from the operands and the row range alone, not from the workspace or the number of SMs.
 // The entries in pieces of 16 or 32 cells (by the number of the matrix's rows), by window of 128 genes, a word each: {code, less 128 if it has 8 bits, place in the operand
 // tile << 8}; scales and zero-points are read at launch.
 struct digit_layout {
@@ -222,13 +223,13 @@ cb200_status build_digit_words(const qcsr_view &x, device_arena &arena, cudaStre
 digit_layout digit_words_at(void *memory, const qcsr_view &x);
 cb200_status launch_digit_words(const qcsr_view &x, std::int64_t row_begin, std::int64_t row_end, std::uint32_t *words, std::uint32_t *bounds,
                                 std::int64_t *bases, int *status, cudaStream_t stream);
-std::uint64_t qcsr_transpose_digits_workspace_bytes(std::int64_t rows, std::int64_t cols, std::int64_t n, int slices);
-std::uint64_t qcsr_transpose_digits_least_workspace(std::int64_t rows, std::int64_t cols, std::int64_t n, int slices, int sm_count); // slower
+std::uint64_t qcsr_transpose_digits_workspace_bytes(std::int64_t rows, std::int64_t cols, std::int64_t n, int slices, bool repeatable);
+std::uint64_t qcsr_transpose_digits_least_workspace(std::int64_t rows, std::int64_t cols, std::int64_t n, int slices, bool repeatable, int sm_count); // slower
 // Whether a call that sees its matrix once should make the words in its workspace (0: no), and what it then needs
 std::uint64_t qcsr_transpose_digits_once_bytes(std::int64_t rows, std::int64_t cols, std::int64_t n, std::int64_t nnz, int bits, int policy);
 // layout null: the words are made in the workspace.  *taken is false where the shape or the workspace rules it out.
 cb200_status launch_qcsr_transpose_digits(const qcsr_view &x, const dense_args &d, std::int64_t row_begin, std::int64_t row_end, void *workspace,
-                                          std::uint64_t workspace_bytes, const digit_layout *layout, int slices, int sm_count, cudaStream_t stream, bool *taken);
+                                          std::uint64_t workspace_bytes, const digit_layout *layout, int slices, bool repeatable, int sm_count, cudaStream_t stream, bool *taken);
 
 // G'[g,:] = alpha * sum_{r in range, col_i == g} deq(code_i) * G[r,:] + beta * G'[g,:]
 // `blocked` (optional): the window-blocked copy of a prepared bf16-product operation.  `digits` (optional): the words of a prepared

@@ -173,7 +173,7 @@ cb200_status launch_qcsr_transpose(const qcsr_view &x, const dense_args &d, std:
     if (prepared_words || (!copied && qcsr_transpose_digits_once_bytes(row_end - row_begin, x.cols, d.n, part_nnz, x.bits, x.policy) != 0u)) {
         bool taken = false;
         const cb200_status st = launch_qcsr_transpose_digits(x, d, row_begin, row_end, workspace, workspace_bytes, prepared_words ? digits : nullptr,
-                                                             prepared_words ? slices : 4, sm_count, stream, &taken);
+                                                             prepared_words ? slices : 4, prepared_words && slices == 4, sm_count, stream, &taken);
         if (st != CB200_STATUS_SUCCESS || taken) return st;
     }
     if (blocked != nullptr && blocked->seg_ptr != nullptr) {

@@ -10,7 +10,10 @@
 // its largest magnitude, as S signed digits of base 256 (S = 4: rounded at 2^-31 of the largest; S = 3: at 2^-23).  Codes
 // (less 128, to be signed) and digits are what the tensor cores' 8-bit integer MMAs multiply, and these add in 32 bits without
 // rounding: every product and every sum up to the end of a run is exact, whatever their order.  The only errors are the rounding
-// of G to its fixed point and a handful of fp32 roundings at the end.  Against 64 bits (2-norm, genes of the 33,538-gene
+// of G to its fixed point and a handful of fp32 roundings at the end: of each run, and of the sum of a set's runs, of which there are as many as
+// CTAs share the set.  A request that has to be repeatable (EXACT) adds the runs up as whole numbers instead, 64 bits in L2, and rounds once:
+// its bits follow from the operands and the row range alone, not from the number of SMs nor from the workspace, whose lack
+// only cuts the launch into slices of groups and chunks of windows (100,003 x 33,538, N = 64: 1,099 us, with rounded runs 1,093).  Against 64 bits (2-norm, genes of the 33,538-gene
 // matrices): S = 4 4e-8, where fp32 FMAs leave 1.2e-7 (8,191 cells) to 4.8e-7 (100,003 cells, in a fixed order); S = 3 2e-7, where
 // products put together from three bf16 products and summed by the fp32 MMAs leave 6.2e-6.
 //
@@ -433,7 +436,8 @@ __global__ void __launch_bounds__(1024) column_range_kernel(const float *g, std:
 template<int NB, int SLICES>
 __global__ void __launch_bounds__(256) pack_digits_kernel(const float *g, std::int64_t ld, int n, int padded, std::int64_t first_row, std::int64_t row_begin,
                                                           std::int64_t row_end, std::int64_t groups, const unsigned *part_max, const ulonglong2 *part_sum,
-                                                          double *steps, unsigned char *records, const std::int64_t *bases, std::int64_t word_pieces, int *wide) {
+                                                          double *steps, unsigned char *records, const std::int64_t *bases, std::int64_t word_pieces, int *wide,
+                                                          uint4 *totals, std::int64_t total_items) { // the totals to clear, 16 bytes each, of one pass
     __shared__ unsigned most_of[256];
     __shared__ ulonglong2 sum_of[256];
     __shared__ double factor[kMaxColumns]; // 2^k: what a column is multiplied by
@@ -499,6 +503,7 @@ __global__ void __launch_bounds__(256) pack_digits_kernel(const float *g, std::i
         if (blockIdx.x == 0 && tid == 0) *wide = by_entry ? 2 : second ? 1 : 0;
         passes = second ? 2 : 1;
     }
+    for (std::int64_t i = blockIdx.x * 256 + tid; i < passes * total_items; i += gridDim.x * 256) totals[i] = make_uint4(0u, 0u, 0u, 0u);
     constexpr int NC = mma_columns(NB, SLICES);
     const std::int64_t pieces = static_cast<std::int64_t>((n + NB - 1) / NB) * groups * kGPieces;
     for (std::int64_t b = blockIdx.x; b < passes * pieces; b += gridDim.x) {
@@ -553,9 +558,11 @@ struct digit_params {
     const unsigned char *records;
     const double *steps;
     const int *wide;         // 0: one pass, 1: two, 2: entry by entry
-    float *partials;         // [run_of + CTA][window of the set][gene][NB]
+    float *partials;         // [run_of + CTA][window of the set][column][gene]: a run's sums, rounded
+    long long *totals;       // EXACT: [set][window of the set][codes, ones][column][gene], which the runs add to
     std::int64_t cols;
     std::int64_t group_begin, group_count;
+    std::int64_t first_set, set_count; // of the launch
     std::int64_t run_groups; // groups after which a run ends at the latest
     int windows, column_blocks, code_bias;
     int *status;
@@ -578,11 +585,11 @@ __device__ __forceinline__ std::int64_t cta_of(std::int64_t unit, std::int64_t t
 struct tile_cursor {
     std::int64_t unit;
     int group, set, wl, windows_of_set; // group: of the launch; set: of the column block
-    const int groups, sets, windows, per_set;
+    const int groups, sets, windows, per_set; // windows: from the launch's first one on
     __device__ __forceinline__ int windows_in(int s) const { return min(per_set, windows - s * per_set); }
     __device__ __forceinline__ tile_cursor(const digit_params &p, std::int64_t sets_, std::int64_t first, int per_set_)
         : unit(first), group(static_cast<int>(first % p.group_count)), set(static_cast<int>(first / p.group_count % sets_)), wl(0), windows_of_set(0),
-          groups(static_cast<int>(p.group_count)), sets(static_cast<int>(sets_)), windows(p.windows), per_set(per_set_) {
+          groups(static_cast<int>(p.group_count)), sets(static_cast<int>(sets_)), windows(p.windows - static_cast<int>(p.first_set) * per_set_), per_set(per_set_) {
         windows_of_set = windows_in(set);
     }
     __device__ __forceinline__ void next() {
@@ -595,6 +602,10 @@ struct tile_cursor {
         windows_of_set = windows_in(set);
     }
 };
+// A gene's sum in one column.  The sums are below 2^57: in double precision scale and offset may cancel to the last bits of fp32.
+__device__ __forceinline__ double value_of(long long coded, long long present, int code_bias, double scale, double offset, double step) {
+    return (scale * static_cast<double>(coded + code_bias * present) + offset * static_cast<double>(present)) * step;
+}
 // K-major operand, no swizzle (a piece of G): core matrices of 8 columns x 16 cells; the next 16 cells 128 bytes on, the next 8
 // columns 512.
 __device__ __forceinline__ std::uint64_t smem_desc_digits(std::uint32_t addr) {
@@ -606,7 +617,7 @@ __device__ __forceinline__ std::uint64_t smem_desc_digits(std::uint32_t addr) {
     return d;
 }
 
-template<int NB, int SLICES>
+template<int NB, int SLICES, bool EXACT>
 __global__ void __launch_bounds__(kThreads, 1) qcsr_transpose_digits_kernel(const digit_params p) {
     constexpr int NC = mma_columns(NB, SLICES), kSet = set_windows(NB, SLICES), GPIECE = g_piece_bytes(NB, SLICES), kPieces = ring_pieces(NB, SLICES);
     constexpr std::uint32_t IDESC = instr_desc_i8(NC);
@@ -656,7 +667,7 @@ __global__ void __launch_bounds__(kThreads, 1) qcsr_transpose_digits_kernel(cons
     const std::uint32_t tmem_base = *tmem_slot;
     wait_for_previous_launch();
 
-    const std::int64_t sets = (p.windows + kSet - 1) / kSet;
+    const std::int64_t sets = p.set_count;
     const int wide = __ldcg(p.wide);
     // the second pass: as many column blocks again
     const std::int64_t total_units = sets * p.column_blocks * p.group_count * (wide == 1 ? 2 : 1);
@@ -681,19 +692,20 @@ __global__ void __launch_bounds__(kThreads, 1) qcsr_transpose_digits_kernel(cons
         // number allows, sixteen columns of one window.  `from` is the run's first unit, `to` the one behind its last.
         const auto put_together = [&](std::int64_t from, std::int64_t to) {
             const std::int64_t set_of_all = from / p.group_count, set = set_of_all % sets;
-            const int nwin = static_cast<int>(min(static_cast<std::int64_t>(kSet), p.windows - set * kSet));
+            const int nwin = static_cast<int>(min(static_cast<std::int64_t>(kSet), p.windows - (p.first_set + set) * kSet));
             bar_wait(smem_addr(acc_full), static_cast<std::uint32_t>(run & 1), abort_flag);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const int quarter = warp & 3, wl = NB == 64 ? 0 : warp >> 3, c0 = (NB == 64 ? warp >> 2 : (warp >> 2) & 1) * 16;
-            const std::int64_t gene = (set * kSet + wl) * kWin + quarter * 32 + lane;
+            const std::int64_t gene = ((p.first_set + set) * kSet + wl) * kWin + quarter * 32 + lane;
             if (wl < nwin) { // warp-uniform
                 double scale = 0.0, offset = 0.0;
-                if (gene < p.cols) {
+                if (!EXACT && gene < p.cols) {
                     scale = p.scales != nullptr ? static_cast<double>(__ldg(p.scales + gene)) : 1.0;
                     offset = p.offsets != nullptr ? static_cast<double>(__ldg(p.offsets + gene)) : 0.0;
                 }
                 const std::uint32_t at = tmem_base + (static_cast<std::uint32_t>(quarter * 32) << 16) + wl * 2 * NC + c0;
-                float *slot = p.partials + (((run_of(to - 1, p.group_count, p.run_groups) + blockIdx.x) * kSet + wl) * kWin + quarter * 32 + lane) * NB + c0;
+                float *slot = p.partials + (((run_of(to - 1, p.group_count, p.run_groups) + blockIdx.x) * kSet + wl) * NB + c0) * kWin + quarter * 32 + lane;
+                unsigned long long *total = reinterpret_cast<unsigned long long *>(p.totals) + ((set_of_all * kSet + wl) * 2 * NB + c0) * kWin + quarter * 32 + lane;
                 const double *steps = p.steps + set_of_all / sets * NB + c0;
 #pragma unroll
                 for (int h = 0; h < 16; h += 8) {
@@ -709,13 +721,16 @@ __global__ void __launch_bounds__(kThreads, 1) qcsr_transpose_digits_kernel(cons
                             present[c] = k == 0 ? b[c] : present[c] * 256 + b[c];
                         }
                     }
-                    float v[8];
-#pragma unroll
-                    for (int c = 0; c < 8; ++c) // below 2^56: in double precision scale and offset may cancel to the last bits of fp32
-                        v[c] = static_cast<float>((scale * static_cast<double>(coded[c] + p.code_bias * present[c]) + offset * static_cast<double>(present[c])) * __ldg(steps + h + c));
                     if (gene < p.cols && *abort_flag == 0) {
-                        *reinterpret_cast<float4 *>(slot + h) = make_float4(v[0], v[1], v[2], v[3]);
-                        *reinterpret_cast<float4 *>(slot + h + 4) = make_float4(v[4], v[5], v[6], v[7]);
+#pragma unroll
+                        for (int c = 0; c < 8; ++c) {
+                            if constexpr (EXACT) { // whole numbers: the same totals in whatever order and pieces
+                                atomicAdd(total + (h + c) * kWin, static_cast<unsigned long long>(coded[c]));
+                                atomicAdd(total + (NB + h + c) * kWin, static_cast<unsigned long long>(present[c]));
+                            } else {
+                                slot[(h + c) * kWin] = static_cast<float>(value_of(coded[c], present[c], p.code_bias, scale, offset, __ldg(steps + h + c)));
+                            }
+                        }
                     }
                 }
             }
@@ -793,7 +808,7 @@ __global__ void __launch_bounds__(kThreads, 1) qcsr_transpose_digits_kernel(cons
             for (std::int64_t u = u0; u < u1; ++run) {
                 const std::int64_t ub = u, ue = run_end(u, u1, p.group_count, p.run_groups);
                 const std::int64_t set = u / p.group_count % sets;
-                const int nwin = static_cast<int>(min(static_cast<std::int64_t>(kSet), p.windows - set * kSet));
+                const int nwin = static_cast<int>(min(static_cast<std::int64_t>(kSet), p.windows - (p.first_set + set) * kSet));
                 bar_wait(smem_addr(acc_empty), static_cast<std::uint32_t>((run & 1) ^ 1), abort_flag);
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 for (; u < ue; ++u) {
@@ -865,7 +880,7 @@ __global__ void __launch_bounds__(kThreads, 1) qcsr_transpose_digits_kernel(cons
             lo = hi = 0u;
             const std::int64_t piece = (p.group_begin + at.group) * p.group_pieces + lane;
             if (at.unit < u1 && lane < p.group_pieces && piece < p.pieces) {
-                const std::uint32_t *bound = p.bounds + piece * (p.windows + 1) + at.set * kSet + at.wl;
+                const std::uint32_t *bound = p.bounds + piece * (p.windows + 1) + (p.first_set + at.set) * kSet + at.wl;
                 lo = __ldcg(bound);
                 hi = __ldcg(bound + 1);
                 base = __ldcg(p.bases + piece) & (kTwice - 1);
@@ -944,20 +959,22 @@ struct finish_params {
     float alpha, beta;
 };
 
-// G'[genes of one window, columns of one block] = beta * G' + alpha * (the sums of the set's runs, added in run order).
+// G'[genes of one window, columns of one block] = beta * G' + alpha * (the sums of the set's runs, added in run order; EXACT: the totals).
 // Where a column's range is too wide for fixed point, or a scale or a zero-point of the window is not finite (0 * infinity, in a
-// product of sums, would reach cells that hold no entry): from the entries, in double precision.  A warp has every eighth gene
-// of the window to itself and walks the words in order, so this too has the same bits on every run.
-template<int NB, int SLICES>
-__global__ void __launch_bounds__(256) finish_kernel(const finish_params p) {
+// product of sums, would reach cells that hold no entry): from the entries, in double precision.  A warp has every eighth or
+// sixteenth gene of the window to itself and walks the words in order, so this too has the same bits on every run.
+// A thread has a gene and sixteen columns, so that a warp's loads are contiguous.
+__host__ __device__ constexpr int finish_threads(int nb) { return nb / 16 * kWin; }
+template<int NB, int SLICES, bool EXACT>
+__global__ void __launch_bounds__(finish_threads(NB)) finish_kernel(const finish_params p) {
     extern __shared__ double slow_sums[]; // [kWin][NB]
-    constexpr int kSet = set_windows(NB, SLICES);
+    constexpr int kSet = set_windows(NB, SLICES), kFinish = finish_threads(NB);
     __shared__ float2 meta[kWin];
     wait_for_previous_launch();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const std::int64_t sets = (p.d.windows + kSet - 1) / kSet;
+    const std::int64_t sets = p.d.set_count;
     const int wl = static_cast<int>(blockIdx.x % kSet);
-    const std::int64_t set = blockIdx.x / kSet, window = set * kSet + wl;
+    const std::int64_t set = blockIdx.x / kSet, window = (p.d.first_set + set) * kSet + wl;
     const int c0 = static_cast<int>(blockIdx.y) * NB;
     if (window >= p.d.windows) return;
     int odd = 0;
@@ -971,7 +988,7 @@ __global__ void __launch_bounds__(256) finish_kernel(const finish_params p) {
     const int wide = __ldcg(p.d.wide);
     const bool slow = __syncthreads_or(odd) != 0 || wide == 2;
     if (slow) {
-        for (int i = tid; i < kWin * NB; i += 256) slow_sums[i] = 0.0;
+        for (int i = tid; i < kWin * NB; i += kFinish) slow_sums[i] = 0.0;
         __syncthreads();
         const std::int64_t piece0 = (p.row_begin - p.first_row) / p.d.piece_rows, piece1 = (p.row_end - p.first_row + p.d.piece_rows - 1) / p.d.piece_rows;
         for (std::int64_t piece = piece0; piece < piece1; ++piece) {
@@ -984,7 +1001,7 @@ __global__ void __launch_bounds__(256) finish_kernel(const finish_params p) {
                 const int place = static_cast<int>((e >> 8) & 0x7fffu), gl = (place >> 7) & (kWin - 1);
                 const int cell = (place >> 14) * 128 + ((((place >> 4) & 7) ^ (gl & 7)) << 4) + (place & 15);
                 const std::int64_t row = group_row + cell;
-                std::uint32_t todo = __ballot_sync(0xffffffffu, static_cast<int>(e) >= 0 && (gl & 7) == warp && row >= p.row_begin && row < p.row_end);
+                std::uint32_t todo = __ballot_sync(0xffffffffu, static_cast<int>(e) >= 0 && gl % (kFinish / 32) == warp && row >= p.row_begin && row < p.row_end);
                 while (todo != 0u) {
                     const int j = __ffs(todo) - 1;
                     todo &= todo - 1u;
@@ -1003,50 +1020,76 @@ __global__ void __launch_bounds__(256) finish_kernel(const finish_params p) {
     // the set's slots: the CTAs whose shares meet its runs, run after run, pass after pass
     const int passes = wide == 1 ? 2 : 1;
     const std::int64_t total = sets * p.d.column_blocks * p.d.group_count * passes, L = p.d.group_count, cuts = (L + p.d.run_groups - 1) / p.d.run_groups;
-    constexpr int kItems = kWin * (NB / 4) / 256; // of a thread
-    float4 sums[kItems];
+    const int gl = tid & (kWin - 1);
+    const std::int64_t gene = window * kWin + gl;
+    const int c = tid / kWin * 16;
+    if (gene >= p.d.cols || c0 + c >= p.n) return;
+    float v[16];
+    if (slow) {
 #pragma unroll
-    for (int k = 0; k < kItems; ++k) sums[k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    for (int pass = 0; pass < passes && !slow; ++pass) {
-        const std::int64_t set_of_all = (static_cast<std::int64_t>(pass) * p.d.column_blocks + blockIdx.y) * sets + set;
-        for (std::int64_t cut = 0; cut < cuts; ++cut) {
-            const std::int64_t from = set_of_all * L + cut * p.d.run_groups, to = min(from + p.d.run_groups, (set_of_all + 1) * L);
-            const std::int64_t last = cta_of(to - 1, total, p.grid);
-            for (std::int64_t b = cta_of(from, total, p.grid); b <= last; ++b) {
-                const float4 *slot = reinterpret_cast<const float4 *>(p.d.partials + ((set_of_all * cuts + cut + b) * kSet + wl) * kWin * NB) + tid;
-                float4 v[kItems];
+        for (int k = 0; k < 16; ++k) v[k] = static_cast<float>(slow_sums[gl * NB + c + k]);
+    } else if constexpr (EXACT) {
+        const double scale = static_cast<double>(meta[gl].x), offset = static_cast<double>(meta[gl].y);
+        double sum[16];
 #pragma unroll
-                for (int k = 0; k < kItems; ++k) v[k] = __ldcg(slot + k * 256);
+        for (int k = 0; k < 16; ++k) sum[k] = 0.0;
+        for (int pass = 0; pass < passes; ++pass) {
+            const std::int64_t block = static_cast<std::int64_t>(pass) * p.d.column_blocks + blockIdx.y;
+            const long long *total = p.d.totals + (((block * sets + set) * kSet + wl) * 2 * NB + c) * kWin + gl;
+            const double *steps = p.d.steps + block * NB + c;
+            long long coded[16], present[16];
 #pragma unroll
-                for (int k = 0; k < kItems; ++k) { sums[k].x += v[k].x; sums[k].y += v[k].y; sums[k].z += v[k].z; sums[k].w += v[k].w; }
+            for (int k = 0; k < 16; ++k) {
+                coded[k] = __ldcg(total + k * kWin);
+                present[k] = __ldcg(total + (NB + k) * kWin);
+            }
+#pragma unroll
+            for (int k = 0; k < 16; ++k) sum[k] += value_of(coded[k], present[k], p.d.code_bias, scale, offset, __ldg(steps + k));
+        }
+#pragma unroll
+        for (int k = 0; k < 16; ++k) v[k] = static_cast<float>(sum[k]);
+    } else {
+#pragma unroll
+        for (int k = 0; k < 16; ++k) v[k] = 0.0f;
+        for (int pass = 0; pass < passes; ++pass) {
+            const std::int64_t set_of_all = (static_cast<std::int64_t>(pass) * p.d.column_blocks + blockIdx.y) * sets + set;
+            for (std::int64_t cut = 0; cut < cuts; ++cut) {
+                const std::int64_t from = set_of_all * L + cut * p.d.run_groups, to = min(from + p.d.run_groups, (set_of_all + 1) * L);
+                const std::int64_t last = cta_of(to - 1, total, p.grid);
+                for (std::int64_t b = cta_of(from, total, p.grid); b <= last; ++b) {
+                    const float *slot = p.d.partials + (((set_of_all * cuts + cut + b) * kSet + wl) * NB + c) * kWin + gl;
+                    float u[16];
+#pragma unroll
+                    for (int k = 0; k < 16; ++k) u[k] = __ldcg(slot + k * kWin);
+#pragma unroll
+                    for (int k = 0; k < 16; ++k) v[k] += u[k];
+                }
             }
         }
     }
+    float *dst = p.out + gene * p.out_ld + c0 + c;
+    if (p.out_vector != 0) {
 #pragma unroll
-    for (int k = 0; k < kItems; ++k) {
-        const int i = tid + k * 256, gl = i / (NB / 4), c = i % (NB / 4) * 4;
-        const std::int64_t gene = window * kWin + gl;
-        if (gene >= p.d.cols || c0 + c >= p.n) continue;
-        float4 sum = sums[k];
-        if (slow) {
-            const double *s = slow_sums + gl * NB + c;
-            sum = make_float4(static_cast<float>(s[0]), static_cast<float>(s[1]), static_cast<float>(s[2]), static_cast<float>(s[3]));
-        }
-        float *dst = p.out + gene * p.out_ld + c0 + c;
-        const float v[4] = {sum.x, sum.y, sum.z, sum.w};
-        if (p.out_vector != 0) {
+        for (int k = 0; k < 16; k += 4) {
+            if (c0 + c + k >= p.n) break;
             float4 o = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             if (p.beta != 0.0f) {
-                o = *reinterpret_cast<const float4 *>(dst);
+                o = *reinterpret_cast<const float4 *>(dst + k);
                 o.x *= p.beta; o.y *= p.beta; o.z *= p.beta; o.w *= p.beta;
             }
-            *reinterpret_cast<float4 *>(dst) = make_float4(fmaf(p.alpha, v[0], o.x), fmaf(p.alpha, v[1], o.y), fmaf(p.alpha, v[2], o.z), fmaf(p.alpha, v[3], o.w));
-        } else {
-            for (int j = 0; j < 4 && c0 + c + j < p.n; ++j) dst[j] = fmaf(p.alpha, v[j], p.beta == 0.0f ? 0.0f : p.beta * dst[j]);
+            *reinterpret_cast<float4 *>(dst + k) =
+                make_float4(fmaf(p.alpha, v[k], o.x), fmaf(p.alpha, v[k + 1], o.y), fmaf(p.alpha, v[k + 2], o.z), fmaf(p.alpha, v[k + 3], o.w));
         }
+    } else {
+#pragma unroll
+        for (int k = 0; k < 16; ++k)
+            if (c0 + c + k < p.n) dst[k] = fmaf(p.alpha, v[k], p.beta == 0.0f ? 0.0f : p.beta * dst[k]);
     }
 }
 
+// Digits of a repeatable launch, and the groups and sets of windows a launch with the least workspace takes at a time.
+constexpr int kExactSlices = 4;
+constexpr std::int64_t kLeastGroups = 2, kLeastSets = 4;
 int column_block(std::int64_t n) { return n <= 32 ? 32 : 64; }
 int padded_columns(std::int64_t n) { return n <= 32 ? 32 : n <= 64 ? 64 : n <= 128 ? 128 : 256; }
 
@@ -1065,6 +1108,18 @@ std::uint64_t partial_bytes(std::int64_t groups, std::int64_t cols, std::int64_t
 std::uint64_t launch_bytes(std::int64_t groups, std::int64_t cols, std::int64_t n, int slices, int ctas) {
     return kRecordsAt + record_bytes(groups, n, slices) + partial_bytes(groups, cols, n, slices, ctas);
 }
+// ... and a repeatable one over `sets` sets of windows at a time
+std::int64_t set_count_of(std::int64_t cols, std::int64_t n) {
+    const std::int64_t per_set = set_windows(column_block(n), kExactSlices), windows = (cols + kWin - 1) / kWin;
+    return (windows + per_set - 1) / per_set;
+}
+std::uint64_t total_bytes(std::int64_t sets, std::int64_t n) { // of one pass
+    const std::int64_t nb = column_block(n);
+    return static_cast<std::uint64_t>(sets * ((n + nb - 1) / nb) * set_windows(static_cast<int>(nb), kExactSlices) * kWin * nb) * 16u;
+}
+std::uint64_t exact_bytes(std::int64_t groups, std::int64_t sets, std::int64_t n) {
+    return kRecordsAt + record_bytes(groups, n, kExactSlices) + 2u * total_bytes(sets, n);
+}
 std::int64_t group_count_of(std::int64_t rows) { return (rows + kRows - 1) / kRows; }
 std::int64_t piece_count(std::int64_t rows) { return (rows + piece_rows_of(rows) - 1) / piece_rows_of(rows); }
 std::uint64_t word_bytes(std::int64_t rows, std::int64_t cols, std::int64_t nnz) {
@@ -1081,6 +1136,7 @@ struct digit_launch {
     digit_params main;       // group_begin, group_count: of the whole row range
     finish_params finish;
     std::int64_t slice;      // groups at a time
+    std::int64_t chunk;      // EXACT: sets of windows at a time
     unsigned *part_max;
     ulonglong2 *part_sum;
     double *steps;
@@ -1089,40 +1145,60 @@ struct digit_launch {
     bool early; // the launch in front is a kernel of this call
 };
 
-template<int NB, int SLICES>
+// Slice after slice of the groups: the runs' sums are rounded and a slice's are added to G'.  EXACT (a request that has to be
+// repeatable): chunk after chunk of the windows and slice after slice of the groups, whose sums meet as whole numbers, so that neither the
+// grid nor the room for slices and chunks changes a bit.
+template<int NB, int SLICES, bool EXACT>
 cb200_status launch_digits(const digit_launch &l, int sm_count, cudaStream_t stream) {
     constexpr std::size_t smem = digits_smem_bytes<NB, SLICES>();
     static_assert(smem <= 232448, "shared memory budget");
-    constexpr int slow_smem = kWin * NB * 8;
-    CB200_CUDA_OK(cudaFuncSetAttribute(qcsr_transpose_digits_kernel<NB, SLICES>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-    CB200_CUDA_OK(cudaFuncSetAttribute(finish_kernel<NB, SLICES>, cudaFuncAttributeMaxDynamicSharedMemorySize, slow_smem));
+    constexpr int slow_smem = kWin * NB * 8, kSet = set_windows(NB, SLICES);
+    const auto main_kernel = qcsr_transpose_digits_kernel<NB, SLICES, EXACT>;
+    const auto finish = finish_kernel<NB, SLICES, EXACT>;
+    CB200_CUDA_OK(cudaFuncSetAttribute(main_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+    CB200_CUDA_OK(cudaFuncSetAttribute(finish, cudaFuncAttributeMaxDynamicSharedMemorySize, slow_smem));
     const int n = l.finish.n, padded = padded_columns(n);
     CB200_CUDA_OK(launch_kernel(l.early, column_range_kernel, dim3(kParts), 1024, 0, stream, l.finish.g, l.finish.g_ld, n, padded, l.finish.row_begin, l.finish.row_end,
                                 l.part_max, l.part_sum, l.early ? nullptr : l.main.status));
-    const std::int64_t group_end = l.main.group_begin + l.main.group_count;
-    for (std::int64_t begin = l.main.group_begin; begin < group_end; begin += l.slice) {
+    count_launch();
+    const std::int64_t group_end = l.main.group_begin + l.main.group_count, sets = (l.main.windows + kSet - 1) / kSet;
+    const std::int64_t chunk = EXACT ? l.chunk : sets;
+    for (std::int64_t first_set = 0; first_set < sets; first_set += chunk) {
         digit_params m = l.main;
         finish_params f = l.finish;
-        m.group_begin = begin;
-        m.group_count = std::min(l.slice, group_end - begin);
-        m.partials = reinterpret_cast<float *>(l.records + record_bytes(m.group_count, n, SLICES));
-        const std::int64_t row0 = f.first_row + begin * kRows, blocks = m.group_count * m.column_blocks;
-        CB200_CUDA_OK(launch_kernel(true, pack_digits_kernel<NB, SLICES>, dim3(static_cast<unsigned>(std::min<std::int64_t>(blocks * kGPieces, 4 * sm_count))), 256, 0, stream, f.g,
-                                    f.g_ld, n, padded, row0, f.row_begin, f.row_end, m.group_count, l.part_max, l.part_sum, l.steps, l.records, m.bases, m.pieces,
-                                    l.wide));
-        const std::int64_t sets = (m.windows + set_windows(NB, SLICES) - 1) / set_windows(NB, SLICES);
-        const unsigned grid = static_cast<unsigned>(std::min<std::int64_t>(sets * blocks, sm_count));
-        CB200_CUDA_OK(launch_kernel(true, qcsr_transpose_digits_kernel<NB, SLICES>, dim3(grid), kThreads, smem, stream, m));
-        f.d = m;
-        f.grid = grid;
-        f.row_begin = std::max(f.row_begin, row0);
-        f.row_end = std::min(f.row_end, row0 + m.group_count * kRows);
-        if (begin != l.main.group_begin) f.beta = 1.0f;
-        CB200_CUDA_OK(launch_kernel(true, finish_kernel<NB, SLICES>, dim3(static_cast<unsigned>(sets * set_windows(NB, SLICES)), static_cast<unsigned>(m.column_blocks)), 256,
-                                    slow_smem, stream, f));
-        count_launch(3);
+        m.first_set = first_set;
+        m.set_count = std::min(chunk, sets - first_set);
+        bool clear = true;
+        const auto finish_groups = [&](std::int64_t grid) {
+            f.d = m;
+            f.grid = grid;
+            count_launch();
+            return launch_kernel(true, finish, dim3(static_cast<unsigned>(m.set_count * kSet), static_cast<unsigned>(m.column_blocks)), finish_threads(NB), slow_smem, stream, f);
+        };
+        for (std::int64_t begin = l.main.group_begin; begin < group_end; begin += l.slice) {
+            m.group_begin = begin;
+            m.group_count = std::min(l.slice, group_end - begin);
+            unsigned char *sums = l.records + record_bytes(m.group_count, n, SLICES);
+            if (EXACT) sums = l.records + record_bytes(l.slice, n, SLICES); // the same place for all slices
+            m.partials = EXACT ? nullptr : reinterpret_cast<float *>(sums);
+            m.totals = EXACT ? reinterpret_cast<long long *>(sums) : nullptr;
+            const std::int64_t row0 = l.finish.first_row + begin * kRows, blocks = m.group_count * m.column_blocks;
+            const std::int64_t to_clear = EXACT && clear ? static_cast<std::int64_t>(total_bytes(m.set_count, n) / 16u) : 0;
+            CB200_CUDA_OK(launch_kernel(true, pack_digits_kernel<NB, SLICES>, dim3(static_cast<unsigned>(std::min<std::int64_t>(blocks * kGPieces, 4 * sm_count))), 256, 0, stream,
+                                        f.g, f.g_ld, n, padded, row0, l.finish.row_begin, l.finish.row_end, m.group_count, l.part_max, l.part_sum, l.steps, l.records, m.bases,
+                                        m.pieces, l.wide, reinterpret_cast<uint4 *>(m.totals), to_clear));
+            clear = false;
+            const unsigned grid = static_cast<unsigned>(std::min<std::int64_t>(m.set_count * blocks, sm_count));
+            CB200_CUDA_OK(launch_kernel(true, main_kernel, dim3(grid), kThreads, smem, stream, m));
+            count_launch(2);
+            if (EXACT) continue;
+            f.row_begin = std::max(l.finish.row_begin, row0);
+            f.row_end = std::min(l.finish.row_end, row0 + m.group_count * kRows);
+            f.beta = begin != l.main.group_begin ? 1.0f : l.finish.beta;
+            CB200_CUDA_OK(finish_groups(grid));
+        }
+        if (EXACT) CB200_CUDA_OK(finish_groups(0));
     }
-    count_launch();
     CB200_CUDA_OK(cudaGetLastError());
     return CB200_STATUS_SUCCESS;
 }
@@ -1169,11 +1245,14 @@ digit_layout digit_words_at(void *memory, const qcsr_view &x) {
     l.bases = reinterpret_cast<std::int64_t *>(at);
     return l;
 }
-std::uint64_t qcsr_transpose_digits_workspace_bytes(std::int64_t rows, std::int64_t cols, std::int64_t n, int slices) {
+std::uint64_t qcsr_transpose_digits_workspace_bytes(std::int64_t rows, std::int64_t cols, std::int64_t n, int slices, bool repeatable) {
+    if (repeatable) return exact_bytes(group_count_of(rows), set_count_of(cols, n), n);
     return launch_bytes(group_count_of(rows), cols, n, slices, kMaxCtas);
 }
-std::uint64_t qcsr_transpose_digits_least_workspace(std::int64_t rows, std::int64_t cols, std::int64_t n, int slices, int sm_count) {
-    return launch_bytes(std::min<std::int64_t>(group_count_of(rows), 16), cols, n, slices, std::min(sm_count, kMaxCtas));
+std::uint64_t qcsr_transpose_digits_least_workspace(std::int64_t rows, std::int64_t cols, std::int64_t n, int slices, bool repeatable, int sm_count) {
+    const std::int64_t groups = group_count_of(rows);
+    if (repeatable) return exact_bytes(std::min<std::int64_t>(groups, kLeastGroups), std::min<std::int64_t>(set_count_of(cols, n), kLeastSets), n);
+    return launch_bytes(std::min<std::int64_t>(groups, 16), cols, n, slices, std::min(sm_count, kMaxCtas));
 }
 std::uint64_t qcsr_transpose_digits_once_bytes(std::int64_t rows, std::int64_t cols, std::int64_t n, std::int64_t nnz, int bits, int policy) {
     if (!qcsr_transpose_digits_shape_ok(rows, cols, n, bits, policy)) return 0u;
@@ -1181,7 +1260,7 @@ std::uint64_t qcsr_transpose_digits_once_bytes(std::int64_t rows, std::int64_t c
     // 64: 2,000 x 8,000 (1.6 M entries) 48 us against 45, 1,500 x 33,538 (2.7 M) 75 against 75, 4,000 x 4,000 (2.1 M) 49 against 57,
     // 8,191 x 33,538 (14.7 M) 171 against 318; at N = 32 8,000 x 2,000 (2.9 M) 51 against 53, 16,384 x 2,000 (5.9 M) 74 against 108.
     if (static_cast<double>(nnz) < 0.02 * static_cast<double>(rows) * static_cast<double>(cols) || nnz < kLeastOnceEntries || nnz > kMostOnceEntries) return 0u;
-    return qcsr_transpose_digits_workspace_bytes(rows, cols, n, 4) + qcsr_digit_words_bytes_bound(rows, cols, nnz);
+    return qcsr_transpose_digits_workspace_bytes(rows, cols, n, 4, false) + qcsr_digit_words_bytes_bound(rows, cols, nnz);
 }
 
 cb200_status build_digit_words(const qcsr_view &x, device_arena &arena, cudaStream_t stream, digit_layout *out) {
@@ -1214,20 +1293,22 @@ cb200_status build_digit_words(const qcsr_view &x, device_arena &arena, cudaStre
 }
 
 cb200_status launch_qcsr_transpose_digits(const qcsr_view &x, const dense_args &d, std::int64_t row_begin, std::int64_t row_end, void *workspace,
-                                          std::uint64_t workspace_bytes, const digit_layout *layout, int slices, int sm_count, cudaStream_t stream, bool *taken) {
+                                          std::uint64_t workspace_bytes, const digit_layout *layout, int slices, bool repeatable, int sm_count, cudaStream_t stream, bool *taken) {
     *taken = false;
     if (row_end <= row_begin || d.dense_dtype != CB200_DTYPE_F32 || !qcsr_transpose_digits_shape_ok(x.rows, x.cols, d.n, x.bits, x.policy)) return CB200_STATUS_SUCCESS;
     if (workspace == nullptr || reinterpret_cast<std::uintptr_t>(workspace) % 256u != 0u || sm_count > kMaxCtas) return CB200_STATUS_SUCCESS;
     if (x.bits == 4 && x.packed_row_ptr == nullptr) return CB200_STATUS_SUCCESS;
     // With less workspace than for the whole range the groups are taken in slices.  A call that has to make its words has room for
     // everything or is another kernel's.
-    const std::uint64_t own = qcsr_transpose_digits_workspace_bytes(x.rows, x.cols, d.n, slices);
+    const std::uint64_t own = qcsr_transpose_digits_workspace_bytes(x.rows, x.cols, d.n, slices, false);
     if (layout == nullptr && workspace_bytes < own + qcsr_digit_words_bytes_bound(x.rows, x.cols, x.nnz)) return CB200_STATUS_SUCCESS;
     const std::int64_t first_row = layout != nullptr ? 0 : row_begin, rows_of_words = layout != nullptr ? x.rows : row_end - row_begin;
     const std::int64_t group_begin = (row_begin - first_row) / kRows, group_count = (row_end - first_row + kRows - 1) / kRows - group_begin;
-    std::int64_t slice = group_count;
-    while (slice > 1 && launch_bytes(slice, x.cols, d.n, slices, sm_count) > workspace_bytes) slice = (slice + 1) / 2;
-    if (launch_bytes(slice, x.cols, d.n, slices, sm_count) > workspace_bytes) return CB200_STATUS_SUCCESS;
+    std::int64_t slice = group_count, chunk = repeatable ? set_count_of(x.cols, d.n) : 0;
+    const auto needs = [&](std::int64_t groups) { return repeatable ? exact_bytes(groups, chunk, d.n) : launch_bytes(groups, x.cols, d.n, slices, sm_count); };
+    while (chunk > 1 && needs(std::min<std::int64_t>(slice, kLeastGroups)) > workspace_bytes) chunk = (chunk + 1) / 2;
+    while (slice > 1 && needs(slice) > workspace_bytes) slice = (slice + 1) / 2;
+    if (needs(slice) > workspace_bytes) return CB200_STATUS_SUCCESS;
     if (layout != nullptr && (x.row_ptr != layout->src_row_ptr || x.col_idx != layout->src_col_idx || x.packed != layout->src_packed))
         return fail(CB200_STATUS_STALE_STRUCTURE, "the launch's matrix is not the one the entry words were built from");
     *taken = true;
@@ -1242,6 +1323,7 @@ cb200_status launch_qcsr_transpose_digits(const qcsr_view &x, const dense_args &
     digit_params &p = l.main;
     p.status = reinterpret_cast<int *>(ws);
     l.slice = slice;
+    l.chunk = chunk;
     if (layout != nullptr) {
         p.words = layout->words; p.bounds = layout->bounds; p.bases = layout->bases;
     } else {
@@ -1270,8 +1352,9 @@ cb200_status launch_qcsr_transpose_digits(const qcsr_view &x, const dense_args &
     f.out = d.out; f.out_ld = d.out_ld; f.n = static_cast<int>(d.n);
     f.out_vector = reinterpret_cast<std::uintptr_t>(d.out) % 16u == 0u && d.out_ld % 4 == 0 && d.n % 4 == 0 ? 1 : 0;
     f.alpha = d.alpha; f.beta = d.beta;
-    if (slices == 4) return nb == 64 ? launch_digits<64, 4>(l, sm_count, stream) : launch_digits<32, 4>(l, sm_count, stream);
-    return nb == 64 ? launch_digits<64, 3>(l, sm_count, stream) : launch_digits<32, 3>(l, sm_count, stream);
+    if (repeatable) return nb == 64 ? launch_digits<64, kExactSlices, true>(l, sm_count, stream) : launch_digits<32, kExactSlices, true>(l, sm_count, stream);
+    if (slices == 4) return nb == 64 ? launch_digits<64, 4, false>(l, sm_count, stream) : launch_digits<32, 4, false>(l, sm_count, stream);
+    return nb == 64 ? launch_digits<64, 3, false>(l, sm_count, stream) : launch_digits<32, 3, false>(l, sm_count, stream);
 }
 
 } // namespace cb200

@@ -328,7 +328,9 @@ cb200_status cb200_spmm_persistent_requirement(const cb200_spmm_problem *problem
 void cb200_prepared_destroy(cb200_prepared *prepared);
 /* workspace_requirement, launch_bindings.hh:67-71: what the schedule can use.  "vector_reductions" reports up to 32 MB (it
  * sorts the entries with it, slice of rows by slice), or for 2 to 50 million entries about 4 bytes an entry (words for integer
- * sums), and also runs with less or with none, slower.  "warp_per_row" (unaligned
+ * sums), and also runs with less or with none, slower.  A deterministic transpose with integer sums reports 8 N bytes a cell
+ * and 32 N a gene (N up to 32 or to a multiple of 64) and also runs with less, slower and with the same bits, down to 512 of these cells and
+ * 512 of these genes (N <= 32: 1,024) and 256 KB; less is refused.  "warp_per_row" (unaligned
  * N) and the tensor_blocked and tensor_dense forward schedules also run with less, down to the status block and the records of
  * W, slower and with the same bits: a row's sum follows from its entries, N and W's type, not from the room, the launch's row
  * range or the rows beside it. */

@@ -175,3 +175,30 @@ def test_bounded_wait_path(cuda_device, oracle):
     assert e.value.status == capi.DEVICE_WAIT_TIMEOUT
     assert torch.equal(op.run(x, g, torch.full((cols, n), float("nan"), device=cuda_device)), good) and op.status() == 0
     op.close()
+
+
+@pytest.mark.parametrize("n,bits,outlier", [(64, 8, 1.0), (32, 4, 1.0), (128, 8, 1e6)])
+def test_repeatable_bits_do_not_follow_from_the_workspace(cuda_device, oracle, n, bits, outlier):
+    """Row groups in slices, windows in chunks, one pass of digits and two: whatever the room is, down to the least that is accepted."""
+    rng = np.random.default_rng(n)
+    rows, cols = 256 * 22 + 7, 128 * 37 - 5
+    x = to_dev(host_pack(oracle, random_csr(rng, rows=rows, cols=cols, max_nnz=400, bits=bits)), cuda_device)
+    g, _ = dense(rng, rows, n, torch.float32, cuda_device, std=1.0)
+    g[77, 5] *= outlier
+    op = prepared(x, n, 4, cuda_device)
+    room = op.workspace_bytes
+    for lo, hi in ((0, rows), (100, rows - 300)):
+        op.workspace_bytes = room
+        want, refused, accepted = op.run(x, g, torch.empty(cols, n, device=cuda_device), row_begin=lo, row_end=hi).clone(), 0, []
+        for part in (0.99, 0.75, 0.5, 0.35, 0.25, 0.18, 0.12, 0.08, 0.05, 0.02):
+            op.workspace_bytes = int(room * part)
+            try:
+                got = op.run(x, g, torch.full((cols, n), float("nan"), device=cuda_device), row_begin=lo, row_end=hi)
+            except capi.Cb200Error as e:
+                assert e.status == capi.INSUFFICIENT_WORKSPACE
+                refused += 1
+                continue
+            assert refused == 0 and op.status() == 0 and torch.equal(got, want), part
+            accepted.append(part)
+        assert refused > 0 and min(accepted) < 0.75
+    op.close()
