@@ -385,7 +385,7 @@ schedule_plan plan_schedule(const cb200_spmm_problem &pr) {
         // inside the 1e-4 bound of an fp32 G.  The cost follows the dense area, so it needs density.
         // Same bits on every run: both give that (integer sums have no order, and every CTA's sums go to a slot of their own and
         // are added in a fixed order), and a deterministic request that names them gets them.  Otherwise such a request is served
-        // under the name "gene_gather": with four digits of G, which are more exact than fp32 sums, where a tile of 256 x 128
+        // under the name "gene_gather": with four digits of G (as many as keep the precision of fp32 products, for every cell's G: qcsr_transpose_digits.cu), where a tile of 256 x 128
         // holds 600 entries or more (every one of them pays for its tile; 2 %) and there are tiles for every SM (256 of them; 5,000
         // x 2,000, 320 tiles: 37 us against 42 gathered at N = 32, 38 against 49 at 64); by the gather gene by gene from a gene-major copy, whose fp32
         // sums the oracle restates entry by entry, below that, with zero-points per row, and where it is asked for by name.
@@ -567,8 +567,8 @@ cb200_status cb200_spmm_prepare(const cb200_spmm_problem *problem, cb200_prepare
             if (st != CB200_STATUS_SUCCESS) return abandon(st);
             p->digit_slices = plan.digits;
             p->schedule_name = plan.digits == 4 ? "gene_gather" : "tensor_blocked_x3";
-            p->workspace_bytes = qcsr_transpose_digits_workspace_bytes(problem->m, problem->k, problem->n, plan.digits, plan.digits == 4);
-            p->workspace_required = qcsr_transpose_digits_least_workspace(problem->m, problem->k, problem->n, plan.digits, plan.digits == 4, p->sm_count);
+            p->workspace_bytes = qcsr_transpose_digits_workspace_bytes(problem->m, problem->k, problem->n, plan.digits == 4);
+            p->workspace_required = qcsr_transpose_digits_least_workspace(problem->m, problem->k, problem->n, plan.digits == 4, p->sm_count);
             p->persistent_bytes += p->digits.bytes;
         }
         if (plan.gene_gather) {

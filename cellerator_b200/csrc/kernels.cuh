@@ -223,8 +223,8 @@ cb200_status build_digit_words(const qcsr_view &x, device_arena &arena, cudaStre
 digit_layout digit_words_at(void *memory, const qcsr_view &x);
 cb200_status launch_digit_words(const qcsr_view &x, std::int64_t row_begin, std::int64_t row_end, std::uint32_t *words, std::uint32_t *bounds,
                                 std::int64_t *bases, int *status, cudaStream_t stream);
-std::uint64_t qcsr_transpose_digits_workspace_bytes(std::int64_t rows, std::int64_t cols, std::int64_t n, int slices, bool repeatable);
-std::uint64_t qcsr_transpose_digits_least_workspace(std::int64_t rows, std::int64_t cols, std::int64_t n, int slices, bool repeatable, int sm_count); // slower
+std::uint64_t qcsr_transpose_digits_workspace_bytes(std::int64_t rows, std::int64_t cols, std::int64_t n, bool repeatable);
+std::uint64_t qcsr_transpose_digits_least_workspace(std::int64_t rows, std::int64_t cols, std::int64_t n, bool repeatable, int sm_count); // slower
 // Whether a call that sees its matrix once should make the words in its workspace (0: no), and what it then needs
 std::uint64_t qcsr_transpose_digits_once_bytes(std::int64_t rows, std::int64_t cols, std::int64_t n, std::int64_t nnz, int bits, int policy);
 // layout null: the words are made in the workspace.  *taken is false where the shape or the workspace rules it out.

@@ -13,13 +13,13 @@
 // of G to its fixed point and a handful of fp32 roundings at the end: of each run, and of the sum of a set's runs, of which there are as many as
 // CTAs share the set.  A request that has to be repeatable (EXACT) adds the runs up as whole numbers instead, 64 bits in L2, and rounds once:
 // its bits follow from the operands and the row range alone, not from the number of SMs nor from the workspace, whose lack
-// only cuts the launch into slices of groups and chunks of windows (100,003 x 33,538, N = 64: 1,099 us, with rounded runs 1,093).  Against 64 bits (2-norm, genes of the 33,538-gene
-// matrices): S = 4 4e-8, where fp32 FMAs leave 1.2e-7 (8,191 cells) to 4.8e-7 (100,003 cells, in a fixed order); S = 3 2e-7, where
-// products put together from three bf16 products and summed by the fp32 MMAs leave 6.2e-6.
+// only cuts the launch into slices of groups and chunks of windows (100,003 x 33,538, N = 64: 1,099 us, with rounded runs 1,093).  Against
+// 64 bits (2-norm, normal G, genes of the 33,538-gene matrices): S = 4 4e-8, where fp32 FMAs leave 1.2e-7 (8,191 cells) to 4.8e-7 (100,003
+// cells, in a fixed order); S = 3 3e-7, where products put together from three bf16 products and summed by the fp32 MMAs leave 6.2e-6.
 //
-// Where the numbers of a column are small beside its largest (kMostSpread), the launch takes as many digits again, those behind the
-// first ones, in a second pass over the tiles: 62 bits (S = 4) or 46.  A column that spreads further, or holds an infinity or a NaN,
-// and a matrix in which a cell holds a gene twice, are taken entry by entry, in double precision and in a fixed order
+// Where G spreads too far for that (most_spread), the launch takes as many digits again, those behind the first ones, in a second pass over
+// the tiles: 62 bits (S = 4) or 46; where three digits are asked for, four in one pass come first.  A G that spreads further still, or holds
+// an infinity or a NaN, and a matrix in which a cell holds a gene twice, are taken entry by entry, in double precision and in a fixed order
 // (finish_kernel).  The device decides; nothing is read back.
 //
 // Data.  The entries lie in pieces of 32 cells; inside a piece they are ordered by window of 128 genes, one word per entry
@@ -37,7 +37,8 @@
 // the scatter groups' chain (release, zeroes, two one-byte stores a word, fence, hand-over), 2,125 cycles against 1,536 of MMAs; over a
 // second of launches the power cap (1.6 GHz).  One B200, start of this kernel's life -> now: 125,000 x 33,538, N = 64, S = 3 1,645 (bf16
 // products) -> 1,186 us; 100,003 cells, S = 4 2,879 (rows of G gathered gene by gene) -> 1,087; 8,191 cells, S = 4 with the words made in
-// the call 313 (sorted in shared memory) -> 171.
+// the call 313 (sorted in shared memory) -> 171.  With one row of G at 1e6: 1,511 -> 2,090, 2,641 -> 1,970, 313 -> 258; Student-t numbers with
+// three degrees of freedom (four digits in one pass instead of three in two, 2,014 us): 125,000 cells, S = 3 1,204.
 #include "dependent_launch.cuh"
 #include "kernels.cuh"
 #include "sm100_primitives.cuh"
@@ -80,16 +81,35 @@ __host__ __device__ constexpr int set_windows(int nb, int slices) { return 512 /
 __host__ __device__ constexpr int g_piece_bytes(int nb, int slices) { return kGPieceRows * mma_columns(nb, slices); }
 __host__ __device__ constexpr int ring_pieces(int nb, int slices) { return mma_columns(nb, slices) >= 256 ? 5 : mma_columns(nb, slices) >= 192 ? 6 : 8; }
 
-// workspace: status block {status, passes, ...}, largest magnitudes and sums of the exponents of the columns in parts, steps of the
-// columns, G in digits, sums of the runs, and for a call that sees its matrix once the words
+// workspace: status block {status, mode, ...}, steps of the columns, what is known of G's columns in parts (largest magnitudes; sums of
+// 1 / sqrt(magnitude) and numbers; smallest row maxima), G in digits, sums of the runs or totals, and for a call that sees its matrix
+// once the words
 constexpr int kParts = 48;
 constexpr int kMaxColumns = 256;
-// One pass serves a column if its numbers are on average (of the binary exponents of those that are not zero, which a few
-// large ones do not move) not more than 2^6 below the largest: half a step is then at most 2^-24 of the average number, what fp32
-// rounds a product at, while a normal distribution leaves 2^-27 (S = 4; S = 3: 2^-16 and 2^-19).
-constexpr unsigned kMostSpread = 6;
+constexpr int kBlockColumns = 16; // columns whose largest number stands for a cell's
+// How far G may spread, in binary orders, for a launch of `slices` digits and `passes`: the numbers are rounded at half a step, 2^-(8 slices - 1) to
+// 2^-(8 slices) of their column's largest, which has to stay below what the products of the kernel this one replaces were rounded
+// at: 2^-24 (fp32; a base of 4 digits) or 2.8e-6, root mean square, of a product put together from bf16 pieces (a base of 3).
+//
+// The spread is the larger of two numbers.  (1) A cell's largest number of sixteen neighbouring columns, against the largest of these columns:
+// the smallest of them over all cells and columns.  A gene that only such cells hold has its result in these columns to the precision of
+// fp32 products.  An average over a column does not see them where they are few: 10 % of the cells at 2^-20 move the average exponent by 2.
+// (2) For a column by itself, where a cell's others are large: the square of the mean of sqrt(largest / number), halved; numbers at 2^-s of the
+// largest raise it from 2^(2 log2 of their share + s) on.  Normal numbers have 3 and 3 (100,000 cells).  20,000 cells, a gene held by 800 cells at 2^-k alone,
+// error against 64 bits of 32-bit FMAs or hi / lo products -> this (one pass whatever the spread): k = 7, S = 4 2.5e-8 -> 1e-9 (6e-9);
+// k = 20, S = 4 3e-8 -> 1e-9 (4e-5); k = 4, S = 3 2.3e-7 -> 2e-9 (2e-7); k = 20, S = 3 2.3e-7 -> 1e-8 (1e-2).
+__host__ __device__ constexpr int most_spread(int base, int slices, int passes) {
+    return 8 * slices - (base == 4 ? 24 : 19) + (passes == 2 ? 8 * slices - 1 : 0);
+}
+// The launch's mode, a word in the workspace that its first kernels write: digits, passes over the tiles, or entry by entry.
+constexpr int kByEntry = 1 << 8;
+__host__ __device__ constexpr int mode_of(int slices, int passes) { return slices << 4 | passes; }
+__host__ __device__ constexpr int slices_of(int mode) { return mode >> 4 & 15; }
+__host__ __device__ constexpr int passes_of(int mode) { return mode & 15; }
+constexpr int kMostSlices = 4;
+
 constexpr std::uint64_t kStepsAt = 256, kPartMaxAt = kStepsAt + 2 * kMaxColumns * 8, kPartSumAt = kPartMaxAt + kParts * kMaxColumns * 4,
-                        kRecordsAt = kPartSumAt + kParts * kMaxColumns * 16;
+                        kPartLeastAt = kPartSumAt + kParts * kMaxColumns * 16, kRecordsAt = kPartLeastAt + kParts * (kMaxColumns / kBlockColumns) * 4;
 static_assert(kParts % 48 == 0, "six at a time on up to eight lanes");
 static_assert(kRecordsAt % 256 == 0, "G's records are copied 16 bytes at a time");
 
@@ -382,48 +402,78 @@ __global__ void __launch_bounds__(kBuildThreads, 2) digit_words_kernel(const wor
 
 // ---- G in digits -----------------------------------------------------------------------------------------------------------
 
-// Largest magnitude (as bits; an infinity or a NaN is the largest) of each column, and the binary exponents' sum and number where
-// a number is not zero, in kParts parts.  HBM or L2.
+// Of each column the largest magnitude (as bits; an infinity or a NaN is the largest) and, over the numbers that are not zero, the sum of 1 /
+// sqrt(magnitude) and their number; of each sixteen columns (the last sixteen for a rest of them) the smallest row maximum that is not
+// zero, as bits; in kParts parts.  HBM or L2.
 __global__ void __launch_bounds__(1024) column_range_kernel(const float *g, std::int64_t ld, int n, int padded, std::int64_t row_begin, std::int64_t row_end,
-                                                            unsigned *part_max, ulonglong2 *part_sum, int *status) {
-    __shared__ unsigned most_of[1024];
-    __shared__ unsigned exponents_of[1024], count_of[1024];
+                                                            unsigned *part_max, double2 *part_sum, unsigned *part_least, int *status) {
+    __shared__ unsigned most_of[1024], least_of[1024], count_of[1024];
+    __shared__ float inverse_of[1024];
     let_next_launch_start();
     if (status != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *status = 0;
     const int c = threadIdx.x % padded, lanes = 1024 / padded;
-    unsigned most = 0u, exponents = 0u, count = 0u;
-    if (c < n) {
-        const std::int64_t step = static_cast<std::int64_t>(gridDim.x) * lanes;
-        std::int64_t r = row_begin + static_cast<std::int64_t>(blockIdx.x) * lanes + threadIdx.x / padded;
-        const float *at = g + r * ld + c;
-        const auto take = [&](float v) {
-            const unsigned bits = __float_as_uint(v) & 0x7fffffffu;
+    // behind the last column of its sixteen a lane has one of the sixteen before
+    const int from = c < n ? c : c / kBlockColumns * kBlockColumns < n && c >= kBlockColumns ? c - kBlockColumns : -1;
+    unsigned most = 0u, count = 0u, least = 0xffffffffu;
+    float inverse = 0.0f;
+    const std::int64_t step = static_cast<std::int64_t>(gridDim.x) * lanes;
+    std::int64_t r = row_begin + static_cast<std::int64_t>(blockIdx.x) * lanes + threadIdx.x / padded; // the same in a warp
+    const float *at = g + r * ld + from;
+    const auto take = [&](float v) {
+        const unsigned bits = __float_as_uint(v) & 0x7fffffffu;
+        if (c < n) {
             most = max(most, bits);
-            exponents += bits >> 23;
-            count += bits != 0u ? 1u : 0u;
-        };
-        for (; r + 7 * step < row_end; r += 8 * step, at += 8 * step * ld) {
-            float v[8];
-#pragma unroll
-            for (int k = 0; k < 8; ++k) v[k] = __ldg(at + k * step * ld);
-#pragma unroll
-            for (int k = 0; k < 8; ++k) take(v[k]);
+            if (bits != 0u) {
+                inverse += rsqrtf(fabsf(v));
+                ++count;
+            }
         }
-        for (; r < row_end; r += step, at += step * ld) take(__ldg(at));
+        return bits;
+    };
+    for (; r + 7 * step < row_end; r += 8 * step, at += 8 * step * ld) {
+        float v[8];
+        unsigned m[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) v[k] = from >= 0 ? __ldg(at + k * step * ld) : 0.0f;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) m[k] = take(v[k]);
+        // eight rows over sixteen lanes: half of the rows stay with half of the lanes, three times, and two lanes have a row's halves
+#pragma unroll
+        for (int d = 4; d > 0; d >>= 1) {
+            const bool upper = (threadIdx.x & d) != 0u;
+#pragma unroll
+            for (int k = 0; k < d; ++k) {
+                const unsigned mine = upper ? m[k + d] : m[k], theirs = upper ? m[k] : m[k + d];
+                m[k] = max(mine, __shfl_xor_sync(0xffffffffu, theirs, d));
+            }
+        }
+        m[0] = max(m[0], __shfl_xor_sync(0xffffffffu, m[0], 8));
+        if (m[0] != 0u) least = min(least, m[0]);
     }
+    for (; r < row_end; r += step, at += step * ld) {
+        unsigned m = take(from >= 0 ? __ldg(at) : 0.0f);
+#pragma unroll
+        for (int d = 8; d > 0; d >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, d));
+        if (m != 0u) least = min(least, m);
+    }
+#pragma unroll
+    for (int d = 8; d > 0; d >>= 1) least = min(least, __shfl_xor_sync(0xffffffffu, least, d));
     most_of[threadIdx.x] = most;
-    exponents_of[threadIdx.x] = exponents;
+    least_of[threadIdx.x] = least;
     count_of[threadIdx.x] = count;
+    inverse_of[threadIdx.x] = inverse;
     __syncthreads();
     if (threadIdx.x < static_cast<unsigned>(padded)) {
-        unsigned long long sum = exponents, number = count;
+        double sum = static_cast<double>(inverse), number = static_cast<double>(count);
         for (int k = 1; k < lanes; ++k) {
             most = max(most, most_of[threadIdx.x + k * padded]);
-            sum += exponents_of[threadIdx.x + k * padded];
-            number += count_of[threadIdx.x + k * padded];
+            least = min(least, least_of[threadIdx.x + k * padded]);
+            sum += static_cast<double>(inverse_of[threadIdx.x + k * padded]);
+            number += static_cast<double>(count_of[threadIdx.x + k * padded]);
         }
         part_max[blockIdx.x * kMaxColumns + threadIdx.x] = most;
-        part_sum[blockIdx.x * kMaxColumns + threadIdx.x] = make_ulonglong2(sum, number);
+        part_sum[blockIdx.x * kMaxColumns + threadIdx.x] = make_double2(sum, number);
+        if (threadIdx.x % kBlockColumns == 0u) part_least[(blockIdx.x * kMaxColumns + threadIdx.x) / kBlockColumns] = least;
     }
     // beside digit_words_kernel in a call that makes its words: what waits for this kernel waits for that one too
     wait_for_previous_launch();
@@ -432,93 +482,43 @@ __global__ void __launch_bounds__(1024) column_range_kernel(const float *g, std:
 // G -> per (pass, block of NB columns, group of 256 cells) a record of four pieces of 64 cells, each the S NB x 64 digits in the no-swizzle
 // K-major operand layout (byte of (column k NB + c: digit k of column c, the highest first; cell r) = column / 8 * 512 + r / 16 *
 // 128 + column % 8 * 16 + r % 16).  Cells outside [row_begin, row_end) and columns from n on are zero.
-// Every block adds the parts up for itself; the first one writes the columns' steps and how the launch goes on (digit_params::wide).
+struct pack_params {
+    const float *g;
+    std::int64_t ld, first_row, row_begin, row_end, groups; // first_row: of the groups; row_begin, row_end: of the launch
+    int n, padded;
+    const unsigned *part_max;
+    const double2 *part_sum;
+    const unsigned *part_least;
+    double *steps;
+    unsigned char *records;
+    const std::int64_t *bases;
+    std::int64_t word_pieces;
+    int *mode;
+    uint4 *totals;            // the totals to clear, 16 bytes each, of one pass
+    std::int64_t total_items;
+};
+// the second pass takes up what the first rounds off, at most half a step
+__host__ __device__ constexpr double second_step(int slices) { return 1.0 / static_cast<double>(1ull << (8 * slices - 1)); }
+
+// factor: 2^k, what a column is multiplied by
 template<int NB, int SLICES>
-__global__ void __launch_bounds__(256) pack_digits_kernel(const float *g, std::int64_t ld, int n, int padded, std::int64_t first_row, std::int64_t row_begin,
-                                                          std::int64_t row_end, std::int64_t groups, const unsigned *part_max, const ulonglong2 *part_sum,
-                                                          double *steps, unsigned char *records, const std::int64_t *bases, std::int64_t word_pieces, int *wide,
-                                                          uint4 *totals, std::int64_t total_items) { // the totals to clear, 16 bytes each, of one pass
-    __shared__ unsigned most_of[256];
-    __shared__ ulonglong2 sum_of[256];
-    __shared__ double factor[kMaxColumns]; // 2^k: what a column is multiplied by
-    // the second pass takes up what the first rounds off, at most half a step
-    constexpr double kSecond = 1.0 / static_cast<double>(1ull << (8 * SLICES - 1));
-    int passes;
-    wait_for_previous_launch();
-    let_next_launch_start();
-    const int tid = threadIdx.x;
-    {
-        const int c = tid % padded, lanes = 256 / padded;
-        unsigned most = 0u;
-        ulonglong2 sum = make_ulonglong2(0u, 0u);
-        for (int k0 = tid / padded; k0 < kParts; k0 += 6 * lanes) { // lanes 1, 2, 4, 8: six loads of each kind in flight
-            unsigned m[6];
-            ulonglong2 q[6];
-#pragma unroll
-            for (int k = 0; k < 6; ++k) {
-                m[k] = __ldcg(part_max + (k0 + k * lanes) * kMaxColumns + c);
-                q[k] = __ldcg(part_sum + (k0 + k * lanes) * kMaxColumns + c);
-            }
-#pragma unroll
-            for (int k = 0; k < 6; ++k) {
-                most = max(most, m[k]);
-                sum.x += q[k].x;
-                sum.y += q[k].y;
-            }
-        }
-        most_of[tid] = most;
-        sum_of[tid] = sum;
-        __syncthreads();
-        int too_wide = 0;
-        if (tid < padded) {
-            for (int k = 1; k < lanes; ++k) {
-                most = max(most, most_of[tid + k * padded]);
-                sum.x += sum_of[tid + k * padded].x;
-                sum.y += sum_of[tid + k * padded].y;
-            }
-            double f = 0.0, step = 0.0;
-            if (most >= 0x7f800000u) {
-                too_wide = 2;
-            } else if (most != 0u) {
-                // largest = m 2^e, m in [0.5, 1); the largest number of S balanced digits is 0.996 * 2^(8 S - 1)
-                const int e = most >= 0x800000u ? static_cast<int>(most >> 23) - 126 : 32 - __clz(most) - 149;
-                const int k = 8 * SLICES - 1 - e - ((most & 0x7fffffu) > 8220000u || most < 0x800000u ? 1 : 0);
-                f = __longlong_as_double(static_cast<long long>(1023 + k) << 52);
-                step = __longlong_as_double(static_cast<long long>(1023 - k) << 52);
-                const unsigned long long spread = (most >> 23) * sum.y - sum.x; // times the number of numbers
-                too_wide = spread <= kMostSpread * sum.y ? 0 : spread <= (kMostSpread + 8 * SLICES - 1) * sum.y ? 1 : 2;
-            }
-            factor[tid] = f;
-            if (blockIdx.x == 0) {
-                const int columns = (n + NB - 1) / NB * NB;
-                if (tid < columns) steps[tid] = step;
-                if (tid < columns) steps[columns + tid] = step * kSecond; // of the second pass
-            }
-        }
-        if (blockIdx.x == 0) {
-#pragma unroll 8
-            for (std::int64_t k = tid; k < word_pieces; k += 256) too_wide |= (__ldcg(bases + k) & kTwice) != 0 ? 2 : 0;
-        }
-        const bool second = __syncthreads_or(too_wide & 1) != 0, by_entry = __syncthreads_or(too_wide & 2) != 0;
-        if (blockIdx.x == 0 && tid == 0) *wide = by_entry ? 2 : second ? 1 : 0;
-        passes = second ? 2 : 1;
-    }
-    for (std::int64_t i = blockIdx.x * 256 + tid; i < passes * total_items; i += gridDim.x * 256) totals[i] = make_uint4(0u, 0u, 0u, 0u);
+__device__ __forceinline__ void pack_records(const pack_params &p, int passes, const double *factor) {
     constexpr int NC = mma_columns(NB, SLICES);
-    const std::int64_t pieces = static_cast<std::int64_t>((n + NB - 1) / NB) * groups * kGPieces;
+    const int tid = threadIdx.x;
+    const std::int64_t pieces = static_cast<std::int64_t>((p.n + NB - 1) / NB) * p.groups * kGPieces;
     for (std::int64_t b = blockIdx.x; b < passes * pieces; b += gridDim.x) {
         const bool second = b >= pieces;
-        const int c0 = static_cast<int>((second ? b - pieces : b) / (groups * kGPieces)) * NB;
-        const std::int64_t row0 = first_row + b % (groups * kGPieces) * kGPieceRows;
-        unsigned char *rec = records + b * (kGPieceRows * NC);
+        const int c0 = static_cast<int>((second ? b - pieces : b) / (p.groups * kGPieces)) * NB;
+        const std::int64_t row0 = p.first_row + b % (p.groups * kGPieces) * kGPieceRows;
+        unsigned char *rec = p.records + b * (kGPieceRows * NC);
         for (int item = tid; item < NB * (kGPieceRows / 16); item += 256) {
             const int c = item % NB, r16 = item / NB;
-            const double f = c0 + c < n ? factor[c0 + c] : 0.0;
+            const double f = c0 + c < p.n ? factor[c0 + c] : 0.0;
             float v[16];
 #pragma unroll
             for (int j = 0; j < 16; ++j) {
                 const std::int64_t row = row0 + r16 * 16 + j;
-                v[j] = row >= row_begin && row < row_end && c0 + c < n ? __ldg(g + row * ld + c0 + c) : 0.0f;
+                v[j] = row >= p.row_begin && row < p.row_end && c0 + c < p.n ? __ldg(p.g + row * p.ld + c0 + c) : 0.0f;
             }
             std::uint32_t digit[SLICES][4];
 #pragma unroll
@@ -529,7 +529,7 @@ __global__ void __launch_bounds__(256) pack_digits_kernel(const float *g, std::i
             for (int j = 0; j < 16; ++j) {
                 const double scaled = static_cast<double>(v[j]) * f;
                 int q = __double2int_rn(scaled);
-                if (second) q = __double2int_rn((scaled - static_cast<double>(q)) * (1.0 / kSecond));
+                if (second) q = __double2int_rn((scaled - static_cast<double>(q)) * (1.0 / second_step(SLICES)));
 #pragma unroll
                 for (int k = SLICES - 1; k >= 0; --k) {
                     digit[k][j >> 2] |= (static_cast<std::uint32_t>(q) & 0xffu) << ((j & 3) * 8);
@@ -546,6 +546,96 @@ __global__ void __launch_bounds__(256) pack_digits_kernel(const float *g, std::i
     }
 }
 
+// Every block adds the parts up for itself and so knows how the launch goes on; the first one writes the mode and the columns' steps.
+template<int NB, int BASE>
+__global__ void __launch_bounds__(256) pack_digits_kernel(const pack_params p) {
+    __shared__ unsigned most_of[kMaxColumns], least_of[kMaxColumns / kBlockColumns];
+    __shared__ double2 sum_of[256];
+    __shared__ double factor[kMaxColumns];
+    __shared__ unsigned long long need_bits; // 2^spread, whose bits have its order
+    const int tid = threadIdx.x;
+    if (tid < kMaxColumns / kBlockColumns) least_of[tid] = 0xffffffffu;
+    if (tid == 0) need_bits = 0u;
+    wait_for_previous_launch();
+    let_next_launch_start();
+    __syncthreads();
+    int mode;
+    {
+        const int c = tid % p.padded, lanes = 256 / p.padded, blocks = p.padded / kBlockColumns;
+        unsigned most = 0u;
+        double2 sum = make_double2(0.0, 0.0);
+        for (int k0 = tid / p.padded; k0 < kParts; k0 += 6 * lanes) { // lanes 1, 2, 4, 8: six loads of each kind in flight
+            unsigned m[6];
+            double2 q[6];
+#pragma unroll
+            for (int k = 0; k < 6; ++k) {
+                m[k] = __ldcg(p.part_max + (k0 + k * lanes) * kMaxColumns + c);
+                q[k] = __ldcg(p.part_sum + (k0 + k * lanes) * kMaxColumns + c);
+            }
+#pragma unroll
+            for (int k = 0; k < 6; ++k) {
+                most = max(most, m[k]);
+                sum.x += q[k].x;
+                sum.y += q[k].y;
+            }
+        }
+        for (int i = tid; i < kParts * blocks; i += 256) atomicMin(least_of + i % blocks, __ldcg(p.part_least + i / blocks * (kMaxColumns / kBlockColumns) + i % blocks));
+        most_of[tid] = most;
+        sum_of[tid] = sum;
+        __syncthreads();
+        int by_entry = 0;
+        if (tid < p.padded) {
+            for (int k = 1; k < lanes; ++k) {
+                most = max(most, most_of[tid + k * p.padded]);
+                sum.x += sum_of[tid + k * p.padded].x;
+                sum.y += sum_of[tid + k * p.padded].y;
+            }
+            if (most >= 0x7f800000u) by_entry = 1;
+            else if (most != 0u) atomicMax(&need_bits, static_cast<unsigned long long>(__double_as_longlong(static_cast<double>(__uint_as_float(most)) * sum.x * sum.x / (2.0 * sum.y * sum.y))));
+        }
+        __syncthreads();
+        if (tid < p.padded) most_of[tid] = most; // the columns'
+        __syncthreads();
+        if (tid < blocks && tid * kBlockColumns < p.n && least_of[tid] < 0x7f800000u) {
+            unsigned largest = 0u;
+            for (int k = max(0, min(tid * kBlockColumns, p.n - kBlockColumns)); k < min((tid + 1) * kBlockColumns, p.n); ++k) largest = max(largest, most_of[k]);
+            if (largest < 0x7f800000u)
+                atomicMax(&need_bits, static_cast<unsigned long long>(__double_as_longlong(static_cast<double>(__uint_as_float(largest)) / static_cast<double>(__uint_as_float(least_of[tid])))));
+        }
+        if (blockIdx.x == 0) {
+#pragma unroll 8
+            for (std::int64_t k = tid; k < p.word_pieces; k += 256) by_entry |= (__ldcg(p.bases + k) & kTwice) != 0 ? 1 : 0;
+        }
+        by_entry = __syncthreads_or(by_entry);
+        const double need = __longlong_as_double(static_cast<long long>(need_bits));
+        const auto serves = [&](int slices, int passes) { return need <= static_cast<double>(1ull << most_spread(BASE, slices, passes)); };
+        mode = BASE == 3 && serves(3, 1) ? mode_of(3, 1) : serves(4, 1) ? mode_of(4, 1) : BASE == 3 && serves(3, 2) ? mode_of(3, 2) : mode_of(4, 2);
+        if (by_entry != 0 || !serves(4, 2)) mode |= kByEntry;
+        if (tid < p.padded) {
+            const int bits = 8 * slices_of(mode) - 1;
+            double f = 0.0, step = 0.0;
+            if (most != 0u && most < 0x7f800000u) {
+                // largest = m 2^e, m in [0.5, 1); the largest number of S balanced digits is 0.996 * 2^(8 S - 1)
+                const int e = most >= 0x800000u ? static_cast<int>(most >> 23) - 126 : 32 - __clz(most) - 149;
+                const int k = bits - e - ((most & 0x7fffffu) > 8220000u || most < 0x800000u ? 1 : 0);
+                f = __longlong_as_double(static_cast<long long>(1023 + k) << 52);
+                step = __longlong_as_double(static_cast<long long>(1023 - k) << 52);
+            }
+            factor[tid] = f;
+            if (blockIdx.x == 0) {
+                const int columns = (p.n + NB - 1) / NB * NB;
+                if (tid < columns) p.steps[tid] = step;
+                if (tid < columns) p.steps[columns + tid] = step * (slices_of(mode) == 3 ? second_step(3) : second_step(4)); // of the second pass
+            }
+        }
+        if (blockIdx.x == 0 && tid == 0) *p.mode = mode;
+        __syncthreads();
+    }
+    for (std::int64_t i = blockIdx.x * 256 + tid; i < passes_of(mode) * p.total_items; i += gridDim.x * 256) p.totals[i] = make_uint4(0u, 0u, 0u, 0u);
+    if (BASE == 3 && slices_of(mode) == 3) pack_records<NB, 3>(p, passes_of(mode), factor);
+    else pack_records<NB, 4>(p, passes_of(mode), factor);
+}
+
 // ---- the sums --------------------------------------------------------------------------------------------------------------
 
 struct digit_params {
@@ -557,7 +647,7 @@ struct digit_params {
     const float *scales, *offsets;
     const unsigned char *records;
     const double *steps;
-    const int *wide;         // 0: one pass, 1: two, 2: entry by entry
+    const int *mode;
     float *partials;         // [run_of + CTA][window of the set][column][gene]: a run's sums, rounded
     long long *totals;       // EXACT: [set][window of the set][codes, ones][column][gene], which the runs add to
     std::int64_t cols;
@@ -618,7 +708,7 @@ __device__ __forceinline__ std::uint64_t smem_desc_digits(std::uint32_t addr) {
 }
 
 template<int NB, int SLICES, bool EXACT>
-__global__ void __launch_bounds__(kThreads, 1) qcsr_transpose_digits_kernel(const digit_params p) {
+__device__ __forceinline__ void transpose_tiles(const digit_params &p) {
     constexpr int NC = mma_columns(NB, SLICES), kSet = set_windows(NB, SLICES), GPIECE = g_piece_bytes(NB, SLICES), kPieces = ring_pieces(NB, SLICES);
     constexpr std::uint32_t IDESC = instr_desc_i8(NC);
     extern __shared__ __align__(1024) unsigned char smem[];
@@ -668,12 +758,12 @@ __global__ void __launch_bounds__(kThreads, 1) qcsr_transpose_digits_kernel(cons
     wait_for_previous_launch();
 
     const std::int64_t sets = p.set_count;
-    const int wide = __ldcg(p.wide);
+    const int mode = __ldcg(p.mode);
     // the second pass: as many column blocks again
-    const std::int64_t total_units = sets * p.column_blocks * p.group_count * (wide == 1 ? 2 : 1);
+    const std::int64_t total_units = sets * p.column_blocks * p.group_count * passes_of(mode);
     const std::int64_t u0 = total_units * blockIdx.x / gridDim.x;
     // entry by entry: nothing to do here, it is finish_kernel's work
-    const std::int64_t u1 = wide == 2 ? u0 : total_units * (blockIdx.x + 1) / gridDim.x;
+    const std::int64_t u1 = (mode & kByEntry) != 0 ? u0 : total_units * (blockIdx.x + 1) / gridDim.x;
 
     if (warp < kProducerWarps) {
         // ================= zero, scatter, read back =================
@@ -944,6 +1034,19 @@ __global__ void __launch_bounds__(kThreads, 1) qcsr_transpose_digits_kernel(cons
     if (tid == 0 && *abort_flag != 0) atomicExch(p.status, 1);
 }
 
+// A base of three digits: three or, where G spreads too far for them and not for four, four; the launches before have decided it.
+template<int NB, int BASE, bool EXACT>
+__global__ void __launch_bounds__(kThreads, 1) qcsr_transpose_digits_kernel(const digit_params p) {
+    if constexpr (BASE == 3) {
+        wait_for_previous_launch();
+        if (slices_of(__ldcg(p.mode)) == 3) {
+            transpose_tiles<NB, 3, EXACT>(p);
+            return;
+        }
+    }
+    transpose_tiles<NB, 4, EXACT>(p);
+}
+
 template<int NB, int SLICES> constexpr std::size_t digits_smem_bytes() {
     return 2 * kTileBytes + ring_pieces(NB, SLICES) * g_piece_bytes(NB, SLICES) + 2 * kChunkBytes + (11 + 2 * ring_pieces(NB, SLICES)) * sizeof(std::uint64_t) + 32;
 }
@@ -965,10 +1068,11 @@ struct finish_params {
 // sixteenth gene of the window to itself and walks the words in order, so this too has the same bits on every run.
 // A thread has a gene and sixteen columns, so that a warp's loads are contiguous.
 __host__ __device__ constexpr int finish_threads(int nb) { return nb / 16 * kWin; }
-template<int NB, int SLICES, bool EXACT>
+template<int NB, bool EXACT>
 __global__ void __launch_bounds__(finish_threads(NB)) finish_kernel(const finish_params p) {
     extern __shared__ double slow_sums[]; // [kWin][NB]
-    constexpr int kSet = set_windows(NB, SLICES), kFinish = finish_threads(NB);
+    constexpr int kSet = set_windows(NB, kMostSlices), kFinish = finish_threads(NB);
+    static_assert(kSet == set_windows(NB, 3), "the sets of a launch do not follow from its mode");
     __shared__ float2 meta[kWin];
     wait_for_previous_launch();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -985,8 +1089,8 @@ __global__ void __launch_bounds__(finish_threads(NB)) finish_kernel(const finish
         meta[tid] = so;
         odd = isfinite(so.x) && isfinite(so.y) ? 0 : 1;
     }
-    const int wide = __ldcg(p.d.wide);
-    const bool slow = __syncthreads_or(odd) != 0 || wide == 2;
+    const int mode = __ldcg(p.d.mode);
+    const bool slow = __syncthreads_or(odd) != 0 || (mode & kByEntry) != 0;
     if (slow) {
         for (int i = tid; i < kWin * NB; i += kFinish) slow_sums[i] = 0.0;
         __syncthreads();
@@ -1018,7 +1122,7 @@ __global__ void __launch_bounds__(finish_threads(NB)) finish_kernel(const finish
         __syncthreads();
     }
     // the set's slots: the CTAs whose shares meet its runs, run after run, pass after pass
-    const int passes = wide == 1 ? 2 : 1;
+    const int passes = passes_of(mode);
     const std::int64_t total = sets * p.d.column_blocks * p.d.group_count * passes, L = p.d.group_count, cuts = (L + p.d.run_groups - 1) / p.d.run_groups;
     const int gl = tid & (kWin - 1);
     const std::int64_t gene = window * kWin + gl;
@@ -1087,38 +1191,37 @@ __global__ void __launch_bounds__(finish_threads(NB)) finish_kernel(const finish
     }
 }
 
-// Digits of a repeatable launch, and the groups and sets of windows a launch with the least workspace takes at a time.
-constexpr int kExactSlices = 4;
-constexpr std::int64_t kLeastGroups = 2, kLeastSets = 4;
+// What a launch with the least workspace takes at a time: groups, and, repeatable, sets of windows.
+constexpr std::int64_t kLeastGroups = 2, kLeastSets = 4, kLeastRoundedGroups = 11;
 int column_block(std::int64_t n) { return n <= 32 ? 32 : 64; }
 int padded_columns(std::int64_t n) { return n <= 32 ? 32 : n <= 64 ? 64 : n <= 128 ? 128 : 256; }
 
-// (both with room for the second pass)
-std::uint64_t record_bytes(std::int64_t groups, std::int64_t n, int slices) {
+// (both with room for a second pass, and for four digits)
+std::uint64_t record_bytes(std::int64_t groups, std::int64_t n) {
     const int nb = column_block(n);
-    return device_arena::rounded(2u * static_cast<std::uint64_t>(groups) * static_cast<std::uint64_t>((n + nb - 1) / nb) * kRows * static_cast<std::uint64_t>(mma_columns(nb, slices)));
+    return device_arena::rounded(2u * static_cast<std::uint64_t>(groups) * static_cast<std::uint64_t>((n + nb - 1) / nb) * kRows * static_cast<std::uint64_t>(mma_columns(nb, kMostSlices)));
 }
 // a run ends with its set, after kRunGroups groups, or with its CTA's share of the units
-std::uint64_t partial_bytes(std::int64_t groups, std::int64_t cols, std::int64_t n, int slices, int ctas) {
-    const std::int64_t nb = column_block(n), per_set = set_windows(static_cast<int>(nb), slices), windows = (cols + kWin - 1) / kWin;
+std::uint64_t partial_bytes(std::int64_t groups, std::int64_t cols, std::int64_t n, int ctas) {
+    const std::int64_t nb = column_block(n), per_set = set_windows(static_cast<int>(nb), kMostSlices), windows = (cols + kWin - 1) / kWin;
     const std::int64_t sets = (windows + per_set - 1) / per_set * ((n + nb - 1) / nb), cuts = (groups + kRunGroups - 1) / kRunGroups;
     return device_arena::rounded(static_cast<std::uint64_t>(2 * sets * cuts + ctas) * static_cast<std::uint64_t>(per_set * kWin * nb) * sizeof(float));
 }
 // what a launch over `groups` groups at a time needs, without the words
-std::uint64_t launch_bytes(std::int64_t groups, std::int64_t cols, std::int64_t n, int slices, int ctas) {
-    return kRecordsAt + record_bytes(groups, n, slices) + partial_bytes(groups, cols, n, slices, ctas);
+std::uint64_t launch_bytes(std::int64_t groups, std::int64_t cols, std::int64_t n, int ctas) {
+    return kRecordsAt + record_bytes(groups, n) + partial_bytes(groups, cols, n, ctas);
 }
 // ... and a repeatable one over `sets` sets of windows at a time
 std::int64_t set_count_of(std::int64_t cols, std::int64_t n) {
-    const std::int64_t per_set = set_windows(column_block(n), kExactSlices), windows = (cols + kWin - 1) / kWin;
+    const std::int64_t per_set = set_windows(column_block(n), kMostSlices), windows = (cols + kWin - 1) / kWin;
     return (windows + per_set - 1) / per_set;
 }
 std::uint64_t total_bytes(std::int64_t sets, std::int64_t n) { // of one pass
     const std::int64_t nb = column_block(n);
-    return static_cast<std::uint64_t>(sets * ((n + nb - 1) / nb) * set_windows(static_cast<int>(nb), kExactSlices) * kWin * nb) * 16u;
+    return static_cast<std::uint64_t>(sets * ((n + nb - 1) / nb) * set_windows(static_cast<int>(nb), kMostSlices) * kWin * nb) * 16u;
 }
 std::uint64_t exact_bytes(std::int64_t groups, std::int64_t sets, std::int64_t n) {
-    return kRecordsAt + record_bytes(groups, n, kExactSlices) + 2u * total_bytes(sets, n);
+    return kRecordsAt + record_bytes(groups, n) + 2u * total_bytes(sets, n);
 }
 std::int64_t group_count_of(std::int64_t rows) { return (rows + kRows - 1) / kRows; }
 std::int64_t piece_count(std::int64_t rows) { return (rows + piece_rows_of(rows) - 1) / piece_rows_of(rows); }
@@ -1137,29 +1240,26 @@ struct digit_launch {
     finish_params finish;
     std::int64_t slice;      // groups at a time
     std::int64_t chunk;      // EXACT: sets of windows at a time
-    unsigned *part_max;
-    ulonglong2 *part_sum;
-    double *steps;
-    unsigned char *records;
-    int *wide;
+    pack_params pack;        // without the groups and what is to be cleared
     bool early; // the launch in front is a kernel of this call
 };
 
 // Slice after slice of the groups: the runs' sums are rounded and a slice's are added to G'.  EXACT (a request that has to be
 // repeatable): chunk after chunk of the windows and slice after slice of the groups, whose sums meet as whole numbers, so that neither the
 // grid nor the room for slices and chunks changes a bit.
-template<int NB, int SLICES, bool EXACT>
+template<int NB, int BASE, bool EXACT>
 cb200_status launch_digits(const digit_launch &l, int sm_count, cudaStream_t stream) {
-    constexpr std::size_t smem = digits_smem_bytes<NB, SLICES>();
+    constexpr std::size_t smem = std::max(digits_smem_bytes<NB, BASE>(), digits_smem_bytes<NB, kMostSlices>());
     static_assert(smem <= 232448, "shared memory budget");
-    constexpr int slow_smem = kWin * NB * 8, kSet = set_windows(NB, SLICES);
-    const auto main_kernel = qcsr_transpose_digits_kernel<NB, SLICES, EXACT>;
-    const auto finish = finish_kernel<NB, SLICES, EXACT>;
+    constexpr int slow_smem = kWin * NB * 8, kSet = set_windows(NB, kMostSlices);
+    const auto main_kernel = qcsr_transpose_digits_kernel<NB, BASE, EXACT>;
+    const auto finish = finish_kernel<NB, EXACT>;
     CB200_CUDA_OK(cudaFuncSetAttribute(main_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
     CB200_CUDA_OK(cudaFuncSetAttribute(finish, cudaFuncAttributeMaxDynamicSharedMemorySize, slow_smem));
-    const int n = l.finish.n, padded = padded_columns(n);
-    CB200_CUDA_OK(launch_kernel(l.early, column_range_kernel, dim3(kParts), 1024, 0, stream, l.finish.g, l.finish.g_ld, n, padded, l.finish.row_begin, l.finish.row_end,
-                                l.part_max, l.part_sum, l.early ? nullptr : l.main.status));
+    const int n = l.finish.n;
+    CB200_CUDA_OK(launch_kernel(l.early, column_range_kernel, dim3(kParts), 1024, 0, stream, l.finish.g, l.finish.g_ld, n, l.pack.padded, l.finish.row_begin, l.finish.row_end,
+                                const_cast<unsigned *>(l.pack.part_max), const_cast<double2 *>(l.pack.part_sum), const_cast<unsigned *>(l.pack.part_least),
+                                l.early ? nullptr : l.main.status));
     count_launch();
     const std::int64_t group_end = l.main.group_begin + l.main.group_count, sets = (l.main.windows + kSet - 1) / kSet;
     const std::int64_t chunk = EXACT ? l.chunk : sets;
@@ -1178,15 +1278,17 @@ cb200_status launch_digits(const digit_launch &l, int sm_count, cudaStream_t str
         for (std::int64_t begin = l.main.group_begin; begin < group_end; begin += l.slice) {
             m.group_begin = begin;
             m.group_count = std::min(l.slice, group_end - begin);
-            unsigned char *sums = l.records + record_bytes(m.group_count, n, SLICES);
-            if (EXACT) sums = l.records + record_bytes(l.slice, n, SLICES); // the same place for all slices
+            // behind the slice's records; EXACT: the same place for all slices
+            unsigned char *sums = l.pack.records + record_bytes(EXACT ? l.slice : m.group_count, n);
             m.partials = EXACT ? nullptr : reinterpret_cast<float *>(sums);
             m.totals = EXACT ? reinterpret_cast<long long *>(sums) : nullptr;
             const std::int64_t row0 = l.finish.first_row + begin * kRows, blocks = m.group_count * m.column_blocks;
-            const std::int64_t to_clear = EXACT && clear ? static_cast<std::int64_t>(total_bytes(m.set_count, n) / 16u) : 0;
-            CB200_CUDA_OK(launch_kernel(true, pack_digits_kernel<NB, SLICES>, dim3(static_cast<unsigned>(std::min<std::int64_t>(blocks * kGPieces, 4 * sm_count))), 256, 0, stream,
-                                        f.g, f.g_ld, n, padded, row0, l.finish.row_begin, l.finish.row_end, m.group_count, l.part_max, l.part_sum, l.steps, l.records, m.bases,
-                                        m.pieces, l.wide, reinterpret_cast<uint4 *>(m.totals), to_clear));
+            pack_params k = l.pack;
+            k.first_row = row0;
+            k.groups = m.group_count;
+            k.totals = reinterpret_cast<uint4 *>(m.totals);
+            k.total_items = EXACT && clear ? static_cast<std::int64_t>(total_bytes(m.set_count, n) / 16u) : 0;
+            CB200_CUDA_OK(launch_kernel(true, pack_digits_kernel<NB, BASE>, dim3(static_cast<unsigned>(std::min<std::int64_t>(blocks * kGPieces, 4 * sm_count))), 256, 0, stream, k));
             clear = false;
             const unsigned grid = static_cast<unsigned>(std::min<std::int64_t>(m.set_count * blocks, sm_count));
             CB200_CUDA_OK(launch_kernel(true, main_kernel, dim3(grid), kThreads, smem, stream, m));
@@ -1245,14 +1347,14 @@ digit_layout digit_words_at(void *memory, const qcsr_view &x) {
     l.bases = reinterpret_cast<std::int64_t *>(at);
     return l;
 }
-std::uint64_t qcsr_transpose_digits_workspace_bytes(std::int64_t rows, std::int64_t cols, std::int64_t n, int slices, bool repeatable) {
+std::uint64_t qcsr_transpose_digits_workspace_bytes(std::int64_t rows, std::int64_t cols, std::int64_t n, bool repeatable) {
     if (repeatable) return exact_bytes(group_count_of(rows), set_count_of(cols, n), n);
-    return launch_bytes(group_count_of(rows), cols, n, slices, kMaxCtas);
+    return launch_bytes(group_count_of(rows), cols, n, kMaxCtas);
 }
-std::uint64_t qcsr_transpose_digits_least_workspace(std::int64_t rows, std::int64_t cols, std::int64_t n, int slices, bool repeatable, int sm_count) {
+std::uint64_t qcsr_transpose_digits_least_workspace(std::int64_t rows, std::int64_t cols, std::int64_t n, bool repeatable, int sm_count) {
     const std::int64_t groups = group_count_of(rows);
     if (repeatable) return exact_bytes(std::min<std::int64_t>(groups, kLeastGroups), std::min<std::int64_t>(set_count_of(cols, n), kLeastSets), n);
-    return launch_bytes(std::min<std::int64_t>(groups, 16), cols, n, slices, std::min(sm_count, kMaxCtas));
+    return launch_bytes(std::min<std::int64_t>(groups, kLeastRoundedGroups), cols, n, std::min(sm_count, kMaxCtas));
 }
 std::uint64_t qcsr_transpose_digits_once_bytes(std::int64_t rows, std::int64_t cols, std::int64_t n, std::int64_t nnz, int bits, int policy) {
     if (!qcsr_transpose_digits_shape_ok(rows, cols, n, bits, policy)) return 0u;
@@ -1260,7 +1362,7 @@ std::uint64_t qcsr_transpose_digits_once_bytes(std::int64_t rows, std::int64_t c
     // 64: 2,000 x 8,000 (1.6 M entries) 48 us against 45, 1,500 x 33,538 (2.7 M) 75 against 75, 4,000 x 4,000 (2.1 M) 49 against 57,
     // 8,191 x 33,538 (14.7 M) 171 against 318; at N = 32 8,000 x 2,000 (2.9 M) 51 against 53, 16,384 x 2,000 (5.9 M) 74 against 108.
     if (static_cast<double>(nnz) < 0.02 * static_cast<double>(rows) * static_cast<double>(cols) || nnz < kLeastOnceEntries || nnz > kMostOnceEntries) return 0u;
-    return qcsr_transpose_digits_workspace_bytes(rows, cols, n, 4, false) + qcsr_digit_words_bytes_bound(rows, cols, nnz);
+    return qcsr_transpose_digits_workspace_bytes(rows, cols, n, false) + qcsr_digit_words_bytes_bound(rows, cols, nnz);
 }
 
 cb200_status build_digit_words(const qcsr_view &x, device_arena &arena, cudaStream_t stream, digit_layout *out) {
@@ -1300,12 +1402,12 @@ cb200_status launch_qcsr_transpose_digits(const qcsr_view &x, const dense_args &
     if (x.bits == 4 && x.packed_row_ptr == nullptr) return CB200_STATUS_SUCCESS;
     // With less workspace than for the whole range the groups are taken in slices.  A call that has to make its words has room for
     // everything or is another kernel's.
-    const std::uint64_t own = qcsr_transpose_digits_workspace_bytes(x.rows, x.cols, d.n, slices, false);
+    const std::uint64_t own = qcsr_transpose_digits_workspace_bytes(x.rows, x.cols, d.n, false);
     if (layout == nullptr && workspace_bytes < own + qcsr_digit_words_bytes_bound(x.rows, x.cols, x.nnz)) return CB200_STATUS_SUCCESS;
     const std::int64_t first_row = layout != nullptr ? 0 : row_begin, rows_of_words = layout != nullptr ? x.rows : row_end - row_begin;
     const std::int64_t group_begin = (row_begin - first_row) / kRows, group_count = (row_end - first_row + kRows - 1) / kRows - group_begin;
     std::int64_t slice = group_count, chunk = repeatable ? set_count_of(x.cols, d.n) : 0;
-    const auto needs = [&](std::int64_t groups) { return repeatable ? exact_bytes(groups, chunk, d.n) : launch_bytes(groups, x.cols, d.n, slices, sm_count); };
+    const auto needs = [&](std::int64_t groups) { return repeatable ? exact_bytes(groups, chunk, d.n) : launch_bytes(groups, x.cols, d.n, sm_count); };
     while (chunk > 1 && needs(std::min<std::int64_t>(slice, kLeastGroups)) > workspace_bytes) chunk = (chunk + 1) / 2;
     while (slice > 1 && needs(slice) > workspace_bytes) slice = (slice + 1) / 2;
     if (needs(slice) > workspace_bytes) return CB200_STATUS_SUCCESS;
@@ -1315,11 +1417,6 @@ cb200_status launch_qcsr_transpose_digits(const qcsr_view &x, const dense_args &
     unsigned char *ws = static_cast<unsigned char *>(workspace);
     digit_launch l{};
     l.early = layout == nullptr;
-    l.part_max = reinterpret_cast<unsigned *>(ws + kPartMaxAt);
-    l.part_sum = reinterpret_cast<ulonglong2 *>(ws + kPartSumAt);
-    l.steps = reinterpret_cast<double *>(ws + kStepsAt);
-    l.records = ws + kRecordsAt;
-    l.wide = reinterpret_cast<int *>(ws) + 1;
     digit_params &p = l.main;
     p.status = reinterpret_cast<int *>(ws);
     l.slice = slice;
@@ -1337,7 +1434,17 @@ cb200_status launch_qcsr_transpose_digits(const qcsr_view &x, const dense_args &
     p.group_pieces = kRows / p.piece_rows;
     p.pieces = (rows_of_words + p.piece_rows - 1) / p.piece_rows;
     p.scales = x.scales; p.offsets = x.offsets;
-    p.records = l.records; p.steps = l.steps; p.wide = l.wide;
+    pack_params &k = l.pack;
+    k.g = static_cast<const float *>(d.dense); k.ld = d.dense_ld; k.row_begin = row_begin; k.row_end = row_end;
+    k.n = static_cast<int>(d.n); k.padded = padded_columns(d.n);
+    k.part_max = reinterpret_cast<const unsigned *>(ws + kPartMaxAt);
+    k.part_sum = reinterpret_cast<const double2 *>(ws + kPartSumAt);
+    k.part_least = reinterpret_cast<const unsigned *>(ws + kPartLeastAt);
+    k.steps = reinterpret_cast<double *>(ws + kStepsAt);
+    k.records = ws + kRecordsAt;
+    k.bases = p.bases; k.word_pieces = p.pieces;
+    k.mode = reinterpret_cast<int *>(ws) + 1;
+    p.records = k.records; p.steps = k.steps; p.mode = k.mode;
     p.cols = x.cols;
     p.group_begin = group_begin;
     p.group_count = group_count;
@@ -1352,7 +1459,7 @@ cb200_status launch_qcsr_transpose_digits(const qcsr_view &x, const dense_args &
     f.out = d.out; f.out_ld = d.out_ld; f.n = static_cast<int>(d.n);
     f.out_vector = reinterpret_cast<std::uintptr_t>(d.out) % 16u == 0u && d.out_ld % 4 == 0 && d.n % 4 == 0 ? 1 : 0;
     f.alpha = d.alpha; f.beta = d.beta;
-    if (repeatable) return nb == 64 ? launch_digits<64, kExactSlices, true>(l, sm_count, stream) : launch_digits<32, kExactSlices, true>(l, sm_count, stream);
+    if (repeatable) return nb == 64 ? launch_digits<64, kMostSlices, true>(l, sm_count, stream) : launch_digits<32, kMostSlices, true>(l, sm_count, stream);
     if (slices == 4) return nb == 64 ? launch_digits<64, 4, false>(l, sm_count, stream) : launch_digits<32, 4, false>(l, sm_count, stream);
     return nb == 64 ? launch_digits<64, 3, false>(l, sm_count, stream) : launch_digits<32, 3, false>(l, sm_count, stream);
 }

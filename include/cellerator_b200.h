@@ -265,7 +265,7 @@ typedef struct cb200_spmm_problem {
      * hi + lo; hi*hi + hi*lo + lo*hi), relative error about 3 * 2^-17 per product: inside the 1e-4
      * bound of an fp32 operand, not bit-equal to an fp32 multiply.  The transpose with zero-points per gene
      * multiplies the codes with three digits of G in fixed point instead (2^-23 of a column's largest
-     * magnitude) and adds without rounding.  Without device_matrix "gene_tiled" / "warp_per_row" (fp32 FMAs)
+     * magnitude; four, or a second pass of digits, where cells with a small G need them) and adds without rounding.  Without device_matrix "gene_tiled" / "warp_per_row" (fp32 FMAs)
      * and "vector_reductions" (fp32 FMAs, or four digits of G and integer sums) run. */
     int32_t multiply;
     /* Optional: the device-resident matrix itself (arrays on `device`, final contents).  With bf16

@@ -202,3 +202,91 @@ def test_repeatable_bits_do_not_follow_from_the_workspace(cuda_device, oracle, n
             accepted.append(part)
         assert refused > 0 and min(accepted) < 0.75
     op.close()
+
+
+def mode_of(op):
+    """Digits, passes and whether the last launch went entry by entry: the word behind the workspace's status word."""
+    mode = op.workspace[4:8].view(torch.int32).item()
+    return mode >> 4 & 15, mode & 15, bool(mode & 256)
+
+
+# cells scaled down (share, binary orders, all columns or every fifth alone), and how many digits and passes that takes from three and from four
+@pytest.mark.parametrize("share,orders,column,from3,from4", [
+    (0.0, 0, None, (3, 1, False), (4, 1, False)), (0.3, 7, None, (4, 1, False), (4, 2, False)), (0.1, 20, None, (3, 2, False), (4, 2, False)),
+    (0.02, 36, None, (4, 2, False), (4, 2, False)), (0.05, 30, None, (4, 2, False), (4, 2, False)), (0.1, 70, None, (4, 2, True), (4, 2, True)),
+    (0.3, 22, 5, (3, 2, False), (4, 2, False))])
+@pytest.mark.parametrize("slices,n,bits", [(3, 64, 8), (3, 32, 4), (4, 64, 8), (4, 32, 8), (4, 128, 4)])
+def test_few_small_cells_keep_their_bits(cuda_device, oracle, share, orders, column, from3, from4, slices, n, bits):
+    """A gene that only cells with a small G hold has the precision of its own products, whatever the rest of G's columns hold.  No cell holds a
+    gene twice: nothing here goes entry by entry but numbers beyond two passes.  Row ranges; slices of the groups."""
+    rng = np.random.default_rng(int(100 * share) + orders)
+    rows, cols = 256 * 20 + 3, 1664
+    c = random_csr(rng, rows=rows, cols=cols - 1, max_nnz=120, bits=bits)
+    small = rng.permutation(rows)[:int(share * rows)]
+    is_small = np.zeros(rows, dtype=bool)
+    is_small[small] = True
+    c["col_idx"][c["col_idx"] >= 7] += 1                              # gene 7: held by the small cells alone
+    at = np.repeat(np.arange(rows), np.diff(c["row_ptr"]))
+    keys = np.concatenate([at.astype(np.int64) * cols + c["col_idx"], small.astype(np.int64) * cols + 7])
+    order = np.argsort(keys)
+    values = np.concatenate([c["values"], rng.uniform(-2.0, 40.0, size=len(small)).astype(np.float32)])[order]
+    c.update(cols=cols, col_idx=(keys[order] % cols).astype(np.int32), values=values, row_ptr=np.searchsorted(keys[order], np.arange(rows + 1) * cols).astype(np.int64),
+             scales=np.append(c["scales"], np.float32(0.3)), offsets=np.append(c["offsets"], np.float32(-0.7)))
+    c = host_pack(oracle, c)
+    x = to_dev(c, cuda_device)
+    g_host = rng.normal(size=(rows, n)).astype(np.float32)
+    if column is None:
+        g_host[is_small] *= np.float32(2.0 ** -orders)
+    else:
+        g_host[np.ix_(is_small, np.arange(0, n, column))] *= np.float32(2.0 ** -orders)
+    g = torch.from_numpy(g_host).to(cuda_device)
+    # what a number's rounding is measured against: the cell's largest of sixteen neighbouring columns, or the number itself
+    reach = np.abs(g_host).astype(np.float64) if column is not None else np.repeat(np.abs(g_host).reshape(rows, n // 16, 16).max(2), 16, axis=1).astype(np.float64)
+    op = prepared(x, n, slices, cuda_device)
+    dec = oracle.unpack_csr(bits, 1, c["row_ptr"], c["packed_row_ptr"], c["col_idx"], c["scales"], c["offsets"], c["packed"]).astype(np.float64)
+    at, room = np.repeat(np.arange(rows), np.diff(c["row_ptr"])), op.workspace_bytes
+    for lo, hi, part in ((0, rows, 1.0), (0, rows, 0.8), (300, rows - 100, 1.0)):
+        op.workspace_bytes = int(room * part)
+        out = op.run(x, g, torch.full((cols, n), float("nan"), device=cuda_device), row_begin=lo, row_end=hi)
+        assert op.status() == 0
+        if part == 1.0 and lo == 0:
+            assert mode_of(op) == (from3 if slices == 3 else from4)
+        sel = (at >= lo) & (at < hi)
+        value, size = np.zeros((rows, cols)), np.zeros((rows, cols))
+        value[at[sel], c["col_idx"][sel]] = dec[sel]
+        size[at[sel], c["col_idx"][sel]] = np.abs(dec[sel]) + np.abs(c["offsets"][c["col_idx"][sel]])
+        want, scale = value.T @ g_host.astype(np.float64), size.T @ reach
+        # half a step: 1.02 * 2^(1 - 8 S) of a column's largest, which the launch's spread makes 2^-23 (from 4 digits) or 2^-18 (from 3) of `reach`; for a
+        # column by itself the mean over its numbers is bounded, and with a third of them small theirs by ten times that (1 / 0.3^2); the oracle's
+        # decoding and the roundings of up to eight runs at 2^-24 each
+        half = 1.02 * (2.0 ** -23 if slices == 4 else 2.0 ** -18) * (1.0 if column is None else 12.0)
+        assert np.all(np.abs(out.cpu().numpy() - want) <= (half + 10 * 2.0 ** -24) * scale + 1e-37), np.max(np.abs(out.cpu().numpy() - want) / (scale + 1e-37))
+    op.close()
+
+
+def test_more_genes_than_one_round_of_windows(cuda_device, oracle):
+    """The places of more than 98,304 genes' windows are added up in two rounds; prepared and with words made in the call."""
+    rng = np.random.default_rng(11)
+    rows, cols, n = 300, 120_000, 32
+    lengths = np.full(rows, 7200)
+    row_ptr = np.concatenate([[0], np.cumsum(lengths)]).astype(np.int64)
+    col_idx = np.concatenate([np.sort(rng.permutation(cols)[:k]) for k in lengths]).astype(np.int32)
+    c = host_pack(oracle, dict(rows=rows, cols=cols, bits=8, policy=1, row_ptr=row_ptr, col_idx=col_idx, scales=rng.uniform(0.01, 0.5, size=cols).astype(np.float32),
+                               offsets=rng.uniform(-1.0, 1.0, size=cols).astype(np.float32), values=rng.uniform(-2.0, 40.0, size=len(col_idx)).astype(np.float32)))
+    x = to_dev(c, cuda_device)
+    g, g_host = dense(rng, rows, n, torch.float32, cuda_device, std=1.0)
+    want, l1 = reference(oracle, c, g_host)
+    op = prepared(x, n, 4, cuda_device)
+    assert mode_of_run(op, x, g, cols) == (4, 1, False)
+    assert_within(op.run(x, g, torch.empty(cols, n, device=cuda_device)).cpu().numpy(), want, l1, g_host, 4)
+    op.close()
+    op = ops.PreparedSpmm(capi.PROJECTION_TRANSPOSE, rows, cols, n, x.nnz, 8, 1, torch.float32, cuda_device)
+    assert x.nnz >= 2_000_000 and mode_of_run(op, x, g, cols) == (4, 1, False)
+    assert_within(op.run(x, g, torch.empty(cols, n, device=cuda_device)).cpu().numpy(), want, l1, g_host, 4)
+    op.close()
+
+
+def mode_of_run(op, x, g, cols):
+    op.run(x, g, torch.empty(cols, g.shape[1], device=g.device))
+    assert op.status() == 0
+    return mode_of(op)
