@@ -210,7 +210,7 @@ cb200_status launch_qcsr_transpose_blocked(const qcsr_view &x, const dense_args 
 struct digit_layout {
     std::uint32_t *words = nullptr;
     std::uint32_t *bounds = nullptr; // [pieces][windows + 1], from the piece's base
-    std::int64_t *bases = nullptr;   // [pieces]; kDigitWordsTwice: a cell of the piece holds a gene more than once
+    std::int64_t *bases = nullptr;   // [pieces]; kDigitWordsTwice: a cell of the piece holds a gene more than once, and words are marked
     std::uint64_t bytes = 0;
     const void *src_row_ptr = nullptr, *src_col_idx = nullptr, *src_packed = nullptr; // arrays it was built from
 };

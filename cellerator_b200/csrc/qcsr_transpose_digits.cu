@@ -19,8 +19,7 @@
 //
 // Where G spreads too far for that (most_spread), the launch takes as many digits again, those behind the first ones, in a second pass over
 // the tiles: 62 bits (S = 4) or 46; where three digits are asked for, four in one pass come first.  A G that spreads further still, or holds
-// an infinity or a NaN, and a matrix in which a cell holds a gene twice, are taken entry by entry, in double precision and in a fixed order
-// (finish_kernel).  The device decides; nothing is read back.
+// an infinity or a NaN, is taken entry by entry, in double precision and in a fixed order (finish_kernel).  The device decides; nothing is read back.
 //
 // Data.  The entries lie in pieces of 32 cells; inside a piece they are ordered by window of 128 genes, one word per entry
 // {code, place in the operand tile}, cell after cell (digit_words_kernel: a CTA per piece counts the entries of each cell and window in
@@ -59,6 +58,7 @@ constexpr int kPieceRows = 32;                  // most cells whose words one CT
 constexpr int kBuildThreads = 768;
 constexpr int kBuildWarps = kBuildThreads / 32;
 constexpr std::uint32_t kPadding = 0x80000000u; // a word that holds no entry
+constexpr std::uint32_t kAgain = 0xc0000000u;   // added to a word whose place in the tile another entry has: a gene that its cell holds already
 
 constexpr int kMostGroupPieces = kRows / 16;
 constexpr int kProducerWarps = 16;
@@ -101,8 +101,9 @@ constexpr int kBlockColumns = 16; // columns whose largest number stands for a c
 __host__ __device__ constexpr int most_spread(int base, int slices, int passes) {
     return 8 * slices - (base == 4 ? 24 : 19) + (passes == 2 ? 8 * slices - 1 : 0);
 }
-// The launch's mode, a word in the workspace that its first kernels write: digits, passes over the tiles, or entry by entry.
-constexpr int kByEntry = 1 << 8;
+// The launch's mode, a word in the workspace that its first kernels write: digits, passes over the tiles, or entry by entry; whether there are
+// words with kAgain.
+constexpr int kByEntry = 1 << 8, kRepeats = 1 << 9;
 __host__ __device__ constexpr int mode_of(int slices, int passes) { return slices << 4 | passes; }
 __host__ __device__ constexpr int slices_of(int mode) { return mode >> 4 & 15; }
 __host__ __device__ constexpr int passes_of(int mode) { return mode & 15; }
@@ -137,8 +138,8 @@ constexpr std::int64_t kTwice = kDigitWordsTwice;
 // are of very different lengths: a warp per row took 240 us for 8,191 x 33,538 with 14.7 M entries, this takes 59).  Where genes ascend,
 // an entry starts a window if the one before it lies in another; from those starts follow the sizes, the places of the windows and
 // so the place of every entry, without an atomic, which the second pass computes from a look-up per entry.  A CTA that finds a gene
-// outside the matrix or not above the one before it counts and places entry by entry with atomics instead, and looks for genes that a cell
-// holds twice: a tile has one place for them.
+// outside the matrix or not above the one before it counts and places entry by entry with atomics instead, and marks the genes that a cell
+// holds already (kAgain): a tile has one place for them, and finish_kernel adds the others.
 //
 // What bounds it: the latency of the genes' loads (eight in flight per warp, 48 warps per SM) and issue, half of the slots.
 template<int BITS>
@@ -353,7 +354,10 @@ __global__ void __launch_bounds__(kBuildThreads, 2) digit_words_kernel(const wor
                 if (static_cast<int>(e) < 0) continue;
                 const std::uint32_t place = e >> 8;
                 const std::uint32_t gl = (place >> 7) & (kWin - 1), cell = (((place >> 4 ^ gl) & 7u) << 4 | (place & 15u)) & (kPieceRows - 1);
-                twice = twice || (atomicOr(seen + gl, 1u << cell) >> cell & 1u) != 0u;
+                if ((atomicOr(seen + gl, 1u << cell) >> cell & 1u) != 0u) {
+                    twice = true;
+                    out[i] = e | kAgain;
+                }
             }
             __syncwarp();
         }
@@ -430,13 +434,24 @@ __global__ void __launch_bounds__(1024) column_range_kernel(const float *g, std:
         }
         return bits;
     };
-    for (; r + 7 * step < row_end; r += 8 * step, at += 8 * step * ld) {
-        float v[8];
-        unsigned m[8];
+    float v[8]; // the next eight rows are on their way while eight are looked at
+    const auto load = [&]() {
 #pragma unroll
         for (int k = 0; k < 8; ++k) v[k] = from >= 0 ? __ldg(at + k * step * ld) : 0.0f;
+    };
+    bool eight = r + 7 * step < row_end;
+    if (eight) load();
+    while (eight) {
+        unsigned m[8];
+        float now[8];
 #pragma unroll
-        for (int k = 0; k < 8; ++k) m[k] = take(v[k]);
+        for (int k = 0; k < 8; ++k) now[k] = v[k];
+        r += 8 * step;
+        at += 8 * step * ld;
+        eight = r + 7 * step < row_end;
+        if (eight) load();
+#pragma unroll
+        for (int k = 0; k < 8; ++k) m[k] = take(now[k]);
         // eight rows over sixteen lanes: half of the rows stay with half of the lanes, three times, and two lanes have a row's halves
 #pragma unroll
         for (int d = 4; d > 0; d >>= 1) {
@@ -602,15 +617,18 @@ __global__ void __launch_bounds__(256) pack_digits_kernel(const pack_params p) {
             if (largest < 0x7f800000u)
                 atomicMax(&need_bits, static_cast<unsigned long long>(__double_as_longlong(static_cast<double>(__uint_as_float(largest)) / static_cast<double>(__uint_as_float(least_of[tid])))));
         }
+        int repeats = 0;
         if (blockIdx.x == 0) {
 #pragma unroll 8
-            for (std::int64_t k = tid; k < p.word_pieces; k += 256) by_entry |= (__ldcg(p.bases + k) & kTwice) != 0 ? 1 : 0;
+            for (std::int64_t k = tid; k < p.word_pieces; k += 256) repeats |= (__ldcg(p.bases + k) & kTwice) != 0 ? 1 : 0;
         }
         by_entry = __syncthreads_or(by_entry);
+        repeats = __syncthreads_or(repeats); // (the first block's: it writes the mode)
         const double need = __longlong_as_double(static_cast<long long>(need_bits));
         const auto serves = [&](int slices, int passes) { return need <= static_cast<double>(1ull << most_spread(BASE, slices, passes)); };
         mode = BASE == 3 && serves(3, 1) ? mode_of(3, 1) : serves(4, 1) ? mode_of(4, 1) : BASE == 3 && serves(3, 2) ? mode_of(3, 2) : mode_of(4, 2);
         if (by_entry != 0 || !serves(4, 2)) mode |= kByEntry;
+        if (repeats != 0) mode |= kRepeats;
         if (tid < p.padded) {
             const int bits = 8 * slices_of(mode) - 1;
             double f = 0.0, step = 0.0;
@@ -1062,20 +1080,102 @@ struct finish_params {
     float alpha, beta;
 };
 
-// G'[genes of one window, columns of one block] = beta * G' + alpha * (the sums of the set's runs, added in run order; EXACT: the totals).
-// Where a column's range is too wide for fixed point, or a scale or a zero-point of the window is not finite (0 * infinity, in a
-// product of sums, would reach cells that hold no entry): from the entries, in double precision.  A warp has every eighth or
-// sixteenth gene of the window to itself and walks the words in order, so this too has the same bits on every run.
-// A thread has a gene and sixteen columns, so that a warp's loads are contiguous.
 __host__ __device__ constexpr int finish_threads(int nb) { return nb / 16 * kWin; }
+constexpr int finish_smem_bytes(int nb) { return kWin * nb * 8 + kWin * (nb / 4) * 16; }
+// f(word, gene within the window, row), a word of the window to a lane and 32 at a time, for the warp's share of the pieces of the row range; where `marked`,
+// of those that hold genes again.  Lanes without a word of the range have kPadding.
+template<typename F>
+__device__ __forceinline__ void each_words(const finish_params &p, std::int64_t window, int share, int shares, bool marked, F &&f) {
+    const int lane = threadIdx.x & 31;
+    const std::int64_t piece1 = (p.row_end - p.first_row + p.d.piece_rows - 1) / p.d.piece_rows;
+    for (std::int64_t piece = (p.row_begin - p.first_row) / p.d.piece_rows + share; piece < piece1; piece += shares) {
+        const std::int64_t base = __ldcg(p.d.bases + piece);
+        if (marked && (base & kTwice) == 0) continue;
+        const std::uint32_t *at = p.d.bounds + piece * (p.d.windows + 1) + window;
+        const int words = static_cast<int>(__ldcg(at + 1) - __ldcg(at));
+        const std::uint32_t *w = p.d.words + (base & (kTwice - 1)) + __ldcg(at);
+        const std::int64_t group_row = p.first_row + piece / p.d.group_pieces * kRows;
+        for (int i0 = 0; i0 < words; i0 += 32) {
+            const std::uint32_t e = i0 + lane < words ? __ldcg(w + i0 + lane) : kPadding;
+            const int place = static_cast<int>((e >> 8) & 0x7fffu), gene = (place >> 7) & (kWin - 1);
+            const std::int64_t row = group_row + (place >> 14) * 128 + ((((place >> 4) & 7) ^ (gene & 7)) << 4) + (place & 15);
+            f(row >= p.row_begin && row < p.row_end ? e : kPadding, gene, row);
+        }
+    }
+}
+
+// What tiles do not hold, in values[gene][column].  by_entry: all of it, in double precision; a warp has every eighth or sixteenth gene to
+// itself and takes the words in order, so that the bits are the same on every run.  Otherwise the genes that their cells hold already, in
+// whole numbers (whole[gene][column of a quarter] {codes, ones}), whose order does not matter.
+template<int NB>
+__device__ __noinline__ void beside_tiles(const finish_params &p, int mode, bool by_entry, std::int64_t window, const float2 *meta, double *values,
+                                          unsigned long long *whole) {
+    constexpr int kFinish = finish_threads(NB), kWarps = kFinish / 32, kQuarter = NB / 4;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, c0 = static_cast<int>(blockIdx.y) * NB;
+    for (int i = tid; i < kWin * NB; i += kFinish) values[i] = 0.0;
+    __syncthreads();
+    if (by_entry) {
+        each_words(p, window, 0, 1, false, [&](std::uint32_t e, int gene, std::int64_t row) {
+            std::uint32_t todo = __ballot_sync(0xffffffffu, e != kPadding && gene % kWarps == warp);
+            while (todo != 0u) {
+                const int j = __ffs(todo) - 1;
+                todo &= todo - 1u;
+                const int code = static_cast<int>(static_cast<signed char>(__shfl_sync(0xffffffffu, e, j) & 0xffu)) + p.d.code_bias, gj = __shfl_sync(0xffffffffu, gene, j);
+                const std::int64_t rj = __shfl_sync(0xffffffffu, row, j);
+                const double value = static_cast<double>(fmaf(static_cast<float>(code), meta[gj].x, meta[gj].y));
+                for (int c = lane; c < NB; c += 32)
+                    if (c0 + c < p.n) values[gj * NB + c] += value * static_cast<double>(__ldg(p.g + rj * p.g_ld + c0 + c));
+            }
+        });
+        __syncthreads();
+        return;
+    }
+    if ((mode & kRepeats) == 0) return;
+    const double rest = slices_of(mode) == 3 ? second_step(3) : second_step(4);
+    for (int quarter = 0; quarter < 4; ++quarter)
+        for (int pass = 0; pass < passes_of(mode); ++pass) {
+            for (int i = tid; i < kWin * kQuarter * 2; i += kFinish) whole[i] = 0u;
+            __syncthreads();
+            each_words(p, window, warp, kWarps, true, [&](std::uint32_t e, int gene, std::int64_t row) {
+                std::uint32_t todo = __ballot_sync(0xffffffffu, e >= kAgain);
+                while (todo != 0u) {
+                    const int j = __ffs(todo) - 1;
+                    todo &= todo - 1u;
+                    const int code = static_cast<signed char>(__shfl_sync(0xffffffffu, e, j) & 0xffu), gj = __shfl_sync(0xffffffffu, gene, j);
+                    const std::int64_t rj = __shfl_sync(0xffffffffu, row, j);
+                    const int c = quarter * kQuarter + lane;
+                    if (lane < kQuarter && c0 + c < p.n) {
+                        const double step = __ldg(p.d.steps + c0 + c), scaled = step != 0.0 ? static_cast<double>(__ldg(p.g + rj * p.g_ld + c0 + c)) / step : 0.0;
+                        int q = __double2int_rn(scaled);
+                        if (pass != 0) q = __double2int_rn((scaled - static_cast<double>(q)) / rest);
+                        atomicAdd(whole + (gj * kQuarter + lane) * 2, static_cast<unsigned long long>(static_cast<long long>(code) * q));
+                        atomicAdd(whole + (gj * kQuarter + lane) * 2 + 1, static_cast<unsigned long long>(static_cast<long long>(q)));
+                    }
+                }
+            });
+            __syncthreads();
+            for (int i = tid; i < kWin * kQuarter; i += kFinish) {
+                const int gene = i / kQuarter, c = quarter * kQuarter + i % kQuarter;
+                values[gene * NB + c] += value_of(static_cast<long long>(whole[2 * i]), static_cast<long long>(whole[2 * i + 1]), p.d.code_bias, static_cast<double>(meta[gene].x),
+                                                  static_cast<double>(meta[gene].y), __ldg(p.d.steps + pass * p.d.column_blocks * NB + c0 + c));
+            }
+            __syncthreads();
+        }
+}
+
+// G'[genes of one window, columns of one block] = beta * G' + alpha * (the sums of the set's runs, added in run order; EXACT: the totals).
+// Genes that a cell holds again (kAgain) are added here.  Where G spreads too far for fixed point, or a scale or a zero-point of the window is not
+// finite (0 * infinity, in a product of sums, would reach cells that hold no entry): everything, entry by entry (beside_tiles, which is no part
+// of this function's registers: two CTAs of 512 threads to an SM, or the 262 of 33,538 genes take two rounds, 12 us instead of 9).
+// A thread has a gene and sixteen columns, so that a warp's loads are contiguous.
 template<int NB, bool EXACT>
-__global__ void __launch_bounds__(finish_threads(NB)) finish_kernel(const finish_params p) {
-    extern __shared__ double slow_sums[]; // [kWin][NB]
-    constexpr int kSet = set_windows(NB, kMostSlices), kFinish = finish_threads(NB);
+__global__ void __launch_bounds__(finish_threads(NB), 1024 / finish_threads(NB)) finish_kernel(const __grid_constant__ finish_params p) {
+    extern __shared__ double beside[]; // [kWin][NB], and behind it [kWin][NB / 4] {codes, ones}
+    constexpr int kSet = set_windows(NB, kMostSlices);
     static_assert(kSet == set_windows(NB, 3), "the sets of a launch do not follow from its mode");
     __shared__ float2 meta[kWin];
     wait_for_previous_launch();
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x;
     const std::int64_t sets = p.d.set_count;
     const int wl = static_cast<int>(blockIdx.x % kSet);
     const std::int64_t set = blockIdx.x / kSet, window = (p.d.first_set + set) * kSet + wl;
@@ -1090,87 +1190,58 @@ __global__ void __launch_bounds__(finish_threads(NB)) finish_kernel(const finish
         odd = isfinite(so.x) && isfinite(so.y) ? 0 : 1;
     }
     const int mode = __ldcg(p.d.mode);
-    const bool slow = __syncthreads_or(odd) != 0 || (mode & kByEntry) != 0;
-    if (slow) {
-        for (int i = tid; i < kWin * NB; i += kFinish) slow_sums[i] = 0.0;
-        __syncthreads();
-        const std::int64_t piece0 = (p.row_begin - p.first_row) / p.d.piece_rows, piece1 = (p.row_end - p.first_row + p.d.piece_rows - 1) / p.d.piece_rows;
-        for (std::int64_t piece = piece0; piece < piece1; ++piece) {
-            const std::uint32_t *at = p.d.bounds + piece * (p.d.windows + 1) + window;
-            const int words = static_cast<int>(__ldcg(at + 1) - __ldcg(at));
-            const std::uint32_t *w = p.d.words + (__ldcg(p.d.bases + piece) & (kTwice - 1)) + __ldcg(at);
-            const std::int64_t group_row = p.first_row + piece / p.d.group_pieces * kRows;
-            for (int i0 = 0; i0 < words; i0 += 32) {
-                const std::uint32_t e = i0 + lane < words ? __ldcg(w + i0 + lane) : kPadding;
-                const int place = static_cast<int>((e >> 8) & 0x7fffu), gl = (place >> 7) & (kWin - 1);
-                const int cell = (place >> 14) * 128 + ((((place >> 4) & 7) ^ (gl & 7)) << 4) + (place & 15);
-                const std::int64_t row = group_row + cell;
-                std::uint32_t todo = __ballot_sync(0xffffffffu, static_cast<int>(e) >= 0 && gl % (kFinish / 32) == warp && row >= p.row_begin && row < p.row_end);
-                while (todo != 0u) {
-                    const int j = __ffs(todo) - 1;
-                    todo &= todo - 1u;
-                    const std::uint32_t ej = __shfl_sync(0xffffffffu, e, j);
-                    const int gj = __shfl_sync(0xffffffffu, gl, j);
-                    const std::int64_t rj = group_row + __shfl_sync(0xffffffffu, cell, j);
-                    const int code = static_cast<int>(static_cast<signed char>(ej & 0xffu)) + p.d.code_bias;
-                    const double value = static_cast<double>(fmaf(static_cast<float>(code), meta[gj].x, meta[gj].y));
-                    for (int c = lane; c < NB; c += 32)
-                        if (c0 + c < p.n) slow_sums[gj * NB + c] += value * static_cast<double>(__ldg(p.g + rj * p.g_ld + c0 + c));
-                }
-            }
-        }
-        __syncthreads();
-    }
+    const bool by_entry = __syncthreads_or(odd) != 0 || (mode & kByEntry) != 0, more = by_entry || (mode & kRepeats) != 0;
+    if (more) beside_tiles<NB>(p, mode, by_entry, window, meta, beside, reinterpret_cast<unsigned long long *>(beside + kWin * NB));
+    const int passes = passes_of(mode), c = tid / kWin * 16;
     // the set's slots: the CTAs whose shares meet its runs, run after run, pass after pass
-    const int passes = passes_of(mode);
     const std::int64_t total = sets * p.d.column_blocks * p.d.group_count * passes, L = p.d.group_count, cuts = (L + p.d.run_groups - 1) / p.d.run_groups;
     const int gl = tid & (kWin - 1);
     const std::int64_t gene = window * kWin + gl;
-    const int c = tid / kWin * 16;
     if (gene >= p.d.cols || c0 + c >= p.n) return;
-    float v[16];
-    if (slow) {
+    double sum[16];
 #pragma unroll
-        for (int k = 0; k < 16; ++k) v[k] = static_cast<float>(slow_sums[gl * NB + c + k]);
-    } else if constexpr (EXACT) {
-        const double scale = static_cast<double>(meta[gl].x), offset = static_cast<double>(meta[gl].y);
-        double sum[16];
+    for (int k = 0; k < 16; ++k) sum[k] = 0.0;
+    if (more) {
 #pragma unroll
-        for (int k = 0; k < 16; ++k) sum[k] = 0.0;
+        for (int k = 0; k < 16; ++k) sum[k] = beside[gl * NB + c + k];
+    }
+    if (!by_entry) {
         for (int pass = 0; pass < passes; ++pass) {
-            const std::int64_t block = static_cast<std::int64_t>(pass) * p.d.column_blocks + blockIdx.y;
-            const long long *total = p.d.totals + (((block * sets + set) * kSet + wl) * 2 * NB + c) * kWin + gl;
-            const double *steps = p.d.steps + block * NB + c;
-            long long coded[16], present[16];
+            const std::int64_t block = static_cast<std::int64_t>(pass) * p.d.column_blocks + blockIdx.y, set_of_all = block * sets + set;
+            if constexpr (EXACT) {
+                const double scale = static_cast<double>(meta[gl].x), offset = static_cast<double>(meta[gl].y);
+                const long long *at = p.d.totals + ((set_of_all * kSet + wl) * 2 * NB + c) * kWin + gl;
+                const double *steps = p.d.steps + block * NB + c;
 #pragma unroll
-            for (int k = 0; k < 16; ++k) {
-                coded[k] = __ldcg(total + k * kWin);
-                present[k] = __ldcg(total + (NB + k) * kWin);
-            }
+                for (int h = 0; h < 16; h += 8) {
+                    long long coded[8], present[8];
 #pragma unroll
-            for (int k = 0; k < 16; ++k) sum[k] += value_of(coded[k], present[k], p.d.code_bias, scale, offset, __ldg(steps + k));
-        }
+                    for (int k = 0; k < 8; ++k) {
+                        coded[k] = __ldcg(at + (h + k) * kWin);
+                        present[k] = __ldcg(at + (NB + h + k) * kWin);
+                    }
 #pragma unroll
-        for (int k = 0; k < 16; ++k) v[k] = static_cast<float>(sum[k]);
-    } else {
+                    for (int k = 0; k < 8; ++k) sum[h + k] += value_of(coded[k], present[k], p.d.code_bias, scale, offset, __ldg(steps + h + k));
+                }
+            } else {
+                for (std::int64_t cut = 0; cut < cuts; ++cut) {
+                    const std::int64_t from = set_of_all * L + cut * p.d.run_groups, to = min(from + p.d.run_groups, (set_of_all + 1) * L);
+                    const std::int64_t last = cta_of(to - 1, total, p.grid);
+                    for (std::int64_t b = cta_of(from, total, p.grid); b <= last; ++b) {
+                        const float *slot = p.d.partials + (((set_of_all * cuts + cut + b) * kSet + wl) * NB + c) * kWin + gl;
+                        float u[16];
 #pragma unroll
-        for (int k = 0; k < 16; ++k) v[k] = 0.0f;
-        for (int pass = 0; pass < passes; ++pass) {
-            const std::int64_t set_of_all = (static_cast<std::int64_t>(pass) * p.d.column_blocks + blockIdx.y) * sets + set;
-            for (std::int64_t cut = 0; cut < cuts; ++cut) {
-                const std::int64_t from = set_of_all * L + cut * p.d.run_groups, to = min(from + p.d.run_groups, (set_of_all + 1) * L);
-                const std::int64_t last = cta_of(to - 1, total, p.grid);
-                for (std::int64_t b = cta_of(from, total, p.grid); b <= last; ++b) {
-                    const float *slot = p.d.partials + (((set_of_all * cuts + cut + b) * kSet + wl) * NB + c) * kWin + gl;
-                    float u[16];
+                        for (int k = 0; k < 16; ++k) u[k] = __ldcg(slot + k * kWin);
 #pragma unroll
-                    for (int k = 0; k < 16; ++k) u[k] = __ldcg(slot + k * kWin);
-#pragma unroll
-                    for (int k = 0; k < 16; ++k) v[k] += u[k];
+                        for (int k = 0; k < 16; ++k) sum[k] += static_cast<double>(u[k]);
+                    }
                 }
             }
         }
     }
+    float v[16];
+#pragma unroll
+    for (int k = 0; k < 16; ++k) v[k] = static_cast<float>(sum[k]);
     float *dst = p.out + gene * p.out_ld + c0 + c;
     if (p.out_vector != 0) {
 #pragma unroll
@@ -1251,11 +1322,11 @@ template<int NB, int BASE, bool EXACT>
 cb200_status launch_digits(const digit_launch &l, int sm_count, cudaStream_t stream) {
     constexpr std::size_t smem = std::max(digits_smem_bytes<NB, BASE>(), digits_smem_bytes<NB, kMostSlices>());
     static_assert(smem <= 232448, "shared memory budget");
-    constexpr int slow_smem = kWin * NB * 8, kSet = set_windows(NB, kMostSlices);
+    constexpr int finish_smem = finish_smem_bytes(NB), kSet = set_windows(NB, kMostSlices);
     const auto main_kernel = qcsr_transpose_digits_kernel<NB, BASE, EXACT>;
     const auto finish = finish_kernel<NB, EXACT>;
     CB200_CUDA_OK(cudaFuncSetAttribute(main_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-    CB200_CUDA_OK(cudaFuncSetAttribute(finish, cudaFuncAttributeMaxDynamicSharedMemorySize, slow_smem));
+    CB200_CUDA_OK(cudaFuncSetAttribute(finish, cudaFuncAttributeMaxDynamicSharedMemorySize, finish_smem));
     const int n = l.finish.n;
     CB200_CUDA_OK(launch_kernel(l.early, column_range_kernel, dim3(kParts), 1024, 0, stream, l.finish.g, l.finish.g_ld, n, l.pack.padded, l.finish.row_begin, l.finish.row_end,
                                 const_cast<unsigned *>(l.pack.part_max), const_cast<double2 *>(l.pack.part_sum), const_cast<unsigned *>(l.pack.part_least),
@@ -1273,7 +1344,7 @@ cb200_status launch_digits(const digit_launch &l, int sm_count, cudaStream_t str
             f.d = m;
             f.grid = grid;
             count_launch();
-            return launch_kernel(true, finish, dim3(static_cast<unsigned>(m.set_count * kSet), static_cast<unsigned>(m.column_blocks)), finish_threads(NB), slow_smem, stream, f);
+            return launch_kernel(true, finish, dim3(static_cast<unsigned>(m.set_count * kSet), static_cast<unsigned>(m.column_blocks)), finish_threads(NB), finish_smem, stream, f);
         };
         for (std::int64_t begin = l.main.group_begin; begin < group_end; begin += l.slice) {
             m.group_begin = begin;

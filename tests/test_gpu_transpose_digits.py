@@ -290,3 +290,47 @@ def mode_of_run(op, x, g, cols):
     op.run(x, g, torch.empty(cols, g.shape[1], device=g.device))
     assert op.status() == 0
     return mode_of(op)
+
+
+@pytest.mark.parametrize("slices,n,bits,outlier", [(3, 64, 8, 1.0), (3, 32, 4, 1e6), (4, 64, 8, 1e6), (4, 32, 8, 1.0), (4, 128, 4, 1.0), (0, 50, 8, 1.0), (0, 130, 4, 1e6)])
+def test_a_gene_held_again_changes_no_others(cuda_device, oracle, slices, n, bits, outlier):
+    """A cell that holds genes twice and three times, one that holds a gene a hundred times: these genes count as often, and all others keep the bits that they have without
+    them.  0 digits: the words made in the call."""
+    rng = np.random.default_rng(n)
+    rows, cols = (2111, 1500) if slices == 0 else (256 * 20, 1664)
+    c = random_csr(rng, rows=rows, cols=cols, max_nnz=3000 if slices == 0 else 200, bits=bits)
+    again = {77: [100, 101, 101, 600], rows - 1: [5], 256 * 3 + 31: [1400] * 100}
+    keys = np.repeat(np.arange(rows), np.diff(c["row_ptr"])).astype(np.int64) * cols + c["col_idx"]
+    keep = np.isin(keys, [r * cols + g for r, genes in again.items() for g in genes], invert=True)
+    keys, values = keys[keep], c["values"][keep]
+    once = np.array([r * cols + g for r, genes in again.items() for g in sorted(set(genes))])
+    more = np.array([r * cols + g for r, genes in again.items() for g in genes])
+
+    def matrix(extra):
+        all_keys = np.concatenate([keys, extra])
+        order = np.argsort(all_keys, kind="stable")
+        k = all_keys[order]
+        v = np.concatenate([values, np.linspace(1.0, 30.0, len(extra), dtype=np.float32)])[order]
+        return host_pack(oracle, dict(c, row_ptr=np.searchsorted(k, np.arange(rows + 1) * cols).astype(np.int64), col_idx=(k % cols).astype(np.int32), values=v))
+
+    g_host = rng.normal(size=(rows, n)).astype(np.float32)
+    g_host[9, n - 1] = outlier
+    g = torch.from_numpy(g_host).to(cuda_device)
+    outs = []
+    for m in (matrix(once), matrix(np.concatenate([once, more])), matrix(np.concatenate([once, more]))):
+        x = to_dev(m, cuda_device)
+        op = prepared(x, n, slices, cuda_device) if slices else ops.PreparedSpmm(capi.PROJECTION_TRANSPOSE, rows, cols, n, x.nnz, bits, 1, torch.float32, cuda_device)
+        out = op.run(x, g, torch.full((cols, n), float("nan"), device=cuda_device))
+        assert op.status() == 0 and not mode_of(op)[2] and (outlier == 1.0) == (mode_of(op)[1] == 1)
+        outs.append(out.cpu().numpy())
+        op.close()
+    held = sorted({g for genes in again.values() for g in genes})
+    others = np.delete(np.arange(cols), held)
+    assert np.array_equal(outs[0][others], outs[1][others]) and np.array_equal(outs[1], outs[2])
+    dec = oracle.unpack_csr(bits, 1, m["row_ptr"], m["packed_row_ptr"], m["col_idx"], m["scales"], m["offsets"], m["packed"]).astype(np.float64)
+    at = np.repeat(np.arange(rows), np.diff(m["row_ptr"]))
+    for gene in held:
+        sel = m["col_idx"] == gene
+        want, size = dec[sel] @ g_host[at[sel]].astype(np.float64), (np.abs(dec[sel]) + abs(m["offsets"][gene])).sum() * np.abs(g_host).max(0)
+        # as in assert_within, two passes as four digits at least
+        assert np.all(np.abs(outs[1][gene] - want) <= (1.02 * 2.0 ** (1 - 8 * (3 if slices == 3 else 4)) + 10 * 2.0 ** -24) * size), gene
