@@ -18,8 +18,9 @@
 // cells, in a fixed order); S = 3 3e-7, where products put together from three bf16 products and summed by the fp32 MMAs leave 6.2e-6.
 //
 // Where G spreads too far for that (most_spread), the launch takes as many digits again, those behind the first ones, in a second pass over
-// the tiles: 62 bits (S = 4) or 46; where three digits are asked for, four in one pass come first.  A G that spreads further still, or holds
-// an infinity or a NaN, is taken entry by entry, in double precision and in a fixed order (finish_kernel).  The device decides; nothing is read back.
+// the tiles: 62 bits (S = 4) or 46; where three digits are asked for, four in one pass come first.  A G that spreads further still is taken entry
+// by entry, in double precision and in a fixed order (beside_tiles).  Infinities and NaNs are zeroes in the digits; the last kernel finds the
+// entries of their cells and what they make of these genes' sums.  The device decides; nothing is read back.
 //
 // Data.  The entries lie in pieces of 32 cells; inside a piece they are ordered by window of 128 genes, one word per entry
 // {code, place in the operand tile}, cell after cell (digit_words_kernel: a CTA per piece counts the entries of each cell and window in
@@ -43,6 +44,7 @@
 #include "sm100_primitives.cuh"
 
 #include <algorithm>
+#include <math_constants.h>
 
 namespace cb200 {
 
@@ -102,8 +104,8 @@ __host__ __device__ constexpr int most_spread(int base, int slices, int passes) 
     return 8 * slices - (base == 4 ? 24 : 19) + (passes == 2 ? 8 * slices - 1 : 0);
 }
 // The launch's mode, a word in the workspace that its first kernels write: digits, passes over the tiles, or entry by entry; whether there are
-// words with kAgain.
-constexpr int kByEntry = 1 << 8, kRepeats = 1 << 9;
+// words with kAgain; whether G holds infinities or NaNs.
+constexpr int kByEntry = 1 << 8, kRepeats = 1 << 9, kNonFinite = 1 << 10;
 __host__ __device__ constexpr int mode_of(int slices, int passes) { return slices << 4 | passes; }
 __host__ __device__ constexpr int slices_of(int mode) { return mode >> 4 & 15; }
 __host__ __device__ constexpr int passes_of(int mode) { return mode & 15; }
@@ -406,7 +408,7 @@ __global__ void __launch_bounds__(kBuildThreads, 2) digit_words_kernel(const wor
 
 // ---- G in digits -----------------------------------------------------------------------------------------------------------
 
-// Of each column the largest magnitude (as bits; an infinity or a NaN is the largest) and, over the numbers that are not zero, the sum of 1 /
+// Of each column the largest finite magnitude (as bits; the top bit: there is an infinity or a NaN too) and, over the finite numbers that are not zero, the sum of 1 /
 // sqrt(magnitude) and their number; of each sixteen columns (the last sixteen for a rest of them) the smallest row maximum that is not
 // zero, as bits; in kParts parts.  HBM or L2.
 __global__ void __launch_bounds__(1024) column_range_kernel(const float *g, std::int64_t ld, int n, int padded, std::int64_t row_begin, std::int64_t row_end,
@@ -418,13 +420,17 @@ __global__ void __launch_bounds__(1024) column_range_kernel(const float *g, std:
     const int c = threadIdx.x % padded, lanes = 1024 / padded;
     // behind the last column of its sixteen a lane has one of the sixteen before
     const int from = c < n ? c : c / kBlockColumns * kBlockColumns < n && c >= kBlockColumns ? c - kBlockColumns : -1;
-    unsigned most = 0u, count = 0u, least = 0xffffffffu;
+    unsigned most = 0u, count = 0u, least = 0xffffffffu, odd = 0u;
     float inverse = 0.0f;
     const std::int64_t step = static_cast<std::int64_t>(gridDim.x) * lanes;
     std::int64_t r = row_begin + static_cast<std::int64_t>(blockIdx.x) * lanes + threadIdx.x / padded; // the same in a warp
     const float *at = g + r * ld + from;
     const auto take = [&](float v) {
-        const unsigned bits = __float_as_uint(v) & 0x7fffffffu;
+        unsigned bits = __float_as_uint(v) & 0x7fffffffu;
+        if (bits >= 0x7f800000u) {
+            odd |= c < n ? 0x80000000u : 0u;
+            bits = 0u;
+        }
         if (c < n) {
             most = max(most, bits);
             if (bits != 0u) {
@@ -473,7 +479,7 @@ __global__ void __launch_bounds__(1024) column_range_kernel(const float *g, std:
     }
 #pragma unroll
     for (int d = 8; d > 0; d >>= 1) least = min(least, __shfl_xor_sync(0xffffffffu, least, d));
-    most_of[threadIdx.x] = most;
+    most_of[threadIdx.x] = most | odd;
     least_of[threadIdx.x] = least;
     count_of[threadIdx.x] = count;
     inverse_of[threadIdx.x] = inverse;
@@ -481,12 +487,13 @@ __global__ void __launch_bounds__(1024) column_range_kernel(const float *g, std:
     if (threadIdx.x < static_cast<unsigned>(padded)) {
         double sum = static_cast<double>(inverse), number = static_cast<double>(count);
         for (int k = 1; k < lanes; ++k) {
-            most = max(most, most_of[threadIdx.x + k * padded]);
+            odd |= most_of[threadIdx.x + k * padded] & 0x80000000u;
+            most = max(most, most_of[threadIdx.x + k * padded] & 0x7fffffffu);
             least = min(least, least_of[threadIdx.x + k * padded]);
             sum += static_cast<double>(inverse_of[threadIdx.x + k * padded]);
             number += static_cast<double>(count_of[threadIdx.x + k * padded]);
         }
-        part_max[blockIdx.x * kMaxColumns + threadIdx.x] = most;
+        part_max[blockIdx.x * kMaxColumns + threadIdx.x] = most | odd;
         part_sum[blockIdx.x * kMaxColumns + threadIdx.x] = make_double2(sum, number);
         if (threadIdx.x % kBlockColumns == 0u) part_least[(blockIdx.x * kMaxColumns + threadIdx.x) / kBlockColumns] = least;
     }
@@ -511,15 +518,18 @@ struct pack_params {
     int *mode;
     uint4 *totals;            // the totals to clear, 16 bytes each, of one pass
     std::int64_t total_items;
+    unsigned short *odd_rows; // [16 cells][32 columns]: which of the cells have an infinity or a NaN there; written if there is one at all
 };
 // the second pass takes up what the first rounds off, at most half a step
 __host__ __device__ constexpr double second_step(int slices) { return 1.0 / static_cast<double>(1ull << (8 * slices - 1)); }
 
+__host__ __device__ constexpr int odd_chunks(int n) { return n <= 32 ? 1 : (n + 63) / 64 * 2; } // of 32 columns, in blocks of NB
+
 // factor: 2^k, what a column is multiplied by
 template<int NB, int SLICES>
-__device__ __forceinline__ void pack_records(const pack_params &p, int passes, const double *factor) {
+__device__ __forceinline__ void pack_records(const pack_params &p, int mode, const double *factor) {
     constexpr int NC = mma_columns(NB, SLICES);
-    const int tid = threadIdx.x;
+    const int tid = threadIdx.x, passes = passes_of(mode);
     const std::int64_t pieces = static_cast<std::int64_t>((p.n + NB - 1) / NB) * p.groups * kGPieces;
     for (std::int64_t b = blockIdx.x; b < passes * pieces; b += gridDim.x) {
         const bool second = b >= pieces;
@@ -534,6 +544,18 @@ __device__ __forceinline__ void pack_records(const pack_params &p, int passes, c
             for (int j = 0; j < 16; ++j) {
                 const std::int64_t row = row0 + r16 * 16 + j;
                 v[j] = row >= p.row_begin && row < p.row_end && c0 + c < p.n ? __ldg(p.g + row * p.ld + c0 + c) : 0.0f;
+            }
+            if ((mode & kNonFinite) != 0) { // (a warp has 32 columns of sixteen cells)
+                unsigned odd = 0u;
+#pragma unroll
+                for (int j = 0; j < 16; ++j) {
+                    if (isfinite(v[j])) continue;
+                    odd |= 1u << j;
+                    v[j] = 0.0f;
+                }
+                odd = __reduce_or_sync(0xffffffffu, odd);
+                if (!second && (tid & 31) == 0)
+                    p.odd_rows[(b % (p.groups * kGPieces) * (kGPieceRows / 16) + r16) * odd_chunks(p.n) + (c0 + c) / 32] = static_cast<unsigned short>(odd);
             }
             std::uint32_t digit[SLICES][4];
 #pragma unroll
@@ -577,7 +599,7 @@ __global__ void __launch_bounds__(256) pack_digits_kernel(const pack_params p) {
     int mode;
     {
         const int c = tid % p.padded, lanes = 256 / p.padded, blocks = p.padded / kBlockColumns;
-        unsigned most = 0u;
+        unsigned most = 0u, odd = 0u;
         double2 sum = make_double2(0.0, 0.0);
         for (int k0 = tid / p.padded; k0 < kParts; k0 += 6 * lanes) { // lanes 1, 2, 4, 8: six loads of each kind in flight
             unsigned m[6];
@@ -589,7 +611,8 @@ __global__ void __launch_bounds__(256) pack_digits_kernel(const pack_params p) {
             }
 #pragma unroll
             for (int k = 0; k < 6; ++k) {
-                most = max(most, m[k]);
+                odd |= m[k] & 0x80000000u;
+                most = max(most, m[k] & 0x7fffffffu);
                 sum.x += q[k].x;
                 sum.y += q[k].y;
             }
@@ -598,41 +621,39 @@ __global__ void __launch_bounds__(256) pack_digits_kernel(const pack_params p) {
         most_of[tid] = most;
         sum_of[tid] = sum;
         __syncthreads();
-        int by_entry = 0;
         if (tid < p.padded) {
             for (int k = 1; k < lanes; ++k) {
                 most = max(most, most_of[tid + k * p.padded]);
                 sum.x += sum_of[tid + k * p.padded].x;
                 sum.y += sum_of[tid + k * p.padded].y;
             }
-            if (most >= 0x7f800000u) by_entry = 1;
-            else if (most != 0u) atomicMax(&need_bits, static_cast<unsigned long long>(__double_as_longlong(static_cast<double>(__uint_as_float(most)) * sum.x * sum.x / (2.0 * sum.y * sum.y))));
+            if (most != 0u) atomicMax(&need_bits, static_cast<unsigned long long>(__double_as_longlong(static_cast<double>(__uint_as_float(most)) * sum.x * sum.x / (2.0 * sum.y * sum.y))));
         }
         __syncthreads();
         if (tid < p.padded) most_of[tid] = most; // the columns'
         __syncthreads();
-        if (tid < blocks && tid * kBlockColumns < p.n && least_of[tid] < 0x7f800000u) {
+        if (tid < blocks && tid * kBlockColumns < p.n && least_of[tid] != 0xffffffffu) {
             unsigned largest = 0u;
             for (int k = max(0, min(tid * kBlockColumns, p.n - kBlockColumns)); k < min((tid + 1) * kBlockColumns, p.n); ++k) largest = max(largest, most_of[k]);
-            if (largest < 0x7f800000u)
-                atomicMax(&need_bits, static_cast<unsigned long long>(__double_as_longlong(static_cast<double>(__uint_as_float(largest)) / static_cast<double>(__uint_as_float(least_of[tid])))));
+            atomicMax(&need_bits, static_cast<unsigned long long>(__double_as_longlong(static_cast<double>(__uint_as_float(largest)) / static_cast<double>(__uint_as_float(least_of[tid])))));
         }
         int repeats = 0;
         if (blockIdx.x == 0) {
 #pragma unroll 8
             for (std::int64_t k = tid; k < p.word_pieces; k += 256) repeats |= (__ldcg(p.bases + k) & kTwice) != 0 ? 1 : 0;
         }
-        by_entry = __syncthreads_or(by_entry);
+        const int non_finite = __syncthreads_or(odd != 0u ? 1 : 0);
         repeats = __syncthreads_or(repeats); // (the first block's: it writes the mode)
         const double need = __longlong_as_double(static_cast<long long>(need_bits));
         const auto serves = [&](int slices, int passes) { return need <= static_cast<double>(1ull << most_spread(BASE, slices, passes)); };
         mode = BASE == 3 && serves(3, 1) ? mode_of(3, 1) : serves(4, 1) ? mode_of(4, 1) : BASE == 3 && serves(3, 2) ? mode_of(3, 2) : mode_of(4, 2);
-        if (by_entry != 0 || !serves(4, 2)) mode |= kByEntry;
+        if (!serves(4, 2)) mode |= kByEntry;
+        if (non_finite != 0) mode |= kNonFinite;
         if (repeats != 0) mode |= kRepeats;
         if (tid < p.padded) {
             const int bits = 8 * slices_of(mode) - 1;
             double f = 0.0, step = 0.0;
-            if (most != 0u && most < 0x7f800000u) {
+            if (most != 0u) {
                 // largest = m 2^e, m in [0.5, 1); the largest number of S balanced digits is 0.996 * 2^(8 S - 1)
                 const int e = most >= 0x800000u ? static_cast<int>(most >> 23) - 126 : 32 - __clz(most) - 149;
                 const int k = bits - e - ((most & 0x7fffffu) > 8220000u || most < 0x800000u ? 1 : 0);
@@ -650,8 +671,8 @@ __global__ void __launch_bounds__(256) pack_digits_kernel(const pack_params p) {
         __syncthreads();
     }
     for (std::int64_t i = blockIdx.x * 256 + tid; i < passes_of(mode) * p.total_items; i += gridDim.x * 256) p.totals[i] = make_uint4(0u, 0u, 0u, 0u);
-    if (BASE == 3 && slices_of(mode) == 3) pack_records<NB, 3>(p, passes_of(mode), factor);
-    else pack_records<NB, 4>(p, passes_of(mode), factor);
+    if (BASE == 3 && slices_of(mode) == 3) pack_records<NB, 3>(p, mode, factor);
+    else pack_records<NB, 4>(p, mode, factor);
 }
 
 // ---- the sums --------------------------------------------------------------------------------------------------------------
@@ -1073,6 +1094,8 @@ struct finish_params {
     digit_params d;
     const float *g;
     std::int64_t g_ld, first_row, row_begin, row_end; // row_begin, row_end: of the launch; first_row: of the words
+    const unsigned short *odd_rows; // from the first group of the call
+    std::int64_t odd_from;          // its first row
     float *out;
     std::int64_t out_ld;
     std::int64_t grid; // CTAs of the main kernel
@@ -1082,15 +1105,15 @@ struct finish_params {
 
 __host__ __device__ constexpr int finish_threads(int nb) { return nb / 16 * kWin; }
 constexpr int finish_smem_bytes(int nb) { return kWin * nb * 8 + kWin * (nb / 4) * 16; }
-// f(word, gene within the window, row), a word of the window to a lane and 32 at a time, for the warp's share of the pieces of the row range; where `marked`,
-// of those that hold genes again.  Lanes without a word of the range have kPadding.
-template<typename F>
-__device__ __forceinline__ void each_words(const finish_params &p, std::int64_t window, int share, int shares, bool marked, F &&f) {
+// f(word, gene within the window, row), a word of the window to a lane and 32 at a time, for the warp's share of the pieces of the row range that
+// wanted(first row, base) lets through.  Lanes without a word of the range have kPadding.
+template<typename W, typename F>
+__device__ __forceinline__ void each_words(const finish_params &p, std::int64_t window, int share, int shares, W &&wanted, F &&f) {
     const int lane = threadIdx.x & 31;
     const std::int64_t piece1 = (p.row_end - p.first_row + p.d.piece_rows - 1) / p.d.piece_rows;
     for (std::int64_t piece = (p.row_begin - p.first_row) / p.d.piece_rows + share; piece < piece1; piece += shares) {
         const std::int64_t base = __ldcg(p.d.bases + piece);
-        if (marked && (base & kTwice) == 0) continue;
+        if (!wanted(p.first_row + piece * p.d.piece_rows, base)) continue;
         const std::uint32_t *at = p.d.bounds + piece * (p.d.windows + 1) + window;
         const int words = static_cast<int>(__ldcg(at + 1) - __ldcg(at));
         const std::uint32_t *w = p.d.words + (base & (kTwice - 1)) + __ldcg(at);
@@ -1106,7 +1129,8 @@ __device__ __forceinline__ void each_words(const finish_params &p, std::int64_t 
 
 // What tiles do not hold, in values[gene][column].  by_entry: all of it, in double precision; a warp has every eighth or sixteenth gene to
 // itself and takes the words in order, so that the bits are the same on every run.  Otherwise the genes that their cells hold already, in
-// whole numbers (whole[gene][column of a quarter] {codes, ones}), whose order does not matter.
+// whole numbers (whole[gene][column of a quarter] {codes, ones}), and what infinities and NaNs of G come to (flags[gene][column]: 1, 2, 4 for
+// a product of +infinity, of -infinity, or neither); the order of neither matters.
 template<int NB>
 __device__ __noinline__ void beside_tiles(const finish_params &p, int mode, bool by_entry, std::int64_t window, const float2 *meta, double *values,
                                           unsigned long long *whole) {
@@ -1115,7 +1139,7 @@ __device__ __noinline__ void beside_tiles(const finish_params &p, int mode, bool
     for (int i = tid; i < kWin * NB; i += kFinish) values[i] = 0.0;
     __syncthreads();
     if (by_entry) {
-        each_words(p, window, 0, 1, false, [&](std::uint32_t e, int gene, std::int64_t row) {
+        each_words(p, window, 0, 1, [](std::int64_t, std::int64_t) { return true; }, [&](std::uint32_t e, int gene, std::int64_t row) {
             std::uint32_t todo = __ballot_sync(0xffffffffu, e != kPadding && gene % kWarps == warp);
             while (todo != 0u) {
                 const int j = __ffs(todo) - 1;
@@ -1130,13 +1154,56 @@ __device__ __noinline__ void beside_tiles(const finish_params &p, int mode, bool
         __syncthreads();
         return;
     }
+    if ((mode & kNonFinite) != 0) {
+        static_assert(kWin * NB * sizeof(int) <= kWin * kQuarter * 16, "shares the memory");
+        __shared__ unsigned settled[kWin / 32]; // genes whose sums are NaN in every column: nothing changes them any more
+        int *flags = reinterpret_cast<int *>(whole);
+        for (int i = tid; i < kWin * NB; i += kFinish) flags[i] = 0;
+        if (tid < kWin / 32) settled[tid] = 0u;
+        __syncthreads();
+        const auto is_nan = [](int f) { return (f & 4) != 0 || (f & 3) == 3; };
+        unsigned odd = 0u; // the piece's cells with an infinity or a NaN in these columns; most pieces have none
+        const auto has_odd = [&](std::int64_t first, std::int64_t) {
+            odd = 0u;
+            for (int i = 0; i < p.d.piece_rows / 16; ++i) {
+                const unsigned short *at = p.odd_rows + ((first - p.odd_from) / 16 + i) * odd_chunks(p.n) + c0 / 32;
+                odd |= static_cast<unsigned>(__ldcg(at) | (NB > 32 ? __ldcg(at + 1) : 0)) << (16 * i);
+            }
+            return odd != 0u;
+        };
+        each_words(p, window, warp, kWarps, has_odd, [&](std::uint32_t e, int gene, std::int64_t row) {
+            const bool mine = e != kPadding && (odd >> ((row - p.odd_from) & (p.d.piece_rows - 1)) & 1u) != 0u &&
+                              (*const_cast<volatile unsigned *>(settled + gene / 32) >> (gene & 31) & 1u) == 0u;
+            std::uint32_t todo = __ballot_sync(0xffffffffu, mine);
+            while (todo != 0u) {
+                const int j = __ffs(todo) - 1;
+                todo &= todo - 1u;
+                const int code = static_cast<int>(static_cast<signed char>(__shfl_sync(0xffffffffu, e, j) & 0xffu)) + p.d.code_bias, gj = __shfl_sync(0xffffffffu, gene, j);
+                const std::int64_t rj = __shfl_sync(0xffffffffu, row, j);
+                const float value = fmaf(static_cast<float>(code), meta[gj].x, meta[gj].y);
+                bool all = true;
+                for (int c = lane; c < NB && c0 + c < p.n; c += 32) {
+                    const float g = __ldg(p.g + rj * p.g_ld + c0 + c), product = value * g;
+                    const int flag = isfinite(g) ? 0 : isnan(product) ? 4 : product > 0.0f ? 1 : 2;
+                    int had = *const_cast<volatile int *>(flags + gj * NB + c);
+                    if ((flag & ~had) != 0) had = atomicOr(flags + gj * NB + c, flag) | flag;
+                    all = all && is_nan(had);
+                }
+                if (__all_sync(0xffffffffu, all) && lane == 0) atomicOr(settled + gj / 32, 1u << (gj & 31));
+            }
+        });
+        __syncthreads();
+        for (int i = tid; i < kWin * NB; i += kFinish)
+            if (flags[i] != 0) values[i] = is_nan(flags[i]) ? CUDART_NAN : flags[i] == 1 ? CUDART_INF : -CUDART_INF;
+        __syncthreads();
+    }
     if ((mode & kRepeats) == 0) return;
     const double rest = slices_of(mode) == 3 ? second_step(3) : second_step(4);
     for (int quarter = 0; quarter < 4; ++quarter)
         for (int pass = 0; pass < passes_of(mode); ++pass) {
             for (int i = tid; i < kWin * kQuarter * 2; i += kFinish) whole[i] = 0u;
             __syncthreads();
-            each_words(p, window, warp, kWarps, true, [&](std::uint32_t e, int gene, std::int64_t row) {
+            each_words(p, window, warp, kWarps, [](std::int64_t, std::int64_t base) { return (base & kTwice) != 0; }, [&](std::uint32_t e, int gene, std::int64_t row) {
                 std::uint32_t todo = __ballot_sync(0xffffffffu, e >= kAgain);
                 while (todo != 0u) {
                     const int j = __ffs(todo) - 1;
@@ -1145,7 +1212,9 @@ __device__ __noinline__ void beside_tiles(const finish_params &p, int mode, bool
                     const std::int64_t rj = __shfl_sync(0xffffffffu, row, j);
                     const int c = quarter * kQuarter + lane;
                     if (lane < kQuarter && c0 + c < p.n) {
-                        const double step = __ldg(p.d.steps + c0 + c), scaled = step != 0.0 ? static_cast<double>(__ldg(p.g + rj * p.g_ld + c0 + c)) / step : 0.0;
+                        const double step = __ldg(p.d.steps + c0 + c);
+                        const float g = __ldg(p.g + rj * p.g_ld + c0 + c);
+                        const double scaled = step != 0.0 && isfinite(g) ? static_cast<double>(g) / step : 0.0;
                         int q = __double2int_rn(scaled);
                         if (pass != 0) q = __double2int_rn((scaled - static_cast<double>(q)) / rest);
                         atomicAdd(whole + (gj * kQuarter + lane) * 2, static_cast<unsigned long long>(static_cast<long long>(code) * q));
@@ -1164,7 +1233,7 @@ __device__ __noinline__ void beside_tiles(const finish_params &p, int mode, bool
 }
 
 // G'[genes of one window, columns of one block] = beta * G' + alpha * (the sums of the set's runs, added in run order; EXACT: the totals).
-// Genes that a cell holds again (kAgain) are added here.  Where G spreads too far for fixed point, or a scale or a zero-point of the window is not
+// What genes that a cell holds again (kAgain) and infinities and NaNs of G come to is added here.  Where G spreads too far for fixed point, or a scale or a zero-point of the window is not
 // finite (0 * infinity, in a product of sums, would reach cells that hold no entry): everything, entry by entry (beside_tiles, which is no part
 // of this function's registers: two CTAs of 512 threads to an SM, or the 262 of 33,538 genes take two rounds, 12 us instead of 9).
 // A thread has a gene and sixteen columns, so that a warp's loads are contiguous.
@@ -1190,7 +1259,7 @@ __global__ void __launch_bounds__(finish_threads(NB), 1024 / finish_threads(NB))
         odd = isfinite(so.x) && isfinite(so.y) ? 0 : 1;
     }
     const int mode = __ldcg(p.d.mode);
-    const bool by_entry = __syncthreads_or(odd) != 0 || (mode & kByEntry) != 0, more = by_entry || (mode & kRepeats) != 0;
+    const bool by_entry = __syncthreads_or(odd) != 0 || (mode & kByEntry) != 0, more = by_entry || (mode & (kRepeats | kNonFinite)) != 0;
     if (more) beside_tiles<NB>(p, mode, by_entry, window, meta, beside, reinterpret_cast<unsigned long long *>(beside + kWin * NB));
     const int passes = passes_of(mode), c = tid / kWin * 16;
     // the set's slots: the CTAs whose shares meet its runs, run after run, pass after pass
@@ -1263,7 +1332,7 @@ __global__ void __launch_bounds__(finish_threads(NB), 1024 / finish_threads(NB))
 }
 
 // What a launch with the least workspace takes at a time: groups, and, repeatable, sets of windows.
-constexpr std::int64_t kLeastGroups = 2, kLeastSets = 4, kLeastRoundedGroups = 11;
+constexpr std::int64_t kLeastGroups = 2, kLeastSets = 4, kLeastRoundedGroups = 8;
 int column_block(std::int64_t n) { return n <= 32 ? 32 : 64; }
 int padded_columns(std::int64_t n) { return n <= 32 ? 32 : n <= 64 ? 64 : n <= 128 ? 128 : 256; }
 
@@ -1278,9 +1347,12 @@ std::uint64_t partial_bytes(std::int64_t groups, std::int64_t cols, std::int64_t
     const std::int64_t sets = (windows + per_set - 1) / per_set * ((n + nb - 1) / nb), cuts = (groups + kRunGroups - 1) / kRunGroups;
     return device_arena::rounded(static_cast<std::uint64_t>(2 * sets * cuts + ctas) * static_cast<std::uint64_t>(per_set * kWin * nb) * sizeof(float));
 }
-// what a launch over `groups` groups at a time needs, without the words
-std::uint64_t launch_bytes(std::int64_t groups, std::int64_t cols, std::int64_t n, int ctas) {
-    return kRecordsAt + record_bytes(groups, n) + partial_bytes(groups, cols, n, ctas);
+std::uint64_t odd_bytes(std::int64_t groups, std::int64_t n) {
+    return device_arena::rounded(static_cast<std::uint64_t>(groups * (kRows / 16) * odd_chunks(static_cast<int>(n))) * sizeof(unsigned short));
+}
+// what a launch over `groups` of `all` groups at a time needs, without the words
+std::uint64_t launch_bytes(std::int64_t all, std::int64_t groups, std::int64_t cols, std::int64_t n, int ctas) {
+    return kRecordsAt + odd_bytes(all, n) + record_bytes(groups, n) + partial_bytes(groups, cols, n, ctas);
 }
 // ... and a repeatable one over `sets` sets of windows at a time
 std::int64_t set_count_of(std::int64_t cols, std::int64_t n) {
@@ -1291,8 +1363,8 @@ std::uint64_t total_bytes(std::int64_t sets, std::int64_t n) { // of one pass
     const std::int64_t nb = column_block(n);
     return static_cast<std::uint64_t>(sets * ((n + nb - 1) / nb) * set_windows(static_cast<int>(nb), kMostSlices) * kWin * nb) * 16u;
 }
-std::uint64_t exact_bytes(std::int64_t groups, std::int64_t sets, std::int64_t n) {
-    return kRecordsAt + record_bytes(groups, n) + 2u * total_bytes(sets, n);
+std::uint64_t exact_bytes(std::int64_t all, std::int64_t groups, std::int64_t sets, std::int64_t n) {
+    return kRecordsAt + odd_bytes(all, n) + record_bytes(groups, n) + 2u * total_bytes(sets, n);
 }
 std::int64_t group_count_of(std::int64_t rows) { return (rows + kRows - 1) / kRows; }
 std::int64_t piece_count(std::int64_t rows) { return (rows + piece_rows_of(rows) - 1) / piece_rows_of(rows); }
@@ -1357,6 +1429,7 @@ cb200_status launch_digits(const digit_launch &l, int sm_count, cudaStream_t str
             pack_params k = l.pack;
             k.first_row = row0;
             k.groups = m.group_count;
+            k.odd_rows = l.pack.odd_rows + (begin - l.main.group_begin) * (kRows / 16) * odd_chunks(n);
             k.totals = reinterpret_cast<uint4 *>(m.totals);
             k.total_items = EXACT && clear ? static_cast<std::int64_t>(total_bytes(m.set_count, n) / 16u) : 0;
             CB200_CUDA_OK(launch_kernel(true, pack_digits_kernel<NB, BASE>, dim3(static_cast<unsigned>(std::min<std::int64_t>(blocks * kGPieces, 4 * sm_count))), 256, 0, stream, k));
@@ -1419,13 +1492,14 @@ digit_layout digit_words_at(void *memory, const qcsr_view &x) {
     return l;
 }
 std::uint64_t qcsr_transpose_digits_workspace_bytes(std::int64_t rows, std::int64_t cols, std::int64_t n, bool repeatable) {
-    if (repeatable) return exact_bytes(group_count_of(rows), set_count_of(cols, n), n);
-    return launch_bytes(group_count_of(rows), cols, n, kMaxCtas);
+    const std::int64_t groups = group_count_of(rows);
+    if (repeatable) return exact_bytes(groups, groups, set_count_of(cols, n), n);
+    return launch_bytes(groups, groups, cols, n, kMaxCtas);
 }
 std::uint64_t qcsr_transpose_digits_least_workspace(std::int64_t rows, std::int64_t cols, std::int64_t n, bool repeatable, int sm_count) {
     const std::int64_t groups = group_count_of(rows);
-    if (repeatable) return exact_bytes(std::min<std::int64_t>(groups, kLeastGroups), std::min<std::int64_t>(set_count_of(cols, n), kLeastSets), n);
-    return launch_bytes(std::min<std::int64_t>(groups, kLeastRoundedGroups), cols, n, std::min(sm_count, kMaxCtas));
+    if (repeatable) return exact_bytes(groups, std::min<std::int64_t>(groups, kLeastGroups), std::min<std::int64_t>(set_count_of(cols, n), kLeastSets), n);
+    return launch_bytes(groups, std::min<std::int64_t>(groups, kLeastRoundedGroups), cols, n, std::min(sm_count, kMaxCtas));
 }
 std::uint64_t qcsr_transpose_digits_once_bytes(std::int64_t rows, std::int64_t cols, std::int64_t n, std::int64_t nnz, int bits, int policy) {
     if (!qcsr_transpose_digits_shape_ok(rows, cols, n, bits, policy)) return 0u;
@@ -1478,7 +1552,7 @@ cb200_status launch_qcsr_transpose_digits(const qcsr_view &x, const dense_args &
     const std::int64_t first_row = layout != nullptr ? 0 : row_begin, rows_of_words = layout != nullptr ? x.rows : row_end - row_begin;
     const std::int64_t group_begin = (row_begin - first_row) / kRows, group_count = (row_end - first_row + kRows - 1) / kRows - group_begin;
     std::int64_t slice = group_count, chunk = repeatable ? set_count_of(x.cols, d.n) : 0;
-    const auto needs = [&](std::int64_t groups) { return repeatable ? exact_bytes(groups, chunk, d.n) : launch_bytes(groups, x.cols, d.n, sm_count); };
+    const auto needs = [&](std::int64_t groups) { return repeatable ? exact_bytes(group_count, groups, chunk, d.n) : launch_bytes(group_count, groups, x.cols, d.n, sm_count); };
     while (chunk > 1 && needs(std::min<std::int64_t>(slice, kLeastGroups)) > workspace_bytes) chunk = (chunk + 1) / 2;
     while (slice > 1 && needs(slice) > workspace_bytes) slice = (slice + 1) / 2;
     if (needs(slice) > workspace_bytes) return CB200_STATUS_SUCCESS;
@@ -1512,7 +1586,8 @@ cb200_status launch_qcsr_transpose_digits(const qcsr_view &x, const dense_args &
     k.part_sum = reinterpret_cast<const double2 *>(ws + kPartSumAt);
     k.part_least = reinterpret_cast<const unsigned *>(ws + kPartLeastAt);
     k.steps = reinterpret_cast<double *>(ws + kStepsAt);
-    k.records = ws + kRecordsAt;
+    k.odd_rows = reinterpret_cast<unsigned short *>(ws + kRecordsAt);
+    k.records = ws + kRecordsAt + odd_bytes(group_count, d.n);
     k.bases = p.bases; k.word_pieces = p.pieces;
     k.mode = reinterpret_cast<int *>(ws) + 1;
     p.records = k.records; p.steps = k.steps; p.mode = k.mode;
@@ -1526,6 +1601,7 @@ cb200_status launch_qcsr_transpose_digits(const qcsr_view &x, const dense_args &
     p.poll_limit = test_poll_limit();
     finish_params &f = l.finish;
     f.g = static_cast<const float *>(d.dense); f.g_ld = d.dense_ld;
+    f.odd_rows = k.odd_rows; f.odd_from = first_row + group_begin * kRows;
     f.first_row = first_row; f.row_begin = row_begin; f.row_end = row_end;
     f.out = d.out; f.out_ld = d.out_ld; f.n = static_cast<int>(d.n);
     f.out_vector = reinterpret_cast<std::uintptr_t>(d.out) % 16u == 0u && d.out_ld % 4 == 0 && d.n % 4 == 0 ? 1 : 0;

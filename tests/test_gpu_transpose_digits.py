@@ -334,3 +334,45 @@ def test_a_gene_held_again_changes_no_others(cuda_device, oracle, slices, n, bit
         want, size = dec[sel] @ g_host[at[sel]].astype(np.float64), (np.abs(dec[sel]) + abs(m["offsets"][gene])).sum() * np.abs(g_host).max(0)
         # as in assert_within, two passes as four digits at least
         assert np.all(np.abs(outs[1][gene] - want) <= (1.02 * 2.0 ** (1 - 8 * (3 if slices == 3 else 4)) + 10 * 2.0 ** -24) * size), gene
+
+
+@pytest.mark.parametrize("slices,n,bits", [(3, 64, 8), (3, 32, 4), (4, 64, 8), (4, 32, 8), (4, 128, 4), (0, 50, 8), (0, 130, 4)])
+def test_infinities_and_nans_reach_their_genes_alone(cuda_device, oracle, slices, n, bits):
+    """Every sum that no infinity or NaN is part of has the bits it has with zeroes in their place; the others are what 64 bits make of them.  Few cells,
+    all cells, cells outside the row range; genes held again; slices of the groups; alpha and beta.  0 digits: the words made in the call."""
+    rng = np.random.default_rng(n)
+    rows, cols = (2111, 1500) if slices == 0 else (256 * 20 + 9, 1664)
+    c = host_pack(oracle, random_csr(rng, rows=rows, cols=cols, max_nnz=3000 if slices == 0 else 120, bits=bits))
+    if bits == 4:
+        c["col_idx"][c["col_idx"] == 300] = 303                       # gene 300 is in no cell, some cells hold 303 twice
+    x = to_dev(c, cuda_device)
+    dec = oracle.unpack_csr(bits, 1, c["row_ptr"], c["packed_row_ptr"], c["col_idx"], c["scales"], c["offsets"], c["packed"]).astype(np.float64)
+    at = np.repeat(np.arange(rows), np.diff(c["row_ptr"]))
+    op = prepared(x, n, slices, cuda_device) if slices else ops.PreparedSpmm(capi.PROJECTION_TRANSPOSE, rows, cols, n, x.nnz, bits, 1, torch.float32, cuda_device)
+    room = op.workspace_bytes
+    base = rng.normal(size=(rows, n)).astype(np.float32)
+    few = base.copy()
+    few[[5, 400, 401, rows - 1], [0, 31, n - 1, n - 1]] = [np.inf, -np.inf, np.nan, np.inf]
+    few[700:703, :] = np.inf
+    many = np.where(rng.random(base.shape) < 0.5, np.inf, base).astype(np.float32)
+    many[::3, 7] = -np.inf
+    for g_host in (few, many, np.full_like(base, np.nan)):
+        for lo, hi, part in ((0, rows, 1.0), (6, rows - 1, 1.0)) + (((0, rows, 0.8),) if slices else ()):
+            op.workspace_bytes = int(room * part)
+            init = torch.from_numpy(rng.normal(size=(cols, n)).astype(np.float32)).to(cuda_device)
+            def run(g):
+                out = op.run(x, torch.from_numpy(g).to(cuda_device), init.clone(), alpha=2.0, beta=0.5, row_begin=lo, row_end=hi)
+                assert op.status() == 0 and not mode_of(op)[2]
+                return out.cpu().numpy()
+            got, zeroed = run(g_host), run(np.where(np.isfinite(g_host), g_host, 0.0).astype(np.float32))
+            sel = (at >= lo) & (at < hi)
+            want = np.zeros((cols, n))
+            with np.errstate(invalid="ignore"):
+                for j in range(n):                                    # what the sums are made of, not their rounding
+                    odd = sel & ~np.isfinite(g_host[at, j])
+                    np.add.at(want[:, j], c["col_idx"][odd], 2.0 * dec[odd] * g_host[at[odd], j])
+            touched = ~np.isfinite(want)
+            assert touched.any() and np.array_equal(got[~touched], zeroed[~touched])
+            assert np.array_equal(got[touched], want[touched].astype(np.float32), equal_nan=True)
+            assert np.array_equal(run(g_host).view(np.int32), got.view(np.int32))
+    op.close()
