@@ -563,7 +563,7 @@ cb200_status cb200_spmm_prepare(const cb200_spmm_problem *problem, cb200_prepare
         if (problem->device_matrix == nullptr)
             p->workspace_bytes = std::max(p->workspace_bytes, qcsr_transpose_digits_once_bytes(problem->m, problem->k, problem->n, problem->nnz, problem->bits, problem->policy));
         if (plan.digits != 0) {
-            const cb200_status st = build_digit_words(view_of(*problem->device_matrix), p->arena, stream, &p->digits);
+            const cb200_status st = build_digit_words(view_of(*problem->device_matrix), plan.digits == 4, p->arena, stream, &p->digits);
             if (st != CB200_STATUS_SUCCESS) return abandon(st);
             p->digit_slices = plan.digits;
             p->schedule_name = plan.digits == 4 ? "gene_gather" : "tensor_blocked_x3";

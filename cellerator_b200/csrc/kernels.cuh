@@ -218,11 +218,12 @@ constexpr std::int64_t kDigitWordsTwice = 1ll << 62;
 bool qcsr_transpose_digits_shape_ok(std::int64_t rows, std::int64_t cols, std::int64_t n, int bits, int policy);
 std::uint64_t qcsr_digit_words_bytes_bound(std::int64_t rows, std::int64_t cols, std::int64_t nnz);
 // current device; memory from `arena`, kernels on `stream`, which is waited for
-cb200_status build_digit_words(const qcsr_view &x, device_arena &arena, cudaStream_t stream, digit_layout *out);
+// refuse_outside: a gene outside the matrix is CB200_STATUS_INVALID_SHAPE, else its entry is left out
+cb200_status build_digit_words(const qcsr_view &x, bool refuse_outside, device_arena &arena, cudaStream_t stream, digit_layout *out);
 // ... and without the wait, into memory of that size
 digit_layout digit_words_at(void *memory, const qcsr_view &x);
 cb200_status launch_digit_words(const qcsr_view &x, std::int64_t row_begin, std::int64_t row_end, std::uint32_t *words, std::uint32_t *bounds,
-                                std::int64_t *bases, int *status, cudaStream_t stream);
+                                std::int64_t *bases, int *status, int *outside, cudaStream_t stream);
 std::uint64_t qcsr_transpose_digits_workspace_bytes(std::int64_t rows, std::int64_t cols, std::int64_t n, bool repeatable);
 std::uint64_t qcsr_transpose_digits_least_workspace(std::int64_t rows, std::int64_t cols, std::int64_t n, bool repeatable, int sm_count); // slower
 // Whether a call that sees its matrix once should make the words in its workspace (0: no), and what it then needs

@@ -133,6 +133,7 @@ struct words_params {
     std::uint32_t *bounds; // [pieces][windows + 1], from the piece's base
     std::int64_t *bases;   // [pieces]; kTwice: a cell of the piece holds a gene more than once
     int *status;           // cleared, where given
+    int *outside;          // CHECK: set if a gene lies outside the matrix; such entries have no word
 };
 constexpr std::int64_t kTwice = kDigitWordsTwice;
 
@@ -144,7 +145,8 @@ constexpr std::int64_t kTwice = kDigitWordsTwice;
 // holds already (kAgain): a tile has one place for them, and finish_kernel adds the others.
 //
 // What bounds it: the latency of the genes' loads (eight in flight per warp, 48 warps per SM) and issue, half of the slots.
-template<int BITS>
+// CHECK: genes outside the matrix are reported (at prepare; in a call the test cost registers, 68 us instead of 66 for 8,191 cells).
+template<int BITS, bool CHECK>
 __global__ void __launch_bounds__(kBuildThreads, 2) digit_words_kernel(const words_params p) {
     extern __shared__ std::uint32_t place_of[]; // [kPieceRows][pitch]; see below.  Behind it [chunks][kPieceRows + 1] and [windows]
     __shared__ std::int64_t codes_of[kPieceRows]; // where the codes of a cell begin
@@ -241,6 +243,7 @@ __global__ void __launch_bounds__(kBuildThreads, 2) digit_words_kernel(const wor
             for (int e = cell_start[r] + lane; e < cell_start[r + 1]; e += 32) {
                 const int gene = __ldg(genes + e);
                 if (static_cast<unsigned>(gene) < static_cast<unsigned>(p.cols)) f(r, gene, e - cell_start[r]);
+                else if constexpr (CHECK) *p.outside = 1;
             }
     };
     const auto word_of = [&](std::uint32_t bits, int gene, std::uint32_t code) {
@@ -1452,13 +1455,13 @@ cb200_status launch_digits(const digit_launch &l, int sm_count, cudaStream_t str
 } // namespace
 
 cb200_status launch_digit_words(const qcsr_view &x, std::int64_t row_begin, std::int64_t row_end, std::uint32_t *words, std::uint32_t *bounds,
-                                std::int64_t *bases, int *status, cudaStream_t stream) {
+                                std::int64_t *bases, int *status, int *outside, cudaStream_t stream) {
     words_params p{};
     p.row_ptr = x.row_ptr; p.packed_row_ptr = x.packed_row_ptr; p.col_idx = x.col_idx; p.packed = x.packed;
     p.row_begin = row_begin; p.row_end = row_end; p.cols = x.cols; p.windows = static_cast<int>((x.cols + kWin - 1) / kWin);
     p.code_bias = x.bits == 8 ? 128 : 0;
     p.piece_rows = piece_rows_of(x.rows);
-    p.words = words; p.bounds = bounds; p.bases = bases; p.status = status;
+    p.words = words; p.bounds = bounds; p.bases = bases; p.status = status; p.outside = outside;
     const int smem = build_smem_bytes(x.cols);
     const unsigned grid = static_cast<unsigned>((row_end - row_begin + p.piece_rows - 1) / p.piece_rows);
     const auto run = [&](auto kernel) {
@@ -1466,7 +1469,8 @@ cb200_status launch_digit_words(const qcsr_view &x, std::int64_t row_begin, std:
         if (err == cudaSuccess) kernel<<<grid, kBuildThreads, smem, stream>>>(p);
         return err;
     };
-    CB200_CUDA_OK(x.bits == 8 ? run(digit_words_kernel<8>) : run(digit_words_kernel<4>));
+    if (outside != nullptr) CB200_CUDA_OK(x.bits == 8 ? run(digit_words_kernel<8, true>) : run(digit_words_kernel<4, true>));
+    else CB200_CUDA_OK(x.bits == 8 ? run(digit_words_kernel<8, false>) : run(digit_words_kernel<4, false>));
     count_launch();
     CB200_CUDA_OK(cudaGetLastError());
     return CB200_STATUS_SUCCESS;
@@ -1479,7 +1483,7 @@ bool qcsr_transpose_digits_shape_ok(std::int64_t rows, std::int64_t cols, std::i
 }
 std::uint64_t qcsr_digit_words_bytes_bound(std::int64_t rows, std::int64_t cols, std::int64_t nnz) {
     return device_arena::rounded(word_bytes(rows, cols, nnz)) + device_arena::rounded(bound_bytes(rows, cols)) +
-           device_arena::rounded(static_cast<std::uint64_t>(piece_count(rows)) * 8u);
+           device_arena::rounded(static_cast<std::uint64_t>(piece_count(rows)) * 8u) + device_arena::rounded(sizeof(int)); // (the last: while they are built)
 }
 digit_layout digit_words_at(void *memory, const qcsr_view &x) {
     unsigned char *at = static_cast<unsigned char *>(memory);
@@ -1510,7 +1514,7 @@ std::uint64_t qcsr_transpose_digits_once_bytes(std::int64_t rows, std::int64_t c
     return qcsr_transpose_digits_workspace_bytes(rows, cols, n, false) + qcsr_digit_words_bytes_bound(rows, cols, nnz);
 }
 
-cb200_status build_digit_words(const qcsr_view &x, device_arena &arena, cudaStream_t stream, digit_layout *out) {
+cb200_status build_digit_words(const qcsr_view &x, bool refuse_outside, device_arena &arena, cudaStream_t stream, digit_layout *out) {
     *out = digit_layout{};
     if (x.row_ptr == nullptr || (x.nnz != 0 && (x.col_idx == nullptr || x.packed == nullptr)))
         return fail(CB200_STATUS_INVALID_ARGUMENT, "the matrix handed to prepare has null arrays");
@@ -1519,14 +1523,22 @@ cb200_status build_digit_words(const qcsr_view &x, device_arena &arena, cudaStre
     out->words = static_cast<std::uint32_t *>(arena.take(words));
     out->bounds = static_cast<std::uint32_t *>(arena.take(bounds));
     out->bases = static_cast<std::int64_t *>(arena.take(bases));
+    int *outside = static_cast<int *>(arena.take(sizeof(int)));
     cb200_status st = CB200_STATUS_SUCCESS;
-    if (out->words == nullptr || out->bounds == nullptr || out->bases == nullptr)
+    if (out->words == nullptr || out->bounds == nullptr || out->bases == nullptr || outside == nullptr)
         st = fail(CB200_STATUS_INSUFFICIENT_WORKSPACE, "no device memory for the entry words");
-    if (st == CB200_STATUS_SUCCESS) st = launch_digit_words(x, 0, x.rows, out->words, out->bounds, out->bases, nullptr, stream);
+    const auto check = [&](cudaError_t err) {
+        if (err != cudaSuccess && st == CB200_STATUS_SUCCESS) st = fail(CB200_STATUS_CUDA_ERROR, "building the entry words: %s", cudaGetErrorString(err));
+    };
+    if (st == CB200_STATUS_SUCCESS) check(cudaMemsetAsync(outside, 0, sizeof(int), stream));
+    if (st == CB200_STATUS_SUCCESS) st = launch_digit_words(x, 0, x.rows, out->words, out->bounds, out->bases, nullptr, outside, stream);
     if (st == CB200_STATUS_SUCCESS) {
-        const cudaError_t err = cudaStreamSynchronize(stream);
-        if (err != cudaSuccess) st = fail(CB200_STATUS_CUDA_ERROR, "building the entry words: %s", cudaGetErrorString(err));
+        int found = 0;
+        check(cudaMemcpyAsync(&found, outside, sizeof(int), cudaMemcpyDeviceToHost, stream));
+        check(cudaStreamSynchronize(stream));
+        if (st == CB200_STATUS_SUCCESS && refuse_outside && found != 0) st = fail(CB200_STATUS_INVALID_SHAPE, "a column index lies outside the matrix");
     }
+    arena.give_back(outside, sizeof(int));
     if (st != CB200_STATUS_SUCCESS) {
         arena.give_back(out->bases, bases);
         arena.give_back(out->bounds, bounds);
@@ -1570,7 +1582,7 @@ cb200_status launch_qcsr_transpose_digits(const qcsr_view &x, const dense_args &
         p.words = layout->words; p.bounds = layout->bounds; p.bases = layout->bases;
     } else {
         const digit_layout made = digit_words_at(ws + own, x);
-        const cb200_status st = launch_digit_words(x, row_begin, row_end, made.words, made.bounds, made.bases, p.status, stream);
+        const cb200_status st = launch_digit_words(x, row_begin, row_end, made.words, made.bounds, made.bases, p.status, nullptr, stream);
         if (st != CB200_STATUS_SUCCESS) return st;
         p.words = made.words; p.bounds = made.bounds; p.bases = made.bases;
     }

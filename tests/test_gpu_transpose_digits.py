@@ -376,3 +376,28 @@ def test_infinities_and_nans_reach_their_genes_alone(cuda_device, oracle, slices
             assert np.array_equal(got[touched], want[touched].astype(np.float32), equal_nan=True)
             assert np.array_equal(run(g_host).view(np.int32), got.view(np.int32))
     op.close()
+
+
+@pytest.mark.parametrize("gene", [-1, 1664, 2 ** 31 - 1])
+def test_a_gene_outside_the_matrix_is_refused(cuda_device, oracle, gene):
+    """Preparing a repeatable transpose refuses it whatever kernel is chosen; the other requests leave its entry out."""
+    rng = np.random.default_rng(5)
+    rows, cols, n = 256 * 20, 1664, 64
+    c = host_pack(oracle, random_csr(rng, rows=rows, cols=cols, max_nnz=100, bits=8, empty_rows=False))
+    x = to_dev(c, cuda_device)
+    at = int(c["row_ptr"][1234])
+    x.col_idx[at] = gene
+    for hint in (None, "gene_gather"):
+        with pytest.raises(capi.Cb200Error) as e:
+            ops.PreparedSpmm(capi.PROJECTION_TRANSPOSE, rows, cols, n, x.nnz, 8, 1, torch.float32, cuda_device, device_matrix=x, deterministic=True, schedule=hint)
+        assert e.value.status == capi.INVALID_SHAPE
+    g, g_host = dense(rng, rows, n, torch.float32, cuda_device, std=1.0)
+    op = prepared(x, n, 3, cuda_device)
+    got = op.run(x, g, torch.empty(cols, n, device=cuda_device)).cpu().numpy()
+    assert op.status() == 0
+    op.close()
+    want, l1 = reference(oracle, c, g_host)                           # with the entry's own gene in place
+    held = c["col_idx"][at]
+    dec = oracle.unpack_csr(8, 1, c["row_ptr"], c["packed_row_ptr"], c["col_idx"], c["scales"], c["offsets"], c["packed"])
+    want[held] -= float(dec[at]) * g_host[1234].astype(np.float64)
+    assert_within(got, want, l1, g_host, 3)
