@@ -560,7 +560,8 @@ cb200_status cb200_spmm_prepare(const cb200_spmm_problem *problem, cb200_prepare
     if (problem->projection == CB200_PROJECTION_TRANSPOSE) {
         p->workspace_bytes = qcsr_transpose_workspace_bytes(problem->m, problem->k, p->sm_count);
         p->schedule_name = "vector_reductions";
-        if (problem->device_matrix == nullptr)
+        // a matrix that prepare has no use for is no reason to do without integer sums at launch
+        if (plan.digits == 0 && !plan.gene_gather && !plan.blocked)
             p->workspace_bytes = std::max(p->workspace_bytes, qcsr_transpose_digits_once_bytes(problem->m, problem->k, problem->n, problem->nnz, problem->bits, problem->policy));
         if (plan.digits != 0) {
             const cb200_status st = build_digit_words(view_of(*problem->device_matrix), plan.digits == 4, p->arena, stream, &p->digits);

@@ -401,3 +401,22 @@ def test_a_gene_outside_the_matrix_is_refused(cuda_device, oracle, gene):
     dec = oracle.unpack_csr(8, 1, c["row_ptr"], c["packed_row_ptr"], c["col_idx"], c["scales"], c["offsets"], c["packed"])
     want[held] -= float(dec[at]) * g_host[1234].astype(np.float64)
     assert_within(got, want, l1, g_host, 3)
+
+
+@pytest.mark.parametrize("n,multiply", [(1, capi.DTYPE_F32), (50, capi.DTYPE_F32), (100, capi.DTYPE_BF16), (128, capi.DTYPE_F32)])
+def test_handing_the_matrix_over_takes_nothing_away(cuda_device, oracle, n, multiply):
+    """Widths that no prepared schedule serves: the same kernels, workspace and bits as without the matrix in hand."""
+    rng = np.random.default_rng(n)
+    rows, cols = 4500, 1400
+    x = to_dev(host_pack(oracle, random_csr(rng, rows=rows, cols=cols, max_nnz=1300, bits=8)), cuda_device)
+    assert x.nnz >= 2_000_000
+    g, _ = dense(rng, rows, n, torch.float32, cuda_device, std=1.0)
+    outs = []
+    for matrix in (None, x):
+        op = ops.PreparedSpmm(capi.PROJECTION_TRANSPOSE, rows, cols, n, x.nnz, 8, 1, torch.float32, cuda_device, device_matrix=matrix, multiply=multiply)
+        launches = capi.lib().cb200_kernel_launch_count()
+        out = op.run(x, g, torch.empty(cols, n, device=cuda_device))
+        assert op.status() == 0
+        outs.append((op.schedule, op.workspace_bytes, capi.lib().cb200_kernel_launch_count() - launches, out.cpu().numpy().tobytes()))
+        op.close()
+    assert outs[0] == outs[1] and outs[0][0] == "vector_reductions"
