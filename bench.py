@@ -490,7 +490,7 @@ def measure_workload(name, args, device, rank, world, steps, warmup, fleet, mult
     if world > 1:
         dist.barrier()
         torch.cuda.synchronize()
-    rec = {"schedule": op.schedule, "steps": steps, "ms_per_step": total_ms / steps, "step_ms": summary_stats(per_step),
+    rec = {"schedule": op.schedule, "digits": op.digits, "steps": steps, "ms_per_step": total_ms / steps, "step_ms": summary_stats(per_step),
            "rows": wl["rows"], "cols": wl["cfg"]["cols"], "n": wl["n"], "bits": x.bits,
            "units_per_gpu": int(wl["units"]), "gpu_launches": int(launches),
            "prepare_ms_once": round(wl.get("prepare_ms", 0.0), 2), "prepare_ms_first_in_process": round(wl.get("prepare_first_ms", 0.0), 2),
@@ -722,10 +722,7 @@ def run_ours(args):
 
     kind_bell = args.workload == "c5_bell"
     schedule = main["schedule"]
-    # transpose by exact integer sums: zero-points are per gene here, the density is 5 %; fixed order below 2^23 places
-    digits = 0
-    if args.workload == "c3_transpose":
-        digits = {"tensor_blocked_x3": 3, "gene_gather": 4 if main["rows"] * main["cols"] >= 1 << 23 else 0}.get(schedule, 0)
+    digits = main["digits"]                            # of the dense operand, where the kernel adds whole numbers
     baked = digits == 0 and schedule in ("tensor_blocked", "tensor_blocked_x2", "tensor_blocked_x3", "tensor_dense", "gene_gather")
     result = {
         "metric": ("quantized Blocked-ELL projection throughput" if kind_bell else

@@ -388,13 +388,15 @@ schedule_plan plan_schedule(const cb200_spmm_problem &pr) {
         // under the name "gene_gather": with four digits of G (as many as keep the precision of fp32 products, for every cell's G: qcsr_transpose_digits.cu), where a tile of 256 x 128
         // holds 600 entries or more (every one of them pays for its tile; 2 %) and there are tiles for every SM (256 of them; 5,000
         // x 2,000, 320 tiles: 37 us against 42 gathered at N = 32, 38 against 49 at 64); by the gather gene by gene from a gene-major copy, whose fp32
-        // sums the oracle restates entry by entry, below that, with zero-points per row, and where it is asked for by name.
+        // sums the oracle restates entry by entry, below that, with zero-points per row, and where it is asked for by name.  By its own name,
+        // "integer_windows", the former is had at any size.
         const bool digits_ok = pr.device_matrix != nullptr && qcsr_transpose_digits_shape_ok(pr.m, pr.k, pr.n, pr.bits, pr.policy) &&
                                (limit == 0u || qcsr_digit_words_bytes_bound(pr.m, pr.k, pr.nnz) <= limit);
         const bool named_blocked = hint != nullptr && hint_starts(hint, "tensor_blocked") && pr.device_matrix != nullptr &&
                                    qcsr_transpose_blocked_shape_ok(pr.m, pr.k, pr.n, pr.bits) && (limit == 0u || nnz * 4u <= limit);
         if (pr.deterministic && !named_blocked) {
-            if (hint == nullptr && digits_ok && plan.mean_row_nnz >= 0.02 * static_cast<double>(pr.k) && pr.m * pr.k >= (1ll << 23)) {
+            const bool large = plan.mean_row_nnz >= 0.02 * static_cast<double>(pr.k) && pr.m * pr.k >= (1ll << 23);
+            if (digits_ok && (hint_is(hint, "integer_windows") || (hint == nullptr && large))) {
                 plan.digits = 4;
                 return plan;
             }
@@ -567,7 +569,7 @@ cb200_status cb200_spmm_prepare(const cb200_spmm_problem *problem, cb200_prepare
             const cb200_status st = build_digit_words(view_of(*problem->device_matrix), plan.digits == 4, p->arena, stream, &p->digits);
             if (st != CB200_STATUS_SUCCESS) return abandon(st);
             p->digit_slices = plan.digits;
-            p->schedule_name = plan.digits == 4 ? "gene_gather" : "tensor_blocked_x3";
+            p->schedule_name = plan.digits == 3 ? "tensor_blocked_x3" : hint_is(problem->schedule_hint, "integer_windows") ? "integer_windows" : "gene_gather";
             p->workspace_bytes = qcsr_transpose_digits_workspace_bytes(problem->m, problem->k, problem->n, plan.digits == 4);
             p->workspace_required = qcsr_transpose_digits_least_workspace(problem->m, problem->k, problem->n, plan.digits == 4, p->sm_count);
             p->persistent_bytes += p->digits.bytes;
@@ -701,6 +703,15 @@ cb200_status cb200_prepared_workspace(const cb200_prepared *prepared, uint64_t *
 
 const char *cb200_prepared_schedule(const cb200_prepared *prepared) {
     return prepared != nullptr ? prepared->schedule_name : "";
+}
+
+int32_t cb200_prepared_digits(const cb200_prepared *prepared) {
+    if (prepared == nullptr) return 0;
+    if (prepared->digits.words != nullptr) return prepared->digit_slices;
+    const cb200_spmm_problem &pr = prepared->problem;
+    const bool in_the_call = pr.projection == CB200_PROJECTION_TRANSPOSE && prepared->gene_major.col_ptr == nullptr && prepared->blocked.seg_ptr == nullptr &&
+                             qcsr_transpose_digits_once_bytes(pr.m, pr.k, pr.n, pr.nnz, pr.bits, pr.policy) != 0u;
+    return in_the_call ? 4 : 0;
 }
 
 uint64_t cb200_prepared_persistent_bytes(const cb200_prepared *prepared) {

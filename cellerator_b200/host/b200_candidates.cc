@@ -496,7 +496,7 @@ const char *prepared_schedule(const core::prepared_operation &prepared) noexcept
 const char *schedule_name(std::uint32_t variant) noexcept {
     static const char *const names[schedule_variant_count] = {"", "warp_per_row", "gene_tiled", "tensor_windows", "tensor_blocked",
                                                                "tensor_dense", "vector_reductions", "gene_gather",
-                                                               "tcgen05_block_rows", "cuda_cores", "tensor_codes"};
+                                                               "tcgen05_block_rows", "cuda_cores", "tensor_codes", "integer_windows"};
     return variant < schedule_variant_count ? names[variant] : "";
 }
 
@@ -520,7 +520,8 @@ const char *schedule_name(std::uint32_t variant) noexcept {
     case schedule_tensor_dense: fraction = 0.395; break;
     case schedule_tensor_codes: fraction = 0.570; break;
     case schedule_vector_reductions: fraction = 0.013; break;
-    case schedule_gene_gather: fraction = 0.111; break;
+    case schedule_gene_gather: fraction = 0.047; break;
+    case schedule_integer_windows: fraction = 0.111; break;
     case schedule_tcgen05_block_rows: fraction = 0.267; break;
     case schedule_cuda_cores: fraction = 0.013; break;
     default: break;
@@ -536,13 +537,18 @@ const char *schedule_name(std::uint32_t variant) noexcept {
     p.bits = shape.bits; p.policy = shape.decode_policy; p.dense_dtype = shape.dense_dtype; p.device = shape.device;
     p.structure_epoch = 1u;
     p.host_row_ptr = shape.host_row_ptr;
-    p.deterministic = variant == schedule_gene_gather ? 1 : 0;
+    p.deterministic = variant == schedule_gene_gather || variant == schedule_integer_windows ? 1 : 0;
     p.multiply = multiply;
     p.device_matrix = shape.device_matrix;
     p.schedule_hint = schedule_name(variant);
     std::uint64_t persistent = 0u;
     if (cb200_spmm_persistent_requirement(&p, &persistent) != CB200_STATUS_SUCCESS) persistent = 0u;
     record.analytical.persistent_bytes = persistent;
+    // G's digits and the 64-bit totals, two passes of each (cb200_prepared_workspace)
+    if (variant == schedule_integer_windows) {
+        const std::uint64_t columns = shape.n <= 32 ? 32u : (static_cast<std::uint64_t>(shape.n) + 63u) / 64u * 64u;
+        record.analytical.transient_bytes = (static_cast<std::uint64_t>(shape.m) * 8u + static_cast<std::uint64_t>(shape.k) * 32u) * columns;
+    }
     // building the copies: measured 18 ms of kernels for the 7.2 GB window-blocked copy of the 1M x 33,538 matrix
     // (two passes over the matrix with an atomic per run of entries), i.e. 0.06 of the copy bandwidth per byte kept
     record.analytical.backend_prepare_ns = 2.0e4 + static_cast<double>(persistent) / (hbm_bytes_per_ns * 0.06);

@@ -126,11 +126,12 @@ enum schedule_variant : std::uint32_t {
     schedule_tensor_blocked = 4u,     // forward: one bf16 pass, or split passes when fp32 products are asked for; transpose alike
     schedule_tensor_dense = 5u,
     schedule_vector_reductions = 6u,  // transpose, fp32 FMA + vector reductions
-    schedule_gene_gather = 7u,        // transpose, fixed order of the sums
+    schedule_gene_gather = 7u,        // transpose, fp32 sums in a fixed order, gene by gene
     schedule_tcgen05_block_rows = 8u, // Blocked-ELL
     schedule_cuda_cores = 9u,
     schedule_tensor_codes = 10u,      // forward, 4-bit codes on dense matrices: tiles of codes, decoded at launch
-    schedule_variant_count = 11u
+    schedule_integer_windows = 11u,   // transpose, repeatable: integer sums over entry words (zero-points per gene)
+    schedule_variant_count = 12u
 };
 const char *schedule_name(std::uint32_t variant) noexcept; // "" for the backend's choice or an unknown variant
 

@@ -302,6 +302,11 @@ class PreparedSpmm:
         return capi.lib().cb200_prepared_schedule(self.handle).decode()
 
     @property
+    def digits(self) -> int:
+        """Digits of the dense operand where the kernel adds whole numbers (3 or 4), else 0."""
+        return int(capi.lib().cb200_prepared_digits(self.handle))
+
+    @property
     def persistent_bytes(self) -> int:
         """Device bytes the prepared operation owns (row order, window-blocked copy)."""
         return int(capi.lib().cb200_prepared_persistent_bytes(self.handle))

@@ -251,7 +251,8 @@ typedef struct cb200_spmm_problem {
                             * device_matrix for it, else prepare is refused: schedule "gene_gather" (exact
                             * integer sums of codes times four digits of G where the matrix is large and dense
                             * enough and its zero-points are per gene, else fp32 FMAs entry by entry; the latter
-                            * always with schedule_hint "gene_gather"), or, with schedule_hint "tensor_blocked", the
+                            * always with schedule_hint "gene_gather", the former at any size with
+                            * "integer_windows"; cb200_prepared_digits tells them apart), or, with schedule_hint "tensor_blocked", the
                             * tensor-core schedules over the window-blocked copy, whose CTAs' sums are added in a
                             * fixed order too */
     /* numeric_policy.multiply of the request: 0 or CB200_DTYPE_F32 = exact fp32 products;
@@ -299,7 +300,7 @@ typedef struct cb200_spmm_problem {
     uint64_t value_generation;
     /* Optional request for one schedule by the name cb200_prepared_schedule reports ("gene_tiled",
      * "warp_per_row", "tensor_windows", "tensor_blocked", "tensor_dense", "tensor_codes"; transpose:
-     * "tensor_blocked", "vector_reductions", "gene_gather"; Blocked-ELL: "cuda_cores"); NULL or "" lets prepare choose from the shape and
+     * "tensor_blocked", "vector_reductions", "gene_gather", "integer_windows" (deterministic); Blocked-ELL: "cuda_cores"); NULL or "" lets prepare choose from the shape and
      * the row statistics.  A request the shape or the policy cannot serve is not an error: prepare
      * keeps its own choice, and cb200_prepared_schedule tells which schedule runs.  This is the
      * planner's lever (one candidate per schedule); nothing in the library reads the environment. */
@@ -338,8 +339,13 @@ cb200_status cb200_prepared_workspace(const cb200_prepared *prepared, uint64_t *
 /* kernel choice made at prepare time, as text: "warp_per_row", "gene_tiled" (exact fp32 products);
  * "tensor_windows", "tensor_blocked", "tensor_dense", "tensor_codes" (CSR, 16-bit products on tcgen05);
  * "tensor_blocked_x2" / "_x3" (fp32 products from bf16 passes); "tcgen05_block_rows" (Blocked-ELL);
- * transpose: "vector_reductions" (exact) or "tensor_blocked" */
+ * transpose: "vector_reductions", "gene_gather", "integer_windows", "tensor_blocked" / "_x3" */
 const char *cb200_prepared_schedule(const cb200_prepared *prepared);
+/* Three of the names stand for two kernels each: "tensor_blocked_x3", "gene_gather" and "vector_reductions" are served by integer
+ * sums where the matrix allows it.  This is the number of digits of the dense operand these start from (3 or 4; the device takes more
+ * where the operand's spread needs them), for "vector_reductions" of a launch over all rows with the workspace it reports;
+ * 0: the kernel multiplies floating-point numbers. */
+int32_t cb200_prepared_digits(const cb200_prepared *prepared);
 /* device bytes the prepared operation owns (row order, window-blocked copy): prepared_operation.persistent.bytes,
  * operation_core.hh:126-129,167-181; freed by cb200_prepared_destroy */
 uint64_t cb200_prepared_persistent_bytes(const cb200_prepared *prepared);

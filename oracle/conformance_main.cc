@@ -170,14 +170,18 @@ static void planner_leg(const core::candidate_registry &registry) {
     problem_ids t = make_ids(31u, core::projection_kind::transpose_or_backward, static_cast<std::uint64_t>(dm.nnz));
     host::projection_catalog_entry ts = fs;
     ts.projection = t.projection.runtime; ts.projection_kind = CB200_PROJECTION_TRANSPOSE; ts.dense_dtype = CB200_DTYPE_F32;
-    const pl::planner_candidate transposes[3] = {
+    const pl::planner_candidate transposes[4] = {
         host::make_schedule_candidate(*tr, t.projection, ts, host::schedule_vector_reductions, CB200_DTYPE_F32, 6553.9),
         host::make_schedule_candidate(*tr, t.projection, ts, host::schedule_tensor_blocked, CB200_DTYPE_F32, 6553.9),
-        host::make_schedule_candidate(*ord, t.projection, ts, host::schedule_gene_gather, CB200_DTYPE_F32, 6553.9)};
+        host::make_schedule_candidate(*ord, t.projection, ts, host::schedule_gene_gather, CB200_DTYPE_F32, 6553.9),
+        host::make_schedule_candidate(*ord, t.projection, ts, host::schedule_integer_windows, CB200_DTYPE_F32, 6553.9)};
     CHECK((transposes[0].flags & pl::planner_candidate_deterministic) == 0u && (transposes[2].flags & pl::planner_candidate_deterministic) != 0u,
           "planner: only the ordered transpose is flagged deterministic");
-    CHECK(transposes[1].analytical.persistent_bytes > 14000000000ull && transposes[2].analytical.persistent_bytes > 8900000000ull,
-          "planner: split-product words (8 B per entry) and the gene-major copy (5 B per entry) are declared");
+    CHECK(transposes[1].analytical.persistent_bytes > 7100000000ull && transposes[1].analytical.persistent_bytes < 7500000000ull &&
+              transposes[2].analytical.persistent_bytes > 8900000000ull && transposes[3].analytical.persistent_bytes == transposes[1].analytical.persistent_bytes,
+          "planner: the integer kernels' words (4 B per entry) and the gene-major copy (5 B per entry) are declared");
+    CHECK(transposes[3].analytical.kernel_ns < 0.5 * transposes[2].analytical.kernel_ns && transposes[3].analytical.transient_bytes > 500000000ull,
+          "planner: each repeatable transpose has the time and the workspace of the kernel its name selects");
     pl::planner_request treq = request_for(t, transposes, 3u);
     st = pl::plan_end_to_end(treq, &res);
     CHECK(static_cast<bool>(st) && res.legal_count == 3u && variant_of(res) == host::schedule_tensor_blocked,
@@ -187,6 +191,11 @@ static void planner_leg(const core::candidate_registry &registry) {
     CHECK(static_cast<bool>(st) && res.legal_count == 1u && res.diagnostics[0].rejection == pl::candidate_rejection::nondeterministic &&
               res.diagnostics[1].rejection == pl::candidate_rejection::nondeterministic && variant_of(res) == host::schedule_gene_gather,
           "planner: a deterministic policy rejects the atomic-order transposes and selects the ordered gather");
+    pl::planner_request ireq = request_for(t, transposes, 4u);
+    ireq.policy.deterministic = true;
+    st = pl::plan_end_to_end(ireq, &res);
+    CHECK(static_cast<bool>(st) && res.legal_count == 2u && variant_of(res) == host::schedule_integer_windows,
+          "planner: of the two repeatable transposes the integer one is the faster");
     treq.policy.maximum_persistent_bytes = 1ull << 30; // ... which needs its gene-major copy
     st = pl::plan_end_to_end(treq, &res);
     CHECK(st.code == pl::planner_status_code::no_legal_candidate, "planner: deterministic and no room for the gene-major copy -> no legal candidate");

@@ -420,3 +420,28 @@ def test_handing_the_matrix_over_takes_nothing_away(cuda_device, oracle, n, mult
         outs.append((op.schedule, op.workspace_bytes, capi.lib().cb200_kernel_launch_count() - launches, out.cpu().numpy().tobytes()))
         op.close()
     assert outs[0] == outs[1] and outs[0][0] == "vector_reductions"
+
+
+def test_names_and_digits(cuda_device, oracle):
+    """The integer kernel of a repeatable request by its name, at a size that would not choose it, and which kernel a name that two share stands for."""
+    rng = np.random.default_rng(6)
+    rows, cols, n = 700, 640, 64
+    c = host_pack(oracle, random_csr(rng, rows=rows, cols=cols, max_nnz=200, bits=8))
+    x = to_dev(c, cuda_device)
+    g, g_host = dense(rng, rows, n, torch.float32, cuda_device, std=1.0)
+    want, l1 = reference(oracle, c, g_host)
+
+    def make(hint, deterministic=True, matrix=x, nnz=x.nnz, rows=rows, cols=cols):
+        return ops.PreparedSpmm(capi.PROJECTION_TRANSPOSE, rows, cols, n, nnz, 8, 1, torch.float32, cuda_device, device_matrix=matrix, deterministic=deterministic, schedule=hint)
+    for hint, name, digits in ((None, "gene_gather", 0), ("gene_gather", "gene_gather", 0), ("integer_windows", "integer_windows", 4)):
+        op = make(hint)
+        assert (op.schedule, op.digits) == (name, digits)
+        got = op.run(x, g, torch.empty(cols, n, device=cuda_device)).cpu().numpy()
+        assert op.status() == 0
+        if digits:
+            assert_within(got, want, l1, g_host, 4)
+        op.close()
+    for op, name, digits in ((make("tensor_blocked", False), "tensor_blocked_x3", 3), (make(None, False, None, 5_000_000, 8_000, 4_000), "vector_reductions", 4),
+                             (make(None, False, None, 100_000, 8_000, 4_000), "vector_reductions", 0)):
+        assert (op.schedule, op.digits) == (name, digits)
+        op.close()

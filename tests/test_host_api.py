@@ -200,3 +200,22 @@ def test_routed_scratch_is_what_the_calls_use(bits):
     assert need.value < back.value <= need.value + (40 << 20)
     l.layout, l.block_size, l.ell_cols, l.block_col_idx = capi.PUBLIC_LAYOUT_QUANTIZED_BLOCKED_ELL, 32, 64, 256
     assert L.cb200_public_projection_scratch(C.byref(l), C.c_int64(64), C.byref(need)) == capi.SUCCESS and need.value <= 512
+
+
+@pytest.mark.parametrize("rows,cols,nnz,chosen", [(1_000_000, 33_538, 1_800_000_000, 4), (3_000, 2_000, 600_000, 5)])
+def test_each_repeatable_transpose_has_a_name_of_its_own(rows, cols, nnz, chosen):
+    """What prepare would keep: words of four bytes an entry by the name "integer_windows" (at any size) and without a name where the matrix is large,
+    the gene-major copy's five by "gene_gather" and without a name where it is small."""
+    m = capi.header(capi.QCsr())
+    m.rows, m.cols, m.nnz, m.bits, m.policy = rows, cols, nnz, 8, 1
+
+    def bytes_an_entry(hint):
+        pr = capi.header(capi.SpmmProblem())
+        pr.projection, pr.m, pr.k, pr.n, pr.nnz, pr.bits, pr.policy, pr.dense_dtype = capi.PROJECTION_TRANSPOSE, rows, cols, 64, nnz, 8, 1, capi.DTYPE_F32
+        pr.structure_epoch, pr.deterministic, pr.device_matrix, pr.schedule_hint = 1, 1, C.pointer(m), hint
+        need = C.c_uint64()
+        assert capi.lib().cb200_spmm_persistent_requirement(C.byref(pr), C.byref(need)) == capi.SUCCESS
+        return need.value / nnz
+    words, gathered = bytes_an_entry(b"integer_windows"), bytes_an_entry(b"gene_gather")
+    assert 4.0 <= words < 4.4 and gathered >= 5.0
+    assert bytes_an_entry(None) == (words if chosen == 4 else gathered)
