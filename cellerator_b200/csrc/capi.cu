@@ -396,7 +396,7 @@ schedule_plan plan_schedule(const cb200_spmm_problem &pr) {
                                    qcsr_transpose_blocked_shape_ok(pr.m, pr.k, pr.n, pr.bits) && (limit == 0u || nnz * 4u <= limit);
         if (pr.deterministic && !named_blocked) {
             const bool large = plan.mean_row_nnz >= 0.02 * static_cast<double>(pr.k) && pr.m * pr.k >= (1ll << 23);
-            if (digits_ok && (hint_is(hint, "integer_windows") || (hint == nullptr && large))) {
+            if (digits_ok && pr.m <= qcsr_transpose_exact_rows && (hint_is(hint, "integer_windows") || (hint == nullptr && large))) {
                 plan.digits = 4;
                 return plan;
             }

@@ -219,3 +219,17 @@ def test_each_repeatable_transpose_has_a_name_of_its_own(rows, cols, nnz, chosen
     words, gathered = bytes_an_entry(b"integer_windows"), bytes_an_entry(b"gene_gather")
     assert 4.0 <= words < 4.4 and gathered >= 5.0
     assert bytes_an_entry(None) == (words if chosen == 4 else gathered)
+
+
+def test_the_totals_of_a_repeatable_transpose_fit_64_bits():
+    """A gene that more than 2^25 cells hold, with the largest codes and a constant G, could leave them: fp32 sums gene by gene from there on."""
+    def bytes_an_entry(rows):
+        m = capi.header(capi.QCsr())
+        m.rows, m.cols, m.nnz, m.bits, m.policy = rows, 64, 4 * rows, 8, 1
+        pr = capi.header(capi.SpmmProblem())
+        pr.projection, pr.m, pr.k, pr.n, pr.nnz, pr.bits, pr.policy, pr.dense_dtype = capi.PROJECTION_TRANSPOSE, rows, 64, 64, 4 * rows, 8, 1, capi.DTYPE_F32
+        pr.structure_epoch, pr.deterministic, pr.device_matrix = 1, 1, C.pointer(m)
+        need = C.c_uint64()
+        assert capi.lib().cb200_spmm_persistent_requirement(C.byref(pr), C.byref(need)) == capi.SUCCESS
+        return need.value / (4 * rows)
+    assert bytes_an_entry(2 ** 25 - 1) < 5.0 <= bytes_an_entry(2 ** 25)
