@@ -1107,7 +1107,8 @@ struct finish_params {
 };
 
 __host__ __device__ constexpr int finish_threads(int nb) { return nb / 16 * kWin; }
-constexpr int finish_smem_bytes(int nb) { return kWin * nb * 8 + kWin * (nb / 4) * 16; }
+__host__ __device__ constexpr int finish_pitch(int nb) { return nb + 4; } // of a gene's results in shared memory: 16-byte stores of a warp's 32 genes meet no bank twice
+constexpr int finish_smem_bytes(int nb) { return kWin * nb * 8 + std::max(kWin * (nb / 4) * 16, kWin * finish_pitch(nb) * 4); }
 // f(word, gene within the window, row), a word of the window to a lane and 32 at a time, for the warp's share of the pieces of the row range that
 // wanted(first row, base) lets through.  Lanes without a word of the range have kPadding.
 template<typename W, typename F>
@@ -1239,10 +1240,11 @@ __device__ __noinline__ void beside_tiles(const finish_params &p, int mode, bool
 // What genes that a cell holds again (kAgain) and infinities and NaNs of G come to is added here.  Where G spreads too far for fixed point, or a scale or a zero-point of the window is not
 // finite (0 * infinity, in a product of sums, would reach cells that hold no entry): everything, entry by entry (beside_tiles, which is no part
 // of this function's registers: two CTAs of 512 threads to an SM, or the 262 of 33,538 genes take two rounds, 12 us instead of 9).
-// A thread has a gene and sixteen columns, so that a warp's loads are contiguous.
+// A thread has a gene and sixteen columns, so that a warp's loads are contiguous; the results change places in shared memory, so that
+// its stores are too (10.6 us otherwise).
 template<int NB, bool EXACT>
 __global__ void __launch_bounds__(finish_threads(NB), 1024 / finish_threads(NB)) finish_kernel(const __grid_constant__ finish_params p) {
-    extern __shared__ double beside[]; // [kWin][NB], and behind it [kWin][NB / 4] {codes, ones}
+    extern __shared__ __align__(16) double beside[]; // [kWin][NB], and behind it [kWin][NB / 4] {codes, ones}, later the results
     constexpr int kSet = set_windows(NB, kMostSlices);
     static_assert(kSet == set_windows(NB, 3), "the sets of a launch do not follow from its mode");
     __shared__ float2 meta[kWin];
@@ -1268,69 +1270,72 @@ __global__ void __launch_bounds__(finish_threads(NB), 1024 / finish_threads(NB))
     // the set's slots: the CTAs whose shares meet its runs, run after run, pass after pass
     const std::int64_t total = sets * p.d.column_blocks * p.d.group_count * passes, L = p.d.group_count, cuts = (L + p.d.run_groups - 1) / p.d.run_groups;
     const int gl = tid & (kWin - 1);
-    const std::int64_t gene = window * kWin + gl;
-    if (gene >= p.d.cols || c0 + c >= p.n) return;
-    double sum[16];
+    const bool mine = window * kWin + gl < p.d.cols && c0 + c < p.n;
+    float *results = reinterpret_cast<float *>(beside + kWin * NB);
+    constexpr int kPitch = finish_pitch(NB), kAtOnce = EXACT ? 8 : 16; // columns
+#pragma unroll 1
+    for (int h = 0; h < 16; h += kAtOnce) {
+        double sum[kAtOnce];
 #pragma unroll
-    for (int k = 0; k < 16; ++k) sum[k] = 0.0;
-    if (more) {
-#pragma unroll
-        for (int k = 0; k < 16; ++k) sum[k] = beside[gl * NB + c + k];
-    }
-    if (!by_entry) {
-        for (int pass = 0; pass < passes; ++pass) {
+        for (int k = 0; k < kAtOnce; ++k) sum[k] = more ? beside[gl * NB + c + h + k] : 0.0;
+        for (int pass = 0; pass < passes && !by_entry && mine; ++pass) {
             const std::int64_t block = static_cast<std::int64_t>(pass) * p.d.column_blocks + blockIdx.y, set_of_all = block * sets + set;
             if constexpr (EXACT) {
                 const double scale = static_cast<double>(meta[gl].x), offset = static_cast<double>(meta[gl].y);
-                const long long *at = p.d.totals + ((set_of_all * kSet + wl) * 2 * NB + c) * kWin + gl;
-                const double *steps = p.d.steps + block * NB + c;
+                const long long *at = p.d.totals + ((set_of_all * kSet + wl) * 2 * NB + c + h) * kWin + gl;
+                const double *steps = p.d.steps + block * NB + c + h;
+                long long coded[kAtOnce], present[kAtOnce];
 #pragma unroll
-                for (int h = 0; h < 16; h += 8) {
-                    long long coded[8], present[8];
-#pragma unroll
-                    for (int k = 0; k < 8; ++k) {
-                        coded[k] = __ldcg(at + (h + k) * kWin);
-                        present[k] = __ldcg(at + (NB + h + k) * kWin);
-                    }
-#pragma unroll
-                    for (int k = 0; k < 8; ++k) sum[h + k] += value_of(coded[k], present[k], p.d.code_bias, scale, offset, __ldg(steps + h + k));
+                for (int k = 0; k < kAtOnce; ++k) {
+                    coded[k] = __ldcg(at + k * kWin);
+                    present[k] = __ldcg(at + (NB + k) * kWin);
                 }
+#pragma unroll
+                for (int k = 0; k < kAtOnce; ++k) sum[k] += value_of(coded[k], present[k], p.d.code_bias, scale, offset, __ldg(steps + k));
             } else {
                 for (std::int64_t cut = 0; cut < cuts; ++cut) {
                     const std::int64_t from = set_of_all * L + cut * p.d.run_groups, to = min(from + p.d.run_groups, (set_of_all + 1) * L);
                     const std::int64_t last = cta_of(to - 1, total, p.grid);
                     for (std::int64_t b = cta_of(from, total, p.grid); b <= last; ++b) {
                         const float *slot = p.d.partials + (((set_of_all * cuts + cut + b) * kSet + wl) * NB + c) * kWin + gl;
-                        float u[16];
+                        float u[kAtOnce];
 #pragma unroll
-                        for (int k = 0; k < 16; ++k) u[k] = __ldcg(slot + k * kWin);
+                        for (int k = 0; k < kAtOnce; ++k) u[k] = __ldcg(slot + k * kWin);
 #pragma unroll
-                        for (int k = 0; k < 16; ++k) sum[k] += static_cast<double>(u[k]);
+                        for (int k = 0; k < kAtOnce; ++k) sum[k] += static_cast<double>(u[k]);
                     }
                 }
             }
         }
-    }
-    float v[16];
 #pragma unroll
-    for (int k = 0; k < 16; ++k) v[k] = static_cast<float>(sum[k]);
-    float *dst = p.out + gene * p.out_ld + c0 + c;
+        for (int k = 0; k < kAtOnce; k += 4)
+            *reinterpret_cast<float4 *>(results + gl * kPitch + c + h + k) =
+                make_float4(static_cast<float>(sum[k]), static_cast<float>(sum[k + 1]), static_cast<float>(sum[k + 2]), static_cast<float>(sum[k + 3]));
+    }
+    __syncthreads();
+    const int genes = static_cast<int>(min(static_cast<std::int64_t>(kWin), p.d.cols - window * kWin)), columns = min(NB, p.n - c0);
+    float *out = p.out + window * kWin * p.out_ld + c0;
     if (p.out_vector != 0) {
 #pragma unroll
-        for (int k = 0; k < 16; k += 4) {
-            if (c0 + c + k >= p.n) break;
+        for (int i = tid; i < kWin * (NB / 4); i += finish_threads(NB)) {
+            const int gene = i / (NB / 4), at = i % (NB / 4) * 4;
+            if (gene >= genes || at >= columns) continue;
+            float4 *dst = reinterpret_cast<float4 *>(out + gene * p.out_ld + at);
+            const float4 v = *reinterpret_cast<const float4 *>(results + gene * kPitch + at);
             float4 o = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             if (p.beta != 0.0f) {
-                o = *reinterpret_cast<const float4 *>(dst + k);
+                o = *dst;
                 o.x *= p.beta; o.y *= p.beta; o.z *= p.beta; o.w *= p.beta;
             }
-            *reinterpret_cast<float4 *>(dst + k) =
-                make_float4(fmaf(p.alpha, v[k], o.x), fmaf(p.alpha, v[k + 1], o.y), fmaf(p.alpha, v[k + 2], o.z), fmaf(p.alpha, v[k + 3], o.w));
+            *dst = make_float4(fmaf(p.alpha, v.x, o.x), fmaf(p.alpha, v.y, o.y), fmaf(p.alpha, v.z, o.z), fmaf(p.alpha, v.w, o.w));
         }
     } else {
-#pragma unroll
-        for (int k = 0; k < 16; ++k)
-            if (c0 + c + k < p.n) dst[k] = fmaf(p.alpha, v[k], p.beta == 0.0f ? 0.0f : p.beta * dst[k]);
+        for (int i = tid; i < kWin * NB; i += finish_threads(NB)) {
+            const int gene = i / NB, at = i % NB;
+            if (gene >= genes || at >= columns) continue;
+            float *dst = out + gene * p.out_ld + at;
+            *dst = fmaf(p.alpha, results[gene * kPitch + at], p.beta == 0.0f ? 0.0f : p.beta * *dst);
+        }
     }
 }
 
