@@ -36,8 +36,8 @@
 // What bounds it: at S = 4, N = 64 the tensor pipe, sixteen 128 x 256 x 32 MMAs of 128 cycles in the 2,410 cycles of a tile; at S = 3
 // the scatter groups' chain (release, zeroes, two one-byte stores a word, fence, hand-over), 2,125 cycles against 1,536 of MMAs; over a
 // second of launches the power cap (1.6 GHz).  One B200, start of this kernel's life -> now: 125,000 x 33,538, N = 64, S = 3 1,645 (bf16
-// products) -> 1,186 us; 100,003 cells, S = 4 2,879 (rows of G gathered gene by gene) -> 1,087; 8,191 cells, S = 4 with the words made in
-// the call 313 (sorted in shared memory) -> 171.  With one row of G at 1e6: 1,511 -> 2,090, 2,641 -> 1,970, 313 -> 258; Student-t numbers with
+// products) -> 1,170 us; 100,003 cells, S = 4 2,879 (rows of G gathered gene by gene) -> 1,096; 8,191 cells, S = 4 with the words made in
+// the call 313 (sorted in shared memory) -> 175.  With one row of G at 1e6: 1,511 -> 2,090, 2,641 -> 1,970, 313 -> 258; Student-t numbers with
 // three degrees of freedom (four digits in one pass instead of three in two, 2,014 us): 125,000 cells, S = 3 1,204.
 #include "dependent_launch.cuh"
 #include "kernels.cuh"

@@ -328,8 +328,8 @@ cb200_status cb200_spmm_prepare(const cb200_spmm_problem *problem, cb200_prepare
 cb200_status cb200_spmm_persistent_requirement(const cb200_spmm_problem *problem, uint64_t *bytes);
 void cb200_prepared_destroy(cb200_prepared *prepared);
 /* workspace_requirement, launch_bindings.hh:67-71: what the schedule can use.  "vector_reductions" reports up to 32 MB (it
- * sorts the entries with it, slice of rows by slice), or for 2 to 50 million entries about 4 bytes an entry (words for integer
- * sums), and also runs with less or with none, slower.  A deterministic transpose with integer sums reports 8 N bytes a cell
+ * sorts the entries with it, slice of rows by slice), or for 2 to 50 million entries about 4 bytes an entry, 8 N a cell and 25 to 60 MB (words,
+ * digits and sums of the integer kernel), and also runs with less or with none, slower.  A deterministic transpose with integer sums reports 8 N bytes a cell
  * and 32 N a gene (N up to 32 or to a multiple of 64) and also runs with less, slower and with the same bits, down to 512 of these cells and
  * 512 of these genes (N <= 32: 1,024) and 256 KB; less is refused.  "warp_per_row" (unaligned
  * N) and the tensor_blocked and tensor_dense forward schedules also run with less, down to the status block and the records of
