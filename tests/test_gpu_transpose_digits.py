@@ -143,7 +143,7 @@ def test_what_integer_sums_do_not_cover(cuda_device, oracle, slices):
         assert np.all(np.abs(got[finite] - want[finite]) <= 2.0 ** -22 * scale[finite] + 1e-30)
 
     check()
-    g_host[77, 5] = 1e6                                               # in double precision, one rounding at the end
+    g_host[77, 5] = 1e6                                               # a second pass of digits
     check()
     g_host[123, 9], g_host[4000, 9], g_host[4001, 11] = np.inf, -np.inf, np.nan
     check()
