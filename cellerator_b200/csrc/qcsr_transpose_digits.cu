@@ -31,7 +31,8 @@
 // of 256 cells x 128 genes (32 KB of codes, 32 KB of ones, K-major with the 128-byte swizzle) and scatter its words; warp 16
 // issues the MMAs (M = genes, K = cells, N = S digits x the columns of G); warp 18 feeds the ring of G; warps 17 and 19 the
 // words, each to one of the groups.  The two sums of a window take 2 S N columns of tensor memory, all 512 at S = 4, N = 64, and stay there while
-// the CTA walks the groups of its run.  Every wait is bounded (sm100_primitives.cuh).
+// the CTA walks the groups of its run.  Every wait is bounded (sm100_primitives.cuh); if one runs out, the status word is set and the last kernel
+// adds the entries up by itself, ten to fifty times slower: the callers of a call without a handle cannot ask for the status.
 //
 // What bounds it: at S = 4, N = 64 the tensor pipe, sixteen 128 x 256 x 32 MMAs of 128 cycles in the 2,410 cycles of a tile; at S = 3
 // the scatter groups' chain (release, zeroes, two one-byte stores a word, fence, hand-over), 2,125 cycles against 1,536 of MMAs; over a
@@ -1238,8 +1239,9 @@ __device__ __noinline__ void beside_tiles(const finish_params &p, int mode, bool
 
 // G'[genes of one window, columns of one block] = beta * G' + alpha * (the sums of the set's runs, added in run order; EXACT: the totals).
 // What genes that a cell holds again (kAgain) and infinities and NaNs of G come to is added here.  Where G spreads too far for fixed point, or a scale or a zero-point of the window is not
-// finite (0 * infinity, in a product of sums, would reach cells that hold no entry): everything, entry by entry (beside_tiles, which is no part
-// of this function's registers: two CTAs of 512 threads to an SM, or the 262 of 33,538 genes take two rounds, 12 us instead of 9).
+// finite (0 * infinity, in a product of sums, would reach cells that hold no entry), or a wait of the main kernel ran out: everything, entry by entry
+// (beside_tiles, which is no part of this function's registers: two CTAs of 512 threads to an SM, or the 262 of 33,538 genes take two rounds, 12
+// us instead of 9).
 // A thread has a gene and sixteen columns, so that a warp's loads are contiguous; the results change places in shared memory, so that
 // its stores are too (10.6 us otherwise).
 template<int NB, bool EXACT>
@@ -1264,6 +1266,7 @@ __global__ void __launch_bounds__(finish_threads(NB), 1024 / finish_threads(NB))
         odd = isfinite(so.x) && isfinite(so.y) ? 0 : 1;
     }
     const int mode = __ldcg(p.d.mode);
+    if (__ldcg(p.d.status) != 0) odd = 1;
     const bool by_entry = __syncthreads_or(odd) != 0 || (mode & kByEntry) != 0, more = by_entry || (mode & (kRepeats | kNonFinite)) != 0;
     if (more) beside_tiles<NB>(p, mode, by_entry, window, meta, beside, reinterpret_cast<unsigned long long *>(beside + kWin * NB));
     const int passes = passes_of(mode), c = tid / kWin * 16;

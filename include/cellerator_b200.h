@@ -357,8 +357,9 @@ cb200_status cb200_prepared_output_shape(const cb200_prepared *prepared, uint64_
 /* launch_bindings, launch_bindings.hh:90-102: everything that changes per launch.
  *
  * Status word.  The kernels wait on barriers with a bound; when a bound runs out the launch ends early,
- * its output is not valid, and the first 32-bit word of `workspace` is non-zero afterwards.  Every launch
- * clears that word on its stream first.  cb200_spmm_run cannot report it (it returns before the kernels
+ * its output is not valid, and the first 32-bit word of `workspace` is non-zero afterwards (a transpose with
+ * integer sums, cb200_prepared_digits, has then added the entries up one by one: its output is whole).  Every
+ * launch clears that word on its stream first.  cb200_spmm_run cannot report it (it returns before the kernels
  * run): read it with cb200_prepared_status once the stream has passed the launch. */
 typedef struct cb200_launch {
     uint32_t version;

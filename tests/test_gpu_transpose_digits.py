@@ -177,6 +177,50 @@ def test_bounded_wait_path(cuda_device, oracle):
     op.close()
 
 
+@pytest.mark.parametrize("slices,room", [(3, 1.0), (3, 0.8), (4, 1.0), (4, 0.3), (0, 1.0)])
+def test_sums_are_whole_when_a_wait_ran_out(cuda_device, oracle, slices, room):
+    """The status word is set, and the launch's last kernel has added the entries up by itself: a call that keeps no handle to ask has its result.
+    Slices of the groups; a row range; 0 digits: the words made in the call, and the one-call function."""
+    rng = np.random.default_rng(slices)
+    rows, cols, n = (2111, 1500, 50) if slices == 0 else (256 * 20 + 9, 1664, 64)
+    c = host_pack(oracle, random_csr(rng, rows=rows, cols=cols, max_nnz=3000 if slices == 0 else 120, bits=8))
+    x = to_dev(c, cuda_device)
+    g, g_host = dense(rng, rows, n, torch.float32, cuda_device, std=1.0)
+    op = prepared(x, n, slices, cuda_device) if slices else ops.PreparedSpmm(capi.PROJECTION_TRANSPOSE, rows, cols, n, x.nnz, 8, 1, torch.float32, cuda_device)
+    op.workspace_bytes = int(op.workspace_bytes * room)
+    init = rng.normal(size=(cols, n)).astype(np.float32)
+    for lo, hi in ((0, rows), (5, rows - 40)):
+        want, l1 = reference(oracle, c, g_host, lo, hi)
+        outs = []
+        for polls in (4096, 4096, 0):
+            out = torch.from_numpy(init).to(cuda_device)
+            if polls:
+                capi.lib().cb200_test_arm_wait_timeout(polls)
+            try:
+                op.run(x, g, out, alpha=2.0, beta=0.5, row_begin=lo, row_end=hi)
+            finally:
+                capi.lib().cb200_test_disarm_wait_timeout()
+            if polls:
+                with pytest.raises(capi.Cb200Error) as e:
+                    op.status()
+                assert e.value.status == capi.DEVICE_WAIT_TIMEOUT
+            else:
+                assert op.status() == 0
+            outs.append(out.cpu().numpy())
+            # in 64 bits where the wait ran out: inside the bound of the digits
+            assert_within(outs[-1], 2.0 * want + 0.5 * init, 2.0 * l1 + 1.0, np.maximum(np.abs(g_host[lo:hi]), 1.0), 3 if polls == 0 and slices == 3 else 4)
+        assert np.array_equal(outs[0], outs[1])
+    op.close()
+    if slices == 0:
+        want, l1 = reference(oracle, c, g_host)
+        capi.lib().cb200_test_arm_wait_timeout(4096)
+        try:
+            out = ops.spmm_transpose(x, g)
+        finally:
+            capi.lib().cb200_test_disarm_wait_timeout()
+        assert_within(out.cpu().numpy(), want, l1, g_host, 4)
+
+
 @pytest.mark.parametrize("n,bits,outlier", [(64, 8, 1.0), (32, 4, 1.0), (128, 8, 1e6)])
 def test_repeatable_bits_do_not_follow_from_the_workspace(cuda_device, oracle, n, bits, outlier):
     """Row groups in slices, windows in chunks, one pass of digits and two: whatever the room is, down to the least that is accepted."""
