@@ -215,8 +215,9 @@ struct digit_layout {
     const void *src_row_ptr = nullptr, *src_col_idx = nullptr, *src_packed = nullptr; // arrays it was built from
 };
 constexpr std::int64_t kDigitWordsTwice = 1ll << 62;
-// Of a repeatable launch: |code| <= 128 times a number of 31 bits, so many times, stays inside the totals' 64 bits.
-constexpr std::int64_t qcsr_transpose_exact_rows = (1ll << 25) - 1;
+// Of a repeatable launch: a code of up to 255 times a number below 0.996 * 2^31, so many times, stays inside the 64 bits of the totals and of what is
+// put together from them (value_of).
+constexpr std::int64_t qcsr_transpose_exact_rows = 1ll << 24;
 bool qcsr_transpose_digits_shape_ok(std::int64_t rows, std::int64_t cols, std::int64_t n, int bits, int policy);
 std::uint64_t qcsr_digit_words_bytes_bound(std::int64_t rows, std::int64_t cols, std::int64_t nnz);
 // current device; memory from `arena`, kernels on `stream`, which is waited for

@@ -735,7 +735,8 @@ struct tile_cursor {
         windows_of_set = windows_in(set);
     }
 };
-// A gene's sum in one column.  The sums are below 2^57: in double precision scale and offset may cancel to the last bits of fp32.
+// A gene's sum in one column.  A run's sums are below 2^56, totals below 2^63 (qcsr_transpose_exact_rows), so the whole numbers do not leave their 64
+// bits: in double precision scale and offset may cancel to the last bits of fp32.
 __device__ __forceinline__ double value_of(long long coded, long long present, int code_bias, double scale, double offset, double step) {
     return (scale * static_cast<double>(coded + code_bias * present) + offset * static_cast<double>(present)) * step;
 }

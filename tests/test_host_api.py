@@ -222,7 +222,11 @@ def test_each_repeatable_transpose_has_a_name_of_its_own(rows, cols, nnz, chosen
 
 
 def test_the_totals_of_a_repeatable_transpose_fit_64_bits():
-    """A gene that more than 2^25 cells hold, with the largest codes and a constant G, could leave them: fp32 sums gene by gene from there on."""
+    """A gene that more than 2^24 cells hold, with the largest codes and a constant G, could leave them: fp32 sums gene by gene from there on.  A code
+    of up to 255 times a number of up to 0.99 * 2^31 (a column's largest takes 0.99 of the digits' range), so many times, for the sum of the products;
+    the total of the codes less 128 and 128 times the total of the ones, from which it is put together, are smaller."""
+    most = int(0.99 * 2 ** 31) * 255
+    assert most * 2 ** 24 < 2 ** 63 <= most * 2 ** 25
     def bytes_an_entry(rows):
         m = capi.header(capi.QCsr())
         m.rows, m.cols, m.nnz, m.bits, m.policy = rows, 64, 4 * rows, 8, 1
@@ -232,4 +236,4 @@ def test_the_totals_of_a_repeatable_transpose_fit_64_bits():
         need = C.c_uint64()
         assert capi.lib().cb200_spmm_persistent_requirement(C.byref(pr), C.byref(need)) == capi.SUCCESS
         return need.value / (4 * rows)
-    assert bytes_an_entry(2 ** 25 - 1) < 5.0 <= bytes_an_entry(2 ** 25)
+    assert bytes_an_entry(2 ** 24) < 5.0 <= bytes_an_entry(2 ** 24 + 1)
