@@ -515,7 +515,9 @@ const char *schedule_name(std::uint32_t variant) noexcept {
     case schedule_gene_tiled: fraction = 0.070; break;
     case schedule_tensor_windows: fraction = 0.062; break;
     case schedule_tensor_blocked:
-        fraction = transpose ? (split ? 0.128 : 0.275) : (split ? (shape.dense_dtype == CB200_DTYPE_BF16 ? 0.150 : 0.100) : 0.300);
+        if (!transpose) fraction = split ? (shape.dense_dtype == CB200_DTYPE_BF16 ? 0.150 : 0.100) : 0.300;
+        else if (!split) fraction = 0.275;
+        else fraction = shape.decode_policy == CB200_DECODE_PER_GENE_AFFINE ? 0.128 : 0.110; // integer sums; bf16 passes (zero-points per row)
         break;
     case schedule_tensor_dense: fraction = 0.395; break;
     case schedule_tensor_codes: fraction = 0.570; break;

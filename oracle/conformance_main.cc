@@ -182,6 +182,12 @@ static void planner_leg(const core::candidate_registry &registry) {
           "planner: the integer kernels' words (4 B per entry) and the gene-major copy (5 B per entry) are declared");
     CHECK(transposes[3].analytical.kernel_ns < 0.5 * transposes[2].analytical.kernel_ns && transposes[3].analytical.transient_bytes > 500000000ull,
           "planner: each repeatable transpose has the time and the workspace of the kernel its name selects");
+    host::projection_catalog_entry per_row = ts;
+    per_row.decode_policy = CB200_DECODE_COLUMN_SCALE_ROW_OFFSET;
+    const double per_gene_ns = host::make_schedule_candidate(*tr, t.projection, ts, host::schedule_tensor_blocked, CB200_DTYPE_F32, 6553.9).analytical.kernel_ns;
+    const double per_row_ns = host::make_schedule_candidate(*tr, t.projection, per_row, host::schedule_tensor_blocked, CB200_DTYPE_F32, 6553.9).analytical.kernel_ns;
+    CHECK(per_row_ns > 1.1 * per_gene_ns && per_row_ns < 1.25 * per_gene_ns,
+          "planner: the split transpose with zero-points per row has the time of its bf16 passes, not the integer sums'");
     pl::planner_request treq = request_for(t, transposes, 3u);
     st = pl::plan_end_to_end(treq, &res);
     CHECK(static_cast<bool>(st) && res.legal_count == 3u && variant_of(res) == host::schedule_tensor_blocked,
