@@ -1266,9 +1266,9 @@ __global__ void __launch_bounds__(finish_threads(NB), 1024 / finish_threads(NB))
         meta[tid] = so;
         odd = isfinite(so.x) && isfinite(so.y) ? 0 : 1;
     }
-    const int mode = __ldcg(p.d.mode);
-    if (__ldcg(p.d.status) != 0) odd = 1;
-    const bool by_entry = __syncthreads_or(odd) != 0 || (mode & kByEntry) != 0, more = by_entry || (mode & (kRepeats | kNonFinite)) != 0;
+    const int2 head = __ldcg(reinterpret_cast<const int2 *>(p.d.status)); // {status, mode}
+    const int mode = head.y;
+    const bool by_entry = __syncthreads_or(odd) != 0 || (mode & kByEntry) != 0 || head.x != 0, more = by_entry || (mode & (kRepeats | kNonFinite)) != 0;
     if (more) beside_tiles<NB>(p, mode, by_entry, window, meta, beside, reinterpret_cast<unsigned long long *>(beside + kWin * NB));
     const int passes = passes_of(mode), c = tid / kWin * 16;
     // the set's slots: the CTAs whose shares meet its runs, run after run, pass after pass
@@ -1610,7 +1610,7 @@ cb200_status launch_qcsr_transpose_digits(const qcsr_view &x, const dense_args &
     k.odd_rows = reinterpret_cast<unsigned short *>(ws + kRecordsAt);
     k.records = ws + kRecordsAt + odd_bytes(group_count, d.n);
     k.bases = p.bases; k.word_pieces = p.pieces;
-    k.mode = reinterpret_cast<int *>(ws) + 1;
+    k.mode = reinterpret_cast<int *>(ws) + 1; // finish_kernel reads both words at once
     p.records = k.records; p.steps = k.steps; p.mode = k.mode;
     p.cols = x.cols;
     p.group_begin = group_begin;
