@@ -370,7 +370,7 @@ __global__ void __launch_bounds__(kTableThreads, 1) codec_table_kernel(const cod
                             else edge_code = __ldg(codes + edge);
                         }
                         const auto quad_step = [&](auto whole, int at) {
-                                                        const int e0 = at + lane * 4;
+                            const int e0 = at + lane * 4;
                             const auto there = [&](int q) { return decltype(whole)::value || (e0 + q * 128 >= first4 && e0 + q * 128 < last4); };
                             const std::int32_t *step_cols = cols + e0;
                             float *step_values = values + e0;
